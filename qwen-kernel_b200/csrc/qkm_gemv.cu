@@ -101,6 +101,7 @@ cudaError_t launch_gemv_tail(const Launch& L, uint32_t type, const void* W, cons
 // consumed.  Each warp then takes rows of the tile: lanes stride over 8-element units,
 // decode them from shared memory (where the 2-byte alignment of ggml blocks costs nothing)
 // and multiply with x held in shared memory; f32 accumulation, one shuffle tree per row.
+constexpr uint64_t kSplitMinWeights = 4u << 20, kSplitMaxWeights = 32u << 20;
 constexpr size_t kDirectMaxBytes = 48u << 20;   // above this the persistent, staged kernel wins
 
 namespace gv {
@@ -347,10 +348,23 @@ cudaError_t launch_gemv_stream(const Launch& L, uint32_t type, const void* W, co
     const uint8_t* w = (const uint8_t*)W;
     uint32_t done = 0;
     cudaError_t e;
+    // Several rows of x, and one row where latency rather than the rate of unpacking sets the time, take the K-split
+    // form.  One row: below 4 M weights (2048 x 2048) the one-wave kernel is ahead (1000 x 2048: 3.5 us against 4.4),
+    // above 32 M the persistent kernels at the end (24576 x 2048, Q6_K: 15.7 against 19.4); between them it leads
+    // (Q6_K 4096 x 2048: 6.4 against 8.0, 6000 x 2048: 7.8 against 11.0; Q8_0 16384 x 2048: 12.4 against 18.2).  F16 rows
+    // need no unpacking: one wave wins at every size.  IQ3_XXS has no other tensor-core form (65,536 x 2048: 38 against 58).
+    const uint64_t weights = (uint64_t)M * K;
+    const bool split1 = type != QKM_TYPE_F16 && weights > kSplitMinWeights && (weights <= kSplitMaxWeights || type == QKM_TYPE_IQ3_XXS);
+    if (n > 1 || split1) {
+        uint32_t rows = 0;
+        e = launch_gemv_split(L, type, w, x, y, M, K, n, n_sms, &rows);
+        if (e != cudaSuccess || rows == n) return e;
+        x += (size_t)rows * K; y += (size_t)rows * M; n -= rows;
+    }
     const bool aligned = !((uintptr_t)W & 15u) && !((uintptr_t)x & 15u) && (type != QKM_TYPE_IQ4_XS || K % 256 == 0);
-    // (the integer tensor-core kernels win from about 8192 rows on for the two formats whose unpacking is costly)
-    const bool try_mma_small = M >= 8192 && (type == QKM_TYPE_Q6_K || type == QKM_TYPE_IQ4_XS);
-    if (n == 1 && aligned && (size_t)M * row_bytes(type, K) <= kDirectMaxBytes && type != QKM_TYPE_F32 && !try_mma_small) {
+    // (what the K-split form leaves: few weights, or many that the tensor-core kernels below take whatever their bytes)
+    if (n == 1 && aligned && (size_t)M * row_bytes(type, K) <= kDirectMaxBytes && type != QKM_TYPE_F32 &&
+        (type == QKM_TYPE_F16 || weights <= kSplitMaxWeights)) {
         switch (type) {
             case QKM_TYPE_F16: return gemv_direct_launch<QKM_TYPE_F16>(L, w, x, y, M, K);
             case QKM_TYPE_Q8_0: return gemv_direct_launch<QKM_TYPE_Q8_0>(L, w, x, y, M, K);

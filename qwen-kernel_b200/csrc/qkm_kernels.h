@@ -7,6 +7,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <atomic>
+
 #include "../../include/qk_moe.h"
 
 namespace qkm {
@@ -30,6 +32,19 @@ inline cudaError_t launch_kernel(const Launch& L, void (*kernel)(KArgs...), dim3
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr; cfg.numAttrs = L.pdl ? 1 : 0;
     return cudaLaunchKernelEx(&cfg, kernel, KArgs(args)...);
+}
+
+// Raises a kernel's dynamic shared-memory limit, once per device (the call costs the host about as much as a launch).
+template <auto Kernel>
+inline cudaError_t allow_dynamic_smem(int bytes) {
+    static std::atomic<uint64_t> done{0};   // a bit per device
+    int dev = 0;
+    if (const cudaError_t e = cudaGetDevice(&dev)) return e;
+    const uint64_t bit = 1ull << (dev & 63);
+    if (done.load(std::memory_order_relaxed) & bit) return cudaSuccess;
+    const cudaError_t e = cudaFuncSetAttribute(Kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    if (e == cudaSuccess) done.fetch_or(bit, std::memory_order_relaxed);
+    return e;
 }
 
 #ifdef __CUDACC__
@@ -183,6 +198,9 @@ cudaError_t launch_gemv(const Launch& L, uint32_t type, const void* W, const flo
 // streamed form (bulk-copy ring) with the generic kernel for tail rows / unaligned tensors
 cudaError_t launch_gemv_mma(const Launch& L, uint32_t type, const void* W, const float* x, float* y, uint32_t M,
                             uint32_t K, uint32_t n_sms, uint32_t* status, uint32_t* rows_done);
+// 1..16 rows of x a pass, K split over a cluster of blocks (qkm_gemv_split.cu); x rows [0, *rows_done) are done
+cudaError_t launch_gemv_split(const Launch& L, uint32_t type, const void* W, const float* x, float* y, uint32_t M, uint32_t K, uint32_t n,
+                              uint32_t n_sms, uint32_t* rows_done);
 cudaError_t launch_gemv_stream(const Launch& L, uint32_t type, const void* W, const float* x, float* y,
                                uint32_t M, uint32_t K, uint32_t n, uint32_t n_sms, uint32_t* status);
 

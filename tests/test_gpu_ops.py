@@ -96,6 +96,28 @@ def test_gemv_tensor_core_forms(ctx, orc, syn, ttype, M, K):
         b.free()
 
 
+@pytest.mark.parametrize("ttype", [1, 8, 14, 23, 18])
+@pytest.mark.parametrize("M,K,n", [(16, 256, 2), (15, 768, 3), (4100, 1280, 5), (2051, 2048, 9), (33, 4096, 16), (40, 512, 19), (4099, 2048, 1),
+                                   (1030, 4352, 1)])
+def test_gemv_k_split(ctx, orc, syn, ttype, M, K, n):
+    """The K-split form: one to eight column slices of unequal size, every count of column tiles, a second pass
+    over more than 16 rows of x, rows that end inside a tile; a row of x with one huge element and a zero row."""
+    W = syn.random_blocks(ttype, M, K, seed=5 * ttype + M)
+    x = syn.random_x(n, K, seed=46)
+    x[0, 7] = 300.0
+    if n > 2:
+        x[2] = 0.0
+    d_w, d_x, d_y = ctx.to_device(W), ctx.to_device(x), ctx.alloc(n * M * 4)
+    ctx.gemv(ttype, d_w, d_x, d_y, M, K, n)
+    got = d_y.download(np.float32, (n, M))
+    want = orc.gemv(ttype, W, x, M, K, threads=orc.hardware_threads())
+    live = np.arange(n) != 2 if n > 2 else slice(None)
+    assert n <= 2 or not got[2].any()
+    assert syn.rel_err_rows(got[live], want[live]) < TOL_F32
+    for b in (d_w, d_x, d_y):
+        b.free()
+
+
 def test_gemv_rejects_bad_shapes(ctx, pkg):
     d = ctx.alloc(4096)
     for ttype, K in ((8, 48), (14, 128), (18, 300), (99, 256)):
