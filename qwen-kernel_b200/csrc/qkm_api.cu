@@ -15,6 +15,7 @@
 
 #include "qkm_common.cuh"
 #include "qkm_kernels.h"
+#include "qkm_tiles.cuh"
 
 using namespace qkm;
 
@@ -24,11 +25,10 @@ struct qkm_layer_dev {
     void* allocs[8] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
     // tile-ordered copies for the streaming kernels (NULL where the type has none)
     void* tiles[8] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
-    bool tiles_ok = false;   // routed gate/up and down both have tiles
-    bool stream_ok = false;  // tiles, and every expert resident: the fused decode / prefill sequences apply
-    bool gu_only = false;    // as stream_ok for gate/up and the shared expert; the down tensor is Q6_K (tiles[4] holds Q6_K tiles)
-    bool fused_ok = false;   // every tensor has tiles and every expert is resident (any supported type mix): the
-                             // three-kernel decode sequence and the tensor-core prefill apply
+    void* router16 = nullptr;  // the router as f16 in the element order of the prefill GEMMs' rows
+    float* w_norm = nullptr;   // [2][resident experts + 1] largest row norm of the gate / up matrices, the shared expert last
+    bool tiles_ok = false;   // every tensor has tiles: the tensor-core sequences apply
+    bool fused_ok = false;   // and every expert is resident: so does the fused decode sequence
 };
 
 struct qkm_ctx {
@@ -57,40 +57,34 @@ struct qkm_ctx {
     int8_t* xplanes = nullptr;        // [max_tokens][4][n_embd]
     float* xscale = nullptr;          // [max_tokens]
     void* hpieces = nullptr;          // [max_tokens*n_used][3][n_ff] bf16
-    StreamItem* items_gu = nullptr;
-    StreamItem* items_dn = nullptr;
     StreamItem* items_sh_gu = nullptr;
     StreamItem* items_sh_dn = nullptr;
-    uint32_t* n_items = nullptr;      // [0] gate/up, [1] down, [2] shared gate/up, [3] shared down
-    float* contrib_s = nullptr;       // [max_tokens][n_used+1][n_embd]
-    uint32_t* arrivals = nullptr;     // [max_tokens][n_embd / unit rows]
+    uint32_t* n_items = nullptr;      // prefill: units of [0] gate/up, [1] down; [2], [3] their tickets
     uint32_t* status = nullptr;       // kernel status word (device)
-    uint32_t shared_plan_n = 0;        // token count the shared expert's decode work lists were last cut for (0: stale)
     uint32_t* route_counter = nullptr; // ticket counter of the selection kernel's grouping tail (device, stays zero)
     // fused decode sequence (router + grouping + planes -> gate/up -> down, three launches)
     bool dec_ok = false;               // dims fit the fused decode kernels
     int8_t* planes8 = nullptr;         // [max_tokens][n_embd/256][8][256]
     uint8_t* lut_gu = nullptr;         // table images the decode kernels copy to shared memory
     uint8_t* lut_dd = nullptr;         // table image of the decode IQ4_XS down kernel
-    uint8_t* lut_pf = nullptr;         // table image of the prefill IQ3_XXS gate/up kernel
-    uint8_t* lut_dn = nullptr;         // table image of the prefill IQ4_XS down kernel
+    uint8_t* lut_pf = nullptr;         // table image of the prefill GEMMs
     uint32_t* status_host = nullptr;  // pinned mirror
     bool shapes_stream_ok = false;
     // prefill (tcgen05) scratch, allocated on first use
     void* xb = nullptr;               // [max_tokens][n_embd] f16, rows scaled by powers of two (xscale undoes it)
-    void* hb = nullptr;               // [max_tokens*(n_used+1)][n_ff] hidden rows by pair position: f16 scaled per row (bf16 on the f32-down path)
+    float* xnorm = nullptr;           // [max_tokens] 2-norms of the rows
+    void* hb = nullptr;               // [max_tokens*(n_used+1)][n_ff] hidden rows by pair position, f16 scaled per row
     float* hscale = nullptr;          // [max_tokens*(n_used+1)] the scales that undo the rows' scaling
     float* contrib_p = nullptr;       // [max_tokens*(n_used+1)][n_embd]
-    MmaItem* mma_items[4] = {nullptr, nullptr, nullptr, nullptr};  // gate/up, down, shared gate/up, shared down
+    MmaItem* mma_items[2] = {nullptr, nullptr};  // gate/up, down
     uint32_t* pos_of = nullptr;       // [max_tokens*(n_used+1)]
     uint32_t* group_hist = nullptr;   // scratch of the multi-block grouping
     void* argmax_scratch = nullptr; uint32_t argmax_rows = 0;
     // dense matrices for qkm_dense_gemm (tile-ordered copies) and its scratch, sized on demand
     static constexpr int kDenseSlots = 16;
     struct Dense { uint32_t type = 0, M = 0, K = 0; void* tiles = nullptr; } dense[kDenseSlots];
-    void* dense_xb = nullptr; uint32_t* dense_pairs = nullptr; qkm_sel* dense_sel = nullptr; MmaItem* dense_items = nullptr;
-    uint32_t* dense_n_items = nullptr;
-    size_t dense_cap_elems = 0, dense_cap_rows = 0, dense_cap_items = 0;
+    void* dense_xb = nullptr; float* dense_scale = nullptr;
+    size_t dense_cap_elems = 0, dense_cap_rows = 0;
     // expert-parallel exchange plan of the last qkm_ep_dispatch, allocated on first use
     uint32_t ep_ranks = 0;
     uint32_t* ep_counts = nullptr;       // [n_ranks + 1] rows per destination rank, then their sum
@@ -107,9 +101,6 @@ struct qkm_ctx {
     float* pm_xscale = nullptr;                       // [slot_cap] scales of the local rows sent as f16 (small batches)
     EpPeerTable pm_peers{};
     void* pm_opened[kMaxPeerRanks][3] = {};           // mappings this context opened from handles
-    // the shared expert's kernels run on a side stream, beside the routing/grouping kernels
-    cudaStream_t side = nullptr;
-    cudaEvent_t ev_fork = nullptr, ev_join = nullptr, ev_planes = nullptr;
     // the decode stack as CUDA graphs: captured on first use of an argument set, a few sets kept
     // (the host-buffer form runs the stack in chunks of layers, each its own graph)
     static constexpr int kStackGraphs = 8;
@@ -120,7 +111,6 @@ struct qkm_ctx {
         float* y = nullptr;
         cudaStream_t stream = nullptr;
         uint64_t launches = 0;       // kernels one replay launches
-        uint32_t plan_after = 0;     // shared_plan_n once the sequence has run
         uint64_t used = 0;           // for least-recently-used replacement
     } stack_graphs[kStackGraphs];
     uint64_t stack_clock = 0;
@@ -278,20 +268,15 @@ extern "C" QKM_API qkm_ctx* qkm_open(const qkm_config* cfg, char* err, size_t er
                           d.n_ff % gateup_stream_rows_per_item() == 0 &&
                           d.n_embd % down_stream_rows_per_item() == 0;
     if (c->shapes_stream_ok) {
-        const size_t max_groups = (T * d.n_used + 1) / 2 + d.n_expert;  // token pairs per expert, rounded up
         const size_t sh_groups = (T + 1) / 2;
         const size_t chunks_gu = d.n_ff / gateup_stream_rows_per_item(), chunks_dn = d.n_embd / down_stream_rows_per_item();
         struct { void** p; size_t bytes; } more[] = {
             {(void**)&c->xplanes, T * 4 * d.n_embd},
             {(void**)&c->xscale, T * sizeof(float)},
             {(void**)&c->hpieces, T * (d.n_used + 1) * 3 * d.n_ff * 2},
-            {(void**)&c->items_gu, max_groups * chunks_gu * sizeof(StreamItem)},
-            {(void**)&c->items_dn, max_groups * chunks_dn * sizeof(StreamItem)},
             {(void**)&c->items_sh_gu, sh_groups * chunks_gu * sizeof(StreamItem)},
             {(void**)&c->items_sh_dn, sh_groups * chunks_dn * sizeof(StreamItem)},
             {(void**)&c->n_items, 4 * sizeof(uint32_t)},
-            {(void**)&c->contrib_s, T * (d.n_used + 1) * d.n_embd * sizeof(float)},
-            {(void**)&c->arrivals, T * (d.n_embd / down_stream_unit_rows()) * sizeof(uint32_t)},
         };
         for (auto& a : more) {
             if ((e = cudaMalloc(a.p, a.bytes)) != cudaSuccess) {
@@ -300,7 +285,6 @@ extern "C" QKM_API qkm_ctx* qkm_open(const qkm_config* cfg, char* err, size_t er
                 return nullptr;
             }
         }
-        cudaMemset(c->arrivals, 0, T * (d.n_embd / down_stream_unit_rows()) * sizeof(uint32_t));
         c->dec_ok = decode_gateup_ok(d) && d.n_embd <= 4096;
         if (c->dec_ok) {
             struct { void** p; size_t bytes; } dec[] = {
@@ -337,22 +321,12 @@ extern "C" QKM_API qkm_ctx* qkm_open(const qkm_config* cfg, char* err, size_t er
     *c->status_host = 0;
     {
         const Launch L0{nullptr, nullptr};
-        if ((e = cudaMalloc((void**)&c->lut_pf, gateup_iq3_table_bytes())) != cudaSuccess ||
-            (e = launch_gateup_iq3_table(L0, c->lut_pf)) != cudaSuccess ||
-            (e = cudaMalloc((void**)&c->lut_dn, down_iq4_table_bytes())) != cudaSuccess ||
-            (e = launch_down_iq4_table(L0, c->lut_dn)) != cudaSuccess || (e = cudaDeviceSynchronize()) != cudaSuccess) {
+        if ((e = cudaMalloc((void**)&c->lut_pf, wgemm_table_bytes())) != cudaSuccess ||
+            (e = launch_wgemm_table(L0, c->lut_pf)) != cudaSuccess || (e = cudaDeviceSynchronize()) != cudaSuccess) {
             bail("qkm_open: prefill tables", cudaGetErrorString(e));
             qkm_close(c);
             return nullptr;
         }
-    }
-    if (cudaStreamCreateWithFlags(&c->side, cudaStreamNonBlocking) != cudaSuccess ||
-        cudaEventCreateWithFlags(&c->ev_fork, cudaEventDisableTiming) != cudaSuccess ||
-        cudaEventCreateWithFlags(&c->ev_join, cudaEventDisableTiming) != cudaSuccess ||
-        cudaEventCreateWithFlags(&c->ev_planes, cudaEventDisableTiming) != cudaSuccess) {
-        bail("qkm_open: side stream", nullptr);
-        qkm_close(c);
-        return nullptr;
     }
     if (err && err_len) err[0] = 0;
     return c;
@@ -365,13 +339,15 @@ extern "C" QKM_API void qkm_close(qkm_ctx* c) {
     for (auto& l : c->layers) {
         for (void* p : l.allocs) if (p) cudaFree(p);
         for (void* p : l.tiles) if (p) cudaFree(p);
+        if (l.router16) cudaFree(l.router16);
+        if (l.w_norm) cudaFree(l.w_norm);
     }
     for (auto& dm : c->dense) if (dm.tiles) cudaFree(dm.tiles);
-    void* scratch[] = {c->argmax_scratch, c->dense_xb, c->dense_pairs, c->dense_sel, c->dense_items, c->dense_n_items, c->sel, c->h, c->route_scratch, c->offsets, c->pairs, c->contrib, c->y2, c->x_stage, c->y_stage,
-                       c->stack_x, c->stack_y, c->xplanes, c->xscale, c->hpieces, c->items_gu, c->items_dn,
-                       c->items_sh_gu, c->items_sh_dn, c->n_items, c->contrib_s, c->arrivals, c->status, c->route_counter,
-                       c->planes8, c->lut_gu, c->lut_dd, c->lut_pf, c->lut_dn,
-                       c->xb, c->hb, c->hscale, c->contrib_p, c->mma_items[0], c->mma_items[1], c->mma_items[2], c->mma_items[3],
+    void* scratch[] = {c->argmax_scratch, c->dense_xb, c->dense_scale, c->sel, c->h, c->route_scratch, c->offsets, c->pairs, c->contrib, c->y2, c->x_stage, c->y_stage,
+                       c->stack_x, c->stack_y, c->xplanes, c->xscale, c->hpieces,
+                       c->items_sh_gu, c->items_sh_dn, c->n_items, c->status, c->route_counter,
+                       c->planes8, c->lut_gu, c->lut_dd, c->lut_pf,
+                       c->xb, c->xnorm, c->hb, c->hscale, c->contrib_p, c->mma_items[0], c->mma_items[1],
                        c->pos_of, c->group_hist, c->ep_counts, c->ep_send_tok, c->ep_send_pos};
     for (void* p : scratch) if (p) cudaFree(p);
     for (auto& o : c->pm_opened) for (void* p : o) if (p) cudaIpcCloseMemHandle(p);
@@ -384,10 +360,6 @@ extern "C" QKM_API void qkm_close(qkm_ctx* c) {
     if (c->ev_copies) cudaEventDestroy(c->ev_copies);
     if (c->copy_in) cudaStreamDestroy(c->copy_in);
     if (c->copy_out) cudaStreamDestroy(c->copy_out);
-    if (c->ev_fork) cudaEventDestroy(c->ev_fork);
-    if (c->ev_join) cudaEventDestroy(c->ev_join);
-    if (c->ev_planes) cudaEventDestroy(c->ev_planes);
-    if (c->side) cudaStreamDestroy(c->side);
     for (cudaEvent_t ev : c->prof_ev) if (ev) cudaEventDestroy(ev);
     delete c;
 }
@@ -487,7 +459,8 @@ extern "C" QKM_API int qkm_upload_layer(qkm_ctx* c, uint32_t layer, const qkm_la
     }
     // tile-ordered copies for the streaming kernels (same bytes, re-ordered on the device)
     for (void*& p : l.tiles) { if (p) { QKM_CUDA(c, cudaFree(p)); p = nullptr; } }
-    l.stream_ok = l.tiles_ok = l.gu_only = l.fused_ok = false;
+    for (void** p : {&l.router16, (void**)&l.w_norm}) { if (*p) { QKM_CUDA(c, cudaFree(*p)); *p = nullptr; } }
+    l.tiles_ok = l.fused_ok = false;
     if (c->shapes_stream_ok) {
         const qkm_dims& d = c->cfg.dims;
         struct { int idx; uint32_t type, mats, rows, K; } plan[] = {
@@ -496,18 +469,25 @@ extern "C" QKM_API int qkm_upload_layer(qkm_ctx* c, uint32_t layer, const qkm_la
             {5, QKM_TYPE_Q8_0, 1, d.n_ff, d.n_embd}, {6, QKM_TYPE_Q8_0, 1, d.n_ff, d.n_embd},
             {7, QKM_TYPE_Q8_0, 1, d.n_embd, d.n_ff},
         };
-        const bool gu = w->gateup_type == QKM_TYPE_IQ3_XXS, dn = w->down_type == QKM_TYPE_IQ4_XS;
         for (auto& t : plan) {
-            const size_t bytes = tensor_bytes(c, t.idx, *w);
+            const size_t bytes = tiled_bytes(t.type, t.mats, t.rows, t.K);
             QKM_CUDA(c, cudaMalloc(&l.tiles[t.idx], bytes + 256));
             cudaError_t e = launch_repack(c->L(), t.type, l.allocs[t.idx], l.tiles[t.idx], t.mats, t.rows, t.K);
             if (e != cudaSuccess) return fail(c, QKM_ERR_CUDA, "repack: %s", cudaGetErrorString(e));
         }
-        const bool all_resident = c->ecount == c->cfg.dims.n_expert;
-        l.tiles_ok = gu && dn;
-        l.stream_ok = gu && dn && all_resident;
-        l.gu_only = gu && !dn && all_resident;
-        l.fused_ok = all_resident;
+        // what the prefill sequence wants beside the tiles: the router in its rows' order, bounds on the hidden values
+        const size_t n_norm = 2 * ((size_t)c->ecount + 1);
+        QKM_CUDA(c, cudaMalloc(&l.router16, (size_t)d.n_expert * d.n_embd * 2));
+        QKM_CUDA(c, cudaMalloc((void**)&l.w_norm, n_norm * sizeof(float)));
+        QKM_CUDA(c, cudaMemsetAsync(l.w_norm, 0, n_norm * sizeof(float), c->stream));
+        cudaError_t e = launch_router_f16(c->L(), w->router_type, l.allocs[0], l.router16, (uint64_t)d.n_expert * d.n_embd);
+        for (int m = 0; m < 2 && e == cudaSuccess; ++m) {
+            e = launch_row_norm_max(c->L(), w->gateup_type, l.allocs[2 + m], l.w_norm + m * (c->ecount + 1), c->ecount, d.n_ff, d.n_embd);
+            if (e == cudaSuccess) e = launch_row_norm_max(c->L(), QKM_TYPE_Q8_0, l.allocs[5 + m], l.w_norm + m * (c->ecount + 1) + c->ecount, 1, d.n_ff, d.n_embd);
+        }
+        if (e != cudaSuccess) return fail(c, QKM_ERR_CUDA, "upload: %s", cudaGetErrorString(e));
+        l.tiles_ok = true;
+        l.fused_ok = c->ecount == c->cfg.dims.n_expert;
     }
     QKM_CUDA(c, cudaStreamSynchronize(c->stream));
     l.w = *w;
@@ -636,6 +616,38 @@ extern "C" QKM_API int qkm_dequant(qkm_ctx* c, uint32_t type, const void* blocks
 
 // ---------------------------------------------------------------- fused layer calls
 
+// Three launches for the whole layer: (1) router logits, selection and digit planes; (2) pair
+// grouping (in every block's shared memory), then gate/up + SwiGLU of the routed experts and of
+// the shared expert; (3) down projections of both and the weighted sum.  The shared expert rides inside (2)
+// and (3): no side stream, and nothing runs beside the two persistent kernels that they would have to share
+// the SMs with.  At most 64 tokens (the pair grouping's limit).
+static int decode_fused(qkm_ctx* c, const qkm_layer_dev& ld, const float* x, uint32_t n, float* y, qkm_sel* sel, float* h) {
+    const qkm_layer_weights& w = ld.w;
+    const qkm_dims& d = c->cfg.dims;
+    const uint32_t nb = (uint32_t)c->n_sms;
+    RouteDecodeArgs ra{};
+    ra.router = (const uint8_t*)w.router; ra.gis = w.gate_inp_shexp; ra.x = x; ra.sel = sel;
+    ra.logits = (double*)c->route_scratch; ra.counter = c->route_counter; ra.planes = c->planes8; ra.xscale = c->xscale; ra.n_tokens = n; ra.d = d;
+    QKM_LAUNCH(c, launch_route_decode(c->Lchain(), w.router_type, ra));
+    c->prof_mark("moe.route");
+    GateupDecodeArgs ga{};
+    ga.gate_tiles = (const uint8_t*)ld.tiles[2]; ga.up_tiles = (const uint8_t*)ld.tiles[3];
+    ga.sh_gate_tiles = (const uint8_t*)ld.tiles[5]; ga.sh_up_tiles = (const uint8_t*)ld.tiles[6];
+    ga.luts = c->lut_gu; ga.planes = c->planes8; ga.xscale = c->xscale; ga.sel = sel;
+    ga.n_tokens = n; ga.expert_first = c->efirst; ga.expert_count = c->ecount; ga.with_shared = 1;
+    ga.gateup_type = w.gateup_type;
+    ga.h = h; ga.status = c->status; ga.d = d;
+    QKM_LAUNCH(c, launch_decode_gateup(c->Lchain(), ga, nb));
+    c->prof_mark("moe.gu");
+    DownDecodeArgs da{};
+    da.tiles = (const uint8_t*)ld.tiles[4]; da.sh_tiles = (const uint8_t*)ld.tiles[7]; da.lut = c->lut_dd;
+    da.h = h; da.sel = sel; da.y = y; da.n_tokens = n; da.status = c->status; da.d = d;
+    if (w.down_type == QKM_TYPE_IQ4_XS) QKM_LAUNCH(c, launch_decode_down(c->Lchain(), da, nb));
+    else QKM_LAUNCH(c, launch_decode_down_q6k(c->Lchain(), da, nb));
+    c->prof_mark("moe.dn");
+    return QKM_OK;
+}
+
 extern "C" QKM_API int qkm_moe_decode(qkm_ctx* c, uint32_t layer, const float* x, uint32_t n, float* y) {
     if (int rc = layer_ready(c, layer)) return rc;
     if (!x || !y) return QKM_ERR_ARG;
@@ -644,108 +656,21 @@ extern "C" QKM_API int qkm_moe_decode(qkm_ctx* c, uint32_t layer, const float* x
     const qkm_layer_weights& w = ld.w;
     const qkm_dims& d = c->cfg.dims;
     c->prof_begin();
-    const bool fused = ld.fused_ok && c->dec_ok && route_decode_ok(d, n, c->route_scratch_bytes) && decode_down_ok(d);
-    if (!fused && !ld.stream_ok && !ld.gu_only) {  // generic kernels on the raw layout
-        QKM_LAUNCH(c, launch_route_select(c->L(), d, w.router_type, w.router, w.gate_inp_shexp, x, c->sel, n, c->route_scratch, c->route_scratch_bytes));
-        c->prof_mark("moe.route");
-        QKM_LAUNCH(c, launch_shared_gateup(c->L(), d, w.gate_shexp, w.up_shexp, x, c->h, n));
-        c->prof_mark("moe.shared_gu");
-        QKM_LAUNCH(c, launch_gateup_tokens(c->L(), d, w.gateup_type, w.gate_exps, w.up_exps, x, c->sel, c->h, n, c->efirst, c->ecount));
-        c->prof_mark("moe.gu");
-        QKM_LAUNCH(c, launch_down_tokens(c->L(), d, w.down_type, w.down_exps, c->h, c->sel, y, n, c->efirst, c->ecount, w.down_shexp));
-        c->prof_mark("moe.dn");
+    constexpr uint32_t kMost = 64;
+    if (n && ld.fused_ok && c->dec_ok && route_decode_ok(d, n < kMost ? n : kMost, c->route_scratch_bytes) && decode_down_ok(d)) {
+        for (uint32_t t = 0; t < n; t += kMost)
+            if (int rc = decode_fused(c, ld, x + (size_t)t * d.n_embd, n - t < kMost ? n - t : kMost, y + (size_t)t * d.n_embd, c->sel + t,
+                                      c->h + (size_t)t * (d.n_used + 1) * d.n_ff)) return rc;
         return QKM_OK;
     }
-    const uint32_t nb = (uint32_t)c->n_sms;
-    // Three launches for the whole layer: (1) router logits, selection and digit planes; (2) pair
-    // grouping (in every block's shared memory), then gate/up + SwiGLU of the routed experts and of
-    // the shared expert; (3) down
-    // projections of both and the weighted sum.  The shared expert rides inside (2) and (3): no
-    // side stream, and nothing runs beside the two persistent kernels that they would have to
-    // share the SMs with.
-    if (fused) {
-        RouteDecodeArgs ra{};
-        ra.router = (const uint8_t*)w.router; ra.gis = w.gate_inp_shexp; ra.x = x; ra.sel = c->sel;
-        ra.logits = (double*)c->route_scratch; ra.counter = c->route_counter; ra.planes = c->planes8; ra.xscale = c->xscale; ra.n_tokens = n; ra.d = d;
-        QKM_LAUNCH(c, launch_route_decode(c->Lchain(), w.router_type, ra));
-        c->prof_mark("moe.route");
-        GateupDecodeArgs ga{};
-        ga.gate_tiles = (const uint8_t*)ld.tiles[2]; ga.up_tiles = (const uint8_t*)ld.tiles[3];
-        ga.sh_gate_tiles = (const uint8_t*)ld.tiles[5]; ga.sh_up_tiles = (const uint8_t*)ld.tiles[6];
-        ga.luts = c->lut_gu; ga.planes = c->planes8; ga.xscale = c->xscale; ga.sel = c->sel;
-        ga.n_tokens = n; ga.expert_first = c->efirst; ga.expert_count = c->ecount; ga.with_shared = 1;
-        ga.gateup_type = w.gateup_type;
-        ga.h = c->h; ga.status = c->status; ga.d = d;
-        QKM_LAUNCH(c, launch_decode_gateup(c->Lchain(), ga, nb));
-        c->prof_mark("moe.gu");
-        if (w.down_type == QKM_TYPE_IQ4_XS) {
-            DownDecodeArgs da{};
-            da.tiles = (const uint8_t*)ld.tiles[4]; da.sh_tiles = (const uint8_t*)ld.tiles[7]; da.lut = c->lut_dd;
-            da.h = c->h; da.sel = c->sel; da.y = y; da.n_tokens = n; da.status = c->status; da.d = d;
-            QKM_LAUNCH(c, launch_decode_down(c->Lchain(), da, nb));
-        } else {   // Q6_K down
-            DownDecodeArgs da{};
-            da.tiles = (const uint8_t*)ld.tiles[4]; da.sh_tiles = (const uint8_t*)ld.tiles[7];
-            da.h = c->h; da.sel = c->sel; da.y = y; da.n_tokens = n; da.status = c->status; da.d = d;
-            QKM_LAUNCH(c, launch_decode_down_q6k(c->Lchain(), da, nb));
-        }
-        c->prof_mark("moe.dn");
-        c->shared_plan_n = 0;   // pairs / work lists of the older sequence are overwritten
-        return QKM_OK;
-    }
-    // Shared expert: depends on x only (as digit planes), so the whole of it - planes, gate/up,
-    // down - runs on the side stream from the start of the layer, beside the router.  The main
-    // stream needs the planes before the routed gate/up (ev_planes) and y2 before the routed
-    // down kernel (ev_join).  (Sequential while profiling.)
-    const bool fork = !c->profiling;
-    Launch S{fork ? c->side : c->stream, &c->launches};
-    if (fork) {
-        QKM_CUDA(c, cudaEventRecord(c->ev_fork, c->stream));
-        QKM_CUDA(c, cudaStreamWaitEvent(c->side, c->ev_fork, 0));
-    }
-    // the shared gate too, when the selection kernel will not touch it (same condition as below)
-    const bool fused_plan = route_select_plans(d, n, c->route_scratch_bytes);
-    QKM_LAUNCH(c, launch_xplanes(S, x, n, d.n_embd, c->xplanes, c->xscale, fused_plan ? w.gate_inp_shexp : nullptr, c->sel));
-    if (fork) QKM_CUDA(c, cudaEventRecord(c->ev_planes, c->side));
-    // the shared expert's work lists depend on the token count only and live in parts of the
-    // scratch the decode kernels never write: cut once, reused until another kind of call intervenes
-    if (c->shared_plan_n != n) {
-        QKM_LAUNCH(c, launch_shared_plan(S, d, n, c->pairs, c->items_sh_gu, d.n_ff / gateup_stream_rows_per_item(),
-                                         c->items_sh_dn, d.n_embd / down_stream_rows_per_item(), 2, c->n_items + 2));
-        c->shared_plan_n = n;
-    }
-    QKM_LAUNCH(c, launch_gateup_stream(S, d, QKM_TYPE_Q8_0, ld.tiles[5], ld.tiles[6], c->xplanes, c->xscale, c->pairs,
-                                       c->items_sh_gu, c->n_items + 2, c->h, c->hpieces, nb, c->status));
-    if (!fork) c->prof_mark("moe.shared_gu");
-    if (ld.stream_ok) {
-        QKM_LAUNCH(c, launch_down_stream(S, d, QKM_TYPE_Q8_0, ld.tiles[7], c->hpieces, nullptr, c->pairs, c->items_sh_dn,
-                                         c->n_items + 3, nullptr, c->y2, nullptr, nb, c->status));   // unweighted: w_shared is applied by the routed down kernel
-        if (!fork) c->prof_mark("moe.shared_dn");
-    }
-    if (fork) QKM_CUDA(c, cudaEventRecord(c->ev_join, c->side));
-    // Router.  Decode-sized batches: the selection kernel's last block also groups the pairs and
-    // cuts the work lists; otherwise a grouping launch follows.
-    const RoutePlan rplan{c->route_counter, c->offsets, c->pairs, c->items_gu, c->items_dn, c->n_items,
-                          d.n_ff / gateup_stream_rows_per_item(), d.n_embd / down_stream_rows_per_item(), 2, c->efirst, c->ecount, 1};
-    QKM_LAUNCH(c, launch_route_select(c->Lchain(), d, w.router_type, w.router, w.gate_inp_shexp, x, c->sel, n, c->route_scratch, c->route_scratch_bytes,
-                                      nullptr, nullptr, nullptr, nullptr, nullptr, fused_plan ? &rplan : nullptr));
+    // generic kernels on the raw layout
+    QKM_LAUNCH(c, launch_route_select(c->L(), d, w.router_type, w.router, w.gate_inp_shexp, x, c->sel, n, c->route_scratch, c->route_scratch_bytes));
     c->prof_mark("moe.route");
-    if (!fused_plan) {
-        QKM_LAUNCH(c, launch_group_plan(c->L(), d, c->sel, n, c->offsets, c->pairs, c->efirst, c->ecount, c->items_gu,
-                                        d.n_ff / gateup_stream_rows_per_item(), c->items_dn,
-                                        d.n_embd / down_stream_rows_per_item(), nullptr, nullptr, 2, c->n_items));
-        c->prof_mark("moe.pairs");
-    }
-    if (fork) QKM_CUDA(c, cudaStreamWaitEvent(c->stream, c->ev_planes, 0));
-    QKM_LAUNCH(c, launch_gateup_stream(fused_plan ? c->Lchain() : c->L(), d, w.gateup_type, ld.tiles[2], ld.tiles[3], c->xplanes, c->xscale, c->pairs,
-                                       c->items_gu, c->n_items, c->h, c->hpieces, nb, c->status));
+    QKM_LAUNCH(c, launch_shared_gateup(c->L(), d, w.gate_shexp, w.up_shexp, x, c->h, n));
+    c->prof_mark("moe.shared_gu");
+    QKM_LAUNCH(c, launch_gateup_tokens(c->L(), d, w.gateup_type, w.gate_exps, w.up_exps, x, c->sel, c->h, n, c->efirst, c->ecount));
     c->prof_mark("moe.gu");
-    if (fork) QKM_CUDA(c, cudaStreamWaitEvent(c->stream, c->ev_join, 0));
-    if (ld.stream_ok) {
-        QKM_LAUNCH(c, launch_down_tok(c->Lchain(), d, w.down_type, ld.tiles[4], c->hpieces, c->sel, c->y2, y, n, nb, c->status));
-    } else {   // Q6_K down: f32 kernel over h, routed slots and the shared expert in one pass
-        QKM_LAUNCH(c, launch_down_tokens(c->L(), d, w.down_type, w.down_exps, c->h, c->sel, y, n, c->efirst, c->ecount, w.down_shexp));
-    }
+    QKM_LAUNCH(c, launch_down_tokens(c->L(), d, w.down_type, w.down_exps, c->h, c->sel, y, n, c->efirst, c->ecount, w.down_shexp));
     c->prof_mark("moe.dn");
     return QKM_OK;
 }
@@ -773,19 +698,33 @@ static int ensure_prefill_scratch(qkm_ctx* c) {
     if (c->xb) return QKM_OK;
     const qkm_dims& d = c->cfg.dims;
     const size_t T = c->cfg.max_tokens, rows = T * (d.n_used + 1);
-    const uint32_t NT = prefill_pairs_per_block();
-    const uint32_t rt_gu = d.n_ff / 128, rt_dn = d.n_embd / 128;
-    const size_t max_tiles = d.n_expert + (T * d.n_used + NT - 1) / NT, max_sh = (T + NT - 1) / NT;
+    const uint32_t NT = wgemm_rows_per_unit();
+    const size_t max_tiles = d.n_expert + (T * d.n_used + NT - 1) / NT + (T + NT - 1) / NT;   // the shared expert's last
     QKM_CUDA(c, cudaMalloc(&c->xb, T * d.n_embd * 2));
+    QKM_CUDA(c, cudaMalloc((void**)&c->xnorm, T * sizeof(float)));
     QKM_CUDA(c, cudaMalloc(&c->hb, rows * d.n_ff * 2));
     QKM_CUDA(c, cudaMalloc((void**)&c->hscale, rows * sizeof(float)));
     QKM_CUDA(c, cudaMalloc((void**)&c->contrib_p, rows * d.n_embd * sizeof(float)));
-    QKM_CUDA(c, cudaMalloc((void**)&c->mma_items[0], max_tiles * rt_gu * sizeof(MmaItem)));
-    QKM_CUDA(c, cudaMalloc((void**)&c->mma_items[1], max_tiles * rt_dn * sizeof(MmaItem)));
-    QKM_CUDA(c, cudaMalloc((void**)&c->mma_items[2], max_sh * rt_gu * sizeof(MmaItem)));
-    QKM_CUDA(c, cudaMalloc((void**)&c->mma_items[3], max_sh * rt_dn * sizeof(MmaItem)));
+    QKM_CUDA(c, cudaMalloc((void**)&c->mma_items[0], max_tiles * (d.n_ff / 128) * sizeof(MmaItem)));
+    QKM_CUDA(c, cudaMalloc((void**)&c->mma_items[1], max_tiles * (d.n_embd / 256) * sizeof(MmaItem)));
     QKM_CUDA(c, cudaMalloc((void**)&c->pos_of, rows * sizeof(uint32_t)));
     QKM_CUDA(c, cudaMalloc((void**)&c->group_hist, group_wide_scratch_bytes((uint32_t)T, d.n_used, c->ecount)));
+    return QKM_OK;
+}
+
+// The two expert GEMMs over the work lists of launch_mma_plan: c->xb (f16 rows; c->xscale, c->xnorm) -> c->hb -> c->contrib_p.
+// At most np_max routed pairs and sh_max rows of the shared expert.
+static int expert_gemms(qkm_ctx* c, const qkm_layer_dev& ld, const qkm_sel* sel, uint32_t np_max, uint32_t sh_max) {
+    const qkm_dims& d = c->cfg.dims;
+    const uint32_t NT = wgemm_rows_per_unit();
+    const uint32_t tiles = (c->ecount < np_max ? c->ecount + (np_max + NT - 1) / NT : np_max) + (sh_max + NT - 1) / NT;
+    WgemmExperts g{{ld.tiles[2], ld.tiles[3]}, {ld.tiles[5], ld.tiles[6]}, c->mma_items[0], c->n_items, c->n_items + 2, c->pairs, c->lut_pf, c->status, c->ecount, (uint32_t)c->n_sms};
+    QKM_LAUNCH(c, launch_wgemm_gateup(c->L(), d, ld.w.gateup_type, g, c->xb, c->xscale, c->xnorm, ld.w_norm, c->hb, c->hscale, tiles * (d.n_ff / 128)));
+    c->prof_mark("moe.gu");
+    WgemmExperts m{{ld.tiles[4], nullptr}, {ld.tiles[7], nullptr}, c->mma_items[1], c->n_items + 1, c->n_items + 3, c->pairs, c->lut_pf, c->status, c->ecount, (uint32_t)c->n_sms};
+    QKM_LAUNCH(c, launch_wgemm_down(c->L(), d, ld.w.down_type, m, c->hb, (uint64_t)c->cfg.max_tokens * (d.n_used + 1), c->hscale, sel, c->contrib_p,
+                                    tiles * (d.n_embd / 256)));
+    c->prof_mark("moe.dn");
     return QKM_OK;
 }
 
@@ -796,49 +735,19 @@ extern "C" QKM_API int qkm_moe_prefill(qkm_ctx* c, uint32_t layer, const float* 
     const qkm_layer_dev& ld = c->layers[layer];
     const qkm_layer_weights& w = ld.w;
     const qkm_dims& d = c->cfg.dims;
-    c->shared_plan_n = 0;   // this call rewrites the scratch the decode work lists live in
     if (!ld.fused_ok || n == 0) return prefill_generic(c, ld, x, n, y);
-    // tensor-core path: tokens grouped by expert, expert GEMMs on tcgen05 with bf16 operands
-    const uint32_t NT = prefill_pairs_per_block();
-    const uint32_t rt_gu = d.n_ff / 128, rt_dn = d.n_embd / 128;
+    // tensor-core path: tokens grouped by expert, expert GEMMs on tcgen05 with f16 operands; the shared expert's units
+    // ride in the same two launches
     if (int rc = ensure_prefill_scratch(c)) return rc;
-    const uint32_t tiles_now = d.n_expert < n * d.n_used ? d.n_expert + (n * d.n_used + NT - 1) / NT : n * d.n_used;
-    const uint32_t sh_now = (n + NT - 1) / NT;
     c->prof_begin();
-    QKM_LAUNCH(c, launch_to_f16_rows(c->L(), x, c->xb, c->xscale, n, d.n_embd));
+    QKM_LAUNCH(c, launch_f16_rows(c->L(), x, c->xb, c->xscale, c->xnorm, n, d.n_embd));
     QKM_LAUNCH(c, launch_route_select(c->L(), d, w.router_type, w.router, w.gate_inp_shexp, x, c->sel, n, c->route_scratch, c->route_scratch_bytes,
-                                      nullptr, nullptr, c->xb, c->xscale, c->status));
+                                      nullptr, nullptr, c->xb, c->xscale, c->status, nullptr, ld.router16));
     c->prof_mark("moe.route");
     QKM_LAUNCH(c, launch_group_pairs_wide(c->L(), d, c->sel, n, c->offsets, c->pairs, c->efirst, c->ecount, c->group_hist, c->pos_of));
-    QKM_LAUNCH(c, launch_mma_plan(c->L(), d, c->offsets, c->pairs, c->ecount, n, c->mma_items[0], c->mma_items[1],
-                                  c->mma_items[2], c->mma_items[3], c->n_items, c->pos_of, true, true));
+    QKM_LAUNCH(c, launch_mma_plan(c->L(), d, c->offsets, c->pairs, c->ecount, n, c->mma_items[0], c->mma_items[1], c->n_items, c->pos_of, true, true));
     c->prof_mark("moe.pairs");
-    // the shared expert's two GEMMs (few, long blocks) run beside the routed ones
-    const bool fork = !c->profiling;
-    Launch S{fork ? c->side : c->stream, &c->launches};
-    if (fork) {
-        QKM_CUDA(c, cudaEventRecord(c->ev_fork, c->stream));
-        QKM_CUDA(c, cudaStreamWaitEvent(c->side, c->ev_fork, 0));
-    }
-    // Tensor-core down GEMMs take the hidden rows as f16 scaled per row by a power of two: the gate/up kernels
-    // store them in f32 by pair position (in c->h), a conversion pass finds each row's scale.
-    QKM_LAUNCH(c, launch_gateup_mma(S, d, QKM_TYPE_Q8_0, ld.tiles[5], ld.tiles[6], c->xb, c->xscale, c->pairs, c->mma_items[2],
-                                    c->n_items + 2, sh_now * rt_gu, nullptr, c->hb, c->status, sh_now * rt_gu <= 2u * (uint32_t)c->n_sms, nullptr, c->h));
-    if (!fork) c->prof_mark("moe.shared_gu");
-    // the shared expert's rows follow the routed pairs (their number is offsets[ecount], known on the device)
-    QKM_LAUNCH(c, launch_h_rows_to_f16(S, c->h, c->hb, c->hscale, d.n_ff, c->offsets + c->ecount, 0, nullptr, n));
-    QKM_LAUNCH(c, launch_down_mma(S, d, QKM_TYPE_Q8_0, ld.tiles[7], c->hb, c->sel, c->pairs, c->mma_items[3],
-                                  c->n_items + 3, sh_now * rt_dn, c->contrib_p, c->status, false, nullptr, c->hscale));
-    if (!fork) c->prof_mark("moe.shared_dn");
-    if (fork) QKM_CUDA(c, cudaEventRecord(c->ev_join, c->side));
-    QKM_LAUNCH(c, launch_gateup_mma(c->L(), d, w.gateup_type, ld.tiles[2], ld.tiles[3], c->xb, c->xscale, c->pairs, c->mma_items[0],
-                                    c->n_items, tiles_now * rt_gu, nullptr, c->hb, c->status, false, c->lut_pf, c->h));
-    c->prof_mark("moe.gu");
-    QKM_LAUNCH(c, launch_h_rows_to_f16(c->L(), c->h, c->hb, c->hscale, d.n_ff, nullptr, 0, c->offsets + c->ecount, n * d.n_used));
-    QKM_LAUNCH(c, launch_down_mma(c->L(), d, w.down_type, ld.tiles[4], c->hb, c->sel, c->pairs, c->mma_items[1],
-                                  c->n_items + 1, tiles_now * rt_dn, c->contrib_p, c->status, false, c->lut_dn, c->hscale));
-    c->prof_mark("moe.dn");
-    if (fork) QKM_CUDA(c, cudaStreamWaitEvent(c->stream, c->ev_join, 0));
+    if (int rc = expert_gemms(c, ld, c->sel, n * d.n_used, n)) return rc;
     QKM_LAUNCH(c, launch_fold_pairs(c->L(), d, c->contrib_p, c->pos_of, y, n));
     c->prof_mark("moe.fold");
     return QKM_OK;
@@ -876,8 +785,6 @@ extern "C" QKM_API int qkm_moe_decode_stack(qkm_ctx* c, uint32_t first, uint32_t
     for (uint32_t l = 0; l < count; ++l)
         if (int rc = layer_ready(c, first + l)) return rc;
     if (c->stream == nullptr || c->profiling || count < 2) return decode_stack_eager(c, first, count, x, n, y);
-    // A captured sequence always cuts the shared expert's work lists itself (shared_plan_n is cleared
-    // before the capture), so a replay never depends on what ran in between.
     qkm_ctx::StackGraph* g = nullptr;
     for (auto& e : c->stack_graphs)
         if (e.exec && e.first == first && e.count == count && e.n == n && e.x == x && e.y == y && e.stream == c->stream) g = &e;
@@ -888,7 +795,6 @@ extern "C" QKM_API int qkm_moe_decode_stack(qkm_ctx* c, uint32_t first, uint32_t
             if (e.used < slot->used) slot = &e;
         }
         if (slot->exec) { cudaGraphExecDestroy(slot->exec); slot->exec = nullptr; }
-        c->shared_plan_n = 0;   // the captured sequence must cut the list itself
         const uint64_t before = c->launches;
         if (cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal) != cudaSuccess) {
             cudaGetLastError();
@@ -898,9 +804,7 @@ extern "C" QKM_API int qkm_moe_decode_stack(qkm_ctx* c, uint32_t first, uint32_t
         cudaGraph_t graph = nullptr;
         const cudaError_t e = cudaStreamEndCapture(c->stream, &graph);
         slot->launches = c->launches - before;
-        slot->plan_after = c->shared_plan_n;
         c->launches = before;
-        c->shared_plan_n = 0;   // nothing captured has run
         if (rc != QKM_OK || e != cudaSuccess || !graph) {
             if (graph) cudaGraphDestroy(graph);
             cudaGetLastError();
@@ -919,7 +823,6 @@ extern "C" QKM_API int qkm_moe_decode_stack(qkm_ctx* c, uint32_t first, uint32_t
     g->used = ++c->stack_clock;
     QKM_CUDA(c, cudaGraphLaunch(g->exec, c->stream));
     c->launches += g->launches;
-    c->shared_plan_n = g->plan_after;
     return QKM_OK;
 }
 
@@ -1018,12 +921,12 @@ extern "C" QKM_API int qkm_dense_upload(qkm_ctx* c, uint32_t slot, uint32_t type
     if (M == 0 || M % 128 || K == 0 || K % 256) return fail(c, QKM_ERR_ARG, "qkm_dense_upload: M %% 128 and K %% 256 must be 0 (M=%u K=%u)", M, K);
     auto& dm = c->dense[slot];
     if (dm.tiles) { QKM_CUDA(c, cudaFree(dm.tiles)); dm = qkm_ctx::Dense{}; }
-    const size_t bytes = (size_t)M * row_bytes(type, K);
+    const size_t bytes = (size_t)M * row_bytes(type, K), tbytes = tiled_bytes(type, 1, M, K);
     void* raw = nullptr;
     QKM_CUDA(c, cudaMalloc(&raw, bytes + 256));
-    cudaError_t e = cudaMalloc(&dm.tiles, bytes + 256);
+    cudaError_t e = cudaMalloc(&dm.tiles, tbytes + 256);
     if (e == cudaSuccess) e = cudaMemcpyAsync(raw, w_host, bytes, cudaMemcpyHostToDevice, c->stream);
-    if (e == cudaSuccess) e = cudaMemsetAsync((uint8_t*)dm.tiles + bytes, 0, 256, c->stream);
+    if (e == cudaSuccess) e = cudaMemsetAsync((uint8_t*)dm.tiles + tbytes, 0, 256, c->stream);
     if (e == cudaSuccess) e = launch_repack(c->L(), type, raw, dm.tiles, 1, M, K);
     if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
     cudaFree(raw);
@@ -1041,8 +944,7 @@ extern "C" QKM_API int qkm_dense_gemm(qkm_ctx* c, uint32_t slot, const float* x,
     if (slot >= qkm_ctx::kDenseSlots || !c->dense[slot].tiles) return fail(c, QKM_ERR_BUSY, "dense slot %u holds no matrix", slot);
     if (n == 0) return QKM_OK;
     const auto& dm = c->dense[slot];
-    const uint32_t NT = prefill_pairs_per_block();
-    const size_t elems = (size_t)n * dm.K, items = (size_t)((n + NT - 1) / NT) * (dm.M / 128);
+    const size_t elems = (size_t)n * dm.K;
     if (elems > c->dense_cap_elems) {
         if (c->dense_xb) QKM_CUDA(c, cudaFree(c->dense_xb));
         c->dense_xb = nullptr; c->dense_cap_elems = 0;
@@ -1050,21 +952,12 @@ extern "C" QKM_API int qkm_dense_gemm(qkm_ctx* c, uint32_t slot, const float* x,
         c->dense_cap_elems = elems;
     }
     if (n > c->dense_cap_rows) {
-        if (c->dense_pairs) { cudaFree(c->dense_pairs); cudaFree(c->dense_sel); }
-        c->dense_pairs = nullptr; c->dense_sel = nullptr; c->dense_cap_rows = 0;
-        QKM_CUDA(c, cudaMalloc((void**)&c->dense_pairs, (size_t)n * sizeof(uint32_t)));
-        QKM_CUDA(c, cudaMalloc((void**)&c->dense_sel, (size_t)n * sizeof(qkm_sel)));
+        if (c->dense_scale) QKM_CUDA(c, cudaFree(c->dense_scale));
+        c->dense_scale = nullptr; c->dense_cap_rows = 0;
+        QKM_CUDA(c, cudaMalloc((void**)&c->dense_scale, (size_t)n * sizeof(float)));
         c->dense_cap_rows = n;
     }
-    if (items > c->dense_cap_items) {
-        if (c->dense_items) cudaFree(c->dense_items);
-        c->dense_items = nullptr; c->dense_cap_items = 0;
-        QKM_CUDA(c, cudaMalloc((void**)&c->dense_items, items * sizeof(MmaItem)));
-        c->dense_cap_items = items;
-    }
-    if (!c->dense_n_items) QKM_CUDA(c, cudaMalloc((void**)&c->dense_n_items, sizeof(uint32_t)));
-    QKM_LAUNCH(c, launch_dense_gemm(c->L(), dm.type, dm.tiles, dm.M, dm.K, x, n, y, c->dense_xb, c->dense_pairs, c->dense_sel,
-                                    c->dense_items, c->dense_n_items, c->status));
+    QKM_LAUNCH(c, launch_dense_gemm(c->L(), dm.type, dm.tiles, dm.M, dm.K, x, n, y, c->dense_xb, c->dense_scale, c->lut_pf, (uint32_t)c->n_sms, c->status));
     return QKM_OK;
 }
 
@@ -1137,7 +1030,6 @@ extern "C" QKM_API int qkm_moe_layer_step(qkm_ctx* c, uint32_t layer, const floa
 
 static int ep_check(qkm_ctx* c, uint32_t n_ranks) {
     const qkm_dims& d = c->cfg.dims;
-    c->shared_plan_n = 0;
     if (n_ranks == 0 || n_ranks > 64 || d.n_expert % n_ranks) return fail(c, QKM_ERR_ARG, "n_ranks %u does not divide n_expert %u", n_ranks, d.n_expert);
     if (c->ecount != d.n_expert / n_ranks || c->efirst % c->ecount)
         return fail(c, QKM_ERR_MODE, "context holds experts [%u,%u): not one of %u equal shards", c->efirst, c->efirst + c->ecount, n_ranks);
@@ -1165,11 +1057,11 @@ static int ep_route_local(qkm_ctx* c, uint32_t layer, const float* x, uint32_t n
     const bool tc = ld.tiles_ok && n >= 128;      // tensor-core logits from f16 rows
     if (tc) {
         if (int rc = ensure_prefill_scratch(c)) return rc;
-        QKM_LAUNCH(c, launch_to_f16_rows(c->L(), x, c->xb, c->xscale, n, d.n_embd));
+        QKM_LAUNCH(c, launch_f16_rows(c->L(), x, c->xb, c->xscale, c->xnorm, n, d.n_embd));
     }
     QKM_LAUNCH(c, launch_route_select(c->L(), d, w.router_type, w.router, w.gate_inp_shexp, x, c->sel, n, c->route_scratch, c->route_scratch_bytes,
                                       planes ? c->xplanes : nullptr, planes ? c->xscale : nullptr, tc ? c->xb : nullptr,
-                                      tc ? c->xscale : nullptr, c->status));
+                                      tc ? c->xscale : nullptr, c->status, nullptr, ld.router16));
     return QKM_OK;
 }
 
@@ -1209,7 +1101,6 @@ extern "C" QKM_API int qkm_ep_dispatch_dev(qkm_ctx* c, uint32_t layer, const flo
 
 extern "C" QKM_API int qkm_ep_shared(qkm_ctx* c, uint32_t layer, const float* x, uint32_t n) {
     if (int rc = layer_ready(c, layer)) return rc;
-    c->shared_plan_n = 0;
     if (!x) return QKM_ERR_ARG;
     if (int rc = check_tokens(c, n)) return rc;
     if (n == 0) return QKM_OK;
@@ -1233,31 +1124,23 @@ extern "C" QKM_API int qkm_ep_shared(qkm_ctx* c, uint32_t layer, const float* x,
     }
     // tensor-core kernels with an empty routed list: only the shared expert's tiles
     if (int rc = ensure_prefill_scratch(c)) return rc;
-    const uint32_t NT = prefill_pairs_per_block(), sh_now = (n + NT - 1) / NT;
     QKM_CUDA(c, cudaMemsetAsync(c->offsets, 0, sizeof(uint32_t), c->stream));
-    QKM_LAUNCH(c, launch_mma_plan(c->L(), d, c->offsets, c->pairs, 0, n, c->mma_items[0], c->mma_items[1], c->mma_items[2],
-                                  c->mma_items[3], c->n_items, c->pos_of, true));
-    QKM_LAUNCH(c, launch_to_f16_rows(c->L(), x, c->xb, c->xscale, n, d.n_embd));
-    QKM_LAUNCH(c, launch_gateup_mma(c->L(), d, QKM_TYPE_Q8_0, ld.tiles[5], ld.tiles[6], c->xb, c->xscale, c->pairs, c->mma_items[2],
-                                    c->n_items + 2, sh_now * (d.n_ff / 128), nullptr, c->hb, c->status, sh_now * (d.n_ff / 128) <= 2u * (uint32_t)c->n_sms,
-                                    nullptr, c->h));
-    QKM_LAUNCH(c, launch_h_rows_to_f16(c->L(), c->h, c->hb, c->hscale, d.n_ff, nullptr, 0, nullptr, n));   // the routed list is empty: rows 0 .. n-1
-    QKM_LAUNCH(c, launch_down_mma(c->L(), d, QKM_TYPE_Q8_0, ld.tiles[7], c->hb, c->sel, c->pairs, c->mma_items[3],
-                                  c->n_items + 3, sh_now * (d.n_embd / 128), c->contrib_p, c->status, false, nullptr, c->hscale));
+    QKM_LAUNCH(c, launch_mma_plan(c->L(), d, c->offsets, c->pairs, 0, n, c->mma_items[0], c->mma_items[1], c->n_items, c->pos_of, true));
+    QKM_LAUNCH(c, launch_f16_rows(c->L(), x, c->xb, c->xscale, c->xnorm, n, d.n_embd));
+    if (int rc = expert_gemms(c, ld, c->sel, 0, n)) return rc;   // the routed list is empty
     QKM_LAUNCH(c, launch_fold_pairs(c->L(), d, c->contrib_p, c->pos_of, c->y2, n));
     return QKM_OK;
 }
 
 // Resident experts over n_recv rows -> partial.  with_shared: rows [sh_first, sh_first + sh_count)
-// are this rank's own tokens and also get the shared expert (its two GEMMs run beside the routed
-// ones on the side stream, as in qkm_moe_prefill), so their partial rows carry shared + routed.
+// are this rank's own tokens and also get the shared expert (its units ride in the routed experts'
+// launches, as in qkm_moe_prefill), so their partial rows carry shared + routed.
 // slot_rows_peer != 0: the rows are slots of the peer-memory form and every live partial row is
 // stored into its source rank's return buffer instead of staying in `partial`.
 static int ep_expert_forward_impl(qkm_ctx* c, uint32_t layer, const float* xrecv, const qkm_sel* selrecv, uint32_t n_recv,
                                   float* partial, bool with_shared, uint32_t sh_first, uint32_t sh_count,
                                   uint32_t slot_rows_peer = 0, bool rows_f16 = false) {
     if (int rc = layer_ready(c, layer)) return rc;
-    c->shared_plan_n = 0;
     if (n_recv == 0) return QKM_OK;
     if (!xrecv || !selrecv || !partial) return QKM_ERR_ARG;
     if (int rc = check_tokens(c, n_recv)) return rc;
@@ -1285,44 +1168,17 @@ static int ep_expert_forward_impl(qkm_ctx* c, uint32_t layer, const float* xrecv
         return QKM_OK;
     }
     if (int rc = ensure_prefill_scratch(c)) return rc;
-    const uint32_t NT = prefill_pairs_per_block();
-    const uint32_t np_max = n_recv * d.n_used;
-    const uint32_t tiles_now = c->ecount < np_max ? c->ecount + (np_max + NT - 1) / NT : np_max;
-    const uint32_t rt_gu = d.n_ff / 128, rt_dn = d.n_embd / 128;
     QKM_LAUNCH(c, launch_group_pairs_wide(c->L(), d, selrecv, n_recv, c->offsets, c->pairs, c->efirst, c->ecount, c->group_hist, c->pos_of));
-    QKM_LAUNCH(c, launch_mma_plan(c->L(), d, c->offsets, c->pairs, c->ecount, n_recv, c->mma_items[0], c->mma_items[1],
-                                  c->mma_items[2], c->mma_items[3], c->n_items, c->pos_of, with_shared, true, sh_first,
-                                  with_shared ? sh_count : 0));
-    // the rows as scaled f16: converted here, or already so on arrival (then only their scales are gathered)
-    const void* xb_rows = c->xb;
+    QKM_LAUNCH(c, launch_mma_plan(c->L(), d, c->offsets, c->pairs, c->ecount, n_recv, c->mma_items[0], c->mma_items[1], c->n_items, c->pos_of,
+                                  with_shared, true, sh_first, with_shared ? sh_count : 0));
+    // the rows as scaled f16: converted here, or already so on arrival (then their scales and norms are gathered)
     if (rows_f16) {
-        xb_rows = xrecv;
         QKM_LAUNCH(c, launch_ep_row_scales(c->L(), selrecv, c->xscale, n_recv));
+        QKM_LAUNCH(c, launch_f16_rows_in(c->L(), xrecv, c->xscale, c->xb, c->xnorm, n_recv, d.n_embd));
     } else {
-        QKM_LAUNCH(c, launch_to_f16_rows(c->L(), xrecv, c->xb, c->xscale, n_recv, d.n_embd));
+        QKM_LAUNCH(c, launch_f16_rows(c->L(), xrecv, c->xb, c->xscale, c->xnorm, n_recv, d.n_embd));
     }
-    const bool fork = with_shared && sh_count;
-    if (fork) {
-        const uint32_t sh_now = (sh_count + NT - 1) / NT;
-        Launch S{c->side, &c->launches};
-        QKM_CUDA(c, cudaEventRecord(c->ev_fork, c->stream));
-        QKM_CUDA(c, cudaStreamWaitEvent(c->side, c->ev_fork, 0));
-        QKM_LAUNCH(c, launch_gateup_mma(S, d, QKM_TYPE_Q8_0, ld.tiles[5], ld.tiles[6], xb_rows, c->xscale, c->pairs, c->mma_items[2],
-                                        c->n_items + 2, sh_now * rt_gu, nullptr, c->hb, c->status, sh_now * rt_gu <= 2u * (uint32_t)c->n_sms,
-                                        nullptr, c->h));
-        QKM_LAUNCH(c, launch_h_rows_to_f16(S, c->h, c->hb, c->hscale, d.n_ff, c->offsets + c->ecount, 0, nullptr, sh_count));
-        QKM_LAUNCH(c, launch_down_mma(S, d, QKM_TYPE_Q8_0, ld.tiles[7], c->hb, selrecv, c->pairs, c->mma_items[3],
-                                      c->n_items + 3, sh_now * rt_dn, c->contrib_p, c->status, false, nullptr, c->hscale));
-        QKM_CUDA(c, cudaEventRecord(c->ev_join, c->side));
-    }
-    // a shard of few experts launches fewer blocks than the machine holds: faster blocks instead (see the launchers)
-    const bool few_gu = c->ecount * rt_gu <= 2u * (uint32_t)c->n_sms, few_dn = c->ecount * rt_dn / 4 <= 2u * (uint32_t)c->n_sms;
-    QKM_LAUNCH(c, launch_gateup_mma(c->L(), d, w.gateup_type, ld.tiles[2], ld.tiles[3], xb_rows, c->xscale, c->pairs, c->mma_items[0],
-                                    c->n_items, tiles_now * rt_gu, nullptr, c->hb, c->status, few_gu, c->lut_pf, c->h));
-    QKM_LAUNCH(c, launch_h_rows_to_f16(c->L(), c->h, c->hb, c->hscale, d.n_ff, nullptr, 0, c->offsets + c->ecount, n_recv * d.n_used));
-    QKM_LAUNCH(c, launch_down_mma(c->L(), d, w.down_type, ld.tiles[4], c->hb, selrecv, c->pairs, c->mma_items[1],
-                                  c->n_items + 1, tiles_now * rt_dn, c->contrib_p, c->status, few_dn, c->lut_dn, c->hscale));
-    if (fork) QKM_CUDA(c, cudaStreamWaitEvent(c->stream, c->ev_join, 0));
+    if (int rc = expert_gemms(c, ld, selrecv, n_recv * d.n_used, with_shared ? sh_count : 0)) return rc;
     if (slot_rows_peer)
         QKM_LAUNCH(c, launch_fold_pairs_peer(c->L(), d, c->contrib_p, c->pos_of, c->pm_peers, slot_rows_peer, c->pm_rank, c->pm_ranks));
     else
@@ -1468,7 +1324,6 @@ extern "C" QKM_API int qkm_ep_push(qkm_ctx* c, uint32_t layer, const float* x, u
     if (int rc = pm_check(c, slot_rows)) return rc;
     if (!x && n) return QKM_ERR_ARG;
     if (n > slot_rows) return fail(c, QKM_ERR_BOUNDS, "%u tokens exceed slot_rows %u", n, slot_rows);
-    c->shared_plan_n = 0;
     if (n) if (int rc = ep_route_local(c, layer, x, n)) return rc;
     // Layers whose resident experts run on the tensor cores consume the rows as scaled f16: then those
     // travel (half the bytes; every rank decides the same from the layer's types).  The router above
@@ -1479,7 +1334,7 @@ extern "C" QKM_API int qkm_ep_push(qkm_ctx* c, uint32_t layer, const float* x, u
         const float* inv = c->xscale;
         if (n < 128) {   // (the router made digit planes, whose scales sit in xscale for the streamed shared expert)
             if (int rc = ensure_prefill_scratch(c)) return rc;
-            QKM_LAUNCH(c, launch_to_f16_rows(c->L(), x, c->xb, c->pm_xscale, n, c->cfg.dims.n_embd));
+            QKM_LAUNCH(c, launch_f16_rows(c->L(), x, c->xb, c->pm_xscale, nullptr, n, c->cfg.dims.n_embd));
             inv = c->pm_xscale;
         }
         QKM_LAUNCH(c, launch_ep_push(c->L(), c->cfg.dims, x, c->sel, c->pm_peers, n, slot_rows, c->pm_rank, c->pm_ranks, c->xb, inv));

@@ -13,7 +13,7 @@
 // Arithmetic: exact integers until the last step.  When its token changes, a warp encodes the
 // 256 values of h[t][s] it multiplies with as four int8 digit planes (28-bit fixed point
 // relative to the largest of the 256, one power-of-two scale) and keeps them in registers as
-// the B operand of int8 MMAs.  IQ4_XS inner step: a quant byte holds two weights 16 columns
+// the B operand of int8 MMAs.  IQ4_XS inner step: a quant byte holds two weights two columns
 // apart; a 64 KB table image at shared address 0x10000 maps the byte to both codebook values
 // (row = byte value, 256-byte stride, one 4-byte entry per lane: bank = lane, no conflicts),
 // and a look-up address is one byte permute [lane * 4, byte, 0x01, 0x00].  Eight weights cost
@@ -95,9 +95,8 @@ __device__ __forceinline__ void iq4_scales(uint32_t sl, uint32_t sh, uint32_t& e
     od = (to & 0x20202020u) * 6u + to;
 }
 
-// Eight IQ4_XS weights of one quant word (bytes 4t..4t+3 of a sub-block's sixteen: the low nibbles are
-// elements 4t..4t+3, the high nibbles elements 16+4t..16+4t+3) as two int8 MMA A-operand registers:
-// lo = elements (4t, 16+4t, 4t+1, 17+4t), hi = elements (4t+2, 18+4t, 4t+3, 19+4t).
+// Eight IQ4_XS weights of one quant word (elements e0 .. e7 = 8t .. 8t+7 of a sub-block; a byte's nibbles are two
+// elements apart, see qkm_tiles.cuh) as two int8 MMA A-operand registers: lo = (e0, e2, e1, e3), hi = (e4, e6, e5, e7).
 // tab_c: bytes (lane * 4, -, 0x01, 0x00): with a quant byte in byte 1 it is that byte's table entry for this lane.
 __device__ __forceinline__ void iq4_word(uint32_t w, uint32_t tab_c, uint32_t& lo, uint32_t& hi) {
     const uint32_t e0 = lds32(prmt_dd(w, tab_c, 0x7604u)), e1 = lds32(prmt_dd(w, tab_c, 0x7614u));
@@ -188,6 +187,7 @@ decode_down_kernel(DownDecodeArgs a) {
     // digit weights: C columns 2t, 2t+1 are digits 2t, 2t+1 (t < 2); the other columns are zero
     const float dw0 = t == 0 ? 1.f : (t == 1 ? 16384.f : 0.f), dw1 = dw0 * 128.f;
     const uint32_t tab_c = dd::kTab + lane * 4;
+    const uint32_t i_off = 64 * g + piece_at(g, t);   // this lane's quant piece of row g (row g+8: 512 bytes on)
 
     if (!mbar_wait_bounded(tab_bar, 0)) timed_out = true;   // every thread observes the table's arrival itself
 
@@ -213,16 +213,19 @@ decode_down_kernel(DownDecodeArgs a) {
                 const int p = digit_exponent(m);
                 const float up = ldexpf(1.0f, p);
                 __syncwarp();
+                uint32_t dgt[8];
 #pragma unroll
-                for (int i = 0; i < 8; ++i) {
-                    // element e = 8 * lane + i of the 256 -> sub-block lane / 4; inside it the order of iq4_word's
-                    // registers: element 4tt + j -> register j / 2, byte 2 (j & 1); element 16 + 4tt + j one byte later
-                    const uint32_t pos = (lane >> 2) * 32 + ((lane >> 1) & 1u) + (lane & 1u) * 8 + (i >> 2) * 4 + ((i & 3) >> 1) * 16 + (i & 1) * 2;
-                    const uint32_t dgt = any_bad ? 0u : digits4(__float2int_rn(hv[i] * up));
-                    dig[pos] = (uint8_t)(dgt & 255u);
-                    dig[256 + pos] = (uint8_t)((dgt >> 8) & 255u);
-                    dig[512 + pos] = (uint8_t)((dgt >> 16) & 255u);
-                    dig[768 + pos] = (uint8_t)(dgt >> 24);
+                for (int i = 0; i < 8; ++i) dgt[i] = any_bad ? 0u : digits4(__float2int_rn(hv[i] * up));
+                // digit j of elements 8 lane + 4 r .. + 3 (lane t = lane & 3 of sub-block lane / 4, register r), in iq4_word's order 0, 2, 1, 3
+#pragma unroll
+                for (int r = 0; r < 2; ++r) {
+                    const uint32_t x0 = prmt_dd(dgt[4 * r], dgt[4 * r + 2], 0x5140u), x1 = prmt_dd(dgt[4 * r + 1], dgt[4 * r + 3], 0x5140u);
+                    const uint32_t y0 = prmt_dd(dgt[4 * r], dgt[4 * r + 2], 0x7362u), y1 = prmt_dd(dgt[4 * r + 1], dgt[4 * r + 3], 0x7362u);
+                    uint8_t* q = dig + (lane >> 2) * 32 + r * 16 + (lane & 3u) * 4;
+                    *reinterpret_cast<uint32_t*>(q) = prmt_dd(x0, x1, 0x5410u);
+                    *reinterpret_cast<uint32_t*>(q + 256) = prmt_dd(x0, x1, 0x7632u);
+                    *reinterpret_cast<uint32_t*>(q + 512) = prmt_dd(y0, y1, 0x5410u);
+                    *reinterpret_cast<uint32_t*>(q + 768) = prmt_dd(y0, y1, 0x7632u);
                 }
                 __syncwarp();
 #pragma unroll
@@ -277,7 +280,7 @@ decode_down_kernel(DownDecodeArgs a) {
 #pragma unroll
             for (int hf = 0; hf < 2; ++hf) {
                 // quant word t of sub-blocks 4hf..4hf+3: rows g and g+8
-                const uint4 qa4 = lds128(tb + 128 + (hf * 32 + lane) * 16), qb4 = lds128(tb + 128 + ((2 + hf) * 32 + lane) * 16);
+                const uint4 qa4 = lds128(tb + 128 + hf * 1024 + i_off), qb4 = lds128(tb + 640 + hf * 1024 + i_off);
                 const uint32_t wa[4] = {qa4.x, qa4.y, qa4.z, qa4.w}, wb[4] = {qb4.x, qb4.y, qb4.z, qb4.w};
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
@@ -285,8 +288,8 @@ decode_down_kernel(DownDecodeArgs a) {
                     uint32_t a0, a1, a2, a3;
                     iq4_word(wa[j], tab_c, a0, a2);
                     iq4_word(wb[j], tab_c, a1, a3);
-                    int c[4] = {0, 0, 0, 0};
-                    mma_s8(c, a0, a1, a2, a3, b0[sb], b1[sb]);
+                    int c[4];
+                    mma_s8_first(c, a0, a1, a2, a3, b0[sb], b1[sb]);
                     const uint32_t sel = 0x8880u + (uint32_t)(sb >> 1) * 0x1111u;   // byte sb / 2, sign-extended
                     const int la = (int)prmt_dd((sb & 1) ? oa : ea, 0u, sel), lb = (int)prmt_dd((sb & 1) ? ob : eb, 0u, sel);
                     acc[0] += la * c[0]; acc[1] += la * c[1]; acc[2] += lb * c[2]; acc[3] += lb * c[3];
@@ -297,8 +300,8 @@ decode_down_kernel(DownDecodeArgs a) {
             if (with_shared) {
                 const uint2 qa = lds64(qb + 32 + lane * 8);            // row g: qs[4t..4t+3], qs[16+4t..16+4t+3]
                 const uint2 qc = lds64(qb + 32 + 256 + lane * 8);      // row g+8
-                int c[4] = {0, 0, 0, 0};
-                mma_s8(c, qa.x, qc.x, qa.y, qc.y, hb0, hb1);
+                int c[4];
+                mma_s8_first(c, qa.x, qc.x, qa.y, qc.y, hb0, hb1);
                 const uint32_t dw = lds32(qb + 2 * (g & ~1u)), dw8 = lds32(qb + 2 * (8 + (g & ~1u)));
                 const float sda = f16_bits_to_f32((dw >> (16 * (g & 1u))) & 0xFFFFu);
                 const float sdb = f16_bits_to_f32((dw8 >> (16 * (g & 1u))) & 0xFFFFu);

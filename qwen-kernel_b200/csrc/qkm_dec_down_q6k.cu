@@ -136,6 +136,8 @@ decode_down_q6k_kernel(DownDecodeArgs a) {
     const float dw0 = (t & 1u) ? 16384.f : 1.f, dw1 = dw0 * 128.f;
     const float dws0 = t == 0 ? 1.f : (t == 1 ? 16384.f : 0.f), dws1 = dws0 * 128.f;   // the shared expert's MMA: digits in columns 0..3 only
 
+    const uint32_t i_off = 64 * g + piece_at(g, t);   // this lane's quant piece of row g (row g+8: 512 bytes on)
+
     uint32_t tok = u_lo / RT, rt = u_lo - tok * RT;
     bool new_tok = true;
     for (uint32_t u = u_lo; u < u_hi;) {
@@ -218,10 +220,10 @@ decode_down_q6k_kernel(DownDecodeArgs a) {
             // the eight scales of this lane's groups (even groups for t < 2, odd for t >= 2), rows g and g+8
             const uint2 scA = lds64(tb + 16 * g + 8 * (t >> 1)), scB = lds64(tb + 16 * (g + 8) + 8 * (t >> 1));
             int acc[4] = {0, 0, 0, 0};
-            const uint4 hA = lds128(tb + 256 + (2 * 32 + lane) * 16), hB = lds128(tb + 256 + (5 * 32 + lane) * 16);
+            const uint4 hA = lds128(tb + 2304 + i_off), hB = lds128(tb + 2816 + i_off);
 #pragma unroll
             for (int hf = 0; hf < 2; ++hf) {
-                const uint4 qA = lds128(tb + 256 + (hf * 32 + lane) * 16), qB = lds128(tb + 256 + ((3 + hf) * 32 + lane) * 16);
+                const uint4 qA = lds128(tb + 256 + hf * 1024 + i_off), qB = lds128(tb + 768 + hf * 1024 + i_off);
                 uint32_t a0[4], a2[4], a1[4], a3[4];
                 q6k_words(qA.x, qA.z, hf ? hA.z : hA.x, a0);   // row g, l = 4t..
                 q6k_words(qA.y, qA.w, hf ? hA.w : hA.y, a2);   // row g, l = 16 + 4t..
@@ -230,8 +232,8 @@ decode_down_q6k_kernel(DownDecodeArgs a) {
 #pragma unroll
                 for (int qd = 0; qd < 4; ++qd) {
                     const int j = 4 * hf + qd;
-                    int c[4] = {0, 0, 0, 0};
-                    mma_s8(c, a0[qd], a1[qd], a2[qd], a3[qd], b0[j], b1[j]);
+                    int c[4];
+                    mma_s8_first(c, a0[qd], a1[qd], a2[qd], a3[qd], b0[j], b1[j]);
                     const uint32_t sel = 0x8880u + (uint32_t)(j & 3) * 0x1111u;   // byte j & 3, sign-extended
                     const int sa = (int)prmt_dq(hf ? scA.y : scA.x, 0u, sel), sb = (int)prmt_dq(hf ? scB.y : scB.x, 0u, sel);
                     acc[0] += sa * c[0]; acc[1] += sa * c[1]; acc[2] += sb * c[2]; acc[3] += sb * c[3];
@@ -243,8 +245,8 @@ decode_down_q6k_kernel(DownDecodeArgs a) {
             if (with_shared) {
                 const uint2 qa = lds64(qb + 32 + lane * 8);            // row g: qs[4t..4t+3], qs[16+4t..16+4t+3]
                 const uint2 qc = lds64(qb + 32 + 256 + lane * 8);      // row g+8
-                int c[4] = {0, 0, 0, 0};
-                mma_s8(c, qa.x, qc.x, qa.y, qc.y, hb0, hb1);
+                int c[4];
+                mma_s8_first(c, qa.x, qc.x, qa.y, qc.y, hb0, hb1);
                 const uint32_t dw = lds32(qb + 2 * (g & ~1u)), dw8 = lds32(qb + 2 * (8 + (g & ~1u)));
                 const float sda = f16_bits_to_f32((dw >> (16 * (g & 1u))) & 0xFFFFu);
                 const float sdb = f16_bits_to_f32((dw8 >> (16 * (g & 1u))) & 0xFFFFu);

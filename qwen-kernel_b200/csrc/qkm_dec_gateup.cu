@@ -44,12 +44,12 @@ namespace qkm {
 namespace dg {
 constexpr int kWarps = 16;
 constexpr int kStages = 2;
-constexpr int kStageBytes = 2 * kTileIq3;          // gate tile + up tile (3136); a Q8_0 quarter pair needs 2176
+constexpr int kStageBytes = 2 * kTileIq3;          // gate tile + up tile (3392); a Q8_0 quarter pair needs 2176
 constexpr int kRingBytes = kStages * kStageBytes;
 constexpr int kStageBytes4 = 2 * kTileIq4;         // the IQ4_XS form: 4352
 constexpr int kRingBytes4 = kStages * kStageBytes4;
 constexpr uint32_t kTab = 65536, kTabBytes = 65536;   // absolute shared-window address (64 KB aligned) and size
-constexpr int kLowRingWarps = 10;                   // rings below the table; the others above it
+constexpr int kLowRingWarps = 9;                    // rings below the table; the others above it
 constexpr int kGroupTiles = 4;                      // tiles between two team-wide reductions
 constexpr int kRedFloats = kGroupTiles * 16 * 2 * 2;   // per warp and buffer: tile, row, token, matrix
 constexpr uint32_t kHigh = kTab + kTabBytes;
@@ -100,37 +100,36 @@ __device__ __forceinline__ uint32_t prmt(uint32_t a, uint32_t b, uint32_t sel) {
 
 // One IQ3_XXS tile (16 rows x 256 columns) of one matrix against the warp's B operand.
 // acc[0..1]: row g, columns 2t and 2t+1; acc[2..3]: row g+8.  Integer, exact.
-__device__ __forceinline__ void iq3_tile(uint32_t tb, uint32_t lane, uint32_t g, uint32_t grid_c, uint32_t sign_c,
-                                         uint32_t rot, const uint32_t (&b0)[8], const uint32_t (&b1)[8],
+__device__ __forceinline__ void iq3_tile(uint32_t tb, uint32_t i_off, uint32_t s_off, uint32_t g, uint32_t grid_c,
+                                         const uint32_t (&b0)[8], const uint32_t (&b1)[8],
                                          const uint32_t (&n0)[8], const uint32_t (&n1)[8], int (&acc)[4]) {
-    const uint4 ia = lds128(tb + lane * 16);          // row g: 8 index pairs
-    const uint4 ib = lds128(tb + 512 + lane * 16);    // row g+8
-    const uint4 xa0 = lds128(tb + 1024 + 16 * g), xa1 = lds128(tb + 1280 + 16 * g);
-    const uint4 xb0 = lds128(tb + 1152 + 16 * g), xb1 = lds128(tb + 1408 + 16 * g);
+    const uint4 ia = lds128(tb + i_off), ib = lds128(tb + i_off + 512);                          // rows g and g+8: 2 index bytes per sub-block
+    const uint2 sa = lds64(tb + 1024 + s_off), sb2 = lds64(tb + 1280 + s_off);                    // signs
+    const uint2 ca = lds64(tb + 1536 + 8 * g), cb = lds64(tb + 1600 + 8 * g);                     // scales 2 s + 1
     const uint32_t idx_a[4] = {ia.x, ia.y, ia.z, ia.w}, idx_b[4] = {ib.x, ib.y, ib.z, ib.w};
-    const uint32_t aux_a[8] = {xa0.x, xa0.y, xa0.z, xa0.w, xa1.x, xa1.y, xa1.z, xa1.w};
-    const uint32_t aux_b[8] = {xb0.x, xb0.y, xb0.z, xb0.w, xb1.x, xb1.y, xb1.z, xb1.w};
     acc[0] = acc[1] = acc[2] = acc[3] = 0;
 #pragma unroll
     for (int sb = 0; sb < 8; ++sb) {
-        const uint32_t wa = idx_a[2 * (sb & 1) + (sb >> 2)], wb = idx_b[2 * (sb & 1) + (sb >> 2)];   // even sub-blocks in words 0,1; odd in 2,3
-        const uint32_t s_lo = (sb & 2) ? 0x7624u : 0x7604u, s_hi = (sb & 2) ? 0x7634u : 0x7614u;
+        const uint32_t wa = idx_a[sb >> 1], wb = idx_b[sb >> 1];
+        const uint32_t s_lo = (sb & 1) ? 0x7624u : 0x7604u, s_hi = (sb & 1) ? 0x7634u : 0x7614u;
         const uint32_t ga0 = lds32(prmt(wa, grid_c, s_lo)), ga1 = lds32(prmt(wa, grid_c, s_hi));
         const uint32_t gb0 = lds32(prmt(wb, grid_c, s_lo)), gb1 = lds32(prmt(wb, grid_c, s_hi));
-        const uint32_t xa = aux_a[4 * (sb & 1) + (sb >> 1)], xb = aux_b[4 * (sb & 1) + (sb >> 1)];
-        const uint2 ma = lds64((__funnelshift_l(xa, xa, rot) & 0xFE00u) | sign_c);
-        const uint2 mb = lds64((__funnelshift_l(xb, xb, rot) & 0xFE00u) | sign_c);
-        int c[4] = {0, 0, 0, 0};
-        mma_s8(c, ga0 ^ ma.x, gb0 ^ mb.x, ga1 ^ ma.y, gb1 ^ mb.y, b0[sb], b1[sb]);
-        mma_s8(c, ma.x, mb.x, ma.y, mb.y, n0[sb], n1[sb]);
-        const int qa = (int)(2u * (xa >> 28) + 1u), qb = (int)(2u * (xb >> 28) + 1u);
+        // 0xFF bytes where negative: the top bits of the shifted sign word's bytes, replicated (the shift is a multiply's pipe, not the ALU's)
+        const uint32_t va = (sb < 4 ? sa.x : sa.y), vb = (sb < 4 ? sb2.x : sb2.y);
+        const uint32_t ma0 = prmt(va * (1u << (2 * (sb & 3))), 0u, 0xBA98u), ma1 = prmt(va * (2u << (2 * (sb & 3))), 0u, 0xBA98u);
+        const uint32_t mb0 = prmt(vb * (1u << (2 * (sb & 3))), 0u, 0xBA98u), mb1 = prmt(vb * (2u << (2 * (sb & 3))), 0u, 0xBA98u);
+        int c[4];
+        mma_s8_first(c, ga0 ^ ma0, gb0 ^ mb0, ga1 ^ ma1, gb1 ^ mb1, b0[sb], b1[sb]);
+        mma_s8(c, ma0, mb0, ma1, mb1, n0[sb], n1[sb]);
+        const uint32_t sel = 0x4440u + (uint32_t)(sb & 3);
+        const int qa = (int)prmt(sb < 4 ? ca.x : ca.y, 0u, sel), qb = (int)prmt(sb < 4 ? cb.x : cb.y, 0u, sel);
         acc[0] += qa * c[0]; acc[1] += qa * c[1];
         acc[2] += qb * c[2]; acc[3] += qb * c[3];
     }
 }
 
-// Eight IQ4_XS weights of one quant word (low nibbles: elements 4t..4t+3, high nibbles: 16+4t..16+4t+3) as
-// two int8 A-operand registers: lo = elements (4t, 16+4t, 4t+1, 17+4t), hi = (4t+2, 18+4t, 4t+3, 19+4t).
+// Eight IQ4_XS weights of one quant word (elements e0 .. e7 = 8t .. 8t+7 of a sub-block, see qkm_tiles.cuh) as
+// two int8 A-operand registers: lo = (e0, e2, e1, e3), hi = (e4, e6, e5, e7).
 __device__ __forceinline__ void iq4_word_gu(uint32_t w, uint32_t& lo, uint32_t& hi) {
     const uint32_t T0 = 0xBFAD9881u, T1 = 0xF6EADDCFu, T2 = 0x26190D01u, T3 = 0x71594535u;   // kvalues_iq4nl as int8
     const uint32_t s = w & 0x77777777u, s2 = s >> 16, w4 = w << 4;
@@ -152,7 +151,7 @@ __device__ __forceinline__ void iq4_scales_gu(uint32_t sl, uint32_t sh, uint32_t
 }
 // One IQ4_XS tile against the warp's B operand (elements in iq4_word_gu's order).  acc as in iq3_tile;
 // hd: the headers of rows g (x: d | scales_h << 16, y: scales_l) and g+8 (z, w).
-__device__ __forceinline__ void iq4_tile_gu(uint32_t tb, uint32_t lane, uint32_t g, const uint32_t (&b0)[8],
+__device__ __forceinline__ void iq4_tile_gu(uint32_t tb, uint32_t i_off, uint32_t g, const uint32_t (&b0)[8],
                                             const uint32_t (&b1)[8], int (&acc)[4], uint4& hd) {
     hd = lds128(tb + 16 * g);
     uint32_t ea, oa, eb, ob;
@@ -161,7 +160,7 @@ __device__ __forceinline__ void iq4_tile_gu(uint32_t tb, uint32_t lane, uint32_t
     acc[0] = acc[1] = acc[2] = acc[3] = 0;
 #pragma unroll
     for (int hf = 0; hf < 2; ++hf) {
-        const uint4 qa4 = lds128(tb + 128 + (hf * 32 + lane) * 16), qb4 = lds128(tb + 128 + ((2 + hf) * 32 + lane) * 16);
+        const uint4 qa4 = lds128(tb + 128 + hf * 1024 + i_off), qb4 = lds128(tb + 640 + hf * 1024 + i_off);
         const uint32_t wa[4] = {qa4.x, qa4.y, qa4.z, qa4.w}, wb[4] = {qb4.x, qb4.y, qb4.z, qb4.w};
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
@@ -169,8 +168,8 @@ __device__ __forceinline__ void iq4_tile_gu(uint32_t tb, uint32_t lane, uint32_t
             uint32_t a0, a1, a2, a3;
             iq4_word_gu(wa[j], a0, a2);
             iq4_word_gu(wb[j], a1, a3);
-            int c[4] = {0, 0, 0, 0};
-            mma_s8(c, a0, a1, a2, a3, b0[sb], b1[sb]);
+            int c[4];
+            mma_s8_first(c, a0, a1, a2, a3, b0[sb], b1[sb]);
             const uint32_t sel = 0x8880u + (uint32_t)(sb >> 1) * 0x1111u;   // byte sb / 2, sign-extended
             const int la = (int)prmt((sb & 1) ? oa : ea, 0u, sel), lb = (int)prmt((sb & 1) ? ob : eb, 0u, sel);
             acc[0] += la * c[0]; acc[1] += la * c[1]; acc[2] += lb * c[2]; acc[3] += lb * c[3];
@@ -186,8 +185,8 @@ __device__ __forceinline__ void q8_quarter(uint32_t q, uint32_t lane, uint32_t g
         const uint32_t pb = q + 544 * bb;
         const uint2 qa = lds64(pb + 32 + lane * 8);
         const uint2 qb = lds64(pb + 32 + 256 + lane * 8);
-        int c[4] = {0, 0, 0, 0};
-        mma_s8(c, qa.x, qb.x, qa.y, qb.y, bb ? b0b : b0a, bb ? b1b : b1a);
+        int c[4];
+        mma_s8_first(c, qa.x, qb.x, qa.y, qb.y, bb ? b0b : b0a, bb ? b1b : b1a);
         const uint32_t dw = lds32(pb + 2 * (g & ~1u));
         const uint32_t dw8 = lds32(pb + 2 * (8 + (g & ~1u)));
         const float da = f16_bits_to_f32((dw >> (16 * (g & 1u))) & 0xFFFFu);
@@ -302,8 +301,7 @@ decode_gateup_kernel(GateupDecodeArgs a) {
         for (int s = 0; s < dg::kStages; ++s) issue(s);
 
     const uint32_t grid_c = dg::kTab + lane * 4;
-    const uint32_t sign_c = dg::kTab + (lane >> 4) * 256 + 128 + (lane & 15u) * 8;
-    const uint32_t rot = (41u - 7u * t) & 31u;     // rotate-left that brings sign code t to bits 9..15
+    const uint32_t i_off = 64 * g + piece_at(g, t), s_off = 32 * g + 16 * ((t >> 1) ^ ((g >> 2) & 1u)) + 8 * (t & 1u);   // this lane's pieces of row g (rows g+8 alike)
     const uint32_t team_threads = KB * 32, lt = tid - team * team_threads;
     uint32_t cnt = 0;   // stages consumed by this warp
     uint32_t b0[8], b1[8], n0[8], n1[8];
@@ -337,10 +335,9 @@ decode_gateup_kernel(GateupDecodeArgs a) {
                 const int8_t* pl = a.planes + (((size_t)tok * KB + kb) * 8 + dgt) * 256;
 #pragma unroll
                 for (int sb = 0; sb < 8; ++sb) {
-                    if (IQ4 && rec.kind == 0) {   // iq4_word_gu's order: (4t, 16+4t, 4t+1, 17+4t | 4t+2, 18+4t, 4t+3, 19+4t)
-                        const uint32_t v = *reinterpret_cast<const uint32_t*>(pl + 32 * sb + 4 * t);
-                        const uint32_t u = *reinterpret_cast<const uint32_t*>(pl + 32 * sb + 16 + 4 * t);
-                        b0[sb] = prmt(v, u, 0x5140u); b1[sb] = prmt(v, u, 0x7362u);
+                    if (IQ4 && rec.kind == 0) {   // iq4_word_gu's order
+                        const uint2 v = *reinterpret_cast<const uint2*>(pl + 32 * sb + 8 * t);
+                        b0[sb] = prmt(v.x, 0u, 0x3120u); b1[sb] = prmt(v.y, 0u, 0x3120u);
                     } else if (rec.kind == 0) {   // lane t owns elements 8t .. 8t+7 of each sub-block
                         const uint2 v = *reinterpret_cast<const uint2*>(pl + 32 * sb + 8 * t);
                         const uint2 n = *reinterpret_cast<const uint2*>(pl + 1024 + 32 * sb + 8 * t);
@@ -372,8 +369,8 @@ decode_gateup_kernel(GateupDecodeArgs a) {
             int ig[4], iu[4];
             if (IQ4) {
                 uint4 hg, hu;
-                iq4_tile_gu(sbase, lane, g, b0, b1, ig, hg);
-                iq4_tile_gu(sbase + kTileIq4, lane, g, b0, b1, iu, hu);
+                iq4_tile_gu(sbase, i_off, g, b0, b1, ig, hg);
+                iq4_tile_gu(sbase + kTileIq4, i_off, g, b0, b1, iu, hu);
                 __syncwarp();
                 if (lane == 0) issue(stage);
                 ++cnt;
@@ -382,10 +379,10 @@ decode_gateup_kernel(GateupDecodeArgs a) {
                 ua = f16_bits_to_f32(hu.x & 0xFFFFu) * ((float)iu[0] * wcol0 + (float)iu[1] * wcol1);
                 ub = f16_bits_to_f32(hu.z & 0xFFFFu) * ((float)iu[2] * wcol0 + (float)iu[3] * wcol1);
             } else {
-            iq3_tile(sbase, lane, g, grid_c, sign_c, rot, b0, b1, n0, n1, ig);
-            iq3_tile(sbase + kTileIq3, lane, g, grid_c, sign_c, rot, b0, b1, n0, n1, iu);
-            const uint32_t dwa = lds32(sbase + 1536 + 2 * (g & ~1u)), dwb = lds32(sbase + 1536 + 2 * ((g + 8) & ~1u));
-            const uint32_t uwa = lds32(sbase + kTileIq3 + 1536 + 2 * (g & ~1u)), uwb = lds32(sbase + kTileIq3 + 1536 + 2 * ((g + 8) & ~1u));
+            iq3_tile(sbase, i_off, s_off, g, grid_c, b0, b1, n0, n1, ig);
+            iq3_tile(sbase + kTileIq3, i_off, s_off, g, grid_c, b0, b1, n0, n1, iu);
+            const uint32_t dwa = lds32(sbase + 1664 + 2 * (g & ~1u)), dwb = lds32(sbase + 1664 + 2 * ((g + 8) & ~1u));
+            const uint32_t uwa = lds32(sbase + kTileIq3 + 1664 + 2 * (g & ~1u)), uwb = lds32(sbase + kTileIq3 + 1664 + 2 * ((g + 8) & ~1u));
             __syncwarp();
             if (lane == 0) issue(stage);
             ++cnt;

@@ -308,8 +308,6 @@ cudaError_t launch_down_stream(const Launch& L, const qkm_dims& d, uint32_t type
                                uint32_t* arrivals, uint32_t n_blocks, uint32_t* status) {
     const uint32_t KB = d.n_ff / 256;
     if (KB < 2 || KB > 16 || (KB & (KB - 1)) || d.n_embd % dn::kRowsPerItem || d.n_used > 15) return cudaErrorInvalidValue;
-    if (type == QKM_TYPE_IQ4_XS)
-        return down_stream_launch<QKM_TYPE_IQ4_XS>(L, d, tiles, hpieces, sel, pairs, items, n_items, contrib, y, arrivals, n_blocks, status);
     if (type == QKM_TYPE_Q8_0)
         return down_stream_launch<QKM_TYPE_Q8_0>(L, d, tiles, hpieces, sel, pairs, items, n_items, contrib, y, arrivals, n_blocks, status);
     return cudaErrorInvalidValue;

@@ -338,8 +338,6 @@ cudaError_t launch_gateup_stream(const Launch& L, const qkm_dims& d, uint32_t ty
                                  float* h, void* hpieces, uint32_t n_blocks, uint32_t* status) {
     const uint32_t KB = d.n_embd / 256;
     if (KB < 2 || KB > 8 || (KB & (KB - 1)) || d.n_ff % gu::kRowsPerItem || d.n_used > 15) return cudaErrorInvalidValue;
-    if (type == QKM_TYPE_IQ3_XXS)
-        return gateup_stream_launch<QKM_TYPE_IQ3_XXS>(L, d, gate_tiles, up_tiles, xplanes, xscale, pairs, items, n_items, h, hpieces, n_blocks, status);
     if (type == QKM_TYPE_Q8_0)
         return gateup_stream_launch<QKM_TYPE_Q8_0>(L, d, gate_tiles, up_tiles, xplanes, xscale, pairs, items, n_items, h, hpieces, n_blocks, status);
     return cudaErrorInvalidValue;

@@ -150,7 +150,8 @@ ep_push_kernel(const float* __restrict__ x, const __half* __restrict__ xh, const
     if (xh != nullptr) {
         const uint4* src = reinterpret_cast<const uint4*>(xh + (size_t)i * n_embd);
         for (uint32_t c = tid; c < n_embd / 8; c += blockDim.x) {
-            const uint4 v = __ldg(src + c);
+            const uint4 u = __ldg(src + c);   // every four elements as (0, 2, 1, 3); they travel in their own order
+            const uint4 v = make_uint4(__byte_perm(u.x, u.y, 0x5410), __byte_perm(u.x, u.y, 0x7632), __byte_perm(u.z, u.w, 0x5410), __byte_perm(u.z, u.w, 0x7632));
             for (uint32_t d = 0; d < n_ranks; ++d)
                 if (dest >> d & 1u) reinterpret_cast<uint4*>(reinterpret_cast<__half*>(peers.x[d]) + row * n_embd)[c] = v;
         }

@@ -64,7 +64,7 @@ struct StreamItem {
     uint32_t pair_off;
 };
 
-// One block of the prefill GEMMs: an expert, a 128-row tile of its matrix and up to 128
+// One unit of the prefill GEMMs: an expert, 256 rows of its matrices and up to 128
 // of its pairs (pairs[pair_off .. pair_off + n)).
 struct MmaItem {
     uint16_t expert;
@@ -135,34 +135,47 @@ cudaError_t launch_decode_down(const Launch& L, const DownDecodeArgs& a, uint32_
 // the same with the routed experts as Q6_K tiles
 cudaError_t launch_decode_down_q6k(const Launch& L, const DownDecodeArgs& a, uint32_t n_blocks);
 
-// ---- qkm_prefill.cu : tcgen05 expert GEMMs for batched prefill
-uint32_t prefill_pairs_per_block();
-// x rows as f16 scaled per row by a power of two (inv_scale[row] undoes it)
-cudaError_t launch_to_f16_rows(const Launch& L, const float* x, void* xh, float* inv_scale, uint32_t n_rows, uint32_t K);
+// ---- qkm_wgemm.cu : tcgen05 GEMMs with quantised weights (batched prefill, dense projections)
+constexpr uint16_t kSharedItem = 0xFFFFu;   // MmaItem::expert of the shared expert's units
+uint32_t wgemm_rows_per_unit();             // activation rows per unit
+size_t wgemm_table_bytes();
+cudaError_t launch_wgemm_table(const Launch& L, uint8_t* out);
+// x rows as f16 in the kernels' element order (0, 2, 1, 3 in every group of four), scaled per row by a power of two
+// (inv_scale[row] undoes it); norm (optional): the rows' 2-norms
+cudaError_t launch_f16_rows(const Launch& L, const float* x, void* xh, float* inv_scale, float* norm, uint32_t n_rows, uint32_t K);
+// rows that arrived as scaled f16 in their own element order: a copy in the kernels' order, and the norms
+cudaError_t launch_f16_rows_in(const Launch& L, const void* in, const float* inv_scale, void* out, float* norm, uint32_t n_rows, uint32_t K);
+// out[e] (zero before) = largest row 2-norm of matrix e (raw ggml rows), rounded up
+cudaError_t launch_row_norm_max(const Launch& L, uint32_t type, const void* w, float* out, uint32_t n_mats, uint32_t rows, uint32_t K);
+struct WgemmExperts {
+    const void* w[2];          // routed tiles: gate and up, or down
+    const void* sh[2];         // the shared expert's Q8_0 tiles
+    const MmaItem* items;
+    const uint32_t* n_items;   // device word
+    uint32_t* ticket;          // device word, zero before the launch
+    const uint32_t* pairs;
+    const uint8_t* table;
+    uint32_t* status;
+    uint32_t n_experts;        // resident experts
+    uint32_t n_sms;
+};
+// h (f16, scaled per pair position, element order as above) = silu(gate x) * (up x); w_norm [2][n_experts + 1]
+cudaError_t launch_wgemm_gateup(const Launch& L, const qkm_dims& d, uint32_t type, const WgemmExperts& x, const void* xrows,
+                                const float* x_inv_scale, const float* x_norm, const float* w_norm, void* h, float* h_inv_scale, uint32_t max_units);
+// contrib[pair position][n_embd] = routing weight * down h
+cudaError_t launch_wgemm_down(const Launch& L, const qkm_dims& d, uint32_t type, const WgemmExperts& x, const void* h, uint64_t n_hrows,
+                              const float* h_inv_scale, const qkm_sel* sel, float* contrib, uint32_t max_units);
+// Dense quantised GEMM Y[n][M] = X[n][K] . W^T (W tile-ordered Q8_0 / IQ4_XS, M % 128 == 0, K % 256 == 0).
+// Scratch: xh n*K f16, x_inv_scale n floats.
+cudaError_t launch_dense_gemm(const Launch& L, uint32_t type, const void* tiles, uint32_t M, uint32_t K, const float* x, uint32_t n_rows, float* y,
+                              void* xh, float* x_inv_scale, const uint8_t* table, uint32_t n_sms, uint32_t* status);
+
+// ---- qkm_prefill.cu : work lists, router logits and the fold around them
 cudaError_t launch_mma_plan(const Launch& L, const qkm_dims& d, const uint32_t* offsets, uint32_t* pairs,
-                            uint32_t n_expert_local, uint32_t n_tokens, MmaItem* items_gu, MmaItem* items_dn,
-                            MmaItem* items_sh_gu, MmaItem* items_sh_dn, uint32_t* n_items, uint32_t* pos_of,
+                            uint32_t n_expert_local, uint32_t n_tokens, MmaItem* items_gu, MmaItem* items_dn, uint32_t* n_items, uint32_t* pos_of,
                             bool with_shared = true, bool routed_pos_done = false, uint32_t sh_first = 0,
                             uint32_t sh_count = 0xFFFFFFFFu /* all rows */);
-cudaError_t launch_gateup_mma(const Launch& L, const qkm_dims& d, uint32_t type, const void* gate_tiles,
-                              const void* up_tiles, const void* xb, const float* x_inv_scale, const uint32_t* pairs,
-                              const MmaItem* items, const uint32_t* n_items, uint32_t max_items, float* h, void* hb,
-                              uint32_t* status, bool few_blocks = false,   // few_blocks: the grid will not fill the machine
-                              const uint8_t* iq3_table = nullptr,          // IQ3_XXS: the table image (launch_gateup_iq3_table) selects the table-driven kernel
-                              float* hp = nullptr);                        // f32 rows by pair position instead of the bf16 rows in hb (see launch_h_rows_to_f16)
-// rows [first, first + count) of hp (f32, K wide) -> f16 rows scaled per row by a power of two + the inverse scales;
-// first = *first_ptr + first_add (first_ptr may be null), count = min(*count_ptr, count_max) (count_ptr may be null)
-cudaError_t launch_h_rows_to_f16(const Launch& L, const float* hp, void* hh, float* inv_scale, uint32_t K,
-                                 const uint32_t* first_ptr, uint32_t first_add, const uint32_t* count_ptr, uint32_t count_max);
-size_t gateup_iq3_table_bytes();
-cudaError_t launch_gateup_iq3_table(const Launch& L, uint8_t* out);
-cudaError_t launch_down_mma(const Launch& L, const qkm_dims& d, uint32_t type, const void* tiles, const void* hb,
-                            const qkm_sel* sel, const uint32_t* pairs, const MmaItem* items, const uint32_t* n_items,
-                            uint32_t max_items, float* contrib, uint32_t* status, bool few_blocks = false,
-                            const uint8_t* iq4_table = nullptr,    // IQ4_XS: the table image (launch_down_iq4_table) selects the table-driven kernel
-                            const float* h_inv_scale = nullptr);   // hb holds scaled f16 rows (launch_h_rows_to_f16): f16 operands
-size_t down_iq4_table_bytes();
-cudaError_t launch_down_iq4_table(const Launch& L, uint8_t* out);
+cudaError_t launch_router_f16(const Launch& L, uint32_t router_type, const void* router, void* out, uint64_t n_elems);
 cudaError_t launch_fold_pairs(const Launch& L, const qkm_dims& d, const float* contrib, const uint32_t* pos_of,
                               float* y, uint32_t n_tokens);
 
@@ -235,10 +248,10 @@ cudaError_t launch_route_select(const Launch& L, const qkm_dims& d, uint32_t rou
                                 const void* router, const float* gis, const float* x, qkm_sel* sel,
                                 uint32_t n_tokens, void* scratch, size_t scratch_bytes, int8_t* xplanes = nullptr,
                                 float* xscale = nullptr, const void* x_f16 = nullptr, const float* x_f16_inv = nullptr,
-                                uint32_t* status = nullptr, const RoutePlan* plan = nullptr);
-// f32 logits from f16 operands on the tensor cores (x_f16 / x_inv_scale as written by launch_to_f16_rows);
-// |error| <= 2^-9 * |router row| * |x|.  Needs n_expert % 128 == 0 and n_embd <= 4096.
-cudaError_t launch_logits_mma(const Launch& L, const qkm_dims& d, uint32_t router_type, const void* router,
+                                uint32_t* status = nullptr, const RoutePlan* plan = nullptr, const void* router_f16 = nullptr);
+// f32 logits from f16 operands on the tensor cores (router_f16 as written by launch_router_f16, x_f16 / x_inv_scale by
+// launch_f16_rows); |error| <= 2^-9 * |router row| * |x|.  Needs n_expert % 128 == 0 and n_embd <= 4096.
+cudaError_t launch_logits_mma(const Launch& L, const qkm_dims& d, const void* router_f16,
                               const void* x_f16, const float* x_inv_scale, float* logits, uint32_t n_tokens,
                               uint32_t* status, uint32_t splits = 1)   /* splits > 1: partial logits over column ranges, [splits][n_tokens][n_expert] */;
 cudaError_t launch_group_pairs(const Launch& L, const qkm_dims& d, const qkm_sel* sel, uint32_t n_tokens,
@@ -288,13 +301,6 @@ cudaError_t launch_shared_down(const Launch& L, const qkm_dims& d, const void* d
 // y[t][o] = sum over slots (in order) of contrib[t][s][o], plus y2[t][o] when y2 != NULL
 cudaError_t launch_fold_contrib(const Launch& L, const qkm_dims& d, const float* contrib, const float* y2,
                                 float* y, uint32_t n_tokens);
-
-// Dense quantised GEMM Y[n][M] = X[n][K] . W^T on the tcgen05 pipeline (W tile-ordered Q8_0 / IQ4_XS,
-// M % 128 == 0, K % 256 == 0).  Scratch: xb n*K bf16, pairs n words, unit_sel n records,
-// items ceil(n/128) * M/128 entries, n_items one word.
-cudaError_t launch_dense_gemm(const Launch& L, uint32_t type, const void* tiles, uint32_t M, uint32_t K, const float* x,
-                              uint32_t n_rows, float* y, void* xb, uint32_t* pairs, qkm_sel* unit_sel, MmaItem* items,
-                              uint32_t* n_items, uint32_t* status);
 
 // ---- residual adds fused with the RMS norm (qkm_tail.cu) ---------------------------------------
 // mode 0: s = a + b; 1: s = a + b + c2; 2: s = a + sum_k b[row][k][:] + c2 (b = per-slot contributions).

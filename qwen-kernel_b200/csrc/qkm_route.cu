@@ -780,7 +780,7 @@ size_t route_scratch_bytes(uint32_t n_tokens, uint32_t n_expert) {
 cudaError_t launch_route_select(const Launch& L, const qkm_dims& d, uint32_t router_type,
                                 const void* router, const float* gis, const float* x, qkm_sel* sel,
                                 uint32_t n_tokens, void* scratch, size_t scratch_bytes, int8_t* xplanes, float* xscale,
-                                const void* x_f16, const float* x_f16_inv, uint32_t* status, const RoutePlan* plan) {
+                                const void* x_f16, const float* x_f16_inv, uint32_t* status, const RoutePlan* plan, const void* router_f16) {
     if (n_tokens == 0) return cudaSuccess;
     GroupTail tail{};
     if (plan && plan->counter && n_tokens <= kExactMaxTokens && n_tokens * d.n_used <= kTailMaxPairs) {
@@ -808,7 +808,7 @@ cudaError_t launch_route_select(const Launch& L, const qkm_dims& d, uint32_t rou
     const uint8_t* r = (const uint8_t*)router;
     float eps_terms, eps_abs = 0.f;
     uint32_t n_parts = 1;
-    if (x_f16 && x_f16_inv && status && n_tokens >= 128 && d.n_expert % 128 == 0 && d.n_embd <= 4096) {
+    if (x_f16 && x_f16_inv && router_f16 && status && n_tokens >= 128 && d.n_expert % 128 == 0 && d.n_embd <= 4096) {
         // tensor cores, f16 operands: |error| <= 2^-9 |w| |x|, plus the flush of tiny router values.
         // Few output tiles: the columns are split over more blocks, partial logits side by side
         // (summed by the selection kernel).
@@ -822,7 +822,7 @@ cudaError_t launch_route_select(const Launch& L, const qkm_dims& d, uint32_t rou
         else
             row_norm2_kernel<QKM_TYPE_F16><<<(d.n_expert + 7) / 8, 256, 0, L.stream>>>(r, norm2, d.n_expert, d.n_embd);
         L.count();
-        cudaError_t e = launch_logits_mma(L, d, router_type, router, x_f16, x_f16_inv, logits, n_tokens, status, splits);
+        cudaError_t e = launch_logits_mma(L, d, router_f16, x_f16, x_f16_inv, logits, n_tokens, status, splits);
         if (e != cudaSuccess) return e;
         n_parts = splits;
         eps_terms = 32768.f + (float)splits;       // 2^-9 / 2^-24, plus the additions of the partial sums

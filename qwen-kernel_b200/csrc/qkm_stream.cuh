@@ -53,6 +53,24 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint32_t bar, uint32_t parity)
     return false;
 }
 
+// The same for waits that are long as a rule: the hardware may suspend the thread for up to 0.2 ms a poll, so a warp
+// that waits takes no issue slots from those that work.  Gives up after about half a second.
+__device__ __forceinline__ bool mbar_wait_timed(uint32_t bar, uint32_t parity) {
+#pragma unroll 1
+    for (uint32_t i = 0; i < 2500; ++i) {
+        uint32_t ok;
+        asm volatile(
+            "{\n"
+            ".reg .pred p;\n"
+            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n"
+            "selp.u32 %0, 1, 0, p;\n"
+            "}\n"
+            : "=r"(ok) : "r"(bar), "r"(parity), "r"(200000u) : "memory");
+        if (ok) return true;
+    }
+    return false;
+}
+
 // ---- tensor-core MMAs (warp-level; operands in registers) -----------------------------
 // D(16x8, s32) += A(16x32, s8, row) * B(32x8, s8, col)
 __device__ __forceinline__ void mma_s8(int (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3,

@@ -2,43 +2,45 @@
 // activation encoding they consume ("digit planes").
 //
 // TILES.  qkm_upload_layer keeps the raw ggml tensors and additionally stores a
-// re-ordered copy: the same bytes, grouped so that one warp can fetch everything it
-// needs for 16 rows x 256 columns with one bulk copy and read it back from shared
-// memory with aligned, conflict-free 128-bit loads.  A tile holds exactly the bytes
-// of its 16 row-blocks (no padding, nothing recomputed), so tile bytes = 16 x
-// block bytes x (256 / block elements): IQ3_XXS 1568, IQ4_XS 2176, Q6_K 3360, Q8_0 4352.
+// re-ordered copy, grouped so that one bulk copy fetches everything a warp (decode) or a
+// 128-row unit (prefill) needs and both read it back from shared memory with aligned,
+// conflict-free 128-bit loads: a decode lane reads its 16 bytes of two rows, a prefill
+// thread all bytes of one row.  Values are unchanged; bytes per 16 x 256 tile: IQ3_XXS 1696
+// (1568 in the file: the 7-bit sign codes are stored as 8 sign bits, the 4-bit scales as bytes 2 s + 1 -
+// two instructions less per eight weights for 8 % more bytes in kernels bound by instruction issue),
+// IQ4_XS 2176, Q6_K 3360, Q8_0 4352 as in the file.
 // Tiles of one matrix [rows][K] are ordered [kb = K/256][rt = rows/16]: a warp that
-// owns column block kb walks consecutive memory as it moves down the rows.
+// owns column block kb walks consecutive memory as it moves down the rows, and the eight tiles of 128 rows are
+// one run.
 //
 // Inside a tile, "lane" is the MMA lane 4*g + t (g = 0..7 row group, t = 0..3):
-// lane (g,t) works on rows g and g+8 of the tile.
+// lane (g,t) works on rows g and g+8 of the tile, on columns 8t .. 8t+7 of every 32-column sub-block
+// (IQ3_XXS, IQ4_XS).  A row's four 16-byte pieces t of a 64-byte run lie at piece position t ^ ((row >> 1) & 3):
+// eight consecutive rows that each read piece t, and one row group's lanes that read pieces 0..3, both hit
+// all 32 banks once.
 //
 //   IQ3_XXS (block: d f16 | qs[64] grid indices | 8 aux words, src/quants.h:115-119)
-//     [   0,1024)  index pairs: half h (row g + 8h), lane -> 16 B = for each of the 8
-//                  sub-blocks the two grid indices of 8-element group t
-//                  (raw qs[8*ib + 2*t], qs[8*ib + 2*t + 1]), the even sub-blocks 0,2,4,6 in
-//                  the first 8 bytes and the odd ones in the last 8 (a prefill thread owns one
-//                  32-column half of every 64-column k-step: one 8-byte load); address
-//                  h*512 + lane*16
-//     [1024,1536)  aux words (4 x 7 sign bits + 4 scale bits each), unchanged, as two halves:
-//                  the words of sub-blocks par, 2+par, 4+par, 6+par of row r at
-//                  1024 + 256*par + 16*r, so the 16-byte loads of eight rows g (or g+8) hit
-//                  eight consecutive 16-byte slots
-//     [1536,1568)  d[16] f16
+//     [   0,1024)  grid indices: row r at 64 r, piece t: 2 bytes for each of the eight sub-blocks
+//                  (raw qs[8*ib + 2*t], qs[8*ib + 2*t + 1])
+//     [1024,1536)  signs: row r at 1024 + 32 r, lane t's 8 bytes at 16 ((t >> 1) ^ ((r >> 2) & 1)) + 8 (t & 1): two words,
+//                  word q for sub-blocks 4q .. 4q+3; bit 7 - (2 (s & 3) + h) of byte b = element 8t + 4h + b of sub-block s
+//                  is negative (shifted left by 2 (s & 3) + h, the four sign bits of an MMA operand register are the
+//                  top bits of its bytes, and of two f16 pairs)
+//     [1536,1664)  scales: row r at 1536 + 8 r, byte s = 2 * scale + 1 of sub-block s
+//     [1664,1696)  d[16] f16
 //   IQ4_XS (block: d f16 | scales_h u16 | scales_l[4] | qs[128], src/quants.h:107-113)
 //     [   0, 128)  headers: for g: 8 B of row g then 8 B of row g+8, each the raw first
 //                  8 bytes of the block (d, scales_h, scales_l)
-//     [ 128,2176)  quants: chunk c (0..3), lane -> 16 B at 128 + (c*32 + lane)*16;
-//                  c = 2*h + q: row g + 8h, sub-blocks 4q..4q+3, for each the raw qs word t
-//                  (bytes 4t..4t+3 of the sub-block's 16: low nibbles are elements
-//                  4t..4t+3, high nibbles elements 16+4t..16+4t+3)
+//     [ 128,2176)  quants: column half q (sub-blocks 4q .. 4q+3), row r at 128 + 1024 q + 64 r, piece t: one word
+//                  per sub-block with the codes of elements 8t .. 8t+7: byte 0 = (e0 low, e2 high nibble), byte 1 = (e1, e3),
+//                  byte 2 = (e4, e6), byte 3 = (e5, e7)
 //   Q6_K (block: ql[128] | qh[64] | scales[16] int8 | d f16, src/quants.h:98-103).  A 128-column
 //   half hf of a block packs element l + 32*qd (l < 32, qd < 4) as nibble (qd >> 1) of
 //   ql[64*hf + 32*(qd & 1) + l] and bit pair qd of qh[32*hf + l]; its scale is scales[8*hf + 2*qd + l/16].
 //   Word m (0..7) of a 32-byte run holds l = 4m..4m+3.  Lane (g,t) multiplies, for every (hf, qd),
 //   the elements l = 4t..4t+3 (16-column group 2*(4*hf+qd)) and l = 16+4t..16+4t+3 (the group after it):
 //     [   0, 256)  scales: row r at 16*r, the eight even groups 0,2,..,14 then the eight odd ones
-//     [ 256,3328)  quants: chunk c (0..5), lane -> 16 B at 256 + (c*32 + lane)*16; c = 3*h + k, row g + 8h:
+//     [ 256,3328)  quants: k (0..2), row r at 256 + 1024 k + 64 r, piece t:
 //                  k = 0, 1: half hf = k: ql words t and 4+t of the first 32-byte run, then of the second
 //                  k = 2:    qh words t and 4+t of half 0, then of half 1
 //     [3328,3360)  d[16] f16
@@ -60,7 +62,7 @@
 
 namespace qkm {
 
-static constexpr int kTileIq3 = 1568;
+static constexpr int kTileIq3 = 1696;
 static constexpr int kTileIq4 = 2176;
 static constexpr int kTileQ6 = 3360;
 static constexpr int kTileQ8 = 4352;
@@ -74,6 +76,13 @@ __host__ __device__ inline int tile_bytes(uint32_t type) {
         default: return 0;
     }
 }
+
+// bytes of n_mats matrices [rows][K] in tile order
+__host__ __device__ inline size_t tiled_bytes(uint32_t type, size_t n_mats, uint32_t rows, uint32_t K) {
+    return n_mats * (rows / 16) * (K / 256) * (size_t)tile_bytes(type);
+}
+// position of piece t of row r inside the row's 64-byte run
+__host__ __device__ inline uint32_t piece_at(uint32_t r, uint32_t t) { return (t ^ ((r >> 1) & 3u)) * 16u; }
 
 // digit planes of one activation row set: planes[(row * 4 + digit) * K + k], scale[row]
 struct DigitRows {

@@ -1,0 +1,906 @@
+// Quantised-weight GEMMs of batched prefill on the 5th-generation tensor cores (tcgen05 + TMEM): the experts'
+// gate/up + SwiGLU, the experts' down projections and the dense projections, one persistent kernel for all formats.
+//
+// Replaces moe_gateup_iq3_grouped_coopmat.comp / moe_gateup_q8_coopmat.comp, moe_down_{iq4,q6k}_grouped_coopmat.comp /
+// moe_down_q8_coopmat.comp and the batched projections gemm_q8_0*.comp / gemm_iq4_xs.comp.
+//
+// A unit of work is 256 weight rows (gate and up rows of one 128-row tile, or two consecutive row tiles of a down or
+// dense matrix) times up to 128 activation rows.  Weights are the M = 128 operand and live in tensor memory: a
+// producer thread owns one weight row, reads its quant bytes from shared memory, expands them to f16 and stores
+// them with tcgen05.st; activation rows (f16, scaled per row by a power of two) are the N operand in shared memory.
+//
+// Who does what (24 warps, one block per SM; a ticket hands out units, each role walks them on its own):
+//   16 producer warps  row = lane of the four quarters x matrix x column-block parity.  The two parities work on
+//                      different 256-column blocks (the k-steps of a block pair are interleaved, the order of a sum
+//                      is free), so one half's look-up latency hides behind the other's
+//   4 epilogue warps   TMEM -> SwiGLU / routing weight -> global; two accumulator sets while N <= 64, so the next
+//                      unit's MMAs run meanwhile
+//   1 MMA warp         tcgen05.mma kind::f16, A from TMEM, B from shared memory, commits free the stages
+//   1 weight loader    takes the tickets; one bulk copy per matrix and 256-column block (eight consecutive 16-row tiles)
+//   2 row loaders      activation rows into 128-byte swizzled tiles.  Scattered rows (gate/up) with 16-byte cp.async:
+//                      TMA's tile::gather4 took about 60 cycles per four rows of 128 bytes and was the bound from
+//                      64 rows on (588 us against 250 at 4096 tokens); consecutive rows (down, dense) by TMA boxes of 16 rows
+//
+// What bounds it: few rows per expert: the producers' instructions (nominally 1.5 to 3.3 per weight by format, 3.5 with
+// barriers, address and scale work; issue slots 58 % busy at 77 tokens).  Measured per layer (256 experts, top 8), before
+// (operands dequantised into shared memory or, for one format each, into TMEM by threads that also copied the rows) and now:
+//   gate/up IQ3_XXS   77 tokens 167 -> 107 us, 600: 176 -> 124, 4096: 301 -> 295 (the shared expert's units included now)
+//   gate/up IQ4_XS    77: 340 -> 111, 600: 371 -> 127, 4096: 631 -> 301
+//   down IQ4_XS       77: 133 -> 49,  600: 153 -> 59,  4096: 287 -> 178;   down Q6_K 77: 257 -> 64, 600: 273 -> 74, 4096: 479 -> 195
+//   shared expert     82 us beside the routed kernels -> a share of the above
+//   dense 1000 x 4096 x 2048, Q8_0 and IQ4_XS: 103 -> 41 us each
+//
+// K order.  Inside every group of four columns the operands hold elements (0, 2, 1, 3): that is the order in which
+// the bytes and nibbles of the tiles unpack to f16 pairs without a permute.  x and h rows are written in that order.
+#include <cuda.h>
+#include <cuda_fp16.h>
+
+#include "qkm_common.cuh"
+#include "qkm_kernels.h"
+#include "qkm_stream.cuh"
+#include "qkm_tiles.cuh"
+#include "qkm_umma.cuh"
+
+namespace qkm {
+
+namespace wg {
+constexpr int kProducerWarps = 16, kEpilogueWarps = 4;
+constexpr int kMmaWarp = kProducerWarps + kEpilogueWarps, kWeightWarp = kMmaWarp + 1, kRowWarp = kMmaWarp + 2;
+constexpr int kThreads = (kRowWarp + 2) * 32;   // 768
+constexpr int kFeed = 4;                        // units handed out ahead
+constexpr int kStages = 4;                      // of (A: 64 TMEM columns, B: 128 rows x 64 f16)
+constexpr int kNT = 128;                        // activation rows per unit
+constexpr uint32_t kBTile = 128 * 128;
+constexpr uint32_t kTab = 0x10000u, kTabBytes = 0x10000u, kLow = 0x1000u;
+template <int FMT> constexpr bool has_table() { return FMT == QKM_TYPE_IQ3_XXS || FMT == QKM_TYPE_IQ4_XS; }
+// Shared-window addresses.  With a table image (look-up addresses are byte permutes, so it has to start on a 64 KB
+// boundary): three B stages below it, the fourth and the weight buffers above; else everything in one run.
+template <int FMT> __device__ __forceinline__ uint32_t b_addr(uint32_t s) {
+    return has_table<FMT>() && s == 3 ? kTab + kTabBytes : kLow + s * kBTile;
+}
+template <int FMT> constexpr uint32_t w_base() { return has_table<FMT>() ? kTab + kTabBytes + kBTile : kLow + kStages * kBTile; }
+template <int FMT> constexpr uint32_t tile_size() {
+    return FMT == QKM_TYPE_IQ3_XXS ? kTileIq3 : FMT == QKM_TYPE_IQ4_XS ? kTileIq4 : FMT == QKM_TYPE_Q6_K ? kTileQ6 : kTileQ8;
+}
+// one weight buffer: 16 tiles of 256 columns (Q8_0: 128 columns, and so the shared expert's, which share the kernel)
+template <int FMT> constexpr uint32_t w_bytes() {
+    return FMT == QKM_TYPE_Q8_0 ? 16u * kTileQ8 / 2 : (16u * tile_size<FMT>() > 16u * kTileQ8 / 2 ? 16u * tile_size<FMT>() : 16u * kTileQ8 / 2);
+}
+template <int FMT> constexpr uint32_t smem_end() { return w_base<FMT>() + 2 * w_bytes<FMT>(); }
+constexpr uint32_t kTmemA = 256;                // accumulators in columns [0,256), A stages behind them
+enum Mode { kGateUp = 0, kDown = 1, kDense = 2 };
+}  // namespace wg
+
+// ---- table image: row i (256 bytes) = IQ3_XXS grid entry i as f16 in element order (0, 2, 1, 3), 8 bytes for each of
+// 16 lane columns; then the IQ4_XS pair (kvalues[i & 15], kvalues[i >> 4]) as f16, 4 bytes for each of 32 lanes.  A
+// look-up of a warp never conflicts.
+size_t wgemm_table_bytes() { return wg::kTabBytes; }
+__global__ void wgemm_table_kernel(uint8_t* __restrict__ out) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;   // one 4-byte word each
+    if (i >= wg::kTabBytes / 4) return;
+    const uint32_t row = i >> 6, w = i & 63u;
+    __half2 m;
+    if (w < 32) {
+        const uint32_t g = c_iq3_grid[row] >> (8 * (w & 1u));   // elements (0, 2) or (1, 3)
+        m = __floats2half2_rn((float)(g & 0xFFu), (float)((g >> 16) & 0xFFu));
+    } else {
+        m = __floats2half2_rn((float)c_iq4_values[row & 15u], (float)c_iq4_values[row >> 4]);
+    }
+    reinterpret_cast<__half2*>(out)[i] = m;
+}
+cudaError_t launch_wgemm_table(const Launch& L, uint8_t* out) {
+    wgemm_table_kernel<<<wg::kTabBytes / 4 / 256, 256, 0, L.stream>>>(out);
+    L.count();
+    return cudaGetLastError();
+}
+
+// ---- small helpers ---------------------------------------------------------------------------------------
+__device__ __forceinline__ uint32_t prmt_wg(uint32_t a, uint32_t b, uint32_t sel) {
+    uint32_t r;
+    asm("prmt.b32 %0, %1, %2, %3;" : "=r"(r) : "r"(a), "r"(b), "r"(sel));
+    return r;
+}
+__device__ __forceinline__ uint32_t lds_u16_wg(uint32_t addr) {
+    uint32_t v;
+    asm volatile("ld.shared.u16 %0, [%1];" : "=r"(v) : "r"(addr));
+    return v;
+}
+__device__ __forceinline__ uint32_t mul_h2(uint32_t a, __half2 s) {
+    const __half2 v = __hmul2(*reinterpret_cast<const __half2*>(&a), s);
+    return *reinterpret_cast<const uint32_t*>(&v);
+}
+// value * (hi + lo) with one rounding to f16 that counts (value an integer below 2^8, lo = scale - hi)
+struct Scale2 { __half2 hi, lo; };
+__device__ __forceinline__ Scale2 split_scale(float s) {
+    Scale2 r;
+    const __half h = __float2half_rn(s);
+    r.hi = __half2half2(h);
+    r.lo = __half2half2(__float2half_rn(s - __half2float(h)));
+    return r;
+}
+__device__ __forceinline__ uint32_t mul_h2(uint32_t a, const Scale2& s) {
+    const __half2 v = *reinterpret_cast<const __half2*>(&a);
+    const __half2 r = __hfma2(v, s.hi, __hmul2(v, s.lo));
+    return *reinterpret_cast<const uint32_t*>(&r);
+}
+__device__ __forceinline__ uint32_t sub_h2(uint32_t a, __half2 b) {
+    const __half2 v = __hsub2(*reinterpret_cast<const __half2*>(&a), b);
+    return *reinterpret_cast<const uint32_t*>(&v);
+}
+// 32 lanes x 8 consecutive 32-bit columns of tensor memory: thread i of the warp writes lane (base lane + i)
+__device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t (&v)[8]) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"r"(taddr), "r"(v[0]), "r"(v[1]),
+                 "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7])
+                 : "memory");
+}
+__device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+// D[tmem] (+)= A[tmem] * B[smem]: A is 128 lanes (rows) x 8 columns (16 f16), B a K-major shared-memory tile
+__device__ __forceinline__ void mma_f16_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc, bool accumulate) {
+    const uint32_t acc = accumulate ? 1u : 0u;
+    asm volatile(
+        "{\n"
+        ".reg .pred p;\n"
+        "setp.ne.b32 p, %4, 0;\n"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n"
+        "}\n" ::"r"(tmem_d), "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(acc)
+        : "memory");
+}
+// 16 consecutive rows x 64 columns from column x0, row r0 of the tensor map -> 2 KB at dst, swizzled
+__device__ __forceinline__ void tma_rows16(uint32_t dst, const CUtensorMap* map, uint32_t x0, uint32_t r0, uint32_t bar) {
+    asm volatile("cp.async.bulk.tensor.2d.shared::cta.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
+                 ::"r"(dst), "l"(map), "r"(x0), "r"(r0), "r"(bar) : "memory");
+}
+__device__ __forceinline__ void named_sync_wg(uint32_t id, uint32_t n_threads) {
+    asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(n_threads) : "memory");
+}
+
+// ---- producers ---------------------------------------------------------------------------------------------
+// 32 columns (one sub-block) of a thread's row -> 16 tensor-memory columns at `a`.
+
+// IQ3_XXS: ix[t] = the index half-word of group t (in byte 0/1 or 2/3: HI), sg[t] = the sign word that covers the sub-block
+// (bit positions in qkm_tiles.cuh), j = 2 (sub-block & 3).  Per 8 weights two address permutes, two loads, four packed
+// multiplies by the sub-block scale, four shifts and four xor-and (16 instructions).
+template <bool HI>
+__device__ __forceinline__ void put_iq3(uint32_t a, const uint32_t (&ix)[4], const uint32_t (&sg)[4], uint32_t j, __half2 s, uint32_t tab_c) {
+    constexpr uint32_t s0 = HI ? 0x7624u : 0x7604u, s1 = HI ? 0x7634u : 0x7614u;
+#pragma unroll
+    for (int tp = 0; tp < 4; tp += 2) {
+        uint2 m[2][2];
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+            m[u][0] = lds64(prmt_wg(ix[tp + u], tab_c, s0));
+            m[u][1] = lds64(prmt_wg(ix[tp + u], tab_c, s1));
+        }
+        uint32_t o[8];
+#pragma unroll
+        for (int u = 0; u < 2; ++u)
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {   // elements 4h .. 4h+3 of the group
+                const uint32_t w = sg[tp + u], k = j + h;
+                o[4 * u + 2 * h] = mul_h2(m[u][h].x, s) ^ ((w << (8 + k)) & 0x80008000u);
+                o[4 * u + 2 * h + 1] = mul_h2(m[u][h].y, s) ^ ((w << k) & 0x80008000u);
+            }
+        tmem_st8(a + 4 * tp, o);
+    }
+}
+
+// IQ4_XS: w[t] = quant word of group t: four look-ups of value pairs
+template <class S>
+__device__ __forceinline__ void put_iq4(uint32_t a, const uint32_t (&w)[4], const S& s, uint32_t tab_c) {
+#pragma unroll
+    for (int tp = 0; tp < 4; tp += 2) {
+        uint32_t o[8];
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+            o[4 * u + 0] = lds32(prmt_wg(w[tp + u], tab_c, 0x7604u));
+            o[4 * u + 1] = lds32(prmt_wg(w[tp + u], tab_c, 0x7614u));
+            o[4 * u + 2] = lds32(prmt_wg(w[tp + u], tab_c, 0x7624u));
+            o[4 * u + 3] = lds32(prmt_wg(w[tp + u], tab_c, 0x7634u));
+        }
+#pragma unroll
+        for (int i = 0; i < 8; ++i) o[i] = mul_h2(o[i], s);
+        tmem_st8(a + 4 * tp, o);
+    }
+}
+
+// four unsigned bytes v -> f16 pairs (bytes 0, 2) and (1, 3) of 1024 + byte, minus `bias`, times the scale
+__device__ __forceinline__ void bytes_to_h2(uint32_t v, __half2 bias, const Scale2& s, uint32_t& p02, uint32_t& p13) {
+    p02 = mul_h2(sub_h2((v & 0x00FF00FFu) | 0x64006400u, bias), s);
+    p13 = mul_h2(sub_h2(((v >> 8) & 0x00FF00FFu) | 0x64006400u, bias), s);
+}
+
+// Q8_0: q0, q1 = the row's 32 quant bytes of a block (tile order: words t of elements 4t.. and 16 + 4t.. alternate)
+__device__ __forceinline__ void put_q8(uint32_t a, const uint4& q0, const uint4& q1, float d) {
+    const Scale2 s = split_scale(d);
+    const __half2 bias = __float2half2_rn(1152.f);   // 1024 + 128: the bytes have their top bit flipped
+    const uint32_t w[8] = {q0.x, q0.z, q1.x, q1.z, q0.y, q0.w, q1.y, q1.w};   // elements 4m .. 4m+3
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        uint32_t o[8];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) bytes_to_h2(w[4 * h + i] ^ 0x80808080u, bias, s, o[2 * i], o[2 * i + 1]);
+        tmem_st8(a + 8 * h, o);
+    }
+}
+
+// Q6_K: 32 columns: wl / wh [m] = ql / qh words of elements 4m .. 4m+3, NIB: high nibbles, hs = 2 * quarter; scales of the two 16-column groups
+template <bool NIB>
+__device__ __forceinline__ void put_q6(uint32_t a, const uint32_t (&wl)[8], const uint32_t (&wh)[8], uint32_t hs, float s0, float s1) {
+    const __half2 bias = __float2half2_rn(1056.f);   // 1024 + 32
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        const Scale2 s = split_scale(h ? s1 : s0);
+        uint32_t o[8];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const uint32_t lo = (NIB ? wl[4 * h + i] >> 4 : wl[4 * h + i]) & 0x0F0F0F0Fu;
+            const uint32_t hi = (hs >= 4 ? wh[4 * h + i] >> (hs - 4) : wh[4 * h + i] << (4 - hs)) & 0x30303030u;
+            bytes_to_h2(lo | hi, bias, s, o[2 * i], o[2 * i + 1]);
+        }
+        tmem_st8(a + 8 * h, o);
+    }
+}
+
+struct WgemmArgs {
+    const uint8_t* w[2];        // routed (or dense) tiles: gate and up, or the one matrix twice
+    const uint8_t* sh[2];       // the shared expert's Q8_0 tiles, likewise
+    const MmaItem* items;       // expert kSharedItem: the shared expert; rt counts 128-row tiles (gate/up) or pairs of them
+    const uint32_t* n_items;    // device word; unused by the dense form
+    uint32_t* ticket;           // device word, zero before; NULL: units in a fixed stride
+    const __half* xrows;        // gate/up: activation rows [token][K]
+    const uint32_t* pairs;      // (token << 4) | slot in grouped order; unused by the dense form
+    const float* x_inv_scale;   // gate/up: per token; dense: per row
+    const float* x_norm;        // gate/up: 2-norm of the token's row
+    const float* w_norm;        // gate/up: [2][experts + 1] largest row norm of an expert's gate / up matrix, the shared expert last
+    __half* h;                  // gate/up out: [pair position][rows] f16, scaled per pair
+    float* h_inv_scale;         // gate/up out, down in: per pair position
+    const qkm_sel* sel;         // down: routing weights
+    float* out;                 // down: contributions [pair position][rows]; dense: y [n][rows]
+    const uint8_t* table;
+    uint32_t* status;
+    uint32_t rows, K;           // weight rows of a matrix, columns
+    uint32_t n_experts, n_used; // resident experts
+    uint32_t n_dense;           // dense: activation rows
+};
+
+template <int FMT, int MODE>
+__global__ void __launch_bounds__(wg::kThreads, 1)
+wgemm_kernel(const WgemmArgs a, const __grid_constant__ CUtensorMap rows_map) {
+    extern __shared__ __align__(1024) uint8_t smem_dyn[];
+    constexpr int kSt = wg::kStages;
+    __shared__ __align__(8) unsigned long long s_bar[2 * kSt + 13 + 2 * wg::kFeed];
+    __shared__ MmaItem s_feed[wg::kFeed];
+    __shared__ uint32_t s_tmem;
+    __shared__ float s_col[2][2][wg::kNT];   // epilogue, per unit parity: factors of the unit's columns
+    const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31u;
+    const uint32_t KB = a.K / 256, RT16 = a.rows / 16;
+    const uint32_t row_units = MODE == wg::kGateUp ? a.rows / 128 : (a.rows / 128 + 1) / 2;
+    const uint32_t n_units = MODE == wg::kDense ? (a.n_dense + wg::kNT - 1) / wg::kNT * row_units : *a.n_items;
+    if (blockIdx.x >= n_units) return;
+    {   // the fixed addresses must lie inside the dynamic area
+        const uint32_t dyn_base = smem_addr(smem_dyn);
+        uint32_t dyn_size;
+        asm("mov.u32 %0, %%dynamic_smem_size;" : "=r"(dyn_size));
+        if (dyn_base > wg::kLow || dyn_base + dyn_size < wg::smem_end<FMT>()) {
+            if (tid == 0) atomicExch(a.status, (uint32_t)kStatusBadLayout);
+            return;
+        }
+    }
+    const uint32_t bar = smem_addr(&s_bar[0]);
+    const uint32_t bar_full = bar, bar_empty = bar + 8 * kSt, bar_wfull = bar + 16 * kSt, bar_wempty = bar_wfull + 32;   // [parity][slot]
+    const uint32_t bar_accfull = bar_wempty + 32, bar_accfree = bar_accfull + 16, bar_tab = bar_accfree + 16;
+    const uint32_t bar_ufull = bar_tab + 8, bar_uempty = bar_ufull + 8 * wg::kFeed;
+    constexpr uint32_t kRowArrivals = MODE == wg::kGateUp ? 2 : 1;
+    if (tid == 0) {
+        for (int s = 0; s < kSt; ++s) { mbar_init(bar_full + 8 * s, 8 + kRowArrivals); mbar_init(bar_empty + 8 * s, 1); }   // eight producer warps + the row loaders; one commit
+        for (int b = 0; b < 4; ++b) { mbar_init(bar_wfull + 8 * b, 1); mbar_init(bar_wempty + 8 * b, 8); }
+        for (int b = 0; b < wg::kFeed; ++b) { mbar_init(bar_ufull + 8 * b, 1); mbar_init(bar_uempty + 8 * b, wg::kProducerWarps + wg::kEpilogueWarps + 1 + kRowArrivals); }
+        for (int b = 0; b < 2; ++b) {
+            mbar_init(bar_accfull + 8 * b, 1); mbar_init(bar_accfree + 8 * b, wg::kEpilogueWarps);
+        }
+        mbar_init(bar_tab, 1);
+        mbar_fence_init();
+    }
+    if (warp == 0) { umma::tmem_alloc(smem_addr(&s_tmem), 512); umma::tmem_relinquish(); }
+    umma::fence_before_sync();
+    __syncthreads();
+    umma::fence_after_sync();
+    const uint32_t tmem = s_tmem;
+    bool timed_out = false;
+    auto wait_bar = [&](uint32_t b, uint32_t parity) -> bool { return timed_out || mbar_wait_timed(b, parity); };   // a thread waits out the limit once at most
+
+
+    auto unit_item = [&](uint32_t u) -> MmaItem {
+        if (MODE != wg::kDense) return a.items[u];
+        MmaItem it;
+        it.expert = 0;
+        it.rt = (uint16_t)(u % row_units);
+        it.pair_off = (u / row_units) * wg::kNT;
+        it.n = min((uint32_t)wg::kNT, a.n_dense - it.pair_off);
+        return it;
+    };
+    // the k-th unit of this block, from the weight loader; false after the last
+    auto next_unit = [&](uint32_t k, MmaItem& it) -> bool {
+        const uint32_t s = k % wg::kFeed;
+        timed_out = __any_sync(0xFFFFFFFFu, !wait_bar(bar_ufull + 8 * s, (k / wg::kFeed) & 1u));   // the same for the whole warp
+        if (timed_out) return false;
+        it = s_feed[s];
+        __syncwarp();
+        if (lane == 0) mbar_arrive(bar_uempty + 8 * s);
+        return it.n != 0;
+    };
+    // k-step i of a unit: 256-column block and 64-column quarter.  Blocks 2p and 2p + 1 are interleaved (see above).
+    auto step_kb = [&](uint32_t i) -> uint32_t { return i < (KB & ~1u) * 4 ? 2 * (i >> 3) + (i & 1u) : KB - 1; };
+    auto step_q = [&](uint32_t i) -> uint32_t { return i < (KB & ~1u) * 4 ? (i >> 1) & 3u : i & 3u; };
+    const uint32_t KS = KB * 4;
+
+    if (warp < (uint32_t)wg::kProducerWarps) {
+        // ---- producers
+        const uint32_t lq = warp & 3u, mat = (warp >> 2) & 1u, par = warp >> 3;
+        const uint32_t r = 32 * lq + lane, r16 = r & 15u, g = r16 & 7u, tl = r >> 4;   // row of the 128, row of its tile, tile
+        const uint32_t a_lane = tmem + ((32 * lq) << 16) + wg::kTmemA + mat * 32u;
+        const uint32_t wbuf = wg::w_base<FMT>() + par * wg::w_bytes<FMT>();
+        const uint32_t tab_c = wg::kTab + (FMT == QKM_TYPE_IQ3_XXS ? (lane & 15u) * 8u : 128u + lane * 4u);
+        if (FMT == QKM_TYPE_IQ3_XXS || FMT == QKM_TYPE_IQ4_XS)
+            if (!wait_bar(bar_tab, 0)) timed_out = true;
+        uint32_t round0 = 0, wcnt = 0, wcnt1 = 0;   // stage rounds before this unit; weight slots consumed
+        MmaItem it;
+        for (uint32_t k = 0; next_unit(k, it); ++k, round0 += KB) {
+            const bool shared = MODE != wg::kDense && it.expert == kSharedItem;
+            auto open = [&](uint32_t i) -> uint32_t {   // stage of k-step i, free to be written
+                const uint32_t round = round0 + (i >> 2);
+                if (round && !wait_bar(bar_empty + 8 * (i & 3u), (round - 1) & 1u)) timed_out = true;
+                umma::fence_after_sync();
+                return a_lane + (i & 3u) * 64u;
+            };
+            auto close = [&](uint32_t i) {
+                tmem_st_wait();
+                umma::fence_before_sync();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(bar_full + 8 * (i & 3u));
+            };
+            auto w_wait = [&]() {
+                if (!wait_bar(bar_wfull + 16 * par, wcnt & 1u)) timed_out = true;
+                ++wcnt;
+            };
+            auto w_free = [&]() {
+                __syncwarp();
+                if (lane == 0) mbar_arrive(bar_wempty + 16 * par);
+            };
+            for (uint32_t kb = par; kb < KB; kb += 2) {
+                const uint32_t i0 = kb < (KB & ~1u) ? (kb >> 1) * 8 + par : kb * 4, istep = kb < (KB & ~1u) ? 2u : 1u;   // its k-steps: i0 + q * istep
+                if (FMT == QKM_TYPE_Q8_0 || shared) {
+                    // 64 columns a slot, two slots: two 544-byte pieces of each tile
+#pragma unroll 1
+                    for (uint32_t q = 0; q < 4; ++q) {
+                        const uint32_t slot = q & 1u, cnt = slot ? wcnt1++ : wcnt++;
+                        if (!wait_bar(bar_wfull + 16 * par + 8 * slot, cnt & 1u)) timed_out = true;
+                        const uint32_t t0 = wbuf + slot * (16u * 1088u) + (mat * 8 + tl) * 1088u;
+                        uint4 v[2][2];
+                        float d[2];
+#pragma unroll
+                        for (int s = 0; s < 2; ++s) {
+                            const uint32_t p = t0 + s * 544u;
+                            v[s][0] = lds128(p + 32 + ((r16 >> 3) * 32 + 4 * g) * 8);
+                            v[s][1] = lds128(p + 48 + ((r16 >> 3) * 32 + 4 * g) * 8);
+                            d[s] = f16_bits_to_f32(lds_u16_wg(p + 2 * r16));
+                        }
+                        __syncwarp();
+                        if (lane == 0) mbar_arrive(bar_wempty + 16 * par + 8 * slot);
+                        const uint32_t i = i0 + q * istep, st = open(i);
+                        put_q8(st, v[0][0], v[0][1], d[0]);
+                        put_q8(st + 16, v[1][0], v[1][1], d[1]);
+                        close(i);
+                    }
+                    continue;
+                }
+                if constexpr (FMT != QKM_TYPE_Q8_0) {
+                w_wait();
+                const uint32_t tb = wbuf + (mat * 8 + tl) * wg::tile_size<FMT>();
+                if constexpr (FMT == QKM_TYPE_IQ3_XXS) {
+                    uint4 ix[4];
+#pragma unroll
+                    for (int t = 0; t < 4; ++t) ix[t] = lds128(tb + 64 * r16 + piece_at(r16, t));
+                    uint32_t sg[2][4];   // [word q][t]
+#pragma unroll
+                    for (int tp = 0; tp < 2; ++tp) {
+                        const uint4 v = lds128(tb + 1024 + 32 * r16 + 16 * (tp ^ ((r16 >> 2) & 1u)));
+                        sg[0][2 * tp] = v.x; sg[1][2 * tp] = v.y; sg[0][2 * tp + 1] = v.z; sg[1][2 * tp + 1] = v.w;
+                    }
+                    const uint2 sc = lds64(tb + 1536 + 8 * r16);
+                    const float d4 = f16_bits_to_f32(lds_u16_wg(tb + 1664 + 2 * r16)) * 0.25f;
+                    w_free();
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) {   // sub-blocks 2q, 2q + 1: scale d (2s + 1) / 4, exact in f32, one rounding to f16
+                        const uint32_t i = i0 + q * istep, st = open(i);
+                        const uint32_t w4 = q < 2 ? sc.x : sc.y, sh = 16 * (q & 1);
+                        const __half2 s0 = __float2half2_rn(d4 * (float)((w4 >> sh) & 255u)), s1 = __float2half2_rn(d4 * (float)((w4 >> (sh + 8)) & 255u));
+                        const uint32_t w[4] = {q == 0 ? ix[0].x : q == 1 ? ix[0].y : q == 2 ? ix[0].z : ix[0].w, q == 0 ? ix[1].x : q == 1 ? ix[1].y : q == 2 ? ix[1].z : ix[1].w,
+                                               q == 0 ? ix[2].x : q == 1 ? ix[2].y : q == 2 ? ix[2].z : ix[2].w, q == 0 ? ix[3].x : q == 1 ? ix[3].y : q == 2 ? ix[3].z : ix[3].w};
+                        put_iq3<false>(st, w, sg[q >> 1], 4 * (q & 1), s0, tab_c);
+                        put_iq3<true>(st + 16, w, sg[q >> 1], 4 * (q & 1) + 2, s1, tab_c);
+                        close(i);
+                    }
+                } else if constexpr (FMT == QKM_TYPE_IQ4_XS) {
+                    const uint2 hd = lds64(tb + 16 * g + 8 * (r16 >> 3));   // d | scales_h << 16, scales_l
+                    const float d = f16_bits_to_f32(hd.x & 0xFFFFu);
+#pragma unroll
+                    for (int hf = 0; hf < 2; ++hf) {
+                        uint4 v[4];
+#pragma unroll
+                        for (int t = 0; t < 4; ++t) v[t] = lds128(tb + 128 + 1024 * hf + 64 * r16 + piece_at(r16, t));
+                        if (hf) w_free();
+#pragma unroll
+                        for (int q = 0; q < 2; ++q) {
+                            const uint32_t i = i0 + (2 * hf + q) * istep, st = open(i);
+#pragma unroll
+                            for (int s = 0; s < 2; ++s) {
+                                const int sb = 4 * hf + 2 * q + s;
+                                const int ls = (int)(((hd.y >> (4 * sb)) & 15u) | (((hd.x >> (16 + 2 * sb)) & 3u) << 4)) - 32;
+                                const float dl = d * (float)ls;
+                                const int c = 2 * q + s;
+                                const uint32_t w[4] = {c == 0 ? v[0].x : c == 1 ? v[0].y : c == 2 ? v[0].z : v[0].w, c == 0 ? v[1].x : c == 1 ? v[1].y : c == 2 ? v[1].z : v[1].w,
+                                                       c == 0 ? v[2].x : c == 1 ? v[2].y : c == 2 ? v[2].z : v[2].w, c == 0 ? v[3].x : c == 1 ? v[3].y : c == 2 ? v[3].z : v[3].w};
+                                if (MODE == wg::kDown) put_iq4(st + 16 * s, w, __float2half2_rn(dl), tab_c);   // two roundings of 2^-12
+                                else put_iq4(st + 16 * s, w, split_scale(dl), tab_c);
+                            }
+                            close(i);
+                        }
+                    }
+                } else {   // Q6_K: k-step q = half q / 2, quarters 2 (q & 1) and the one after it: nibble q & 1 of both 32-byte runs
+                    uint4 hq[4];
+#pragma unroll
+                    for (int t = 0; t < 4; ++t) hq[t] = lds128(tb + 2304 + 64 * r16 + piece_at(r16, t));
+                    const uint4 sc = lds128(tb + 16 * r16);   // eight even groups, eight odd groups
+                    const float d = f16_bits_to_f32(lds_u16_wg(tb + 3328 + 2 * r16));
+#pragma unroll
+                    for (int hf = 0; hf < 2; ++hf) {
+                        uint4 v[4];
+#pragma unroll
+                        for (int t = 0; t < 4; ++t) v[t] = lds128(tb + 256 + 1024 * hf + 64 * r16 + piece_at(r16, t));
+                        if (hf) w_free();
+                        uint32_t wh[8];
+#pragma unroll
+                        for (int t = 0; t < 4; ++t) { wh[t] = hf ? hq[t].z : hq[t].x; wh[4 + t] = hf ? hq[t].w : hq[t].y; }
+#pragma unroll
+                        for (int q = 0; q < 2; ++q) {
+                            const uint32_t i = i0 + (2 * hf + q) * istep, st = open(i);
+#pragma unroll
+                            for (int s = 0; s < 2; ++s) {
+                                const int qd = 2 * q + s;
+                                uint32_t wl[8];
+#pragma unroll
+                                for (int t = 0; t < 4; ++t) { wl[t] = s ? v[t].z : v[t].x; wl[4 + t] = s ? v[t].w : v[t].y; }
+                                const float f0 = d * (float)(int8_t)((hf ? sc.y : sc.x) >> (8 * qd)), f1 = d * (float)(int8_t)((hf ? sc.w : sc.z) >> (8 * qd));
+                                if (q) put_q6<true>(st + 16 * s, wl, wh, 2 * qd, f0, f1);
+                                else put_q6<false>(st + 16 * s, wl, wh, 2 * qd, f0, f1);
+                            }
+                            close(i);
+                        }
+                    }
+                }
+                }
+            }
+        }
+    } else if (warp < (uint32_t)wg::kMmaWarp) {
+        // ---- epilogue: warp e reads TMEM lanes 32 e .. 32 e + 31
+        const uint32_t e = warp - wg::kProducerWarps, c = tid - wg::kProducerWarps * 32;   // c: the column this thread prepares
+        uint32_t used[2] = {0, 0}, next = 0, iter = 0;
+        MmaItem it;
+        for (; next_unit(iter, it); ++iter) {
+            const uint32_t n = it.n, n_mma = (n + 15u) & ~15u;
+            const bool big = n_mma > 64;
+            float* f0 = s_col[iter & 1u][0];
+            float* f1 = s_col[iter & 1u][1];
+            if (c < n) {
+                const uint32_t p = it.pair_off + c;
+                if (MODE == wg::kGateUp) {
+                    const uint32_t tok = a.pairs[p] >> 4, ex = it.expert == kSharedItem ? a.n_experts : it.expert;
+                    // |h| <= |g| |u| <= (largest gate row norm x |x|) (largest up row norm x |x|): a power of two that keeps every h below
+                    // 2^15 without knowing the row.  Loose by 2^7 to 2^13 as a rule, which f16 affords (2^-14 .. 2^15 at full precision)
+                    const float xn = a.x_norm[tok], bound = (a.w_norm[ex] * xn) * (a.w_norm[a.n_experts + 1 + ex] * xn);
+                    int q = 0;
+                    if (bound > 0.f && bound <= 3.0e38f) { int b; frexpf(bound, &b); q = max(-126, min(126, 14 - b)); }
+                    f0[c] = a.x_inv_scale[tok];
+                    f1[c] = ldexpf(1.0f, q);
+                    if (it.rt == 0) a.h_inv_scale[p] = ldexpf(1.0f, -q);
+                } else if (MODE == wg::kDown) {
+                    const uint32_t pr = a.pairs[p], tok = pr >> 4, slot = pr & 15u;
+                    f0[c] = (slot < a.n_used ? a.sel[tok].w[slot] : a.sel[tok].w_shared) * a.h_inv_scale[p];
+                } else {
+                    f0[c] = a.x_inv_scale[p];
+                }
+            }
+            named_sync_wg(1, wg::kEpilogueWarps * 32);
+            const uint32_t b = big ? 0u : next;
+            if (!wait_bar(bar_accfull + 8 * b, used[b] & 1u)) timed_out = true;
+            if (big) { if (!wait_bar(bar_accfull + 8, used[1] & 1u)) timed_out = true; ++used[0]; ++used[1]; next = 0; }
+            else { ++used[b]; next ^= 1u; }
+            umma::fence_after_sync();
+            const uint32_t t0 = tmem + ((32 * e) << 16) + b * 128u, t1 = t0 + (big ? 128u : 64u);
+            const uint32_t row = 32 * e + lane;
+            for (uint32_t cb = 0; cb < n_mma; cb += 16) {
+                uint32_t v0[16], v1[16];
+                umma::tmem_ld16(t0 + cb, v0);
+                umma::tmem_ld16(t1 + cb, v1);
+                umma::tmem_ld_wait();
+                if (MODE == wg::kGateUp) {
+                    // silu with the fast exponential and division: their error (a few ulp) is far below the operands' f16 rounding
+                    const uint32_t ff = it.rt * 128u + (row & ~3u) + ((row & 1u) << 1) + ((row >> 1) & 1u);   // element order 0, 2, 1, 3
+                    __half* hp = a.h + (size_t)(it.pair_off + cb) * a.rows + ff;
+#pragma unroll
+                    for (int i = 0; i < 16; ++i)
+                        if (cb + i < n) {
+                            const float us = f0[cb + i], gv = __uint_as_float(v0[i]) * us, uv = __uint_as_float(v1[i]) * us;
+                            hp[(size_t)i * a.rows] = __float2half_rn(__fdividef(gv, 1.0f + __expf(-gv)) * uv * f1[cb + i]);
+                        }
+                } else {
+                    const uint32_t o0 = it.rt * 256u + row;
+                    float* op = a.out + (size_t)(it.pair_off + cb) * a.rows + o0;
+                    const bool second = o0 + 128 < a.rows;   // a dense matrix may end with a lone row tile
+#pragma unroll
+                    for (int i = 0; i < 16; ++i)
+                        if (cb + i < n) {
+                            op[(size_t)i * a.rows] = f0[cb + i] * __uint_as_float(v0[i]);
+                            if (second) op[(size_t)i * a.rows + 128] = f0[cb + i] * __uint_as_float(v1[i]);
+                        }
+                }
+            }
+            umma::fence_before_sync();
+            __syncwarp();
+            if (lane == 0) { mbar_arrive(bar_accfree + 8 * b); if (big) mbar_arrive(bar_accfree + 8); }
+        }
+    } else if (warp == (uint32_t)wg::kMmaWarp) {
+        // ---- MMA issue: the whole warp walks the loop, one elected lane issues
+        const bool leader = umma::elect_one();
+        uint32_t used[2] = {0, 0}, next = 0, round0 = 0;
+        MmaItem it;
+        for (uint32_t k = 0; next_unit(k, it); ++k, round0 += KB) {
+            const uint32_t n_mma = (it.n + 15u) & ~15u;
+            const bool big = n_mma > 64;
+            const uint32_t b = big ? 0u : next, idesc = umma::instr_desc_f16(n_mma);
+            // the accumulators' previous contents have been read
+            if (used[b] && !wait_bar(bar_accfree + 8 * b, (used[b] - 1) & 1u)) timed_out = true;
+            if (big && used[1] && !wait_bar(bar_accfree + 8, (used[1] - 1) & 1u)) timed_out = true;
+            if (big) { ++used[0]; ++used[1]; next = 0; } else { ++used[b]; next ^= 1u; }
+            umma::fence_after_sync();
+            const uint32_t t0 = tmem + b * 128u, t1 = t0 + (big ? 128u : 64u);
+            for (uint32_t i = 0; i < KS; ++i) {
+                const uint32_t stage = i & 3u;
+                if (!wait_bar(bar_full + 8 * stage, (round0 + (i >> 2)) & 1u)) timed_out = true;
+                umma::fence_after_sync();
+                const uint64_t d_b = umma::smem_desc(wg::b_addr<FMT>(stage));
+                const uint32_t t_a = tmem + wg::kTmemA + stage * 64u;
+                if (leader) {
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {   // 16 columns of K further: 8 tensor-memory columns, 32 bytes of the row tile
+                        const bool acc = (i | (uint32_t)j) != 0;
+                        mma_f16_ts(t0, t_a + 8 * j, d_b + 2 * j, idesc, acc);
+                        mma_f16_ts(t1, t_a + 32 + 8 * j, d_b + 2 * j, idesc, acc);
+                    }
+                    umma::commit(bar_empty + 8 * stage);
+                    if (i + 1 == KS) { umma::commit(bar_accfull + 8 * b); if (big) umma::commit(bar_accfull + 8); }
+                }
+                __syncwarp();
+            }
+        }
+    } else if (warp == (uint32_t)wg::kWeightWarp) {
+        // ---- units and weights
+        if (wg::has_table<FMT>() && lane == 0) {
+            mbar_expect_tx(bar_tab, wg::kTabBytes);
+            for (uint32_t i = 0; i < 4; ++i) bulk_g2s(wg::kTab + i * 16384u, a.table + i * 16384u, 16384u, bar_tab);
+        }
+        uint32_t cnt[2][2] = {{0, 0}, {0, 0}};   // uses of (parity, slot)
+        auto drained = [&](uint32_t par, uint32_t slot) {
+            if (cnt[par][slot] && !wait_bar(bar_wempty + 16 * par + 8 * slot, (cnt[par][slot] - 1) & 1u)) timed_out = true;
+        };
+        uint32_t u = blockIdx.x;
+        for (uint32_t k = 0;; ++k) {
+            MmaItem it{0, 0, 0, 0};
+            timed_out = __any_sync(0xFFFFFFFFu, timed_out);
+            if (u < n_units && !timed_out) it = unit_item(u);
+            const uint32_t s = k % wg::kFeed;
+            if (k >= (uint32_t)wg::kFeed && !wait_bar(bar_uempty + 8 * s, (k / wg::kFeed - 1) & 1u)) timed_out = true;
+            if (lane == 0) {
+                s_feed[s] = it;
+                mbar_arrive(bar_ufull + 8 * s);
+            }
+            if (it.n == 0) break;
+            uint32_t ticket = 0;
+            if (lane == 0) ticket = a.ticket ? gridDim.x + atomicAdd(a.ticket, 1u) : u + gridDim.x;   // back by the time this unit's copies are issued
+            const bool shared = MODE != wg::kDense && it.expert == kSharedItem, q8 = FMT == QKM_TYPE_Q8_0 || shared;
+            const uint32_t tile = q8 ? (uint32_t)kTileQ8 : wg::tile_size<FMT>();
+            auto tiles_of = [&](uint32_t m) -> const uint8_t* {   // first of the eight tiles of matrix (row tile) m, column block 0
+                const uint32_t rt128 = MODE == wg::kGateUp ? it.rt : min(2u * it.rt + m, a.rows / 128 - 1);
+                return (shared ? a.sh[m] : a.w[m]) + ((size_t)(shared ? 0u : it.expert) * KB * RT16 + rt128 * 8) * tile;
+            };
+            const uint8_t* src = q8 ? tiles_of((lane >> 3) & 1u) + (size_t)(lane & 7u) * kTileQ8 : tiles_of(lane & 1u);   // this lane's share
+            for (uint32_t kp = 0; kp < KB; kp += 2) {
+                const uint32_t np = min(2u, KB - kp);
+                if (q8) {
+                    for (uint32_t q = 0; q < 4; ++q)
+                        for (uint32_t par = 0; par < np; ++par) {
+                            const uint32_t slot = q & 1u, wf = bar_wfull + 16 * par + 8 * slot;
+                            drained(par, slot);
+                            ++cnt[par][slot];
+                            if (lane == 0) mbar_expect_tx(wf, 16u * 1088u);
+                            __syncwarp();
+                            if (lane < 16) bulk_g2s(wg::w_base<FMT>() + par * wg::w_bytes<FMT>() + slot * (16u * 1088u) + lane * 1088u,
+                                                    src + (size_t)(kp + par) * RT16 * kTileQ8 + q * 1088u, 1088u, wf);
+                        }
+                } else {
+                    for (uint32_t par = 0; par < np; ++par) {
+                        const uint32_t wf = bar_wfull + 16 * par;
+                        drained(par, 0);
+                        drained(par, 1);   // a block covers both slots
+                        ++cnt[par][0];
+                        if (lane == 0) mbar_expect_tx(wf, 16 * tile);
+                        __syncwarp();
+                        if (lane < 2) bulk_g2s(wg::w_base<FMT>() + par * wg::w_bytes<FMT>() + lane * 8 * tile, src + (size_t)(kp + par) * RT16 * tile, 8 * tile, wf);
+                    }
+                }
+            }
+            u = __shfl_sync(0xFFFFFFFFu, ticket, 0);
+        }
+    } else if (MODE == wg::kGateUp) {
+        // ---- scattered activation rows: each of two warps copies four rows x 64 columns per instruction, rows 4 (w + 2m) + lane / 8; a step is
+        // announced two steps after its copies were issued.  Past the unit's end: the last row again (nobody reads those columns)
+        const uint32_t w = warp - wg::kRowWarp, rr = lane >> 3, c = lane & 7u;
+        const uint32_t dst0 = (4 * w + rr) * 128u + ((c ^ (4 * w + rr)) << 4);
+        uint32_t gs = 0;
+        auto announce = [&](uint32_t step) {
+            umma::fence_smem_to_async();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(bar_full + 8 * (step & 3u));
+        };
+        MmaItem it;
+        for (uint32_t k = 0; next_unit(k, it); ++k) {
+            const uint32_t groups = ((it.n + 15u) & ~15u) / 8;   // of eight rows
+            const __half* src[16];
+#pragma unroll
+            for (int m = 0; m < 16; ++m)
+                src[m] = (uint32_t)m < groups ? a.xrows + (size_t)(a.pairs[it.pair_off + min(8u * m + 4 * w + rr, it.n - 1)] >> 4) * a.K + 8 * c : a.xrows;
+            for (uint32_t i = 0; i < KS; ++i, ++gs) {
+                if (gs >= 4 && !wait_bar(bar_empty + 8 * (gs & 3u), ((gs >> 2) - 1) & 1u)) timed_out = true;
+                const uint32_t st = wg::b_addr<FMT>(gs & 3u) + dst0, k0 = step_kb(i) * 256u + step_q(i) * 64u;
+#pragma unroll
+                for (int m = 0; m < 16; ++m)
+                    if ((uint32_t)m < groups) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(st + m * 1024u), "l"(src[m] + k0) : "memory");
+                asm volatile("cp.async.commit_group;" ::: "memory");
+                if (gs >= 2) {
+                    asm volatile("cp.async.wait_group 2;" ::: "memory");
+                    announce(gs - 2);
+                }
+            }
+        }
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        if (gs >= 2) announce(gs - 2);
+        if (gs >= 1) announce(gs - 1);
+    } else if (warp == (uint32_t)wg::kRowWarp) {
+        // ---- consecutive activation rows: boxes of 16
+        uint32_t gs = 0;
+        MmaItem it;
+        for (uint32_t k = 0; next_unit(k, it); ++k) {
+            const uint32_t boxes = (it.n + 15u) / 16;
+            for (uint32_t i = 0; i < KS; ++i, ++gs) {
+                const uint32_t stage = gs & 3u;
+                if (gs >= 4 && !wait_bar(bar_empty + 8 * stage, ((gs >> 2) - 1) & 1u)) timed_out = true;
+                if (lane == 0) mbar_expect_tx(bar_full + 8 * stage, boxes * 2048u);
+                __syncwarp();
+                if (lane < boxes) tma_rows16(wg::b_addr<FMT>(stage) + lane * 2048u, &rows_map, step_kb(i) * 256u + step_q(i) * 64u, it.pair_off + 16 * lane, bar_full + 8 * stage);
+            }
+        }
+    }
+    umma::fence_before_sync();
+    const int any_timed_out = __syncthreads_or(timed_out ? 1 : 0);   // any role's wait that ran out counts
+    if (warp == 0) umma::tmem_dealloc(tmem, 512);
+    if (any_timed_out && tid == 0) atomicExch(a.status, (uint32_t)kStatusWaitTimeout);
+}
+
+// ---- activation rows ---------------------------------------------------------------------------------------
+// x -> f16 rows in the kernels' element order, each scaled by a power of two so that max|x| lands in [2^13, 2^14), the
+// inverse scale and (optional) the row's 2-norm.  A warp per row: two passes over it, the second from L1.
+__global__ void __launch_bounds__(256)
+f16_rows_kernel(const float* __restrict__ x, __half* __restrict__ xh, float* __restrict__ inv_scale, float* __restrict__ norm, uint32_t n_rows, uint32_t K) {
+    const uint32_t t = (blockIdx.x * 256u + threadIdx.x) >> 5, lane = threadIdx.x & 31u;
+    if (t >= n_rows) return;
+    const float4* xt = reinterpret_cast<const float4*>(x + (size_t)t * K);
+    float m = 0.f, ss = 0.f;
+#pragma unroll 8
+    for (uint32_t k = lane; k < K / 4; k += 32) {
+        const float4 v = xt[k];
+        m = fmaxf(fmaxf(m, fmaxf(fabsf(v.x), fabsf(v.y))), fmaxf(fabsf(v.z), fabsf(v.w)));
+        ss += v.x * v.x; ss += v.y * v.y; ss += v.z * v.z; ss += v.w * v.w;
+    }
+    m = __uint_as_float(__reduce_max_sync(0xFFFFFFFFu, __float_as_uint(m)));   // non-negative floats order like their bits
+    ss = warp_sum(ss);
+    int p = 0;
+    if (m > 0.f && m <= 3.0e38f) { int e; frexpf(m, &e); p = min(14 - e, 126); }   // m * 2^p in [2^13, 2^14)
+    const float up = ldexpf(1.0f, p);
+    uint2* dst = reinterpret_cast<uint2*>(xh + (size_t)t * K);
+#pragma unroll 8
+    for (uint32_t k = lane; k < K / 4; k += 32) {
+        const float4 v = xt[k];
+        const __half2 a = __floats2half2_rn(v.x * up, v.z * up), b = __floats2half2_rn(v.y * up, v.w * up);
+        dst[k] = make_uint2(*reinterpret_cast<const uint32_t*>(&a), *reinterpret_cast<const uint32_t*>(&b));
+    }
+    if (lane == 0) {
+        inv_scale[t] = ldexpf(1.0f, -p);
+        if (norm) norm[t] = sqrtf(ss);
+    }
+}
+cudaError_t launch_f16_rows(const Launch& L, const float* x, void* xh, float* inv_scale, float* norm, uint32_t n_rows, uint32_t K) {
+    if (n_rows == 0) return cudaSuccess;
+    if (K % 4) return cudaErrorInvalidValue;
+    f16_rows_kernel<<<(n_rows + 7) / 8, 256, 0, L.stream>>>(x, (__half*)xh, inv_scale, norm, n_rows, K);
+    L.count();
+    return cudaGetLastError();
+}
+// rows that arrived as scaled f16 (expert parallel): their 2-norms, and a copy in the kernels' element order
+__global__ void __launch_bounds__(256)
+f16_rows_in_kernel(const __half* __restrict__ in, const float* __restrict__ inv_scale, __half* __restrict__ out, float* __restrict__ norm, uint32_t n_rows, uint32_t K) {
+    const uint32_t t = (blockIdx.x * 256u + threadIdx.x) >> 5, lane = threadIdx.x & 31u;
+    if (t >= n_rows) return;
+    const uint4* xt = reinterpret_cast<const uint4*>(in + (size_t)t * K);
+    uint4* dst = reinterpret_cast<uint4*>(out + (size_t)t * K);
+    float ss = 0.f;
+    for (uint32_t k = lane; k < K / 8; k += 32) {
+        const uint4 v = xt[k];
+        const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&w[i]));
+            ss += f.x * f.x; ss += f.y * f.y;
+        }
+        dst[k] = make_uint4(__byte_perm(v.x, v.y, 0x5410), __byte_perm(v.x, v.y, 0x7632), __byte_perm(v.z, v.w, 0x5410), __byte_perm(v.z, v.w, 0x7632));
+    }
+    ss = warp_sum(ss);
+    if (lane == 0) norm[t] = sqrtf(ss) * inv_scale[t];
+}
+cudaError_t launch_f16_rows_in(const Launch& L, const void* in, const float* inv_scale, void* out, float* norm, uint32_t n_rows, uint32_t K) {
+    if (n_rows == 0) return cudaSuccess;
+    f16_rows_in_kernel<<<(n_rows + 7) / 8, 256, 0, L.stream>>>((const __half*)in, inv_scale, (__half*)out, norm, n_rows, K);
+    L.count();
+    return cudaGetLastError();
+}
+// out[e] = largest row 2-norm of expert e's matrix [rows][K] (raw ggml rows; at upload), rounded up a little.
+// out has to be zero before (the maximum is taken on the bits of non-negative floats).
+// A warp per row, a 32-column sub-block per lane; squares of codebook entries from a table in shared memory.
+template <int TYPE>
+__global__ void __launch_bounds__(256)
+row_norm_max_kernel(const uint8_t* __restrict__ w, float* __restrict__ out, uint32_t rows, uint32_t K) {
+    __shared__ float s_sq[256];   // IQ3_XXS: a grid entry's four magnitudes squared and summed; IQ4_XS: a byte's two values
+    const uint32_t tid = threadIdx.x, lane = tid & 31u, e = blockIdx.y;
+    if (TYPE == QKM_TYPE_IQ3_XXS) {
+        const uint32_t g = c_iq3_grid[tid];
+        s_sq[tid] = (float)__dp4a(g, g, 0u);
+    } else if (TYPE == QKM_TYPE_IQ4_XS) {
+        const float a = (float)c_iq4_values[tid & 15u], b = (float)c_iq4_values[tid >> 4];
+        s_sq[tid] = a * a + b * b;
+    }
+    __syncthreads();
+    const size_t rb = row_bytes(TYPE, K);
+    float best = 0.f;
+    for (uint32_t r = blockIdx.x * 8 + (tid >> 5); r < rows; r += gridDim.x * 8) {
+        const uint8_t* row = w + ((size_t)e * rows + r) * rb;
+        float ss = 0.f;
+        for (uint32_t sb = lane; sb < K / 32; sb += 32) {
+            const uint8_t* b = row + (size_t)(sb >> 3) * Fmt<TYPE>::kBytes;
+            const uint32_t ib = sb & 7u;
+            float sum = 0.f, sc;
+            if (TYPE == QKM_TYPE_IQ3_XXS) {
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const uint32_t q = ld_u16(b + 2 + 8 * ib + 2 * i);
+                    sum += s_sq[q & 255u] + s_sq[q >> 8];
+                }
+                sc = f16_bits_to_f32(ld_u16(b)) * (0.5f + (float)(ld_u32_a2(b + 66 + 4 * ib) >> 28)) * 0.5f;
+            } else if (TYPE == QKM_TYPE_IQ4_XS) {
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const uint32_t q = *reinterpret_cast<const uint32_t*>(b + 8 + 16 * ib + 4 * i);
+                    sum += (s_sq[q & 255u] + s_sq[(q >> 8) & 255u]) + (s_sq[(q >> 16) & 255u] + s_sq[q >> 24]);
+                }
+                const uint32_t ls = (((uint32_t)b[4 + (ib >> 1)] >> (4 * (ib & 1u))) & 15u) | (((ld_u16(b + 2) >> (2 * ib)) & 3u) << 4);
+                sc = f16_bits_to_f32(ld_u16(b)) * (float)((int)ls - 32);
+            } else {   // Q8_0: a block of 34 bytes per sub-block
+                const uint8_t* q8 = row + (size_t)sb * 34;
+                int s = 0;
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    const int q = (int)ld_u32_a2(q8 + 2 + 4 * i);
+                    s = __dp4a(q, q, s);
+                }
+                sum = (float)s;
+                sc = f16_bits_to_f32(ld_u16(q8));
+            }
+            ss += sum * sc * sc;
+        }
+        best = fmaxf(best, warp_sum(ss));
+    }
+    if (lane == 0 && best > 0.f) atomicMax(reinterpret_cast<uint32_t*>(out + e), __float_as_uint(sqrtf(best) * 1.001f));
+}
+cudaError_t launch_row_norm_max(const Launch& L, uint32_t type, const void* w, float* out, uint32_t n_mats, uint32_t rows, uint32_t K) {
+    const dim3 grid((rows + 63) / 64, n_mats);   // eight rows a warp
+    const uint8_t* p = (const uint8_t*)w;
+    switch (type) {
+        case QKM_TYPE_IQ3_XXS: row_norm_max_kernel<QKM_TYPE_IQ3_XXS><<<grid, 256, 0, L.stream>>>(p, out, rows, K); break;
+        case QKM_TYPE_IQ4_XS: row_norm_max_kernel<QKM_TYPE_IQ4_XS><<<grid, 256, 0, L.stream>>>(p, out, rows, K); break;
+        case QKM_TYPE_Q8_0: row_norm_max_kernel<QKM_TYPE_Q8_0><<<grid, 256, 0, L.stream>>>(p, out, rows, K); break;
+        default: return cudaErrorInvalidValue;
+    }
+    L.count();
+    return cudaGetLastError();
+}
+
+// ---- launchers ---------------------------------------------------------------------------------------------
+// tensor map over f16 rows [n_rows][K]: boxes of 16 rows x 64 columns, 128-byte swizzle
+static bool rows_tensor_map(CUtensorMap* map, const void* rows, uint64_t n_rows, uint32_t K) {
+    typedef CUresult (*EncodeFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
+                                 const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
+                                 CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+    static const EncodeFn encode = [] {
+        void* fn = nullptr;
+        cudaDriverEntryPointQueryResult qres;
+        return cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &qres) == cudaSuccess ? (EncodeFn)fn : (EncodeFn) nullptr;
+    }();
+    if (!encode) return false;
+    const cuuint64_t dim[2] = {K, n_rows}, stride[1] = {(cuuint64_t)K * 2};
+    const cuuint32_t box[2] = {64, 16}, estride[2] = {1, 1};
+    return encode(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<void*>(rows), dim, stride, box, estride, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                  CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+template <int FMT, int MODE>
+static cudaError_t wgemm_launch(const Launch& L, const WgemmArgs& a, const void* rows, uint64_t n_rows, uint32_t max_units, uint32_t n_sms) {
+    if (max_units == 0) return cudaSuccess;
+    if (const cudaError_t e = allow_dynamic_smem<wgemm_kernel<FMT, MODE>>((int)wg::smem_end<FMT>())) return e;
+    CUtensorMap map{};
+    if (((uintptr_t)rows & 15u) || (MODE != wg::kGateUp && !rows_tensor_map(&map, rows, n_rows, a.K))) return cudaErrorInvalidValue;
+    wgemm_kernel<FMT, MODE><<<max_units < n_sms ? max_units : n_sms, wg::kThreads, wg::smem_end<FMT>(), L.stream>>>(a, map);
+    L.count();
+    return cudaGetLastError();
+}
+
+uint32_t wgemm_rows_per_unit() { return wg::kNT; }
+
+cudaError_t launch_wgemm_gateup(const Launch& L, const qkm_dims& d, uint32_t type, const WgemmExperts& x, const void* xrows,
+                                const float* x_inv_scale, const float* x_norm, const float* w_norm, void* h, float* h_inv_scale, uint32_t max_units) {
+    WgemmArgs a{};
+    a.w[0] = (const uint8_t*)x.w[0]; a.w[1] = (const uint8_t*)x.w[1]; a.sh[0] = (const uint8_t*)x.sh[0]; a.sh[1] = (const uint8_t*)x.sh[1];
+    a.items = x.items; a.n_items = x.n_items; a.ticket = x.ticket; a.pairs = x.pairs; a.x_inv_scale = x_inv_scale; a.x_norm = x_norm; a.w_norm = w_norm;
+    a.xrows = (const __half*)xrows; a.h = (__half*)h; a.h_inv_scale = h_inv_scale; a.table = x.table; a.status = x.status; a.rows = d.n_ff; a.K = d.n_embd;
+    a.n_experts = x.n_experts; a.n_used = d.n_used;
+    if (type == QKM_TYPE_IQ3_XXS) return wgemm_launch<QKM_TYPE_IQ3_XXS, wg::kGateUp>(L, a, xrows, 0, max_units, x.n_sms);
+    if (type == QKM_TYPE_IQ4_XS) return wgemm_launch<QKM_TYPE_IQ4_XS, wg::kGateUp>(L, a, xrows, 0, max_units, x.n_sms);
+    return cudaErrorInvalidValue;
+}
+
+cudaError_t launch_wgemm_down(const Launch& L, const qkm_dims& d, uint32_t type, const WgemmExperts& x, const void* h, uint64_t n_hrows,
+                              const float* h_inv_scale, const qkm_sel* sel, float* contrib, uint32_t max_units) {
+    if (d.n_embd % 256) return cudaErrorInvalidValue;
+    WgemmArgs a{};
+    a.w[0] = a.w[1] = (const uint8_t*)x.w[0]; a.sh[0] = a.sh[1] = (const uint8_t*)x.sh[0];
+    a.items = x.items; a.n_items = x.n_items; a.ticket = x.ticket; a.pairs = x.pairs; a.h_inv_scale = const_cast<float*>(h_inv_scale); a.sel = sel; a.out = contrib;
+    a.table = x.table; a.status = x.status; a.rows = d.n_embd; a.K = d.n_ff; a.n_experts = x.n_experts; a.n_used = d.n_used;
+    if (type == QKM_TYPE_IQ4_XS) return wgemm_launch<QKM_TYPE_IQ4_XS, wg::kDown>(L, a, h, n_hrows, max_units, x.n_sms);
+    if (type == QKM_TYPE_Q6_K) return wgemm_launch<QKM_TYPE_Q6_K, wg::kDown>(L, a, h, n_hrows, max_units, x.n_sms);
+    return cudaErrorInvalidValue;
+}
+
+// Y[n][M] = X[n][K] . W^T: x rows to scaled f16, then one launch
+cudaError_t launch_dense_gemm(const Launch& L, uint32_t type, const void* tiles, uint32_t M, uint32_t K, const float* x, uint32_t n_rows, float* y,
+                              void* xh, float* x_inv_scale, const uint8_t* table, uint32_t n_sms, uint32_t* status) {
+    if (n_rows == 0) return cudaSuccess;
+    if (M % 128 || K % 256 || M / 128 > 65535) return cudaErrorInvalidValue;
+    if (const cudaError_t e = launch_f16_rows(L, x, xh, x_inv_scale, nullptr, n_rows, K)) return e;
+    WgemmArgs a{};
+    a.w[0] = a.w[1] = (const uint8_t*)tiles;
+    a.x_inv_scale = x_inv_scale; a.out = y; a.table = table; a.status = status; a.rows = M; a.K = K; a.n_dense = n_rows;
+    const uint32_t units = (n_rows + wg::kNT - 1) / wg::kNT * ((M / 128 + 1) / 2);
+    if (type == QKM_TYPE_Q8_0) return wgemm_launch<QKM_TYPE_Q8_0, wg::kDense>(L, a, xh, n_rows, units, n_sms);
+    if (type == QKM_TYPE_IQ4_XS) return wgemm_launch<QKM_TYPE_IQ4_XS, wg::kDense>(L, a, xh, n_rows, units, n_sms);
+    return cudaErrorInvalidValue;
+}
+
+}  // namespace qkm

@@ -33,6 +33,23 @@ def test_dense_gemm(ctx, orc, syn, ttype, M, K, n):
     d_x.free(); d_y.free()
 
 
+@pytest.mark.parametrize("ttype", [8, 23])
+@pytest.mark.parametrize("M,K,n", [(128, 256, 16), (384, 768, 65), (640, 1280, 129), (256, 512, 64), (4480, 256, 257)])
+def test_dense_gemm_edges(ctx, orc, syn, ttype, M, K, n):
+    """An odd number of 256-column blocks, a lone last row tile, row counts around the 64-row change of accumulator
+    sets and the 128-row unit, more units than blocks."""
+    W = syn.random_blocks(ttype, M, K, seed=19, tag="dense")
+    x = syn.random_x(n, K, seed=20)
+    x[n // 2] *= 1e4
+    ctx.dense_upload(4, ttype, W, M, K)
+    d_x, d_y = ctx.to_device(x), ctx.alloc(n * M * 4)
+    ctx.dense_gemm(4, d_x, n, d_y)
+    ctx.sync()
+    want = orc.gemv(ttype, W, x, M, K, threads=orc.hardware_threads())
+    assert syn.rel_err_rows(d_y.download(np.float32, (n, M)), want) < TOL / 4   # f16 operands
+    d_x.free(); d_y.free()
+
+
 def test_dense_rejects(ctx, pkg, syn):
     W = syn.random_blocks(8, 128, 256, seed=1)
     d = ctx.alloc(1 << 16)
