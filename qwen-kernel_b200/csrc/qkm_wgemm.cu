@@ -9,26 +9,26 @@
 // producer thread owns one weight row, reads its quant bytes from shared memory, expands them to f16 and stores
 // them with tcgen05.st; activation rows (f16, scaled per row by a power of two) are the N operand in shared memory.
 //
-// Who does what (24 warps, one block per SM; a ticket hands out units, each role walks them on its own):
+// Who does what (32 warps, one block per SM, registers split between the warpgroups; a ticket hands out units, each role walks them on its own):
 //   16 producer warps  row = lane of the four quarters x matrix x column-block parity.  The two parities work on
 //                      different 256-column blocks (the k-steps of a block pair are interleaved, the order of a sum
 //                      is free), so one half's look-up latency hides behind the other's
-//   4 epilogue warps   TMEM -> SwiGLU / routing weight -> global; two accumulator sets while N <= 64, so the next
+//   8 epilogue warps   TMEM -> SwiGLU / routing weight -> global; two accumulator sets while N <= 64, so the next
 //                      unit's MMAs run meanwhile
 //   1 MMA warp         tcgen05.mma kind::f16, A from TMEM, B from shared memory, commits free the stages
 //   1 weight loader    takes the tickets; one bulk copy per matrix and 256-column block (eight consecutive 16-row tiles)
-//   2 row loaders      activation rows into 128-byte swizzled tiles.  Scattered rows (gate/up) with 16-byte cp.async:
+//   row loaders        activation rows into 128-byte swizzled tiles.  Scattered rows (gate/up) with 16-byte cp.async:
 //                      TMA's tile::gather4 took about 60 cycles per four rows of 128 bytes and was the bound from
 //                      64 rows on (588 us against 250 at 4096 tokens); consecutive rows (down, dense) by TMA boxes of 16 rows
 //
 // What bounds it: few rows per expert: the producers' instructions (nominally 1.5 to 3.3 per weight by format, 3.5 with
 // barriers, address and scale work; issue slots 58 % busy at 77 tokens).  Measured per layer (256 experts, top 8), before
 // (operands dequantised into shared memory or, for one format each, into TMEM by threads that also copied the rows) and now:
-//   gate/up IQ3_XXS   77 tokens 167 -> 107 us, 600: 176 -> 124, 4096: 301 -> 295 (the shared expert's units included now)
-//   gate/up IQ4_XS    77: 340 -> 111, 600: 371 -> 127, 4096: 631 -> 301
-//   down IQ4_XS       77: 133 -> 49,  600: 153 -> 59,  4096: 287 -> 178;   down Q6_K 77: 257 -> 64, 600: 273 -> 74, 4096: 479 -> 195
+//   gate/up IQ3_XXS   77 tokens 167 -> 89 us, 600: 176 -> 103, 4096: 301 -> 247 (the shared expert's units included now)
+//   gate/up IQ4_XS    77: 340 -> 91, 600: 371 -> 112, 4096: 631 -> 248
+//   down IQ4_XS       77: 133 -> 51, 600: 153 -> 61, 4096: 287 -> 155;   down Q6_K 600: 273 -> 82, 4096: 479 -> 170
 //   shared expert     82 us beside the routed kernels -> a share of the above
-//   dense 1000 x 4096 x 2048, Q8_0 and IQ4_XS: 103 -> 41 us each
+//   dense 1000 x 4096 x 2048, Q8_0 and IQ4_XS: 103 -> 37 us each
 //
 // K order.  Inside every group of four columns the operands hold elements (0, 2, 1, 3): that is the order in which
 // the bytes and nibbles of the tiles unpack to f16 pairs without a permute.  x and h rows are written in that order.
@@ -44,14 +44,18 @@
 namespace qkm {
 
 namespace wg {
-constexpr int kProducerWarps = 16, kEpilogueWarps = 4;
+constexpr int kProducerWarps = 16, kEpilogueWarps = 8;
 constexpr int kMmaWarp = kProducerWarps + kEpilogueWarps, kWeightWarp = kMmaWarp + 1, kRowWarp = kMmaWarp + 2;
-constexpr int kThreads = (kRowWarp + 2) * 32;   // 768
+constexpr int kThreads = 1024;                  // eight warpgroups at 64 registers = all 65,536 of the SM
+// registers a thread after the split; 512 x 80 + 256 x 56 + 256 x 40 = 65,536, what the block was launched with
+constexpr int kProducerRegs = 80, kEpilogueRegs = 56, kOtherRegs = 40;
+static_assert(kProducerWarps * 32 * kProducerRegs + kEpilogueWarps * 32 * kEpilogueRegs + (32 - kProducerWarps - kEpilogueWarps) * 32 * kOtherRegs <= kThreads * 64,
+              "the shares must not exceed the launch's registers");
 constexpr int kFeed = 4;                        // units handed out ahead
 constexpr int kStages = 4;                      // of (A: 64 TMEM columns, B: 128 rows x 64 f16)
 constexpr int kNT = 128;                        // activation rows per unit
 constexpr uint32_t kBTile = 128 * 128;
-constexpr uint32_t kTab = 0x10000u, kTabBytes = 0x10000u, kLow = 0x1000u;
+constexpr uint32_t kTab = 0x10000u, kTabBytes = 0x10000u, kLow = 0x1800u;
 template <int FMT> constexpr bool has_table() { return FMT == QKM_TYPE_IQ3_XXS || FMT == QKM_TYPE_IQ4_XS; }
 // Shared-window addresses.  With a table image (look-up addresses are byte permutes, so it has to start on a 64 KB
 // boundary): three B stages below it, the fourth and the weight buffers above; else everything in one run.
@@ -62,13 +66,18 @@ template <int FMT> constexpr uint32_t w_base() { return has_table<FMT>() ? kTab 
 template <int FMT> constexpr uint32_t tile_size() {
     return FMT == QKM_TYPE_IQ3_XXS ? kTileIq3 : FMT == QKM_TYPE_IQ4_XS ? kTileIq4 : FMT == QKM_TYPE_Q6_K ? kTileQ6 : kTileQ8;
 }
-// one weight buffer: 16 tiles of 256 columns (Q8_0: 128 columns, and so the shared expert's, which share the kernel)
+// Weight buffers, one per parity: 16 tiles of 256 columns, or two slots of 64 columns of the shared expert's Q8_0 tiles (those copies
+// are of 1088 bytes and take about 90 cycles each, so the Q8_0 kernels load whole tiles: 41 -> 35 us at 1000 x 4096 x 2048)
+template <int FMT> constexpr uint32_t q8_slots() { return FMT == QKM_TYPE_Q8_0 ? 1 : 2; }
+constexpr uint32_t kQ8Slot = 16 * 1088;
 template <int FMT> constexpr uint32_t w_bytes() {
-    return FMT == QKM_TYPE_Q8_0 ? 16u * kTileQ8 / 2 : (16u * tile_size<FMT>() > 16u * kTileQ8 / 2 ? 16u * tile_size<FMT>() : 16u * kTileQ8 / 2);
+    const uint32_t slots = q8_slots<FMT>() * kQ8Slot, tiles = 16u * tile_size<FMT>();
+    return tiles > slots ? tiles : slots;
 }
 template <int FMT> constexpr uint32_t smem_end() { return w_base<FMT>() + 2 * w_bytes<FMT>(); }
 constexpr uint32_t kTmemA = 256;                // accumulators in columns [0,256), A stages behind them
 enum Mode { kGateUp = 0, kDown = 1, kDense = 2 };
+template <int MODE> constexpr uint32_t row_warps() { return MODE == kGateUp ? kStages : 1; }
 }  // namespace wg
 
 // ---- table image: row i (256 bytes) = IQ3_XXS grid entry i as f16 in element order (0, 2, 1, 3), 8 bytes for each of
@@ -127,10 +136,11 @@ __device__ __forceinline__ uint32_t sub_h2(uint32_t a, __half2 b) {
     const __half2 v = __hsub2(*reinterpret_cast<const __half2*>(&a), b);
     return *reinterpret_cast<const uint32_t*>(&v);
 }
-// 32 lanes x 8 consecutive 32-bit columns of tensor memory: thread i of the warp writes lane (base lane + i)
-__device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t (&v)[8]) {
-    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"r"(taddr), "r"(v[0]), "r"(v[1]),
-                 "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7])
+// 32 lanes x 16 consecutive 32-bit columns of tensor memory: thread i of the warp writes lane (base lane + i)
+__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&v)[16]) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};" ::"r"(taddr), "r"(v[0]), "r"(v[1]),
+                 "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]), "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]),
+                 "r"(v[14]), "r"(v[15])
                  : "memory");
 }
 __device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
@@ -150,57 +160,43 @@ __device__ __forceinline__ void tma_rows16(uint32_t dst, const CUtensorMap* map,
     asm volatile("cp.async.bulk.tensor.2d.shared::cta.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
                  ::"r"(dst), "l"(map), "r"(x0), "r"(r0), "r"(bar) : "memory");
 }
-__device__ __forceinline__ void named_sync_wg(uint32_t id, uint32_t n_threads) {
-    asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(n_threads) : "memory");
-}
 
 // ---- producers ---------------------------------------------------------------------------------------------
-// 32 columns (one sub-block) of a thread's row -> 16 tensor-memory columns at `a`.
+// 32 columns (one sub-block) of a thread's row -> 16 tensor-memory columns.
 
 // IQ3_XXS: ix[t] = the index half-word of group t (in byte 0/1 or 2/3: HI), sg[t] = the sign word that covers the sub-block
 // (bit positions in qkm_tiles.cuh), j = 2 (sub-block & 3).  Per 8 weights two address permutes, two loads, four packed
 // multiplies by the sub-block scale, four shifts and four xor-and (16 instructions).
 template <bool HI>
-__device__ __forceinline__ void put_iq3(uint32_t a, const uint32_t (&ix)[4], const uint32_t (&sg)[4], uint32_t j, __half2 s, uint32_t tab_c) {
+__device__ __forceinline__ void make_iq3(uint32_t (&o)[16], const uint32_t (&ix)[4], const uint32_t (&sg)[4], uint32_t j, __half2 s, uint32_t tab_c) {
     constexpr uint32_t s0 = HI ? 0x7624u : 0x7604u, s1 = HI ? 0x7634u : 0x7614u;
 #pragma unroll
-    for (int tp = 0; tp < 4; tp += 2) {
-        uint2 m[2][2];
-#pragma unroll
-        for (int u = 0; u < 2; ++u) {
-            m[u][0] = lds64(prmt_wg(ix[tp + u], tab_c, s0));
-            m[u][1] = lds64(prmt_wg(ix[tp + u], tab_c, s1));
-        }
-        uint32_t o[8];
-#pragma unroll
-        for (int u = 0; u < 2; ++u)
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {   // elements 4h .. 4h+3 of the group
-                const uint32_t w = sg[tp + u], k = j + h;
-                o[4 * u + 2 * h] = mul_h2(m[u][h].x, s) ^ ((w << (8 + k)) & 0x80008000u);
-                o[4 * u + 2 * h + 1] = mul_h2(m[u][h].y, s) ^ ((w << k) & 0x80008000u);
-            }
-        tmem_st8(a + 4 * tp, o);
+    for (int t = 0; t < 4; ++t) {
+        const uint2 m0 = lds64(prmt_wg(ix[t], tab_c, s0)), m1 = lds64(prmt_wg(ix[t], tab_c, s1));
+        o[4 * t] = m0.x; o[4 * t + 1] = m0.y; o[4 * t + 2] = m1.x; o[4 * t + 3] = m1.y;
     }
+#pragma unroll
+    for (int t = 0; t < 4; ++t)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {   // elements 4h .. 4h+3 of the group
+            const uint32_t w = sg[t], k = j + h;
+            o[4 * t + 2 * h] = mul_h2(o[4 * t + 2 * h], s) ^ ((w << (8 + k)) & 0x80008000u);
+            o[4 * t + 2 * h + 1] = mul_h2(o[4 * t + 2 * h + 1], s) ^ ((w << k) & 0x80008000u);
+        }
 }
 
 // IQ4_XS: w[t] = quant word of group t: four look-ups of value pairs
 template <class S>
-__device__ __forceinline__ void put_iq4(uint32_t a, const uint32_t (&w)[4], const S& s, uint32_t tab_c) {
+__device__ __forceinline__ void make_iq4(uint32_t (&o)[16], const uint32_t (&w)[4], const S& s, uint32_t tab_c) {
 #pragma unroll
-    for (int tp = 0; tp < 4; tp += 2) {
-        uint32_t o[8];
-#pragma unroll
-        for (int u = 0; u < 2; ++u) {
-            o[4 * u + 0] = lds32(prmt_wg(w[tp + u], tab_c, 0x7604u));
-            o[4 * u + 1] = lds32(prmt_wg(w[tp + u], tab_c, 0x7614u));
-            o[4 * u + 2] = lds32(prmt_wg(w[tp + u], tab_c, 0x7624u));
-            o[4 * u + 3] = lds32(prmt_wg(w[tp + u], tab_c, 0x7634u));
-        }
-#pragma unroll
-        for (int i = 0; i < 8; ++i) o[i] = mul_h2(o[i], s);
-        tmem_st8(a + 4 * tp, o);
+    for (int t = 0; t < 4; ++t) {
+        o[4 * t + 0] = lds32(prmt_wg(w[t], tab_c, 0x7604u));
+        o[4 * t + 1] = lds32(prmt_wg(w[t], tab_c, 0x7614u));
+        o[4 * t + 2] = lds32(prmt_wg(w[t], tab_c, 0x7624u));
+        o[4 * t + 3] = lds32(prmt_wg(w[t], tab_c, 0x7634u));
     }
+#pragma unroll
+    for (int i = 0; i < 16; ++i) o[i] = mul_h2(o[i], s);
 }
 
 // four unsigned bytes v -> f16 pairs (bytes 0, 2) and (1, 3) of 1024 + byte, minus `bias`, times the scale
@@ -210,34 +206,27 @@ __device__ __forceinline__ void bytes_to_h2(uint32_t v, __half2 bias, const Scal
 }
 
 // Q8_0: q0, q1 = the row's 32 quant bytes of a block (tile order: words t of elements 4t.. and 16 + 4t.. alternate)
-__device__ __forceinline__ void put_q8(uint32_t a, const uint4& q0, const uint4& q1, float d) {
+__device__ __forceinline__ void make_q8(uint32_t (&o)[16], const uint4& q0, const uint4& q1, float d) {
     const Scale2 s = split_scale(d);
     const __half2 bias = __float2half2_rn(1152.f);   // 1024 + 128: the bytes have their top bit flipped
     const uint32_t w[8] = {q0.x, q0.z, q1.x, q1.z, q0.y, q0.w, q1.y, q1.w};   // elements 4m .. 4m+3
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
-        uint32_t o[8];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) bytes_to_h2(w[4 * h + i] ^ 0x80808080u, bias, s, o[2 * i], o[2 * i + 1]);
-        tmem_st8(a + 8 * h, o);
-    }
+    for (int i = 0; i < 8; ++i) bytes_to_h2(w[i] ^ 0x80808080u, bias, s, o[2 * i], o[2 * i + 1]);
 }
 
 // Q6_K: 32 columns: wl / wh [m] = ql / qh words of elements 4m .. 4m+3, NIB: high nibbles, hs = 2 * quarter; scales of the two 16-column groups
 template <bool NIB>
-__device__ __forceinline__ void put_q6(uint32_t a, const uint32_t (&wl)[8], const uint32_t (&wh)[8], uint32_t hs, float s0, float s1) {
+__device__ __forceinline__ void make_q6(uint32_t (&o)[16], const uint32_t (&wl)[8], const uint32_t (&wh)[8], uint32_t hs, float s0, float s1) {
     const __half2 bias = __float2half2_rn(1056.f);   // 1024 + 32
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
         const Scale2 s = split_scale(h ? s1 : s0);
-        uint32_t o[8];
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
             const uint32_t lo = (NIB ? wl[4 * h + i] >> 4 : wl[4 * h + i]) & 0x0F0F0F0Fu;
             const uint32_t hi = (hs >= 4 ? wh[4 * h + i] >> (hs - 4) : wh[4 * h + i] << (4 - hs)) & 0x30303030u;
-            bytes_to_h2(lo | hi, bias, s, o[2 * i], o[2 * i + 1]);
+            bytes_to_h2(lo | hi, bias, s, o[8 * h + 2 * i], o[8 * h + 2 * i + 1]);
         }
-        tmem_st8(a + 8 * h, o);
     }
 }
 
@@ -268,9 +257,11 @@ __global__ void __launch_bounds__(wg::kThreads, 1)
 wgemm_kernel(const WgemmArgs a, const __grid_constant__ CUtensorMap rows_map) {
     extern __shared__ __align__(1024) uint8_t smem_dyn[];
     constexpr int kSt = wg::kStages;
-    __shared__ __align__(8) unsigned long long s_bar[2 * kSt + 13 + 2 * wg::kFeed];
+    constexpr uint32_t kSlots = wg::q8_slots<FMT>();
+    __shared__ __align__(8) unsigned long long s_bar[2 * kSt + 4 * kSlots + 6 + 2 * wg::kFeed];
     __shared__ MmaItem s_feed[wg::kFeed];
     __shared__ uint32_t s_tmem;
+    __shared__ __align__(16) uint32_t s_rows[MODE == wg::kGateUp ? wg::kStages : 1][wg::kNT];   // row loaders: where the unit's rows start, [row % 4][row / 4]
     __shared__ float s_col[2][2][wg::kNT];   // epilogue, per unit parity: factors of the unit's columns
     const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31u;
     const uint32_t KB = a.K / 256, RT16 = a.rows / 16;
@@ -287,18 +278,20 @@ wgemm_kernel(const WgemmArgs a, const __grid_constant__ CUtensorMap rows_map) {
         }
     }
     const uint32_t bar = smem_addr(&s_bar[0]);
-    const uint32_t bar_full = bar, bar_empty = bar + 8 * kSt, bar_wfull = bar + 16 * kSt, bar_wempty = bar_wfull + 32;   // [parity][slot]
-    const uint32_t bar_accfull = bar_wempty + 32, bar_accfree = bar_accfull + 16, bar_tab = bar_accfree + 16;
+    const uint32_t bar_full = bar, bar_empty = bar + 8 * kSt, bar_wfull = bar + 16 * kSt, bar_wempty = bar_wfull + 16 * kSlots;   // [parity][slot]
+    const uint32_t bar_accfull = bar_wempty + 16 * kSlots, bar_accfree = bar_accfull + 16, bar_tab = bar_accfree + 16;
     const uint32_t bar_ufull = bar_tab + 8, bar_uempty = bar_ufull + 8 * wg::kFeed;
-    constexpr uint32_t kRowArrivals = MODE == wg::kGateUp ? 2 : 1;
+    const uint32_t bar_cols = bar_uempty + 8 * wg::kFeed;   // the epilogue's warps among themselves
+    constexpr uint32_t kRowWarps = wg::row_warps<MODE>();
     if (tid == 0) {
-        for (int s = 0; s < kSt; ++s) { mbar_init(bar_full + 8 * s, 8 + kRowArrivals); mbar_init(bar_empty + 8 * s, 1); }   // eight producer warps + the row loaders; one commit
-        for (int b = 0; b < 4; ++b) { mbar_init(bar_wfull + 8 * b, 1); mbar_init(bar_wempty + 8 * b, 8); }
-        for (int b = 0; b < wg::kFeed; ++b) { mbar_init(bar_ufull + 8 * b, 1); mbar_init(bar_uempty + 8 * b, wg::kProducerWarps + wg::kEpilogueWarps + 1 + kRowArrivals); }
+        for (int s = 0; s < kSt; ++s) { mbar_init(bar_full + 8 * s, 9); mbar_init(bar_empty + 8 * s, 1); }   // eight producer warps + the row loader; one commit
+        for (uint32_t b = 0; b < 2 * kSlots; ++b) { mbar_init(bar_wfull + 8 * b, 1); mbar_init(bar_wempty + 8 * b, 8); }
+        for (int b = 0; b < wg::kFeed; ++b) { mbar_init(bar_ufull + 8 * b, 1); mbar_init(bar_uempty + 8 * b, wg::kProducerWarps + wg::kEpilogueWarps + 1 + kRowWarps); }
         for (int b = 0; b < 2; ++b) {
             mbar_init(bar_accfull + 8 * b, 1); mbar_init(bar_accfree + 8 * b, wg::kEpilogueWarps);
         }
         mbar_init(bar_tab, 1);
+        mbar_init(bar_cols, wg::kEpilogueWarps);
         mbar_fence_init();
     }
     if (warp == 0) { umma::tmem_alloc(smem_addr(&s_tmem), 512); umma::tmem_relinquish(); }
@@ -329,13 +322,15 @@ wgemm_kernel(const WgemmArgs a, const __grid_constant__ CUtensorMap rows_map) {
         if (lane == 0) mbar_arrive(bar_uempty + 8 * s);
         return it.n != 0;
     };
-    // k-step i of a unit: 256-column block and 64-column quarter.  Blocks 2p and 2p + 1 are interleaved (see above).
+    // k-step i of a unit: 256-column block and 64-column quarter.  Blocks 2p and 2p + 1 are interleaved (see above).  Of a lone last
+    // block both producer groups get a copy and expand every other quarter, so that a stage always belongs to the same group.
     auto step_kb = [&](uint32_t i) -> uint32_t { return i < (KB & ~1u) * 4 ? 2 * (i >> 3) + (i & 1u) : KB - 1; };
     auto step_q = [&](uint32_t i) -> uint32_t { return i < (KB & ~1u) * 4 ? (i >> 1) & 3u : i & 3u; };
     const uint32_t KS = KB * 4;
 
     if (warp < (uint32_t)wg::kProducerWarps) {
         // ---- producers
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(wg::kProducerRegs));
         const uint32_t lq = warp & 3u, mat = (warp >> 2) & 1u, par = warp >> 3;
         const uint32_t r = 32 * lq + lane, r16 = r & 15u, g = r16 & 7u, tl = r >> 4;   // row of the 128, row of its tile, tile
         const uint32_t a_lane = tmem + ((32 * lq) << 16) + wg::kTmemA + mat * 32u;
@@ -343,39 +338,50 @@ wgemm_kernel(const WgemmArgs a, const __grid_constant__ CUtensorMap rows_map) {
         const uint32_t tab_c = wg::kTab + (FMT == QKM_TYPE_IQ3_XXS ? (lane & 15u) * 8u : 128u + lane * 4u);
         if (FMT == QKM_TYPE_IQ3_XXS || FMT == QKM_TYPE_IQ4_XS)
             if (!wait_bar(bar_tab, 0)) timed_out = true;
-        uint32_t round0 = 0, wcnt = 0, wcnt1 = 0;   // stage rounds before this unit; weight slots consumed
+        uint32_t round0 = 0, wcnt = 0, qcnt = 0;   // stage rounds before this unit; blocks and Q8_0 slots consumed
         MmaItem it;
         for (uint32_t k = 0; next_unit(k, it); ++k, round0 += KB) {
             const bool shared = MODE != wg::kDense && it.expert == kSharedItem;
-            auto open = [&](uint32_t i) -> uint32_t {   // stage of k-step i, free to be written
-                const uint32_t round = round0 + (i >> 2);
-                if (round && !wait_bar(bar_empty + 8 * (i & 3u), (round - 1) & 1u)) timed_out = true;
-                umma::fence_after_sync();
-                return a_lane + (i & 3u) * 64u;
-            };
-            auto close = [&](uint32_t i) {
+            // A step's stores are not waited for at its end: it is announced when the next step's first values have been computed,
+            // by which time they are through (waiting at once cost a tenth of the kernel).
+            uint32_t pending = 0xFFFFFFFFu, st = 0;
+            auto announce = [&]() {
+                if (pending == 0xFFFFFFFFu) return;
                 tmem_st_wait();
                 umma::fence_before_sync();
                 __syncwarp();
-                if (lane == 0) mbar_arrive(bar_full + 8 * (i & 3u));
+                if (lane == 0) mbar_arrive(bar_full + 8 * (pending & 3u));
+            };
+            auto store = [&](uint32_t i, uint32_t half, const uint32_t (&o)[16]) {   // half `half` of k-step i's 64 columns
+                if (half == 0) {
+                    announce();
+                    const uint32_t round = round0 + (i >> 2);   // the stage is free to be written
+                    if (round && !wait_bar(bar_empty + 8 * (i & 3u), (round - 1) & 1u)) timed_out = true;
+                    umma::fence_after_sync();
+                    st = a_lane + (i & 3u) * 64u;
+                    pending = i;
+                }
+                tmem_st16(st + 16 * half, o);
             };
             auto w_wait = [&]() {
-                if (!wait_bar(bar_wfull + 16 * par, wcnt & 1u)) timed_out = true;
+                // slot 0's barrier counts blocks and every kSlots-th Q8_0 slot
+                if (!wait_bar(bar_wfull + 8 * kSlots * par, (wcnt + qcnt / kSlots) & 1u)) timed_out = true;
                 ++wcnt;
             };
             auto w_free = [&]() {
                 __syncwarp();
-                if (lane == 0) mbar_arrive(bar_wempty + 16 * par);
+                if (lane == 0) mbar_arrive(bar_wempty + 8 * kSlots * par);
             };
-            for (uint32_t kb = par; kb < KB; kb += 2) {
-                const uint32_t i0 = kb < (KB & ~1u) ? (kb >> 1) * 8 + par : kb * 4, istep = kb < (KB & ~1u) ? 2u : 1u;   // its k-steps: i0 + q * istep
-                if (FMT == QKM_TYPE_Q8_0 || shared) {
-                    // 64 columns a slot, two slots: two 544-byte pieces of each tile
+            for (uint32_t kp = 0; kp < KB; kp += 2) {
+                const bool lone = kp + 1 == KB;
+                const uint32_t i0 = lone ? kp * 4 : kp * 4 + par, istep = lone ? 1u : 2u;   // the block's k-steps: i0 + q * istep
+                if (shared) {
+                    // Q8_0, 64 columns a slot: two 544-byte pieces of each tile
 #pragma unroll 1
-                    for (uint32_t q = 0; q < 4; ++q) {
-                        const uint32_t slot = q & 1u, cnt = slot ? wcnt1++ : wcnt++;
-                        if (!wait_bar(bar_wfull + 16 * par + 8 * slot, cnt & 1u)) timed_out = true;
-                        const uint32_t t0 = wbuf + slot * (16u * 1088u) + (mat * 8 + tl) * 1088u;
+                    for (uint32_t q = lone ? par : 0; q < 4; q += lone ? 2 : 1, ++qcnt) {
+                        const uint32_t slot = qcnt % kSlots, bars = 8 * (kSlots * par + slot);
+                        if (!wait_bar(bar_wfull + bars, (qcnt / kSlots + (slot ? 0u : wcnt)) & 1u)) timed_out = true;
+                        const uint32_t t0 = wbuf + slot * wg::kQ8Slot + (mat * 8 + tl) * 1088u;
                         uint4 v[2][2];
                         float d[2];
 #pragma unroll
@@ -386,15 +392,15 @@ wgemm_kernel(const WgemmArgs a, const __grid_constant__ CUtensorMap rows_map) {
                             d[s] = f16_bits_to_f32(lds_u16_wg(p + 2 * r16));
                         }
                         __syncwarp();
-                        if (lane == 0) mbar_arrive(bar_wempty + 16 * par + 8 * slot);
-                        const uint32_t i = i0 + q * istep, st = open(i);
-                        put_q8(st, v[0][0], v[0][1], d[0]);
-                        put_q8(st + 16, v[1][0], v[1][1], d[1]);
-                        close(i);
+                        if (lane == 0) mbar_arrive(bar_wempty + bars);
+                        uint32_t o[16];
+                        make_q8(o, v[0][0], v[0][1], d[0]);
+                        store(i0 + q * istep, 0, o);
+                        make_q8(o, v[1][0], v[1][1], d[1]);
+                        store(i0 + q * istep, 1, o);
                     }
                     continue;
                 }
-                if constexpr (FMT != QKM_TYPE_Q8_0) {
                 w_wait();
                 const uint32_t tb = wbuf + (mat * 8 + tl) * wg::tile_size<FMT>();
                 if constexpr (FMT == QKM_TYPE_IQ3_XXS) {
@@ -411,15 +417,18 @@ wgemm_kernel(const WgemmArgs a, const __grid_constant__ CUtensorMap rows_map) {
                     const float d4 = f16_bits_to_f32(lds_u16_wg(tb + 1664 + 2 * r16)) * 0.25f;
                     w_free();
 #pragma unroll
-                    for (int q = 0; q < 4; ++q) {   // sub-blocks 2q, 2q + 1: scale d (2s + 1) / 4, exact in f32, one rounding to f16
-                        const uint32_t i = i0 + q * istep, st = open(i);
+                    for (int q = 0; q < 4; ++q) {
+                        if (lone && ((q ^ par) & 1u)) continue;
+                        // sub-blocks 2q, 2q + 1: scale d (2s + 1) / 4, exact in f32, one rounding to f16
                         const uint32_t w4 = q < 2 ? sc.x : sc.y, sh = 16 * (q & 1);
                         const __half2 s0 = __float2half2_rn(d4 * (float)((w4 >> sh) & 255u)), s1 = __float2half2_rn(d4 * (float)((w4 >> (sh + 8)) & 255u));
                         const uint32_t w[4] = {q == 0 ? ix[0].x : q == 1 ? ix[0].y : q == 2 ? ix[0].z : ix[0].w, q == 0 ? ix[1].x : q == 1 ? ix[1].y : q == 2 ? ix[1].z : ix[1].w,
                                                q == 0 ? ix[2].x : q == 1 ? ix[2].y : q == 2 ? ix[2].z : ix[2].w, q == 0 ? ix[3].x : q == 1 ? ix[3].y : q == 2 ? ix[3].z : ix[3].w};
-                        put_iq3<false>(st, w, sg[q >> 1], 4 * (q & 1), s0, tab_c);
-                        put_iq3<true>(st + 16, w, sg[q >> 1], 4 * (q & 1) + 2, s1, tab_c);
-                        close(i);
+                        uint32_t o[16];
+                        make_iq3<false>(o, w, sg[q >> 1], 4 * (q & 1), s0, tab_c);
+                        store(i0 + q * istep, 0, o);
+                        make_iq3<true>(o, w, sg[q >> 1], 4 * (q & 1) + 2, s1, tab_c);
+                        store(i0 + q * istep, 1, o);
                     }
                 } else if constexpr (FMT == QKM_TYPE_IQ4_XS) {
                     const uint2 hd = lds64(tb + 16 * g + 8 * (r16 >> 3));   // d | scales_h << 16, scales_l
@@ -432,7 +441,7 @@ wgemm_kernel(const WgemmArgs a, const __grid_constant__ CUtensorMap rows_map) {
                         if (hf) w_free();
 #pragma unroll
                         for (int q = 0; q < 2; ++q) {
-                            const uint32_t i = i0 + (2 * hf + q) * istep, st = open(i);
+                            if (lone && ((q ^ par) & 1u)) continue;
 #pragma unroll
                             for (int s = 0; s < 2; ++s) {
                                 const int sb = 4 * hf + 2 * q + s;
@@ -441,13 +450,14 @@ wgemm_kernel(const WgemmArgs a, const __grid_constant__ CUtensorMap rows_map) {
                                 const int c = 2 * q + s;
                                 const uint32_t w[4] = {c == 0 ? v[0].x : c == 1 ? v[0].y : c == 2 ? v[0].z : v[0].w, c == 0 ? v[1].x : c == 1 ? v[1].y : c == 2 ? v[1].z : v[1].w,
                                                        c == 0 ? v[2].x : c == 1 ? v[2].y : c == 2 ? v[2].z : v[2].w, c == 0 ? v[3].x : c == 1 ? v[3].y : c == 2 ? v[3].z : v[3].w};
-                                if (MODE == wg::kDown) put_iq4(st + 16 * s, w, __float2half2_rn(dl), tab_c);   // two roundings of 2^-12
-                                else put_iq4(st + 16 * s, w, split_scale(dl), tab_c);
+                                uint32_t o[16];
+                                if (MODE == wg::kDown) make_iq4(o, w, __float2half2_rn(dl), tab_c);   // two roundings of 2^-12
+                                else make_iq4(o, w, split_scale(dl), tab_c);
+                                store(i0 + (2 * hf + q) * istep, s, o);
                             }
-                            close(i);
                         }
                     }
-                } else {   // Q6_K: k-step q = half q / 2, quarters 2 (q & 1) and the one after it: nibble q & 1 of both 32-byte runs
+                } else if constexpr (FMT == QKM_TYPE_Q6_K) {   // k-step k-step q = half q / 2, quarters 2 (q & 1) and the one after it: nibble q & 1 of both 32-byte runs
                     uint4 hq[4];
 #pragma unroll
                     for (int t = 0; t < 4; ++t) hq[t] = lds128(tb + 2304 + 64 * r16 + piece_at(r16, t));
@@ -464,7 +474,7 @@ wgemm_kernel(const WgemmArgs a, const __grid_constant__ CUtensorMap rows_map) {
                         for (int t = 0; t < 4; ++t) { wh[t] = hf ? hq[t].z : hq[t].x; wh[4 + t] = hf ? hq[t].w : hq[t].y; }
 #pragma unroll
                         for (int q = 0; q < 2; ++q) {
-                            const uint32_t i = i0 + (2 * hf + q) * istep, st = open(i);
+                            if (lone && ((q ^ par) & 1u)) continue;
 #pragma unroll
                             for (int s = 0; s < 2; ++s) {
                                 const int qd = 2 * q + s;
@@ -472,19 +482,43 @@ wgemm_kernel(const WgemmArgs a, const __grid_constant__ CUtensorMap rows_map) {
 #pragma unroll
                                 for (int t = 0; t < 4; ++t) { wl[t] = s ? v[t].z : v[t].x; wl[4 + t] = s ? v[t].w : v[t].y; }
                                 const float f0 = d * (float)(int8_t)((hf ? sc.y : sc.x) >> (8 * qd)), f1 = d * (float)(int8_t)((hf ? sc.w : sc.z) >> (8 * qd));
-                                if (q) put_q6<true>(st + 16 * s, wl, wh, 2 * qd, f0, f1);
-                                else put_q6<false>(st + 16 * s, wl, wh, 2 * qd, f0, f1);
+                                uint32_t o[16];
+                                if (q) make_q6<true>(o, wl, wh, 2 * qd, f0, f1);
+                                else make_q6<false>(o, wl, wh, 2 * qd, f0, f1);
+                                store(i0 + (2 * hf + q) * istep, s, o);
                             }
-                            close(i);
                         }
                     }
-                }
+                } else {   // Q8_0
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) {
+                        const bool skip = lone && ((q ^ par) & 1u);
+                        uint4 v[2][2];
+                        float d[2];
+#pragma unroll
+                        for (int s = 0; s < 2; ++s) {
+                            const uint32_t p = tb + (2 * q + s) * 544u;
+                            v[s][0] = lds128(p + 32 + ((r16 >> 3) * 32 + 4 * g) * 8);
+                            v[s][1] = lds128(p + 48 + ((r16 >> 3) * 32 + 4 * g) * 8);
+                            d[s] = f16_bits_to_f32(lds_u16_wg(p + 2 * r16));
+                        }
+                        if (q == 3) w_free();
+                        if (skip) continue;
+                        uint32_t o[16];
+                        make_q8(o, v[0][0], v[0][1], d[0]);
+                        store(i0 + q * istep, 0, o);
+                        make_q8(o, v[1][0], v[1][1], d[1]);
+                        store(i0 + q * istep, 1, o);
+                    }
                 }
             }
+            announce();
         }
     } else if (warp < (uint32_t)wg::kMmaWarp) {
-        // ---- epilogue: warp e reads TMEM lanes 32 e .. 32 e + 31
-        const uint32_t e = warp - wg::kProducerWarps, c = tid - wg::kProducerWarps * 32;   // c: the column this thread prepares
+        // ---- epilogue: warps e and e + 4 read TMEM lanes 32 e .. 32 e + 31, every other 16 columns each (with four warps the drain of
+        // 128 columns took 13,000 cycles a gate/up unit, a third of the time at 4096 tokens)
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(wg::kEpilogueRegs));
+        const uint32_t e = warp & 3u, eh = (warp >> 2) & 1u, c = tid - wg::kProducerWarps * 32;   // c: the column this thread prepares
         uint32_t used[2] = {0, 0}, next = 0, iter = 0;
         MmaItem it;
         for (; next_unit(iter, it); ++iter) {
@@ -511,7 +545,9 @@ wgemm_kernel(const WgemmArgs a, const __grid_constant__ CUtensorMap rows_map) {
                     f0[c] = a.x_inv_scale[p];
                 }
             }
-            named_sync_wg(1, wg::kEpilogueWarps * 32);
+            __syncwarp();
+            if (lane == 0) mbar_arrive(bar_cols);
+            if (!wait_bar(bar_cols, iter & 1u)) timed_out = true;
             const uint32_t b = big ? 0u : next;
             if (!wait_bar(bar_accfull + 8 * b, used[b] & 1u)) timed_out = true;
             if (big) { if (!wait_bar(bar_accfull + 8, used[1] & 1u)) timed_out = true; ++used[0]; ++used[1]; next = 0; }
@@ -519,7 +555,7 @@ wgemm_kernel(const WgemmArgs a, const __grid_constant__ CUtensorMap rows_map) {
             umma::fence_after_sync();
             const uint32_t t0 = tmem + ((32 * e) << 16) + b * 128u, t1 = t0 + (big ? 128u : 64u);
             const uint32_t row = 32 * e + lane;
-            for (uint32_t cb = 0; cb < n_mma; cb += 16) {
+            for (uint32_t cb = 16 * eh; cb < n_mma; cb += 32) {
                 uint32_t v0[16], v1[16];
                 umma::tmem_ld16(t0 + cb, v0);
                 umma::tmem_ld16(t1 + cb, v1);
@@ -550,7 +586,9 @@ wgemm_kernel(const WgemmArgs a, const __grid_constant__ CUtensorMap rows_map) {
             __syncwarp();
             if (lane == 0) { mbar_arrive(bar_accfree + 8 * b); if (big) mbar_arrive(bar_accfree + 8); }
         }
-    } else if (warp == (uint32_t)wg::kMmaWarp) {
+    } else {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(wg::kOtherRegs));
+    if (warp == (uint32_t)wg::kMmaWarp) {
         // ---- MMA issue: the whole warp walks the loop, one elected lane issues
         const bool leader = umma::elect_one();
         uint32_t used[2] = {0, 0}, next = 0, round0 = 0;
@@ -590,9 +628,10 @@ wgemm_kernel(const WgemmArgs a, const __grid_constant__ CUtensorMap rows_map) {
             mbar_expect_tx(bar_tab, wg::kTabBytes);
             for (uint32_t i = 0; i < 4; ++i) bulk_g2s(wg::kTab + i * 16384u, a.table + i * 16384u, 16384u, bar_tab);
         }
-        uint32_t cnt[2][2] = {{0, 0}, {0, 0}};   // uses of (parity, slot)
-        auto drained = [&](uint32_t par, uint32_t slot) {
-            if (cnt[par][slot] && !wait_bar(bar_wempty + 16 * par + 8 * slot, (cnt[par][slot] - 1) & 1u)) timed_out = true;
+        uint32_t blocks[2] = {0, 0}, slots[2] = {0, 0};   // handed out so far, per parity
+        auto drained = [&](uint32_t par, uint32_t slot) {   // everything put there has been read
+            const uint32_t uses = (slots[par] + kSlots - 1 - slot) / kSlots + (slot ? 0u : blocks[par]);
+            if (uses && !wait_bar(bar_wempty + 8 * (kSlots * par + slot), (uses - 1) & 1u)) timed_out = true;
         };
         uint32_t u = blockIdx.x;
         for (uint32_t k = 0;; ++k) {
@@ -608,7 +647,7 @@ wgemm_kernel(const WgemmArgs a, const __grid_constant__ CUtensorMap rows_map) {
             if (it.n == 0) break;
             uint32_t ticket = 0;
             if (lane == 0) ticket = a.ticket ? gridDim.x + atomicAdd(a.ticket, 1u) : u + gridDim.x;   // back by the time this unit's copies are issued
-            const bool shared = MODE != wg::kDense && it.expert == kSharedItem, q8 = FMT == QKM_TYPE_Q8_0 || shared;
+            const bool shared = MODE != wg::kDense && it.expert == kSharedItem, q8 = shared;
             const uint32_t tile = q8 ? (uint32_t)kTileQ8 : wg::tile_size<FMT>();
             auto tiles_of = [&](uint32_t m) -> const uint8_t* {   // first of the eight tiles of matrix (row tile) m, column block 0
                 const uint32_t rt128 = MODE == wg::kGateUp ? it.rt : min(2u * it.rt + m, a.rows / 128 - 1);
@@ -616,67 +655,69 @@ wgemm_kernel(const WgemmArgs a, const __grid_constant__ CUtensorMap rows_map) {
             };
             const uint8_t* src = q8 ? tiles_of((lane >> 3) & 1u) + (size_t)(lane & 7u) * kTileQ8 : tiles_of(lane & 1u);   // this lane's share
             for (uint32_t kp = 0; kp < KB; kp += 2) {
-                const uint32_t np = min(2u, KB - kp);
+                const bool lone = kp + 1 == KB;   // both groups get the block, of Q8_0 their quarters of it
                 if (q8) {
                     for (uint32_t q = 0; q < 4; ++q)
-                        for (uint32_t par = 0; par < np; ++par) {
-                            const uint32_t slot = q & 1u, wf = bar_wfull + 16 * par + 8 * slot;
+                        for (uint32_t par = 0; par < 2; ++par) {
+                            if (lone && ((q ^ par) & 1u)) continue;
+                            const uint32_t slot = slots[par] % kSlots, wf = bar_wfull + 8 * (kSlots * par + slot);
                             drained(par, slot);
-                            ++cnt[par][slot];
-                            if (lane == 0) mbar_expect_tx(wf, 16u * 1088u);
+                            if (__any_sync(0xFFFFFFFFu, timed_out)) break;   // a barrier that still counts bytes takes no second arrival
+                            ++slots[par];
+                            if (lane == 0) mbar_expect_tx(wf, wg::kQ8Slot);
                             __syncwarp();
-                            if (lane < 16) bulk_g2s(wg::w_base<FMT>() + par * wg::w_bytes<FMT>() + slot * (16u * 1088u) + lane * 1088u,
-                                                    src + (size_t)(kp + par) * RT16 * kTileQ8 + q * 1088u, 1088u, wf);
+                            if (lane < 16) bulk_g2s(wg::w_base<FMT>() + par * wg::w_bytes<FMT>() + slot * wg::kQ8Slot + lane * 1088u,
+                                                    src + (size_t)(lone ? kp : kp + par) * RT16 * kTileQ8 + q * 1088u, 1088u, wf);
                         }
                 } else {
-                    for (uint32_t par = 0; par < np; ++par) {
-                        const uint32_t wf = bar_wfull + 16 * par;
-                        drained(par, 0);
-                        drained(par, 1);   // a block covers both slots
-                        ++cnt[par][0];
+                    for (uint32_t par = 0; par < 2; ++par) {
+                        const uint32_t wf = bar_wfull + 8 * kSlots * par;
+                        for (uint32_t slot = 0; slot < kSlots; ++slot) drained(par, slot);   // a block covers them all
+                        if (__any_sync(0xFFFFFFFFu, timed_out)) break;
+                        ++blocks[par];
                         if (lane == 0) mbar_expect_tx(wf, 16 * tile);
                         __syncwarp();
-                        if (lane < 2) bulk_g2s(wg::w_base<FMT>() + par * wg::w_bytes<FMT>() + lane * 8 * tile, src + (size_t)(kp + par) * RT16 * tile, 8 * tile, wf);
+                        if (lane < 2) bulk_g2s(wg::w_base<FMT>() + par * wg::w_bytes<FMT>() + lane * 8 * tile, src + (size_t)(lone ? kp : kp + par) * RT16 * tile, 8 * tile, wf);
                     }
                 }
             }
             u = __shfl_sync(0xFFFFFFFFu, ticket, 0);
         }
-    } else if (MODE == wg::kGateUp) {
-        // ---- scattered activation rows: each of two warps copies four rows x 64 columns per instruction, rows 4 (w + 2m) + lane / 8; a step is
-        // announced two steps after its copies were issued.  Past the unit's end: the last row again (nobody reads those columns)
+    } else if (MODE == wg::kGateUp && warp < wg::kRowWarp + wg::row_warps<MODE>()) {
+        // ---- scattered activation rows: a warp per stage, which copies four rows x 64 columns per instruction, waits for their
+        // arrival and announces the step.  (Two warps that shared every step and announced it two steps later, so as
+        // not to wait, kept two stages in flight: the producers waited 40 to 60 % of their time for a free stage.)
+        // Past the unit's end: the last row again (nobody reads those columns)
         const uint32_t w = warp - wg::kRowWarp, rr = lane >> 3, c = lane & 7u;
-        const uint32_t dst0 = (4 * w + rr) * 128u + ((c ^ (4 * w + rr)) << 4);
-        uint32_t gs = 0;
-        auto announce = [&](uint32_t step) {
-            umma::fence_smem_to_async();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(bar_full + 8 * (step & 3u));
-        };
+        const uint32_t dst = wg::b_addr<FMT>(w), d0 = dst + rr * 128u + ((c ^ rr) << 4), d1 = dst + (rr + 4) * 128u + ((c ^ (rr + 4)) << 4);
+        const uint32_t rows = smem_addr(&s_rows[w][rr * 32]);
+        uint32_t round = 0;
         MmaItem it;
         for (uint32_t k = 0; next_unit(k, it); ++k) {
-            const uint32_t groups = ((it.n + 15u) & ~15u) / 8;   // of eight rows
-            const __half* src[16];
+            const uint32_t groups = ((it.n + 15u) & ~15u) / 4;   // of four rows, a multiple of four
+            for (uint32_t r = lane; r < 4 * groups; r += 32)
+                s_rows[w][(r & 3u) * 32 + (r >> 2)] = (a.pairs[it.pair_off + min(r, it.n - 1)] >> 4) * (a.K / 8);   // in 16-byte pieces
+            __syncwarp();
+            for (uint32_t i = w; i < KS; i += 4, ++round) {
+                if (round && !wait_bar(bar_empty + 8 * w, (round - 1) & 1u)) timed_out = true;
+                const uint4* src = reinterpret_cast<const uint4*>(a.xrows) + step_kb(i) * 32u + step_q(i) * 8u + c;
 #pragma unroll
-            for (int m = 0; m < 16; ++m)
-                src[m] = (uint32_t)m < groups ? a.xrows + (size_t)(a.pairs[it.pair_off + min(8u * m + 4 * w + rr, it.n - 1)] >> 4) * a.K + 8 * c : a.xrows;
-            for (uint32_t i = 0; i < KS; ++i, ++gs) {
-                if (gs >= 4 && !wait_bar(bar_empty + 8 * (gs & 3u), ((gs >> 2) - 1) & 1u)) timed_out = true;
-                const uint32_t st = wg::b_addr<FMT>(gs & 3u) + dst0, k0 = step_kb(i) * 256u + step_q(i) * 64u;
+                for (int b = 0; b < 8; ++b)
+                    if (4u * b < groups) {
+                        const uint4 o4 = lds128(rows + 16 * b);
+                        const uint32_t o[4] = {o4.x, o4.y, o4.z, o4.w};
 #pragma unroll
-                for (int m = 0; m < 16; ++m)
-                    if ((uint32_t)m < groups) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(st + m * 1024u), "l"(src[m] + k0) : "memory");
-                asm volatile("cp.async.commit_group;" ::: "memory");
-                if (gs >= 2) {
-                    asm volatile("cp.async.wait_group 2;" ::: "memory");
-                    announce(gs - 2);
-                }
+                        for (int j = 0; j < 4; ++j)
+                            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(((j & 1) ? d1 : d0) + (2 * b + (j >> 1)) * 1024u), "l"(src + o[j]) : "memory");
+                    }
+                asm volatile("cp.async.wait_all;" ::: "memory");
+                umma::fence_smem_to_async();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(bar_full + 8 * w);
             }
+            __syncwarp();   // every lane is done with this unit's offsets
         }
-        asm volatile("cp.async.wait_group 0;" ::: "memory");
-        if (gs >= 2) announce(gs - 2);
-        if (gs >= 1) announce(gs - 1);
-    } else if (warp == (uint32_t)wg::kRowWarp) {
+    } else if (MODE != wg::kGateUp && warp == (uint32_t)wg::kRowWarp) {
         // ---- consecutive activation rows: boxes of 16
         uint32_t gs = 0;
         MmaItem it;
@@ -685,14 +726,17 @@ wgemm_kernel(const WgemmArgs a, const __grid_constant__ CUtensorMap rows_map) {
             for (uint32_t i = 0; i < KS; ++i, ++gs) {
                 const uint32_t stage = gs & 3u;
                 if (gs >= 4 && !wait_bar(bar_empty + 8 * stage, ((gs >> 2) - 1) & 1u)) timed_out = true;
+                if (__any_sync(0xFFFFFFFFu, timed_out)) break;   // a barrier that still counts bytes takes no second arrival
                 if (lane == 0) mbar_expect_tx(bar_full + 8 * stage, boxes * 2048u);
                 __syncwarp();
                 if (lane < boxes) tma_rows16(wg::b_addr<FMT>(stage) + lane * 2048u, &rows_map, step_kb(i) * 256u + step_q(i) * 64u, it.pair_off + 16 * lane, bar_full + 8 * stage);
             }
         }
     }
+    }
     umma::fence_before_sync();
     const int any_timed_out = __syncthreads_or(timed_out ? 1 : 0);   // any role's wait that ran out counts
+    if (any_timed_out) for (int i = 0; i < 100; ++i) __nanosleep(1000);   // copies and MMAs still under way end long before this does
     if (warp == 0) umma::tmem_dealloc(tmem, 512);
     if (any_timed_out && tid == 0) atomicExch(a.status, (uint32_t)kStatusWaitTimeout);
 }
