@@ -642,7 +642,8 @@ static int decode_fused(qkm_ctx* c, const qkm_layer_dev& ld, const float* x, uin
     DownDecodeArgs da{};
     da.tiles = (const uint8_t*)ld.tiles[4]; da.sh_tiles = (const uint8_t*)ld.tiles[7]; da.lut = c->lut_dd;
     da.h = h; da.sel = sel; da.y = y; da.n_tokens = n; da.status = c->status; da.d = d;
-    if (w.down_type == QKM_TYPE_IQ4_XS) QKM_LAUNCH(c, launch_decode_down(c->Lchain(), da, nb));
+    if (!decode_down_ok(d)) QKM_LAUNCH(c, launch_decode_down_any(c->Lchain(), da, w.down_type, nb));
+    else if (w.down_type == QKM_TYPE_IQ4_XS) QKM_LAUNCH(c, launch_decode_down(c->Lchain(), da, nb));
     else QKM_LAUNCH(c, launch_decode_down_q6k(c->Lchain(), da, nb));
     c->prof_mark("moe.dn");
     return QKM_OK;
@@ -657,7 +658,7 @@ extern "C" QKM_API int qkm_moe_decode(qkm_ctx* c, uint32_t layer, const float* x
     const qkm_dims& d = c->cfg.dims;
     c->prof_begin();
     constexpr uint32_t kMost = 64;
-    if (n && ld.fused_ok && c->dec_ok && route_decode_ok(d, n < kMost ? n : kMost, c->route_scratch_bytes) && decode_down_ok(d)) {
+    if (n && ld.fused_ok && c->dec_ok && route_decode_ok(d, n < kMost ? n : kMost, c->route_scratch_bytes) && (decode_down_ok(d) || decode_down_any_ok(d))) {
         for (uint32_t t = 0; t < n; t += kMost)
             if (int rc = decode_fused(c, ld, x + (size_t)t * d.n_embd, n - t < kMost ? n - t : kMost, y + (size_t)t * d.n_embd, c->sel + t,
                                       c->h + (size_t)t * (d.n_used + 1) * d.n_ff)) return rc;

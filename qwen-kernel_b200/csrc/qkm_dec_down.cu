@@ -29,6 +29,7 @@
 //
 // Shared memory: the table occupies [0x10000, 0x20000) of the shared window; barriers, the first
 // rings and the shared row's planes lie below it, the other rings and the scratch above.
+#include "qkm_dec_tiles.cuh"
 #include "qkm_kernels.h"
 #include "qkm_stream.cuh"
 #include "qkm_tiles.cuh"
@@ -74,35 +75,6 @@ cudaError_t launch_decode_down_lut(const Launch& L, uint8_t* lut) {
     decode_down_lut_kernel<<<dd::kTabBytes / 4 / 256, 256, 0, L.stream>>>(lut);
     L.count();
     return cudaGetLastError();
-}
-
-__device__ __forceinline__ uint32_t prmt_dd(uint32_t a, uint32_t b, uint32_t sel) {
-    uint32_t r;
-    asm("prmt.b32 %0, %1, %2, %3;" : "=r"(r) : "r"(a), "r"(b), "r"(sel));
-    return r;
-}
-
-// The eight sub-block scales ls - 32 of one row as int8: even sub-blocks 0,2,4,6 in ev, odd 1,3,5,7 in od.
-// sl: scales_l (eight 4-bit fields), sh: scales_h (eight 2-bit fields)  (src/quants.h:107-113, :139-146)
-__device__ __forceinline__ void iq4_scales(uint32_t sl, uint32_t sh, uint32_t& ev, uint32_t& od) {
-    const uint32_t r = prmt_dd(sh, 0u, 0x1100u);                       // bytes (B0, B0, B1, B1) of scales_h
-    const uint32_t he = ((r << 4) & 0x00300030u) | (r & 0x30003000u);  // top two bits of sub-blocks 0,2,4,6 at bits 4..5
-    const uint32_t ho = ((r << 2) & 0x00300030u) | ((r >> 2) & 0x30003000u);
-    const uint32_t te = ((sl & 0x0F0F0F0Fu) | he) ^ 0x20202020u;       // ls ^ 32 per byte
-    const uint32_t to = (((sl >> 4) & 0x0F0F0F0Fu) | ho) ^ 0x20202020u;
-    // ls - 32 as int8: bit 5 of (ls ^ 32) extended into bits 6..7 (no carry leaves a byte)
-    ev = (te & 0x20202020u) * 6u + te;
-    od = (to & 0x20202020u) * 6u + to;
-}
-
-// Eight IQ4_XS weights of one quant word (elements e0 .. e7 = 8t .. 8t+7 of a sub-block; a byte's nibbles are two
-// elements apart, see qkm_tiles.cuh) as two int8 MMA A-operand registers: lo = (e0, e2, e1, e3), hi = (e4, e6, e5, e7).
-// tab_c: bytes (lane * 4, -, 0x01, 0x00): with a quant byte in byte 1 it is that byte's table entry for this lane.
-__device__ __forceinline__ void iq4_word(uint32_t w, uint32_t tab_c, uint32_t& lo, uint32_t& hi) {
-    const uint32_t e0 = lds32(prmt_dd(w, tab_c, 0x7604u)), e1 = lds32(prmt_dd(w, tab_c, 0x7614u));
-    const uint32_t e2 = lds32(prmt_dd(w, tab_c, 0x7624u)), e3 = lds32(prmt_dd(w, tab_c, 0x7634u));
-    lo = prmt_dd(e0, e1, 0x5410u);
-    hi = prmt_dd(e2, e3, 0x5410u);
 }
 
 __global__ void __launch_bounds__(dd::kWarps * 32, 1)
@@ -219,13 +191,13 @@ decode_down_kernel(DownDecodeArgs a) {
                 // digit j of elements 8 lane + 4 r .. + 3 (lane t = lane & 3 of sub-block lane / 4, register r), in iq4_word's order 0, 2, 1, 3
 #pragma unroll
                 for (int r = 0; r < 2; ++r) {
-                    const uint32_t x0 = prmt_dd(dgt[4 * r], dgt[4 * r + 2], 0x5140u), x1 = prmt_dd(dgt[4 * r + 1], dgt[4 * r + 3], 0x5140u);
-                    const uint32_t y0 = prmt_dd(dgt[4 * r], dgt[4 * r + 2], 0x7362u), y1 = prmt_dd(dgt[4 * r + 1], dgt[4 * r + 3], 0x7362u);
+                    const uint32_t x0 = prmt_dec(dgt[4 * r], dgt[4 * r + 2], 0x5140u), x1 = prmt_dec(dgt[4 * r + 1], dgt[4 * r + 3], 0x5140u);
+                    const uint32_t y0 = prmt_dec(dgt[4 * r], dgt[4 * r + 2], 0x7362u), y1 = prmt_dec(dgt[4 * r + 1], dgt[4 * r + 3], 0x7362u);
                     uint8_t* q = dig + (lane >> 2) * 32 + r * 16 + (lane & 3u) * 4;
-                    *reinterpret_cast<uint32_t*>(q) = prmt_dd(x0, x1, 0x5410u);
-                    *reinterpret_cast<uint32_t*>(q + 256) = prmt_dd(x0, x1, 0x7632u);
-                    *reinterpret_cast<uint32_t*>(q + 512) = prmt_dd(y0, y1, 0x5410u);
-                    *reinterpret_cast<uint32_t*>(q + 768) = prmt_dd(y0, y1, 0x7632u);
+                    *reinterpret_cast<uint32_t*>(q) = prmt_dec(x0, x1, 0x5410u);
+                    *reinterpret_cast<uint32_t*>(q + 256) = prmt_dec(x0, x1, 0x7632u);
+                    *reinterpret_cast<uint32_t*>(q + 512) = prmt_dec(y0, y1, 0x5410u);
+                    *reinterpret_cast<uint32_t*>(q + 768) = prmt_dec(y0, y1, 0x7632u);
                 }
                 __syncwarp();
 #pragma unroll
@@ -291,7 +263,7 @@ decode_down_kernel(DownDecodeArgs a) {
                     int c[4];
                     mma_s8_first(c, a0, a1, a2, a3, b0[sb], b1[sb]);
                     const uint32_t sel = 0x8880u + (uint32_t)(sb >> 1) * 0x1111u;   // byte sb / 2, sign-extended
-                    const int la = (int)prmt_dd((sb & 1) ? oa : ea, 0u, sel), lb = (int)prmt_dd((sb & 1) ? ob : eb, 0u, sel);
+                    const int la = (int)prmt_dec((sb & 1) ? oa : ea, 0u, sel), lb = (int)prmt_dec((sb & 1) ? ob : eb, 0u, sel);
                     acc[0] += la * c[0]; acc[1] += la * c[1]; acc[2] += lb * c[2]; acc[3] += lb * c[3];
                 }
             }

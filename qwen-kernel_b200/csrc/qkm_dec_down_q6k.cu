@@ -20,6 +20,7 @@
 // routing weight are applied once per tile in f32.
 //
 // Shared expert: warp w also takes 32-column block w of the Q8_0 matrix for the tile's rows.
+#include "qkm_dec_tiles.cuh"
 #include "qkm_kernels.h"
 #include "qkm_stream.cuh"
 #include "qkm_tiles.cuh"
@@ -43,25 +44,6 @@ constexpr uint32_t kHd = kRed + 2 * kWarps * kChunk * 16 * 4;              // 4 
 constexpr uint32_t kMisc = kHd + 4 * kMaxFf;                               // 16 warp maxima
 constexpr uint32_t kEnd = kMisc + 128;
 }  // namespace dq
-
-__device__ __forceinline__ uint32_t prmt_dq(uint32_t a, uint32_t b, uint32_t sel) {
-    uint32_t r;
-    asm("prmt.b32 %0, %1, %2, %3;" : "=r"(r) : "r"(a), "r"(b), "r"(sel));
-    return r;
-}
-
-// Sixteen Q6_K weights as four int8 MMA A-operand registers, each 4 * (q - 32): w1 / w2 are the ql
-// words of elements l..l+3 in the first / second 32-byte run of a half, hq the qh word of the same
-// l; r[qd] holds elements l + 32 * qd .. + 3  (src/quants.h:148-163).
-__device__ __forceinline__ void q6k_words(uint32_t w1, uint32_t w2, uint32_t hq, uint32_t (&r)[4]) {
-    const uint32_t hx = hq ^ 0xAAAAAAAAu;          // top bit of every pair flipped: the sign of q - 32
-    const uint32_t lo1 = w1 & 0x0F0F0F0Fu, hi1 = w1 & 0xF0F0F0F0u;
-    const uint32_t lo2 = w2 & 0x0F0F0F0Fu, hi2 = w2 & 0xF0F0F0F0u;
-    r[0] = ((hx << 6) & 0xC0C0C0C0u) | (lo1 << 2);
-    r[1] = ((hx << 4) & 0xC0C0C0C0u) | (lo2 << 2);
-    r[2] = ((hx << 2) & 0xC0C0C0C0u) | (hi1 >> 2);
-    r[3] = (hx & 0xC0C0C0C0u) | (hi2 >> 2);
-}
 
 __global__ void __launch_bounds__(dq::kWarps * 32, 1)
 decode_down_q6k_kernel(DownDecodeArgs a) {
@@ -167,10 +149,10 @@ decode_down_q6k_kernel(DownDecodeArgs a) {
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
                     const uint32_t sel = 0x4040u + 0x1111u * j;   // byte j of a, byte j of b, twice
-                    const uint32_t p01 = prmt_dq(dg[0], dg[1], sel), p23 = prmt_dq(dg[2], dg[3], sel);
-                    const uint32_t p45 = prmt_dq(dg[4], dg[5], sel), p67 = prmt_dq(dg[6], dg[7], sel);
+                    const uint32_t p01 = prmt_dec(dg[0], dg[1], sel), p23 = prmt_dec(dg[2], dg[3], sel);
+                    const uint32_t p45 = prmt_dec(dg[4], dg[5], sel), p67 = prmt_dec(dg[6], dg[7], sel);
                     *reinterpret_cast<uint2*>(dig + 256 * j + 8 * lane) =
-                        make_uint2(prmt_dq(p01, p23, 0x5410u), prmt_dq(p45, p67, 0x5410u));
+                        make_uint2(prmt_dec(p01, p23, 0x5410u), prmt_dec(p45, p67, 0x5410u));
                 }
                 __syncwarp();
 #pragma unroll
@@ -235,7 +217,7 @@ decode_down_q6k_kernel(DownDecodeArgs a) {
                     int c[4];
                     mma_s8_first(c, a0[qd], a1[qd], a2[qd], a3[qd], b0[j], b1[j]);
                     const uint32_t sel = 0x8880u + (uint32_t)(j & 3) * 0x1111u;   // byte j & 3, sign-extended
-                    const int sa = (int)prmt_dq(hf ? scA.y : scA.x, 0u, sel), sb = (int)prmt_dq(hf ? scB.y : scB.x, 0u, sel);
+                    const int sa = (int)prmt_dec(hf ? scA.y : scA.x, 0u, sel), sb = (int)prmt_dec(hf ? scB.y : scB.x, 0u, sel);
                     acc[0] += sa * c[0]; acc[1] += sa * c[1]; acc[2] += sb * c[2]; acc[3] += sb * c[3];
                 }
             }

@@ -134,6 +134,9 @@ cudaError_t launch_decode_down_lut(const Launch& L, uint8_t* lut);
 cudaError_t launch_decode_down(const Launch& L, const DownDecodeArgs& a, uint32_t n_blocks);
 // the same with the routed experts as Q6_K tiles
 cudaError_t launch_decode_down_q6k(const Launch& L, const DownDecodeArgs& a, uint32_t n_blocks);
+// either type, other numbers of slots
+bool decode_down_any_ok(const qkm_dims& d);
+cudaError_t launch_decode_down_any(const Launch& L, const DownDecodeArgs& a, uint32_t type, uint32_t n_blocks);
 
 // ---- qkm_wgemm.cu : tcgen05 GEMMs with quantised weights (batched prefill, dense projections)
 constexpr uint16_t kSharedItem = 0xFFFFu;   // MmaItem::expert of the shared expert's units

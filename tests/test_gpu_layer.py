@@ -148,6 +148,20 @@ def test_decode_512_experts(pkg, orc, syn, T):
         assert np.array_equal(y, ctx.moe_forward_host(0, x, mode=0))
 
 
+@pytest.mark.parametrize("n_ff,n_used,dt,T", [(512, 10, 23, 3), (512, 10, 14, 40), (512, 1, 23, 1), (256, 15, 14, 7), (256, 15, 23, 64), (512, 9, 23, 2)])
+def test_decode_numbers_of_slots(pkg, orc, syn, n_ff, n_used, dt, T):
+    """(slot, column block) pairs other than sixteen: more and fewer warps, fewer pairs than shared blocks."""
+    dims = syn.Dims(n_embd=512, n_ff=n_ff, n_expert=32, n_used=n_used)
+    layer = syn.make_layer(dims, seed=16, gateup_type=23, down_type=dt)
+    x = syn.random_x(T, dims.n_embd, seed=17)
+    ref = orc.moe_layer(layer, x, threads=orc.hardware_threads())
+    with pkg.Context(dims, n_layer=1, max_tokens=T, device=0) as ctx:
+        ctx.upload_layer(0, layer)
+        y = ctx.moe_forward_host(0, x, mode=0)
+        check_layer(syn, y, ctx.last_sel(T), ref, n_used)
+        assert np.array_equal(y, ctx.moe_forward_host(0, x, mode=0))
+
+
 def test_decode_router_is_deterministic_over_many_calls(pkg, orc, syn):
     """200 calls of the fused decode sequence on the same 16 rows: ids, weights and outputs are the
     same bits every time (a last-arriving block ranks the logits; the reference removed such a
