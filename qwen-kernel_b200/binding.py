@@ -1,5 +1,6 @@
 """ctypes binding of include/qk_moe.h (libqkmoe.so) and a thin host-side mirror
-of the reference engine's per-layer MoE interface.
+of the reference engine's per-layer MoE interface.  The calls made on every decode step go
+through an extension module instead (csrc/py_calls.cpp).
 
 There is no CPU path here: if the CUDA library is missing or no B200 is
 present, loading or opening fails with an error.
@@ -186,6 +187,8 @@ class Context:
     def __init__(self, dims: synth.Dims = None, n_layer=1, max_tokens=16, device=-1, expert_first=0,
                  expert_count=0):
         self.lib = load_library()
+        from . import qkm_calls
+        self._calls = qkm_calls
         dims = dims or synth.Dims()
         self.dims = dims
         cfg = Config(Dims(dims.n_embd, dims.n_ff, dims.n_expert, dims.n_used), n_layer, max_tokens, device, 0,
@@ -281,24 +284,34 @@ class Context:
         self.check(self.lib.qkm_moe_shared_down(self.h, _p(down), _p(h), _p(sel), _p(y2), n))
 
     def gemv(self, ttype, W, x, y, M, K, n=1):
-        self.check(self.lib.qkm_gemv(self.h, ttype, _p(W), _p(x), _p(y), M, K, n))
+        rc = self._calls.gemv(self.h, ttype, W, x, y, M, K, n)
+        if rc:
+            self.check(rc)
 
     def dequant(self, ttype, blocks, y, n_elems):
         self.check(self.lib.qkm_dequant(self.h, ttype, _p(blocks), _p(y), n_elems))
 
     # -- fused
     def moe_decode(self, layer_idx, x, n, y):
-        self.check(self.lib.qkm_moe_decode(self.h, layer_idx, _p(x), n, _p(y)))
+        rc = self._calls.moe_decode(self.h, layer_idx, x, n, y)
+        if rc:
+            self.check(rc)
 
     def moe_prefill(self, layer_idx, x, n, y):
-        self.check(self.lib.qkm_moe_prefill(self.h, layer_idx, _p(x), n, _p(y)))
+        rc = self._calls.moe_prefill(self.h, layer_idx, x, n, y)
+        if rc:
+            self.check(rc)
 
     def moe_decode_stack(self, first, count, x, n, y):
-        self.check(self.lib.qkm_moe_decode_stack(self.h, first, count, _p(x), n, _p(y)))
+        rc = self._calls.moe_decode_stack(self.h, first, count, x, n, y)
+        if rc:
+            self.check(rc)
 
     def moe_decode_stack_host(self, first, count, x_host_ptr, n, y_host_ptr):
         """x/y: host addresses (ints) of [count][n][n_embd] f32, ideally pinned."""
-        self.check(self.lib.qkm_moe_decode_stack_host(self.h, first, count, x_host_ptr, n, y_host_ptr))
+        rc = self._calls.moe_decode_stack_host(self.h, first, count, x_host_ptr, n, y_host_ptr)
+        if rc:
+            self.check(rc)
 
     def moe_forward_host(self, layer_idx, x: np.ndarray, mode=0) -> np.ndarray:
         """Host in, host out (copies inside): the call an engine with host-resident
@@ -314,7 +327,9 @@ class Context:
         self.check(self.lib.qkm_dense_upload(self.h, slot, ttype, W.ctypes.data, M, K))
 
     def dense_gemm(self, slot, x, n, y):
-        self.check(self.lib.qkm_dense_gemm(self.h, slot, _p(x), n, _p(y)))
+        rc = self._calls.dense_gemm(self.h, slot, x, n, y)
+        if rc:
+            self.check(rc)
 
     # -- layer entry / tail
     def add_rmsnorm(self, a, b, w, y, xn, n_rows, n, eps=1e-6):
@@ -327,11 +342,14 @@ class Context:
         self.check(self.lib.qkm_add_rms3_grouped(self.h, _p(a), _p(routed), _p(c2), _p(w), _p(s), _p(xn), n_rows, n, n_used, eps))
 
     def argmax(self, logits, n_rows, n, tok):
-        self.check(self.lib.qkm_argmax(self.h, _p(logits), n_rows, n, _p(tok)))
+        rc = self._calls.argmax(self.h, logits, n_rows, n, tok)
+        if rc:
+            self.check(rc)
 
     def moe_layer_step(self, layer_idx, resid, attn_out, w_post, w_next, n, resid_out, xn_next, eps=1e-6):
-        self.check(self.lib.qkm_moe_layer_step(self.h, layer_idx, _p(resid), _p(attn_out), _p(w_post), _p(w_next), n, eps,
-                                               _p(resid_out), _p(xn_next)))
+        rc = self._calls.moe_layer_step(self.h, layer_idx, resid, attn_out, w_post, w_next, n, eps, resid_out, xn_next)
+        if rc:
+            self.check(rc)
 
     # -- expert parallel (this context is one shard; see include/qk_moe.h)
     def ep_dispatch(self, layer_idx, x, n, n_ranks, xsend, selsend) -> list:

@@ -1,4 +1,5 @@
-"""Builds the CUDA library in-tree: csrc/*.cu -> libqkmoe.so (sm_100a only).
+"""Builds the CUDA library in-tree: csrc/*.cu -> libqkmoe.so (sm_100a only), and the extension
+module of the binding, csrc/py_calls.cpp -> qkm_calls.so.
 
     python qwen-kernel_b200/build.py [--force] [--verbose]
 
@@ -13,10 +14,12 @@ import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 OUT = os.path.join(HERE, "libqkmoe.so")
+CALLS = os.path.join(HERE, "qkm_calls.so")
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 NVCC_FLAGS = ["-O3", "-std=c++17", "-lineinfo", "--expt-relaxed-constexpr", "-Xcompiler",
               "-fPIC,-fvisibility=hidden,-Wall,-Wno-unused-function", "-Xptxas", "-v"]
@@ -38,7 +41,7 @@ def _digest() -> str:
     for root in (CSRC, os.path.join(HERE, "..", "include")):
         for f in sorted(os.listdir(root)):
             p = os.path.join(root, f)
-            if os.path.isfile(p) and f.endswith((".cu", ".cuh", ".h", ".inc")):
+            if os.path.isfile(p) and f.endswith((".cu", ".cuh", ".h", ".inc", ".cpp")):
                 h.update(f.encode())
                 h.update(open(p, "rb").read())
     h.update(" ".join(ARCH + NVCC_FLAGS).encode())
@@ -51,7 +54,7 @@ def build(force: bool = False, verbose: bool = False) -> str:
     os.makedirs(bdir, exist_ok=True)
     stamp = os.path.join(bdir, "stamp")
     dig = _digest()
-    if not force and os.path.exists(OUT) and os.path.exists(stamp) and open(stamp).read() == dig:
+    if not force and os.path.exists(OUT) and os.path.exists(CALLS) and os.path.exists(stamp) and open(stamp).read() == dig:
         return OUT
     cc = nvcc()
 
@@ -74,6 +77,11 @@ def build(force: bool = False, verbose: bool = False) -> str:
     r = subprocess.run([cc, *ARCH, "-shared", "-o", OUT, *objs], capture_output=True, text=True)
     if r.returncode != 0:
         raise RuntimeError("link failed:\n" + r.stdout + r.stderr)
+    r = subprocess.run(["g++", "-O2", "-std=c++17", "-Wall", "-shared", "-fPIC", "-fvisibility=hidden", "-I" + sysconfig.get_paths()["include"],
+                        os.path.join(CSRC, "py_calls.cpp"), "-o", CALLS, "-L" + HERE, "-l:libqkmoe.so", "-Wl,-rpath,$ORIGIN"],
+                       capture_output=True, text=True)
+    if r.returncode != 0:
+        raise RuntimeError("g++ failed on py_calls.cpp:\n" + r.stdout + r.stderr)
     open(stamp, "w").write(dig)
     return OUT
 

@@ -993,9 +993,10 @@ extern "C" QKM_API int qkm_argmax(qkm_ctx* c, const float* logits, uint32_t n_ro
         if (c->argmax_scratch) QKM_CUDA(c, cudaFree(c->argmax_scratch));
         c->argmax_scratch = nullptr; c->argmax_rows = 0;
         QKM_CUDA(c, cudaMalloc(&c->argmax_scratch, argmax_scratch_bytes(n_rows)));
+        QKM_CUDA(c, cudaMemsetAsync(c->argmax_scratch, 0, argmax_scratch_bytes(n_rows), c->stream));
         c->argmax_rows = n_rows;
     }
-    QKM_LAUNCH(c, launch_argmax(c->L(), logits, n_rows, n, c->argmax_scratch, tok));
+    QKM_LAUNCH(c, launch_argmax(c->L(), logits, n_rows, n, c->argmax_scratch, c->argmax_rows, tok));
     return QKM_OK;
 }
 

@@ -253,13 +253,15 @@ gemv_stream_kernel(const uint8_t* __restrict__ W, const float* __restrict__ x, f
 // decode of one row.
 template <int TYPE>
 __global__ void __launch_bounds__(256)
-gemv_direct_kernel(const uint8_t* __restrict__ W, const float* __restrict__ x, float* __restrict__ y,
+gemv_direct_kernel(const uint8_t* __restrict__ W, const float* x, float* __restrict__ y,
                    uint32_t M, uint32_t K, uint32_t split) {   // split = warps per row: 1, 2, 4 or 8
     __shared__ gv::Luts s_lut;
     __shared__ float s_part[8];
     const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31u;
     if (TYPE == QKM_TYPE_IQ3_XXS) s_lut.grid[tid] = c_iq3_grid[tid];
     if (TYPE == QKM_TYPE_IQ4_XS && tid < 16) s_lut.iq4[tid] = (float)c_iq4_values[tid];
+    pdl_trigger();
+    pdl_wait();   // nothing that other kernels write has been touched yet
     if (TYPE == QKM_TYPE_IQ3_XXS || TYPE == QKM_TYPE_IQ4_XS) __syncthreads();
     const uint32_t rows_per_block = 8 / split;
     const uint32_t r = blockIdx.x * rows_per_block + warp / split, part = warp % split;
@@ -272,8 +274,8 @@ gemv_direct_kernel(const uint8_t* __restrict__ W, const float* __restrict__ x, f
             const uint32_t u = part * units + i;
             float w[8];
             gv::unit8<TYPE>(row, u * 8, w, s_lut);
-            const float4 a = __ldg(reinterpret_cast<const float4*>(x + u * 8));
-            const float4 b = __ldg(reinterpret_cast<const float4*>(x + u * 8 + 4));
+            const float4 a = *reinterpret_cast<const float4*>(x + u * 8);
+            const float4 b = *reinterpret_cast<const float4*>(x + u * 8 + 4);
             acc0 += w[0] * a.x; acc1 += w[1] * a.y; acc0 += w[2] * a.z; acc1 += w[3] * a.w;
             acc0 += w[4] * b.x; acc1 += w[5] * b.y; acc0 += w[6] * b.z; acc1 += w[7] * b.w;
         }
@@ -299,9 +301,10 @@ static cudaError_t gemv_direct_launch(const Launch& L, const uint8_t* W, const f
     uint32_t split = 1;
     while (split < 8 && (uint64_t)M * split * 2 <= 148u * 64u && (K / 8) % (split * 2 * 32) == 0) split *= 2;
     const uint32_t rows_per_block = 8 / split;
-    gemv_direct_kernel<TYPE><<<(M + rows_per_block - 1) / rows_per_block, 256, 0, L.stream>>>(W, x, y, M, K, split);
+    const cudaError_t e = launch_kernel(Launch{L.stream, nullptr, true}, gemv_direct_kernel<TYPE>, dim3((M + rows_per_block - 1) / rows_per_block), dim3(256), 0,
+                                        W, x, y, M, K, split);
     L.count();
-    return cudaGetLastError();
+    return e != cudaSuccess ? e : cudaGetLastError();
 }
 
 template <int TYPE>

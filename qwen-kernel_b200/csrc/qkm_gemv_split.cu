@@ -343,11 +343,18 @@ gemv_split_kernel(GemvSplitArgs a) {
         if (++p_kb == kb_n) { p_kb = 0; ++p_round; }
         return true;
     };
+    // Nothing that other kernels write is read or written before the wait, but the table can be filled and the first step's
+    // weights asked into the L2 while the kernel before this one ends.
+    pdl_trigger();
+    if (TYPE == QKM_TYPE_IQ3_XXS)
+        for (uint32_t i = tid; i < 256; i += blockDim.x) sts32(s_lut + i * 4, c_iq3_grid[i]);
+    if (kb_n && tile_of(0) < n_tiles)
+        for (uint32_t o = (lane >> 4) * 128u; o < (uint32_t)G::kBytes; o += 256u)
+            asm volatile("prefetch.global.L2 [%0];" ::"l"(a.W + (size_t)min(tile_of(0) * 16u + (lane & 15u), a.M - 1) * rb + (size_t)kb0 * G::kBytes + o));
+    pdl_wait();
     fetch_next();
 
     // x of this block's slice as B fragments, a warp per (row, 256 columns)
-    if (TYPE == QKM_TYPE_IQ3_XXS)
-        for (uint32_t i = tid; i < 256; i += blockDim.x) sts32(s_lut + i * 4, c_iq3_grid[i]);
     constexpr int kAhead = NT >= 4 ? 4 : NT;   // rows whose loads are in flight together (one at a time would cost a memory latency each)
     for (uint32_t i0 = warp; i0 < kb_n * 2 * NT; i0 += n_warps * kAhead) {
         float v[kAhead][8];
@@ -485,10 +492,12 @@ static cudaError_t gemv_split_launch_nt(const Launch& L, GemvSplitArgs a, uint32
     const uint32_t clusters = want < clusters_max ? want : clusters_max;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(clusters * slices); cfg.blockDim = dim3(warps * 32); cfg.dynamicSmemBytes = smem; cfg.stream = L.stream;
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = slices; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr; cfg.numAttrs = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr; cfg.numAttrs = 2;
     const cudaError_t e = cudaLaunchKernelEx(&cfg, gemv_split_kernel<TYPE, NT>, a);
     L.count();
     return e != cudaSuccess ? e : cudaGetLastError();

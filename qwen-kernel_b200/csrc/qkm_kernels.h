@@ -311,9 +311,9 @@ cudaError_t launch_fold_contrib(const Launch& L, const qkm_dims& d, const float*
 cudaError_t launch_add_rms(const Launch& L, int mode, const float* a, const float* b, const float* c2, const float* w,
                            float* s, float* xn, uint32_t n_rows, uint32_t n, uint32_t n_used, float eps);
 
-// greedy token per row of logits: largest value, lowest index on ties (scratch: argmax_scratch_bytes)
+// greedy token per row of logits: largest value, lowest index on ties (scratch: argmax_scratch_bytes(scratch_rows), zero before the first call)
 size_t argmax_scratch_bytes(uint32_t n_rows);
-cudaError_t launch_argmax(const Launch& L, const float* logits, uint32_t n_rows, uint32_t n, void* scratch, uint32_t* tok);
+cudaError_t launch_argmax(const Launch& L, const float* logits, uint32_t n_rows, uint32_t n, void* scratch, uint32_t scratch_rows, uint32_t* tok);
 
 // ---- expert-parallel exchange helpers (qkm_ep.cu) --------------------------------------------
 // counts[0..n_ranks) rows per destination rank and counts[n_ranks] their sum; send_tok the

@@ -98,11 +98,12 @@ cudaError_t launch_add_rms(const Launch& L, int mode, const float* a, const floa
 // ---- greedy token: argmax over a row of logits ----------------------------------------------------
 // shaders/argmax1.comp:17-40 + argmax2.comp:16-32: the largest value wins, the lower index on
 // ties; a value must exceed -3.4e38 to be taken (so NaN never wins and an all-floor row gives 0).
-// Two launches as in the reference: up to 64 spans per row, then one block per row.
+// One launch: a block per span of a row, the block that finishes a row last (a ticket per row) takes the best of its spans.
+// (Two launches, spans of 4096 and then a block per row, took 10 us for 151,936 logits, mostly latencies.)
 namespace qkm {
 namespace {
 
-constexpr uint32_t kArgSpans = 64;
+constexpr uint32_t kArgSpans = 256, kArgSpan = 1024;   // spans per row at most; logits per span at least
 
 __device__ __forceinline__ void arg_better(float& bv, uint32_t& bi, float v, uint32_t i) {
     if (v > bv || (v == bv && i < bi)) { bv = v; bi = i; }
@@ -124,46 +125,53 @@ __device__ __forceinline__ void arg_block_reduce(float& bv, uint32_t& bi) {
 }
 
 __global__ void __launch_bounds__(256)
-argmax_spans_kernel(const float* __restrict__ logits, uint32_t n, uint32_t span, float* __restrict__ vals,
-                    uint32_t* __restrict__ idxs) {
-    const uint32_t row = blockIdx.y, w = blockIdx.x;
+argmax_kernel(const float* logits, uint32_t n, uint32_t span, float* vals, uint32_t* idxs, uint32_t* tickets, uint32_t* __restrict__ tok) {
+    const uint32_t row = blockIdx.y, w = blockIdx.x, t = threadIdx.x;
+    pdl_wait();
     const float* l = logits + (size_t)row * n;
     const uint32_t start = w * span, end = min(start + span, n);
     float bv = -3.4e38f;
     uint32_t bi = 0xFFFFFFFFu;     // "nothing taken": loses every tie
-    for (uint32_t i = start + threadIdx.x; i < end; i += 256) {
+#pragma unroll 4
+    for (uint32_t i = start + t; i < end; i += 256) {
         const float v = l[i];
         if (v > bv) { bv = v; bi = i; }
     }
     arg_block_reduce(bv, bi);
-    if (threadIdx.x == 0) { vals[row * kArgSpans + w] = bv; idxs[row * kArgSpans + w] = bi; }
-}
-
-__global__ void __launch_bounds__(256)
-argmax_final_kernel(const float* __restrict__ vals, const uint32_t* __restrict__ idxs, uint32_t m, uint32_t* __restrict__ tok) {
-    const uint32_t row = blockIdx.x, t = threadIdx.x;
-    float bv = t < m ? vals[row * kArgSpans + t] : -3.4e38f;
-    uint32_t bi = t < m ? idxs[row * kArgSpans + t] : 0xFFFFFFFFu;
+    __shared__ uint32_t s_last;
+    if (t == 0) {
+        vals[row * kArgSpans + w] = bv; idxs[row * kArgSpans + w] = bi;
+        __threadfence();
+        s_last = atomicAdd(tickets + row, 1u) == gridDim.x - 1 ? 1u : 0u;
+    }
+    __syncthreads();
+    if (!s_last) return;
+    __threadfence();
+    bv = t < gridDim.x ? __ldcg(vals + row * kArgSpans + t) : -3.4e38f;
+    bi = t < gridDim.x ? __ldcg(idxs + row * kArgSpans + t) : 0xFFFFFFFFu;
     arg_block_reduce(bv, bi);
-    if (t == 0) tok[row] = bi == 0xFFFFFFFFu ? 0u : bi;
+    if (t == 0) {
+        tok[row] = bi == 0xFFFFFFFFu ? 0u : bi;
+        tickets[row] = 0;   // ready for the next launch
+    }
 }
 
 }  // namespace
 
-size_t argmax_scratch_bytes(uint32_t n_rows) { return (size_t)n_rows * kArgSpans * 8; }
+size_t argmax_scratch_bytes(uint32_t n_rows) { return (size_t)n_rows * (kArgSpans * 8 + 4); }
 
-cudaError_t launch_argmax(const Launch& L, const float* logits, uint32_t n_rows, uint32_t n, void* scratch, uint32_t* tok) {
+cudaError_t launch_argmax(const Launch& L, const float* logits, uint32_t n_rows, uint32_t n, void* scratch, uint32_t scratch_rows, uint32_t* tok) {
     if (n_rows == 0) return cudaSuccess;
     if (n == 0) return cudaErrorInvalidValue;
-    uint32_t spans = (n + 4095) / 4096;
+    uint32_t spans = (n + kArgSpan - 1) / kArgSpan;
     if (spans > kArgSpans) spans = kArgSpans;
-    const uint32_t span = (n + spans - 1) / spans;
-    float* vals = (float*)scratch;
-    uint32_t* idxs = (uint32_t*)(vals + (size_t)n_rows * kArgSpans);
-    argmax_spans_kernel<<<dim3(spans, n_rows), 256, 0, L.stream>>>(logits, n, span, vals, idxs);
-    argmax_final_kernel<<<n_rows, 256, 0, L.stream>>>(vals, idxs, spans, tok);
-    L.count(2);
-    return cudaGetLastError();
+    uint32_t* tickets = (uint32_t*)scratch;
+    float* vals = (float*)(tickets + scratch_rows);
+    uint32_t* idxs = (uint32_t*)(vals + (size_t)scratch_rows * kArgSpans);
+    const cudaError_t e = launch_kernel(Launch{L.stream, nullptr, true}, argmax_kernel, dim3(spans, n_rows), dim3(256), 0, logits, n, (n + spans - 1) / spans, vals, idxs,
+                                        tickets, tok);
+    L.count();
+    return e != cudaSuccess ? e : cudaGetLastError();
 }
 
 }  // namespace qkm
