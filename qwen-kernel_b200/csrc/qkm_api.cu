@@ -26,6 +26,7 @@ struct qkm_layer_dev {
     // tile-ordered copies for the streaming kernels (NULL where the type has none)
     void* tiles[8] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
     void* router16 = nullptr;  // the router as f16 in the element order of the prefill GEMMs' rows
+    float* router_norm2 = nullptr;   // [n_expert] |router row|^2
     float* w_norm = nullptr;   // [2][resident experts + 1] largest row norm of the gate / up matrices, the shared expert last
     bool tiles_ok = false;   // every tensor has tiles: the tensor-core sequences apply
     bool fused_ok = false;   // and every expert is resident: so does the fused decode sequence
@@ -78,7 +79,7 @@ struct qkm_ctx {
     float* contrib_p = nullptr;       // [max_tokens*(n_used+1)][n_embd]
     MmaItem* mma_items[2] = {nullptr, nullptr};  // gate/up, down
     uint32_t* pos_of = nullptr;       // [max_tokens*(n_used+1)]
-    uint32_t* group_hist = nullptr;   // scratch of the multi-block grouping
+    uint32_t* group_counts = nullptr; // [resident experts] pairs, then [max_tokens*n_used] a pair's number inside its expert
     void* argmax_scratch = nullptr; uint32_t argmax_rows = 0;
     // dense matrices for qkm_dense_gemm (tile-ordered copies) and its scratch, sized on demand
     static constexpr int kDenseSlots = 16;
@@ -341,6 +342,7 @@ extern "C" QKM_API void qkm_close(qkm_ctx* c) {
         for (void* p : l.tiles) if (p) cudaFree(p);
         if (l.router16) cudaFree(l.router16);
         if (l.w_norm) cudaFree(l.w_norm);
+        if (l.router_norm2) cudaFree(l.router_norm2);
     }
     for (auto& dm : c->dense) if (dm.tiles) cudaFree(dm.tiles);
     void* scratch[] = {c->argmax_scratch, c->dense_xb, c->dense_scale, c->sel, c->h, c->route_scratch, c->offsets, c->pairs, c->contrib, c->y2, c->x_stage, c->y_stage,
@@ -348,7 +350,7 @@ extern "C" QKM_API void qkm_close(qkm_ctx* c) {
                        c->items_sh_gu, c->items_sh_dn, c->n_items, c->status, c->route_counter,
                        c->planes8, c->lut_gu, c->lut_dd, c->lut_pf,
                        c->xb, c->xnorm, c->hb, c->hscale, c->contrib_p, c->mma_items[0], c->mma_items[1],
-                       c->pos_of, c->group_hist, c->ep_counts, c->ep_send_tok, c->ep_send_pos};
+                       c->pos_of, c->group_counts, c->ep_counts, c->ep_send_tok, c->ep_send_pos};
     for (void* p : scratch) if (p) cudaFree(p);
     for (auto& o : c->pm_opened) for (void* p : o) if (p) cudaIpcCloseMemHandle(p);
     for (void* p : {(void*)c->pm_xrecv, (void*)c->pm_selrecv, (void*)c->pm_back, (void*)c->pm_partial, (void*)c->pm_xscale}) if (p) cudaFree(p);
@@ -459,7 +461,7 @@ extern "C" QKM_API int qkm_upload_layer(qkm_ctx* c, uint32_t layer, const qkm_la
     }
     // tile-ordered copies for the streaming kernels (same bytes, re-ordered on the device)
     for (void*& p : l.tiles) { if (p) { QKM_CUDA(c, cudaFree(p)); p = nullptr; } }
-    for (void** p : {&l.router16, (void**)&l.w_norm}) { if (*p) { QKM_CUDA(c, cudaFree(*p)); *p = nullptr; } }
+    for (void** p : {&l.router16, (void**)&l.w_norm, (void**)&l.router_norm2}) { if (*p) { QKM_CUDA(c, cudaFree(*p)); *p = nullptr; } }
     l.tiles_ok = l.fused_ok = false;
     if (c->shapes_stream_ok) {
         const qkm_dims& d = c->cfg.dims;
@@ -479,8 +481,10 @@ extern "C" QKM_API int qkm_upload_layer(qkm_ctx* c, uint32_t layer, const qkm_la
         const size_t n_norm = 2 * ((size_t)c->ecount + 1);
         QKM_CUDA(c, cudaMalloc(&l.router16, (size_t)d.n_expert * d.n_embd * 2));
         QKM_CUDA(c, cudaMalloc((void**)&l.w_norm, n_norm * sizeof(float)));
+        QKM_CUDA(c, cudaMalloc((void**)&l.router_norm2, d.n_expert * sizeof(float)));
         QKM_CUDA(c, cudaMemsetAsync(l.w_norm, 0, n_norm * sizeof(float), c->stream));
         cudaError_t e = launch_router_f16(c->L(), w->router_type, l.allocs[0], l.router16, (uint64_t)d.n_expert * d.n_embd);
+        if (e == cudaSuccess) e = launch_row_norm2(c->L(), d, w->router_type, l.allocs[0], l.router_norm2);
         for (int m = 0; m < 2 && e == cudaSuccess; ++m) {
             e = launch_row_norm_max(c->L(), w->gateup_type, l.allocs[2 + m], l.w_norm + m * (c->ecount + 1), c->ecount, d.n_ff, d.n_embd);
             if (e == cudaSuccess) e = launch_row_norm_max(c->L(), QKM_TYPE_Q8_0, l.allocs[5 + m], l.w_norm + m * (c->ecount + 1) + c->ecount, 1, d.n_ff, d.n_embd);
@@ -709,11 +713,23 @@ static int ensure_prefill_scratch(qkm_ctx* c) {
     QKM_CUDA(c, cudaMalloc((void**)&c->mma_items[0], max_tiles * (d.n_ff / 128) * sizeof(MmaItem)));
     QKM_CUDA(c, cudaMalloc((void**)&c->mma_items[1], max_tiles * (d.n_embd / 256) * sizeof(MmaItem)));
     QKM_CUDA(c, cudaMalloc((void**)&c->pos_of, rows * sizeof(uint32_t)));
-    QKM_CUDA(c, cudaMalloc((void**)&c->group_hist, group_wide_scratch_bytes((uint32_t)T, d.n_used, c->ecount)));
+    QKM_CUDA(c, cudaMalloc((void**)&c->group_counts, (c->ecount + T * d.n_used) * sizeof(uint32_t)));
     return QKM_OK;
 }
 
-// The two expert GEMMs over the work lists of launch_mma_plan: c->xb (f16 rows; c->xscale, c->xnorm) -> c->hb -> c->contrib_p.
+// work lists of the GEMMs from c->group_counts; with_routed false: of the shared expert's rows only
+static int expert_plan(qkm_ctx* c, const qkm_sel* sel, uint32_t n, bool with_routed, uint32_t sh_first, uint32_t sh_count) {
+    const qkm_dims& d = c->cfg.dims;
+    GroupPlace g{};
+    g.counts = c->group_counts; g.ranks = c->group_counts + c->ecount; g.sel = sel; g.n_tokens = n; g.n_used = d.n_used; g.n_expert = d.n_expert;
+    g.expert_first = c->efirst; g.expert_count = with_routed ? c->ecount : 0; g.sh_first = sh_first; g.sh_count = sh_count;
+    g.tile = wgemm_rows_per_unit(); g.rt_gu = d.n_ff / 128; g.rt_dn = d.n_embd / 256; g.pairs = c->pairs; g.pos_of = c->pos_of;
+    g.items_gu = c->mma_items[0]; g.items_dn = c->mma_items[1]; g.n_items = c->n_items;
+    QKM_LAUNCH(c, launch_group_place(c->L(), g));
+    return QKM_OK;
+}
+
+// The two expert GEMMs over the work lists of expert_plan: c->xb (f16 rows; c->xscale, c->xnorm) -> c->hb -> c->contrib_p.
 // At most np_max routed pairs and sh_max rows of the shared expert.
 static int expert_gemms(qkm_ctx* c, const qkm_layer_dev& ld, const qkm_sel* sel, uint32_t np_max, uint32_t sh_max) {
     const qkm_dims& d = c->cfg.dims;
@@ -741,12 +757,13 @@ extern "C" QKM_API int qkm_moe_prefill(qkm_ctx* c, uint32_t layer, const float* 
     // ride in the same two launches
     if (int rc = ensure_prefill_scratch(c)) return rc;
     c->prof_begin();
-    QKM_LAUNCH(c, launch_f16_rows(c->L(), x, c->xb, c->xscale, c->xnorm, n, d.n_embd));
-    QKM_LAUNCH(c, launch_route_select(c->L(), d, w.router_type, w.router, w.gate_inp_shexp, x, c->sel, n, c->route_scratch, c->route_scratch_bytes,
-                                      nullptr, nullptr, c->xb, c->xscale, c->status, nullptr, ld.router16));
+    QKM_LAUNCH(c, launch_f16_rows(c->L(), x, c->xb, c->xscale, c->xnorm, n, d.n_embd, c->group_counts, c->ecount));
+    RouteExtra ex;
+    ex.x_f16 = c->xb; ex.x_f16_inv = c->xscale; ex.router_f16 = ld.router16; ex.router_norm2 = ld.router_norm2; ex.status = c->status;
+    ex.counts = c->group_counts; ex.ranks = c->group_counts + c->ecount; ex.expert_first = c->efirst; ex.expert_count = c->ecount;
+    QKM_LAUNCH(c, launch_route_select(c->L(), d, w.router_type, w.router, w.gate_inp_shexp, x, c->sel, n, c->route_scratch, c->route_scratch_bytes, ex));
     c->prof_mark("moe.route");
-    QKM_LAUNCH(c, launch_group_pairs_wide(c->L(), d, c->sel, n, c->offsets, c->pairs, c->efirst, c->ecount, c->group_hist, c->pos_of));
-    QKM_LAUNCH(c, launch_mma_plan(c->L(), d, c->offsets, c->pairs, c->ecount, n, c->mma_items[0], c->mma_items[1], c->n_items, c->pos_of, true, true));
+    if (int rc = expert_plan(c, c->sel, n, true, 0, n)) return rc;
     c->prof_mark("moe.pairs");
     if (int rc = expert_gemms(c, ld, c->sel, n * d.n_used, n)) return rc;
     QKM_LAUNCH(c, launch_fold_pairs(c->L(), d, c->contrib_p, c->pos_of, y, n));
@@ -1056,14 +1073,15 @@ static int ep_route_local(qkm_ctx* c, uint32_t layer, const float* x, uint32_t n
     const qkm_layer_weights& w = ld.w;
     const qkm_dims& d = c->cfg.dims;
     const bool planes = ld.tiles_ok && n <= 64;   // the streamed shared-expert kernels read digit planes
-    const bool tc = ld.tiles_ok && n >= 128;      // tensor-core logits from f16 rows
+    const bool tc = ld.tiles_ok && n > 64;        // tensor-core logits from f16 rows
+    RouteExtra ex;
+    if (planes) { ex.xplanes = c->xplanes; ex.xscale = c->xscale; }
     if (tc) {
         if (int rc = ensure_prefill_scratch(c)) return rc;
         QKM_LAUNCH(c, launch_f16_rows(c->L(), x, c->xb, c->xscale, c->xnorm, n, d.n_embd));
+        ex.x_f16 = c->xb; ex.x_f16_inv = c->xscale; ex.router_f16 = ld.router16; ex.router_norm2 = ld.router_norm2; ex.status = c->status;
     }
-    QKM_LAUNCH(c, launch_route_select(c->L(), d, w.router_type, w.router, w.gate_inp_shexp, x, c->sel, n, c->route_scratch, c->route_scratch_bytes,
-                                      planes ? c->xplanes : nullptr, planes ? c->xscale : nullptr, tc ? c->xb : nullptr,
-                                      tc ? c->xscale : nullptr, c->status, nullptr, ld.router16));
+    QKM_LAUNCH(c, launch_route_select(c->L(), d, w.router_type, w.router, w.gate_inp_shexp, x, c->sel, n, c->route_scratch, c->route_scratch_bytes, ex));
     return QKM_OK;
 }
 
@@ -1126,8 +1144,7 @@ extern "C" QKM_API int qkm_ep_shared(qkm_ctx* c, uint32_t layer, const float* x,
     }
     // tensor-core kernels with an empty routed list: only the shared expert's tiles
     if (int rc = ensure_prefill_scratch(c)) return rc;
-    QKM_CUDA(c, cudaMemsetAsync(c->offsets, 0, sizeof(uint32_t), c->stream));
-    QKM_LAUNCH(c, launch_mma_plan(c->L(), d, c->offsets, c->pairs, 0, n, c->mma_items[0], c->mma_items[1], c->n_items, c->pos_of, true));
+    if (int rc = expert_plan(c, c->sel, n, false, 0, n)) return rc;
     QKM_LAUNCH(c, launch_f16_rows(c->L(), x, c->xb, c->xscale, c->xnorm, n, d.n_embd));
     if (int rc = expert_gemms(c, ld, c->sel, 0, n)) return rc;   // the routed list is empty
     QKM_LAUNCH(c, launch_fold_pairs(c->L(), d, c->contrib_p, c->pos_of, c->y2, n));
@@ -1170,9 +1187,9 @@ static int ep_expert_forward_impl(qkm_ctx* c, uint32_t layer, const float* xrecv
         return QKM_OK;
     }
     if (int rc = ensure_prefill_scratch(c)) return rc;
-    QKM_LAUNCH(c, launch_group_pairs_wide(c->L(), d, selrecv, n_recv, c->offsets, c->pairs, c->efirst, c->ecount, c->group_hist, c->pos_of));
-    QKM_LAUNCH(c, launch_mma_plan(c->L(), d, c->offsets, c->pairs, c->ecount, n_recv, c->mma_items[0], c->mma_items[1], c->n_items, c->pos_of,
-                                  with_shared, true, sh_first, with_shared ? sh_count : 0));
+    QKM_CUDA(c, cudaMemsetAsync(c->group_counts, 0, c->ecount * sizeof(uint32_t), c->stream));
+    QKM_LAUNCH(c, launch_group_rank(c->L(), d, selrecv, n_recv, c->efirst, c->ecount, c->group_counts, c->group_counts + c->ecount));
+    if (int rc = expert_plan(c, selrecv, n_recv, true, with_shared ? sh_first : 0, with_shared ? sh_count : 0)) return rc;
     // the rows as scaled f16: converted here, or already so on arrival (then their scales and norms are gathered)
     if (rows_f16) {
         QKM_LAUNCH(c, launch_ep_row_scales(c->L(), selrecv, c->xscale, n_recv));
@@ -1329,12 +1346,12 @@ extern "C" QKM_API int qkm_ep_push(qkm_ctx* c, uint32_t layer, const float* x, u
     if (n) if (int rc = ep_route_local(c, layer, x, n)) return rc;
     // Layers whose resident experts run on the tensor cores consume the rows as scaled f16: then those
     // travel (half the bytes; every rank decides the same from the layer's types).  The router above
-    // has made them already for 128 tokens and more.
+    // has made them already for more than 64 tokens.
     const qkm_layer_dev& ld = c->layers[layer];
     c->pm_rows_f16 = ld.tiles_ok && c->cfg.dims.n_embd % 8 == 0;
     if (c->pm_rows_f16 && n) {
         const float* inv = c->xscale;
-        if (n < 128) {   // (the router made digit planes, whose scales sit in xscale for the streamed shared expert)
+        if (n <= 64) {   // (the router made digit planes, whose scales sit in xscale for the streamed shared expert)
             if (int rc = ensure_prefill_scratch(c)) return rc;
             QKM_LAUNCH(c, launch_f16_rows(c->L(), x, c->xb, c->pm_xscale, nullptr, n, c->cfg.dims.n_embd));
             inv = c->pm_xscale;

@@ -144,8 +144,9 @@ uint32_t wgemm_rows_per_unit();             // activation rows per unit
 size_t wgemm_table_bytes();
 cudaError_t launch_wgemm_table(const Launch& L, uint8_t* out);
 // x rows as f16 in the kernels' element order (0, 2, 1, 3 in every group of four), scaled per row by a power of two
-// (inv_scale[row] undoes it); norm (optional): the rows' 2-norms
-cudaError_t launch_f16_rows(const Launch& L, const float* x, void* xh, float* inv_scale, float* norm, uint32_t n_rows, uint32_t K);
+// (inv_scale[row] undoes it); norm (optional): the rows' 2-norms; zero (optional): n_zero words set to zero on the way
+cudaError_t launch_f16_rows(const Launch& L, const float* x, void* xh, float* inv_scale, float* norm, uint32_t n_rows, uint32_t K,
+                            uint32_t* zero = nullptr, uint32_t n_zero = 0);
 // rows that arrived as scaled f16 in their own element order: a copy in the kernels' order, and the norms
 cudaError_t launch_f16_rows_in(const Launch& L, const void* in, const float* inv_scale, void* out, float* norm, uint32_t n_rows, uint32_t K);
 // out[e] (zero before) = largest row 2-norm of matrix e (raw ggml rows), rounded up
@@ -173,11 +174,7 @@ cudaError_t launch_wgemm_down(const Launch& L, const qkm_dims& d, uint32_t type,
 cudaError_t launch_dense_gemm(const Launch& L, uint32_t type, const void* tiles, uint32_t M, uint32_t K, const float* x, uint32_t n_rows, float* y,
                               void* xh, float* x_inv_scale, const uint8_t* table, uint32_t n_sms, uint32_t* status);
 
-// ---- qkm_prefill.cu : work lists, router logits and the fold around them
-cudaError_t launch_mma_plan(const Launch& L, const qkm_dims& d, const uint32_t* offsets, uint32_t* pairs,
-                            uint32_t n_expert_local, uint32_t n_tokens, MmaItem* items_gu, MmaItem* items_dn, uint32_t* n_items, uint32_t* pos_of,
-                            bool with_shared = true, bool routed_pos_done = false, uint32_t sh_first = 0,
-                            uint32_t sh_count = 0xFFFFFFFFu /* all rows */);
+// ---- qkm_prefill.cu : router logits and the fold around them
 cudaError_t launch_router_f16(const Launch& L, uint32_t router_type, const void* router, void* out, uint64_t n_elems);
 cudaError_t launch_fold_pairs(const Launch& L, const qkm_dims& d, const float* contrib, const uint32_t* pos_of,
                               float* y, uint32_t n_tokens);
@@ -221,37 +218,69 @@ cudaError_t launch_gemv_stream(const Launch& L, uint32_t type, const void* W, co
                                uint32_t M, uint32_t K, uint32_t n, uint32_t n_sms, uint32_t* status);
 
 // ---- qkm_route.cu
-// x rows as int8 digit planes + per-row scale (the selection kernel can write the same).
-cudaError_t launch_xplanes(const Launch& L, const float* x, uint32_t n_tokens, uint32_t n_embd, int8_t* xplanes, float* xscale,
-                           const float* gis = nullptr, qkm_sel* sel = nullptr);   // gis given: also sel[t].w_shared = sigmoid(gis . x)
-// Optional tail of launch_route_select for decode-sized batches (<= 64 tokens, <= 1024 pairs,
-// f64-logit path): the selection kernel's last block also groups the pairs and cuts the
-// streaming kernels' work lists (what launch_group_plan does), saving a launch.  `counter` is a
-// zero-initialised device word the kernel leaves at zero.  route_select_plans() tells whether
-// a call with these sizes takes that path.
-struct RoutePlan {
-    uint32_t* counter;
-    uint32_t* offsets;
-    uint32_t* pairs;
-    StreamItem* items_gu;
-    StreamItem* items_dn;
-    uint32_t* n_items;
-    uint32_t chunks_gu, chunks_dn, tok_per_item, expert_first, expert_count;
-    uint32_t shared_gate_elsewhere;   // 1: sel[t].w_shared is written by launch_xplanes (given gis); the selection kernel skips x
-};
-bool route_select_plans(const qkm_dims& d, uint32_t n_tokens, size_t scratch_bytes);
-// Scratch the refined router needs: n_tokens * n_expert f32 logits + n_expert f32 row norms,
-// or n_tokens * n_expert f64 logits for the small batches that are ranked in f64 directly.
+// Scratch of launch_route_select: f32 logits (partial sums side by side) and f32 row norms, or f64
+// logits for the small batches that are ranked in f64 directly.
 size_t route_scratch_bytes(uint32_t n_tokens, uint32_t n_expert);
 cudaError_t launch_logits(const Launch& L, const qkm_dims& d, uint32_t router_type, const void* router,
                           const float* x, float* logits, float* row_norm2, uint32_t n_tokens);
 cudaError_t launch_select(const Launch& L, const qkm_dims& d, const float* logits, const float* gis,
                           const float* x, qkm_sel* sel, uint32_t n_tokens);
-cudaError_t launch_route_select(const Launch& L, const qkm_dims& d, uint32_t router_type,
-                                const void* router, const float* gis, const float* x, qkm_sel* sel,
-                                uint32_t n_tokens, void* scratch, size_t scratch_bytes, int8_t* xplanes = nullptr,
-                                float* xscale = nullptr, const void* x_f16 = nullptr, const float* x_f16_inv = nullptr,
-                                uint32_t* status = nullptr, const RoutePlan* plan = nullptr, const void* router_f16 = nullptr);
+// out[e] = |router row e|^2
+cudaError_t launch_row_norm2(const Launch& L, const qkm_dims& d, uint32_t router_type, const void* router, float* norm2);
+struct RouteExtra {                      // all optional
+    int8_t* xplanes = nullptr;           // out: x rows as digit planes [kb][digit][256], and their scales
+    float* xscale = nullptr;
+    const void* x_f16 = nullptr;         // with these four (more than 64 tokens) the logits come from the tensor cores: rows and
+    const float* x_f16_inv = nullptr;    // scales of launch_f16_rows, the router as launch_router_f16 wrote it, its rows' squared norms
+    const void* router_f16 = nullptr;
+    const float* router_norm2 = nullptr;
+    uint32_t* status = nullptr;
+    uint32_t* counts = nullptr;          // in zero, out: pairs per resident expert; ranks[t * n_used + s]: the pair's number inside its expert
+    uint32_t* ranks = nullptr;
+    uint32_t expert_first = 0, expert_count = 0;
+};
+cudaError_t launch_route_select(const Launch& L, const qkm_dims& d, uint32_t router_type, const void* router, const float* gis, const float* x, qkm_sel* sel,
+                                uint32_t n_tokens, void* scratch, size_t scratch_bytes, const RouteExtra& extra = RouteExtra());
+// ---- qkm_select.cu
+struct SelectIn {
+    const void* router;
+    const void* logits;        // f64 (exact), or n_parts times [n_tokens][n_expert] f32 partial sums with an error bound
+    const float *norm2, *gis, *x;
+    int8_t* xplanes; float* xscale;
+    uint32_t *counts, *ranks;
+    uint32_t n_parts, n_norm, expert_first, expert_count;
+    float eps_terms, eps_abs;  // |error of a logit| <= (eps_terms * |router row| + eps_abs) * |x| * 2^-24
+    bool exact;
+};
+cudaError_t launch_select_tokens(const Launch& L, const qkm_dims& d, uint32_t router_type, const SelectIn& in, qkm_sel* sel, uint32_t n_tokens);
+// counts (zero before) and ranks of records that were selected elsewhere
+cudaError_t launch_group_rank(const Launch& L, const qkm_dims& d, const qkm_sel* sel, uint32_t n_tokens, uint32_t expert_first, uint32_t expert_count,
+                              uint32_t* counts, uint32_t* ranks);
+// work lists of the two expert GEMMs from counts and ranks
+struct GroupPlace {
+    const uint32_t *counts, *ranks;
+    const qkm_sel* sel;
+    uint32_t n_tokens, n_used, n_expert, expert_first, expert_count;   // expert_count 0: no routed pairs
+    uint32_t sh_first, sh_count;                                       // rows of the shared expert
+    uint32_t tile, rt_gu, rt_dn;                                       // pairs per unit; units per tile of pairs
+    uint32_t *pairs, *pos_of;
+    MmaItem *items_gu, *items_dn;
+    uint32_t* n_items;         // out: [0], [1] units; [2], [3] zero
+};
+cudaError_t launch_group_place(const Launch& L, const GroupPlace& a);
+#ifdef __CUDACC__
+// Expert id -> index inside the resident range [expert_first, expert_first + expert_count);
+// a result >= expert_count means "not here" (the subtraction wraps for ids below the range).
+// With every expert resident an id past the table is clamped to the last expert, as the
+// reference's moe_group_pairs.comp does; on a shard it marks an empty record that no rank
+// takes (the peer-memory exchange fills unused slots with such records).
+__device__ __forceinline__ uint32_t local_expert_of(uint32_t id, uint32_t n_expert, uint32_t expert_first,
+                                                    uint32_t expert_count) {
+    if (expert_count >= n_expert) return min(id, n_expert - 1) - expert_first;
+    return id < n_expert ? id - expert_first : 0xFFFFFFFFu;
+}
+
+#endif
 // f32 logits from f16 operands on the tensor cores (router_f16 as written by launch_router_f16, x_f16 / x_inv_scale by
 // launch_f16_rows); |error| <= 2^-9 * |router row| * |x|.  Needs n_expert % 128 == 0 and n_embd <= 4096.
 cudaError_t launch_logits_mma(const Launch& L, const qkm_dims& d, const void* router_f16,
@@ -260,20 +289,6 @@ cudaError_t launch_logits_mma(const Launch& L, const qkm_dims& d, const void* ro
 cudaError_t launch_group_pairs(const Launch& L, const qkm_dims& d, const qkm_sel* sel, uint32_t n_tokens,
                                uint32_t* offsets, uint32_t* pairs, uint32_t expert_first,
                                uint32_t expert_count);
-// The same grouping spread over many blocks (large batches).  `hist` is scratch of
-// group_wide_scratch_bytes(); pos_of (optional) gets, for every (token, slot), the position of
-// the pair in `pairs`, or 0xFFFFFFFF when its expert is not resident.
-size_t group_wide_scratch_bytes(uint32_t n_tokens, uint32_t n_used, uint32_t expert_count);
-cudaError_t launch_group_pairs_wide(const Launch& L, const qkm_dims& d, const qkm_sel* sel, uint32_t n_tokens,
-                                    uint32_t* offsets, uint32_t* pairs, uint32_t expert_first, uint32_t expert_count,
-                                    uint32_t* hist, uint32_t* pos_of);
-// group_pairs plus, in the same launch, the work lists of the streaming kernels
-cudaError_t launch_group_plan(const Launch& L, const qkm_dims& d, const qkm_sel* sel, uint32_t n_tokens,
-                              uint32_t* offsets, uint32_t* pairs, uint32_t expert_first, uint32_t expert_count,
-                              StreamItem* items_gu, uint32_t chunks_gu, StreamItem* items_dn,
-                              uint32_t chunks_dn, StreamItem* items_sh_gu, StreamItem* items_sh_dn,
-                              uint32_t tok_per_item, uint32_t* n_items);
-
 // shared-expert work lists: n_items[0] gate/up, n_items[1] down; pairs[n_tokens*n_used + t] = (t<<4)|n_used
 cudaError_t launch_shared_plan(const Launch& L, const qkm_dims& d, uint32_t n_tokens, uint32_t* pairs,
                                StreamItem* items_gu, uint32_t chunks_gu, StreamItem* items_dn,

@@ -1,5 +1,5 @@
-// Batched prefill around the expert GEMMs (qkm_wgemm.cu): the work lists, the router logits on the tensor cores and the
-// slot-order fold of add_rms3_grouped.comp:22-27.
+// Batched prefill around the expert GEMMs (qkm_wgemm.cu): the router logits on the tensor cores and the slot-order fold
+// of add_rms3_grouped.comp:22-27.
 #include <cuda_fp16.h>
 
 #include "qkm_common.cuh"
@@ -13,61 +13,8 @@ namespace qkm {
 namespace pf {
 constexpr int kThreads = 256;                  // copying threads of the logits kernel; one more warp issues the MMAs
 constexpr int kBlock = kThreads + 32;
-constexpr int kNT = 128;                       // pairs per unit of the GEMMs
 constexpr int kTileBytes = 128 * 128;          // 128 rows x 64 f16
 }  // namespace pf
-
-// ---- work list ------------------------------------------------------------------------------------------
-// The units of the two GEMMs: the shared expert's first (its units are the longest: all tokens, 128 at a time), then for
-// every expert its pairs in tiles of kNT, times the 128-row tiles of the gate/up matrices (items_gu) and the 256-row
-// units of the down matrix (items_dn).  The shared expert's "pairs" are tokens, stored after the routed pairs.
-// Also pos_of[t * (n_used+1) + s] = position of pair (t, s) in the grouped order, or
-// 0xFFFFFFFF when the pair is not in the lists (its expert lives on another GPU, or the
-// shared expert is left out with with_shared == 0).
-__global__ void __launch_bounds__(512)
-mma_plan_kernel(const uint32_t* __restrict__ offsets, uint32_t* __restrict__ pairs, uint32_t n_expert_local,
-                uint32_t n_tokens, uint32_t n_used, uint32_t rt_gu, uint32_t rt_dn, uint32_t with_shared,
-                uint32_t routed_pos_done, uint32_t sh_first, uint32_t sh_count,
-                MmaItem* __restrict__ items_gu, MmaItem* __restrict__ items_dn, uint32_t* __restrict__ n_items, uint32_t* __restrict__ pos_of) {
-    __shared__ uint32_t s_scan[512];
-    const uint32_t e = threadIdx.x;
-    const uint32_t np = offsets[n_expert_local];
-    if (!routed_pos_done)   // else the grouping kernels have written every routed (token, slot) entry
-        for (uint32_t i = e; i < n_tokens * (n_used + 1); i += 512) pos_of[i] = 0xFFFFFFFFu;
-    uint32_t tiles = 0, p0 = 0, n = 0;
-    if (e < n_expert_local) { p0 = offsets[e]; n = offsets[e + 1] - p0; tiles = (n + pf::kNT - 1) / pf::kNT; }
-    s_scan[e] = tiles;
-    __syncthreads();
-    for (uint32_t o = 1; o < 512; o <<= 1) {
-        const uint32_t v = e >= o ? s_scan[e - o] : 0;
-        __syncthreads();
-        s_scan[e] += v;
-        __syncthreads();
-    }
-    // the shared expert takes rows [sh_first, sh_first + sh_count): all rows of a single-GPU
-    // chunk, this rank's own tokens among the received rows of an expert-parallel shard
-    const uint32_t sh_n = with_shared ? sh_count : 0;
-    const uint32_t sh_tiles = (sh_n + pf::kNT - 1) / pf::kNT;
-    const uint32_t first = sh_tiles + s_scan[e] - tiles;
-    auto put = [&](uint32_t at, MmaItem it) {
-        for (uint32_t r = 0; r < rt_gu; ++r) { it.rt = (uint16_t)r; items_gu[(size_t)at * rt_gu + r] = it; }
-        for (uint32_t r = 0; r < rt_dn; ++r) { it.rt = (uint16_t)r; items_dn[(size_t)at * rt_dn + r] = it; }
-    };
-    for (uint32_t ti = 0; ti < tiles; ++ti) put(first + ti, MmaItem{(uint16_t)e, 0, p0 + ti * pf::kNT, min((uint32_t)pf::kNT, n - ti * pf::kNT)});
-    for (uint32_t ti = e; ti < sh_tiles; ti += 512) put(ti, MmaItem{(uint16_t)kSharedItem, 0, np + ti * pf::kNT, min((uint32_t)pf::kNT, sh_n - ti * pf::kNT)});
-    if (e == 511) { n_items[0] = (sh_tiles + s_scan[511]) * rt_gu; n_items[1] = (sh_tiles + s_scan[511]) * rt_dn; n_items[2] = n_items[3] = 0; }
-    if (!routed_pos_done)
-        for (uint32_t p = e; p < np; p += 512) {
-            const uint32_t pr = pairs[p];
-            pos_of[(pr >> 4) * (n_used + 1) + (pr & 15u)] = p;
-        }
-    for (uint32_t t = e; t < n_tokens; t += 512) {
-        const uint32_t j = t - sh_first;          // wraps below the range
-        const bool in = j < sh_n;
-        if (in) pairs[np + j] = (t << 4) | n_used;
-        pos_of[t * (n_used + 1) + n_used] = in ? np + j : 0xFFFFFFFFu;
-    }
-}
 
 // ---- router logits on the tensor cores -----------------------------------------------------------------
 // logits[t][e] = router[e] . x[t] with f16 operands (router rows as written by router_f16_kernel, x rows by
@@ -114,6 +61,8 @@ logits_mma_kernel(const uint8_t* __restrict__ router, const __half* __restrict__
     }
     if (warp == 0) { umma::tmem_alloc(smem_addr(&s_tmem), 128); umma::tmem_relinquish(); }
     umma::fence_before_sync();
+    pdl_trigger();
+    pdl_wait();
     __syncthreads();
     umma::fence_after_sync();
     const uint32_t tmem = s_tmem;
@@ -154,7 +103,8 @@ logits_mma_kernel(const uint8_t* __restrict__ router, const __half* __restrict__
                 }
                 cp_async_commit();
             };
-            for (uint32_t ks = 0; ks < (uint32_t)kLgDepth && ks < KS; ++ks) issue(ks);
+            for (uint32_t ks = 0; ks < (uint32_t)kLgDepth; ++ks)
+                if (ks < KS) issue(ks); else cp_async_commit();
             for (uint32_t ks = 0; ks < KS; ++ks) {
                 if (ks + kLgDepth < KS) issue(ks + kLgDepth); else cp_async_commit();   // keep the group count in step
                 cp_async_wait<kLgDepth>();          // the copies of step ks have landed
@@ -191,9 +141,10 @@ cudaError_t launch_logits_mma(const Launch& L, const qkm_dims& d, const void* ro
     const size_t smem = (size_t)kLgStages * 2 * pf::kTileBytes + 1024;
     const dim3 grid((n_tokens + 127) / 128, d.n_expert / 128, splits);
     if (const cudaError_t e = allow_dynamic_smem<logits_mma_kernel>((int)smem)) return e;
-    logits_mma_kernel<<<grid, pf::kBlock, smem, L.stream>>>((const uint8_t*)router_f16, (const __half*)x_f16, x_inv_scale, logits, d.n_expert, d.n_embd, n_tokens, status);
+    const cudaError_t e = launch_kernel(Launch{L.stream, nullptr, true}, logits_mma_kernel, grid, dim3(pf::kBlock), smem, (const uint8_t*)router_f16, (const __half*)x_f16,
+                                        x_inv_scale, logits, d.n_expert, d.n_embd, n_tokens, status);
     L.count();
-    return cudaGetLastError();
+    return e != cudaSuccess ? e : cudaGetLastError();
 }
 
 // router rows as f16 in the element order of the f16 activation rows (0, 2, 1, 3 in every group of four)
@@ -216,8 +167,10 @@ cudaError_t launch_router_f16(const Launch& L, uint32_t router_type, const void*
 }
 
 // ---- fold: y[t] = sum over slots (in order) of contrib[pos(t,s)], then the shared expert -----------------
-__global__ void fold_pairs_kernel(const float* __restrict__ contrib, const uint32_t* __restrict__ pos_of,
+__global__ void fold_pairs_kernel(const float* contrib, const uint32_t* pos_of,
                                   float* __restrict__ y, uint32_t n_used, uint32_t n_embd) {
+    pdl_trigger();
+    pdl_wait();
     const uint32_t t = blockIdx.y;
     const uint32_t o = (blockIdx.x * blockDim.x + threadIdx.x) * 4;
     if (o >= n_embd) return;
@@ -255,25 +208,13 @@ __global__ void fold_pairs_peer_kernel(const float* __restrict__ contrib, const 
 }
 
 // ---- launchers ---------------------------------------------------------------------------------------------
-cudaError_t launch_mma_plan(const Launch& L, const qkm_dims& d, const uint32_t* offsets, uint32_t* pairs,
-                            uint32_t n_expert_local, uint32_t n_tokens, MmaItem* items_gu, MmaItem* items_dn, uint32_t* n_items, uint32_t* pos_of,
-                            bool with_shared, bool routed_pos_done, uint32_t sh_first, uint32_t sh_count) {
-    if (n_expert_local > 512) return cudaErrorInvalidValue;
-    if (sh_count == 0xFFFFFFFFu) { sh_first = 0; sh_count = n_tokens; }
-    if (sh_first > n_tokens || sh_count > n_tokens - sh_first) return cudaErrorInvalidValue;
-    mma_plan_kernel<<<1, 512, 0, L.stream>>>(offsets, pairs, n_expert_local, n_tokens, d.n_used, d.n_ff / 128,
-                                             d.n_embd / 256, with_shared ? 1u : 0u, routed_pos_done ? 1u : 0u, sh_first, sh_count, items_gu, items_dn, n_items, pos_of);
-    L.count();
-    return cudaGetLastError();
-}
-
 cudaError_t launch_fold_pairs(const Launch& L, const qkm_dims& d, const float* contrib, const uint32_t* pos_of,
                               float* y, uint32_t n_tokens) {
     if (n_tokens == 0) return cudaSuccess;
     const dim3 grid((d.n_embd / 4 + 255) / 256, n_tokens);
-    fold_pairs_kernel<<<grid, 256, 0, L.stream>>>(contrib, pos_of, y, d.n_used, d.n_embd);
+    const cudaError_t e = launch_kernel(Launch{L.stream, nullptr, true}, fold_pairs_kernel, grid, dim3(256), 0, contrib, pos_of, y, d.n_used, d.n_embd);
     L.count();
-    return cudaGetLastError();
+    return e != cudaSuccess ? e : cudaGetLastError();
 }
 
 cudaError_t launch_fold_pairs_peer(const Launch& L, const qkm_dims& d, const float* contrib, const uint32_t* pos_of,

@@ -266,8 +266,6 @@ wgemm_kernel(const WgemmArgs a, const __grid_constant__ CUtensorMap rows_map) {
     const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31u;
     const uint32_t KB = a.K / 256, RT16 = a.rows / 16;
     const uint32_t row_units = MODE == wg::kGateUp ? a.rows / 128 : (a.rows / 128 + 1) / 2;
-    const uint32_t n_units = MODE == wg::kDense ? (a.n_dense + wg::kNT - 1) / wg::kNT * row_units : *a.n_items;
-    if (blockIdx.x >= n_units) return;
     {   // the fixed addresses must lie inside the dynamic area
         const uint32_t dyn_base = smem_addr(smem_dyn);
         uint32_t dyn_size;
@@ -296,8 +294,11 @@ wgemm_kernel(const WgemmArgs a, const __grid_constant__ CUtensorMap rows_map) {
     }
     if (warp == 0) { umma::tmem_alloc(smem_addr(&s_tmem), 512); umma::tmem_relinquish(); }
     umma::fence_before_sync();
+    pdl_trigger();
+    pdl_wait();   // up to here nothing depended on the kernel before
     __syncthreads();
     umma::fence_after_sync();
+    const uint32_t n_units = MODE == wg::kDense ? (a.n_dense + wg::kNT - 1) / wg::kNT * row_units : *a.n_items;
     const uint32_t tmem = s_tmem;
     bool timed_out = false;
     auto wait_bar = [&](uint32_t b, uint32_t parity) -> bool { return timed_out || mbar_wait_timed(b, parity); };   // a thread waits out the limit once at most
@@ -745,8 +746,13 @@ wgemm_kernel(const WgemmArgs a, const __grid_constant__ CUtensorMap rows_map) {
 // x -> f16 rows in the kernels' element order, each scaled by a power of two so that max|x| lands in [2^13, 2^14), the
 // inverse scale and (optional) the row's 2-norm.  A warp per row: two passes over it, the second from L1.
 __global__ void __launch_bounds__(256)
-f16_rows_kernel(const float* __restrict__ x, __half* __restrict__ xh, float* __restrict__ inv_scale, float* __restrict__ norm, uint32_t n_rows, uint32_t K) {
+f16_rows_kernel(const float* x, __half* __restrict__ xh, float* __restrict__ inv_scale, float* __restrict__ norm, uint32_t n_rows, uint32_t K, uint32_t* __restrict__ zero,
+                uint32_t n_zero) {
     const uint32_t t = (blockIdx.x * 256u + threadIdx.x) >> 5, lane = threadIdx.x & 31u;
+    pdl_trigger();
+    pdl_wait();
+    if (blockIdx.x == 0)
+        for (uint32_t i = threadIdx.x; i < n_zero; i += 256) zero[i] = 0;
     if (t >= n_rows) return;
     const float4* xt = reinterpret_cast<const float4*>(x + (size_t)t * K);
     float m = 0.f, ss = 0.f;
@@ -773,12 +779,13 @@ f16_rows_kernel(const float* __restrict__ x, __half* __restrict__ xh, float* __r
         if (norm) norm[t] = sqrtf(ss);
     }
 }
-cudaError_t launch_f16_rows(const Launch& L, const float* x, void* xh, float* inv_scale, float* norm, uint32_t n_rows, uint32_t K) {
+cudaError_t launch_f16_rows(const Launch& L, const float* x, void* xh, float* inv_scale, float* norm, uint32_t n_rows, uint32_t K, uint32_t* zero, uint32_t n_zero) {
     if (n_rows == 0) return cudaSuccess;
     if (K % 4) return cudaErrorInvalidValue;
-    f16_rows_kernel<<<(n_rows + 7) / 8, 256, 0, L.stream>>>(x, (__half*)xh, inv_scale, norm, n_rows, K);
+    const cudaError_t e = launch_kernel(Launch{L.stream, nullptr, true}, f16_rows_kernel, dim3((n_rows + 7) / 8), dim3(256), 0, x, (__half*)xh, inv_scale, norm, n_rows, K,
+                                        zero, n_zero);
     L.count();
-    return cudaGetLastError();
+    return e != cudaSuccess ? e : cudaGetLastError();
 }
 // rows that arrived as scaled f16 (expert parallel): their 2-norms, and a copy in the kernels' element order
 __global__ void __launch_bounds__(256)
@@ -901,9 +908,10 @@ static cudaError_t wgemm_launch(const Launch& L, const WgemmArgs& a, const void*
     if (const cudaError_t e = allow_dynamic_smem<wgemm_kernel<FMT, MODE>>((int)wg::smem_end<FMT>())) return e;
     CUtensorMap map{};
     if (((uintptr_t)rows & 15u) || (MODE != wg::kGateUp && !rows_tensor_map(&map, rows, n_rows, a.K))) return cudaErrorInvalidValue;
-    wgemm_kernel<FMT, MODE><<<max_units < n_sms ? max_units : n_sms, wg::kThreads, wg::smem_end<FMT>(), L.stream>>>(a, map);
+    const cudaError_t e = launch_kernel(Launch{L.stream, nullptr, true}, wgemm_kernel<FMT, MODE>, dim3(max_units < n_sms ? max_units : n_sms), dim3(wg::kThreads),
+                                        wg::smem_end<FMT>(), a, map);
     L.count();
-    return cudaGetLastError();
+    return e != cudaSuccess ? e : cudaGetLastError();
 }
 
 uint32_t wgemm_rows_per_unit() { return wg::kNT; }
