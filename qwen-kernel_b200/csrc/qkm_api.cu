@@ -26,7 +26,7 @@ struct qkm_layer_dev {
     // tile-ordered copies for the streaming kernels (NULL where the type has none)
     void* tiles[8] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
     void* router16 = nullptr;  // the router as f16 in the element order of the prefill GEMMs' rows
-    float* router_norm2 = nullptr;   // [n_expert] |router row|^2
+    float* router_norm2 = nullptr;   // largest |router row|^2
     float* w_norm = nullptr;   // [2][resident experts + 1] largest row norm of the gate / up matrices, the shared expert last
     bool tiles_ok = false;   // every tensor has tiles: the tensor-core sequences apply
     bool fused_ok = false;   // and every expert is resident: so does the fused decode sequence
@@ -481,10 +481,11 @@ extern "C" QKM_API int qkm_upload_layer(qkm_ctx* c, uint32_t layer, const qkm_la
         const size_t n_norm = 2 * ((size_t)c->ecount + 1);
         QKM_CUDA(c, cudaMalloc(&l.router16, (size_t)d.n_expert * d.n_embd * 2));
         QKM_CUDA(c, cudaMalloc((void**)&l.w_norm, n_norm * sizeof(float)));
-        QKM_CUDA(c, cudaMalloc((void**)&l.router_norm2, d.n_expert * sizeof(float)));
+        QKM_CUDA(c, cudaMalloc((void**)&l.router_norm2, sizeof(float)));
+        QKM_CUDA(c, cudaMemsetAsync(l.router_norm2, 0, sizeof(float), c->stream));
         QKM_CUDA(c, cudaMemsetAsync(l.w_norm, 0, n_norm * sizeof(float), c->stream));
         cudaError_t e = launch_router_f16(c->L(), w->router_type, l.allocs[0], l.router16, (uint64_t)d.n_expert * d.n_embd);
-        if (e == cudaSuccess) e = launch_row_norm2(c->L(), d, w->router_type, l.allocs[0], l.router_norm2);
+        if (e == cudaSuccess) e = launch_row_norm2(c->L(), d, w->router_type, l.allocs[0], nullptr, l.router_norm2);
         for (int m = 0; m < 2 && e == cudaSuccess; ++m) {
             e = launch_row_norm_max(c->L(), w->gateup_type, l.allocs[2 + m], l.w_norm + m * (c->ecount + 1), c->ecount, d.n_ff, d.n_embd);
             if (e == cudaSuccess) e = launch_row_norm_max(c->L(), QKM_TYPE_Q8_0, l.allocs[5 + m], l.w_norm + m * (c->ecount + 1) + c->ecount, 1, d.n_ff, d.n_embd);

@@ -225,13 +225,13 @@ cudaError_t launch_logits(const Launch& L, const qkm_dims& d, uint32_t router_ty
                           const float* x, float* logits, float* row_norm2, uint32_t n_tokens);
 cudaError_t launch_select(const Launch& L, const qkm_dims& d, const float* logits, const float* gis,
                           const float* x, qkm_sel* sel, uint32_t n_tokens);
-// out[e] = |router row e|^2
-cudaError_t launch_row_norm2(const Launch& L, const qkm_dims& d, uint32_t router_type, const void* router, float* norm2);
+// norm2[e] = |router row e|^2; largest (zero before): their maximum; either may be NULL
+cudaError_t launch_row_norm2(const Launch& L, const qkm_dims& d, uint32_t router_type, const void* router, float* norm2, float* largest);
 struct RouteExtra {                      // all optional
     int8_t* xplanes = nullptr;           // out: x rows as digit planes [kb][digit][256], and their scales
     float* xscale = nullptr;
     const void* x_f16 = nullptr;         // with these four (more than 64 tokens) the logits come from the tensor cores: rows and
-    const float* x_f16_inv = nullptr;    // scales of launch_f16_rows, the router as launch_router_f16 wrote it, its rows' squared norms
+    const float* x_f16_inv = nullptr;    // scales of launch_f16_rows, the router as launch_router_f16 wrote it, its rows' largest squared norm
     const void* router_f16 = nullptr;
     const float* router_norm2 = nullptr;
     uint32_t* status = nullptr;

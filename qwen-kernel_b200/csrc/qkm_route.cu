@@ -204,7 +204,7 @@ logits_gemm_kernel(const uint8_t* __restrict__ router, const float* __restrict__
 // |router row|^2, one warp per row
 template <int TYPE>
 __global__ void __launch_bounds__(256)
-row_norm2_kernel(const uint8_t* __restrict__ router, float* __restrict__ row_norm2, uint32_t n_expert, uint32_t K) {
+row_norm2_kernel(const uint8_t* __restrict__ router, float* __restrict__ row_norm2, uint32_t* __restrict__ max_bits, uint32_t n_expert, uint32_t K) {
     const uint32_t e = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31u;
     if (e >= n_expert) return;
     const uint8_t* row = router + (size_t)e * row_bytes(TYPE, K);
@@ -216,13 +216,14 @@ row_norm2_kernel(const uint8_t* __restrict__ router, float* __restrict__ row_nor
         for (int i = 0; i < 8; ++i) nrm += w[i] * w[i];
     }
     nrm = warp_sum(nrm);
-    if (lane == 0) row_norm2[e] = nrm;
+    if (lane == 0 && row_norm2) row_norm2[e] = nrm;
+    if (lane == 0 && max_bits) atomicMax(max_bits, __float_as_uint(nrm));   // non-negative floats order like their bits, a NaN above them
 }
 
-cudaError_t launch_row_norm2(const Launch& L, const qkm_dims& d, uint32_t router_type, const void* router, float* norm2) {
+cudaError_t launch_row_norm2(const Launch& L, const qkm_dims& d, uint32_t router_type, const void* router, float* norm2, float* largest) {
     const uint8_t* r = (const uint8_t*)router;
-    if (router_type == QKM_TYPE_F32) row_norm2_kernel<QKM_TYPE_F32><<<(d.n_expert + 7) / 8, 256, 0, L.stream>>>(r, norm2, d.n_expert, d.n_embd);
-    else if (router_type == QKM_TYPE_F16) row_norm2_kernel<QKM_TYPE_F16><<<(d.n_expert + 7) / 8, 256, 0, L.stream>>>(r, norm2, d.n_expert, d.n_embd);
+    if (router_type == QKM_TYPE_F32) row_norm2_kernel<QKM_TYPE_F32><<<(d.n_expert + 7) / 8, 256, 0, L.stream>>>(r, norm2, (uint32_t*)largest, d.n_expert, d.n_embd);
+    else if (router_type == QKM_TYPE_F16) row_norm2_kernel<QKM_TYPE_F16><<<(d.n_expert + 7) / 8, 256, 0, L.stream>>>(r, norm2, (uint32_t*)largest, d.n_expert, d.n_embd);
     else return cudaErrorInvalidValue;
     L.count();
     return cudaGetLastError();
@@ -376,7 +377,7 @@ cudaError_t launch_route_select(const Launch& L, const qkm_dims& d, uint32_t rou
         in.eps_abs = 2.f * sqrtf((float)d.n_embd);                                   // 2^-25 per router element that f16 flushes
     } else if (n_tokens >= 1024) {   // many tokens: tiled GEMM, one chain of n_embd additions per logit
         const dim3 grid((d.n_expert + 63) / 64, (n_tokens + 63) / 64);
-        if (const cudaError_t e = launch_row_norm2(L, d, router_type, router, norm2)) return e;
+        if (const cudaError_t e = launch_row_norm2(L, d, router_type, router, norm2, nullptr)) return e;
         if (router_type == QKM_TYPE_F32) logits_gemm_kernel<QKM_TYPE_F32><<<grid, 256, 0, L.stream>>>(r, x, logits, d.n_expert, d.n_embd, n_tokens);
         else logits_gemm_kernel<QKM_TYPE_F16><<<grid, 256, 0, L.stream>>>(r, x, logits, d.n_expert, d.n_embd, n_tokens);
         L.count();
