@@ -24,15 +24,15 @@ constexpr int kTailMaxPerThread = 8;   // float4 units per thread: n <= 256 * 8 
 // MODE 0: a + b;  1: a + b + c2;  2: a + (sum over slots of routed) + c2
 template <int MODE>
 __global__ void __launch_bounds__(kTailThreads)
-add_rms_kernel(const float* __restrict__ a, const float* __restrict__ b, const float* __restrict__ c2,
-               const float* __restrict__ w, float* __restrict__ s, float* __restrict__ xn, uint32_t n,
-               uint32_t n_used, float eps) {
+add_rms_kernel(const float* a, const float* b, const float* c2, const float* w, float* s, float* xn, uint32_t n, uint32_t n_used, float eps) {
     __shared__ float s_red[kTailThreads / 32];
     const uint32_t row = blockIdx.x, tid = threadIdx.x, n4 = n / 4;
     const float4* a4 = reinterpret_cast<const float4*>(a + (size_t)row * n);
     const float4* c4 = MODE >= 1 ? reinterpret_cast<const float4*>(c2 + (size_t)row * n) : nullptr;
     float4 v[kTailMaxPerThread];
     float ss = 0.f;
+    pdl_trigger();
+    pdl_wait();   // the launch overlaps the end of the kernel before
 #pragma unroll
     for (int i = 0; i < kTailMaxPerThread; ++i) {
         const uint32_t u = tid + i * kTailThreads;
@@ -53,11 +53,13 @@ add_rms_kernel(const float* __restrict__ a, const float* __restrict__ b, const f
                 const float4 q = c4[u];
                 x.x += q.x; x.y += q.y; x.z += q.z; x.w += q.w;
             }
-            reinterpret_cast<float4*>(s + (size_t)row * n)[u] = x;
             ss += x.x * x.x; ss += x.y * x.y; ss += x.z * x.z; ss += x.w * x.w;
             v[i] = x;
         }
     }
+#pragma unroll
+    for (int i = 0; i < kTailMaxPerThread; ++i)   // (after all loads: s may be a)
+        if (tid + i * kTailThreads < n4) reinterpret_cast<float4*>(s + (size_t)row * n)[tid + i * kTailThreads] = v[i];
     ss = warp_sum(ss);
     if ((tid & 31u) == 0) s_red[tid >> 5] = ss;
     __syncthreads();
@@ -83,14 +85,16 @@ cudaError_t launch_add_rms(const Launch& L, int mode, const float* a, const floa
                            float* s, float* xn, uint32_t n_rows, uint32_t n, uint32_t n_used, float eps) {
     if (n_rows == 0) return cudaSuccess;
     if (n == 0 || n % 4 || n > kTailThreads * kTailMaxPerThread * 4) return cudaErrorInvalidValue;
+    const Launch P{L.stream, nullptr, true};
+    cudaError_t e = cudaErrorInvalidValue;
     switch (mode) {
-        case 0: add_rms_kernel<0><<<n_rows, kTailThreads, 0, L.stream>>>(a, b, c2, w, s, xn, n, n_used, eps); break;
-        case 1: add_rms_kernel<1><<<n_rows, kTailThreads, 0, L.stream>>>(a, b, c2, w, s, xn, n, n_used, eps); break;
-        case 2: add_rms_kernel<2><<<n_rows, kTailThreads, 0, L.stream>>>(a, b, c2, w, s, xn, n, n_used, eps); break;
-        default: return cudaErrorInvalidValue;
+        case 0: e = launch_kernel(P, add_rms_kernel<0>, dim3(n_rows), dim3(kTailThreads), 0, a, b, c2, w, s, xn, n, n_used, eps); break;
+        case 1: e = launch_kernel(P, add_rms_kernel<1>, dim3(n_rows), dim3(kTailThreads), 0, a, b, c2, w, s, xn, n, n_used, eps); break;
+        case 2: e = launch_kernel(P, add_rms_kernel<2>, dim3(n_rows), dim3(kTailThreads), 0, a, b, c2, w, s, xn, n, n_used, eps); break;
+        default: return e;
     }
     L.count();
-    return cudaGetLastError();
+    return e != cudaSuccess ? e : cudaGetLastError();
 }
 
 }  // namespace qkm
