@@ -378,13 +378,12 @@ gemv_tile_kernel(const uint8_t* __restrict__ W, const float* __restrict__ x, flo
     }
     __syncthreads();
     const uint32_t my_tiles = blockIdx.x < n_tiles ? (n_tiles - blockIdx.x + gridDim.x - 1) / gridDim.x : 0u;
-    auto issue = [&](uint32_t i) {   // tile number i of this block into stage i % n_stages: one copy; thread 0
-        const uint32_t s = i % n_stages;
+    auto issue = [&](uint32_t i, uint32_t s) {   // tile number i of this block into stage s = i % n_stages: one copy; thread 0
         mbar_expect_tx(bar_full + 8 * s, gq::kRows * rb);
         bulk_g2s(stage0 + s * stage_bytes, W + (size_t)(blockIdx.x + i * gridDim.x) * gq::kRows * rb, gq::kRows * rb, bar_full + 8 * s);
     };
     if (tid == 0)
-        for (uint32_t i = 0; i + 1 < n_stages && i < my_tiles; ++i) issue(i);
+        for (uint32_t i = 0; i + 1 < n_stages && i < my_tiles; ++i) issue(i, i);
 
     // x as digit planes (the first tiles are on their way meanwhile)
     {
@@ -443,43 +442,37 @@ gemv_tile_kernel(const uint8_t* __restrict__ W, const float* __restrict__ x, flo
     const float xscale = s_scale;
     const bool odd = TYPE == QKM_TYPE_Q6_K && (warp & 1u) != 0;   // 210 * warp is 2 mod 4 for odd warps (K / 256 is even: rows start on word boundaries)
 
+    uint32_t c_stage = 0, c_phase = 0, p_stage = n_stages - 1, p_phase = 0;   // next tile's stage, and that of the tile refilled meanwhile
     uint32_t buf = 0;
     for (uint32_t i0 = 0; i0 < my_tiles; i0 += gq::kGroup) {
         const uint32_t in_group = min((uint32_t)gq::kGroup, my_tiles - i0);
-        float acc[gq::kGroup][2];
-#pragma unroll
-        for (int q = 0; q < gq::kGroup; ++q) {
-            acc[q][0] = acc[q][1] = 0.f;
-            const uint32_t i = i0 + q;
-            if (i < my_tiles) {   // block-uniform
-                const uint32_t s = i % n_stages;
-                if (tid == 0 && i + n_stages - 1 < my_tiles) {   // refill the stage the block left one tile ago
-                    const uint32_t j = i + n_stages - 1, sj = j % n_stages;
-                    if (j >= n_stages && !mbar_wait_bounded(bar_empty + 8 * sj, ((j / n_stages) - 1) & 1u)) timed_out = true;
-                    issue(j);
-                }
-                if (!mbar_wait_bounded(bar_full + 8 * s, (i / n_stages) & 1u)) timed_out = true;
-                const uint32_t blk0 = stage0 + s * stage_bytes + g * rb + kBlockBytes * warp, blk1 = blk0 + 8u * rb;
-                float f0, f1;
-                uint32_t b0[8], b1[8];
-#pragma unroll
-                for (int sb = 0; sb < 8; ++sb) { b0[sb] = bq[sb]; b1[sb] = bq[8 + sb]; }
-                if (TYPE == QKM_TYPE_IQ4_XS) {
-                    iq4_tile(blk0, blk1, t, b0, b1, plane_w, f0, f1);
-                } else if (odd) {
-                    q6k_tile<true>(blk0, blk1, t, b0, b1, f0, f1);
-                } else {
-                    q6k_tile<false>(blk0, blk1, t, b0, b1, f0, f1);
-                }
-                __syncwarp();
-                if (lane == 0) mbar_arrive(bar_empty + 8 * s);
-                acc[q][0] = f0; acc[q][1] = f1;
-            }
-        }
         float* rw = red + (size_t)buf * red_floats + (size_t)warp * gq::kGroup * gq::kRows;
+        // (not unrolled: four tiles' code, twice for the two alignments, does not stay in the instruction caches)
+#pragma unroll 1
+        for (uint32_t q = 0; q < in_group; ++q) {
+            const uint32_t i = i0 + q;
+            if (tid == 0 && i + n_stages - 1 < my_tiles) {   // refill the stage the block left one tile ago
+                const uint32_t j = i + n_stages - 1, sj = p_stage;
+                if (j >= n_stages && !mbar_wait_bounded(bar_empty + 8 * sj, p_phase ^ 1u)) timed_out = true;
+                issue(j, sj);
+            }
+            if (++p_stage == n_stages) { p_stage = 0; p_phase ^= 1u; }
+            if (!mbar_wait_bounded(bar_full + 8 * c_stage, c_phase)) timed_out = true;
+            const uint32_t blk0 = stage0 + c_stage * stage_bytes + g * rb + kBlockBytes * warp, blk1 = blk0 + 8u * rb;
+            float v0, v1;
+            uint32_t b0[8], b1[8];
 #pragma unroll
-        for (int q = 0; q < gq::kGroup; ++q) {
-            float v0 = acc[q][0], v1 = acc[q][1];
+            for (int sb = 0; sb < 8; ++sb) { b0[sb] = bq[sb]; b1[sb] = bq[8 + sb]; }
+            if (TYPE == QKM_TYPE_IQ4_XS) {
+                iq4_tile(blk0, blk1, t, b0, b1, plane_w, v0, v1);
+            } else if (odd) {
+                q6k_tile<true>(blk0, blk1, t, b0, b1, v0, v1);
+            } else {
+                q6k_tile<false>(blk0, blk1, t, b0, b1, v0, v1);
+            }
+            __syncwarp();
+            if (lane == 0) mbar_arrive(bar_empty + 8 * c_stage);
+            if (++c_stage == n_stages) { c_stage = 0; c_phase ^= 1u; }
             v0 += __shfl_xor_sync(0xFFFFFFFFu, v0, 1); v1 += __shfl_xor_sync(0xFFFFFFFFu, v1, 1);
             if (TYPE == QKM_TYPE_Q6_K) {   // all four lanes of a row hold a share
                 v0 += __shfl_xor_sync(0xFFFFFFFFu, v0, 2); v1 += __shfl_xor_sync(0xFFFFFFFFu, v1, 2);

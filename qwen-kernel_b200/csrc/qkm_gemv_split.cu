@@ -444,14 +444,17 @@ gemv_split_kernel(GemvSplitArgs a) {
             const uint32_t w = o / (a.n * 16u), row = (o >> 4) - w * a.n, r = o & 15u;
             const uint32_t m = (cluster + n_clusters * (w + n_warps * round)) * 16u + r;
             if (m < a.M) {
-                float v = 0.f;
-                for (uint32_t q = 0; q < n_ctas; ++q) {   // slice order
-                    uint32_t remote;
-                    float p;
-                    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(part + o * 4u), "r"(q));
-                    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(p) : "r"(remote) : "memory");
-                    v += p;
-                }
+                float p[8], v = 0.f;   // at most eight slices; all reads under way before the first is used
+#pragma unroll
+                for (uint32_t q = 0; q < 8; ++q)
+                    if (q < n_ctas) {
+                        uint32_t remote;
+                        asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(part + o * 4u), "r"(q));
+                        asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(p[q]) : "r"(remote) : "memory");
+                    }
+#pragma unroll
+                for (uint32_t q = 0; q < 8; ++q)   // slice order
+                    if (q < n_ctas) v += p[q];
                 a.y[(size_t)row * a.M + m] = v;
             }
         }
