@@ -200,14 +200,15 @@ __device__ __forceinline__ void make_iq4(uint32_t (&o)[16], const uint32_t (&w)[
 }
 
 // four unsigned bytes v -> f16 pairs (bytes 0, 2) and (1, 3) of 1024 + byte, minus `bias`, times the scale
-__device__ __forceinline__ void bytes_to_h2(uint32_t v, __half2 bias, const Scale2& s, uint32_t& p02, uint32_t& p13) {
+template <class S>
+__device__ __forceinline__ void bytes_to_h2(uint32_t v, __half2 bias, const S& s, uint32_t& p02, uint32_t& p13) {
     p02 = mul_h2(sub_h2((v & 0x00FF00FFu) | 0x64006400u, bias), s);
     p13 = mul_h2(sub_h2(((v >> 8) & 0x00FF00FFu) | 0x64006400u, bias), s);
 }
 
 // Q8_0: q0, q1 = the row's 32 quant bytes of a block (tile order: words t of elements 4t.. and 16 + 4t.. alternate)
-__device__ __forceinline__ void make_q8(uint32_t (&o)[16], const uint4& q0, const uint4& q1, float d) {
-    const Scale2 s = split_scale(d);
+template <class S>
+__device__ __forceinline__ void make_q8(uint32_t (&o)[16], const uint4& q0, const uint4& q1, const S& s) {
     const __half2 bias = __float2half2_rn(1152.f);   // 1024 + 128: the bytes have their top bit flipped
     const uint32_t w[8] = {q0.x, q0.z, q1.x, q1.z, q0.y, q0.w, q1.y, q1.w};   // elements 4m .. 4m+3
 #pragma unroll
@@ -339,6 +340,8 @@ wgemm_kernel(const WgemmArgs a, const __grid_constant__ CUtensorMap rows_map) {
         const uint32_t tab_c = wg::kTab + (FMT == QKM_TYPE_IQ3_XXS ? (lane & 15u) * 8u : 128u + lane * 4u);
         if (FMT == QKM_TYPE_IQ3_XXS || FMT == QKM_TYPE_IQ4_XS)
             if (!wait_bar(bar_tab, 0)) timed_out = true;
+        // dense: scale and product rounded to f16 (two roundings of 2^-12, a fifth fewer instructions); experts: one rounding that counts
+        auto weight_scale = [](float v) { if constexpr (MODE == wg::kDense) return __float2half2_rn(v); else return split_scale(v); };
         uint32_t round0 = 0, wcnt = 0, qcnt = 0;   // stage rounds before this unit; blocks and Q8_0 slots consumed
         MmaItem it;
         for (uint32_t k = 0; next_unit(k, it); ++k, round0 += KB) {
@@ -395,9 +398,9 @@ wgemm_kernel(const WgemmArgs a, const __grid_constant__ CUtensorMap rows_map) {
                         __syncwarp();
                         if (lane == 0) mbar_arrive(bar_wempty + bars);
                         uint32_t o[16];
-                        make_q8(o, v[0][0], v[0][1], d[0]);
+                        make_q8(o, v[0][0], v[0][1], weight_scale(d[0]));
                         store(i0 + q * istep, 0, o);
-                        make_q8(o, v[1][0], v[1][1], d[1]);
+                        make_q8(o, v[1][0], v[1][1], weight_scale(d[1]));
                         store(i0 + q * istep, 1, o);
                     }
                     continue;
@@ -453,7 +456,7 @@ wgemm_kernel(const WgemmArgs a, const __grid_constant__ CUtensorMap rows_map) {
                                                        c == 0 ? v[2].x : c == 1 ? v[2].y : c == 2 ? v[2].z : v[2].w, c == 0 ? v[3].x : c == 1 ? v[3].y : c == 2 ? v[3].z : v[3].w};
                                 uint32_t o[16];
                                 if (MODE == wg::kDown) make_iq4(o, w, __float2half2_rn(dl), tab_c);   // two roundings of 2^-12
-                                else make_iq4(o, w, split_scale(dl), tab_c);
+                                else make_iq4(o, w, weight_scale(dl), tab_c);
                                 store(i0 + (2 * hf + q) * istep, s, o);
                             }
                         }
@@ -506,9 +509,9 @@ wgemm_kernel(const WgemmArgs a, const __grid_constant__ CUtensorMap rows_map) {
                         if (q == 3) w_free();
                         if (skip) continue;
                         uint32_t o[16];
-                        make_q8(o, v[0][0], v[0][1], d[0]);
+                        make_q8(o, v[0][0], v[0][1], weight_scale(d[0]));
                         store(i0 + q * istep, 0, o);
-                        make_q8(o, v[1][0], v[1][1], d[1]);
+                        make_q8(o, v[1][0], v[1][1], weight_scale(d[1]));
                         store(i0 + q * istep, 1, o);
                     }
                 }
