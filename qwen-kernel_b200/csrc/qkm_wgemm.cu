@@ -292,11 +292,17 @@ wgemm_kernel(const WgemmArgs a, const __grid_constant__ CUtensorMap rows_map) {
         mbar_init(bar_tab, 1);
         mbar_init(bar_cols, wg::kEpilogueWarps);
         mbar_fence_init();
+        if (wg::has_table<FMT>()) {   // does not depend on the kernel before either
+            mbar_expect_tx(bar_tab, wg::kTabBytes);
+            for (uint32_t i = 0; i < 4; ++i) bulk_g2s(wg::kTab + i * 16384u, a.table + i * 16384u, 16384u, bar_tab);
+        }
     }
     if (warp == 0) { umma::tmem_alloc(smem_addr(&s_tmem), 512); umma::tmem_relinquish(); }
     umma::fence_before_sync();
     pdl_trigger();
-    pdl_wait();   // up to here nothing depended on the kernel before
+    // What depends on the kernel before: the work lists and everything read by their indices.  A dense matrix's units are known: its
+    // weights are fetched and expanded while the kernel that writes the activation rows ends.
+    if (MODE != wg::kDense) pdl_wait();
     __syncthreads();
     umma::fence_after_sync();
     const uint32_t n_units = MODE == wg::kDense ? (a.n_dense + wg::kNT - 1) / wg::kNT * row_units : *a.n_items;
@@ -522,6 +528,7 @@ wgemm_kernel(const WgemmArgs a, const __grid_constant__ CUtensorMap rows_map) {
         // ---- epilogue: warps e and e + 4 read TMEM lanes 32 e .. 32 e + 31, every other 16 columns each (with four warps the drain of
         // 128 columns took 13,000 cycles a gate/up unit, a third of the time at 4096 tokens)
         asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(wg::kEpilogueRegs));
+        if (MODE == wg::kDense) pdl_wait();
         const uint32_t e = warp & 3u, eh = (warp >> 2) & 1u, c = tid - wg::kProducerWarps * 32;   // c: the column this thread prepares
         uint32_t used[2] = {0, 0}, next = 0, iter = 0;
         MmaItem it;
@@ -628,10 +635,6 @@ wgemm_kernel(const WgemmArgs a, const __grid_constant__ CUtensorMap rows_map) {
         }
     } else if (warp == (uint32_t)wg::kWeightWarp) {
         // ---- units and weights
-        if (wg::has_table<FMT>() && lane == 0) {
-            mbar_expect_tx(bar_tab, wg::kTabBytes);
-            for (uint32_t i = 0; i < 4; ++i) bulk_g2s(wg::kTab + i * 16384u, a.table + i * 16384u, 16384u, bar_tab);
-        }
         uint32_t blocks[2] = {0, 0}, slots[2] = {0, 0};   // handed out so far, per parity
         auto drained = [&](uint32_t par, uint32_t slot) {   // everything put there has been read
             const uint32_t uses = (slots[par] + kSlots - 1 - slot) / kSlots + (slot ? 0u : blocks[par]);
@@ -723,6 +726,7 @@ wgemm_kernel(const WgemmArgs a, const __grid_constant__ CUtensorMap rows_map) {
         }
     } else if (MODE != wg::kGateUp && warp == (uint32_t)wg::kRowWarp) {
         // ---- consecutive activation rows: boxes of 16
+        if (MODE == wg::kDense) pdl_wait();
         uint32_t gs = 0;
         MmaItem it;
         for (uint32_t k = 0; next_unit(k, it); ++k) {
