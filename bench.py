@@ -608,8 +608,8 @@ def run_prefill_or_ep(args, pkg, syn, torch, R: Ranks, orc, layers, peaks):
         out["stages_us_at_2048"] = acc
         gu = acc.get("moe.gu", 0.0)
         if gu > 0:
-            fl = T * dims.n_used * 2 * 2 * dims.n_ff * dims.n_embd
-            out["roofline"] = {"bound": "tensor", "kernel": "gateup_iq3_kernel at 2048 tokens",
+            fl = T * (dims.n_used + 1) * 2 * 2 * dims.n_ff * dims.n_embd   # the shared expert is in the same launch
+            out["roofline"] = {"bound": "tensor", "kernel": "wgemm_kernel (gate/up) at 2048 tokens",
                                "achieved": fl / (gu * 1e-6) / 1e12, "peak": peaks["bf16_tflops"], "unit": "TFLOP/s",
                                "frac": fl / (gu * 1e-6) / 1e12 / peaks["bf16_tflops"],
                                "peak_source": peaks["source"] + " cuBLAS bf16 burst", "traffic": None}

@@ -254,14 +254,14 @@ QKM_API int qkm_profile_read(qkm_ctx *c, char *labels, float *ms, uint32_t max_s
 QKM_API int qkm_last_sel(qkm_ctx *c, qkm_sel *sel_host, uint32_t n_tokens);
 /* Device address of the context's selection / h scratch of the last fused call (h in f32 is
  * written by the decode calls and by the prefill calls that take the f32 kernels; the tensor-core
- * prefill writes f32 rows by pair position there, not [T][slot]). */
+ * prefill keeps its hidden rows elsewhere, as f16 by pair position). */
 QKM_API const qkm_sel *qkm_sel_device(const qkm_ctx *c);
 QKM_API const float   *qkm_h_device(const qkm_ctx *c);
 
 /* ---- dense quantised GEMM (gemm_q8_0*.comp, gemm_iq4_xs.comp; src/main.cpp:4806-4835) -----
  * Y[n][M] = X[n][K] . W^T for a Q8_0 or IQ4_XS matrix W [M][K] (ggml rows), M % 128 == 0,
  * K % 256 == 0.  qkm_dense_upload copies W (host pointer) into one of 16 slots; qkm_dense_gemm
- * takes device x [n][K] / y [n][M] f32 and runs on the tensor cores with bf16 operands
+ * takes device x [n][K] / y [n][M] f32 and runs on the tensor cores with f16 operands (x rows scaled by powers of two)
  * (the prefill tolerance applies).  Scratch grows to the largest n seen. */
 QKM_API int qkm_dense_upload(qkm_ctx *c, uint32_t slot, uint32_t type, const void *w_host,
                              uint32_t M, uint32_t K);
