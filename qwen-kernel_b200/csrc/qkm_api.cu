@@ -55,11 +55,7 @@ struct qkm_ctx {
     float* stack_y = nullptr;
     // streaming path scratch
     int n_sms = 0;
-    int8_t* xplanes = nullptr;        // [max_tokens][4][n_embd]
     float* xscale = nullptr;          // [max_tokens]
-    void* hpieces = nullptr;          // [max_tokens*n_used][3][n_ff] bf16
-    StreamItem* items_sh_gu = nullptr;
-    StreamItem* items_sh_dn = nullptr;
     uint32_t* n_items = nullptr;      // prefill: units of [0] gate/up, [1] down; [2], [3] their tickets
     uint32_t* status = nullptr;       // kernel status word (device)
     uint32_t* route_counter = nullptr; // ticket counter of the selection kernel's grouping tail (device, stays zero)
@@ -261,17 +257,10 @@ extern "C" QKM_API qkm_ctx* qkm_open(const qkm_config* cfg, char* err, size_t er
     // also need every expert resident; a sharded context uses the tiles through qkm_ep_*.)
     auto pow2_2_16 = [](uint32_t v) { return v >= 2 && v <= 16 && (v & (v - 1)) == 0; };
     c->shapes_stream_ok = pow2_2_16(d.n_embd / 256) && d.n_embd / 256 <= 8 && pow2_2_16(d.n_ff / 256) && d.n_used <= 15 &&
-                          d.n_ff % gateup_stream_rows_per_item() == 0 &&
-                          d.n_embd % down_stream_rows_per_item() == 0;
+                          d.n_ff % 128 == 0;
     if (c->shapes_stream_ok) {
-        const size_t sh_groups = (T + 1) / 2;
-        const size_t chunks_gu = d.n_ff / gateup_stream_rows_per_item(), chunks_dn = d.n_embd / down_stream_rows_per_item();
         struct { void** p; size_t bytes; } more[] = {
-            {(void**)&c->xplanes, T * 4 * d.n_embd},
             {(void**)&c->xscale, T * sizeof(float)},
-            {(void**)&c->hpieces, T * (d.n_used + 1) * 3 * d.n_ff * 2},
-            {(void**)&c->items_sh_gu, sh_groups * chunks_gu * sizeof(StreamItem)},
-            {(void**)&c->items_sh_dn, sh_groups * chunks_dn * sizeof(StreamItem)},
             {(void**)&c->n_items, 4 * sizeof(uint32_t)},
         };
         for (auto& a : more) {
@@ -341,8 +330,7 @@ extern "C" QKM_API void qkm_close(qkm_ctx* c) {
     }
     for (auto& dm : c->dense) if (dm.tiles) cudaFree(dm.tiles);
     void* scratch[] = {c->argmax_scratch, c->dense_xb, c->dense_scale, c->sel, c->h, c->route_scratch, c->offsets, c->pairs, c->contrib, c->y2, c->x_stage, c->y_stage,
-                       c->stack_x, c->stack_y, c->xplanes, c->xscale, c->hpieces,
-                       c->items_sh_gu, c->items_sh_dn, c->n_items, c->status, c->route_counter,
+                       c->stack_x, c->stack_y, c->xscale, c->n_items, c->status, c->route_counter,
                        c->planes8, c->lut_gu, c->lut_dd, c->lut_pf,
                        c->xb, c->xnorm, c->hb, c->hscale, c->contrib_p, c->mma_items[0], c->mma_items[1],
                        c->pos_of, c->group_counts, c->ep_counts, c->ep_send_tok, c->ep_send_pos};
@@ -1062,16 +1050,19 @@ static int ep_check(qkm_ctx* c, uint32_t n_ranks) {
     return QKM_OK;
 }
 
+// the shared expert of so few local tokens runs on the decode kernels
+static bool ep_shared_decode(const qkm_ctx* c, const qkm_layer_dev& ld, uint32_t n) { return ld.tiles_ok && n <= 64 && c->dec_ok && decode_down_any_ok(c->cfg.dims); }
+
 // router logits and selection of the n local tokens into c->sel (digit planes / f16 rows as the
 // shared-expert kernels of that size want them)
 static int ep_route_local(qkm_ctx* c, uint32_t layer, const float* x, uint32_t n) {
     const qkm_layer_dev& ld = c->layers[layer];
     const qkm_layer_weights& w = ld.w;
     const qkm_dims& d = c->cfg.dims;
-    const bool planes = ld.tiles_ok && n <= 64;   // the streamed shared-expert kernels read digit planes
+    const bool planes = ep_shared_decode(c, ld, n);   // the decode kernels of the shared expert read digit planes
     const bool tc = ld.tiles_ok && n > 64;        // tensor-core logits from f16 rows
     RouteExtra ex;
-    if (planes) { ex.xplanes = c->xplanes; ex.xscale = c->xscale; }
+    if (planes) { ex.xplanes = c->planes8; ex.xscale = c->xscale; }
     if (tc) {
         if (int rc = ensure_prefill_scratch(c)) return rc;
         QKM_LAUNCH(c, launch_f16_rows(c->L(), x, c->xb, c->xscale, c->xnorm, n, d.n_embd));
@@ -1123,19 +1114,21 @@ extern "C" QKM_API int qkm_ep_shared(qkm_ctx* c, uint32_t layer, const float* x,
     const qkm_layer_dev& ld = c->layers[layer];
     const qkm_layer_weights& w = ld.w;
     const qkm_dims& d = c->cfg.dims;
-    if (!ld.tiles_ok) {
+    const bool dec = ep_shared_decode(c, ld, n);
+    if (!dec && (!ld.tiles_ok || n <= 64)) {
         QKM_LAUNCH(c, launch_shared_gateup(c->L(), d, w.gate_shexp, w.up_shexp, x, c->h, n));
         QKM_LAUNCH(c, launch_shared_down(c->L(), d, w.down_shexp, c->h, c->sel, c->y2, n));
         return QKM_OK;
     }
-    if (n <= 64) {   // streamed kernels of the decode sequence (digit planes written by qkm_ep_dispatch)
-        const uint32_t nb = (uint32_t)c->n_sms;
-        QKM_LAUNCH(c, launch_shared_plan(c->L(), d, n, c->pairs, c->items_sh_gu, d.n_ff / gateup_stream_rows_per_item(),
-                                         c->items_sh_dn, d.n_embd / down_stream_rows_per_item(), 2, c->n_items + 2));
-        QKM_LAUNCH(c, launch_gateup_stream(c->L(), d, QKM_TYPE_Q8_0, ld.tiles[5], ld.tiles[6], c->xplanes, c->xscale, c->pairs,
-                                           c->items_sh_gu, c->n_items + 2, c->h, c->hpieces, nb, c->status));
-        QKM_LAUNCH(c, launch_down_stream(c->L(), d, QKM_TYPE_Q8_0, ld.tiles[7], c->hpieces, c->sel, c->pairs, c->items_sh_dn,
-                                         c->n_items + 3, nullptr, c->y2, nullptr, nb, c->status));
+    if (dec) {   // the decode kernels without routed experts (digit planes written by qkm_ep_dispatch)
+        GateupDecodeArgs ga{};
+        ga.sh_gate_tiles = (const uint8_t*)ld.tiles[5]; ga.sh_up_tiles = (const uint8_t*)ld.tiles[6];
+        ga.luts = c->lut_gu; ga.planes = c->planes8; ga.xscale = c->xscale; ga.sel = c->sel;
+        ga.n_tokens = n; ga.with_shared = 1; ga.gateup_type = w.gateup_type; ga.h = c->h; ga.status = c->status; ga.d = d;
+        QKM_LAUNCH(c, launch_decode_gateup(c->L(), ga, (uint32_t)c->n_sms));
+        DownDecodeArgs da{};
+        da.sh_tiles = (const uint8_t*)ld.tiles[7]; da.h = c->h; da.sel = c->sel; da.y = c->y2; da.n_tokens = n; da.status = c->status; da.d = d;
+        QKM_LAUNCH(c, launch_decode_down_any(c->L(), da, w.down_type, (uint32_t)c->n_sms));
         return QKM_OK;
     }
     // tensor-core kernels with an empty routed list: only the shared expert's tiles

@@ -43,7 +43,7 @@ decode_down_any_kernel(DownDecodeArgs a) {
     const qkm_dims d = a.d;
     const uint32_t n_slots = d.n_used + 1, n_warps = blockDim.x >> 5;
     const uint32_t KB = d.n_ff / 256, RT = d.n_embd / 16, slot = warp / KB, kb = warp - slot * KB;
-    const bool has_tile = slot < d.n_used, has_sh = a.sh_tiles != nullptr && warp < d.n_ff / 32;
+    const bool has_tile = a.tiles != nullptr && slot < d.n_used, has_sh = a.sh_tiles != nullptr && warp < d.n_ff / 32;
     const uint32_t win0 = smem_addr(smem_raw), base = Q6 ? (win0 + 127u) & ~127u : 0u;
     if (!Q6) {   // the fixed addresses must lie inside the dynamic area
         uint32_t dyn_size;
@@ -283,7 +283,7 @@ static cudaError_t any_launch(const Launch& L, const DownDecodeArgs& a, uint32_t
 cudaError_t launch_decode_down_any(const Launch& L, const DownDecodeArgs& a, uint32_t type, uint32_t n_blocks) {
     if (!decode_down_any_ok(a.d)) return cudaErrorInvalidValue;
     if (a.n_tokens == 0) return cudaSuccess;
-    if (type == QKM_TYPE_Q6_K) return any_launch<true>(L, a, n_blocks);
+    if (type == QKM_TYPE_Q6_K || a.tiles == nullptr) return any_launch<true>(L, a, n_blocks);
     if (type != QKM_TYPE_IQ4_XS || !a.lut) return cudaErrorInvalidValue;
     return any_launch<false>(L, a, n_blocks);
 }

@@ -55,15 +55,6 @@ __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;"
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 #endif
 
-// One unit of work of a streaming kernel: an expert, a chunk of its rows and up to
-// tok_per_item of the tokens routed to it (pairs[pair_off .. pair_off + ntok)).
-struct StreamItem {
-    uint16_t expert;   // resident-expert index
-    uint8_t chunk;     // row chunk within the expert's matrix
-    uint8_t ntok;
-    uint32_t pair_off;
-};
-
 // One unit of the prefill GEMMs: an expert, 256 rows of its matrices and up to 128
 // of its pairs (pairs[pair_off .. pair_off + n)).
 struct MmaItem {
@@ -118,7 +109,7 @@ bool decode_gateup_ok(const qkm_dims& d);
 cudaError_t launch_decode_gateup(const Launch& L, const GateupDecodeArgs& a, uint32_t n_blocks);
 // routed (IQ4_XS) down + shared (Q8_0) down + weighted sum: y[t] = sum_s w_s D[ids_s] h[t][s] + w_shared DS h[t][n_used]
 struct DownDecodeArgs {
-    const uint8_t* tiles;           // routed experts, IQ4_XS tiles
+    const uint8_t* tiles;           // routed experts, IQ4_XS tiles (launch_decode_down_any: NULL for the shared term alone)
     const uint8_t* sh_tiles;        // shared expert, Q8_0 tiles (NULL: no shared term)
     const uint8_t* lut;             // IQ4_XS form: decode_down_lut_bytes() bytes written by launch_decode_down_lut
     const float* h;                 // [T][n_used+1][n_ff] f32 (encoded as int8 digit planes inside the kernel)
@@ -183,26 +174,6 @@ cudaError_t launch_fold_pairs(const Launch& L, const qkm_dims& d, const float* c
 cudaError_t launch_repack(const Launch& L, uint32_t type, const void* raw, void* out, uint32_t n_mats,
                           uint32_t rows, uint32_t K);
 
-// ---- qkm_decode_gateup.cu / qkm_decode_down.cu : streaming kernels for small token counts
-cudaError_t launch_encode_digits(const Launch& L, const float* x, int8_t* planes, float* scale,
-                                 uint32_t n_rows, uint32_t K);
-cudaError_t launch_gateup_stream(const Launch& L, const qkm_dims& d, uint32_t type, const void* gate_tiles,
-                                 const void* up_tiles, const int8_t* xplanes, const float* xscale,
-                                 const uint32_t* pairs, const StreamItem* items, const uint32_t* n_items,
-                                 float* h, void* hpieces, uint32_t n_blocks, uint32_t* status);
-// contrib [T][n_used+1][n_embd]; arrivals [T][n_embd/unit rows] zero before the first call
-cudaError_t launch_down_stream(const Launch& L, const qkm_dims& d, uint32_t type, const void* tiles,
-                               const void* hpieces, const qkm_sel* sel, const uint32_t* pairs,
-                               const StreamItem* items, const uint32_t* n_items, float* contrib, float* y,
-                               uint32_t* arrivals, uint32_t n_blocks, uint32_t* status);
-uint32_t down_stream_unit_rows();
-// token-major routed down: y[t] = sum_s w_s * D[ids_s].h[t][s] + y2[t] (y2 may be NULL)
-cudaError_t launch_down_tok(const Launch& L, const qkm_dims& d, uint32_t type, const void* tiles,
-                            const void* hpieces, const qkm_sel* sel, const float* y2, float* y,
-                            uint32_t n_tokens, uint32_t n_blocks, uint32_t* status);
-uint32_t gateup_stream_rows_per_item();
-uint32_t down_stream_rows_per_item();
-
 // ---- qkm_gemv.cu
 cudaError_t launch_dequant(const Launch& L, uint32_t type, const void* blocks, float* y, uint64_t n_elems);
 cudaError_t launch_gemv(const Launch& L, uint32_t type, const void* W, const float* x, float* y,
@@ -228,7 +199,7 @@ cudaError_t launch_select(const Launch& L, const qkm_dims& d, const float* logit
 // norm2[e] = |router row e|^2; largest (zero before): their maximum; either may be NULL
 cudaError_t launch_row_norm2(const Launch& L, const qkm_dims& d, uint32_t router_type, const void* router, float* norm2, float* largest);
 struct RouteExtra {                      // all optional
-    int8_t* xplanes = nullptr;           // out: x rows as digit planes [kb][digit][256], and their scales
+    int8_t* xplanes = nullptr;           // out: x rows as digit planes and their negatives [kb][8][256], and their scales
     float* xscale = nullptr;
     const void* x_f16 = nullptr;         // with these four (more than 64 tokens) the logits come from the tensor cores: rows and
     const float* x_f16_inv = nullptr;    // scales of launch_f16_rows, the router as launch_router_f16 wrote it, its rows' largest squared norm
@@ -289,11 +260,6 @@ cudaError_t launch_logits_mma(const Launch& L, const qkm_dims& d, const void* ro
 cudaError_t launch_group_pairs(const Launch& L, const qkm_dims& d, const qkm_sel* sel, uint32_t n_tokens,
                                uint32_t* offsets, uint32_t* pairs, uint32_t expert_first,
                                uint32_t expert_count);
-// shared-expert work lists: n_items[0] gate/up, n_items[1] down; pairs[n_tokens*n_used + t] = (t<<4)|n_used
-cudaError_t launch_shared_plan(const Launch& L, const qkm_dims& d, uint32_t n_tokens, uint32_t* pairs,
-                               StreamItem* items_gu, uint32_t chunks_gu, StreamItem* items_dn,
-                               uint32_t chunks_dn, uint32_t tok_per_item, uint32_t* n_items);
-
 // ---- qkm_moe_simple.cu : one warp per output element, raw ggml layout
 cudaError_t launch_gateup_tokens(const Launch& L, const qkm_dims& d, uint32_t type, const void* gate,
                                  const void* up, const float* x, const qkm_sel* sel, float* h,

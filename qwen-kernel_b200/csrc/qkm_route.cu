@@ -491,34 +491,4 @@ cudaError_t launch_group_pairs(const Launch& L, const qkm_dims& d, const qkm_sel
     return cudaGetLastError();
 }
 
-// Work lists of the shared expert: every token is a "pair" (token, slot n_used) stored
-// after the routed pairs, in groups of tok_per_item.  Depends on n_tokens only.
-__global__ void shared_plan_kernel(uint32_t n_tokens, uint32_t n_used, uint32_t* __restrict__ pairs,
-                                   StreamItem* __restrict__ items_gu, uint32_t chunks_gu,
-                                   StreamItem* __restrict__ items_dn, uint32_t chunks_dn,
-                                   uint32_t tok_per_item, uint32_t* __restrict__ n_items) {
-    const uint32_t np = n_tokens * n_used, tid = threadIdx.x;
-    const uint32_t groups = (n_tokens + tok_per_item - 1) / tok_per_item;
-    for (uint32_t t = tid; t < n_tokens; t += blockDim.x) pairs[np + t] = (t << 4) | n_used;
-    for (uint32_t gi = tid; gi < groups; gi += blockDim.x) {
-        StreamItem it;
-        it.expert = 0;
-        it.ntok = (uint8_t)min(tok_per_item, n_tokens - gi * tok_per_item);
-        it.pair_off = np + gi * tok_per_item;
-        for (uint32_t c = 0; c < chunks_gu; ++c) { it.chunk = (uint8_t)c; items_gu[(size_t)gi * chunks_gu + c] = it; }
-        for (uint32_t c = 0; c < chunks_dn; ++c) { it.chunk = (uint8_t)c; items_dn[(size_t)gi * chunks_dn + c] = it; }
-    }
-    if (tid == 0) { n_items[0] = groups * chunks_gu; n_items[1] = groups * chunks_dn; }
-}
-
-cudaError_t launch_shared_plan(const Launch& L, const qkm_dims& d, uint32_t n_tokens, uint32_t* pairs,
-                               StreamItem* items_gu, uint32_t chunks_gu, StreamItem* items_dn,
-                               uint32_t chunks_dn, uint32_t tok_per_item, uint32_t* n_items) {
-    if (n_tokens == 0) return cudaSuccess;
-    shared_plan_kernel<<<1, 256, 0, L.stream>>>(n_tokens, d.n_used, pairs, items_gu, chunks_gu, items_dn, chunks_dn,
-                                                tok_per_item, n_items);
-    L.count();
-    return cudaGetLastError();
-}
-
 }  // namespace qkm

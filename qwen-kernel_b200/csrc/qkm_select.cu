@@ -34,7 +34,7 @@ struct SelectArgs {
     const float* gis;
     const float* x;
     qkm_sel* sel;
-    int8_t* xplanes;           // optional: x as digit planes [kb][digit][256], and their scale
+    int8_t* xplanes;           // optional: x as digit planes and their negatives [kb][8][256], and their scale
     float* xscale;
     uint32_t* counts;          // optional: pairs per resident expert, added to; ranks[t * n_used + s] = a pair's number inside its expert
     uint32_t* ranks;
@@ -159,11 +159,12 @@ select_tokens_kernel(const SelectArgs a) {
             const float4 v = xt[u];
             const uint32_t e[4] = {bad ? 0u : digits4(__float2int_rn(v.x * up_f)), bad ? 0u : digits4(__float2int_rn(v.y * up_f)),
                                    bad ? 0u : digits4(__float2int_rn(v.z * up_f)), bad ? 0u : digits4(__float2int_rn(v.w * up_f))};
-            uint32_t* q = reinterpret_cast<uint32_t*>(a.xplanes + (size_t)t * 4 * d.n_embd + (size_t)(u >> 6) * 1024 + 4 * (u & 63u));
+            uint32_t* q = reinterpret_cast<uint32_t*>(a.xplanes + (size_t)t * 8 * d.n_embd + (size_t)(u >> 6) * 2048 + 4 * (u & 63u));
 #pragma unroll
             for (int j = 0; j < 4; ++j) {   // digit j of the four
                 const uint32_t s = 0x4040u + 0x1111u * j;
                 q[64 * j] = __byte_perm(__byte_perm(e[0], e[1], s), __byte_perm(e[2], e[3], s), 0x5410u);
+                q[64 * (j + 4)] = __vneg4(q[64 * j]);
             }
         }
         if (tid == 0) a.xscale[t] = bad ? __int_as_float(0x7FC00000) : ldexpf(1.0f, -p);

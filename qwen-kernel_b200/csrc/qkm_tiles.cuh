@@ -84,10 +84,4 @@ __host__ __device__ inline size_t tiled_bytes(uint32_t type, size_t n_mats, uint
 // position of piece t of row r inside the row's 64-byte run
 __host__ __device__ inline uint32_t piece_at(uint32_t r, uint32_t t) { return (t ^ ((r >> 1) & 3u)) * 16u; }
 
-// digit planes of one activation row set: planes[(row * 4 + digit) * K + k], scale[row]
-struct DigitRows {
-    const int8_t* planes;
-    const float* scale;  // 2^-p per row (per chunk where stated)
-};
-
 }  // namespace qkm
