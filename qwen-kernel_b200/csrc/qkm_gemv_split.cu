@@ -469,7 +469,8 @@ static cudaError_t gemv_split_launch_nt(const Launch& L, GemvSplitArgs a, uint32
     const uint32_t KB = a.K / 256, n_tiles = (a.M + 15) / 16;
     // Eight slices while one round of tiles covers the matrix (33 such clusters are resident), four beyond: more
     // slices share the work of few tiles between more warps, fewer waste less on the cluster's barriers and sums.
-    uint32_t slices = KB >= 8 && n_tiles <= 33u * 8u ? 8u : KB >= 4 ? 4u : KB >= 2 ? 2u : 1u;
+    // (More than eight rows of F16 x above 2048 columns: eight always, a quarter's fragments would leave room for one block an SM.)
+    uint32_t slices = KB >= 8 && (n_tiles <= 33u * 8u || (TYPE == QKM_TYPE_F16 && NT > 4 && KB > 8)) ? 8u : KB >= 4 ? 4u : KB >= 2 ? 2u : 1u;
     a.kb_slice = (KB + slices - 1) / slices;
     slices = (KB + a.kb_slice - 1) / a.kb_slice;   // no empty slice
     a.slices = slices;
@@ -511,7 +512,7 @@ static cudaError_t gemv_split_launch(const Launch& L, const uint8_t* W, const fl
                                      uint32_t n_sms, uint32_t* rows_done) {
     *rows_done = 0;
     while (n) {   // sixteen rows of x a pass (eight where the fragments of sixteen would not leave room for the tiles)
-        const uint32_t most = TYPE == QKM_TYPE_F16 && K > 2048 ? 8u : 16u;
+        const uint32_t most = TYPE == QKM_TYPE_F16 && K > 4096 ? 8u : 16u;
         GemvSplitArgs a{};
         a.W = W; a.x = x + (size_t)*rows_done * K; a.y = y + (size_t)*rows_done * M; a.M = M; a.K = K;
         a.n = n < most ? n : most;
@@ -519,7 +520,9 @@ static cudaError_t gemv_split_launch(const Launch& L, const uint8_t* W, const fl
         cudaError_t e;
         if (a.n <= 2) e = gemv_split_launch_nt<TYPE, 1>(L, a, n_sms, &taken);
         else if (a.n <= 4) e = gemv_split_launch_nt<TYPE, 2>(L, a, n_sms, &taken);
+        else if (a.n <= 6) e = gemv_split_launch_nt<TYPE, 3>(L, a, n_sms, &taken);
         else if (a.n <= 8) e = gemv_split_launch_nt<TYPE, 4>(L, a, n_sms, &taken);
+        else if (a.n <= 12) e = gemv_split_launch_nt<TYPE, 6>(L, a, n_sms, &taken);
         else e = gemv_split_launch_nt<TYPE, 8>(L, a, n_sms, &taken);
         if (e != cudaSuccess || !taken) return e;
         *rows_done += a.n;
