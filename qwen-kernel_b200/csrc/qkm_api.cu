@@ -64,6 +64,7 @@ struct qkm_ctx {
     int8_t* planes8 = nullptr;         // [max_tokens][n_embd/256][8][256]
     uint8_t* lut_gu = nullptr;         // table images the decode kernels copy to shared memory
     uint8_t* lut_dd = nullptr;         // table image of the decode IQ4_XS down kernel
+    float* contrib_dec = nullptr;      // [min(max_tokens, 64)][n_used+1][n_embd], for the down kernel that groups by expert
     uint8_t* lut_pf = nullptr;         // table image of the prefill GEMMs
     uint32_t* status_host = nullptr;  // pinned mirror
     bool shapes_stream_ok = false;
@@ -276,6 +277,7 @@ extern "C" QKM_API qkm_ctx* qkm_open(const qkm_config* cfg, char* err, size_t er
                 {(void**)&c->planes8, T * 8 * d.n_embd},
                 {(void**)&c->lut_gu, decode_gateup_lut_bytes()},
                 {(void**)&c->lut_dd, decode_down_lut_bytes()},
+                {(void**)&c->contrib_dec, decode_down_group_ok(d) && (T >= 40 || !decode_down_any_ok(d)) ? (T < 64 ? T : 64) * (d.n_used + 1) * d.n_embd * sizeof(float) : 0},
             };
             for (auto& a : dec) {
                 if ((e = cudaMalloc(a.p, a.bytes)) != cudaSuccess) {
@@ -331,7 +333,7 @@ extern "C" QKM_API void qkm_close(qkm_ctx* c) {
     for (auto& dm : c->dense) if (dm.tiles) cudaFree(dm.tiles);
     void* scratch[] = {c->argmax_scratch, c->dense_xb, c->dense_scale, c->sel, c->h, c->route_scratch, c->offsets, c->pairs, c->contrib, c->y2, c->x_stage, c->y_stage,
                        c->stack_x, c->stack_y, c->xscale, c->n_items, c->status, c->route_counter,
-                       c->planes8, c->lut_gu, c->lut_dd, c->lut_pf,
+                       c->planes8, c->lut_gu, c->lut_dd, c->contrib_dec, c->lut_pf,
                        c->xb, c->xnorm, c->hb, c->hscale, c->contrib_p, c->mma_items[0], c->mma_items[1],
                        c->pos_of, c->group_counts, c->ep_counts, c->ep_send_tok, c->ep_send_pos};
     for (void* p : scratch) if (p) cudaFree(p);
@@ -604,7 +606,7 @@ extern "C" QKM_API int qkm_dequant(qkm_ctx* c, uint32_t type, const void* blocks
 
 // ---------------------------------------------------------------- fused layer calls
 
-// Three launches for the whole layer: (1) router logits, selection and digit planes; (2) pair
+// Three launches for the whole layer (four from 40 tokens on, where the down kernel that groups by expert is followed by a fold): (1) router logits, selection and digit planes; (2) pair
 // grouping (in every block's shared memory), then gate/up + SwiGLU of the routed experts and of
 // the shared expert; (3) down projections of both and the weighted sum.  The shared expert rides inside (2)
 // and (3): no side stream, and nothing runs beside the two persistent kernels that they would have to share
@@ -630,7 +632,9 @@ static int decode_fused(qkm_ctx* c, const qkm_layer_dev& ld, const float* x, uin
     DownDecodeArgs da{};
     da.tiles = (const uint8_t*)ld.tiles[4]; da.sh_tiles = (const uint8_t*)ld.tiles[7]; da.lut = c->lut_dd;
     da.h = h; da.sel = sel; da.y = y; da.n_tokens = n; da.status = c->status; da.d = d;
-    if (!decode_down_ok(d)) QKM_LAUNCH(c, launch_decode_down_any(c->Lchain(), da, w.down_type, nb));
+    da.contrib = c->contrib_dec;
+    if (c->contrib_dec && decode_down_group_better(d, w.down_type, n)) QKM_LAUNCH(c, launch_decode_down_group(c->Lchain(), da, w.down_type, nb));
+    else if (!decode_down_ok(d)) QKM_LAUNCH(c, launch_decode_down_any(c->Lchain(), da, w.down_type, nb));
     else if (w.down_type == QKM_TYPE_IQ4_XS) QKM_LAUNCH(c, launch_decode_down(c->Lchain(), da, nb));
     else QKM_LAUNCH(c, launch_decode_down_q6k(c->Lchain(), da, nb));
     c->prof_mark("moe.dn");
@@ -646,7 +650,7 @@ extern "C" QKM_API int qkm_moe_decode(qkm_ctx* c, uint32_t layer, const float* x
     const qkm_dims& d = c->cfg.dims;
     c->prof_begin();
     constexpr uint32_t kMost = 64;
-    if (n && ld.fused_ok && c->dec_ok && route_decode_ok(d, n < kMost ? n : kMost, c->route_scratch_bytes) && (decode_down_ok(d) || decode_down_any_ok(d))) {
+    if (n && ld.fused_ok && c->dec_ok && route_decode_ok(d, n < kMost ? n : kMost, c->route_scratch_bytes) && (decode_down_ok(d) || decode_down_any_ok(d) || c->contrib_dec)) {
         for (uint32_t t = 0; t < n; t += kMost)
             if (int rc = decode_fused(c, ld, x + (size_t)t * d.n_embd, n - t < kMost ? n - t : kMost, y + (size_t)t * d.n_embd, c->sel + t,
                                       c->h + (size_t)t * (d.n_used + 1) * d.n_ff)) return rc;

@@ -115,6 +115,7 @@ struct DownDecodeArgs {
     const float* h;                 // [T][n_used+1][n_ff] f32 (encoded as int8 digit planes inside the kernel)
     const qkm_sel* sel;
     float* y;
+    float* contrib;                 // launch_decode_down_group: scratch [T][n_used+1][n_embd]
     uint32_t n_tokens;
     uint32_t* status;
     qkm_dims d;
@@ -127,6 +128,10 @@ cudaError_t launch_decode_down(const Launch& L, const DownDecodeArgs& a, uint32_
 cudaError_t launch_decode_down_q6k(const Launch& L, const DownDecodeArgs& a, uint32_t n_blocks);
 // either type, other numbers of slots
 bool decode_down_any_ok(const qkm_dims& d);
+// either type, grouped by expert: may run, and is the faster one for n tokens
+bool decode_down_group_ok(const qkm_dims& d);
+bool decode_down_group_better(const qkm_dims& d, uint32_t type, uint32_t n);
+cudaError_t launch_decode_down_group(const Launch& L, const DownDecodeArgs& a, uint32_t type, uint32_t n_blocks);
 cudaError_t launch_decode_down_any(const Launch& L, const DownDecodeArgs& a, uint32_t type, uint32_t n_blocks);
 
 // ---- qkm_wgemm.cu : tcgen05 GEMMs with quantised weights (batched prefill, dense projections)

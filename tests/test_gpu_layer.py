@@ -162,6 +162,24 @@ def test_decode_numbers_of_slots(pkg, orc, syn, n_ff, n_used, dt, T):
         assert np.array_equal(y, ctx.moe_forward_host(0, x, mode=0))
 
 
+@pytest.mark.parametrize("n_embd,n_ff,n_expert,n_used,dt,T", [(512, 512, 256, 8, 23, 40), (256, 512, 32, 1, 23, 41), (1024, 512, 64, 6, 14, 40), (256, 512, 48, 13, 14, 63), (512, 512, 32, 15, 23, 1),
+                                                             (512, 512, 8, 4, 23, 64), (512, 512, 512, 10, 23, 110)])
+def test_decode_down_grouped_by_expert(pkg, orc, syn, n_embd, n_ff, n_expert, n_used, dt, T):
+    """Forty tokens on, or more slots than the token-major kernel takes: odd and full groups, ranges that begin inside a group, a second chunk of 46."""
+    dims = syn.Dims(n_embd=n_embd, n_ff=n_ff, n_expert=n_expert, n_used=n_used)
+    layer = syn.make_layer(dims, seed=18, gateup_type=23, down_type=dt)
+    x = syn.random_x(T, dims.n_embd, seed=19)
+    ref = orc.moe_layer(layer, x, threads=orc.hardware_threads())
+    with pkg.Context(dims, n_layer=1, max_tokens=T, device=0) as ctx:
+        ctx.upload_layer(0, layer)
+        d_x, d_y = ctx.to_device(x), ctx.alloc(x.nbytes)
+        ctx.moe_decode(0, d_x, T, d_y)
+        y = d_y.download(np.float32, x.shape)
+        check_layer(syn, y, ctx.last_sel(T), ref, n_used)
+        ctx.moe_decode(0, d_x, T, d_y)
+        assert np.array_equal(y, d_y.download(np.float32, x.shape))
+
+
 def test_decode_router_is_deterministic_over_many_calls(pkg, orc, syn):
     """200 calls of the fused decode sequence on the same 16 rows: ids, weights and outputs are the
     same bits every time (a last-arriving block ranks the logits; the reference removed such a
