@@ -74,6 +74,7 @@ struct qkm_ctx {
     void* hb = nullptr;               // [max_tokens*(n_used+1)][n_ff] hidden rows by pair position, f16 scaled per row
     float* hscale = nullptr;          // [max_tokens*(n_used+1)] the scales that undo the rows' scaling
     float* contrib_p = nullptr;       // [max_tokens*(n_used+1)][n_embd]
+    uint32_t unit_rows = kWgemmRows;             // activation rows per unit of the work lists
     MmaItem* mma_items[2] = {nullptr, nullptr};  // gate/up, down
     uint32_t* pos_of = nullptr;       // [max_tokens*(n_used+1)]
     uint32_t* group_counts = nullptr; // [resident experts] pairs, then [max_tokens*n_used] a pair's number inside its expert
@@ -691,7 +692,7 @@ static int ensure_prefill_scratch(qkm_ctx* c) {
     if (c->xb) return QKM_OK;
     const qkm_dims& d = c->cfg.dims;
     const size_t T = c->cfg.max_tokens, rows = T * (d.n_used + 1);
-    const uint32_t NT = wgemm_rows_per_unit();
+    const uint32_t NT = kWgemmRows;
     const size_t max_tiles = d.n_expert + (T * d.n_used + NT - 1) / NT + (T + NT - 1) / NT;   // the shared expert's last
     QKM_CUDA(c, cudaMalloc(&c->xb, T * d.n_embd * 2));
     QKM_CUDA(c, cudaMalloc((void**)&c->xnorm, T * sizeof(float)));
@@ -711,7 +712,7 @@ static int expert_plan(qkm_ctx* c, const qkm_sel* sel, uint32_t n, bool with_rou
     GroupPlace g{};
     g.counts = c->group_counts; g.ranks = c->group_counts + c->ecount; g.sel = sel; g.n_tokens = n; g.n_used = d.n_used; g.n_expert = d.n_expert;
     g.expert_first = c->efirst; g.expert_count = with_routed ? c->ecount : 0; g.sh_first = sh_first; g.sh_count = sh_count;
-    g.tile = wgemm_rows_per_unit(); g.rt_gu = d.n_ff / 128; g.rt_dn = d.n_embd / 256; g.pairs = c->pairs; g.pos_of = c->pos_of;
+    g.tile = c->unit_rows = with_routed ? wgemm_rows_per_unit(d, n) : kWgemmRows; g.rt_gu = d.n_ff / 128; g.rt_dn = d.n_embd / 256; g.pairs = c->pairs; g.pos_of = c->pos_of;
     g.items_gu = c->mma_items[0]; g.items_dn = c->mma_items[1]; g.n_items = c->n_items;
     QKM_LAUNCH(c, launch_group_place(c->L(), g));
     return QKM_OK;
@@ -721,12 +722,12 @@ static int expert_plan(qkm_ctx* c, const qkm_sel* sel, uint32_t n, bool with_rou
 // At most np_max routed pairs and sh_max rows of the shared expert.
 static int expert_gemms(qkm_ctx* c, const qkm_layer_dev& ld, const qkm_sel* sel, uint32_t np_max, uint32_t sh_max) {
     const qkm_dims& d = c->cfg.dims;
-    const uint32_t NT = wgemm_rows_per_unit();
+    const uint32_t NT = c->unit_rows;
     const uint32_t tiles = (c->ecount < np_max ? c->ecount + (np_max + NT - 1) / NT : np_max) + (sh_max + NT - 1) / NT;
-    WgemmExperts g{{ld.tiles[2], ld.tiles[3]}, {ld.tiles[5], ld.tiles[6]}, c->mma_items[0], c->n_items, c->n_items + 2, c->pairs, c->lut_pf, c->status, c->ecount, (uint32_t)c->n_sms};
+    WgemmExperts g{{ld.tiles[2], ld.tiles[3]}, {ld.tiles[5], ld.tiles[6]}, c->mma_items[0], c->n_items, c->n_items + 2, c->pairs, c->lut_pf, c->status, c->ecount, (uint32_t)c->n_sms, NT};
     QKM_LAUNCH(c, launch_wgemm_gateup(c->L(), d, ld.w.gateup_type, g, c->xb, c->xscale, c->xnorm, ld.w_norm, c->hb, c->hscale, tiles * (d.n_ff / 128)));
     c->prof_mark("moe.gu");
-    WgemmExperts m{{ld.tiles[4], nullptr}, {ld.tiles[7], nullptr}, c->mma_items[1], c->n_items + 1, c->n_items + 3, c->pairs, c->lut_pf, c->status, c->ecount, (uint32_t)c->n_sms};
+    WgemmExperts m{{ld.tiles[4], nullptr}, {ld.tiles[7], nullptr}, c->mma_items[1], c->n_items + 1, c->n_items + 3, c->pairs, c->lut_pf, c->status, c->ecount, (uint32_t)c->n_sms, NT};
     QKM_LAUNCH(c, launch_wgemm_down(c->L(), d, ld.w.down_type, m, c->hb, (uint64_t)c->cfg.max_tokens * (d.n_used + 1), c->hscale, sel, c->contrib_p,
                                     tiles * (d.n_embd / 256)));
     c->prof_mark("moe.dn");

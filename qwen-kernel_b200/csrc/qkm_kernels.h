@@ -136,7 +136,8 @@ cudaError_t launch_decode_down_any(const Launch& L, const DownDecodeArgs& a, uin
 
 // ---- qkm_wgemm.cu : tcgen05 GEMMs with quantised weights (batched prefill, dense projections)
 constexpr uint16_t kSharedItem = 0xFFFFu;   // MmaItem::expert of the shared expert's units
-uint32_t wgemm_rows_per_unit();             // activation rows per unit
+constexpr uint32_t kWgemmRows = 128, kWgemmRowsWide = 160;   // activation rows per unit
+uint32_t wgemm_rows_per_unit(const qkm_dims& d, uint32_t n_tokens);
 size_t wgemm_table_bytes();
 cudaError_t launch_wgemm_table(const Launch& L, uint8_t* out);
 // x rows as f16 in the kernels' element order (0, 2, 1, 3 in every group of four), scaled per row by a power of two
@@ -158,6 +159,7 @@ struct WgemmExperts {
     uint32_t* status;
     uint32_t n_experts;        // resident experts
     uint32_t n_sms;
+    uint32_t tile;             // rows per unit that `items` were cut with
 };
 // h (f16, scaled per pair position, element order as above) = silu(gate x) * (up x); w_norm [2][n_experts + 1]
 cudaError_t launch_wgemm_gateup(const Launch& L, const qkm_dims& d, uint32_t type, const WgemmExperts& x, const void* xrows,

@@ -47,22 +47,30 @@ namespace wg {
 constexpr int kProducerWarps = 16, kEpilogueWarps = 8;
 constexpr int kMmaWarp = kProducerWarps + kEpilogueWarps, kWeightWarp = kMmaWarp + 1, kRowWarp = kMmaWarp + 2;
 constexpr int kThreads = 1024;                  // eight warpgroups at 64 registers = all 65,536 of the SM
-// registers a thread after the split; 512 x 80 + 256 x 56 + 256 x 40 = 65,536, what the block was launched with
-constexpr int kProducerRegs = 80, kEpilogueRegs = 56, kOtherRegs = 40;
-static_assert(kProducerWarps * 32 * kProducerRegs + kEpilogueWarps * 32 * kEpilogueRegs + (32 - kProducerWarps - kEpilogueWarps) * 32 * kOtherRegs <= kThreads * 64,
-              "the shares must not exceed the launch's registers");
+// Registers a thread after the split, producers / epilogue / others; 512 P + 256 E + 256 O must not exceed the launch's 65,536.
+// (Gate/up with 160 rows: the row loaders' addresses; down: the epilogue, which is 40 % of a unit of eight k-steps, but for
+// Q6_K, whose producers would spill.)
+template <int FMT, int MODE, int NT> struct Regs { static constexpr int kProducer = 80, kEpilogue = 56, kOther = 40; };
+template <int FMT> struct Regs<FMT, 0, 160> { static constexpr int kProducer = 72, kEpilogue = 56, kOther = 56; };
+template <int NT> struct Regs<QKM_TYPE_IQ4_XS, 1, NT> { static constexpr int kProducer = 72, kEpilogue = 72, kOther = 40; };
+template <int N> __device__ __forceinline__ void set_regs() {   // from the launch's 64
+    static_assert(N % 8 == 0, "a multiple of eight");
+    if constexpr (N > 64) asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N));
+    if constexpr (N < 64) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N));
+}
 constexpr int kFeed = 4;                        // units handed out ahead
-constexpr int kStages = 4;                      // of (A: 64 TMEM columns, B: 128 rows x 64 f16)
-constexpr int kNT = 128;                        // activation rows per unit
-constexpr uint32_t kBTile = 128 * 128;
+// NT: activation rows per unit, 128 or 160.  Tensor memory's 512 columns hold two accumulators of NT and the A stages
+constexpr int kNT = kWgemmRows, kWideNT = kWgemmRowsWide;
+template <int NT> constexpr int stages() { return NT > 128 ? 3 : 4; }   // of (A: 64 TMEM columns, B: NT rows x 64 f16)
+template <int NT> constexpr uint32_t b_tile() { return NT * 128; }
 constexpr uint32_t kTab = 0x10000u, kTabBytes = 0x10000u, kLow = 0x1800u;
 template <int FMT> constexpr bool has_table() { return FMT == QKM_TYPE_IQ3_XXS || FMT == QKM_TYPE_IQ4_XS; }
 // Shared-window addresses.  With a table image (look-up addresses are byte permutes, so it has to start on a 64 KB
-// boundary): three B stages below it, the fourth and the weight buffers above; else everything in one run.
-template <int FMT> __device__ __forceinline__ uint32_t b_addr(uint32_t s) {
-    return has_table<FMT>() && s == 3 ? kTab + kTabBytes : kLow + s * kBTile;
+// boundary): all B stages but one below it, the last and the weight buffers above; else everything in one run.
+template <int FMT, int NT> __device__ __forceinline__ uint32_t b_addr(uint32_t s) {
+    return has_table<FMT>() && s + 1 == stages<NT>() ? kTab + kTabBytes : kLow + s * b_tile<NT>();
 }
-template <int FMT> constexpr uint32_t w_base() { return has_table<FMT>() ? kTab + kTabBytes + kBTile : kLow + kStages * kBTile; }
+template <int FMT, int NT> constexpr uint32_t w_base() { return has_table<FMT>() ? kTab + kTabBytes + b_tile<NT>() : kLow + stages<NT>() * b_tile<NT>(); }
 template <int FMT> constexpr uint32_t tile_size() {
     return FMT == QKM_TYPE_IQ3_XXS ? kTileIq3 : FMT == QKM_TYPE_IQ4_XS ? kTileIq4 : FMT == QKM_TYPE_Q6_K ? kTileQ6 : kTileQ8;
 }
@@ -74,10 +82,11 @@ template <int FMT> constexpr uint32_t w_bytes() {
     const uint32_t slots = q8_slots<FMT>() * kQ8Slot, tiles = 16u * tile_size<FMT>();
     return tiles > slots ? tiles : slots;
 }
-template <int FMT> constexpr uint32_t smem_end() { return w_base<FMT>() + 2 * w_bytes<FMT>(); }
-constexpr uint32_t kTmemA = 256;                // accumulators in columns [0,256), A stages behind them
+template <int FMT, int NT> constexpr uint32_t smem_end() { return w_base<FMT, NT>() + 2 * w_bytes<FMT>(); }
+template <int NT> constexpr uint32_t tmem_a() { return 2 * NT; }   // accumulators first, A stages behind them
 enum Mode { kGateUp = 0, kDown = 1, kDense = 2 };
-template <int MODE> constexpr uint32_t row_warps() { return MODE == kGateUp ? kStages : 1; }
+template <int MODE, int NT> constexpr uint32_t warps_per_stage() { return MODE == kGateUp && NT > 128 ? 2 : 1; }   // row loaders
+template <int MODE, int NT> constexpr uint32_t row_warps() { return MODE == kGateUp ? stages<NT>() * warps_per_stage<MODE, NT>() : 1; }
 }  // namespace wg
 
 // ---- table image: row i (256 bytes) = IQ3_XXS grid entry i as f16 in element order (0, 2, 1, 3), 8 bytes for each of
@@ -253,17 +262,22 @@ struct WgemmArgs {
     uint32_t n_dense;           // dense: activation rows
 };
 
-template <int FMT, int MODE>
+template <int FMT, int MODE, int NT>
 __global__ void __launch_bounds__(wg::kThreads, 1)
 wgemm_kernel(const WgemmArgs a, const __grid_constant__ CUtensorMap rows_map) {
     extern __shared__ __align__(1024) uint8_t smem_dyn[];
-    constexpr int kSt = wg::kStages;
-    constexpr uint32_t kSlots = wg::q8_slots<FMT>();
+    constexpr int kSt = wg::stages<NT>();
+    using R = wg::Regs<FMT, MODE, NT>;
+    static_assert(wg::kProducerWarps * 32 * R::kProducer + wg::kEpilogueWarps * 32 * R::kEpilogue + (32 - wg::kProducerWarps - wg::kEpilogueWarps) * 32 * R::kOther <= wg::kThreads * 64,
+                  "the shares must not exceed the launch's registers");
+    static_assert(wg::tmem_a<NT>() + kSt * 64 <= 512 && (!wg::has_table<FMT>() || wg::kLow + (kSt - 1) * wg::b_tile<NT>() <= wg::kTab), "room");
+    constexpr uint32_t kSlots = wg::q8_slots<FMT>(), kRowWarps = wg::row_warps<MODE, NT>(), kPer = wg::warps_per_stage<MODE, NT>();
+    static_assert(wg::kRowWarp + kRowWarps <= 32, "room");
     __shared__ __align__(8) unsigned long long s_bar[2 * kSt + 4 * kSlots + 6 + 2 * wg::kFeed];
     __shared__ MmaItem s_feed[wg::kFeed];
     __shared__ uint32_t s_tmem;
-    __shared__ __align__(16) uint32_t s_rows[MODE == wg::kGateUp ? wg::kStages : 1][wg::kNT];   // row loaders: where the unit's rows start, [row % 4][row / 4]
-    __shared__ float s_col[2][2][wg::kNT];   // epilogue, per unit parity: factors of the unit's columns
+    __shared__ __align__(16) uint32_t s_rows[MODE == wg::kGateUp ? kRowWarps : 1][NT / kPer];   // row loaders: where the unit's rows start, [row % 4][row / 4]
+    __shared__ float s_col[2][2][NT];   // epilogue, per unit parity: factors of the unit's columns
     const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31u;
     const uint32_t KB = a.K / 256, RT16 = a.rows / 16;
     const uint32_t row_units = MODE == wg::kGateUp ? a.rows / 128 : (a.rows / 128 + 1) / 2;
@@ -271,7 +285,7 @@ wgemm_kernel(const WgemmArgs a, const __grid_constant__ CUtensorMap rows_map) {
         const uint32_t dyn_base = smem_addr(smem_dyn);
         uint32_t dyn_size;
         asm("mov.u32 %0, %%dynamic_smem_size;" : "=r"(dyn_size));
-        if (dyn_base > wg::kLow || dyn_base + dyn_size < wg::smem_end<FMT>()) {
+        if (dyn_base > wg::kLow || dyn_base + dyn_size < wg::smem_end<FMT, NT>()) {
             if (tid == 0) atomicExch(a.status, (uint32_t)kStatusBadLayout);
             return;
         }
@@ -281,9 +295,8 @@ wgemm_kernel(const WgemmArgs a, const __grid_constant__ CUtensorMap rows_map) {
     const uint32_t bar_accfull = bar_wempty + 16 * kSlots, bar_accfree = bar_accfull + 16, bar_tab = bar_accfree + 16;
     const uint32_t bar_ufull = bar_tab + 8, bar_uempty = bar_ufull + 8 * wg::kFeed;
     const uint32_t bar_cols = bar_uempty + 8 * wg::kFeed;   // the epilogue's warps among themselves
-    constexpr uint32_t kRowWarps = wg::row_warps<MODE>();
     if (tid == 0) {
-        for (int s = 0; s < kSt; ++s) { mbar_init(bar_full + 8 * s, 9); mbar_init(bar_empty + 8 * s, 1); }   // eight producer warps + the row loader; one commit
+        for (int s = 0; s < kSt; ++s) { mbar_init(bar_full + 8 * s, 8 + kPer); mbar_init(bar_empty + 8 * s, 1); }   // eight producer warps + the row loaders; one commit
         for (uint32_t b = 0; b < 2 * kSlots; ++b) { mbar_init(bar_wfull + 8 * b, 1); mbar_init(bar_wempty + 8 * b, 8); }
         for (int b = 0; b < wg::kFeed; ++b) { mbar_init(bar_ufull + 8 * b, 1); mbar_init(bar_uempty + 8 * b, wg::kProducerWarps + wg::kEpilogueWarps + 1 + kRowWarps); }
         for (int b = 0; b < 2; ++b) {
@@ -305,7 +318,7 @@ wgemm_kernel(const WgemmArgs a, const __grid_constant__ CUtensorMap rows_map) {
     if (MODE != wg::kDense) pdl_wait();
     __syncthreads();
     umma::fence_after_sync();
-    const uint32_t n_units = MODE == wg::kDense ? (a.n_dense + wg::kNT - 1) / wg::kNT * row_units : *a.n_items;
+    const uint32_t n_units = MODE == wg::kDense ? (a.n_dense + NT - 1) / NT * row_units : *a.n_items;
     const uint32_t tmem = s_tmem;
     bool timed_out = false;
     auto wait_bar = [&](uint32_t b, uint32_t parity) -> bool { return timed_out || mbar_wait_timed(b, parity); };   // a thread waits out the limit once at most
@@ -316,8 +329,8 @@ wgemm_kernel(const WgemmArgs a, const __grid_constant__ CUtensorMap rows_map) {
         MmaItem it;
         it.expert = 0;
         it.rt = (uint16_t)(u % row_units);
-        it.pair_off = (u / row_units) * wg::kNT;
-        it.n = min((uint32_t)wg::kNT, a.n_dense - it.pair_off);
+        it.pair_off = (u / row_units) * NT;
+        it.n = min((uint32_t)NT, a.n_dense - it.pair_off);
         return it;
     };
     // the k-th unit of this block, from the weight loader; false after the last
@@ -335,22 +348,26 @@ wgemm_kernel(const WgemmArgs a, const __grid_constant__ CUtensorMap rows_map) {
     auto step_kb = [&](uint32_t i) -> uint32_t { return i < (KB & ~1u) * 4 ? 2 * (i >> 3) + (i & 1u) : KB - 1; };
     auto step_q = [&](uint32_t i) -> uint32_t { return i < (KB & ~1u) * 4 ? (i >> 1) & 3u : i & 3u; };
     const uint32_t KS = KB * 4;
+    // stage of k-step i of a unit, and how often the stage was used earlier; `before` grows by `advance` a unit: k-steps, or rounds of four stages
+    const uint32_t advance = kSt == 4 ? KB : KS;
+    auto stage_of = [](uint32_t before, uint32_t i) -> uint32_t { return kSt == 4 ? i & 3u : (before + i) % kSt; };
+    auto round_of = [](uint32_t before, uint32_t i) -> uint32_t { return kSt == 4 ? before + (i >> 2) : (before + i) / kSt; };
 
     if (warp < (uint32_t)wg::kProducerWarps) {
         // ---- producers
-        asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(wg::kProducerRegs));
+        wg::set_regs<R::kProducer>();
         const uint32_t lq = warp & 3u, mat = (warp >> 2) & 1u, par = warp >> 3;
         const uint32_t r = 32 * lq + lane, r16 = r & 15u, g = r16 & 7u, tl = r >> 4;   // row of the 128, row of its tile, tile
-        const uint32_t a_lane = tmem + ((32 * lq) << 16) + wg::kTmemA + mat * 32u;
-        const uint32_t wbuf = wg::w_base<FMT>() + par * wg::w_bytes<FMT>();
+        const uint32_t a_lane = tmem + ((32 * lq) << 16) + wg::tmem_a<NT>() + mat * 32u;
+        const uint32_t wbuf = wg::w_base<FMT, NT>() + par * wg::w_bytes<FMT>();
         const uint32_t tab_c = wg::kTab + (FMT == QKM_TYPE_IQ3_XXS ? (lane & 15u) * 8u : 128u + lane * 4u);
         if (FMT == QKM_TYPE_IQ3_XXS || FMT == QKM_TYPE_IQ4_XS)
             if (!wait_bar(bar_tab, 0)) timed_out = true;
         // dense: scale and product rounded to f16 (two roundings of 2^-12, a fifth fewer instructions); experts: one rounding that counts
         auto weight_scale = [](float v) { if constexpr (MODE == wg::kDense) return __float2half2_rn(v); else return split_scale(v); };
-        uint32_t round0 = 0, wcnt = 0, qcnt = 0;   // stage rounds before this unit; blocks and Q8_0 slots consumed
+        uint32_t before = 0, wcnt = 0, qcnt = 0;   // what came before this unit; blocks and Q8_0 slots consumed
         MmaItem it;
-        for (uint32_t k = 0; next_unit(k, it); ++k, round0 += KB) {
+        for (uint32_t k = 0; next_unit(k, it); ++k, before += advance) {
             const bool shared = MODE != wg::kDense && it.expert == kSharedItem;
             // A step's stores are not waited for at its end: it is announced when the next step's first values have been computed,
             // by which time they are through (waiting at once cost a tenth of the kernel).
@@ -360,16 +377,16 @@ wgemm_kernel(const WgemmArgs a, const __grid_constant__ CUtensorMap rows_map) {
                 tmem_st_wait();
                 umma::fence_before_sync();
                 __syncwarp();
-                if (lane == 0) mbar_arrive(bar_full + 8 * (pending & 3u));
+                if (lane == 0) mbar_arrive(bar_full + 8 * pending);
             };
             auto store = [&](uint32_t i, uint32_t half, const uint32_t (&o)[16]) {   // half `half` of k-step i's 64 columns
                 if (half == 0) {
                     announce();
-                    const uint32_t round = round0 + (i >> 2);   // the stage is free to be written
-                    if (round && !wait_bar(bar_empty + 8 * (i & 3u), (round - 1) & 1u)) timed_out = true;
+                    const uint32_t stage = stage_of(before, i), round = round_of(before, i);   // the stage is free to be written
+                    if (round && !wait_bar(bar_empty + 8 * stage, (round - 1) & 1u)) timed_out = true;
                     umma::fence_after_sync();
-                    st = a_lane + (i & 3u) * 64u;
-                    pending = i;
+                    st = a_lane + stage * 64u;
+                    pending = stage;
                 }
                 tmem_st16(st + 16 * half, o);
             };
@@ -527,7 +544,7 @@ wgemm_kernel(const WgemmArgs a, const __grid_constant__ CUtensorMap rows_map) {
     } else if (warp < (uint32_t)wg::kMmaWarp) {
         // ---- epilogue: warps e and e + 4 read TMEM lanes 32 e .. 32 e + 31, every other 16 columns each (with four warps the drain of
         // 128 columns took 13,000 cycles a gate/up unit, a third of the time at 4096 tokens)
-        asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(wg::kEpilogueRegs));
+        wg::set_regs<R::kEpilogue>();
         if (MODE == wg::kDense) pdl_wait();
         const uint32_t e = warp & 3u, eh = (warp >> 2) & 1u, c = tid - wg::kProducerWarps * 32;   // c: the column this thread prepares
         uint32_t used[2] = {0, 0}, next = 0, iter = 0;
@@ -564,7 +581,7 @@ wgemm_kernel(const WgemmArgs a, const __grid_constant__ CUtensorMap rows_map) {
             if (big) { if (!wait_bar(bar_accfull + 8, used[1] & 1u)) timed_out = true; ++used[0]; ++used[1]; next = 0; }
             else { ++used[b]; next ^= 1u; }
             umma::fence_after_sync();
-            const uint32_t t0 = tmem + ((32 * e) << 16) + b * 128u, t1 = t0 + (big ? 128u : 64u);
+            const uint32_t t0 = tmem + ((32 * e) << 16) + b * 128u, t1 = t0 + (big ? (uint32_t)NT : 64u);
             const uint32_t row = 32 * e + lane;
             for (uint32_t cb = 16 * eh; cb < n_mma; cb += 32) {
                 uint32_t v0[16], v1[16];
@@ -598,13 +615,13 @@ wgemm_kernel(const WgemmArgs a, const __grid_constant__ CUtensorMap rows_map) {
             if (lane == 0) { mbar_arrive(bar_accfree + 8 * b); if (big) mbar_arrive(bar_accfree + 8); }
         }
     } else {
-    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(wg::kOtherRegs));
+    wg::set_regs<R::kOther>();
     if (warp == (uint32_t)wg::kMmaWarp) {
         // ---- MMA issue: the whole warp walks the loop, one elected lane issues
         const bool leader = umma::elect_one();
-        uint32_t used[2] = {0, 0}, next = 0, round0 = 0;
+        uint32_t used[2] = {0, 0}, next = 0, before = 0;
         MmaItem it;
-        for (uint32_t k = 0; next_unit(k, it); ++k, round0 += KB) {
+        for (uint32_t k = 0; next_unit(k, it); ++k, before += advance) {
             const uint32_t n_mma = (it.n + 15u) & ~15u;
             const bool big = n_mma > 64;
             const uint32_t b = big ? 0u : next, idesc = umma::instr_desc_f16(n_mma);
@@ -613,13 +630,13 @@ wgemm_kernel(const WgemmArgs a, const __grid_constant__ CUtensorMap rows_map) {
             if (big && used[1] && !wait_bar(bar_accfree + 8, (used[1] - 1) & 1u)) timed_out = true;
             if (big) { ++used[0]; ++used[1]; next = 0; } else { ++used[b]; next ^= 1u; }
             umma::fence_after_sync();
-            const uint32_t t0 = tmem + b * 128u, t1 = t0 + (big ? 128u : 64u);
+            const uint32_t t0 = tmem + b * 128u, t1 = t0 + (big ? (uint32_t)NT : 64u);
             for (uint32_t i = 0; i < KS; ++i) {
-                const uint32_t stage = i & 3u;
-                if (!wait_bar(bar_full + 8 * stage, (round0 + (i >> 2)) & 1u)) timed_out = true;
+                const uint32_t stage = stage_of(before, i);
+                if (!wait_bar(bar_full + 8 * stage, round_of(before, i) & 1u)) timed_out = true;
                 umma::fence_after_sync();
-                const uint64_t d_b = umma::smem_desc(wg::b_addr<FMT>(stage));
-                const uint32_t t_a = tmem + wg::kTmemA + stage * 64u;
+                const uint64_t d_b = umma::smem_desc(wg::b_addr<FMT, NT>(stage));
+                const uint32_t t_a = tmem + wg::tmem_a<NT>() + stage * 64u;
                 if (leader) {
 #pragma unroll
                     for (int j = 0; j < 4; ++j) {   // 16 columns of K further: 8 tensor-memory columns, 32 bytes of the row tile
@@ -673,7 +690,7 @@ wgemm_kernel(const WgemmArgs a, const __grid_constant__ CUtensorMap rows_map) {
                             ++slots[par];
                             if (lane == 0) mbar_expect_tx(wf, wg::kQ8Slot);
                             __syncwarp();
-                            if (lane < 16) bulk_g2s(wg::w_base<FMT>() + par * wg::w_bytes<FMT>() + slot * wg::kQ8Slot + lane * 1088u,
+                            if (lane < 16) bulk_g2s(wg::w_base<FMT, NT>() + par * wg::w_bytes<FMT>() + slot * wg::kQ8Slot + lane * 1088u,
                                                     src + (size_t)(lone ? kp : kp + par) * RT16 * kTileQ8 + q * 1088u, 1088u, wf);
                         }
                 } else {
@@ -684,38 +701,41 @@ wgemm_kernel(const WgemmArgs a, const __grid_constant__ CUtensorMap rows_map) {
                         ++blocks[par];
                         if (lane == 0) mbar_expect_tx(wf, 16 * tile);
                         __syncwarp();
-                        if (lane < 2) bulk_g2s(wg::w_base<FMT>() + par * wg::w_bytes<FMT>() + lane * 8 * tile, src + (size_t)(lone ? kp : kp + par) * RT16 * tile, 8 * tile, wf);
+                        if (lane < 2) bulk_g2s(wg::w_base<FMT, NT>() + par * wg::w_bytes<FMT>() + lane * 8 * tile, src + (size_t)(lone ? kp : kp + par) * RT16 * tile, 8 * tile, wf);
                     }
                 }
             }
             u = __shfl_sync(0xFFFFFFFFu, ticket, 0);
         }
-    } else if (MODE == wg::kGateUp && warp < wg::kRowWarp + wg::row_warps<MODE>()) {
-        // ---- scattered activation rows: a warp per stage, which copies four rows x 64 columns per instruction, waits for their
-        // arrival and announces the step.  (Two warps that shared every step and announced it two steps later, so as
+    } else if (MODE == wg::kGateUp && warp < wg::kRowWarp + wg::row_warps<MODE, NT>()) {
+        // ---- scattered activation rows: a warp per stage (two, which take every other 16 rows, for tiles of 160), which copies four rows
+        // x 64 columns per instruction, waits for their arrival and announces the step.  A copy issues every 55 cycles or so, and from
+        // about 100 rows on that is what a stage waits for: gate/up at 4096 tokens 236 -> 227 us with more registers for the
+        // addresses (56 a thread), 213 with the second warp; the tiles of 128 have four stages and no warps left.  (Two warps that shared every step and announced it two steps later, so as
         // not to wait, kept two stages in flight: the producers waited 40 to 60 % of their time for a free stage.)
         // Past the unit's end: the last row again (nobody reads those columns)
-        const uint32_t w = warp - wg::kRowWarp, rr = lane >> 3, c = lane & 7u;
-        const uint32_t dst = wg::b_addr<FMT>(w), d0 = dst + rr * 128u + ((c ^ rr) << 4), d1 = dst + (rr + 4) * 128u + ((c ^ (rr + 4)) << 4);
-        const uint32_t rows = smem_addr(&s_rows[w][rr * 32]);
-        uint32_t round = 0;
+        const uint32_t wi = warp - wg::kRowWarp, w = wi % kSt, part = wi / kSt, rr = lane >> 3, c = lane & 7u;   // groups of 16 rows: part, part + kPer, ...
+        const uint32_t dst = wg::b_addr<FMT, NT>(w) + part * 2048u, d0 = dst + rr * 128u + ((c ^ rr) << 4), d1 = dst + (rr + 4) * 128u + ((c ^ (rr + 4)) << 4);
+        const uint32_t rows = smem_addr(&s_rows[wi][rr * (NT / 4 / kPer)]);
+        uint32_t round = 0, before = 0;
         MmaItem it;
-        for (uint32_t k = 0; next_unit(k, it); ++k) {
+        for (uint32_t k = 0; next_unit(k, it); ++k, before += advance) {
             const uint32_t groups = ((it.n + 15u) & ~15u) / 4;   // of four rows, a multiple of four
             for (uint32_t r = lane; r < 4 * groups; r += 32)
-                s_rows[w][(r & 3u) * 32 + (r >> 2)] = (a.pairs[it.pair_off + min(r, it.n - 1)] >> 4) * (a.K / 8);   // in 16-byte pieces
+                if (kPer == 1 || (r >> 4) % kPer == part)
+                    s_rows[wi][(r & 3u) * (NT / 4 / kPer) + (r >> 4) / kPer * 4 + ((r >> 2) & 3u)] = (a.pairs[it.pair_off + min(r, it.n - 1)] >> 4) * (a.K / 8);   // in 16-byte pieces
             __syncwarp();
-            for (uint32_t i = w; i < KS; i += 4, ++round) {
+            for (uint32_t i = kSt == 4 ? w : (w + kSt - before % kSt) % kSt; i < KS; i += kSt, ++round) {
                 if (round && !wait_bar(bar_empty + 8 * w, (round - 1) & 1u)) timed_out = true;
                 const uint4* src = reinterpret_cast<const uint4*>(a.xrows) + step_kb(i) * 32u + step_q(i) * 8u + c;
 #pragma unroll
-                for (int b = 0; b < 8; ++b)
-                    if (4u * b < groups) {
+                for (int b = 0; b < NT / 16 / (int)kPer; ++b)
+                    if (4u * (kPer * b + part) < groups) {
                         const uint4 o4 = lds128(rows + 16 * b);
                         const uint32_t o[4] = {o4.x, o4.y, o4.z, o4.w};
 #pragma unroll
                         for (int j = 0; j < 4; ++j)
-                            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(((j & 1) ? d1 : d0) + (2 * b + (j >> 1)) * 1024u), "l"(src + o[j]) : "memory");
+                            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(((j & 1) ? d1 : d0) + (2 * kPer * b + (j >> 1)) * 1024u), "l"(src + o[j]) : "memory");
                     }
                 asm volatile("cp.async.wait_all;" ::: "memory");
                 umma::fence_smem_to_async();
@@ -732,12 +752,12 @@ wgemm_kernel(const WgemmArgs a, const __grid_constant__ CUtensorMap rows_map) {
         for (uint32_t k = 0; next_unit(k, it); ++k) {
             const uint32_t boxes = (it.n + 15u) / 16;
             for (uint32_t i = 0; i < KS; ++i, ++gs) {
-                const uint32_t stage = gs & 3u;
-                if (gs >= 4 && !wait_bar(bar_empty + 8 * stage, ((gs >> 2) - 1) & 1u)) timed_out = true;
+                const uint32_t stage = gs % kSt;
+                if (gs >= kSt && !wait_bar(bar_empty + 8 * stage, (gs / kSt - 1) & 1u)) timed_out = true;
                 if (__any_sync(0xFFFFFFFFu, timed_out)) break;   // a barrier that still counts bytes takes no second arrival
                 if (lane == 0) mbar_expect_tx(bar_full + 8 * stage, boxes * 2048u);
                 __syncwarp();
-                if (lane < boxes) tma_rows16(wg::b_addr<FMT>(stage) + lane * 2048u, &rows_map, step_kb(i) * 256u + step_q(i) * 64u, it.pair_off + 16 * lane, bar_full + 8 * stage);
+                if (lane < boxes) tma_rows16(wg::b_addr<FMT, NT>(stage) + lane * 2048u, &rows_map, step_kb(i) * 256u + step_q(i) * 64u, it.pair_off + 16 * lane, bar_full + 8 * stage);
             }
         }
     }
@@ -933,19 +953,24 @@ static bool rows_tensor_map(CUtensorMap* map, const void* rows, uint64_t n_rows,
                   CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-template <int FMT, int MODE>
+template <int FMT, int MODE, int NT = wg::kNT>
 static cudaError_t wgemm_launch(const Launch& L, const WgemmArgs& a, const void* rows, uint64_t n_rows, uint32_t max_units, uint32_t n_sms) {
     if (max_units == 0) return cudaSuccess;
-    if (const cudaError_t e = allow_dynamic_smem<wgemm_kernel<FMT, MODE>>((int)wg::smem_end<FMT>())) return e;
+    if (const cudaError_t e = allow_dynamic_smem<wgemm_kernel<FMT, MODE, NT>>((int)wg::smem_end<FMT, NT>())) return e;
     CUtensorMap map{};
     if (((uintptr_t)rows & 15u) || (MODE != wg::kGateUp && !rows_tensor_map(&map, rows, n_rows, a.K))) return cudaErrorInvalidValue;
-    const cudaError_t e = launch_kernel(Launch{L.stream, nullptr, true}, wgemm_kernel<FMT, MODE>, dim3(max_units < n_sms ? max_units : n_sms), dim3(wg::kThreads),
-                                        wg::smem_end<FMT>(), a, map);
+    const cudaError_t e = launch_kernel(Launch{L.stream, nullptr, true}, wgemm_kernel<FMT, MODE, NT>, dim3(max_units < n_sms ? max_units : n_sms), dim3(wg::kThreads),
+                                        wg::smem_end<FMT, NT>(), a, map);
     L.count();
     return e != cudaSuccess ? e : cudaGetLastError();
 }
 
-uint32_t wgemm_rows_per_unit() { return wg::kNT; }
+// 160 rows from an average of 104 pairs an expert on: with tiles of 128 more and more experts need a second expansion of their weights for
+// a few pairs, and two row loaders a stage make up for the fourth stage.  Layer, 256 experts, top 8, IQ3_XXS and IQ4_XS, tiles of 128 -> 160:
+// 3000 tokens 423 -> 426 us, 3500: 462 -> 459, 3840: 518 -> 495, 4096: 561 -> 507, 5120: 697 -> 649, 6144: 776 -> 778, 8192: 990 -> 939.
+uint32_t wgemm_rows_per_unit(const qkm_dims& d, uint32_t n) {
+    return (uint64_t)n * d.n_used > 104ull * d.n_expert ? kWgemmRowsWide : kWgemmRows;
+}
 
 cudaError_t launch_wgemm_gateup(const Launch& L, const qkm_dims& d, uint32_t type, const WgemmExperts& x, const void* xrows,
                                 const float* x_inv_scale, const float* x_norm, const float* w_norm, void* h, float* h_inv_scale, uint32_t max_units) {
@@ -954,8 +979,10 @@ cudaError_t launch_wgemm_gateup(const Launch& L, const qkm_dims& d, uint32_t typ
     a.items = x.items; a.n_items = x.n_items; a.ticket = x.ticket; a.pairs = x.pairs; a.x_inv_scale = x_inv_scale; a.x_norm = x_norm; a.w_norm = w_norm;
     a.xrows = (const __half*)xrows; a.h = (__half*)h; a.h_inv_scale = h_inv_scale; a.table = x.table; a.status = x.status; a.rows = d.n_ff; a.K = d.n_embd;
     a.n_experts = x.n_experts; a.n_used = d.n_used;
-    if (type == QKM_TYPE_IQ3_XXS) return wgemm_launch<QKM_TYPE_IQ3_XXS, wg::kGateUp>(L, a, xrows, 0, max_units, x.n_sms);
-    if (type == QKM_TYPE_IQ4_XS) return wgemm_launch<QKM_TYPE_IQ4_XS, wg::kGateUp>(L, a, xrows, 0, max_units, x.n_sms);
+    if (type == QKM_TYPE_IQ3_XXS)
+        return x.tile > wg::kNT ? wgemm_launch<QKM_TYPE_IQ3_XXS, wg::kGateUp, wg::kWideNT>(L, a, xrows, 0, max_units, x.n_sms) : wgemm_launch<QKM_TYPE_IQ3_XXS, wg::kGateUp>(L, a, xrows, 0, max_units, x.n_sms);
+    if (type == QKM_TYPE_IQ4_XS)
+        return x.tile > wg::kNT ? wgemm_launch<QKM_TYPE_IQ4_XS, wg::kGateUp, wg::kWideNT>(L, a, xrows, 0, max_units, x.n_sms) : wgemm_launch<QKM_TYPE_IQ4_XS, wg::kGateUp>(L, a, xrows, 0, max_units, x.n_sms);
     return cudaErrorInvalidValue;
 }
 
@@ -966,8 +993,10 @@ cudaError_t launch_wgemm_down(const Launch& L, const qkm_dims& d, uint32_t type,
     a.w[0] = a.w[1] = (const uint8_t*)x.w[0]; a.sh[0] = a.sh[1] = (const uint8_t*)x.sh[0];
     a.items = x.items; a.n_items = x.n_items; a.ticket = x.ticket; a.pairs = x.pairs; a.h_inv_scale = const_cast<float*>(h_inv_scale); a.sel = sel; a.out = contrib;
     a.table = x.table; a.status = x.status; a.rows = d.n_embd; a.K = d.n_ff; a.n_experts = x.n_experts; a.n_used = d.n_used;
-    if (type == QKM_TYPE_IQ4_XS) return wgemm_launch<QKM_TYPE_IQ4_XS, wg::kDown>(L, a, h, n_hrows, max_units, x.n_sms);
-    if (type == QKM_TYPE_Q6_K) return wgemm_launch<QKM_TYPE_Q6_K, wg::kDown>(L, a, h, n_hrows, max_units, x.n_sms);
+    if (type == QKM_TYPE_IQ4_XS)
+        return x.tile > wg::kNT ? wgemm_launch<QKM_TYPE_IQ4_XS, wg::kDown, wg::kWideNT>(L, a, h, n_hrows, max_units, x.n_sms) : wgemm_launch<QKM_TYPE_IQ4_XS, wg::kDown>(L, a, h, n_hrows, max_units, x.n_sms);
+    if (type == QKM_TYPE_Q6_K)
+        return x.tile > wg::kNT ? wgemm_launch<QKM_TYPE_Q6_K, wg::kDown, wg::kWideNT>(L, a, h, n_hrows, max_units, x.n_sms) : wgemm_launch<QKM_TYPE_Q6_K, wg::kDown>(L, a, h, n_hrows, max_units, x.n_sms);
     return cudaErrorInvalidValue;
 }
 
