@@ -58,7 +58,7 @@ struct qkm_ctx {
     float* xscale = nullptr;          // [max_tokens]
     uint32_t* n_items = nullptr;      // prefill: units of [0] gate/up, [1] down; [2], [3] their tickets
     uint32_t* status = nullptr;       // kernel status word (device)
-    uint32_t* route_counter = nullptr; // ticket counter of the selection kernel's grouping tail (device, stays zero)
+    uint32_t* route_counter = nullptr; // ticket counter of the decode router's selection (device, stays zero)
     // fused decode sequence (router + grouping + planes -> gate/up -> down, three launches)
     bool dec_ok = false;               // dims fit the fused decode kernels
     int8_t* planes8 = nullptr;         // [max_tokens][n_embd/256][8][256]
