@@ -85,8 +85,8 @@ template <int FMT> constexpr uint32_t w_bytes() {
 template <int FMT, int NT> constexpr uint32_t smem_end() { return w_base<FMT, NT>() + 2 * w_bytes<FMT>(); }
 template <int NT> constexpr uint32_t tmem_a() { return 2 * NT; }   // accumulators first, A stages behind them
 enum Mode { kGateUp = 0, kDown = 1, kDense = 2 };
-template <int MODE, int NT> constexpr uint32_t warps_per_stage() { return MODE == kGateUp && NT > 128 ? 2 : 1; }   // row loaders
-template <int MODE, int NT> constexpr uint32_t row_warps() { return MODE == kGateUp ? stages<NT>() * warps_per_stage<MODE, NT>() : 1; }
+template <int MODE> constexpr uint32_t warps_per_step() { return MODE == kGateUp ? 2 : 1; }   // row loaders
+template <int MODE> constexpr uint32_t row_warps() { return MODE == kGateUp ? 6 : 1; }
 }  // namespace wg
 
 // ---- table image: row i (256 bytes) = IQ3_XXS grid entry i as f16 in element order (0, 2, 1, 3), 8 bytes for each of
@@ -271,7 +271,7 @@ wgemm_kernel(const WgemmArgs a, const __grid_constant__ CUtensorMap rows_map) {
     static_assert(wg::kProducerWarps * 32 * R::kProducer + wg::kEpilogueWarps * 32 * R::kEpilogue + (32 - wg::kProducerWarps - wg::kEpilogueWarps) * 32 * R::kOther <= wg::kThreads * 64,
                   "the shares must not exceed the launch's registers");
     static_assert(wg::tmem_a<NT>() + kSt * 64 <= 512 && (!wg::has_table<FMT>() || wg::kLow + (kSt - 1) * wg::b_tile<NT>() <= wg::kTab), "room");
-    constexpr uint32_t kSlots = wg::q8_slots<FMT>(), kRowWarps = wg::row_warps<MODE, NT>(), kPer = wg::warps_per_stage<MODE, NT>();
+    constexpr uint32_t kSlots = wg::q8_slots<FMT>(), kRowWarps = wg::row_warps<MODE>(), kPer = wg::warps_per_step<MODE>();
     static_assert(wg::kRowWarp + kRowWarps <= 32, "room");
     __shared__ __align__(8) unsigned long long s_bar[2 * kSt + 4 * kSlots + 6 + 2 * wg::kFeed];
     __shared__ MmaItem s_feed[wg::kFeed];
@@ -707,17 +707,18 @@ wgemm_kernel(const WgemmArgs a, const __grid_constant__ CUtensorMap rows_map) {
             }
             u = __shfl_sync(0xFFFFFFFFu, ticket, 0);
         }
-    } else if (MODE == wg::kGateUp && warp < wg::kRowWarp + wg::row_warps<MODE, NT>()) {
-        // ---- scattered activation rows: a warp per stage (two, which take every other 16 rows, for tiles of 160), which copies four rows
-        // x 64 columns per instruction, waits for their arrival and announces the step.  A copy issues every 55 cycles or so, and from
-        // about 100 rows on that is what a stage waits for: gate/up at 4096 tokens 236 -> 227 us with more registers for the
-        // addresses (56 a thread), 213 with the second warp; the tiles of 128 have four stages and no warps left.  (Two warps that shared every step and announced it two steps later, so as
-        // not to wait, kept two stages in flight: the producers waited 40 to 60 % of their time for a free stage.)
+    } else if (MODE == wg::kGateUp && warp < wg::kRowWarp + wg::row_warps<MODE>()) {
+        // ---- scattered activation rows: six warps; two, which take every other 16 rows, copy a step (four rows x 64 columns per
+        // instruction), wait for its arrival and announce it, and three pairs take the steps in turn.  A copy issues every 55 cycles or
+        // so, and from about 100 rows on that is what a stage waits for: gate/up at 4096 tokens, tiles of 160, 236 us with one warp
+        // a step, 227 with more registers for the addresses (56 a thread), 213 with two; 3200 tokens, tiles of 128, 189 -> 181.
+        // (Two warps that shared every step and announced it two steps later, so as not to wait, kept two stages in flight: the
+        // producers waited 40 to 60 % of their time for a free stage.)
         // Past the unit's end: the last row again (nobody reads those columns)
-        const uint32_t wi = warp - wg::kRowWarp, w = wi % kSt, part = wi / kSt, rr = lane >> 3, c = lane & 7u;   // groups of 16 rows: part, part + kPer, ...
-        const uint32_t dst = wg::b_addr<FMT, NT>(w) + part * 2048u, d0 = dst + rr * 128u + ((c ^ rr) << 4), d1 = dst + (rr + 4) * 128u + ((c ^ (rr + 4)) << 4);
+        const uint32_t wi = warp - wg::kRowWarp, w = wi % 3u, part = wi / 3u, rr = lane >> 3, c = lane & 7u;   // groups of 16 rows: part, part + kPer, ...
+        const uint32_t d0 = part * 2048u + rr * 128u + ((c ^ rr) << 4), d1 = part * 2048u + (rr + 4) * 128u + ((c ^ (rr + 4)) << 4);
         const uint32_t rows = smem_addr(&s_rows[wi][rr * (NT / 4 / kPer)]);
-        uint32_t round = 0, before = 0;
+        uint32_t before = 0, first = w;   // first: this warp's first step of the unit
         MmaItem it;
         for (uint32_t k = 0; next_unit(k, it); ++k, before += advance) {
             const uint32_t groups = ((it.n + 15u) & ~15u) / 4;   // of four rows, a multiple of four
@@ -725,8 +726,10 @@ wgemm_kernel(const WgemmArgs a, const __grid_constant__ CUtensorMap rows_map) {
                 if (kPer == 1 || (r >> 4) % kPer == part)
                     s_rows[wi][(r & 3u) * (NT / 4 / kPer) + (r >> 4) / kPer * 4 + ((r >> 2) & 3u)] = (a.pairs[it.pair_off + min(r, it.n - 1)] >> 4) * (a.K / 8);   // in 16-byte pieces
             __syncwarp();
-            for (uint32_t i = kSt == 4 ? w : (w + kSt - before % kSt) % kSt; i < KS; i += kSt, ++round) {
-                if (round && !wait_bar(bar_empty + 8 * w, (round - 1) & 1u)) timed_out = true;
+            uint32_t i = first;
+            for (; i < KS; i += 3) {
+                const uint32_t stage = stage_of(before, i), round = round_of(before, i), dst = wg::b_addr<FMT, NT>(stage);
+                if (round && !wait_bar(bar_empty + 8 * stage, (round - 1) & 1u)) timed_out = true;
                 const uint4* src = reinterpret_cast<const uint4*>(a.xrows) + step_kb(i) * 32u + step_q(i) * 8u + c;
 #pragma unroll
                 for (int b = 0; b < NT / 16 / (int)kPer; ++b)
@@ -735,13 +738,14 @@ wgemm_kernel(const WgemmArgs a, const __grid_constant__ CUtensorMap rows_map) {
                         const uint32_t o[4] = {o4.x, o4.y, o4.z, o4.w};
 #pragma unroll
                         for (int j = 0; j < 4; ++j)
-                            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(((j & 1) ? d1 : d0) + (2 * kPer * b + (j >> 1)) * 1024u), "l"(src + o[j]) : "memory");
+                            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + ((j & 1) ? d1 : d0) + (2 * kPer * b + (j >> 1)) * 1024u), "l"(src + o[j]) : "memory");
                     }
                 asm volatile("cp.async.wait_all;" ::: "memory");
                 umma::fence_smem_to_async();
                 __syncwarp();
-                if (lane == 0) mbar_arrive(bar_full + 8 * w);
+                if (lane == 0) mbar_arrive(bar_full + 8 * stage);
             }
+            first = i - KS;
             __syncwarp();   // every lane is done with this unit's offsets
         }
     } else if (MODE != wg::kGateUp && warp == (uint32_t)wg::kRowWarp) {
@@ -965,11 +969,12 @@ static cudaError_t wgemm_launch(const Launch& L, const WgemmArgs& a, const void*
     return e != cudaSuccess ? e : cudaGetLastError();
 }
 
-// 160 rows from an average of 104 pairs an expert on: with tiles of 128 more and more experts need a second expansion of their weights for
-// a few pairs, and two row loaders a stage make up for the fourth stage.  Layer, 256 experts, top 8, IQ3_XXS and IQ4_XS, tiles of 128 -> 160:
-// 3000 tokens 423 -> 426 us, 3500: 462 -> 459, 3840: 518 -> 495, 4096: 561 -> 507, 5120: 697 -> 649, 6144: 776 -> 778, 8192: 990 -> 939.
+// 160 rows where the average expert has 116 to 165 pairs: most of those would need a second expansion of their weights for a few pairs
+// over 128.  Elsewhere the fourth stage is worth more.  Layer, 256 experts, top 8, IQ3_XXS and IQ4_XS, tiles of 128 -> 160:
+// 3400 tokens 443 -> 454 us, 3600: 471 -> 472, 3750: 493 -> 485, 3900: 517 -> 494, 4096: 561 -> 508, 5120: 697 -> 649, 5600: 717 -> 724.
 uint32_t wgemm_rows_per_unit(const qkm_dims& d, uint32_t n) {
-    return (uint64_t)n * d.n_used > 104ull * d.n_expert ? kWgemmRowsWide : kWgemmRows;
+    const uint64_t pairs = (uint64_t)n * d.n_used;
+    return pairs > 115ull * d.n_expert && pairs <= 165ull * d.n_expert ? kWgemmRowsWide : kWgemmRows;
 }
 
 cudaError_t launch_wgemm_gateup(const Launch& L, const qkm_dims& d, uint32_t type, const WgemmExperts& x, const void* xrows,
