@@ -592,12 +592,18 @@ wgemm_kernel(const WgemmArgs a, const __grid_constant__ CUtensorMap rows_map) {
                     // silu with the fast exponential and division: their error (a few ulp) is far below the operands' f16 rounding
                     const uint32_t ff = it.rt * 128u + (row & ~3u) + ((row & 1u) << 1) + ((row >> 1) & 1u);   // element order 0, 2, 1, 3
                     __half* hp = a.h + (size_t)(it.pair_off + cb) * a.rows + ff;
+                    auto put = [&](int i) {
+                        const float us = f0[cb + i], gv = __uint_as_float(v0[i]) * us, uv = __uint_as_float(v1[i]) * us;
+                        hp[(size_t)i * a.rows] = __float2half_rn(__fdividef(gv, 1.0f + __expf(-gv)) * uv * f1[cb + i]);
+                    };
+                    if (cb + 16 <= n) {   // without a branch per column the columns' chains overlap
 #pragma unroll
-                    for (int i = 0; i < 16; ++i)
-                        if (cb + i < n) {
-                            const float us = f0[cb + i], gv = __uint_as_float(v0[i]) * us, uv = __uint_as_float(v1[i]) * us;
-                            hp[(size_t)i * a.rows] = __float2half_rn(__fdividef(gv, 1.0f + __expf(-gv)) * uv * f1[cb + i]);
-                        }
+                        for (int i = 0; i < 16; ++i) put(i);
+                    } else {
+#pragma unroll
+                        for (int i = 0; i < 16; ++i)
+                            if (cb + i < n) put(i);
+                    }
                 } else {
                     const uint32_t o0 = it.rt * 256u + row;
                     float* op = a.out + (size_t)(it.pair_off + cb) * a.rows + o0;
