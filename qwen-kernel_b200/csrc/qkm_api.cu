@@ -81,7 +81,7 @@ struct qkm_ctx {
     void* argmax_scratch = nullptr; uint32_t argmax_rows = 0;
     // dense matrices for qkm_dense_gemm (tile-ordered copies) and its scratch, sized on demand
     static constexpr int kDenseSlots = 16;
-    struct Dense { uint32_t type = 0, M = 0, K = 0; void* tiles = nullptr; } dense[kDenseSlots];
+    struct Dense { uint32_t type = 0, M = 0, K = 0; float w_scale = 1.f; void* tiles = nullptr; } dense[kDenseSlots];
     void* dense_xb = nullptr; float* dense_scale = nullptr;
     size_t dense_cap_elems = 0, dense_cap_rows = 0;
     // expert-parallel exchange plan of the last qkm_ep_dispatch, allocated on first use
@@ -918,8 +918,8 @@ extern "C" QKM_API const float* qkm_h_device(const qkm_ctx* c) { return c ? c->h
 // ---------------------------------------------------------------- dense quantised GEMM
 // The reference's batched-prefill projections (gemm_q8_0*.comp, gemm_iq4_xs.comp; dispatched at
 // src/main.cpp:4806-4835): Y[n][M] = X[n][K] . W^T with W a Q8_0 or IQ4_XS matrix.  The matrix is
-// uploaded once into a slot (copied and tile-ordered on the device); the GEMM runs on the same
-// dequantise-to-shared-memory + tcgen05 pipeline as the experts' down projection, bf16 operands.
+// uploaded once into a slot (copied and tile-ordered on the device); the GEMM runs on the experts'
+// tcgen05 kernel (qkm_wgemm.cu): weights expanded to f16 in tensor memory, x rows as f16 scaled by powers of two.
 
 extern "C" QKM_API int qkm_dense_upload(qkm_ctx* c, uint32_t slot, uint32_t type, const void* w_host, uint32_t M, uint32_t K) {
     if (!c || !w_host) return QKM_ERR_ARG;
@@ -935,6 +935,11 @@ extern "C" QKM_API int qkm_dense_upload(qkm_ctx* c, uint32_t slot, uint32_t type
     if (e == cudaSuccess) e = cudaMemcpyAsync(raw, w_host, bytes, cudaMemcpyHostToDevice, c->stream);
     if (e == cudaSuccess) e = cudaMemsetAsync((uint8_t*)dm.tiles + tbytes, 0, 256, c->stream);
     if (e == cudaSuccess) e = launch_repack(c->L(), type, raw, dm.tiles, 1, M, K);
+    // the largest block scale, by way of the spare bytes behind the tiles
+    uint32_t* spare = (uint32_t*)((uint8_t*)dm.tiles + tbytes);
+    uint32_t d_bits = 0;
+    if (e == cudaSuccess) e = launch_scale_max(c->L(), type, raw, spare, M, K);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(&d_bits, spare, sizeof d_bits, cudaMemcpyDeviceToHost, c->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
     cudaFree(raw);
     if (e != cudaSuccess) {
@@ -942,7 +947,7 @@ extern "C" QKM_API int qkm_dense_upload(qkm_ctx* c, uint32_t slot, uint32_t type
         dm = qkm_ctx::Dense{};
         return fail(c, QKM_ERR_CUDA, "qkm_dense_upload: %s", cudaGetErrorString(e));
     }
-    dm.type = type; dm.M = M; dm.K = K;
+    dm.type = type; dm.M = M; dm.K = K; dm.w_scale = dense_weight_scale(type, d_bits);
     return QKM_OK;
 }
 
@@ -964,7 +969,7 @@ extern "C" QKM_API int qkm_dense_gemm(qkm_ctx* c, uint32_t slot, const float* x,
         QKM_CUDA(c, cudaMalloc((void**)&c->dense_scale, (size_t)n * sizeof(float)));
         c->dense_cap_rows = n;
     }
-    QKM_LAUNCH(c, launch_dense_gemm(c->L(), dm.type, dm.tiles, dm.M, dm.K, x, n, y, c->dense_xb, c->dense_scale, c->lut_pf, (uint32_t)c->n_sms, c->status));
+    QKM_LAUNCH(c, launch_dense_gemm(c->L(), dm.type, dm.tiles, dm.w_scale, dm.M, dm.K, x, n, y, c->dense_xb, c->dense_scale, c->lut_pf, (uint32_t)c->n_sms, c->status));
     return QKM_OK;
 }
 

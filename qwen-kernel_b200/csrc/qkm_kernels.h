@@ -168,9 +168,11 @@ cudaError_t launch_wgemm_gateup(const Launch& L, const qkm_dims& d, uint32_t typ
 cudaError_t launch_wgemm_down(const Launch& L, const qkm_dims& d, uint32_t type, const WgemmExperts& x, const void* h, uint64_t n_hrows,
                               const float* h_inv_scale, const qkm_sel* sel, float* contrib, uint32_t max_units);
 // Dense quantised GEMM Y[n][M] = X[n][K] . W^T (W tile-ordered Q8_0 / IQ4_XS, M % 128 == 0, K % 256 == 0).
-// Scratch: xh n*K f16, x_inv_scale n floats.
-cudaError_t launch_dense_gemm(const Launch& L, uint32_t type, const void* tiles, uint32_t M, uint32_t K, const float* x, uint32_t n_rows, float* y,
+// Scratch: xh n*K f16, x_inv_scale n floats.  w_scale: the power of two by which the weights are multiplied as f16 operands.
+cudaError_t launch_dense_gemm(const Launch& L, uint32_t type, const void* tiles, float w_scale, uint32_t M, uint32_t K, const float* x, uint32_t n_rows, float* y,
                               void* xh, float* x_inv_scale, const uint8_t* table, uint32_t n_sms, uint32_t* status);
+// w_scale for a matrix whose largest |d| has the f16 bits d_bits
+float dense_weight_scale(uint32_t type, uint32_t d_bits);
 
 // ---- qkm_prefill.cu : router logits and the fold around them
 cudaError_t launch_router_f16(const Launch& L, uint32_t router_type, const void* router, void* out, uint64_t n_elems);
@@ -180,6 +182,8 @@ cudaError_t launch_fold_pairs(const Launch& L, const qkm_dims& d, const float* c
 // ---- qkm_repack.cu : raw ggml -> tile layout (same bytes, see qkm_tiles.cuh)
 cudaError_t launch_repack(const Launch& L, uint32_t type, const void* raw, void* out, uint32_t n_mats,
                           uint32_t rows, uint32_t K);
+// *out (zero before) = largest finite |d| of a Q8_0 / IQ4_XS matrix's blocks (raw ggml rows), as f16 bits
+cudaError_t launch_scale_max(const Launch& L, uint32_t type, const void* raw, uint32_t* out, uint32_t rows, uint32_t K);
 
 // ---- qkm_gemv.cu
 cudaError_t launch_dequant(const Launch& L, uint32_t type, const void* blocks, float* y, uint64_t n_elems);

@@ -111,4 +111,23 @@ cudaError_t launch_repack(const Launch& L, uint32_t type, const void* raw, void*
     return cudaGetLastError();
 }
 
+// Largest finite |d| of a matrix's blocks, as f16 bits in *out (zero before): a thread a block.
+__global__ void __launch_bounds__(256)
+scale_max_kernel(const uint8_t* __restrict__ raw, uint32_t* __restrict__ out, uint64_t n_blocks, uint32_t block_bytes) {
+    const uint64_t i = (uint64_t)blockIdx.x * 256 + threadIdx.x;
+    uint32_t d = i < n_blocks ? *reinterpret_cast<const uint16_t*>(raw + i * block_bytes) & 0x7FFFu : 0u;
+    if (d >= 0x7C00u) d = 0;
+    d = __reduce_max_sync(0xFFFFFFFFu, d);
+    if ((threadIdx.x & 31u) == 0 && d) atomicMax(out, d);
+}
+cudaError_t launch_scale_max(const Launch& L, uint32_t type, const void* raw, uint32_t* out, uint32_t rows, uint32_t K) {
+    if (type != QKM_TYPE_Q8_0 && type != QKM_TYPE_IQ4_XS) return cudaErrorInvalidValue;   // d comes first in a block
+    const uint32_t elems = type == QKM_TYPE_Q8_0 ? 32 : 256;
+    const uint64_t n = (uint64_t)rows * (K / elems);
+    if (n == 0) return cudaSuccess;
+    scale_max_kernel<<<(unsigned)((n + 255) / 256), 256, 0, L.stream>>>((const uint8_t*)raw, out, n, (uint32_t)row_bytes(type, elems));
+    L.count();
+    return cudaGetLastError();
+}
+
 }  // namespace qkm

@@ -260,6 +260,7 @@ struct WgemmArgs {
     uint32_t rows, K;           // weight rows of a matrix, columns
     uint32_t n_experts, n_used; // resident experts
     uint32_t n_dense;           // dense: activation rows
+    float w_scale, w_inv_scale; // dense: power of two on the weights as operands, and what undoes it
 };
 
 template <int FMT, int MODE, int NT>
@@ -363,8 +364,8 @@ wgemm_kernel(const WgemmArgs a, const __grid_constant__ CUtensorMap rows_map) {
         const uint32_t tab_c = wg::kTab + (FMT == QKM_TYPE_IQ3_XXS ? (lane & 15u) * 8u : 128u + lane * 4u);
         if (FMT == QKM_TYPE_IQ3_XXS || FMT == QKM_TYPE_IQ4_XS)
             if (!wait_bar(bar_tab, 0)) timed_out = true;
-        // dense: scale and product rounded to f16 (two roundings of 2^-12, a fifth fewer instructions); experts: one rounding that counts
-        auto weight_scale = [](float v) { if constexpr (MODE == wg::kDense) return __float2half2_rn(v); else return split_scale(v); };
+        // dense: scale and product rounded to f16 (two roundings of 2^-11 at most, a fifth fewer instructions); experts: one rounding that counts
+        auto weight_scale = [&](float v) { if constexpr (MODE == wg::kDense) return __float2half2_rn(v * a.w_scale); else return split_scale(v); };
         uint32_t before = 0, wcnt = 0, qcnt = 0;   // what came before this unit; blocks and Q8_0 slots consumed
         MmaItem it;
         for (uint32_t k = 0; next_unit(k, it); ++k, before += advance) {
@@ -570,7 +571,7 @@ wgemm_kernel(const WgemmArgs a, const __grid_constant__ CUtensorMap rows_map) {
                     const uint32_t pr = a.pairs[p], tok = pr >> 4, slot = pr & 15u;
                     f0[c] = (slot < a.n_used ? a.sel[tok].w[slot] : a.sel[tok].w_shared) * a.h_inv_scale[p];
                 } else {
-                    f0[c] = a.x_inv_scale[p];
+                    f0[c] = a.x_inv_scale[p] * a.w_inv_scale;
                 }
             }
             __syncwarp();
@@ -1011,8 +1012,21 @@ cudaError_t launch_wgemm_down(const Launch& L, const qkm_dims& d, uint32_t type,
     return cudaErrorInvalidValue;
 }
 
+// A weight is at most 128 |d| (Q8_0) or 32 * 127 |d| (IQ4_XS); where that would pass f16's 65504 the matrix's weights are scaled
+// to at most 2^15.  Downwards nothing is needed: d is a multiple of 2^-24, the sub-block scales and codebook values are integers,
+// so a scale or weight below f16's normal range (2^-14) is a multiple of 2^-24 too and exact as a subnormal.
+float dense_weight_scale(uint32_t type, uint32_t d_bits) {
+    const int e = (int)(d_bits >> 10);
+    const float d = e ? ldexpf(1024.f + (float)(d_bits & 1023u), e - 25) : ldexpf((float)d_bits, -24);
+    const float most = d * (type == QKM_TYPE_Q8_0 ? 128.f : 32.f * 127.f);
+    if (most < 65504.f) return 1.f;
+    int b;
+    frexpf(most, &b);   // most < 2^b
+    return ldexpf(1.f, 15 - b);
+}
+
 // Y[n][M] = X[n][K] . W^T: x rows to scaled f16, then one launch
-cudaError_t launch_dense_gemm(const Launch& L, uint32_t type, const void* tiles, uint32_t M, uint32_t K, const float* x, uint32_t n_rows, float* y,
+cudaError_t launch_dense_gemm(const Launch& L, uint32_t type, const void* tiles, float w_scale, uint32_t M, uint32_t K, const float* x, uint32_t n_rows, float* y,
                               void* xh, float* x_inv_scale, const uint8_t* table, uint32_t n_sms, uint32_t* status) {
     if (n_rows == 0) return cudaSuccess;
     if (M % 128 || K % 256 || M / 128 > 65535) return cudaErrorInvalidValue;
@@ -1020,6 +1034,7 @@ cudaError_t launch_dense_gemm(const Launch& L, uint32_t type, const void* tiles,
     WgemmArgs a{};
     a.w[0] = a.w[1] = (const uint8_t*)tiles;
     a.x_inv_scale = x_inv_scale; a.out = y; a.table = table; a.status = status; a.rows = M; a.K = K; a.n_dense = n_rows;
+    a.w_scale = w_scale; a.w_inv_scale = 1.f / w_scale;
     const uint32_t units = (n_rows + wg::kNT - 1) / wg::kNT * ((M / 128 + 1) / 2);
     if (type == QKM_TYPE_Q8_0) return wgemm_launch<QKM_TYPE_Q8_0, wg::kDense>(L, a, xh, n_rows, units, n_sms);
     if (type == QKM_TYPE_IQ4_XS) return wgemm_launch<QKM_TYPE_IQ4_XS, wg::kDense>(L, a, xh, n_rows, units, n_sms);

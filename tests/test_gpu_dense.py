@@ -50,6 +50,24 @@ def test_dense_gemm_edges(ctx, orc, syn, ttype, M, K, n):
     d_x.free(); d_y.free()
 
 
+@pytest.mark.parametrize("ttype,lo,hi", [(8, 6e-8, 1e-6), (23, 6e-8, 1e-6), (23, 1e-5, 1e-4), (8, 300.0, 2000.0), (23, 5.0, 100.0), (8, 2e4, 6.5e4), (23, 2e4, 6.5e4)])
+def test_dense_gemm_weight_range(ctx, orc, syn, ttype, lo, hi):
+    """Block scales from f16's smallest subnormal to its largest number: weights as f16 operands would overflow above 65504
+    (IQ4_XS from d = 16 on, Q8_0 from 512).  Rounding: x 2^-11, a weight's scale and product 2^-11 each."""
+    M, K, n = 256, 512, 70
+    W = syn.random_blocks(ttype, M, K, seed=21, tag="dense", scale=(lo, hi))
+    x = syn.random_x(n, K, seed=22)
+    ctx.dense_upload(6, ttype, W, M, K)
+    d_x, d_y = ctx.to_device(x), ctx.alloc(n * M * 4)
+    ctx.dense_gemm(6, d_x, n, d_y)
+    want = orc.gemv(ttype, W, x, M, K, threads=orc.hardware_threads())
+    got = d_y.download(np.float32, (n, M)).astype(np.float64)
+    # independent roundings of K products: 3 * 2^-11 of the result's size at the very most, as a norm
+    assert np.linalg.norm(got - want) < 3 * 2.0**-11 * np.linalg.norm(want)
+    assert syn.rel_err_rows(got, want) < 5e-3
+    d_x.free(); d_y.free()
+
+
 def test_dense_rejects(ctx, pkg, syn):
     W = syn.random_blocks(8, 128, 256, seed=1)
     d = ctx.alloc(1 << 16)
