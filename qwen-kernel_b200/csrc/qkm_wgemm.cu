@@ -781,8 +781,8 @@ wgemm_kernel(const WgemmArgs a, const __grid_constant__ CUtensorMap rows_map) {
 }
 
 // ---- activation rows ---------------------------------------------------------------------------------------
-// x -> f16 rows in the kernels' element order, each scaled by a power of two so that max|x| lands in [2^13, 2^14), the
-// inverse scale and (optional) the row's 2-norm.  WARPS warps per row, which hold it in registers (up to four float4 a thread; a longer
+// x -> f16 rows in the kernels' element order, each scaled by a power of two so that the largest finite |x| lands in
+// [2^13, 2^14) (infinities and NaN stay what they are), the inverse scale and (optional) the row's 2-norm.  WARPS warps per row, which hold it in registers (up to four float4 a thread; a longer
 // row is read twice): one trip to memory.  (A warp per row that read it twice: 1000 x 2048 8.0 us, 4096 rows 11.5.)
 template <int WARPS>
 __global__ void __launch_bounds__(256)
@@ -799,8 +799,9 @@ f16_rows_kernel(const float* x, __half* __restrict__ xh, float* __restrict__ inv
     const float4* xt = reinterpret_cast<const float4*>(x + (size_t)(live ? t : 0) * K);
     const uint32_t K4 = K / 4;
     float m = 0.f, ss = 0.f;
+    auto finite_abs = [](float v) { const float a = fabsf(v); return a <= 3.402823466e38f ? a : 0.f; };
     auto take = [&](const float4& v) {
-        m = fmaxf(fmaxf(m, fmaxf(fabsf(v.x), fabsf(v.y))), fmaxf(fabsf(v.z), fabsf(v.w)));
+        m = fmaxf(fmaxf(m, fmaxf(finite_abs(v.x), finite_abs(v.y))), fmaxf(finite_abs(v.z), finite_abs(v.w)));
         ss += v.x * v.x; ss += v.y * v.y; ss += v.z * v.z; ss += v.w * v.w;
     };
     float4 r[4];
@@ -821,7 +822,7 @@ f16_rows_kernel(const float* x, __half* __restrict__ xh, float* __restrict__ inv
     }
     if (!live) return;
     int p = 0;
-    if (m > 0.f && m <= 3.0e38f) { int e; frexpf(m, &e); p = min(14 - e, 126); }   // m * 2^p in [2^13, 2^14)
+    if (m > 0.f) { int e; frexpf(m, &e); p = min(14 - e, 126); }   // m * 2^p in [2^13, 2^14)
     const float up = ldexpf(1.0f, p);
     uint2* dst = reinterpret_cast<uint2*>(xh + (size_t)t * K);
     auto put = [&](uint32_t k, const float4& v) {

@@ -68,6 +68,26 @@ def test_dense_gemm_weight_range(ctx, orc, syn, ttype, lo, hi):
     d_x.free(); d_y.free()
 
 
+@pytest.mark.parametrize("ttype", [8, 23])
+@pytest.mark.parametrize("value", [np.inf, -np.inf, np.nan, 3.4e38])
+def test_dense_gemm_extreme_rows(ctx, orc, syn, ttype, value):
+    """An infinity, a NaN or an element near the largest float beside ordinary large ones: the outputs that are infinite, NaN and
+    finite are those of the f32 formula, and other rows do not notice."""
+    M, K, n = 256, 512, 20
+    W = syn.random_blocks(ttype, M, K, seed=23, tag="dense", scale=(1e-4, 1e-3))
+    x = syn.random_x(n, K, seed=24) * np.float32(1e6)
+    x[3, 77] = value
+    ctx.dense_upload(7, ttype, W, M, K)
+    d_x, d_y = ctx.to_device(x), ctx.alloc(n * M * 4)
+    ctx.dense_gemm(7, d_x, n, d_y)
+    got, want = d_y.download(np.float32, (n, M)), orc.gemv(ttype, W, x, M, K)
+    assert np.array_equal(np.isnan(got), np.isnan(want)) and np.array_equal(np.isposinf(got), np.isposinf(want))
+    assert np.array_equal(np.isneginf(got), np.isneginf(want))
+    live = [r for r in range(n) if r != 3 or np.isfinite(want[3]).all()]
+    assert syn.rel_err_rows(got[live], want[live]) < 5e-3
+    d_x.free(); d_y.free()
+
+
 def test_dense_rejects(ctx, pkg, syn):
     W = syn.random_blocks(8, 128, 256, seed=1)
     d = ctx.alloc(1 << 16)
