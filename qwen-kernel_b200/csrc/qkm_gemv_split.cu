@@ -63,11 +63,11 @@ __device__ __forceinline__ void mma_s8_k16(int (&c)[4], uint32_t a0, uint32_t a1
                  : "=r"(c[0]), "=r"(c[1]), "=r"(c[2]), "=r"(c[3])
                  : "r"(a0), "r"(a1), "r"(b0), "r"(0));
 }
-// D(16x8, f32) += A(16x16, f16, row) * B(16x8, f16, col)
-__device__ __forceinline__ void mma_f16_k16(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
-    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-                 : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+// D(16x8, f32) = A(16x16, f16, row) * B(16x8, f16, col)
+__device__ __forceinline__ void mma_f16_k16_first(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
+                 : "=f"(c[0]), "=f"(c[1]), "=f"(c[2]), "=f"(c[3])
+                 : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "f"(0.f));
 }
 
 // Eight consecutive columns (8 * lane ..) of one activation row into the B fragments of one 256-column block.
@@ -255,7 +255,11 @@ __device__ __forceinline__ void tile_sums(uint32_t r0, uint32_t r1, uint32_t bf,
     }
 }
 
-// F16 weights: rows straight from global memory, eight 16-byte loads per row and 256 columns
+// F16 weights: rows straight from global memory, eight 16-byte loads per row and 256 columns.
+// An f16 MMA adds its products (and the D it is given) by truncation, so a chain of sixteen of them drifts towards zero: 3.5e-7
+// from 64 bits (norm, K 512 to 4096), where f32 FMAs of rounded additions are at 0.9e-7 to 2.1e-7.  Every MMA therefore starts from
+// zero and eight partial sums at a time are added in f32 as a tree: 0.8e-7 to 1.1e-7; one after the other 0.9e-7 to 1.1e-7 (above
+// the FMAs at K = 512).  It costs 4 to 20 % (4096 x 2048: 16 rows 11.1 -> 12.7 us, 2 rows 6.1 -> 6.1).
 template <int NT>
 __device__ __forceinline__ void tile_sums_f16(const uint8_t* __restrict__ p0, const uint8_t* __restrict__ p1, uint32_t bf, const float (&sc)[NT],
                                               float dw0, float dw1, float (&f)[NT][2]) {
@@ -266,12 +270,25 @@ __device__ __forceinline__ void tile_sums_f16(const uint8_t* __restrict__ p0, co
 #pragma unroll
     for (int nt = 0; nt < NT; ++nt) c[nt][0] = c[nt][1] = c[nt][2] = c[nt][3] = 0.f;
 #pragma unroll
-    for (int s = 0; s < 8; ++s) {
+    for (int s0 = 0; s0 < 8; s0 += 4) {
 #pragma unroll
         for (int nt = 0; nt < NT; ++nt) {
-            const uint4 x = lds128(bf + nt * gs::frag_bytes<QKM_TYPE_F16>() + s * 512u);
-            mma_f16_k16(c[nt], a[s].x, b[s].x, a[s].y, b[s].y, x.x, x.y);
-            mma_f16_k16(c[nt], a[s].z, b[s].z, a[s].w, b[s].w, x.z, x.w);
+            float p[2 * 4][4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {   // 32 columns, two MMAs, each
+                const int s = s0 + i;
+                const uint4 x = lds128(bf + nt * gs::frag_bytes<QKM_TYPE_F16>() + s * 512u);
+                mma_f16_k16_first(p[2 * i], a[s].x, b[s].x, a[s].y, b[s].y, x.x, x.y);
+                mma_f16_k16_first(p[2 * i + 1], a[s].z, b[s].z, a[s].w, b[s].w, x.z, x.w);
+            }
+#pragma unroll
+            for (int w = 4; w > 0; w >>= 1)
+#pragma unroll
+                for (int i = 0; i < w; ++i)
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) p[i][j] += p[i + w][j];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) c[nt][j] += p[0][j];
         }
     }
 #pragma unroll

@@ -118,6 +118,21 @@ def test_gemv_k_split(ctx, orc, syn, ttype, M, K, n):
         b.free()
 
 
+@pytest.mark.parametrize("M,K,n", [(600, 512, 2), (600, 2048, 3), (300, 2048, 16), (300, 4096, 5), (200, 8192, 8)])
+def test_gemv_f16_rows_precision(ctx, orc, syn, M, K, n):
+    """Several rows of x against F16 weights are as near to 64 bits as a sum of f32 FMAs: 2^-23 as a norm (independent
+    roundings of 2^-24; sums that are truncated instead drift to three times that)."""
+    W = syn.random_blocks(1, M, K, seed=47)
+    x = syn.random_x(n, K, seed=48)
+    d_w, d_x, d_y = ctx.to_device(W), ctx.to_device(x), ctx.alloc(n * M * 4)
+    ctx.gemv(1, d_w, d_x, d_y, M, K, n)
+    want = x.astype(np.float64) @ W.view(np.float16).reshape(M, K).astype(np.float64).T
+    err = np.linalg.norm(d_y.download(np.float32, (n, M)) - want) / np.linalg.norm(want)
+    assert err < 2.0**-23, err
+    for b in (d_w, d_x, d_y):
+        b.free()
+
+
 def test_gemv_rejects_bad_shapes(ctx, pkg):
     d = ctx.alloc(4096)
     for ttype, K in ((8, 48), (14, 128), (18, 300), (99, 256)):
