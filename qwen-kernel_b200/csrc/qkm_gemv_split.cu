@@ -298,6 +298,22 @@ __device__ __forceinline__ void tile_sums_f16(const uint8_t* __restrict__ p0, co
     }
 }
 
+// One output as the f32 sum that the formula gives.  Rows of x with an infinity, a NaN or an element above 3.0e38 have no digit
+// planes: their sums come out as NaN; and sums of large elements can pass f32 before the weight scale is applied.  What is not
+// finite is taken again here, a thread an output: rare, and only then slow.
+template <int TYPE>
+__device__ __noinline__ float plain_dot(const uint8_t* __restrict__ w, const float* x, uint32_t K) {
+    float s = 0.f;
+#pragma unroll 1
+    for (uint32_t k = 0; k < K; k += 8) {
+        float v[8];
+        dequant8<TYPE>(w, k, v);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) s += v[i] * x[k + i];
+    }
+    return s;
+}
+
 struct GemvSplitArgs {
     const uint8_t* W;
     const float* x;      // [n][K]
@@ -404,7 +420,7 @@ gemv_split_kernel(GemvSplitArgs a) {
                 for (int j = 0; j < 8; ++j) v[u][j] = 0.f;
             }
             encode_fragments<TYPE>(v[u], lane, s_frag + (kb * NT + (row >> 1)) * gs::frag_bytes<TYPE>(), (row & 1u) * 4u, up);
-            if (lane == 0) sts32(s_scale + i * 4, __float_as_uint(bad ? __int_as_float(0x7FC00000) : ldexpf(1.0f, -p)));   // NaN or Inf in x: NaN out
+            if (lane == 0) sts32(s_scale + i * 4, __float_as_uint(bad ? __int_as_float(0x7FC00000) : ldexpf(1.0f, -p)));   // its outputs: plain_dot
         }
     }
     __syncthreads();
@@ -472,6 +488,7 @@ gemv_split_kernel(GemvSplitArgs a) {
 #pragma unroll
                 for (uint32_t q = 0; q < 8; ++q)   // slice order
                     if (q < n_ctas) v += p[q];
+                if (!(fabsf(v) <= 3.402823466e38f)) v = plain_dot<TYPE>(a.W + (size_t)m * rb, a.x + (size_t)row * a.K, a.K);
                 a.y[(size_t)row * a.M + m] = v;
             }
         }

@@ -133,6 +133,27 @@ def test_gemv_f16_rows_precision(ctx, orc, syn, M, K, n):
         b.free()
 
 
+@pytest.mark.parametrize("ttype", [1, 8, 14, 23, 18])
+@pytest.mark.parametrize("M,K,n", [(300, 512, 3), (4100, 2048, 1), (35, 4096, 16)])
+def test_gemv_extreme_rows(ctx, orc, syn, ttype, M, K, n):
+    """x with an infinity, a NaN or an element near the largest float: the outputs that are infinite, NaN and finite are those
+    of the f32 formula (sums of one sign of infinity stay infinite), and other rows do not notice."""
+    W = syn.random_blocks(ttype, M, K, seed=49, scale=(1e-4, 1e-3) if ttype != 1 else None)
+    d_w, d_y = ctx.to_device(W), ctx.alloc(n * M * 4)
+    for value in (np.inf, -np.inf, np.nan, np.float32(3.3e38), np.float32(2e38)):
+        x = syn.random_x(n, K, seed=50)
+        x[n // 2, K - 200] = value
+        d_x = ctx.to_device(x)
+        ctx.gemv(ttype, d_w, d_x, d_y, M, K, n)
+        got, want = d_y.download(np.float32, (n, M)), orc.gemv(ttype, W, x, M, K)
+        for kind in (np.isnan, np.isposinf, np.isneginf):
+            assert np.array_equal(kind(got), kind(want)), (value, kind)
+        live = [r for r in range(n) if np.isfinite(want[r]).all()]
+        assert len(live) >= n - 1 and (not live or syn.rel_err_rows(got[live], want[live]) < TOL_F32)
+        d_x.free()
+    d_w.free(); d_y.free()
+
+
 def test_gemv_rejects_bad_shapes(ctx, pkg):
     d = ctx.alloc(4096)
     for ttype, K in ((8, 48), (14, 128), (18, 300), (99, 256)):
