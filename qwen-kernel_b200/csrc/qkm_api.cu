@@ -719,13 +719,19 @@ static int expert_plan(qkm_ctx* c, const qkm_sel* sel, uint32_t n, bool with_rou
 }
 
 // The two expert GEMMs over the work lists of expert_plan: c->xb (f16 rows; c->xscale, c->xnorm) -> c->hb -> c->contrib_p.
-// At most np_max routed pairs and sh_max rows of the shared expert.
-static int expert_gemms(qkm_ctx* c, const qkm_layer_dev& ld, const qkm_sel* sel, uint32_t np_max, uint32_t sh_max) {
+// n rows; at most np_max routed pairs and sh_max rows of the shared expert.
+static int expert_gemms(qkm_ctx* c, const qkm_layer_dev& ld, const qkm_sel* sel, uint32_t n, uint32_t np_max, uint32_t sh_max) {
     const qkm_dims& d = c->cfg.dims;
     const uint32_t NT = c->unit_rows;
     const uint32_t tiles = (c->ecount < np_max ? c->ecount + (np_max + NT - 1) / NT : np_max) + (sh_max + NT - 1) / NT;
     WgemmExperts g{{ld.tiles[2], ld.tiles[3]}, {ld.tiles[5], ld.tiles[6]}, c->mma_items[0], c->n_items, c->n_items + 2, c->pairs, c->lut_pf, c->status, c->ecount, (uint32_t)c->n_sms, NT};
     QKM_LAUNCH(c, launch_wgemm_gateup(c->L(), d, ld.w.gateup_type, g, c->xb, c->xscale, c->xnorm, ld.w_norm, c->hb, c->hscale, tiles * (d.n_ff / 128)));
+    HiddenRows r{};
+    r.pairs = c->pairs; r.pos_of = c->pos_of; r.sel = sel; r.xrows = (const __half*)c->xb; r.x_inv_scale = c->xscale; r.x_norm = c->xnorm; r.w_norm = ld.w_norm;
+    r.w[0] = (const uint8_t*)ld.w.gate_exps; r.w[1] = (const uint8_t*)ld.w.up_exps; r.sh[0] = (const uint8_t*)ld.w.gate_shexp; r.sh[1] = (const uint8_t*)ld.w.up_shexp;
+    r.h = (__half*)c->hb; r.h_inv_scale = c->hscale; r.n_tokens = n; r.n_used = d.n_used; r.n_expert = d.n_expert; r.expert_first = c->efirst;
+    r.expert_count = c->ecount; r.n_ff = d.n_ff; r.n_embd = d.n_embd;
+    QKM_LAUNCH(c, launch_hidden_rows_check(c->L(), ld.w.gateup_type, r));
     c->prof_mark("moe.gu");
     WgemmExperts m{{ld.tiles[4], nullptr}, {ld.tiles[7], nullptr}, c->mma_items[1], c->n_items + 1, c->n_items + 3, c->pairs, c->lut_pf, c->status, c->ecount, (uint32_t)c->n_sms, NT};
     QKM_LAUNCH(c, launch_wgemm_down(c->L(), d, ld.w.down_type, m, c->hb, (uint64_t)c->cfg.max_tokens * (d.n_used + 1), c->hscale, sel, c->contrib_p,
@@ -754,7 +760,7 @@ extern "C" QKM_API int qkm_moe_prefill(qkm_ctx* c, uint32_t layer, const float* 
     c->prof_mark("moe.route");
     if (int rc = expert_plan(c, c->sel, n, true, 0, n)) return rc;
     c->prof_mark("moe.pairs");
-    if (int rc = expert_gemms(c, ld, c->sel, n * d.n_used, n)) return rc;
+    if (int rc = expert_gemms(c, ld, c->sel, n, n * d.n_used, n)) return rc;
     QKM_LAUNCH(c, launch_fold_pairs(c->L(), d, c->contrib_p, c->pos_of, y, n));
     c->prof_mark("moe.fold");
     return QKM_OK;
@@ -1145,7 +1151,7 @@ extern "C" QKM_API int qkm_ep_shared(qkm_ctx* c, uint32_t layer, const float* x,
     if (int rc = ensure_prefill_scratch(c)) return rc;
     if (int rc = expert_plan(c, c->sel, n, false, 0, n)) return rc;
     QKM_LAUNCH(c, launch_f16_rows(c->L(), x, c->xb, c->xscale, c->xnorm, n, d.n_embd));
-    if (int rc = expert_gemms(c, ld, c->sel, 0, n)) return rc;   // the routed list is empty
+    if (int rc = expert_gemms(c, ld, c->sel, n, 0, n)) return rc;   // the routed list is empty
     QKM_LAUNCH(c, launch_fold_pairs(c->L(), d, c->contrib_p, c->pos_of, c->y2, n));
     return QKM_OK;
 }
@@ -1196,7 +1202,7 @@ static int ep_expert_forward_impl(qkm_ctx* c, uint32_t layer, const float* xrecv
     } else {
         QKM_LAUNCH(c, launch_f16_rows(c->L(), xrecv, c->xb, c->xscale, c->xnorm, n_recv, d.n_embd));
     }
-    if (int rc = expert_gemms(c, ld, selrecv, n_recv * d.n_used, with_shared ? sh_count : 0)) return rc;
+    if (int rc = expert_gemms(c, ld, selrecv, n_recv, n_recv * d.n_used, with_shared ? sh_count : 0)) return rc;
     if (slot_rows_peer)
         QKM_LAUNCH(c, launch_fold_pairs_peer(c->L(), d, c->contrib_p, c->pos_of, c->pm_peers, slot_rows_peer, c->pm_rank, c->pm_ranks));
     else

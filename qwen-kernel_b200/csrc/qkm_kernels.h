@@ -4,6 +4,7 @@
 // kernel launched.
 #pragma once
 
+#include <cuda_fp16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -173,6 +174,20 @@ cudaError_t launch_dense_gemm(const Launch& L, uint32_t type, const void* tiles,
                               void* xh, float* x_inv_scale, const uint8_t* table, uint32_t n_sms, uint32_t* status);
 // w_scale for a matrix whose largest |d| has the f16 bits d_bits
 float dense_weight_scale(uint32_t type, uint32_t d_bits);
+
+// ---- qkm_hrows.cu : hidden rows that the gate/up epilogue's scale served badly are made again
+struct HiddenRows {
+    const uint32_t *pairs, *pos_of;          // as launch_group_place writes them
+    const qkm_sel* sel;
+    const __half* xrows;                     // launch_f16_rows' output
+    const float *x_inv_scale, *x_norm;
+    const float* w_norm;                     // as for launch_wgemm_gateup
+    const uint8_t *w[2], *sh[2];             // raw ggml rows: gate and up of the resident experts, of the shared expert
+    __half* h;                               // in and out
+    float* h_inv_scale;
+    uint32_t n_tokens, n_used, n_expert, expert_first, expert_count, n_ff, n_embd;
+};
+cudaError_t launch_hidden_rows_check(const Launch& L, uint32_t type, const HiddenRows& a);
 
 // ---- qkm_prefill.cu : router logits and the fold around them
 cudaError_t launch_router_f16(const Launch& L, uint32_t router_type, const void* router, void* out, uint64_t n_elems);

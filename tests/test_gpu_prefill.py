@@ -134,6 +134,86 @@ def test_prefill_wide_tiles(pkg, orc, syn, gt, dt, n_embd, n_expert, n_used, T):
     run_prefill(pkg, orc, syn, dims, layer, x)
 
 
+def _token_errors(y, ref):
+    r = ref["y"].astype(np.float64)
+    return np.linalg.norm(y - r, axis=1) / np.linalg.norm(r, axis=1)
+
+
+@pytest.mark.parametrize("gt,dt", [(18, 23), (23, 14)])
+@pytest.mark.parametrize("size", [1e4, 1e6])
+def test_prefill_large_element_without_weights(pkg, orc, syn, gt, dt, size):
+    """x with one large element in 256 columns whose weights are all zero: the products are ordinary and far below what the row
+    norms allow, and the hidden rows keep their precision (0.6e-3 to 0.9e-3 for ordinary x; f16 operands)."""
+    dims = syn.Dims(n_embd=512, n_ff=512, n_expert=8, n_used=2)
+    layer = syn.make_layer(dims, seed=51, gateup_type=gt, down_type=dt)
+    for t, elems, size_b in ((layer.gate_exps, 256, syn.BLOCK[gt][1]), (layer.up_exps, 256, syn.BLOCK[gt][1]), (layer.gate_shexp, 32, 34), (layer.up_shexp, 32, 34)):
+        t.reshape(-1, dims.n_embd // elems, size_b)[:, :256 // elems, 0:2] = 0   # d of the first 256 columns
+    x = syn.random_x(140, dims.n_embd, seed=52)
+    x[::3, 5] = size
+    ref = orc.moe_layer(layer, x, threads=orc.hardware_threads())
+    with pkg.Context(dims, n_layer=1, max_tokens=len(x), device=0) as ctx:
+        ctx.upload_layer(0, layer)
+        err = _token_errors(ctx.moe_forward_host(0, x, mode=1), ref)
+    assert err.max() < 1.5e-3, err
+
+
+def test_prefill_saturated_gates(pkg, orc, syn):
+    """Every gate of every expert between -20 and -45, the shared one too: the hidden values are 1e-8 and less of what the row norms allow.  The
+    gates' error (f16 operands, 2^-11 each, 512 products of one sign) enters the exponential: 45 * 2 * 2^-11 at the very most."""
+    dims = syn.Dims(n_embd=512, n_ff=512, n_expert=8, n_used=2)
+    layer = syn.make_layer(dims, seed=53, gateup_type=23, down_type=23)
+    b = layer.gate_exps.reshape(-1, 136)
+    b[:, 0:2] = np.array([5.5e-3], np.float16).view(np.uint8)
+    b[:, 8:] = 0        # codebook value -127 throughout
+    b[:, 2:8] = 0xFF    # sub-block scales 31
+    s = layer.gate_shexp.reshape(-1, 34)
+    s[:, 2:] = 0x81     # -127
+    s[:, 0:2] = np.array([0.17], np.float16).view(np.uint8)
+    x = np.abs(syn.random_x(96, dims.n_embd, seed=54)) * np.float32(3e-3)
+    ref = orc.moe_layer(layer, x, threads=orc.hardware_threads(), want_h=True)
+    assert 0 < np.abs(ref["h"]).max() < 1e-6
+    with pkg.Context(dims, n_layer=1, max_tokens=len(x), device=0) as ctx:
+        ctx.upload_layer(0, layer)
+        err = _token_errors(ctx.moe_forward_host(0, x, mode=1), ref)
+    assert err.max() < 45 * 2 * 2.0**-11, err
+
+
+def test_prefill_norms_beyond_f32(pkg, orc, syn):
+    """x of 3e18: its squared norm, and so the bound on the hidden values, passes f32; the hidden values do not."""
+    dims = syn.Dims(n_embd=512, n_ff=512, n_expert=8, n_used=2)
+    layer = syn.make_layer(dims, seed=55, gateup_type=23, down_type=23)
+    for t, size_b in ((layer.gate_exps, 136), (layer.up_exps, 136), (layer.gate_shexp, 34), (layer.up_shexp, 34)):
+        v = t.reshape(-1, size_b)
+        v[:, 0:2] = (v[:, 0:2].copy().view(np.float16) * np.float16(2.0**-10)).view(np.uint8)
+    x = syn.random_x(80, dims.n_embd, seed=56)
+    x[10:20] *= np.float32(3e18)
+    ref = orc.moe_layer(layer, x, threads=orc.hardware_threads())
+    assert np.isfinite(ref["y"]).all()
+    with pkg.Context(dims, n_layer=1, max_tokens=len(x), device=0) as ctx:
+        ctx.upload_layer(0, layer)
+        y = ctx.moe_forward_host(0, x, mode=1)
+        live = np.arange(len(x)) if np.isfinite(ref["sel"]["w"]).all() else None
+        err = _token_errors(y, ref)
+    assert live is not None and err.max() < 2.5e-3, err
+
+
+@pytest.mark.parametrize("gt,dt", [(18, 23), (23, 14)])
+def test_prefill_large_weight_rows(pkg, orc, syn, gt, dt):
+    """One gate row and another up row of every expert a thousand times larger than the rest."""
+    dims = syn.Dims(n_embd=512, n_ff=512, n_expert=8, n_used=2)
+    layer = syn.make_layer(dims, seed=57, gateup_type=gt, down_type=dt)
+    for t, r, mats, size_b in ((layer.gate_exps, 3, 8, syn.BLOCK[gt][1]), (layer.up_exps, 7, 8, syn.BLOCK[gt][1]), (layer.gate_shexp, 3, 1, 34), (layer.up_shexp, 7, 1, 34)):
+        v = t.reshape(mats, dims.n_ff, -1, size_b)
+        v[:, r, :, 0:2] = (v[:, r, :, 0:2].copy().view(np.float16) * np.float16(1000)).view(np.uint8)
+    x = syn.random_x(140, dims.n_embd, seed=58)
+    ref = orc.moe_layer(layer, x, threads=orc.hardware_threads())
+    with pkg.Context(dims, n_layer=1, max_tokens=len(x), device=0) as ctx:
+        ctx.upload_layer(0, layer)
+        y = ctx.moe_forward_host(0, x, mode=1)
+    err = np.linalg.norm(y - ref["y"].astype(np.float64)) / np.linalg.norm(ref["y"].astype(np.float64))
+    assert err < 1.5e-3, err
+
+
 def test_prefill_matches_decode_path(pkg, syn):
     """The two fused paths agree to bf16 accuracy on the same inputs."""
     dims = syn.Dims()
