@@ -40,6 +40,7 @@
 #include "qkm_stream.cuh"
 #include "qkm_tiles.cuh"
 #include "qkm_umma.cuh"
+#include "qkm_wait.h"
 
 namespace qkm {
 
@@ -321,9 +322,8 @@ wgemm_kernel(const WgemmArgs a, const __grid_constant__ CUtensorMap rows_map) {
     umma::fence_after_sync();
     const uint32_t n_units = MODE == wg::kDense ? (a.n_dense + NT - 1) / NT * row_units : *a.n_items;
     const uint32_t tmem = s_tmem;
-    bool timed_out = false;
-    auto wait_bar = [&](uint32_t b, uint32_t parity) -> bool { return timed_out || mbar_wait_timed(b, parity); };   // a thread waits out the limit once at most
-
+    Waits waits;
+    auto wait_bar = [&](uint32_t b, uint32_t parity) { waits.wait([&] { return mbar_wait_timed(b, parity); }); };
 
     auto unit_item = [&](uint32_t u) -> MmaItem {
         if (MODE != wg::kDense) return a.items[u];
@@ -337,8 +337,8 @@ wgemm_kernel(const WgemmArgs a, const __grid_constant__ CUtensorMap rows_map) {
     // the k-th unit of this block, from the weight loader; false after the last
     auto next_unit = [&](uint32_t k, MmaItem& it) -> bool {
         const uint32_t s = k % wg::kFeed;
-        timed_out = __any_sync(0xFFFFFFFFu, !wait_bar(bar_ufull + 8 * s, (k / wg::kFeed) & 1u));   // the same for the whole warp
-        if (timed_out) return false;
+        if (!waits.next([&] { return mbar_wait_timed(bar_ufull + 8 * s, (k / wg::kFeed) & 1u); }, [](bool out) { return __any_sync(0xFFFFFFFFu, out) != 0; }))
+            return false;   // the same for the whole warp
         it = s_feed[s];
         __syncwarp();
         if (lane == 0) mbar_arrive(bar_uempty + 8 * s);
@@ -363,7 +363,7 @@ wgemm_kernel(const WgemmArgs a, const __grid_constant__ CUtensorMap rows_map) {
         const uint32_t wbuf = wg::w_base<FMT, NT>() + par * wg::w_bytes<FMT>();
         const uint32_t tab_c = wg::kTab + (FMT == QKM_TYPE_IQ3_XXS ? (lane & 15u) * 8u : 128u + lane * 4u);
         if (FMT == QKM_TYPE_IQ3_XXS || FMT == QKM_TYPE_IQ4_XS)
-            if (!wait_bar(bar_tab, 0)) timed_out = true;
+            wait_bar(bar_tab, 0);
         // dense: scale and product rounded to f16 (two roundings of 2^-11 at most, a fifth fewer instructions); experts: one rounding that counts
         auto weight_scale = [&](float v) { if constexpr (MODE == wg::kDense) return __float2half2_rn(v * a.w_scale); else return split_scale(v); };
         uint32_t before = 0, wcnt = 0, qcnt = 0;   // what came before this unit; blocks and Q8_0 slots consumed
@@ -384,7 +384,7 @@ wgemm_kernel(const WgemmArgs a, const __grid_constant__ CUtensorMap rows_map) {
                 if (half == 0) {
                     announce();
                     const uint32_t stage = stage_of(before, i), round = round_of(before, i);   // the stage is free to be written
-                    if (round && !wait_bar(bar_empty + 8 * stage, (round - 1) & 1u)) timed_out = true;
+                    if (round) wait_bar(bar_empty + 8 * stage, (round - 1) & 1u);
                     umma::fence_after_sync();
                     st = a_lane + stage * 64u;
                     pending = stage;
@@ -393,7 +393,7 @@ wgemm_kernel(const WgemmArgs a, const __grid_constant__ CUtensorMap rows_map) {
             };
             auto w_wait = [&]() {
                 // slot 0's barrier counts blocks and every kSlots-th Q8_0 slot
-                if (!wait_bar(bar_wfull + 8 * kSlots * par, (wcnt + qcnt / kSlots) & 1u)) timed_out = true;
+                wait_bar(bar_wfull + 8 * kSlots * par, (wcnt + qcnt / kSlots) & 1u);
                 ++wcnt;
             };
             auto w_free = [&]() {
@@ -408,7 +408,7 @@ wgemm_kernel(const WgemmArgs a, const __grid_constant__ CUtensorMap rows_map) {
 #pragma unroll 1
                     for (uint32_t q = lone ? par : 0; q < 4; q += lone ? 2 : 1, ++qcnt) {
                         const uint32_t slot = qcnt % kSlots, bars = 8 * (kSlots * par + slot);
-                        if (!wait_bar(bar_wfull + bars, (qcnt / kSlots + (slot ? 0u : wcnt)) & 1u)) timed_out = true;
+                        wait_bar(bar_wfull + bars, (qcnt / kSlots + (slot ? 0u : wcnt)) & 1u);
                         const uint32_t t0 = wbuf + slot * wg::kQ8Slot + (mat * 8 + tl) * 1088u;
                         uint4 v[2][2];
                         float d[2];
@@ -576,10 +576,10 @@ wgemm_kernel(const WgemmArgs a, const __grid_constant__ CUtensorMap rows_map) {
             }
             __syncwarp();
             if (lane == 0) mbar_arrive(bar_cols);
-            if (!wait_bar(bar_cols, iter & 1u)) timed_out = true;
+            wait_bar(bar_cols, iter & 1u);
             const uint32_t b = big ? 0u : next;
-            if (!wait_bar(bar_accfull + 8 * b, used[b] & 1u)) timed_out = true;
-            if (big) { if (!wait_bar(bar_accfull + 8, used[1] & 1u)) timed_out = true; ++used[0]; ++used[1]; next = 0; }
+            wait_bar(bar_accfull + 8 * b, used[b] & 1u);
+            if (big) { wait_bar(bar_accfull + 8, used[1] & 1u); ++used[0]; ++used[1]; next = 0; }
             else { ++used[b]; next ^= 1u; }
             umma::fence_after_sync();
             const uint32_t t0 = tmem + ((32 * e) << 16) + b * 128u, t1 = t0 + (big ? (uint32_t)NT : 64u);
@@ -633,14 +633,14 @@ wgemm_kernel(const WgemmArgs a, const __grid_constant__ CUtensorMap rows_map) {
             const bool big = n_mma > 64;
             const uint32_t b = big ? 0u : next, idesc = umma::instr_desc_f16(n_mma);
             // the accumulators' previous contents have been read
-            if (used[b] && !wait_bar(bar_accfree + 8 * b, (used[b] - 1) & 1u)) timed_out = true;
-            if (big && used[1] && !wait_bar(bar_accfree + 8, (used[1] - 1) & 1u)) timed_out = true;
+            if (used[b]) wait_bar(bar_accfree + 8 * b, (used[b] - 1) & 1u);
+            if (big && used[1]) wait_bar(bar_accfree + 8, (used[1] - 1) & 1u);
             if (big) { ++used[0]; ++used[1]; next = 0; } else { ++used[b]; next ^= 1u; }
             umma::fence_after_sync();
             const uint32_t t0 = tmem + b * 128u, t1 = t0 + (big ? (uint32_t)NT : 64u);
             for (uint32_t i = 0; i < KS; ++i) {
                 const uint32_t stage = stage_of(before, i);
-                if (!wait_bar(bar_full + 8 * stage, round_of(before, i) & 1u)) timed_out = true;
+                wait_bar(bar_full + 8 * stage, round_of(before, i) & 1u);
                 umma::fence_after_sync();
                 const uint64_t d_b = umma::smem_desc(wg::b_addr<FMT, NT>(stage));
                 const uint32_t t_a = tmem + wg::tmem_a<NT>() + stage * 64u;
@@ -662,15 +662,15 @@ wgemm_kernel(const WgemmArgs a, const __grid_constant__ CUtensorMap rows_map) {
         uint32_t blocks[2] = {0, 0}, slots[2] = {0, 0};   // handed out so far, per parity
         auto drained = [&](uint32_t par, uint32_t slot) {   // everything put there has been read
             const uint32_t uses = (slots[par] + kSlots - 1 - slot) / kSlots + (slot ? 0u : blocks[par]);
-            if (uses && !wait_bar(bar_wempty + 8 * (kSlots * par + slot), (uses - 1) & 1u)) timed_out = true;
+            if (uses) wait_bar(bar_wempty + 8 * (kSlots * par + slot), (uses - 1) & 1u);
         };
         uint32_t u = blockIdx.x;
         for (uint32_t k = 0;; ++k) {
             MmaItem it{0, 0, 0, 0};
-            timed_out = __any_sync(0xFFFFFFFFu, timed_out);
-            if (u < n_units && !timed_out) it = unit_item(u);
+            if (u < n_units) it = unit_item(u);
             const uint32_t s = k % wg::kFeed;
-            if (k >= (uint32_t)wg::kFeed && !wait_bar(bar_uempty + 8 * s, (k / wg::kFeed - 1) & 1u)) timed_out = true;
+            if (k >= (uint32_t)wg::kFeed) wait_bar(bar_uempty + 8 * s, (k / wg::kFeed - 1) & 1u);
+            if (__any_sync(0xFFFFFFFFu, waits.out)) break;   // the slot may still be read; the other roles' waits run out too
             if (lane == 0) {
                 s_feed[s] = it;
                 mbar_arrive(bar_ufull + 8 * s);
@@ -693,7 +693,7 @@ wgemm_kernel(const WgemmArgs a, const __grid_constant__ CUtensorMap rows_map) {
                             if (lone && ((q ^ par) & 1u)) continue;
                             const uint32_t slot = slots[par] % kSlots, wf = bar_wfull + 8 * (kSlots * par + slot);
                             drained(par, slot);
-                            if (__any_sync(0xFFFFFFFFu, timed_out)) break;   // a barrier that still counts bytes takes no second arrival
+                            if (__any_sync(0xFFFFFFFFu, waits.out)) break;   // a barrier that still counts bytes takes no second arrival
                             ++slots[par];
                             if (lane == 0) mbar_expect_tx(wf, wg::kQ8Slot);
                             __syncwarp();
@@ -704,7 +704,7 @@ wgemm_kernel(const WgemmArgs a, const __grid_constant__ CUtensorMap rows_map) {
                     for (uint32_t par = 0; par < 2; ++par) {
                         const uint32_t wf = bar_wfull + 8 * kSlots * par;
                         for (uint32_t slot = 0; slot < kSlots; ++slot) drained(par, slot);   // a block covers them all
-                        if (__any_sync(0xFFFFFFFFu, timed_out)) break;
+                        if (__any_sync(0xFFFFFFFFu, waits.out)) break;
                         ++blocks[par];
                         if (lane == 0) mbar_expect_tx(wf, 16 * tile);
                         __syncwarp();
@@ -736,7 +736,7 @@ wgemm_kernel(const WgemmArgs a, const __grid_constant__ CUtensorMap rows_map) {
             uint32_t i = first;
             for (; i < KS; i += 3) {
                 const uint32_t stage = stage_of(before, i), round = round_of(before, i), dst = wg::b_addr<FMT, NT>(stage);
-                if (round && !wait_bar(bar_empty + 8 * stage, (round - 1) & 1u)) timed_out = true;
+                if (round) wait_bar(bar_empty + 8 * stage, (round - 1) & 1u);
                 const uint4* src = reinterpret_cast<const uint4*>(a.xrows) + step_kb(i) * 32u + step_q(i) * 8u + c;
 #pragma unroll
                 for (int b = 0; b < NT / 16 / (int)kPer; ++b)
@@ -764,8 +764,8 @@ wgemm_kernel(const WgemmArgs a, const __grid_constant__ CUtensorMap rows_map) {
             const uint32_t boxes = (it.n + 15u) / 16;
             for (uint32_t i = 0; i < KS; ++i, ++gs) {
                 const uint32_t stage = gs % kSt;
-                if (gs >= kSt && !wait_bar(bar_empty + 8 * stage, (gs / kSt - 1) & 1u)) timed_out = true;
-                if (__any_sync(0xFFFFFFFFu, timed_out)) break;   // a barrier that still counts bytes takes no second arrival
+                if (gs >= kSt) wait_bar(bar_empty + 8 * stage, (gs / kSt - 1) & 1u);
+                if (__any_sync(0xFFFFFFFFu, waits.out)) break;   // a barrier that still counts bytes takes no second arrival
                 if (lane == 0) mbar_expect_tx(bar_full + 8 * stage, boxes * 2048u);
                 __syncwarp();
                 if (lane < boxes) tma_rows16(wg::b_addr<FMT, NT>(stage) + lane * 2048u, &rows_map, step_kb(i) * 256u + step_q(i) * 64u, it.pair_off + 16 * lane, bar_full + 8 * stage);
@@ -774,7 +774,7 @@ wgemm_kernel(const WgemmArgs a, const __grid_constant__ CUtensorMap rows_map) {
     }
     }
     umma::fence_before_sync();
-    const int any_timed_out = __syncthreads_or(timed_out ? 1 : 0);   // any role's wait that ran out counts
+    const int any_timed_out = __syncthreads_or(waits.out ? 1 : 0);   // any role's wait that ran out counts
     if (any_timed_out) for (int i = 0; i < 100; ++i) __nanosleep(1000);   // copies and MMAs still under way end long before this does
     if (warp == 0) umma::tmem_dealloc(tmem, 512);
     if (any_timed_out && tid == 0) atomicExch(a.status, (uint32_t)kStatusWaitTimeout);
