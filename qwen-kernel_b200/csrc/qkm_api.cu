@@ -13,6 +13,7 @@
 #include <new>
 #include <vector>
 
+#include "qkm_alloc.h"
 #include "qkm_common.cuh"
 #include "qkm_kernels.h"
 #include "qkm_tiles.cuh"
@@ -152,6 +153,13 @@ int fail(qkm_ctx* c, int code, const char* fmt, ...) {
         va_end(ap);
     }
     return code;
+}
+
+template <int N>
+cudaError_t dev_alloc_all(const Want (&want)[N]) {
+    const int e = alloc_all(want, [](void** p, size_t bytes) { return (int)cudaMalloc(p, bytes); }, [](void* p) { cudaFree(p); });
+    if (e) cudaGetLastError();   // reported by the caller; the next launch's check must not find it
+    return (cudaError_t)e;
 }
 
 #define QKM_CUDA(c, call)                                                                       \
@@ -694,15 +702,18 @@ static int ensure_prefill_scratch(qkm_ctx* c) {
     const size_t T = c->cfg.max_tokens, rows = T * (d.n_used + 1);
     const uint32_t NT = kWgemmRows;
     const size_t max_tiles = d.n_expert + (T * d.n_used + NT - 1) / NT + (T + NT - 1) / NT;   // the shared expert's last
-    QKM_CUDA(c, cudaMalloc(&c->xb, T * d.n_embd * 2));
-    QKM_CUDA(c, cudaMalloc((void**)&c->xnorm, T * sizeof(float)));
-    QKM_CUDA(c, cudaMalloc(&c->hb, rows * d.n_ff * 2));
-    QKM_CUDA(c, cudaMalloc((void**)&c->hscale, rows * sizeof(float)));
-    QKM_CUDA(c, cudaMalloc((void**)&c->contrib_p, rows * d.n_embd * sizeof(float)));
-    QKM_CUDA(c, cudaMalloc((void**)&c->mma_items[0], max_tiles * (d.n_ff / 128) * sizeof(MmaItem)));
-    QKM_CUDA(c, cudaMalloc((void**)&c->mma_items[1], max_tiles * (d.n_embd / 256) * sizeof(MmaItem)));
-    QKM_CUDA(c, cudaMalloc((void**)&c->pos_of, rows * sizeof(uint32_t)));
-    QKM_CUDA(c, cudaMalloc((void**)&c->group_counts, (c->ecount + T * d.n_used) * sizeof(uint32_t)));
+    const Want want[] = {
+        {&c->xb, T * d.n_embd * 2},
+        {(void**)&c->xnorm, T * sizeof(float)},
+        {&c->hb, rows * d.n_ff * 2},
+        {(void**)&c->hscale, rows * sizeof(float)},
+        {(void**)&c->contrib_p, rows * d.n_embd * sizeof(float)},
+        {(void**)&c->mma_items[0], max_tiles * (d.n_ff / 128) * sizeof(MmaItem)},
+        {(void**)&c->mma_items[1], max_tiles * (d.n_embd / 256) * sizeof(MmaItem)},
+        {(void**)&c->pos_of, rows * sizeof(uint32_t)},
+        {(void**)&c->group_counts, (c->ecount + T * d.n_used) * sizeof(uint32_t)},
+    };
+    QKM_CUDA(c, dev_alloc_all(want));
     return QKM_OK;
 }
 
@@ -846,8 +857,8 @@ extern "C" QKM_API int qkm_moe_decode_stack_host(qkm_ctx* c, uint32_t first, uin
     if ((uint64_t)first + count > c->cfg.n_layer) return fail(c, QKM_ERR_BOUNDS, "layers [%u,%u) out of range", first, first + count);
     if (!c->stack_x) {
         const size_t cap = (size_t)c->cfg.n_layer * c->cfg.max_tokens * c->cfg.dims.n_embd * sizeof(float);
-        QKM_CUDA(c, cudaMalloc((void**)&c->stack_x, cap));
-        QKM_CUDA(c, cudaMalloc((void**)&c->stack_y, cap));
+        const Want want[] = {{(void**)&c->stack_x, cap}, {(void**)&c->stack_y, cap}};
+        QKM_CUDA(c, dev_alloc_all(want));
     }
     const size_t layer_elems = (size_t)n * c->cfg.dims.n_embd;
     const size_t bytes = (size_t)count * layer_elems * sizeof(float);
@@ -860,11 +871,10 @@ extern "C" QKM_API int qkm_moe_decode_stack_host(qkm_ctx* c, uint32_t first, uin
     // Chunks of layers: all input copies are queued on their own stream at once, chunk k computes as soon
     // as its rows are there, and its outputs leave on a third stream while chunk k+1 computes.  Only the
     // first chunk's copy in and the last chunk's copy out are not hidden, so these two chunks are short.
-    if (!c->copy_in) {
-        QKM_CUDA(c, cudaStreamCreateWithFlags(&c->copy_in, cudaStreamNonBlocking));
-        QKM_CUDA(c, cudaStreamCreateWithFlags(&c->copy_out, cudaStreamNonBlocking));
-        for (cudaEvent_t& ev : c->ev_in) QKM_CUDA(c, cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
-        for (cudaEvent_t& ev : c->ev_out) QKM_CUDA(c, cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
+    if (!c->ev_copies) {   // made last; what an earlier try got is kept
+        for (cudaStream_t* s : {&c->copy_in, &c->copy_out}) if (!*s) QKM_CUDA(c, cudaStreamCreateWithFlags(s, cudaStreamNonBlocking));
+        for (cudaEvent_t& ev : c->ev_in) if (!ev) QKM_CUDA(c, cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
+        for (cudaEvent_t& ev : c->ev_out) if (!ev) QKM_CUDA(c, cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
         QKM_CUDA(c, cudaEventCreateWithFlags(&c->ev_copies, cudaEventDisableTiming));
     }
     constexpr uint32_t K = qkm_ctx::kStackChunks;
@@ -1053,13 +1063,15 @@ static int ep_check(qkm_ctx* c, uint32_t n_ranks) {
     if (c->ecount != d.n_expert / n_ranks || c->efirst % c->ecount)
         return fail(c, QKM_ERR_MODE, "context holds experts [%u,%u): not one of %u equal shards", c->efirst, c->efirst + c->ecount, n_ranks);
     if (c->ep_ranks != n_ranks) {
-        if (c->ep_counts) { cudaFree(c->ep_counts); cudaFree(c->ep_send_tok); cudaFree(c->ep_send_pos); cudaFreeHost(c->ep_counts_host); }
+        for (void* p : {c->ep_counts, c->ep_send_tok, c->ep_send_pos}) if (p) cudaFree(p);
+        if (c->ep_counts_host) cudaFreeHost(c->ep_counts_host);
         c->ep_counts = c->ep_send_tok = c->ep_send_pos = c->ep_counts_host = nullptr;
         c->ep_ranks = 0;
         const size_t T = c->cfg.max_tokens, fan = n_ranks < d.n_used ? n_ranks : d.n_used;
-        QKM_CUDA(c, cudaMalloc((void**)&c->ep_counts, (n_ranks + 1) * sizeof(uint32_t)));
-        QKM_CUDA(c, cudaMalloc((void**)&c->ep_send_tok, T * fan * sizeof(uint32_t)));
-        QKM_CUDA(c, cudaMalloc((void**)&c->ep_send_pos, T * n_ranks * sizeof(uint32_t)));
+        const Want want[] = {{(void**)&c->ep_counts, (n_ranks + 1) * sizeof(uint32_t)},
+                             {(void**)&c->ep_send_tok, T * fan * sizeof(uint32_t)},
+                             {(void**)&c->ep_send_pos, T * n_ranks * sizeof(uint32_t)}};
+        QKM_CUDA(c, dev_alloc_all(want));
         QKM_CUDA(c, cudaMallocHost((void**)&c->ep_counts_host, (n_ranks + 1) * sizeof(uint32_t)));
         c->ep_ranks = n_ranks;
     }
