@@ -717,13 +717,13 @@ static int ensure_prefill_scratch(qkm_ctx* c) {
     return QKM_OK;
 }
 
-// work lists of the GEMMs from c->group_counts; with_routed false: of the shared expert's rows only
-static int expert_plan(qkm_ctx* c, const qkm_sel* sel, uint32_t n, bool with_routed, uint32_t sh_first, uint32_t sh_count) {
+// work lists of the GEMMs from c->group_counts; with_routed false: of the shared expert's rows only; picked: see mean_pairs
+static int expert_plan(qkm_ctx* c, const qkm_sel* sel, uint32_t n, bool with_routed, uint32_t sh_first, uint32_t sh_count, bool picked = false) {
     const qkm_dims& d = c->cfg.dims;
     GroupPlace g{};
     g.counts = c->group_counts; g.ranks = c->group_counts + c->ecount; g.sel = sel; g.n_tokens = n; g.n_used = d.n_used; g.n_expert = d.n_expert;
     g.expert_first = c->efirst; g.expert_count = with_routed ? c->ecount : 0; g.sh_first = sh_first; g.sh_count = sh_count;
-    g.tile = c->unit_rows = with_routed ? wgemm_rows_per_unit(d, n) : kWgemmRows; g.rt_gu = d.n_ff / 128; g.rt_dn = d.n_embd / 256; g.pairs = c->pairs; g.pos_of = c->pos_of;
+    g.tile = c->unit_rows = with_routed ? wgemm_rows_per_unit(mean_pairs(n, d.n_used, d.n_expert, c->ecount, picked)) : kWgemmRows; g.rt_gu = d.n_ff / 128; g.rt_dn = d.n_embd / 256; g.pairs = c->pairs; g.pos_of = c->pos_of;
     g.items_gu = c->mma_items[0]; g.items_dn = c->mma_items[1]; g.n_items = c->n_items;
     QKM_LAUNCH(c, launch_group_place(c->L(), g));
     return QKM_OK;
@@ -1206,7 +1206,7 @@ static int ep_expert_forward_impl(qkm_ctx* c, uint32_t layer, const float* xrecv
     if (int rc = ensure_prefill_scratch(c)) return rc;
     QKM_CUDA(c, cudaMemsetAsync(c->group_counts, 0, c->ecount * sizeof(uint32_t), c->stream));
     QKM_LAUNCH(c, launch_group_rank(c->L(), d, selrecv, n_recv, c->efirst, c->ecount, c->group_counts, c->group_counts + c->ecount));
-    if (int rc = expert_plan(c, selrecv, n_recv, true, with_shared ? sh_first : 0, with_shared ? sh_count : 0)) return rc;
+    if (int rc = expert_plan(c, selrecv, n_recv, true, with_shared ? sh_first : 0, with_shared ? sh_count : 0, slot_rows_peer == 0)) return rc;   // (slots: every row of the sources, empty or not)
     // the rows as scaled f16: converted here, or already so on arrival (then their scales and norms are gathered)
     if (rows_f16) {
         QKM_LAUNCH(c, launch_ep_row_scales(c->L(), selrecv, c->xscale, n_recv));

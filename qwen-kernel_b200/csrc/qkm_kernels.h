@@ -11,6 +11,7 @@
 #include <atomic>
 
 #include "../../include/qk_moe.h"
+#include "qkm_units.h"
 
 namespace qkm {
 
@@ -137,8 +138,6 @@ cudaError_t launch_decode_down_any(const Launch& L, const DownDecodeArgs& a, uin
 
 // ---- qkm_wgemm.cu : tcgen05 GEMMs with quantised weights (batched prefill, dense projections)
 constexpr uint16_t kSharedItem = 0xFFFFu;   // MmaItem::expert of the shared expert's units
-constexpr uint32_t kWgemmRows = 128, kWgemmRowsWide = 160;   // activation rows per unit
-uint32_t wgemm_rows_per_unit(const qkm_dims& d, uint32_t n_tokens);
 size_t wgemm_table_bytes();
 cudaError_t launch_wgemm_table(const Launch& L, uint8_t* out);
 // x rows as f16 in the kernels' element order (0, 2, 1, 3 in every group of four), scaled per row by a power of two

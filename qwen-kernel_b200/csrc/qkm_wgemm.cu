@@ -977,14 +977,6 @@ static cudaError_t wgemm_launch(const Launch& L, const WgemmArgs& a, const void*
     return e != cudaSuccess ? e : cudaGetLastError();
 }
 
-// 160 rows where the average expert has 116 to 165 pairs: most of those would need a second expansion of their weights for a few pairs
-// over 128.  Elsewhere the fourth stage is worth more.  Layer, 256 experts, top 8, IQ3_XXS and IQ4_XS, tiles of 128 -> 160:
-// 3400 tokens 443 -> 454 us, 3600: 471 -> 472, 3750: 493 -> 485, 3900: 517 -> 494, 4096: 561 -> 508, 5120: 697 -> 649, 5600: 717 -> 724.
-uint32_t wgemm_rows_per_unit(const qkm_dims& d, uint32_t n) {
-    const uint64_t pairs = (uint64_t)n * d.n_used;
-    return pairs > 115ull * d.n_expert && pairs <= 165ull * d.n_expert ? kWgemmRowsWide : kWgemmRows;
-}
-
 cudaError_t launch_wgemm_gateup(const Launch& L, const qkm_dims& d, uint32_t type, const WgemmExperts& x, const void* xrows,
                                 const float* x_inv_scale, const float* x_norm, const float* w_norm, void* h, float* h_inv_scale, uint32_t max_units) {
     WgemmArgs a{};
