@@ -56,7 +56,7 @@ struct qkm_ctx {
     float* stack_y = nullptr;
     // streaming path scratch
     int n_sms = 0;
-    float* xscale = nullptr;          // [max_tokens]
+    float* xscale = nullptr;          // decode: [max_tokens][n_embd/256] of the digit planes; prefill: [max_tokens] of the f16 rows
     uint32_t* n_items = nullptr;      // prefill: units of [0] gate/up, [1] down; [2], [3] their tickets
     uint32_t* status = nullptr;       // kernel status word (device)
     uint32_t* route_counter = nullptr; // ticket counter of the decode router's selection (device, stays zero)
@@ -270,7 +270,7 @@ extern "C" QKM_API qkm_ctx* qkm_open(const qkm_config* cfg, char* err, size_t er
                           d.n_ff % 128 == 0;
     if (c->shapes_stream_ok) {
         struct { void** p; size_t bytes; } more[] = {
-            {(void**)&c->xscale, T * sizeof(float)},
+            {(void**)&c->xscale, T * (d.n_embd / 256) * sizeof(float)},
             {(void**)&c->n_items, 4 * sizeof(uint32_t)},
         };
         for (auto& a : more) {

@@ -354,7 +354,7 @@ decode_gateup_kernel(GateupDecodeArgs a) {
             const uint32_t cts = t >> 1;   // token slot of C columns 2t, 2t+1
             wcol0 = 0.f; wcol1 = 0.f;
             if (cts < rec.ntok) {
-                const float sc = a.xscale[S.pairs[rec.pair_off + cts] >> 4];
+                const float sc = a.xscale[(S.pairs[rec.pair_off + cts] >> 4) * KB + kb];
                 const float w0 = (t & 1u) ? 16384.f : 1.f;   // 128^(2 * (t & 1))
                 wcol0 = sc * w0;
                 wcol1 = sc * w0 * 128.f;

@@ -50,46 +50,51 @@ route_decode_kernel(RouteDecodeArgs a) {
 
     if (blockIdx.x >= n_logit_blocks) {
         // ---- one token: digit planes + shared gate ----------------------------------------------
-        __shared__ float s_xm[8];
+        __shared__ uint32_t s_xm[16][8];
+        __shared__ float s_up[16];
         __shared__ double s_sg[8];
-        const uint32_t t = blockIdx.x - n_logit_blocks;
+        const uint32_t t = blockIdx.x - n_logit_blocks, KB = d.n_embd / 256;
         const float* xt = a.x + (size_t)t * d.n_embd;
-        float v[16];   // n_embd <= 4096
-        float xm = 0.f;
+        float v[16];   // n_embd <= 4096: element tid of every 256 columns
         double dsg = 0.0;
-        bool bad = false;
 #pragma unroll
         for (int i = 0; i < 16; ++i) {
             const uint32_t k = tid + 256 * i;
             v[i] = k < d.n_embd ? xt[k] : 0.f;
-            xm = fmaxf(xm, fabsf(v[i]));
-            bad |= !(fabsf(v[i]) <= 3.0e38f);
             if (k < d.n_embd) dsg += (double)a.gis[k] * (double)v[i];
         }
+        // a scale per 256 columns: a large element costs the others of its own block bits, not the whole row
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) xm = fmaxf(xm, __shfl_xor_sync(0xFFFFFFFFu, xm, o));
+        for (int i = 0; i < 16; ++i)
+            if (256u * i < d.n_embd) {
+                const float ax = fabsf(v[i]);
+                const uint32_t m = __reduce_max_sync(0xFFFFFFFFu, ax <= 3.0e38f ? __float_as_uint(ax) : 0x7F800000u);   // non-negative floats order like their bits
+                if (lane == 0) s_xm[i][warp] = m;
+            }
         dsg = warp_sum(dsg);
-        const int any_bad = __syncthreads_or(bad ? 1 : 0);
-        if (lane == 0) { s_xm[warp] = xm; s_sg[warp] = dsg; }
+        if (lane == 0) s_sg[warp] = dsg;
         __syncthreads();
-        if (tid == 0) {
+        if (tid < KB) {
+            uint32_t m = 0;
+#pragma unroll
+            for (int w = 0; w < 8; ++w) m = max(m, s_xm[tid][w]);
+            const bool bad = m >= 0x7F800000u;
+            const int p = min(digit_exponent(__uint_as_float(m)), 126);
+            s_up[tid] = bad ? 0.f : ldexpf(1.0f, p);   // (then NaN or zero times zero: digits of zero)
+            a.xscale[t * KB + tid] = bad ? __int_as_float(0x7FC00000) : ldexpf(1.0f, -p);
+        } else if (tid == 32) {
             double sg = 0.0;
 #pragma unroll
             for (int w = 0; w < 8; ++w) sg += s_sg[w];
             a.sel[t].w_shared = (float)(1.0 / (1.0 + exp(-sg)));
         }
-        float xmax = 0.f;
-#pragma unroll
-        for (int w = 0; w < 8; ++w) xmax = fmaxf(xmax, s_xm[w]);
-        const int p = digit_exponent(xmax);
-        const float up = ldexpf(1.0f, p);
+        __syncthreads();
         int8_t* pl = a.planes + (size_t)t * 8 * d.n_embd;
 #pragma unroll
         for (int i = 0; i < 16; ++i) {
             const uint32_t k = tid + 256 * i;
-            if (k < d.n_embd) store_planes8(pl, k, any_bad ? 0u : digits4(__float2int_rn(v[i] * up)));
+            if (k < d.n_embd) store_planes8(pl, k, digits4(__float2int_rn(v[i] * s_up[i])));
         }
-        if (tid == 0) a.xscale[t] = any_bad ? __int_as_float(0x7FC00000) : ldexpf(1.0f, -p);
         return;
     }
 

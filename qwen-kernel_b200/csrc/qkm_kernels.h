@@ -83,7 +83,7 @@ struct RouteDecodeArgs {
     double* logits;            // scratch [n_tokens][n_expert]
     uint32_t* counter;         // ceil(n_tokens / 8) zero words; left at zero
     int8_t* planes;            // out [n_tokens][n_embd/256][8][256]: digit planes 0..3 and their negatives 4..7
-    float* xscale;             // out [n_tokens] 2^-p
+    float* xscale;             // out [n_tokens][n_embd/256] 2^-p
     uint32_t n_tokens;
     qkm_dims d;
 };
@@ -97,7 +97,7 @@ struct GateupDecodeArgs {
     const uint8_t* sh_up_tiles;
     const uint8_t* luts;            // decode_gateup_lut_bytes() bytes written by launch_decode_gateup_luts
     const int8_t* planes;
-    const float* xscale;
+    const float* xscale;            // [n_tokens][n_embd/256]
     const qkm_sel* sel;             // the selection (its pairs are grouped by expert in every block at its start)
     uint32_t n_tokens, expert_first, expert_count, with_shared;
     uint32_t gateup_type;           // QKM_TYPE_IQ3_XXS or QKM_TYPE_IQ4_XS
@@ -224,7 +224,7 @@ cudaError_t launch_select(const Launch& L, const qkm_dims& d, const float* logit
 // norm2[e] = |router row e|^2; largest (zero before): their maximum; either may be NULL
 cudaError_t launch_row_norm2(const Launch& L, const qkm_dims& d, uint32_t router_type, const void* router, float* norm2, float* largest);
 struct RouteExtra {                      // all optional
-    int8_t* xplanes = nullptr;           // out: x rows as digit planes and their negatives [kb][8][256], and their scales
+    int8_t* xplanes = nullptr;           // out (at most 64 tokens): x rows as digit planes and their negatives [kb][8][256], and their scales [token][kb]
     float* xscale = nullptr;
     const void* x_f16 = nullptr;         // with these four (more than 64 tokens) the logits come from the tensor cores: rows and
     const float* x_f16_inv = nullptr;    // scales of launch_f16_rows, the router as launch_router_f16 wrote it, its rows' largest squared norm

@@ -34,7 +34,7 @@ struct SelectArgs {
     const float* gis;
     const float* x;
     qkm_sel* sel;
-    int8_t* xplanes;           // optional: x as digit planes and their negatives [kb][8][256], and their scale
+    int8_t* xplanes;           // optional, with f64 logits: x as digit planes and their negatives [kb][8][256], and their scales [token][kb]
     float* xscale;
     uint32_t* counts;          // optional: pairs per resident expert, added to; ranks[t * n_used + s] = a pair's number inside its expert
     uint32_t* ranks;
@@ -151,23 +151,36 @@ select_tokens_kernel(const SelectArgs a) {
     __syncthreads();
     xs = 0.f; xm = 0.f;
     for (uint32_t w = 0; w < n_warps; ++w) { xs += s_xs[w]; xm = fmaxf(xm, s_xm[w]); }
-    const bool bad = !(xm <= 3.0e38f);
-    if (a.xplanes != nullptr) {
-        const int p = bad ? 0 : digit_exponent(xm);
-        const float up_f = ldexpf(1.0f, p);
-        for (uint32_t u = tid; u < K4; u += n_threads) {
-            const float4 v = xt[u];
-            const uint32_t e[4] = {bad ? 0u : digits4(__float2int_rn(v.x * up_f)), bad ? 0u : digits4(__float2int_rn(v.y * up_f)),
-                                   bad ? 0u : digits4(__float2int_rn(v.z * up_f)), bad ? 0u : digits4(__float2int_rn(v.w * up_f))};
-            uint32_t* q = reinterpret_cast<uint32_t*>(a.xplanes + (size_t)t * 8 * d.n_embd + (size_t)(u >> 6) * 2048 + 4 * (u & 63u));
+    if (EXACT && a.xplanes != nullptr) {   // a scale per 256 columns, a warp per such block at a time
+        for (uint32_t kb = warp; kb < d.n_embd / 256; kb += n_warps) {
+            float4 v[2];
+            float m = 0.f;
+            bool off = false;   // an infinity, a NaN or an element too large
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {   // digit j of the four
-                const uint32_t s = 0x4040u + 0x1111u * j;
-                q[64 * j] = __byte_perm(__byte_perm(e[0], e[1], s), __byte_perm(e[2], e[3], s), 0x5410u);
-                q[64 * (j + 4)] = __vneg4(q[64 * j]);
+            for (int h = 0; h < 2; ++h) {
+                v[h] = xt[64 * kb + 32 * h + lane];
+                const float b = fmaxf(fmaxf(fabsf(v[h].x), fabsf(v[h].y)), fmaxf(fabsf(v[h].z), fabsf(v[h].w)));
+                off |= !(fabsf(v[h].x) <= 3.0e38f && fabsf(v[h].y) <= 3.0e38f && fabsf(v[h].z) <= 3.0e38f && fabsf(v[h].w) <= 3.0e38f);
+                m = fmaxf(m, b);
             }
+            m = __uint_as_float(__reduce_max_sync(0xFFFFFFFFu, __float_as_uint(m)));
+            off = __any_sync(0xFFFFFFFFu, off);
+            const int p = off ? 0 : digit_exponent(m);
+            const float up_f = ldexpf(1.0f, p);
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const uint32_t e[4] = {off ? 0u : digits4(__float2int_rn(v[h].x * up_f)), off ? 0u : digits4(__float2int_rn(v[h].y * up_f)),
+                                       off ? 0u : digits4(__float2int_rn(v[h].z * up_f)), off ? 0u : digits4(__float2int_rn(v[h].w * up_f))};
+                uint32_t* q = reinterpret_cast<uint32_t*>(a.xplanes + (size_t)t * 8 * d.n_embd + (size_t)kb * 2048 + 4 * (32 * h + lane));
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {   // digit j of the four
+                    const uint32_t s = 0x4040u + 0x1111u * j;
+                    q[64 * j] = __byte_perm(__byte_perm(e[0], e[1], s), __byte_perm(e[2], e[3], s), 0x5410u);
+                    q[64 * (j + 4)] = __vneg4(q[64 * j]);
+                }
+            }
+            if (lane == 0) a.xscale[t * (d.n_embd / 256) + kb] = off ? __int_as_float(0x7FC00000) : ldexpf(1.0f, -p);
         }
-        if (tid == 0) a.xscale[t] = bad ? __int_as_float(0x7FC00000) : ldexpf(1.0f, -p);
     }
 
     if (!EXACT) {
@@ -292,6 +305,7 @@ static cudaError_t select_launch(const Launch& L, const SelectArgs& a) {
     return e != cudaSuccess ? e : cudaGetLastError();
 }
 cudaError_t launch_select_tokens(const Launch& L, const qkm_dims& d, uint32_t router_type, const SelectIn& in, qkm_sel* sel, uint32_t n_tokens) {
+    if (in.xplanes && (!in.exact || d.n_embd % 256)) return cudaErrorInvalidValue;
     SelectArgs a{};
     a.router = (const uint8_t*)in.router; a.logits = in.logits; a.norm2 = in.norm2; a.n_norm = in.n_norm; a.gis = in.gis; a.x = in.x; a.sel = sel;
     a.xplanes = in.xplanes; a.xscale = in.xscale; a.counts = in.counts; a.ranks = in.ranks; a.part_stride = (size_t)n_tokens * d.n_expert; a.n_parts = in.n_parts;

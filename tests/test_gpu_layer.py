@@ -180,6 +180,24 @@ def test_decode_down_grouped_by_expert(pkg, orc, syn, n_embd, n_ff, n_expert, n_
         assert np.array_equal(y, d_y.download(np.float32, x.shape))
 
 
+@pytest.mark.parametrize("gt,dt,n_expert,n_used", [(23, 14, 8, 2), (23, 23, 32, 10), (18, 14, 16, 8), (18, 23, 16, 8)])
+@pytest.mark.parametrize("size", [1e4, 1e8])
+def test_decode_large_element_without_weights(pkg, orc, syn, gt, dt, n_expert, n_used, size):
+    """x with one large element in 256 columns whose weights are all zero: the other columns' fixed-point digits keep their bits."""
+    dims = syn.Dims(n_embd=1024, n_ff=512, n_expert=n_expert, n_used=n_used)
+    layer = syn.make_layer(dims, seed=61, gateup_type=gt, down_type=dt)
+    for t, elems, size_b in ((layer.gate_exps, 256, syn.BLOCK[gt][1]), (layer.up_exps, 256, syn.BLOCK[gt][1]), (layer.gate_shexp, 32, 34), (layer.up_shexp, 32, 34)):
+        t.reshape(-1, dims.n_embd // elems, size_b)[:, 256 // elems:512 // elems, 0:2] = 0   # d of columns 256 .. 511
+    x = syn.random_x(13, dims.n_embd, seed=62)
+    x[::2, 300] = size
+    ref = orc.moe_layer(layer, x, threads=orc.hardware_threads())
+    with pkg.Context(dims, n_layer=1, max_tokens=len(x), device=0) as ctx:
+        ctx.upload_layer(0, layer)
+        y = ctx.moe_forward_host(0, x, mode=0)
+        assert np.array_equal(ctx.last_sel(len(x))["ids"][:, :n_used], ref["sel"]["ids"][:, :n_used])
+    assert syn.rel_err_rows(y, ref["y"]) < TOL_F32
+
+
 def test_decode_router_is_deterministic_over_many_calls(pkg, orc, syn):
     """200 calls of the fused decode sequence on the same 16 rows: ids, weights and outputs are the
     same bits every time (a last-arriving block ranks the logits; the reference removed such a
