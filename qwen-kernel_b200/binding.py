@@ -181,6 +181,11 @@ def _p(x):
     return int(x)
 
 
+def _host(p):
+    """Host address as a ctypes void-pointer argument takes it: an int, None, bytes, a c_void_p, an array or a pointer."""
+    return p if p is None or type(p) is int else C.cast(p, C.c_void_p).value
+
+
 class Context:
     """One GPU context (one host thread; calls are asynchronous on its stream)."""
 
@@ -309,7 +314,7 @@ class Context:
 
     def moe_decode_stack_host(self, first, count, x_host_ptr, n, y_host_ptr):
         """x/y: host addresses (ints) of [count][n][n_embd] f32, ideally pinned."""
-        rc = self._calls.moe_decode_stack_host(self.h, first, count, x_host_ptr, n, y_host_ptr)
+        rc = self._calls.moe_decode_stack_host(self.h, first, count, _host(x_host_ptr), n, _host(y_host_ptr))
         if rc:
             self.check(rc)
 

@@ -43,6 +43,24 @@ def test_null_handle_calls_fail_cleanly(pkg):
     lib.qkm_close(None)  # no-op
 
 
+def test_host_stack_takes_what_ctypes_takes(pkg):
+    """Host addresses of the host-buffer stack: every form a ctypes void-pointer argument takes reaches the library (which refuses
+    the NULL context), anything else is refused before."""
+    import numpy as np
+    ctx = object.__new__(pkg.Context)
+    ctx.lib, ctx.h = pkg.load_library(), None
+    from qwen_kernel_b200 import qkm_calls
+    ctx._calls = qkm_calls
+    a = np.zeros(4, np.float32)
+    for p in (a.ctypes.data, None, a.ctypes.data_as(C.c_void_p), a.ctypes.data_as(C.POINTER(C.c_float)), (C.c_float * 4)(), a.ctypes, b"1234"):
+        with pytest.raises(pkg.QkmError) as ei:
+            ctx.moe_decode_stack_host(0, 1, p, 1, p)
+        assert ei.value.code == -1
+    for p in (a, 1.5, [1]):
+        with pytest.raises((C.ArgumentError, TypeError)):
+            ctx.moe_decode_stack_host(0, 1, p, 1, a.ctypes.data)
+
+
 @pytest.mark.skipif(has_gpu(), reason="checks the no-GPU behaviour")
 def test_open_without_gpu_fails_loudly(pkg):
     with pytest.raises(pkg.QkmError) as ei:
