@@ -23,6 +23,7 @@ CALLS = os.path.join(HERE, "qkm_calls.so")
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 NVCC_FLAGS = ["-O3", "-std=c++17", "-lineinfo", "--expt-relaxed-constexpr", "-Xcompiler",
               "-fPIC,-fvisibility=hidden,-Wall,-Wno-unused-function", "-Xptxas", "-v"]
+CALLS_FLAGS = ["-O2", "-std=c++17", "-Wall", "-shared", "-fPIC", "-fvisibility=hidden"]
 
 
 def nvcc() -> str:
@@ -44,7 +45,9 @@ def _digest() -> str:
             if os.path.isfile(p) and f.endswith((".cu", ".cuh", ".h", ".inc", ".cpp")):
                 h.update(f.encode())
                 h.update(open(p, "rb").read())
-    h.update(" ".join(ARCH + NVCC_FLAGS).encode())
+    h.update(" ".join(ARCH + NVCC_FLAGS + CALLS_FLAGS).encode())
+    # the extension module is bound to the interpreter that it was built for
+    h.update(f"{sysconfig.get_config_var('EXT_SUFFIX')} {sysconfig.get_paths()['include']}".encode())
     return h.hexdigest()
 
 
@@ -77,7 +80,7 @@ def build(force: bool = False, verbose: bool = False) -> str:
     r = subprocess.run([cc, *ARCH, "-shared", "-o", OUT, *objs], capture_output=True, text=True)
     if r.returncode != 0:
         raise RuntimeError("link failed:\n" + r.stdout + r.stderr)
-    r = subprocess.run(["g++", "-O2", "-std=c++17", "-Wall", "-shared", "-fPIC", "-fvisibility=hidden", "-I" + sysconfig.get_paths()["include"],
+    r = subprocess.run(["g++", *CALLS_FLAGS, "-I" + sysconfig.get_paths()["include"],
                         os.path.join(CSRC, "py_calls.cpp"), "-o", CALLS, "-L" + HERE, "-l:libqkmoe.so", "-Wl,-rpath,$ORIGIN"],
                        capture_output=True, text=True)
     if r.returncode != 0:

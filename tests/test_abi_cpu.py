@@ -25,6 +25,21 @@ def test_header_symbols_are_exported(pkg):
     assert sorted(pkg.SIGNATURES) == names
 
 
+def test_build_stamp_covers_the_extension_module(pkg, monkeypatch):
+    """The binding's extension module belongs to one interpreter and its own compiler flags: another of either is not up to date."""
+    import sys
+    mod = sys.modules["qwen_kernel_b200.build"]
+    now = mod._digest()
+    assert now == mod._digest()
+    with monkeypatch.context() as m:
+        m.setattr(mod.sysconfig, "get_config_var", lambda name: ".cpython-399.so")
+        assert mod._digest() != now
+    with monkeypatch.context() as m:
+        m.setattr(mod, "CALLS_FLAGS", [*mod.CALLS_FLAGS, "-g"])
+        assert mod._digest() != now
+    assert mod._digest() == now
+
+
 def test_row_bytes_and_version(pkg):
     lib = pkg.load_library()
     assert b"sm_100a" in lib.qkm_version()
