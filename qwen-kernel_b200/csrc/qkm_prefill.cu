@@ -21,7 +21,7 @@ constexpr int kTileBytes = 128 * 128;          // 128 rows x 64 f16
 // f16_rows_kernel: the same element order) and f32 accumulation in tensor
 // memory.  These logits only pre-select: the selection kernel re-evaluates every expert within
 // its error bound of the k-th in f64, so the bound has to hold, not the last bits.
-// Error per logit <= (2^-11 [x rounding] + 2^-11 [router rounding] + K * 2^-22 [accumulation])
+// Error per logit <= (2^-11 [x rounding] + 2^-11 [router rounding] + K * 2^-22 [accumulation, measured 2^-25])
 // * |w| * |x|, below 2^-9 * |w| * |x| for K <= 4096.
 // Block = 128 experts (M) x up to 128 tokens (N); 256 producer threads copy both operand tiles
 // into the swizzled layout, the ninth warp issues the MMAs.

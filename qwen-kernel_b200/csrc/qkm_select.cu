@@ -5,12 +5,13 @@
 // (moe_select_256.comp:60-61); weights are a softmax over the selected logits only (moe_select.comp:71-76);
 // w_shared = sigmoid(gate_inp_shexp . x) (moe_select.comp:36-45).
 //
-// The ids equal those of a router that accumulates in f64 (the CPU reference, src/main.cpp:1320-1341): f32 logits carry a provable
-// error bound, every expert within twice the bound of the k-th largest is a candidate, and the candidates' logits are
-// evaluated again in f64, which also gives the weights.  Small batches come with f64 logits, which are ranked as they are.
+// The ids equal those of a router that accumulates in f64 (the CPU reference, src/main.cpp:1320-1341): f32 logits carry an error
+// bound (the f32 sums' proven, the tensor cores' with a measured allowance for their accumulation, see launch_route_select), every
+// expert within twice the bound of the k-th largest is a candidate, and the candidates' logits are evaluated again in f64, which
+// also gives the weights.  Small batches come with f64 logits, which are ranked as they are.
 //
 // Bound by the candidates' f64 dot products (a router row of 8 KB from the L2 and 2048 conversions each; the converter takes 16 lanes
-// a cycle and SM, so a weight becomes an f64 by shifts instead, see weight4) and, for few tokens, by the chain of phases.
+// a cycle and SM, so a weight becomes an f64 by shifts instead, see weight) and, for few tokens, by the chain of phases.
 // A block per token; four warps where there are tokens enough for every SM to hold many blocks, eight below.
 // 4096 tokens, 256 experts, F32 router: 122 us (twice the candidates, converted weights, 12 k instructions to find the k-th) -> 75;
 // 600: 29 -> 19.

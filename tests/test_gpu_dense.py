@@ -88,6 +88,29 @@ def test_dense_gemm_extreme_rows(ctx, orc, syn, ttype, value):
     d_x.free(); d_y.free()
 
 
+@pytest.mark.parametrize("sign", [1, -1])
+@pytest.mark.parametrize("mantissa", [1.0, 2 - 2.0**-9])
+def test_tensor_core_accumulation(ctx, syn, sign, mantissa):
+    """What the tensor cores lose of a small product beside a large one.  The router's candidate bound allows 2^-22 of the sum a
+    column; one product of 64 and 255 of every size below it lose 2^-24 a column at most (measured: 2^-25)."""
+    M, K, n = 128, 256, 32
+    b = np.zeros((M, K // 32, 34), np.uint8)
+    b[:, :, 0:2] = np.array([1], np.float16).view(np.uint8)
+    b[:, :, 2:] = 1
+    b[:, 0, 2] = 64
+    x = np.zeros((n, K), np.float64)
+    x[:, 0] = 1
+    for j in range(2, n):
+        x[j, 1:] = sign * mantissa * 2.0**-min(j, 27)   # f16 operands: normal numbers down to 2^-28 of the row's largest
+    ctx.dense_upload(8, 8, b.reshape(-1), M, K)
+    d_x, d_y = ctx.to_device(x.astype(np.float32)), ctx.alloc(n * M * 4)
+    ctx.dense_gemm(8, d_x, n, d_y)
+    want = 64 + x[:, 1:].sum(axis=1)
+    err = np.abs(d_y.download(np.float32, (n, M)) - want[:, None]).max(axis=1)
+    assert (err <= 255 * 2.0**-24 * np.maximum(64, np.abs(want))).all(), err / (255 * 64 * 2.0**-24)
+    d_x.free(); d_y.free()
+
+
 def test_dense_rejects(ctx, pkg, syn):
     W = syn.random_blocks(8, 128, 256, seed=1)
     d = ctx.alloc(1 << 16)
