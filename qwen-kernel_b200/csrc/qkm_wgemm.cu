@@ -345,7 +345,7 @@ wgemm_kernel(const WgemmArgs a, const __grid_constant__ CUtensorMap rows_map) {
         return it.n != 0;
     };
     // k-step i of a unit: 256-column block and 64-column quarter.  Blocks 2p and 2p + 1 are interleaved (see above).  Of a lone last
-    // block both producer groups get a copy and expand every other quarter, so that a stage always belongs to the same group.
+    // block (dense matrices only) both producer groups get a copy and expand every other quarter, so that a stage always belongs to the same group.
     auto step_kb = [&](uint32_t i) -> uint32_t { return i < (KB & ~1u) * 4 ? 2 * (i >> 3) + (i & 1u) : KB - 1; };
     auto step_q = [&](uint32_t i) -> uint32_t { return i < (KB & ~1u) * 4 ? (i >> 1) & 3u : i & 3u; };
     const uint32_t KS = KB * 4;
@@ -401,7 +401,7 @@ wgemm_kernel(const WgemmArgs a, const __grid_constant__ CUtensorMap rows_map) {
                 if (lane == 0) mbar_arrive(bar_wempty + 8 * kSlots * par);
             };
             for (uint32_t kp = 0; kp < KB; kp += 2) {
-                const bool lone = kp + 1 == KB;
+                const bool lone = MODE == wg::kDense && kp + 1 == KB;
                 const uint32_t i0 = lone ? kp * 4 : kp * 4 + par, istep = lone ? 1u : 2u;   // the block's k-steps: i0 + q * istep
                 if (shared) {
                     // Q8_0, 64 columns a slot: two 544-byte pieces of each tile
@@ -686,7 +686,7 @@ wgemm_kernel(const WgemmArgs a, const __grid_constant__ CUtensorMap rows_map) {
             };
             const uint8_t* src = q8 ? tiles_of((lane >> 3) & 1u) + (size_t)(lane & 7u) * kTileQ8 : tiles_of(lane & 1u);   // this lane's share
             for (uint32_t kp = 0; kp < KB; kp += 2) {
-                const bool lone = kp + 1 == KB;   // both groups get the block, of Q8_0 their quarters of it
+                const bool lone = MODE == wg::kDense && kp + 1 == KB;   // both groups get the block, of Q8_0 their quarters of it
                 if (q8) {
                     for (uint32_t q = 0; q < 4; ++q)
                         for (uint32_t par = 0; par < 2; ++par) {
@@ -968,6 +968,7 @@ static bool rows_tensor_map(CUtensorMap* map, const void* rows, uint64_t n_rows,
 template <int FMT, int MODE, int NT = wg::kNT>
 static cudaError_t wgemm_launch(const Launch& L, const WgemmArgs& a, const void* rows, uint64_t n_rows, uint32_t max_units, uint32_t n_sms) {
     if (max_units == 0) return cudaSuccess;
+    if (MODE != wg::kDense && a.K % 512) return cudaErrorInvalidValue;   // a lone last column block is compiled for dense matrices only
     if (const cudaError_t e = allow_dynamic_smem<wgemm_kernel<FMT, MODE, NT>>((int)wg::smem_end<FMT, NT>())) return e;
     CUtensorMap map{};
     if (((uintptr_t)rows & 15u) || (MODE != wg::kGateUp && !rows_tensor_map(&map, rows, n_rows, a.K))) return cudaErrorInvalidValue;
