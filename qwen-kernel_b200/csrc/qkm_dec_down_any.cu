@@ -1,6 +1,6 @@
 // Down projection of the fused decode sequence for shapes whose (slot, 256-column block) pairs are not exactly the sixteen
-// warps of the two specialised kernels (n_ff = 512 with eight slots): any number of slots up to twenty pairs, n_ff = 256 or 512,
-// IQ4_XS or Q6_K:  y[t] = sum_s w_s * D[ids_s] . h[t][s]  +  w_shared * DS . h[t][n_used].
+// warps of the two specialised kernels (n_ff = 512 with eight slots): any number of slots up to twenty pairs (ten slots),
+// IQ4_XS or Q6_K, n_ff = 512:  y[t] = sum_s w_s * D[ids_s] . h[t][s]  +  w_shared * DS . h[t][n_used].
 //
 // Replaces moe_down_iq4.comp / moe_down_q6k.comp + moe_down_q8b.comp + the "routed + shared" add for those shapes.  Same
 // organisation and arithmetic as the specialised kernels (see qkm_dec_down.cu, qkm_dec_down_q6k.cu): a unit is (token, 16 output rows)
@@ -24,7 +24,7 @@ constexpr int kChunk = 4;                           // tiles between two block-w
 constexpr uint32_t kTab = 0x10000u, kTabBytes = 0x10000u, kHigh = kTab + kTabBytes;   // IQ4_XS table image, absolute shared-window address
 template <bool Q6> struct Cfg {
     static constexpr int kTile = Q6 ? kTileQ6 : kTileIq4, kStage = kTile + kShBlock;
-    static constexpr uint32_t kStages = Q6 ? 2 : 2, kRing = kStages * kStage;      // 7808, 5440
+    static constexpr uint32_t kStages = 2, kRing = kStages * kStage;      // 7808, 5440
     static constexpr uint32_t kLow = 10;                                           // IQ4_XS: rings below the table, up against it; the others above
     static constexpr uint32_t kScratch = Q6 ? 1024 + kMaxWarps * kRing : kHigh + (kMaxWarps - kLow) * kRing;   // Q6_K: from the aligned start
     static constexpr uint32_t kEnd = kScratch + kMaxWarps * 1024 + 2 * kMaxWarps * kChunk * 16 * 4;
@@ -42,7 +42,8 @@ decode_down_any_kernel(DownDecodeArgs a) {
     const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31u, g = lane >> 2, t = lane & 3u;
     const qkm_dims d = a.d;
     const uint32_t n_slots = d.n_used + 1, n_warps = blockDim.x >> 5;
-    const uint32_t KB = d.n_ff / 256, RT = d.n_embd / 16, slot = warp / KB, kb = warp - slot * KB;
+    constexpr uint32_t KB = 2;   // n_ff = 512
+    const uint32_t RT = d.n_embd / 16, slot = warp / KB, kb = warp - slot * KB;
     const bool has_tile = a.tiles != nullptr && slot < d.n_used, has_sh = a.sh_tiles != nullptr && warp < d.n_ff / 32;
     const uint32_t win0 = smem_addr(smem_raw), base = Q6 ? (win0 + 127u) & ~127u : 0u;
     if (!Q6) {   // the fixed addresses must lie inside the dynamic area
@@ -270,7 +271,7 @@ static uint32_t any_warps(const qkm_dims& d) {
     return pairs > sh ? pairs : sh;
 }
 bool decode_down_any_ok(const qkm_dims& d) {
-    return (d.n_ff == 256 || d.n_ff == 512) && d.n_used <= 16 && any_warps(d) <= da::kMaxWarps && d.n_embd % 32 == 0;
+    return d.n_ff == 512 && any_warps(d) <= da::kMaxWarps && d.n_embd % 32 == 0;
 }
 template <bool Q6>
 static cudaError_t any_launch(const Launch& L, const DownDecodeArgs& a, uint32_t n_blocks) {

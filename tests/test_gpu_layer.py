@@ -148,10 +148,16 @@ def test_decode_512_experts(pkg, orc, syn, T):
         assert np.array_equal(y, ctx.moe_forward_host(0, x, mode=0))
 
 
-@pytest.mark.parametrize("n_ff,n_used,dt,T", [(512, 10, 23, 3), (512, 10, 14, 40), (512, 1, 23, 1), (256, 15, 14, 7), (256, 15, 23, 64), (512, 9, 23, 2)])
-def test_decode_numbers_of_slots(pkg, orc, syn, n_ff, n_used, dt, T):
-    """(slot, column block) pairs other than sixteen: more and fewer warps, fewer pairs than shared blocks."""
-    dims = syn.Dims(n_embd=512, n_ff=n_ff, n_expert=32, n_used=n_used)
+def _launches(ctx, call):
+    before = ctx.launch_count()
+    call()
+    return ctx.launch_count() - before
+
+
+@pytest.mark.parametrize("n_used,dt,T", [(10, 23, 3), (10, 14, 5), (1, 23, 1), (2, 14, 7), (7, 14, 39), (9, 23, 2), (10, 23, 39)])
+def test_decode_numbers_of_slots(pkg, orc, syn, n_used, dt, T):
+    """(slot, column block) pairs other than sixteen, token major: more and fewer warps, fewer pairs than shared blocks."""
+    dims = syn.Dims(n_embd=512, n_ff=512, n_expert=32 if T < 30 else 150, n_used=n_used)
     layer = syn.make_layer(dims, seed=16, gateup_type=23, down_type=dt)
     x = syn.random_x(T, dims.n_embd, seed=17)
     ref = orc.moe_layer(layer, x, threads=orc.hardware_threads())
@@ -159,14 +165,14 @@ def test_decode_numbers_of_slots(pkg, orc, syn, n_ff, n_used, dt, T):
         ctx.upload_layer(0, layer)
         y = ctx.moe_forward_host(0, x, mode=0)
         check_layer(syn, y, ctx.last_sel(T), ref, n_used)
-        assert np.array_equal(y, ctx.moe_forward_host(0, x, mode=0))
+        assert _launches(ctx, lambda: np.testing.assert_array_equal(y, ctx.moe_forward_host(0, x, mode=0))) == 3   # the fused sequence
 
 
-@pytest.mark.parametrize("n_embd,n_ff,n_expert,n_used,dt,T", [(512, 512, 256, 8, 23, 40), (256, 512, 32, 1, 23, 41), (1024, 512, 64, 6, 14, 40), (256, 512, 48, 13, 14, 63), (512, 512, 32, 15, 23, 1),
-                                                             (512, 512, 8, 4, 23, 64), (512, 512, 512, 10, 23, 110)])
-def test_decode_down_grouped_by_expert(pkg, orc, syn, n_embd, n_ff, n_expert, n_used, dt, T):
-    """Forty tokens on, or more slots than the token-major kernel takes: odd and full groups, ranges that begin inside a group, a second chunk of 46."""
-    dims = syn.Dims(n_embd=n_embd, n_ff=n_ff, n_expert=n_expert, n_used=n_used)
+@pytest.mark.parametrize("n_embd,n_expert,n_used,dt,T", [(512, 256, 8, 23, 40), (512, 32, 1, 23, 41), (1024, 64, 6, 14, 40), (512, 48, 13, 14, 63), (512, 32, 15, 23, 1),
+                                                         (512, 8, 4, 23, 64), (512, 512, 10, 23, 110), (512, 20, 11, 14, 2), (512, 30, 1, 14, 61)])
+def test_decode_down_grouped_by_expert(pkg, orc, syn, n_embd, n_expert, n_used, dt, T):
+    """Forty tokens on, or more slots than the token-major kernel takes: odd and full groups, one slot, ranges that begin inside a group, a second chunk of 46."""
+    dims = syn.Dims(n_embd=n_embd, n_ff=512, n_expert=n_expert, n_used=n_used)
     layer = syn.make_layer(dims, seed=18, gateup_type=23, down_type=dt)
     x = syn.random_x(T, dims.n_embd, seed=19)
     ref = orc.moe_layer(layer, x, threads=orc.hardware_threads())
@@ -176,7 +182,7 @@ def test_decode_down_grouped_by_expert(pkg, orc, syn, n_embd, n_ff, n_expert, n_
         ctx.moe_decode(0, d_x, T, d_y)
         y = d_y.download(np.float32, x.shape)
         check_layer(syn, y, ctx.last_sel(T), ref, n_used)
-        ctx.moe_decode(0, d_x, T, d_y)
+        assert _launches(ctx, lambda: ctx.moe_decode(0, d_x, T, d_y)) == 4 * ((T + 63) // 64)   # the fused sequence and its fold
         assert np.array_equal(y, d_y.download(np.float32, x.shape))
 
 
