@@ -190,7 +190,7 @@ def rel_err_reference(got: np.ndarray, ref: np.ndarray) -> float:
 
 def rel_err_rows(got: np.ndarray, ref: np.ndarray) -> float:
     """Row-scaled relative error: |got-ref| / max(|ref|, rms(ref row)), max over
-    all elements.  This is the "relative" figure the f32 (1e-5) and bf16 (2e-2)
+    all elements.  This is the "relative" figure the f32 (1e-5) and f16-operand (1e-2)
     output tolerances are stated in."""
     g = got.astype(np.float64).reshape(ref.shape[0], -1) if ref.ndim > 1 else got.astype(np.float64).reshape(1, -1)
     r = ref.astype(np.float64).reshape(g.shape)

@@ -1,11 +1,11 @@
 """Dense quantised GEMM (the reference's gemm_q8_0 / gemm_iq4_xs prefill projections) on the
-tensor-core pipeline against the oracle's f64 GEMV, row by row.  bf16 operands: 2e-2 relative
-(row-scaled), as for the expert GEMMs."""
+tensor-core pipeline against the oracle's f64 GEMV, row by row.  f16 operands, x and a weight's scale and product rounded to
+2^-11 each: 5e-3 relative for the worst element (row-scaled; about 0.35e-3 as a norm)."""
 import numpy as np
 import pytest
 
 pytestmark = pytest.mark.gpu
-TOL = 2e-2
+TOL = 5e-3
 
 
 @pytest.fixture(scope="module")
@@ -46,7 +46,7 @@ def test_dense_gemm_edges(ctx, orc, syn, ttype, M, K, n):
     ctx.dense_gemm(4, d_x, n, d_y)
     ctx.sync()
     want = orc.gemv(ttype, W, x, M, K, threads=orc.hardware_threads())
-    assert syn.rel_err_rows(d_y.download(np.float32, (n, M)), want) < TOL / 4   # f16 operands
+    assert syn.rel_err_rows(d_y.download(np.float32, (n, M)), want) < TOL
     d_x.free(); d_y.free()
 
 

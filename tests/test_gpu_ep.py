@@ -2,8 +2,8 @@
 ranks, the all-to-all is done by copying rows between their buffers on the host.  No
 kernel waits on another, so running the ranks one after the other is safe on one device.
 
-Tolerance: the expert GEMMs run on the tensor cores (bf16/f16 operands), so outputs are held
-to the prefill tolerance 2e-2 (row-scaled) against the f64 oracle; ids, send order and split
+Tolerance: the expert GEMMs run on the tensor cores (f16 operands), so outputs are held
+to the prefill tolerance 1e-2 (row-scaled) against the f64 oracle; ids, send order and split
 sizes are exact.  Shapes and type mixes outside the shard's tensor-core path take the f32 kernels and are
 held to 1e-5."""
 import numpy as np
@@ -13,7 +13,7 @@ from ep_cpu_engine import plan_send
 
 pytestmark = pytest.mark.gpu
 
-TOL_BF16 = 2e-2
+TOL_TC = 1e-2
 TOL_F32 = 1e-5
 
 
@@ -105,14 +105,14 @@ def test_ep_full_size_shapes(pkg, orc, syn, G, T):
     cuts = np.linspace(0, T, G + 1).astype(int)
     cuts[1] = min(T, cuts[1] + 3)                       # uneven shares
     parts = [x[cuts[r]:cuts[r + 1]] for r in range(G)]
-    run_ep(pkg, orc, syn, dims, layer, parts, G, TOL_BF16)
+    run_ep(pkg, orc, syn, dims, layer, parts, G, TOL_TC)
 
 
 def test_ep_rank_without_tokens(pkg, orc, syn):
     dims = syn.Dims()
     layer = syn.make_layer(dims, seed=43)
     x = syn.random_x(5, dims.n_embd, seed=62)
-    run_ep(pkg, orc, syn, dims, layer, [x, x[:0]], 2, TOL_BF16)
+    run_ep(pkg, orc, syn, dims, layer, [x, x[:0]], 2, TOL_TC)
 
 
 def test_ep_generic_kernels_f32(pkg, orc, syn):
@@ -229,14 +229,14 @@ def test_ep_peer_full_size_shapes(pkg, orc, syn, G, T, extra, merged):
     cuts = np.linspace(0, T, G + 1).astype(int)
     cuts[1] = min(T, cuts[1] + 3)                       # uneven shares
     parts = [x[cuts[r]:cuts[r + 1]] for r in range(G)]
-    run_ep_peer(pkg, orc, syn, dims, layer, parts, G, TOL_BF16, cap_extra=extra, merged=merged)
+    run_ep_peer(pkg, orc, syn, dims, layer, parts, G, TOL_TC, cap_extra=extra, merged=merged)
 
 
 def test_ep_peer_rank_without_tokens_and_tight_slots(pkg, orc, syn):
     dims = syn.Dims()
     layer = syn.make_layer(dims, seed=47)
     x = syn.random_x(5, dims.n_embd, seed=65)
-    run_ep_peer(pkg, orc, syn, dims, layer, [x, x[:0]], 2, TOL_BF16, slot_rows=5, cap_extra=3)
+    run_ep_peer(pkg, orc, syn, dims, layer, [x, x[:0]], 2, TOL_TC, slot_rows=5, cap_extra=3)
 
 
 def test_ep_peer_generic_kernels_f32(pkg, orc, syn):
@@ -311,7 +311,7 @@ def test_ep_peer_layer_single_rank_with_device_barrier(pkg, orc, syn):
             c.sync()
             y = d_y.download(np.float32, x.shape)
             want = orc.moe_layer(layer, x, threads=orc.hardware_threads())["y"]
-            assert syn.rel_err_rows(y, want) < TOL_BF16
+            assert syn.rel_err_rows(y, want) < TOL_TC
         d_x.free(); d_y.free()
 
 

@@ -1,15 +1,16 @@
-"""Batched prefill through the tensor-core path (bf16 operands, f32 accumulation) against the
-f64-accumulating oracle.  Tolerance: 2e-2 on the row-scaled relative error (measured: about 4e-3), expert ids exact,
+"""Batched prefill through the tensor-core path (f16 operands, f32 accumulation) against the
+f64-accumulating oracle.  Tolerance: 1e-2 on the row-scaled relative error of the worst element (measured: about 4e-3; x, weights
+and hidden rows rounded to 2^-11 each, two GEMMs: 0.6e-3 as a norm), expert ids exact,
 argmax of every output row unchanged (where the reference itself is not a near-tie)."""
 import numpy as np
 import pytest
 
 pytestmark = pytest.mark.gpu
 
-TOL_BF16 = 2e-2
+TOL = 1e-2
 
 
-def run_prefill(pkg, orc, syn, dims, layer, x, tol=TOL_BF16):
+def run_prefill(pkg, orc, syn, dims, layer, x, tol=TOL):
     T = x.shape[0]
     ref = orc.moe_layer(layer, x, threads=orc.hardware_threads(), want_h=True)
     with pkg.Context(dims, n_layer=1, max_tokens=max(T, 1), device=0) as ctx:
@@ -42,8 +43,8 @@ def test_prefill_full_size(pkg, orc, syn, T):
 
 def test_prefill_operand_precision(pkg, orc, syn):
     """Both expert GEMMs run on f16 operands (x and the hidden rows scaled per row by a power of two,
-    the dequantised weights rounded once or twice to f16), so the outputs sit well inside the 2e-2
-    budget: a third of it at most on the full-size layer."""
+    the dequantised weights rounded once or twice to f16), so the outputs sit well inside the 1e-2
+    budget on the full-size layer."""
     dims = syn.Dims()
     layer = syn.make_layer(dims, seed=42)
     x = syn.random_x(130, dims.n_embd, seed=78)
@@ -60,7 +61,7 @@ def test_prefill_bench_chunk_sizes(pkg, orc, syn, T):
     is cheap - including tie / NaN / all-zero rows placed beyond row 1024 where the chunk has
     them.  Outputs: the oracle's full layer on >= 64 sampled rows (selection given) that include
     the first and the last row, rows from every 128-pair N-tile of the busiest expert, and the
-    special rows; 2e-2 row-scaled relative."""
+    special rows; 1e-2 row-scaled relative."""
     dims = syn.Dims()
     layer = syn.make_layer(dims, seed=42, router_type=syn.F32)
     r = layer.router.view(np.float32).reshape(256, 2048).copy()
@@ -109,7 +110,7 @@ def test_prefill_bench_chunk_sizes(pkg, orc, syn, T):
         assert counts[busiest] > 128, "the busy expert should span more than one N-tile"
     ref = orc.moe_layer(layer, x[rows], threads=nthr, sel_in=want[rows])
     err = syn.rel_err_rows(y[rows], ref["y"])
-    assert err < TOL_BF16, err
+    assert err < TOL, err
     assert np.isfinite(y[np.setdiff1d(np.arange(T), [x_nan] if x_nan is not None else [])]).all()
 
 
@@ -215,7 +216,7 @@ def test_prefill_large_weight_rows(pkg, orc, syn, gt, dt):
 
 
 def test_prefill_matches_decode_path(pkg, syn):
-    """The two fused paths agree to bf16 accuracy on the same inputs."""
+    """The two fused paths agree to f16 accuracy on the same inputs."""
     dims = syn.Dims()
     layer = syn.make_layer(dims, seed=8)
     x = syn.random_x(24, dims.n_embd, seed=9)
@@ -223,14 +224,14 @@ def test_prefill_matches_decode_path(pkg, syn):
         ctx.upload_layer(0, layer)
         yd = ctx.moe_forward_host(0, x, mode=0)
         yp = ctx.moe_forward_host(0, x, mode=1)
-    assert syn.rel_err_rows(yp, yd) < TOL_BF16
+    assert syn.rel_err_rows(yp, yd) < TOL
 
 
 @pytest.mark.parametrize("gt,dt", [(18, 14), (23, 23), (23, 14)])
 @pytest.mark.parametrize("T", [70, 200])
 def test_prefill_other_type_mixes(pkg, orc, syn, T, gt, dt):
     """Q6_K (14) down tensors and IQ4_XS (23) gate/up tensors: both expert GEMMs on the tensor cores
-    (kernels that dequantise Q6_K / IQ4_XS tiles to f16 in shared memory)."""
+    (Q6_K / IQ4_XS tiles expanded to f16 in tensor memory)."""
     dims = syn.Dims()
     layer = syn.make_layer(dims, seed=46, router_type=syn.F32, gateup_type=gt, down_type=dt)
     x = syn.random_x(T, dims.n_embd, seed=78)
