@@ -737,13 +737,14 @@ static int expert_gemms(qkm_ctx* c, const qkm_layer_dev& ld, const qkm_sel* sel,
     const uint32_t tiles = (c->ecount < np_max ? c->ecount + (np_max + NT - 1) / NT : np_max) + (sh_max + NT - 1) / NT;
     WgemmExperts g{{ld.tiles[2], ld.tiles[3]}, {ld.tiles[5], ld.tiles[6]}, c->mma_items[0], c->n_items, c->n_items + 2, c->pairs, c->lut_pf, c->status, c->ecount, (uint32_t)c->n_sms, NT};
     QKM_LAUNCH(c, launch_wgemm_gateup(c->L(), d, ld.w.gateup_type, g, c->xb, c->xscale, c->xnorm, ld.w_norm, c->hb, c->hscale, tiles * (d.n_ff / 128)));
+    c->prof_mark("moe.gu");
     HiddenRows r{};
     r.pairs = c->pairs; r.pos_of = c->pos_of; r.sel = sel; r.xrows = (const __half*)c->xb; r.x_inv_scale = c->xscale; r.x_norm = c->xnorm; r.w_norm = ld.w_norm;
     r.w[0] = (const uint8_t*)ld.w.gate_exps; r.w[1] = (const uint8_t*)ld.w.up_exps; r.sh[0] = (const uint8_t*)ld.w.gate_shexp; r.sh[1] = (const uint8_t*)ld.w.up_shexp;
     r.h = (__half*)c->hb; r.h_inv_scale = c->hscale; r.n_tokens = n; r.n_used = d.n_used; r.n_expert = d.n_expert; r.expert_first = c->efirst;
     r.expert_count = c->ecount; r.n_ff = d.n_ff; r.n_embd = d.n_embd;
     QKM_LAUNCH(c, launch_hidden_rows_check(c->L(), ld.w.gateup_type, r));
-    c->prof_mark("moe.gu");
+    c->prof_mark("moe.h_check");
     WgemmExperts m{{ld.tiles[4], nullptr}, {ld.tiles[7], nullptr}, c->mma_items[1], c->n_items + 1, c->n_items + 3, c->pairs, c->lut_pf, c->status, c->ecount, (uint32_t)c->n_sms, NT};
     QKM_LAUNCH(c, launch_wgemm_down(c->L(), d, ld.w.down_type, m, c->hb, (uint64_t)c->cfg.max_tokens * (d.n_used + 1), c->hscale, sel, c->contrib_p,
                                     tiles * (d.n_embd / 256)));

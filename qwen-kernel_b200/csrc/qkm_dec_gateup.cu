@@ -20,8 +20,8 @@
 //     each into bits 8..15 of a table address whose other bytes are lane constants (the grid
 //     table has a 256-byte stride per entry and sits at a 64 KB boundary), so a lookup
 //     address costs one instruction;
-//   * the 7-bit sign code is rotated to bits 9..15 and masked into the address of the sign
-//     table, which lives in the unused half of the same 256-byte rows;
+//   * the tiles hold signs as bits at places where a shift brings four of them to the top of their
+//     bytes, and a byte permute in sign mode turns those into 0xFF / 0x00 masks;
 //   * magnitudes ^ mask is -m-1 where the element is negative; a second MMA of the masks
 //     (-1 / 0) with the negated digit planes adds the missing +1 * x, so no per-element
 //     sign arithmetic remains;
@@ -67,23 +67,11 @@ constexpr uint32_t kCostRouted = 8, kCostShared = 11;   // relative time of a ro
 
 size_t decode_gateup_lut_bytes() { return dg::kTabBytes; }
 
-// The table image: row i (256 B) = grid entry i for 32 lanes (4 B each), then, in the upper 128 B,
-// sign masks: row 2c + hl holds code c for lanes 16*hl .. 16*hl+15, 8 B each (byte j = 0xFF when
-// element j of the 8-group is negative).
+// The table image: row i (256 B) = grid entry i for 32 lanes (4 B each); the upper 128 B are not read.
 __global__ void decode_gateup_lut_kernel(uint8_t* __restrict__ out) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;   // one 4-byte word each
     if (i >= dg::kTabBytes / 4) return;
-    const uint32_t row = i >> 6, w = i & 63u;
-    uint32_t v;
-    if (w < 32) {
-        v = c_iq3_grid[row];
-    } else {
-        const uint32_t sg = signs8(row >> 1), hi = w & 1u;
-        v = 0;
-#pragma unroll
-        for (int j = 0; j < 4; ++j) v |= ((sg >> (j + 4 * hi)) & 1u) ? (0xFFu << (8 * j)) : 0u;
-    }
-    reinterpret_cast<uint32_t*>(out)[i] = v;
+    reinterpret_cast<uint32_t*>(out)[i] = (i & 63u) < 32 ? c_iq3_grid[i >> 6] : 0u;
 }
 
 cudaError_t launch_decode_gateup_luts(const Launch& L, uint8_t* luts) {

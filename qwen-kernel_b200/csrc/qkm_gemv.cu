@@ -401,10 +401,4 @@ cudaError_t launch_gemv_stream(const Launch& L, uint32_t type, const void* W, co
     return cudaSuccess;
 }
 
-cudaError_t launch_gemv(const Launch& L, uint32_t type, const void* W, const float* x, float* y,
-                        uint32_t M, uint32_t K, uint32_t n) {
-    if (M == 0 || n == 0) return cudaSuccess;
-    return launch_gemv_tail(L, type, W, x, y, M, K, n, M);
-}
-
 }  // namespace qkm

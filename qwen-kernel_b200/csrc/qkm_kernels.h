@@ -57,7 +57,7 @@ __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;"
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 #endif
 
-// One unit of the prefill GEMMs: an expert, 256 rows of its matrices and up to 128
+// One unit of the prefill GEMMs: an expert, 256 rows of its matrices and up to 128 or 160
 // of its pairs (pairs[pair_off .. pair_off + n)).
 struct MmaItem {
     uint16_t expert;
@@ -201,8 +201,6 @@ cudaError_t launch_scale_max(const Launch& L, uint32_t type, const void* raw, ui
 
 // ---- qkm_gemv.cu
 cudaError_t launch_dequant(const Launch& L, uint32_t type, const void* blocks, float* y, uint64_t n_elems);
-cudaError_t launch_gemv(const Launch& L, uint32_t type, const void* W, const float* x, float* y,
-                        uint32_t M, uint32_t K, uint32_t n);
 
 // streamed form (bulk-copy ring) with the generic kernel for tail rows / unaligned tensors
 cudaError_t launch_gemv_mma(const Launch& L, uint32_t type, const void* W, const float* x, float* y, uint32_t M,
@@ -334,7 +332,7 @@ struct EpPeerTable {
 };
 cudaError_t launch_ep_barrier(const Launch& L, const EpPeerTable& peers, uint32_t rank, uint32_t n_ranks, uint32_t epoch,
                               uint64_t limit_ns, uint32_t* status);
-// xh / x_inv_scale: the rows as scaled f16 (to_f16_rows_kernel) - then those travel instead of the f32 rows
+// xh / x_inv_scale: the rows as scaled f16 (launch_f16_rows) - then those travel instead of the f32 rows
 cudaError_t launch_ep_push(const Launch& L, const qkm_dims& d, const float* x, const qkm_sel* sel, const EpPeerTable& peers,
                            uint32_t n_tokens, uint32_t slot_rows, uint32_t rank, uint32_t n_ranks, const void* xh = nullptr,
                            const float* x_inv_scale = nullptr);

@@ -2,7 +2,6 @@
 // bounded mbarrier waits, tensor-core MMA wrappers, codebook tables in shared memory.
 #pragma once
 
-#include <cuda_bf16.h>
 #include <stdint.h>
 
 #include "qkm_common.cuh"

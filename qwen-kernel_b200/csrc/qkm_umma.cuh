@@ -1,8 +1,8 @@
 // 5th-generation tensor core (tcgen05) building blocks for the batched-prefill GEMMs:
-// tensor-memory allocation, shared-memory matrix descriptors for K-major bf16 tiles in
+// tensor-memory allocation, shared-memory matrix descriptors for K-major f16 tiles in
 // the 128-byte swizzle layout, the MMA issue, commit-to-mbarrier, accumulator loads.
 //
-// Operand layout used throughout (both A and B are K-major, bf16, K extent 64 per tile):
+// Operand layout used throughout (both A and B are K-major, f16, K extent 64 per tile):
 //   a tile of R rows x 64 columns occupies R * 128 bytes; rows are grouped by 8 into
 //   1024-byte atoms; inside an atom row r holds its eight 16-byte chunks at
 //   chunk position (c ^ r): byte offset of element (row, k) =
@@ -45,18 +45,7 @@ __device__ __forceinline__ bool elect_one() {
     return p != 0;
 }
 
-// instruction descriptor: bf16 x bf16 -> f32, both operands K-major, M = 128, N = n (multiple of 16)
-__device__ __forceinline__ uint32_t instr_desc_bf16(uint32_t n) {
-    uint32_t d = 0;
-    d |= 1u << 4;            // D format: f32
-    d |= 1u << 7;            // A format: bf16
-    d |= 1u << 10;           // B format: bf16
-    d |= (n >> 3) << 17;     // N / 8
-    d |= (128u >> 4) << 24;  // M / 16
-    return d;
-}
-
-// same with f16 inputs
+// instruction descriptor: f16 x f16 -> f32, both operands K-major, M = 128, N = n (multiple of 16)
 __device__ __forceinline__ uint32_t instr_desc_f16(uint32_t n) {
     uint32_t d = 0;
     d |= 1u << 4;            // D format: f32; A and B formats 0 = f16
@@ -75,7 +64,7 @@ __device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t ncols) {  
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
 }
 
-// D[tmem] (+)= A[smem] * B[smem] (kind::f16: f16 or bf16 inputs per the instruction descriptor); issued by ONE thread
+// D[tmem] (+)= A[smem] * B[smem] (kind::f16, f16 inputs); issued by ONE thread
 __device__ __forceinline__ void mma_f16_ss(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
                                             bool accumulate) {
     const uint32_t acc = accumulate ? 1u : 0u;
