@@ -70,6 +70,11 @@ __device__ __forceinline__ void mma_f16_k16_first(float (&c)[4], uint32_t a0, ui
                  : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "f"(0.f));
 }
 
+// (a0, a1) += (b0, b1), one instruction
+__device__ __forceinline__ void add_f32x2(float& a0, float& a1, float b0, float b1) {
+    asm("{\n.reg .b64 x, y;\nmov.b64 x, {%0,%1};\nmov.b64 y, {%2,%3};\nadd.rn.f32x2 x, x, y;\nmov.b64 {%0,%1}, x;\n}\n" : "+f"(a0), "+f"(a1) : "f"(b0), "f"(b1));
+}
+
 // Eight consecutive columns (8 * lane ..) of one activation row into the B fragments of one 256-column block.
 // frag: this block's and this row's column tile; cg: the row's first column (0 or 4) in the tile.
 template <int TYPE>
@@ -259,7 +264,7 @@ __device__ __forceinline__ void tile_sums(uint32_t r0, uint32_t r1, uint32_t bf,
 // An f16 MMA adds its products (and the D it is given) by truncation, so a chain of sixteen of them drifts towards zero: 3.5e-7
 // from 64 bits (norm, K 512 to 4096), where f32 FMAs of rounded additions are at 0.9e-7 to 2.1e-7.  Every MMA therefore starts from
 // zero and eight partial sums at a time are added in f32 as a tree: 0.8e-7 to 1.1e-7; one after the other 0.9e-7 to 1.1e-7 (above
-// the FMAs at K = 512).  It costs 4 to 20 % (4096 x 2048: 16 rows 11.1 -> 12.7 us, 2 rows 6.1 -> 6.1).
+// the FMAs at K = 512).  It costs up to 16 % (4096 x 2048: 16 rows 11.1 -> 12.3 us, 2 rows 6.1 -> 6.1; 12.9 with scalar additions).
 template <int NT>
 __device__ __forceinline__ void tile_sums_f16(const uint8_t* __restrict__ p0, const uint8_t* __restrict__ p1, uint32_t bf, const float (&sc)[NT],
                                               float dw0, float dw1, float (&f)[NT][2]) {
@@ -286,9 +291,9 @@ __device__ __forceinline__ void tile_sums_f16(const uint8_t* __restrict__ p0, co
 #pragma unroll
                 for (int i = 0; i < w; ++i)
 #pragma unroll
-                    for (int j = 0; j < 4; ++j) p[i][j] += p[i + w][j];
+                    for (int j = 0; j < 4; j += 2) add_f32x2(p[i][j], p[i][j + 1], p[i + w][j], p[i + w][j + 1]);
 #pragma unroll
-            for (int j = 0; j < 4; ++j) c[nt][j] += p[0][j];
+            for (int j = 0; j < 4; j += 2) add_f32x2(c[nt][j], c[nt][j + 1], p[0][j], p[0][j + 1]);
         }
     }
 #pragma unroll
