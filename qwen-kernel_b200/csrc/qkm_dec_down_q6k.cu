@@ -20,6 +20,8 @@
 // routing weight are applied once per tile in f32.
 //
 // Shared expert: warp w also takes 32-column block w of the Q8_0 matrix for the tile's rows.
+//
+// Against the general form (qkm_dec_down_any.cu): a layer of 16 tokens 70.2 -> 69.0 us, of 39 128.1 -> 126.4.
 #include "qkm_dec_tiles.cuh"
 #include "qkm_kernels.h"
 #include "qkm_stream.cuh"

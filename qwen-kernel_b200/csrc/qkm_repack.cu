@@ -1,7 +1,7 @@
 // Upload-time re-ordering of raw ggml tensors into the tile layout the streaming
-// kernels read (see qkm_tiles.cuh).  Pure byte permutation: every output byte is a
-// copy of one input byte, so dequantised values are unchanged and the byte count of
-// a tensor stays what a GGUF file holds for it.
+// kernels read (see qkm_tiles.cuh).  The weights' values are unchanged: Q6_K and Q8_0 bytes are moved, IQ4_XS
+// nibbles are paired anew (as many bytes), IQ3_XXS sign codes become sign bits and its 4-bit scales bytes
+// 2 s + 1 (1696 bytes a tile for 1568 of the file).
 #include "qkm_common.cuh"
 #include "qkm_kernels.h"
 #include "qkm_tiles.cuh"

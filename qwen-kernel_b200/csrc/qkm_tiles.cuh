@@ -50,11 +50,11 @@
 //     [ 32,544)  quants: half h (row g + 8h), lane -> 8 B at 32 + (h*32 + lane)*8
 //                = raw qs[4t..4t+3] then qs[16+4t..16+4t+3]
 //
-// DIGIT PLANES.  An activation row x[K] is encoded as four int8 planes with one
-// power-of-two scale per row (or per 128-element chunk for the expert hidden rows):
+// DIGIT PLANES.  An activation row x[K] (or a hidden row) is encoded as four int8 planes with one
+// power-of-two scale per 256 columns:
 //   v = rint(x * 2^p),  |v| <= 2^26,  v = d0 + 128*d1 + 128^2*d2 + 128^3*d3,  d_j in [-64, 63]
-// so x = 2^-p * sum_j 128^j d_j up to a rounding error of 2^-(p+1) <= 2^-27 * max|x|:
-// finer than f32 for every element within 2^3 of the row maximum and exact integer
+// so x = 2^-p * sum_j 128^j d_j up to a rounding error of 2^-(p+1) <= 2^-26 * max|x| over the block
+// (max|x| * 2^p lies in [2^25, 2^26)): finer than f32 for the largest elements, coarser below, and exact integer
 // arithmetic from there on (int8 x int8 -> int32 tensor-core MMAs).
 #pragma once
 

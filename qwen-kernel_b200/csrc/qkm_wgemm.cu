@@ -5,7 +5,7 @@
 // moe_down_q8_coopmat.comp and the batched projections gemm_q8_0*.comp / gemm_iq4_xs.comp.
 //
 // A unit of work is 256 weight rows (gate and up rows of one 128-row tile, or two consecutive row tiles of a down or
-// dense matrix) times up to 128 activation rows.  Weights are the M = 128 operand and live in tensor memory: a
+// dense matrix) times up to 128 (or 160, see qkm_units.h) activation rows.  Weights are the M = 128 operand and live in tensor memory: a
 // producer thread owns one weight row, reads its quant bytes from shared memory, expands them to f16 and stores
 // them with tcgen05.st; activation rows (f16, scaled per row by a power of two) are the N operand in shared memory.
 //
@@ -22,13 +22,13 @@
 //                      64 rows on (588 us against 250 at 4096 tokens); consecutive rows (down, dense) by TMA boxes of 16 rows
 //
 // What bounds it: few rows per expert: the producers' instructions (nominally 1.5 to 3.3 per weight by format, 3.5 with
-// barriers, address and scale work; issue slots 58 % busy at 77 tokens).  Measured per layer (256 experts, top 8), before
-// (operands dequantised into shared memory or, for one format each, into TMEM by threads that also copied the rows) and now:
-//   gate/up IQ3_XXS   77 tokens 167 -> 89 us, 600: 176 -> 103, 4096: 301 -> 247 (the shared expert's units included now)
-//   gate/up IQ4_XS    77: 340 -> 91, 600: 371 -> 112, 4096: 631 -> 248
-//   down IQ4_XS       77: 133 -> 51, 600: 153 -> 61, 4096: 287 -> 155;   down Q6_K 600: 273 -> 82, 4096: 479 -> 170
-//   shared expert     82 us beside the routed kernels -> a share of the above
-//   dense 1000 x 4096 x 2048, Q8_0 and IQ4_XS: 103 -> 37 us each
+// barriers, address and scale work; issue slots 74 % busy in gate/up and 60 % in down at 77 tokens).  Measured per layer (256 experts,
+// top 8), before (operands dequantised into shared memory or, for one format each, into TMEM by threads that also copied the rows)
+// and now, the shared expert's units (82 us in kernels of its own before, beside the routed ones) included now:
+//   gate/up IQ3_XXS   77 tokens 167 -> 88 us, 600: 176 -> 102, 4096: 301 -> 206
+//   gate/up IQ4_XS    77: 340 -> 92, 600: 371 -> 107, 4096: 631 -> 214
+//   down IQ4_XS       77: 133 -> 51, 600: 153 -> 62, 4096: 287 -> 150;   down Q6_K 600: 273 -> 76, 4096: 479 -> 165
+//   dense 1000 x 4096 x 2048, Q8_0 and IQ4_XS: 103 -> 29 us each
 //
 // K order.  Inside every group of four columns the operands hold elements (0, 2, 1, 3): that is the order in which
 // the bytes and nibbles of the tiles unpack to f16 pairs without a permute.  x and h rows are written in that order.
