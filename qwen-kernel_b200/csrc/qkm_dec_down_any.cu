@@ -253,8 +253,8 @@ decode_down_any_kernel(DownDecodeArgs a) {
         if (tid < 16 * n_c) {
             const uint32_t i = tid >> 4, r = tid & 15u;   // tile i of the chunk
             float sum = 0.f;
-            for (uint32_t w = 0; w < n_warps; ++w)   // slot order, column blocks inside a slot
-                sum += red[((buf * da::kMaxWarps + w) * da::kChunk + i) * 16 + r];
+            for (uint32_t w = 0; w < n_warps; w += 2)   // slot order; a slot's two column blocks first (half as many roundings in a chain)
+                sum += red[((buf * da::kMaxWarps + w) * da::kChunk + i) * 16 + r] + red[((buf * da::kMaxWarps + w + 1) * da::kChunk + i) * 16 + r];
             a.y[(size_t)tok * d.n_embd + (rt + i) * 16 + r] = sum;
         }
         buf ^= 1u;
