@@ -283,10 +283,11 @@ decode_down_kernel(DownDecodeArgs a) {
                 va += w_sh * (sda * ((float)c[0] * dw0 + (float)c[1] * dw1));
                 vb += w_sh * (sdb * ((float)c[2] * dw0 + (float)c[3] * dw1));
             }
+            // digits 0, 1 sit in lane t = 0 and 2, 3 in t = 1
+            // (before the stage is filled again: no read of it is under way then, which the copy would not wait for)
+            va += __shfl_xor_sync(0xFFFFFFFFu, va, 1); vb += __shfl_xor_sync(0xFFFFFFFFu, vb, 1);
             __syncwarp();
             if (lane == 0) issue(stage);
-            // digits 0, 1 sit in lane t = 0 and 2, 3 in t = 1
-            va += __shfl_xor_sync(0xFFFFFFFFu, va, 1); vb += __shfl_xor_sync(0xFFFFFFFFu, vb, 1);
             if (t == 0) {
                 float* r = red + ((buf * dd::kWarps + warp) * dd::kChunk + i) * 16;
                 r[g] = va; r[g + 8] = vb;

@@ -225,7 +225,6 @@ decode_down_group_kernel(DownDecodeArgs a) {
                     }
                 }
                 const uint32_t d2 = lds32(tb + 3328 + 2 * (g & ~1u)), d8 = lds32(tb + 3328 + 16 + 2 * (g & ~1u));
-                next();
                 const float da = f16_bits_to_f32((d2 >> (16 * (g & 1u))) & 0xFFFFu), db = f16_bits_to_f32((d8 >> (16 * (g & 1u))) & 0xFFFFu);
                 const float q0 = (t & 1u) ? 16384.f : 1.f, q1 = q0 * 128.f;   // columns 2t, 2t+1: digits 2 (t & 1), + 1 of group t / 2
                 va = w0 * (da * ((float)acc[0][0] * q0 + (float)acc[0][1] * q1)); vb = w0 * (db * ((float)acc[0][2] * q0 + (float)acc[0][3] * q1));
@@ -256,7 +255,6 @@ decode_down_group_kernel(DownDecodeArgs a) {
                         acc[0] += la * c[0]; acc[1] += la * c[1]; acc[2] += lb * c[2]; acc[3] += lb * c[3];
                     }
                 }
-                next();
                 va = f16_bits_to_f32(hd.x & 0xFFFFu) * ((float)acc[0] * w0 + (float)acc[1] * w1);
                 vb = f16_bits_to_f32(hd.z & 0xFFFFu) * ((float)acc[2] * w0 + (float)acc[3] * w1);
             }
@@ -275,11 +273,14 @@ decode_down_group_kernel(DownDecodeArgs a) {
                     va += f16_bits_to_f32((dw >> (16 * (g & 1u))) & 0xFFFFu) * ((float)c[0] * w0 + (float)c[1] * w1);
                     vb += f16_bits_to_f32((dw8 >> (16 * (g & 1u))) & 0xFFFFu) * ((float)c[2] * w0 + (float)c[3] * w1);
                 }
+                vb = __shfl_sync(0xFFFFFFFFu, vb, lane);   // (as below)
                 next();
             }
         }
         // the token's other two digits sit in lane t^1
+        // (before the stage is filled again: no read of it is under way then, which the copy would not wait for)
         va += __shfl_xor_sync(0xFFFFFFFFu, va, 1); vb += __shfl_xor_sync(0xFFFFFFFFu, vb, 1);
+        if (rec.kind == 0) next();
         if ((t & 1u) == 0) {
             float* r = red + ((warp * 2 + e_buf) * dp::kGroupTiles + e_n) * 32 + (t >> 1);
             r[2 * g] = va; r[2 * (g + 8)] = vb;

@@ -350,6 +350,13 @@ decode_gateup_kernel(GateupDecodeArgs a) {
         }
         if (e_n == 0) e_first = rt;
         float ga, gb, ua, ub;
+        // The token's other two digits sit in lane t^1.  The exchange comes before the stage is filled again: it needs what was read last, so
+        // no read is under way any more.  (A copy does not wait for reads that are: with the refill first, a tile's last rows got the scales of
+        // the tile after next, once in some ten thousand launches.)
+        auto both_halves = [&]() {
+            ga += __shfl_xor_sync(0xFFFFFFFFu, ga, 1); gb += __shfl_xor_sync(0xFFFFFFFFu, gb, 1);
+            ua += __shfl_xor_sync(0xFFFFFFFFu, ua, 1); ub += __shfl_xor_sync(0xFFFFFFFFu, ub, 1);
+        };
         if (rec.kind == 0) {
             const uint32_t stage = cnt % dg::kStages, parity = (cnt / dg::kStages) & 1u;
             if (!mbar_wait_bounded(my_bar + 8 * stage, parity)) timed_out = true;
@@ -359,9 +366,6 @@ decode_gateup_kernel(GateupDecodeArgs a) {
                 uint4 hg, hu;
                 iq4_tile_gu(sbase, i_off, g, b0, b1, ig, hg);
                 iq4_tile_gu(sbase + kTileIq4, i_off, g, b0, b1, iu, hu);
-                __syncwarp();
-                if (lane == 0) issue(stage);
-                ++cnt;
                 ga = f16_bits_to_f32(hg.x & 0xFFFFu) * ((float)ig[0] * wcol0 + (float)ig[1] * wcol1);
                 gb = f16_bits_to_f32(hg.z & 0xFFFFu) * ((float)ig[2] * wcol0 + (float)ig[3] * wcol1);
                 ua = f16_bits_to_f32(hu.x & 0xFFFFu) * ((float)iu[0] * wcol0 + (float)iu[1] * wcol1);
@@ -371,9 +375,6 @@ decode_gateup_kernel(GateupDecodeArgs a) {
             iq3_tile(sbase + kTileIq3, i_off, s_off, g, grid_c, b0, b1, n0, n1, iu);
             const uint32_t dwa = lds32(sbase + 1664 + 2 * (g & ~1u)), dwb = lds32(sbase + 1664 + 2 * ((g + 8) & ~1u));
             const uint32_t uwa = lds32(sbase + kTileIq3 + 1664 + 2 * (g & ~1u)), uwb = lds32(sbase + kTileIq3 + 1664 + 2 * ((g + 8) & ~1u));
-            __syncwarp();
-            if (lane == 0) issue(stage);
-            ++cnt;
             const uint32_t sh = 16 * (g & 1u);
             // d * 0.25 * (2s+1) * m  ==  d * (0.5 + s) * 0.5 * m
             ga = (f16_bits_to_f32((dwa >> sh) & 0xFFFFu) * 0.25f) * ((float)ig[0] * wcol0 + (float)ig[1] * wcol1);
@@ -381,6 +382,10 @@ decode_gateup_kernel(GateupDecodeArgs a) {
             ua = (f16_bits_to_f32((uwa >> sh) & 0xFFFFu) * 0.25f) * ((float)iu[0] * wcol0 + (float)iu[1] * wcol1);
             ub = (f16_bits_to_f32((uwb >> sh) & 0xFFFFu) * 0.25f) * ((float)iu[2] * wcol0 + (float)iu[3] * wcol1);
             }
+            both_halves();
+            __syncwarp();
+            if (lane == 0) issue(stage);
+            ++cnt;
         } else {
             ga = gb = ua = ub = 0.f;
 #pragma unroll
@@ -390,14 +395,13 @@ decode_gateup_kernel(GateupDecodeArgs a) {
                 const uint32_t sbase = ring + stage * kStageB;
                 q8_quarter(sbase, lane, g, b0[2 * q], b1[2 * q], b0[2 * q + 1], b1[2 * q + 1], wcol0, wcol1, ga, gb);
                 q8_quarter(sbase + dg::kQ8Quarter, lane, g, b0[2 * q], b1[2 * q], b0[2 * q + 1], b1[2 * q + 1], wcol0, wcol1, ua, ub);
+                ub = __shfl_sync(0xFFFFFFFFu, ub, lane);   // (what was read last has come back)
                 __syncwarp();
                 if (lane == 0) issue(stage);
                 ++cnt;
             }
+            both_halves();
         }
-        // the token's other two digits sit in lane t^1
-        ga += __shfl_xor_sync(0xFFFFFFFFu, ga, 1); gb += __shfl_xor_sync(0xFFFFFFFFu, gb, 1);
-        ua += __shfl_xor_sync(0xFFFFFFFFu, ua, 1); ub += __shfl_xor_sync(0xFFFFFFFFu, ub, 1);
         float* my_red = red + (warp * 2 + e_buf) * dg::kRedFloats;
         if ((t & 1u) == 0) {
             const uint32_t ts = t >> 1;   // [tile][row 16][token 2][matrix 2]

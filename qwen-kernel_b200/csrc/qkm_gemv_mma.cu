@@ -183,16 +183,19 @@ gemv_mma_kernel(const __grid_constant__ CUtensorMap tmap, const float* __restric
                     else { q8_block_mma<true>(ca, b0[sb], b1[sb], plane_w, fa0, fa1); q8_block_mma<true>(cb, b0[sb], b1[sb], plane_w, fb0, fb1); }
                     ca = na; cb = nb;
                 }
+                // The two digit-plane pairs of a row sit in lanes t = 0 and t = 1.  (Before the stages are filled again: no read of them is under way
+                // then, which the copies would not wait for.)
+                fa0 += __shfl_xor_sync(0xFFFFFFFFu, fa0, 1); fa1 += __shfl_xor_sync(0xFFFFFFFFu, fa1, 1);
+                fb0 += __shfl_xor_sync(0xFFFFFFFFu, fb0, 1); fb1 += __shfl_xor_sync(0xFFFFFFFFu, fb1, 1);
                 acc[q][0] = fa0; acc[q][1] = fa1;
                 if (two) { acc[q + 1][0] = fb0; acc[q + 1][1] = fb1; }
             }
         }
-        // the two digit-plane pairs of a row sit in lanes t = 0 and t = 1; then the warps' column blocks
+        // then the warps' column blocks
         float* rw = red + (size_t)buf * red_floats + (size_t)warp * gm::kGroup * gm::kRows;
 #pragma unroll
         for (int q = 0; q < gm::kGroup; ++q) {
-            float v0 = acc[q][0], v1 = acc[q][1];
-            v0 += __shfl_xor_sync(0xFFFFFFFFu, v0, 1); v1 += __shfl_xor_sync(0xFFFFFFFFu, v1, 1);
+            const float v0 = acc[q][0], v1 = acc[q][1];
             if (t == 0) { rw[q * gm::kRows + g] = v0; rw[q * gm::kRows + g + 8] = v1; }
         }
         __syncthreads();
