@@ -285,7 +285,7 @@ def run_ours(args, pkg, syn):
     # independent sequences, so ranks are replicas for this workload and no collective is
     # on its data path.  The expert-parallel workloads below shard the experts instead.
     ctx = pkg.Context(dims, n_layer=L, max_tokens=S, device=R.local_rank)
-    stream = torch.cuda.Stream(dev)   # a real stream: the stack is replayed as a CUDA graph
+    stream = torch.cuda.Stream(dev)   # a real stream, as a user's program would have
     ctx.set_stream(stream.cuda_stream)
     layers_keep = []
     x_all = np.empty((L, S, dims.n_embd), np.float32)

@@ -230,8 +230,10 @@ QKM_API int qkm_moe_prefill(qkm_ctx *c, uint32_t layer, const float *x, uint32_t
  * mode 0 = decode path, 1 = prefill path. */
 QKM_API int qkm_moe_forward_host(qkm_ctx *c, uint32_t layer, int mode, const float *x_host,
                                  uint32_t n_tokens, float *y_host);
-/* Decode through layers [0, n_layer) in sequence, feeding each layer the same
- * per-layer input rows x[l] (device [n_layer][T][n_embd]); y likewise. */
+/* Decode through layers [layer_first, layer_first + layer_count), feeding layer l its own
+ * input rows x[l] (device [layer_count][T][n_embd]); y likewise.  The result is that of the
+ * layers in sequence; as every layer's rows are at hand, the layers go through each stage
+ * together, unless x and y overlap without being the same array. */
 QKM_API int qkm_moe_decode_stack(qkm_ctx *c, uint32_t layer_first, uint32_t layer_count,
                                  const float *x, uint32_t n_tokens, float *y);
 /* The same with HOST buffers [layer_count][T][n_embd], then a stream synchronise.  From eight

@@ -60,12 +60,20 @@ struct qkm_ctx {
     uint32_t* n_items = nullptr;      // prefill: units of [0] gate/up, [1] down; [2], [3] their tickets
     uint32_t* status = nullptr;       // kernel status word (device)
     uint32_t* route_counter = nullptr; // ticket counter of the decode router's selection (device, stays zero)
-    // fused decode sequence (router + grouping + planes -> gate/up -> down, three launches)
+    // fused decode sequence (router + grouping + planes -> gate/up -> down, three launches for one or many layers)
     bool dec_ok = false;               // dims fit the fused decode kernels
-    int8_t* planes8 = nullptr;         // [max_tokens][n_embd/256][8][256]
+    int8_t* planes8 = nullptr;         // [min(max_tokens, 64)][n_embd/256][8][256]: of the expert-parallel calls' local tokens
     uint8_t* lut_gu = nullptr;         // table images the decode kernels copy to shared memory
     uint8_t* lut_dd = nullptr;         // table image of the decode IQ4_XS down kernel
-    float* contrib_dec = nullptr;      // [min(max_tokens, 64)][n_used+1][n_embd], for the down kernel that groups by expert
+    // its scratch, for dec_rows (layer, token) rows at a time; the last layer's records and hidden rows go to sel and h
+    uint32_t dec_rows = 0;
+    double* dec_logits = nullptr;      // [row][n_expert]
+    qkm_sel* dec_sel = nullptr;
+    int8_t* dec_planes = nullptr;      // [row][8 n_embd]
+    float *dec_xscale = nullptr, *dec_h = nullptr;        // [row][n_embd/256], [row][n_used+1][n_ff]
+    float* dec_contrib = nullptr;      // [row][n_used+1][n_embd], for the down kernel that groups by expert
+    DecodeGroup* dec_groups = nullptr; // [row][n_used+1]
+    uint32_t* dec_counts = nullptr;    // [kDecMaxLayers]
     uint8_t* lut_pf = nullptr;         // table image of the prefill GEMMs
     uint32_t* status_host = nullptr;  // pinned mirror
     bool shapes_stream_ok = false;
@@ -101,8 +109,7 @@ struct qkm_ctx {
     float* pm_xscale = nullptr;                       // [slot_cap] scales of the local rows sent as f16 (small batches)
     EpPeerTable pm_peers{};
     void* pm_opened[kMaxPeerRanks][3] = {};           // mappings this context opened from handles
-    // the decode stack as CUDA graphs: captured on first use of an argument set, a few sets kept
-    // (the host-buffer form runs the stack in chunks of layers, each its own graph)
+    // decode stacks whose layers do not go together, as CUDA graphs: captured on first use of an argument set, a few sets kept
     static constexpr int kStackGraphs = 8;
     struct StackGraph {
         cudaGraphExec_t exec = nullptr;
@@ -204,6 +211,26 @@ int layer_ready(qkm_ctx* c, uint32_t layer) {
     return QKM_OK;
 }
 
+// Scratch of the fused decode sequence: a stack's layers go through it together, as many as kDecRows (layer, token) rows allow (40 layers of 16
+// tokens, 12 of 64; 113 KB a row for 256 experts, top 8).
+constexpr uint32_t kDecRows = 768;
+cudaError_t alloc_decode(qkm_ctx* c) {
+    const qkm_dims& d = c->cfg.dims;
+    const uint32_t T = c->cfg.max_tokens < 64 ? c->cfg.max_tokens : 64;
+    const uint64_t rows = c->ecount == d.n_expert ? (uint64_t)c->cfg.n_layer * T : 0;
+    c->dec_rows = rows < kDecRows ? (uint32_t)rows : kDecRows;
+    const size_t R = c->dec_rows, S = d.n_used + 1;
+    const bool grouped = decode_down_group_ok(d) && (T >= 40 || !decode_down_any_ok(d));
+    const Want want[] = {
+        {(void**)&c->planes8, (size_t)T * 8 * d.n_embd}, {(void**)&c->lut_gu, decode_gateup_lut_bytes()}, {(void**)&c->lut_dd, decode_down_lut_bytes()},
+        {(void**)&c->dec_logits, R * d.n_expert * sizeof(double)}, {(void**)&c->dec_sel, R * sizeof(qkm_sel)}, {(void**)&c->dec_planes, R * 8 * d.n_embd},
+        {(void**)&c->dec_xscale, R * (d.n_embd / 256) * sizeof(float)}, {(void**)&c->dec_h, R * S * d.n_ff * sizeof(float)},
+        {(void**)&c->dec_contrib, grouped ? R * S * d.n_embd * sizeof(float) : 0}, {(void**)&c->dec_groups, R * S * sizeof(DecodeGroup)},
+        {(void**)&c->dec_counts, kDecMaxLayers * sizeof(uint32_t)},
+    };
+    return dev_alloc_all(want);
+}
+
 }  // namespace
 
 // ---------------------------------------------------------------- lifecycle
@@ -282,18 +309,10 @@ extern "C" QKM_API qkm_ctx* qkm_open(const qkm_config* cfg, char* err, size_t er
         }
         c->dec_ok = decode_gateup_ok(d) && d.n_embd <= 4096;
         if (c->dec_ok) {
-            struct { void** p; size_t bytes; } dec[] = {
-                {(void**)&c->planes8, T * 8 * d.n_embd},
-                {(void**)&c->lut_gu, decode_gateup_lut_bytes()},
-                {(void**)&c->lut_dd, decode_down_lut_bytes()},
-                {(void**)&c->contrib_dec, decode_down_group_ok(d) && (T >= 40 || !decode_down_any_ok(d)) ? (T < 64 ? T : 64) * (d.n_used + 1) * d.n_embd * sizeof(float) : 0},
-            };
-            for (auto& a : dec) {
-                if ((e = cudaMalloc(a.p, a.bytes)) != cudaSuccess) {
-                    bail("qkm_open: cudaMalloc of decode scratch", cudaGetErrorString(e));
-                    qkm_close(c);
-                    return nullptr;
-                }
+            if ((e = alloc_decode(c)) != cudaSuccess) {
+                bail("qkm_open: cudaMalloc of decode scratch", cudaGetErrorString(e));
+                qkm_close(c);
+                return nullptr;
             }
             const Launch L0{nullptr, nullptr};
             if ((e = launch_decode_gateup_luts(L0, c->lut_gu)) != cudaSuccess ||
@@ -307,8 +326,8 @@ extern "C" QKM_API qkm_ctx* qkm_open(const qkm_config* cfg, char* err, size_t er
     }
     if ((e = cudaMalloc((void**)&c->status, sizeof(uint32_t))) != cudaSuccess ||
         (e = cudaMemset(c->status, 0, sizeof(uint32_t))) != cudaSuccess ||
-        (e = cudaMalloc((void**)&c->route_counter, 16 * sizeof(uint32_t))) != cudaSuccess ||
-        (e = cudaMemset(c->route_counter, 0, 16 * sizeof(uint32_t))) != cudaSuccess ||
+        (e = cudaMalloc((void**)&c->route_counter, kDecMaxLayers * kDecCounters * sizeof(uint32_t))) != cudaSuccess ||
+        (e = cudaMemset(c->route_counter, 0, kDecMaxLayers * kDecCounters * sizeof(uint32_t))) != cudaSuccess ||
         (e = cudaMallocHost((void**)&c->status_host, sizeof(uint32_t))) != cudaSuccess) {
         bail("qkm_open: status word", cudaGetErrorString(e));
         qkm_close(c);
@@ -342,7 +361,8 @@ extern "C" QKM_API void qkm_close(qkm_ctx* c) {
     for (auto& dm : c->dense) if (dm.tiles) cudaFree(dm.tiles);
     void* scratch[] = {c->argmax_scratch, c->dense_xb, c->dense_scale, c->sel, c->h, c->route_scratch, c->offsets, c->pairs, c->contrib, c->y2, c->x_stage, c->y_stage,
                        c->stack_x, c->stack_y, c->xscale, c->n_items, c->status, c->route_counter,
-                       c->planes8, c->lut_gu, c->lut_dd, c->contrib_dec, c->lut_pf,
+                       c->planes8, c->lut_gu, c->lut_dd, c->lut_pf, c->dec_logits, c->dec_sel, c->dec_planes, c->dec_xscale, c->dec_h, c->dec_contrib,
+                       c->dec_groups, c->dec_counts,
                        c->xb, c->xnorm, c->hb, c->hscale, c->contrib_p, c->mma_items[0], c->mma_items[1],
                        c->pos_of, c->group_counts, c->ep_counts, c->ep_send_tok, c->ep_send_pos};
     for (void* p : scratch) if (p) cudaFree(p);
@@ -615,38 +635,68 @@ extern "C" QKM_API int qkm_dequant(qkm_ctx* c, uint32_t type, const void* blocks
 
 // ---------------------------------------------------------------- fused layer calls
 
-// Three launches for the whole layer (four from 40 tokens on, where the down kernel that groups by expert is followed by a fold): (1) router logits, selection and digit planes; (2) pair
-// grouping (in every block's shared memory), then gate/up + SwiGLU of the routed experts and of
+// Three launches (four where the down kernel that groups by expert is followed by a fold) for `count` layers of the same types whose rows are at hand
+// together: (1) router logits, selection, the pairs' groups and digit planes; (2) gate/up + SwiGLU of the routed experts and of
 // the shared expert; (3) down projections of both and the weighted sum.  The shared expert rides inside (2)
 // and (3): no side stream, and nothing runs beside the two persistent kernels that they would have to share
-// the SMs with.  At most 64 tokens (the pair grouping's limit).
-static int decode_fused(qkm_ctx* c, const qkm_layer_dev& ld, const float* x, uint32_t n, float* y, qkm_sel* sel, float* h) {
-    const qkm_layer_weights& w = ld.w;
+// the SMs with.  At most 64 tokens (the pair grouping's limit).  Rows of layer first + l at x + l * x_stride and y + l * y_stride; sel and h: where the
+// last layer's go.
+static int decode_fused(qkm_ctx* c, uint32_t first, uint32_t count, const float* x, uint64_t x_stride, uint32_t n, float* y, uint64_t y_stride, qkm_sel* sel, float* h) {
+    const qkm_layer_weights& w = c->layers[first].w;
     const qkm_dims& d = c->cfg.dims;
     const uint32_t nb = (uint32_t)c->n_sms;
+    const DecodeGroups groups{c->dec_counts, c->dec_groups};
     RouteDecodeArgs ra{};
-    ra.router = (const uint8_t*)w.router; ra.gis = w.gate_inp_shexp; ra.x = x; ra.sel = sel;
-    ra.logits = (double*)c->route_scratch; ra.counter = c->route_counter; ra.planes = c->planes8; ra.xscale = c->xscale; ra.n_tokens = n; ra.d = d;
+    GateupDecodeArgs ga{};
+    DownDecodeArgs da{};
+    for (uint32_t l = 0; l < count; ++l) {
+        const qkm_layer_dev& ld = c->layers[first + l];
+        const uint8_t* t[8];
+        for (int i = 0; i < 8; ++i) t[i] = (const uint8_t*)ld.tiles[i];
+        ra.layer[l] = {(const uint8_t*)ld.w.router, ld.w.gate_inp_shexp};
+        ga.layer[l] = {t[2], t[3], t[5], t[6]};
+        da.layer[l] = {t[4], t[7]};
+    }
+    ra.x = x; ra.x_stride = x_stride; ra.sel = c->dec_sel; ra.sel_last = sel; ra.logits = c->dec_logits; ra.counter = c->route_counter;
+    ra.planes = c->dec_planes; ra.xscale = c->dec_xscale; ra.groups = groups; ra.n_tokens = n; ra.n_layers = count; ra.d = d;
     QKM_LAUNCH(c, launch_route_decode(c->Lchain(), w.router_type, ra));
     c->prof_mark("moe.route");
-    GateupDecodeArgs ga{};
-    ga.gate_tiles = (const uint8_t*)ld.tiles[2]; ga.up_tiles = (const uint8_t*)ld.tiles[3];
-    ga.sh_gate_tiles = (const uint8_t*)ld.tiles[5]; ga.sh_up_tiles = (const uint8_t*)ld.tiles[6];
-    ga.luts = c->lut_gu; ga.planes = c->planes8; ga.xscale = c->xscale; ga.sel = sel;
-    ga.n_tokens = n; ga.expert_first = c->efirst; ga.expert_count = c->ecount; ga.with_shared = 1;
-    ga.gateup_type = w.gateup_type;
-    ga.h = h; ga.status = c->status; ga.d = d;
+    ga.luts = c->lut_gu; ga.planes = c->dec_planes; ga.xscale = c->dec_xscale; ga.groups = groups; ga.n_tokens = n; ga.n_layers = count;
+    ga.gateup_type = w.gateup_type; ga.h = c->dec_h; ga.h_last = h; ga.status = c->status; ga.d = d;
     QKM_LAUNCH(c, launch_decode_gateup(c->Lchain(), ga, nb));
     c->prof_mark("moe.gu");
-    DownDecodeArgs da{};
-    da.tiles = (const uint8_t*)ld.tiles[4]; da.sh_tiles = (const uint8_t*)ld.tiles[7]; da.lut = c->lut_dd;
-    da.h = h; da.sel = sel; da.y = y; da.n_tokens = n; da.status = c->status; da.d = d;
-    da.contrib = c->contrib_dec;
-    if (c->contrib_dec && decode_down_group_better(d, w.down_type, n)) QKM_LAUNCH(c, launch_decode_down_group(c->Lchain(), da, w.down_type, nb));
+    da.lut = c->lut_dd; da.h = c->dec_h; da.h_last = h; da.sel = c->dec_sel; da.sel_last = sel; da.y = y; da.y_stride = y_stride;
+    da.groups = groups; da.contrib = c->dec_contrib; da.n_tokens = n; da.n_layers = count; da.status = c->status; da.d = d;
+    if (c->dec_contrib && decode_down_group_better(d, w.down_type, n)) QKM_LAUNCH(c, launch_decode_down_group(c->Lchain(), da, w.down_type, nb));
     else if (!decode_down_ok(d)) QKM_LAUNCH(c, launch_decode_down_any(c->Lchain(), da, w.down_type, nb));
     else if (w.down_type == QKM_TYPE_IQ4_XS) QKM_LAUNCH(c, launch_decode_down(c->Lchain(), da, nb));
     else QKM_LAUNCH(c, launch_decode_down_q6k(c->Lchain(), da, nb));
     c->prof_mark("moe.dn");
+    return QKM_OK;
+}
+
+// The fused sequence's limits; the tensors' are in qkm_layer_dev::fused_ok.
+static bool decode_fused_ok(const qkm_ctx* c, uint32_t n) {
+    const qkm_dims& d = c->cfg.dims;
+    return n && c->dec_ok && c->dec_rows && route_decode_ok(d, n < 64 ? n : 64, c->route_scratch_bytes) && (decode_down_ok(d) || decode_down_any_ok(d) || c->dec_contrib);
+}
+
+// Layers [first, first + count), all ready for the fused sequence, at most 64 tokens at a time: in runs of the same types, as many layers at once
+// as the scratch holds.
+static int decode_layers(qkm_ctx* c, uint32_t first, uint32_t count, const float* x, uint64_t x_stride, uint32_t n, float* y, uint64_t y_stride) {
+    const qkm_dims& d = c->cfg.dims;
+    for (uint32_t t = 0; t < n; t += 64) {
+        const uint32_t nt = n - t < 64 ? n - t : 64, most = c->dec_rows / nt < kDecMaxLayers ? c->dec_rows / nt : kDecMaxLayers;
+        for (uint32_t l = 0, k = 1; l < count; l += k, k = 1) {
+            const qkm_layer_weights& w = c->layers[first + l].w;
+            for (; l + k < count && k < most; ++k) {
+                const qkm_layer_weights& v = c->layers[first + l + k].w;
+                if (v.router_type != w.router_type || v.gateup_type != w.gateup_type || v.down_type != w.down_type) break;
+            }
+            if (int rc = decode_fused(c, first + l, k, x + l * x_stride + (size_t)t * d.n_embd, x_stride, nt, y + l * y_stride + (size_t)t * d.n_embd, y_stride,
+                                      c->sel + t, c->h + (size_t)t * (d.n_used + 1) * d.n_ff)) return rc;
+        }
+    }
     return QKM_OK;
 }
 
@@ -658,13 +708,7 @@ extern "C" QKM_API int qkm_moe_decode(qkm_ctx* c, uint32_t layer, const float* x
     const qkm_layer_weights& w = ld.w;
     const qkm_dims& d = c->cfg.dims;
     c->prof_begin();
-    constexpr uint32_t kMost = 64;
-    if (n && ld.fused_ok && c->dec_ok && route_decode_ok(d, n < kMost ? n : kMost, c->route_scratch_bytes) && (decode_down_ok(d) || decode_down_any_ok(d) || c->contrib_dec)) {
-        for (uint32_t t = 0; t < n; t += kMost)
-            if (int rc = decode_fused(c, ld, x + (size_t)t * d.n_embd, n - t < kMost ? n - t : kMost, y + (size_t)t * d.n_embd, c->sel + t,
-                                      c->h + (size_t)t * (d.n_used + 1) * d.n_ff)) return rc;
-        return QKM_OK;
-    }
+    if (ld.fused_ok && decode_fused_ok(c, n)) return decode_layers(c, layer, 1, x, 0, n, y, 0);
     // generic kernels on the raw layout
     QKM_LAUNCH(c, launch_route_select(c->L(), d, w.router_type, w.router, w.gate_inp_shexp, x, c->sel, n, c->route_scratch, c->route_scratch_bytes));
     c->prof_mark("moe.route");
@@ -798,10 +842,11 @@ static int decode_stack_eager(qkm_ctx* c, uint32_t first, uint32_t count, const 
     return QKM_OK;
 }
 
-// The per-layer launches of the stack are captured into a CUDA graph the first time an
-// argument set is seen and replayed afterwards (a launch-bound inner loop: each layer is a
-// handful of short kernels).  Capture needs a real stream: on the legacy default stream,
-// while profiling, or after an upload, the launches are issued one by one.
+// Layers of the fused sequence go through each of its stages together: three or four launches for the stack, not for a layer (40 layers of
+// 16 tokens 2,740 us as a graph of their launches, 1,920 together; 24 layers of one token 560 and 124).  What is left - an output that
+// overlaps a later layer's input, a layer outside the fused sequence - goes layer by layer: the launches are captured into a CUDA graph the
+// first time an argument set is seen and replayed afterwards.  Capture needs a real stream: on the legacy default stream, while
+// profiling, or after an upload, the launches are issued one by one.
 extern "C" QKM_API int qkm_moe_decode_stack(qkm_ctx* c, uint32_t first, uint32_t count, const float* x,
                                             uint32_t n, float* y) {
     if (!c || !x || !y) return QKM_ERR_ARG;
@@ -809,6 +854,12 @@ extern "C" QKM_API int qkm_moe_decode_stack(qkm_ctx* c, uint32_t first, uint32_t
     if (int rc = check_tokens(c, n)) return rc;
     for (uint32_t l = 0; l < count; ++l)
         if (int rc = layer_ready(c, first + l)) return rc;
+    // every layer's rows are at hand: the layers go through each stage together, unless an output overlaps a later layer's input
+    const qkm_dims& d = c->cfg.dims;
+    const uint64_t stride = (uint64_t)n * d.n_embd, xa = (uint64_t)(uintptr_t)x, ya = (uint64_t)(uintptr_t)y, bytes = count * stride * sizeof(float);
+    bool together = !c->profiling && decode_fused_ok(c, n) && (xa == ya || xa + bytes <= ya || ya + bytes <= xa);
+    for (uint32_t l = 0; l < count && together; ++l) together = c->layers[first + l].fused_ok;
+    if (together) return decode_layers(c, first, count, x, stride, n, y, stride);
     if (c->stream == nullptr || c->profiling || count < 2) return decode_stack_eager(c, first, count, x, n, y);
     qkm_ctx::StackGraph* g = nullptr;
     for (auto& e : c->stack_graphs)
@@ -1151,12 +1202,13 @@ extern "C" QKM_API int qkm_ep_shared(qkm_ctx* c, uint32_t layer, const float* x,
     }
     if (dec) {   // the decode kernels without routed experts (digit planes written by qkm_ep_dispatch)
         GateupDecodeArgs ga{};
-        ga.sh_gate_tiles = (const uint8_t*)ld.tiles[5]; ga.sh_up_tiles = (const uint8_t*)ld.tiles[6];
-        ga.luts = c->lut_gu; ga.planes = c->planes8; ga.xscale = c->xscale; ga.sel = c->sel;
-        ga.n_tokens = n; ga.with_shared = 1; ga.gateup_type = w.gateup_type; ga.h = c->h; ga.status = c->status; ga.d = d;
+        ga.layer[0] = {nullptr, nullptr, (const uint8_t*)ld.tiles[5], (const uint8_t*)ld.tiles[6]};   // no groups: the shared expert's only
+        ga.luts = c->lut_gu; ga.planes = c->planes8; ga.xscale = c->xscale; ga.n_tokens = n; ga.n_layers = 1; ga.gateup_type = w.gateup_type;
+        ga.h_last = c->h; ga.status = c->status; ga.d = d;
         QKM_LAUNCH(c, launch_decode_gateup(c->L(), ga, (uint32_t)c->n_sms));
         DownDecodeArgs da{};
-        da.sh_tiles = (const uint8_t*)ld.tiles[7]; da.h = c->h; da.sel = c->sel; da.y = c->y2; da.n_tokens = n; da.status = c->status; da.d = d;
+        da.layer[0] = {nullptr, (const uint8_t*)ld.tiles[7]};
+        da.h_last = c->h; da.sel_last = c->sel; da.y = c->y2; da.n_tokens = n; da.n_layers = 1; da.status = c->status; da.d = d;
         QKM_LAUNCH(c, launch_decode_down_any(c->L(), da, w.down_type, (uint32_t)c->n_sms));
         return QKM_OK;
     }

@@ -35,7 +35,7 @@ static_assert(Cfg<true>::kDyn <= 231000 && Cfg<false>::kDyn <= 231000, "with the
 
 template <bool Q6>
 __global__ void __launch_bounds__(da::kMaxWarps * 32, 1)
-decode_down_any_kernel(DownDecodeArgs a) {
+decode_down_any_kernel(const __grid_constant__ DownDecodeArgs a) {
     using C = da::Cfg<Q6>;
     extern __shared__ __align__(128) uint8_t smem_raw[];
     __shared__ __align__(8) unsigned long long s_bar[da::kMaxWarps * C::kStages + 1];
@@ -44,7 +44,7 @@ decode_down_any_kernel(DownDecodeArgs a) {
     const uint32_t n_slots = d.n_used + 1, n_warps = blockDim.x >> 5;
     constexpr uint32_t KB = 2;   // n_ff = 512
     const uint32_t RT = d.n_embd / 16, slot = warp / KB, kb = warp - slot * KB;
-    const bool has_tile = a.tiles != nullptr && slot < d.n_used, has_sh = a.sh_tiles != nullptr && warp < d.n_ff / 32;
+    const bool has_tile = a.layer[0].w != nullptr && slot < d.n_used, has_sh = a.layer[0].sh != nullptr && warp < d.n_ff / 32;
     const uint32_t win0 = smem_addr(smem_raw), base = Q6 ? (win0 + 127u) & ~127u : 0u;
     if (!Q6) {   // the fixed addresses must lie inside the dynamic area
         uint32_t dyn_size;
@@ -72,7 +72,7 @@ decode_down_any_kernel(DownDecodeArgs a) {
         for (uint32_t i = 0; i < 4; ++i) bulk_g2s(da::kTab + i * 16384u, a.lut + i * 16384u, 16384u, bar_tab);
     }
 
-    const uint64_t tiles_total = (uint64_t)a.n_tokens * RT;
+    const uint64_t tiles_total = (uint64_t)a.n_layers * a.n_tokens * RT;   // units: (layer, token, tile)
     const uint32_t u_lo = (uint32_t)(tiles_total * blockIdx.x / gridDim.x), u_hi = (uint32_t)(tiles_total * (blockIdx.x + 1) / gridDim.x);
 
     // producer cursor; lane 0 only
@@ -83,8 +83,9 @@ decode_down_any_kernel(DownDecodeArgs a) {
         if (p_u >= u_hi || timed_out || !(has_tile || has_sh)) return;
         if (p_new_tok) {
             p_new_tok = false;
-            if (has_tile) p_src = a.tiles + (((size_t)min(__ldcg(&a.sel[p_tok].ids[slot]), d.n_expert - 1) * KB + kb) * RT + p_rt) * C::kTile;
-            if (has_sh) p_sh = a.sh_tiles + ((size_t)(warp >> 3) * RT + p_rt) * kTileQ8 + da::kShBlock * (warp & 7u);
+            const uint32_t l = layer_of(a, p_tok);
+            if (has_tile) p_src = a.layer[l].w + (((size_t)min(__ldcg(&layer_sel(a, l)[p_tok - l * a.n_tokens].ids[slot]), d.n_expert - 1) * KB + kb) * RT + p_rt) * C::kTile;
+            if (has_sh) p_sh = a.layer[l].sh + ((size_t)(warp >> 3) * RT + p_rt) * kTileQ8 + da::kShBlock * (warp & 7u);
         }
         const uint32_t bar = my_bar + 8 * stage, dst = ring + stage * C::kStage;
         mbar_expect_tx(bar, (has_tile ? C::kTile : 0) + (has_sh ? da::kShBlock : 0));
@@ -113,11 +114,16 @@ decode_down_any_kernel(DownDecodeArgs a) {
 
     uint32_t tok = u_lo / RT, rt = u_lo - tok * RT;
     bool new_tok = true;
+    float* y = nullptr;            // the token's output row
     for (uint32_t u = u_lo; u < u_hi;) {
         if (new_tok) {   // block-uniform
             new_tok = false;
+            const uint32_t l = layer_of(a, tok), lt = tok - l * a.n_tokens;   // layer, token of the layer
+            const float* h = layer_h(a, l) + (size_t)lt * n_slots * d.n_ff;
+            const qkm_sel* rec = layer_sel(a, l) + lt;
+            y = a.y + l * a.y_stride + (size_t)lt * d.n_embd;
             if (has_tile) {   // 256 values of h[tok][slot] as digits (28-bit fixed point relative to their largest)
-                const float* hs = a.h + ((size_t)tok * n_slots + slot) * d.n_ff + 256 * kb + 8 * lane;
+                const float* hs = h + slot * d.n_ff + 256 * kb + 8 * lane;
                 const float4 v0 = *reinterpret_cast<const float4*>(hs), v1 = *reinterpret_cast<const float4*>(hs + 4);
                 const float hv[8] = {v0.x, v0.y, v0.z, v0.w, v1.x, v1.y, v1.z, v1.w};
                 float m = 0.f;
@@ -152,10 +158,10 @@ decode_down_any_kernel(DownDecodeArgs a) {
                         b1[j] = g < 4 ? v.y : 0u;
                     }
                 }
-                w_s = a.sel[tok].w[slot] * (any_bad ? __int_as_float(0x7FC00000) : ldexpf(Q6 ? 0.25f : 1.0f, -p));
+                w_s = rec->w[slot] * (any_bad ? __int_as_float(0x7FC00000) : ldexpf(Q6 ? 0.25f : 1.0f, -p));
             }
             if (has_sh) {   // 32 values of the shared row, one a lane; digit g of elements 4t.. and 16 + 4t.. by shuffles
-                const float hv = a.h[((size_t)tok * n_slots + d.n_used) * d.n_ff + 32 * warp + lane];
+                const float hv = h[d.n_used * d.n_ff + 32 * warp + lane];
                 const bool any_bad = __any_sync(0xFFFFFFFFu, !(fabsf(hv) <= 3.0e38f));
                 const float m = __uint_as_float(__reduce_max_sync(0xFFFFFFFFu, __float_as_uint(fabsf(hv))));
                 const int p = any_bad ? 0 : digit_exponent(m);
@@ -166,7 +172,7 @@ decode_down_any_kernel(DownDecodeArgs a) {
                 const uint32_t sel = 0x4040u + 0x1111u * (g & 3u);
                 hb0 = g < 4 ? prmt_dec(prmt_dec(e[0], e[1], sel), prmt_dec(e[2], e[3], sel), 0x5410u) : 0u;
                 hb1 = g < 4 ? prmt_dec(prmt_dec(e[4], e[5], sel), prmt_dec(e[6], e[7], sel), 0x5410u) : 0u;
-                w_sh = a.sel[tok].w_shared * (any_bad ? __int_as_float(0x7FC00000) : ldexpf(1.0f, -p));
+                w_sh = rec->w_shared * (any_bad ? __int_as_float(0x7FC00000) : ldexpf(1.0f, -p));
             }
         }
         const uint32_t n_c = min((uint32_t)da::kChunk, min(u_hi - u, RT - rt));   // tiles of this chunk
@@ -256,7 +262,7 @@ decode_down_any_kernel(DownDecodeArgs a) {
             float sum = 0.f;
             for (uint32_t w = 0; w < n_warps; w += 2)   // slot order; a slot's two column blocks first (half as many roundings in a chain)
                 sum += red[((buf * da::kMaxWarps + w) * da::kChunk + i) * 16 + r] + red[((buf * da::kMaxWarps + w + 1) * da::kChunk + i) * 16 + r];
-            a.y[(size_t)tok * d.n_embd + (rt + i) * 16 + r] = sum;
+            y[(rt + i) * 16 + r] = sum;
         }
         buf ^= 1u;
         u += n_c;
@@ -285,7 +291,7 @@ static cudaError_t any_launch(const Launch& L, const DownDecodeArgs& a, uint32_t
 cudaError_t launch_decode_down_any(const Launch& L, const DownDecodeArgs& a, uint32_t type, uint32_t n_blocks) {
     if (!decode_down_any_ok(a.d)) return cudaErrorInvalidValue;
     if (a.n_tokens == 0) return cudaSuccess;
-    if (type == QKM_TYPE_Q6_K || a.tiles == nullptr) return any_launch<true>(L, a, n_blocks);
+    if (type == QKM_TYPE_Q6_K || a.layer[0].w == nullptr) return any_launch<true>(L, a, n_blocks);
     if (type != QKM_TYPE_IQ4_XS || !a.lut) return cudaErrorInvalidValue;
     return any_launch<false>(L, a, n_blocks);
 }

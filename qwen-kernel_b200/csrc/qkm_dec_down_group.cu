@@ -5,7 +5,7 @@
 // Replaces moe_down_iq4.comp / moe_down_q6k.comp + moe_down_q8b.comp and the slot-order sum of add_rms3_grouped.comp:22-27.
 //
 // The token-major kernels unpack an expert's weights once for every token that chose it.  Here the pairs are grouped by expert as in
-// the gate/up kernel (qkm_dec_rank.cuh, in every block's shared memory), a group is an expert with up to two of its tokens, and a
+// the gate/up kernel (the router kernel's lists, over all layers of the call), a group is an expert with up to two of its tokens, and a
 // team of two warps (one per 256 columns) walks 16-row tiles of a contiguous share of the (group, tile) list: at 64 tokens of 256 experts,
 // top 8, 317 groups instead of 512 pairs.  The price is the grouping, the contribution rows' way through the L2 and a second
 // launch, about 7 us together.
@@ -38,8 +38,7 @@ template <bool Q6> struct Cfg {
     static constexpr uint32_t kLow = 9;                                                   // IQ4_XS: rings below the table, up against it; the others above
     static constexpr uint32_t kScratch = Q6 ? kWarps * kRing : kHigh + (kWarps - kLow) * kRing;   // Q6_K: from the aligned start
     static constexpr uint32_t kRed = kScratch + kWarps * 1024;                            // digits of a warp's 256 columns, one token at a time
-    static constexpr uint32_t kRank = kRed + kWarps * 2 * kGroupTiles * 16 * 2 * 4;       // [warp][buffer][tile][row][token]
-    static constexpr uint32_t kEnd = kRank + (sizeof(RankShared) + 127) / 128 * 128;
+    static constexpr uint32_t kEnd = kRed + kWarps * 2 * kGroupTiles * 16 * 2 * 4;        // [warp][buffer][tile][row][token]
     static constexpr uint32_t kDyn = Q6 ? kEnd + 128 : kEnd - 1024;                       // the first KB of the window is the system's
 };
 static_assert(Cfg<true>::kDyn <= 231000 && Cfg<false>::kDyn <= 231000 && kHalfQ8 <= kTileIq4, "with the static part at most 227 KB");
@@ -47,10 +46,11 @@ static_assert(Cfg<true>::kDyn <= 231000 && Cfg<false>::kDyn <= 231000 && kHalfQ8
 
 template <bool Q6>
 __global__ void __launch_bounds__(dp::kWarps * 32, 1)
-decode_down_group_kernel(DownDecodeArgs a) {
+decode_down_group_kernel(const __grid_constant__ DownDecodeArgs a) {
     using C = dp::Cfg<Q6>;
     extern __shared__ __align__(128) uint8_t smem_raw[];
     __shared__ __align__(8) unsigned long long s_bar[dp::kWarps * dp::kStages + 1];
+    __shared__ LayerCuts s_cuts;
     const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31u, g = lane >> 2, t = lane & 3u;
     const qkm_dims d = a.d;
     const uint32_t n_slots = d.n_used + 1, KB = 2, RT = d.n_embd / 16;
@@ -68,7 +68,6 @@ decode_down_group_kernel(DownDecodeArgs a) {
     const uint32_t my_dig = base + C::kScratch + warp * 1024;
     uint8_t* dig = smem_raw + (my_dig - win0);
     float* red = reinterpret_cast<float*>(smem_raw + (base + C::kRed - win0));
-    RankShared& S = *reinterpret_cast<RankShared*>(smem_raw + (base + C::kRank - win0));
     const uint32_t my_bar = smem_addr(&s_bar[warp * dp::kStages]), bar_tab = smem_addr(&s_bar[dp::kWarps * dp::kStages]);
     bool timed_out = false;
 
@@ -82,24 +81,30 @@ decode_down_group_kernel(DownDecodeArgs a) {
         mbar_expect_tx(bar_tab, dp::kTabBytes);
         for (uint32_t i = 0; i < 4; ++i) bulk_g2s(dp::kTab + i * 16384u, a.lut + i * 16384u, 16384u, bar_tab);
     }
-    // the selection was final before the gate/up kernel released this one
-    group_pairs_shared(S, a.sel, d, a.n_tokens, 0, d.n_expert, true, dp::kWarps);
+    const uint32_t teams_total = gridDim.x * n_teams, team_global = blockIdx.x * n_teams + team;
+    const Divisor by_teams(teams_total), by_tiles(RT);
 
-    const uint32_t tiles_total = S.n_groups * RT, teams_total = gridDim.x * n_teams, team_global = blockIdx.x * n_teams + team;
-    const uint32_t t_lo = (uint32_t)((uint64_t)tiles_total * team_global / teams_total), t_hi = (uint32_t)((uint64_t)tiles_total * (team_global + 1) / teams_total);
+    // the selection and its groups were final before the gate/up kernel released this one
+    if (warp == 0) layer_cuts(s_cuts, a.groups, a.n_tokens, a.n_layers, 1, 1);
+    __syncthreads();
+    uint32_t left;   // tiles still to do
+    ListPlace at = list_share(s_cuts, a.n_tokens, a.n_layers, by_tiles, 1, 1, team_global, by_teams, left);
+    auto group = [&](const ListPlace& p) { return decode_group(a.groups, a.n_tokens, d.n_used, p.l, p.gi); };
     const size_t mat_tiles = (size_t)KB * RT;
 
     // producer cursor; lane 0 only.  A routed tile is one stage, a shared tile two.
-    uint32_t p_tile = t_lo, p_half = 0, p_rt = RT, p_gi = t_lo / RT;   // p_rt == RT: the group record must be (re)loaded
+    uint32_t p_left = left, p_half = 0;
+    ListPlace p_at = at;
+    bool p_new = true;                     // the group record must be (re)loaded
     const uint8_t* p_src = nullptr;
     bool p_shared = false;
     auto issue = [&](uint32_t stage) {
-        if (p_tile >= t_hi || timed_out) return;
-        if (p_rt >= RT) {
-            p_rt = p_tile - p_gi * RT;
-            const DecodeGroup r = S.groups[p_gi];
-            p_shared = r.kind != 0;
-            p_src = p_shared ? a.sh_tiles + ((size_t)kb * RT + p_rt) * kTileQ8 : a.tiles + ((size_t)r.expert * mat_tiles + (size_t)kb * RT + p_rt) * C::kTile;
+        if (p_left == 0 || timed_out) return;
+        if (p_new) {
+            p_new = false;
+            const DecodeGroup r = group(p_at);
+            p_shared = r.shared();
+            p_src = p_shared ? a.layer[p_at.l].sh + ((size_t)kb * RT + p_at.rt) * kTileQ8 : a.layer[p_at.l].w + ((size_t)r.expert() * mat_tiles + (size_t)kb * RT + p_at.rt) * C::kTile;
         }
         const uint32_t n = p_shared ? dp::kHalfQ8 : C::kTile;
         mbar_expect_tx(my_bar + 8 * stage, n);
@@ -107,8 +112,8 @@ decode_down_group_kernel(DownDecodeArgs a) {
         p_src += n;
         if (p_shared && !p_half) { p_half = 1; return; }
         p_half = 0;
-        ++p_tile;
-        if (++p_rt >= RT) ++p_gi;
+        --p_left;
+        if (++p_at.rt == RT) { p_at.rt = 0; p_at.next_group(s_cuts); p_new = true; }
     };
     if (lane == 0)
         for (uint32_t s = 0; s < dp::kStages; ++s) issue(s);
@@ -117,10 +122,10 @@ decode_down_group_kernel(DownDecodeArgs a) {
     if (!Q6 && !mbar_wait_bounded(bar_tab, 0)) timed_out = true;   // every thread observes the table's arrival itself
 
     const uint32_t i_off = 64 * g + piece_at(g, t), tab_c = dp::kTab + lane * 4;
-    uint32_t stage = 0, phase = 0, e_first = 0, e_n = 0, e_buf = 0;   // tiles waiting for the team's sum: first rt, count, buffer
-    uint32_t gi = t_lo / RT, rt = t_lo - gi * RT;
+    uint32_t stage = 0, phase = 0, e_n = 0, e_buf = 0;   // tiles waiting for the team's sum (the last e_n up to at.rt): count, buffer
     bool new_group = true, live = false;
-    DecodeGroup rec{};
+    DecodeGroup rec{}, rec_next{};
+    if (left) rec_next = group(at);   // a group's record is read while the group before is worked on
     size_t out = 0;                          // where this thread's sums of the current group go: (token, slot) of token slot lt & 1
     constexpr int NB = Q6 ? 2 : 1;
     uint32_t b0[NB][8], b1[NB][8];           // B operands (Q6_K: per token)
@@ -130,24 +135,29 @@ decode_down_group_kernel(DownDecodeArgs a) {
         if (lane == 0) issue(stage);
         if (++stage == dp::kStages) { stage = 0; phase ^= 1u; }
     };
-    for (uint32_t tile = t_lo; tile < t_hi; ++tile) {
+    for (; left; --left) {
         if (new_group) {
             new_group = false;
-            rec = S.groups[gi];
-            const bool shared = rec.kind != 0;
-            live = (lt & 1u) < rec.ntok;
+            rec = rec_next;
+            ListPlace after = at;
+            after.next_group(s_cuts);
+            if (after.l < a.n_layers) rec_next = group(after);
+            const bool shared = rec.shared();
+            const float* h = layer_h(a, at.l);
+            const qkm_sel* sel = layer_sel(a, at.l);
+            live = (lt & 1u) < rec.ntok();
             if (live) {
-                const uint32_t pr = S.pairs[rec.pair_off + (lt & 1u)];
-                out = ((size_t)(pr >> 4) * n_slots + (pr & 15u)) * d.n_embd;
+                const uint32_t pr = rec.pair_of(lt & 1u);
+                out = ((size_t)(at.l * a.n_tokens + (pr >> 4)) * n_slots + (pr & 15u)) * d.n_embd;
             }
             float wt[2] = {0.f, 0.f};        // routing weight x plane scale
             float4 hv4[2][2];
 #pragma unroll
             for (int ts = 0; ts < 2; ++ts) {
-                const uint32_t pr = S.pairs[rec.pair_off + min((uint32_t)ts, rec.ntok - 1u)], tok = pr >> 4, slot = pr & 15u;
-                const float* hs = a.h + ((size_t)tok * n_slots + slot) * d.n_ff + 256 * kb + 8 * lane;
+                const uint32_t pr = rec.pair_of((uint32_t)ts < rec.ntok() ? ts : 0), tok = pr >> 4, slot = pr & 15u;
+                const float* hs = h + ((size_t)tok * n_slots + slot) * d.n_ff + 256 * kb + 8 * lane;
                 hv4[ts][0] = *reinterpret_cast<const float4*>(hs); hv4[ts][1] = *reinterpret_cast<const float4*>(hs + 4);
-                if ((uint32_t)ts < rec.ntok) wt[ts] = slot < d.n_used ? a.sel[tok].w[slot] : a.sel[tok].w_shared;
+                if ((uint32_t)ts < rec.ntok()) wt[ts] = slot < d.n_used ? sel[tok].w[slot] : sel[tok].w_shared;
             }
 #pragma unroll
             for (int ts = 0; ts < 2; ++ts) {
@@ -157,7 +167,7 @@ decode_down_group_kernel(DownDecodeArgs a) {
 #pragma unroll
                 for (int i = 0; i < 8; ++i) { m = fmaxf(m, fabsf(hv[i])); bad |= !(fabsf(hv[i]) <= 3.0e38f); }
                 m = __uint_as_float(__reduce_max_sync(0xFFFFFFFFu, __float_as_uint(m)));   // non-negative floats order like their bits
-                const bool any_bad = __any_sync(0xFFFFFFFFu, bad), off = (uint32_t)ts >= rec.ntok;
+                const bool any_bad = __any_sync(0xFFFFFFFFu, bad), off = (uint32_t)ts >= rec.ntok();
                 const int p = any_bad ? 0 : digit_exponent(m);
                 const float up = ldexpf(1.0f, p);
                 uint32_t dg[8];
@@ -193,9 +203,8 @@ decode_down_group_kernel(DownDecodeArgs a) {
                 w1 = w0 * 128.f;
             }
         }
-        if (e_n == 0) e_first = rt;
         float va = 0.f, vb = 0.f, va1 = 0.f, vb1 = 0.f;   // rows g, g + 8 (Q6_K tiles: of tokens 0 and 1)
-        if (rec.kind == 0) {
+        if (!rec.shared()) {
             if (!mbar_wait_bounded(my_bar + 8 * stage, phase)) timed_out = true;
             const uint32_t tb = ring + stage * C::kTile;
             if (Q6) {
@@ -280,45 +289,45 @@ decode_down_group_kernel(DownDecodeArgs a) {
         // the token's other two digits sit in lane t^1
         // (before the stage is filled again: no read of it is under way then, which the copy would not wait for)
         va += __shfl_xor_sync(0xFFFFFFFFu, va, 1); vb += __shfl_xor_sync(0xFFFFFFFFu, vb, 1);
-        if (rec.kind == 0) next();
+        if (!rec.shared()) next();
         if ((t & 1u) == 0) {
             float* r = red + ((warp * 2 + e_buf) * dp::kGroupTiles + e_n) * 32 + (t >> 1);
             r[2 * g] = va; r[2 * (g + 8)] = vb;
         }
         ++e_n;
-        if (e_n == dp::kGroupTiles || rt + 1 == RT || tile + 1 == t_hi) {
+        if (e_n == dp::kGroupTiles || at.rt + 1 == RT || left == 1) {
             // team-wide: add the column blocks, store.  The scratch is double buffered: one barrier a sum
             asm volatile("bar.sync %0, %1;" ::"r"(team + 1), "r"(team_threads) : "memory");
             for (uint32_t j = lt; j < e_n * 32; j += team_threads)   // team_threads is even: j & 1 == lt & 1
                 if (live) {
                     float v = 0.f;
                     for (uint32_t w = 0; w < KB; ++w) v += red[((team * KB + w) * 2 + e_buf) * dp::kGroupTiles * 32 + j];
-                    a.contrib[out + (size_t)e_first * 16 + (j >> 1)] = v;
+                    a.contrib[out + (size_t)(at.rt + 1 - e_n) * 16 + (j >> 1)] = v;
                 }
             e_n = 0;
             e_buf ^= 1u;
         }
-        if (++rt == RT) { rt = 0; ++gi; new_group = true; }
+        if (++at.rt == RT) { at.rt = 0; at.next_group(s_cuts); new_group = true; }
     }
     if (timed_out && lane == 0) atomicExch(a.status, (uint32_t)kStatusWaitTimeout);
 }
 
-// y[t] = the contributions' sum in slot order
+// y[layer][t] = the contributions' sum in slot order
 __global__ void __launch_bounds__(256)
-decode_fold_kernel(const float* contrib, float* y, uint32_t n_slots, uint32_t n_embd, uint32_t n) {
+decode_fold_kernel(const float* contrib, float* y, uint64_t y_stride, uint32_t n_slots, uint32_t n_embd, uint32_t n_tokens, uint32_t n) {
     const uint32_t i = blockIdx.x * 256 + threadIdx.x, n4 = n_embd / 4;   // a float4 of y each
     pdl_trigger();
     pdl_wait();
     if (i >= n) return;
-    const uint32_t t = i / n4, o = i - t * n4;
-    const float4* c = reinterpret_cast<const float4*>(contrib) + (size_t)t * n_slots * n4 + o;
+    const uint32_t row = i / n4, o = i - row * n4, l = row / n_tokens, t = row - l * n_tokens;
+    const float4* c = reinterpret_cast<const float4*>(contrib) + (size_t)row * n_slots * n4 + o;
     float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll 4
     for (uint32_t s = 0; s < n_slots; ++s) {
         const float4 q = __ldcg(c + (size_t)s * n4);
         v.x += q.x; v.y += q.y; v.z += q.z; v.w += q.w;
     }
-    reinterpret_cast<float4*>(y)[i] = v;
+    reinterpret_cast<float4*>(y + l * y_stride)[(size_t)t * n4 + o] = v;
 }
 
 // IQ4_XS: from 40 tokens on for every expert count and number of slots that was measured (some cross over at 12 to 37); Q6_K: only
@@ -336,13 +345,13 @@ static cudaError_t group_launch(const Launch& L, const DownDecodeArgs& a, uint32
     const size_t smem = dp::Cfg<Q6>::kDyn;
     if (const cudaError_t e = allow_dynamic_smem<decode_down_group_kernel<Q6>>((int)smem)) return e;
     if (const cudaError_t e = launch_kernel(L, decode_down_group_kernel<Q6>, dim3(n_blocks), dim3(dp::kWarps * 32), smem, a)) return e;
-    const uint32_t n = a.n_tokens * (a.d.n_embd / 4);
-    const cudaError_t e = launch_kernel(L, decode_fold_kernel, dim3((n + 255) / 256), dim3(256), 0, (const float*)a.contrib, a.y, a.d.n_used + 1, a.d.n_embd, n);
+    const uint32_t n = a.n_layers * a.n_tokens * (a.d.n_embd / 4);
+    const cudaError_t e = launch_kernel(L, decode_fold_kernel, dim3((n + 255) / 256), dim3(256), 0, (const float*)a.contrib, a.y, a.y_stride, a.d.n_used + 1, a.d.n_embd, a.n_tokens, n);
     L.count(2);
     return e != cudaSuccess ? e : cudaGetLastError();
 }
 cudaError_t launch_decode_down_group(const Launch& L, const DownDecodeArgs& a, uint32_t type, uint32_t n_blocks) {
-    if (!decode_down_group_ok(a.d) || !a.contrib || !a.tiles || !a.sh_tiles || a.n_tokens > rk::kMaxTokens) return cudaErrorInvalidValue;
+    if (!decode_down_group_ok(a.d) || !a.contrib || !a.groups.group || a.n_tokens > rk::kMaxTokens) return cudaErrorInvalidValue;
     if (a.n_tokens == 0) return cudaSuccess;
     if (type == QKM_TYPE_Q6_K) return group_launch<true>(L, a, n_blocks);
     if (type != QKM_TYPE_IQ4_XS || !a.lut) return cudaErrorInvalidValue;

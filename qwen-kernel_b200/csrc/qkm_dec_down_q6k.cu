@@ -48,7 +48,7 @@ constexpr uint32_t kEnd = kMisc + 128;
 }  // namespace dq
 
 __global__ void __launch_bounds__(dq::kWarps * 32, 1)
-decode_down_q6k_kernel(DownDecodeArgs a) {
+decode_down_q6k_kernel(const __grid_constant__ DownDecodeArgs a) {
     extern __shared__ __align__(128) uint8_t smem_raw[];
     uint8_t* sm = reinterpret_cast<uint8_t*>(((uintptr_t)smem_raw + 127) & ~(uintptr_t)127);
     const uint32_t base = smem_addr(sm);
@@ -58,7 +58,7 @@ decode_down_q6k_kernel(DownDecodeArgs a) {
     const uint32_t slot = warp / KB, kb = warp - slot * KB;
     const uint32_t RT = d.n_embd / 16;              // row tiles of the down matrix
     const uint32_t n_slots = d.n_used + 1;
-    const bool with_shared = a.sh_tiles != nullptr;
+    const bool with_shared = a.layer[0].sh != nullptr;
 
     const uint32_t ring = base + dq::kRings + warp * dq::kRingBytes;
     const uint32_t my_bar = base + dq::kBars + warp * dq::kStages * 8;
@@ -75,7 +75,7 @@ decode_down_q6k_kernel(DownDecodeArgs a) {
     }
     __syncthreads();
 
-    const uint64_t tiles_total = (uint64_t)a.n_tokens * RT;
+    const uint64_t tiles_total = (uint64_t)a.n_layers * a.n_tokens * RT;   // units: (layer, token, tile)
     const uint32_t u_lo = (uint32_t)(tiles_total * blockIdx.x / gridDim.x);
     const uint32_t u_hi = (uint32_t)(tiles_total * (blockIdx.x + 1) / gridDim.x);
     const size_t mat_tiles = (size_t)KB * RT;
@@ -89,9 +89,9 @@ decode_down_q6k_kernel(DownDecodeArgs a) {
         if (p_u >= u_hi) return;
         if (p_new_tok) {
             p_new_tok = false;
-            const uint32_t e = min(__ldcg(&a.sel[p_tok].ids[slot]), d.n_expert - 1);
-            p_src = a.tiles + ((size_t)e * mat_tiles + (size_t)kb * RT + p_rt) * kTileQ6;
-            if (with_shared) p_sh = a.sh_tiles + ((size_t)(warp >> 3) * RT + p_rt) * kTileQ8 + dq::kShBlock * (warp & 7u);
+            const uint32_t l = layer_of(a, p_tok), e = min(__ldcg(&layer_sel(a, l)[p_tok - l * a.n_tokens].ids[slot]), d.n_expert - 1);
+            p_src = a.layer[l].w + ((size_t)e * mat_tiles + (size_t)kb * RT + p_rt) * kTileQ6;
+            if (with_shared) p_sh = a.layer[l].sh + ((size_t)(warp >> 3) * RT + p_rt) * kTileQ8 + dq::kShBlock * (warp & 7u);
         }
         const uint32_t bar = my_bar + 8 * stage, dst = ring + stage * dq::kStageBytes;
         mbar_expect_tx(bar, kTileQ6 + (with_shared ? dq::kShBlock : 0));
@@ -124,14 +124,19 @@ decode_down_q6k_kernel(DownDecodeArgs a) {
 
     uint32_t tok = u_lo / RT, rt = u_lo - tok * RT;
     bool new_tok = true;
+    float* y = nullptr;            // the token's output row
     for (uint32_t u = u_lo; u < u_hi;) {
         if (new_tok) {   // block-uniform
             new_tok = false;
-            const float* hs = a.h + ((size_t)tok * n_slots + slot) * d.n_ff + 256 * kb + 8 * lane;
+            const uint32_t l = layer_of(a, tok), lt = tok - l * a.n_tokens;   // layer, token of the layer
+            const float* h = layer_h(a, l) + (size_t)lt * n_slots * d.n_ff;
+            const qkm_sel* rec = layer_sel(a, l) + lt;
+            y = a.y + l * a.y_stride + (size_t)lt * d.n_embd;
+            const float* hs = h + slot * d.n_ff + 256 * kb + 8 * lane;
             const float4 v0 = *reinterpret_cast<const float4*>(hs), v1 = *reinterpret_cast<const float4*>(hs + 4);
-            const float w_slot = a.sel[tok].w[slot];
-            w_sh = a.sel[tok].w_shared;
-            const float hv_sh = (with_shared && tid < d.n_ff) ? a.h[((size_t)tok * n_slots + d.n_used) * d.n_ff + tid] : 0.f;
+            const float w_slot = rec->w[slot];
+            w_sh = rec->w_shared;
+            const float hv_sh = (with_shared && tid < d.n_ff) ? h[d.n_used * d.n_ff + tid] : 0.f;
             {
                 const float hv[8] = {v0.x, v0.y, v0.z, v0.w, v1.x, v1.y, v1.z, v1.w};
                 float m = 0.f;
@@ -254,7 +259,7 @@ decode_down_q6k_kernel(DownDecodeArgs a) {
 #pragma unroll
             for (int w = 0; w < dq::kWarps; ++w)   // slot order, column blocks inside a slot
                 sum += red[((buf * dq::kWarps + w) * dq::kChunk + i) * 16 + r];
-            a.y[(size_t)tok * d.n_embd + (rt + i) * 16 + r] = sum;
+            y[(rt + i) * 16 + r] = sum;
         }
         buf ^= 1u;
         u += n_c;

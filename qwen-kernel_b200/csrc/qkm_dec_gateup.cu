@@ -6,11 +6,11 @@
 // up to two of the tokens that chose it (the reference's "live expert union" of multi-slot
 // decode), and the shared expert rides in the same work list as groups of its own.
 //
-// Every block first groups the selection's (token, slot) pairs by expert in its own shared
-// memory (qkm_dec_rank.cuh), so the work list needs no launch, no serial tail of a single block
-// and no trip through global memory.
+// Several layers whose rows are at hand together go through one launch: the list of work runs over all of them, so start-up, first
+// tiles and the uneven end are paid once (12 to 13 us of each kernel did not depend on the work: one layer of 16 tokens 41 us, 40 layers
+// together 27 us each).
 //
-// Work: the flat list of (group, 16-row tile) pairs - a group is an expert with up to two
+// Work: the flat list of (layer, group, 16-row tile) - a group is an expert with up to two
 // tokens, n_ff / 16 tiles each - is cut evenly and contiguously over teams of KB = n_embd / 256
 // warps; warp kb of a team streams column block kb of every tile of the team's range through
 // a private two-stage ring of bulk copies (TMA, no tensor map, no multicast).
@@ -54,14 +54,13 @@ constexpr int kGroupTiles = 4;                      // tiles between two team-wi
 constexpr int kRedFloats = kGroupTiles * 16 * 2 * 2;   // per warp and buffer: tile, row, token, matrix
 constexpr uint32_t kHigh = kTab + kTabBytes;
 constexpr uint32_t kRed = kHigh + (kWarps - kLowRingWarps) * kRingBytes;
-constexpr uint32_t kRank = kRed + kWarps * 2 * kRedFloats * 4;   // RankShared: selection scratch, group list, pairs
-constexpr uint32_t kEnd = kRank + ((sizeof(RankShared) + 127) / 128) * 128;
+constexpr uint32_t kEnd = kRed + kWarps * 2 * kRedFloats * 4;
 // IQ4_XS form, offsets from the (128-byte aligned) start of the dynamic area: barriers, rings, scratch
 constexpr uint32_t kRings4 = 1024;
 constexpr uint32_t kRed4 = kRings4 + kWarps * kRingBytes4;
-constexpr uint32_t kRank4 = kRed4 + kWarps * 2 * kRedFloats * 4;
-constexpr uint32_t kEnd4 = kRank4 + ((sizeof(RankShared) + 127) / 128) * 128 + 128;
+constexpr uint32_t kEnd4 = kRed4 + kWarps * 2 * kRedFloats * 4 + 128;
 constexpr int kQ8Quarter = 2 * 544;                 // two 32-column blocks of a Q8_0 tile: d and quants of 16 rows each
+constexpr uint32_t kFewGroups = 64;                 // so many groups are read together with their number
 constexpr uint32_t kCostRouted = 8, kCostShared = 11;   // relative time of a routed / a shared tile (measured)
 }  // namespace dg
 
@@ -186,10 +185,13 @@ __device__ __forceinline__ void q8_quarter(uint32_t q, uint32_t lane, uint32_t g
 
 template <bool IQ4>
 __global__ void __launch_bounds__(dg::kWarps * 32, 1)
-decode_gateup_kernel(GateupDecodeArgs a) {
+decode_gateup_kernel(const __grid_constant__ GateupDecodeArgs a) {
     constexpr int kTileR = IQ4 ? kTileIq4 : kTileIq3;                       // routed tile bytes
     constexpr int kStageB = IQ4 ? dg::kStageBytes4 : dg::kStageBytes, kRingB = IQ4 ? dg::kRingBytes4 : dg::kRingBytes;
     extern __shared__ __align__(128) uint8_t smem_raw[];
+    __shared__ LayerCuts s_cuts;
+    __shared__ uint4 s_few[dg::kFewGroups];
+    __shared__ uint4 s_rec[dg::kWarps][2];   // the records of the group a warp works on and of the next one
     const uint32_t base = smem_addr(smem_raw);
     const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31u, g = lane >> 2, t = lane & 3u;
     const qkm_dims d = a.d;
@@ -224,69 +226,92 @@ decode_gateup_kernel(GateupDecodeArgs a) {
         for (uint32_t i = 0; i < 4; ++i) bulk_g2s(dg::kTab + i * 16384u, a.luts + i * 16384u, 16384u, tab_bar);
     }
 
+    const uint32_t teams_total = gridDim.x * n_teams, team_global = blockIdx.x * n_teams + team;
+    const Divisor by_teams(teams_total), by_tiles(RT);
+
     // Up to here nothing depended on the router kernel, so a block scheduled early (programmatic
     // dependent launch) has its barriers and table copy under way while that kernel's tail runs.  The
     // next kernel is released only now: what it reads before its own wait (the selection) is then final.
     pdl_wait();
     pdl_trigger();
 
-    // Every block groups the selection's pairs by expert itself (same lists everywhere).
-    RankShared& S = *reinterpret_cast<RankShared*>(smem_raw + ((IQ4 ? base4 + dg::kRank4 : dg::kRank) - base));
-    group_pairs_shared(S, a.sel, d, a.n_tokens, a.expert_first, a.expert_count, a.with_shared != 0, dg::kWarps);
-
-    // This team's contiguous share of the flat tile list.  A shared-expert (Q8_0) tile takes longer
+    // This team's contiguous share of the flat list.  A shared-expert (Q8_0) tile takes longer
     // than a routed one (four ring stages, each a round trip), so the cut is made in cost units:
-    // kCostRouted per routed tile, kCostShared per shared tile (the shared groups come last).
-    const uint32_t n_groups = S.n_groups, n_routed = S.n_routed;
-    const uint32_t teams_total = gridDim.x * n_teams, team_global = blockIdx.x * n_teams + team;
-    const uint32_t tiles_routed = n_routed * RT, tiles_total = n_groups * RT;
-    const uint64_t cost_routed = (uint64_t)tiles_routed * dg::kCostRouted;
-    const uint64_t cost_total = cost_routed + (uint64_t)(tiles_total - tiles_routed) * dg::kCostShared;
-    auto cut = [&](uint32_t i) -> uint32_t {
-        const uint64_t c = cost_total * i / teams_total;
-        return c <= cost_routed ? (uint32_t)(c / dg::kCostRouted) : tiles_routed + (uint32_t)((c - cost_routed) / dg::kCostShared);
+    // kCostRouted per routed tile, kCostShared per shared tile (a layer's shared groups come last).
+    if (warp == 0) layer_cuts(s_cuts, a.groups, a.n_tokens, a.n_layers, dg::kCostRouted, dg::kCostShared);
+    // A few rows of one layer: the records come with the count, not one trip to L2 after it (unwritten ones are not looked at)
+    const bool few = a.groups.group && a.n_layers == 1 && a.n_tokens * (d.n_used + 1) <= dg::kFewGroups;
+    if (few && tid >= 64 && tid - 64 < a.n_tokens * (d.n_used + 1)) s_few[tid - 64] = __ldcg(reinterpret_cast<const uint4*>(a.groups.group) + (tid - 64));
+    __syncthreads();
+    uint32_t left;   // tiles still to do
+    ListPlace f_at = list_share(s_cuts, a.n_tokens, a.n_layers, by_tiles, dg::kCostRouted, dg::kCostShared, team_global, by_teams, left);   // next group to fetch
+    uint32_t rt = f_at.rt;   // the consumers' tile in its group
+    // Lane 0 brings the records, two groups ahead of the consumers' (the producer is at most one group ahead of them: RT >= 4, two stages).
+    // In shared memory, since a record in registers costs the IQ3_XXS form spills (50 us of 1950 at 40 layers of 16 tokens).
+    const uint32_t my_rec = smem_addr(&s_rec[warp][0]);
+    auto fetch = [&](uint32_t slot) {
+        if (f_at.l >= a.n_layers) return;
+        if (few) s_rec[warp][slot] = s_few[f_at.gi];
+        else if (a.groups.group) ldgsts16(my_rec + 16 * slot, a.groups.group + (size_t)f_at.l * a.n_tokens * (d.n_used + 1) + f_at.gi);
+        else {
+            const DecodeGroup r = decode_group(a.groups, a.n_tokens, d.n_used, f_at.l, f_at.gi);
+            s_rec[warp][slot] = make_uint4(r.head, r.pair[0], r.pair[1], r.layer);
+        }
+        f_at.next_group(s_cuts);
     };
-    const uint32_t t_lo = cut(team_global), t_hi = team_global + 1 == teams_total ? tiles_total : cut(team_global + 1);
+    auto record = [&](uint32_t slot) {
+        const uint4 v = lds128(my_rec + 16 * slot);
+        return DecodeGroup{v.x, {v.y, v.z}, v.w};
+    };
+    uint32_t k = 0, p_k = 0;   // groups begun by the consumers, by the producer: their records' places
     const size_t mat_tiles = (size_t)KB * RT;
 
     // producer cursor over (tile, quarter); lane 0 only.  A routed tile is one stage, a shared
     // tile four (its quarters).
-    uint32_t p_tile = t_lo, p_q = 0, p_rt = RT;   // p_rt == RT: the group record must be (re)loaded
-    uint32_t p_gi = t_lo / RT;
+    uint32_t p_left = left, p_q = 0;
+    uint32_t p_rt = rt;
+    bool p_new = true;                            // the group record must be (re)loaded
     const uint8_t* p_g = nullptr;                 // next tile of the gate (routed) / shared gate matrix
     const uint8_t* p_u = nullptr;
-    uint32_t p_kind = 0;
+    bool p_shared = false;
     auto issue = [&](uint32_t stage) {
-        if (p_tile >= t_hi) return;
-        if (p_rt >= RT) {   // first call, or the previous group is finished
-            p_rt = p_tile - p_gi * RT;
-            const DecodeGroup r = S.groups[p_gi];
-            p_kind = r.kind;
-            if (p_kind == 0) {
-                const size_t tile = (size_t)r.expert * mat_tiles + (size_t)kb * RT + p_rt;
-                p_g = a.gate_tiles + tile * kTileR; p_u = a.up_tiles + tile * kTileR;
+        if (p_left == 0) return;
+        if (p_new) {   // first call, or the previous group is finished
+            p_new = false;
+            ldgsts_wait();
+            const DecodeGroup r = record(p_k++ & 1u);
+            const GateupDecodeArgs::Mats& m = a.layer[r.layer];
+            p_shared = r.shared();
+            if (!p_shared) {
+                const size_t tile = (size_t)r.expert() * mat_tiles + (size_t)kb * RT + p_rt;
+                p_g = m.gate + tile * kTileR; p_u = m.up + tile * kTileR;
             } else {
                 const size_t tile = (size_t)kb * RT + p_rt;
-                p_g = a.sh_gate_tiles + tile * kTileQ8; p_u = a.sh_up_tiles + tile * kTileQ8;
+                p_g = m.sh_gate + tile * kTileQ8; p_u = m.sh_up + tile * kTileQ8;
             }
         }
+        auto next_tile = [&]() {
+            --p_left;
+            if (++p_rt == RT) { p_rt = 0; p_new = true; }
+        };
         const uint32_t bar = my_bar + 8 * stage, dst = ring + stage * kStageB;
-        if (p_kind == 0) {
+        if (!p_shared) {
             mbar_expect_tx(bar, 2 * kTileR);
             bulk_g2s(dst, p_g, kTileR, bar);
             bulk_g2s(dst + kTileR, p_u, kTileR, bar);
             p_g += kTileR; p_u += kTileR;
-            ++p_tile; ++p_rt;
+            next_tile();
         } else {
             mbar_expect_tx(bar, 2 * dg::kQ8Quarter);   // a quarter = two 32-column blocks = one 1088-byte piece
             bulk_g2s(dst, p_g + dg::kQ8Quarter * p_q, dg::kQ8Quarter, bar);
             bulk_g2s(dst + dg::kQ8Quarter, p_u + dg::kQ8Quarter * p_q, dg::kQ8Quarter, bar);
-            if (++p_q == 4) { p_q = 0; p_g += kTileQ8; p_u += kTileQ8; ++p_tile; ++p_rt; }
+            if (++p_q == 4) { p_q = 0; p_g += kTileQ8; p_u += kTileQ8; next_tile(); }
         }
-        if (p_rt >= RT) ++p_gi;
     };
-    if (lane == 0)
+    if (lane == 0) {
+        if (left) { fetch(0); fetch(1); }
         for (int s = 0; s < dg::kStages; ++s) issue(s);
+    }
 
     const uint32_t grid_c = dg::kTab + lane * 4;
     const uint32_t i_off = 64 * g + piece_at(g, t), s_off = 32 * g + 16 * ((t >> 1) ^ ((g >> 2) & 1u)) + 8 * (t & 1u);   // this lane's pieces of row g (rows g+8 alike)
@@ -294,39 +319,40 @@ decode_gateup_kernel(GateupDecodeArgs a) {
     uint32_t cnt = 0;   // stages consumed by this warp
     uint32_t b0[8], b1[8], n0[8], n1[8];
     float wcol0 = 0.f, wcol1 = 0.f;   // digit weights of the two C columns of this lane (2t, 2t+1)
-    DecodeGroup rec{};
-    uint32_t e_first = 0, e_n = 0, e_buf = 0;   // tiles waiting for the team-wide reduction: first rt, count, buffer
-    uint32_t gi = t_lo / RT, rt = t_lo - gi * RT;
+    bool shared = false;   // the group is one of the shared expert's
+    uint32_t e_n = 0, e_buf = 0;   // tiles waiting for the team-wide reduction (the last e_n up to rt): count, buffer
     bool new_group = true;
-    // where this thread's reduction outputs of the current group go: (token, slot) of token slot lt & 1
-    size_t h_base = 0;
-    bool ts_live = false;
+    float* h = nullptr;   // where this thread's reduction outputs of the current group go: (token, slot) of token slot lt & 1; null: none
 
     if (!IQ4 && !mbar_wait_bounded(tab_bar, 0)) timed_out = true;   // every thread observes the table's arrival itself
 
-    for (uint32_t tile = t_lo; tile < t_hi; ++tile) {
+    for (; left; --left) {
         if (new_group) {
             new_group = false;
-            rec = S.groups[gi];
+            if (lane == 0) ldgsts_wait();
+            __syncwarp();
+            const DecodeGroup rec = record(k & 1u);
+            shared = rec.shared();
+            const uint32_t row0 = rec.layer * a.n_tokens;   // the layer's first row of the planes
             {
                 const uint32_t ets = lt & 1u;   // the reduction below gives this thread token slot (j & 1) == (lt & 1)
-                ts_live = ets < rec.ntok;
-                if (ts_live) {
-                    const uint32_t pr = S.pairs[rec.pair_off + ets], tok = pr >> 4, slot = pr & 15u;
-                    h_base = ((size_t)tok * (d.n_used + 1) + slot) * d.n_ff;
+                h = nullptr;
+                if (ets < rec.ntok()) {
+                    const uint32_t pr = rec.pair_of(ets), tok = pr >> 4, slot = pr & 15u;
+                    h = (rec.layer + 1 == a.n_layers ? a.h_last : a.h + (size_t)row0 * (d.n_used + 1) * d.n_ff) + ((size_t)tok * (d.n_used + 1) + slot) * d.n_ff;
                 }
             }
             // B operand: column g of the MMA = (token slot g >> 2, digit g & 3); this warp's 256 columns
             const uint32_t ts = g >> 2, dgt = g & 3u;
-            if (ts < rec.ntok) {
-                const uint32_t tok = S.pairs[rec.pair_off + ts] >> 4;
-                const int8_t* pl = a.planes + (((size_t)tok * KB + kb) * 8 + dgt) * 256;
+            if (ts < rec.ntok()) {
+                const uint32_t row = row0 + (rec.pair_of(ts) >> 4);
+                const int8_t* pl = a.planes + (((size_t)row * KB + kb) * 8 + dgt) * 256;
 #pragma unroll
                 for (int sb = 0; sb < 8; ++sb) {
-                    if (IQ4 && rec.kind == 0) {   // iq4_word_gu's order
+                    if (IQ4 && !rec.shared()) {   // iq4_word_gu's order
                         const uint2 v = *reinterpret_cast<const uint2*>(pl + 32 * sb + 8 * t);
                         b0[sb] = prmt(v.x, 0u, 0x3120u); b1[sb] = prmt(v.y, 0u, 0x3120u);
-                    } else if (rec.kind == 0) {   // lane t owns elements 8t .. 8t+7 of each sub-block
+                    } else if (!rec.shared()) {   // lane t owns elements 8t .. 8t+7 of each sub-block
                         const uint2 v = *reinterpret_cast<const uint2*>(pl + 32 * sb + 8 * t);
                         const uint2 n = *reinterpret_cast<const uint2*>(pl + 1024 + 32 * sb + 8 * t);
                         b0[sb] = v.x; b1[sb] = v.y; n0[sb] = n.x; n1[sb] = n.y;
@@ -341,14 +367,16 @@ decode_gateup_kernel(GateupDecodeArgs a) {
             }
             const uint32_t cts = t >> 1;   // token slot of C columns 2t, 2t+1
             wcol0 = 0.f; wcol1 = 0.f;
-            if (cts < rec.ntok) {
-                const float sc = a.xscale[(S.pairs[rec.pair_off + cts] >> 4) * KB + kb];
+            if (cts < rec.ntok()) {
+                const float sc = a.xscale[(row0 + (rec.pair_of(cts) >> 4)) * KB + kb];
                 const float w0 = (t & 1u) ? 16384.f : 1.f;   // 128^(2 * (t & 1))
                 wcol0 = sc * w0;
                 wcol1 = sc * w0 * 128.f;
             }
+            __syncwarp();   // every lane has used its record
+            if (lane == 0) fetch(k & 1u);
+            ++k;
         }
-        if (e_n == 0) e_first = rt;
         float ga, gb, ua, ub;
         // The token's other two digits sit in lane t^1.  The exchange comes before the stage is filled again: it needs what was read last, so
         // no read is under way any more.  (A copy does not wait for reads that are: with the refill first, a tile's last rows got the scales of
@@ -357,7 +385,7 @@ decode_gateup_kernel(GateupDecodeArgs a) {
             ga += __shfl_xor_sync(0xFFFFFFFFu, ga, 1); gb += __shfl_xor_sync(0xFFFFFFFFu, gb, 1);
             ua += __shfl_xor_sync(0xFFFFFFFFu, ua, 1); ub += __shfl_xor_sync(0xFFFFFFFFu, ub, 1);
         };
-        if (rec.kind == 0) {
+        if (!shared) {
             const uint32_t stage = cnt % dg::kStages, parity = (cnt / dg::kStages) & 1u;
             if (!mbar_wait_bounded(my_bar + 8 * stage, parity)) timed_out = true;
             const uint32_t sbase = ring + stage * kStageB;
@@ -409,28 +437,28 @@ decode_gateup_kernel(GateupDecodeArgs a) {
             *reinterpret_cast<float2*>(my_red + (((e_n * 16 + g + 8) * 2 + ts) * 2)) = make_float2(gb, ub);
         }
         ++e_n;
-        if (e_n == dg::kGroupTiles || (rt & (dg::kGroupTiles - 1)) == dg::kGroupTiles - 1 || tile + 1 == t_hi) {
+        if (e_n == dg::kGroupTiles || (rt & (dg::kGroupTiles - 1)) == dg::kGroupTiles - 1 || left == 1) {
             // team-wide: sum the KB column-block partials, SwiGLU, store.  The scratch is double
             // buffered, so one barrier per reduction is enough.
             asm volatile("bar.sync %0, %1;" ::"r"(team + 1), "r"(team_threads) : "memory");
             for (uint32_t j = lt; j < e_n * 32; j += team_threads) {   // team_threads is even: j & 1 == lt & 1
                 const uint32_t ts = j & 1u, row = j >> 1;   // row within the waiting tiles
-                if (ts_live) {
+                if (h) {
                     float gsum = 0.f, usum = 0.f;
                     for (uint32_t w = 0; w < KB; ++w) {
                         const float2 r = *reinterpret_cast<const float2*>(red + ((team * KB + w) * 2 + e_buf) * dg::kRedFloats + (row * 2 + ts) * 2);
                         gsum += r.x; usum += r.y;
                     }
                     const float hv = swiglu(gsum, usum);
-                    const uint32_t r_ff = e_first * 16 + row;
-                    a.h[h_base + r_ff] = hv;
+                    h[(rt + 1 - e_n) * 16 + row] = hv;
                 }
             }
             e_n = 0;
             e_buf ^= 1u;
         }
-        if (++rt == RT) { rt = 0; ++gi; new_group = true; }
+        if (++rt == RT) { rt = 0; new_group = true; }
     }
+    if (lane == 0) ldgsts_wait();   // a record that the share did not get to
     if (timed_out && lane == 0) atomicExch(a.status, (uint32_t)kStatusWaitTimeout);
 }
 

@@ -1,13 +1,13 @@
-// Decode-sized batches (<= 64 tokens): router logits, top-k selection and the activation rows as
-// int8 digit planes, in one launch.  (The token-expert grouping happens at the start of the
-// gate/up kernel, in every block's own shared memory: qkm_dec_rank.cuh.)
+// Decode-sized batches (<= 64 tokens) of one or more layers: router logits, top-k selection, the pairs grouped by
+// expert and the activation rows as int8 digit planes, in one launch.
 //
 // Replaces, for the fused decode sequence, moe_logits.comp + moe_select_256.comp, i.e. their
 // fused form moe_route_select.comp.  Two kinds of blocks share the grid:
-//   * logits blocks: two router rows and eight tokens each, f64 accumulation - the logits are
+//   * logits blocks: pairs of router rows and up to eight tokens each, f64 accumulation - the logits are
 //     those of the CPU reference's f64 router (src/main.cpp:1320-1324) up to the order of the
 //     f64 additions, so they are ranked as they are, without an error bound; the block that
-//     finishes a group of eight tokens last ranks them, one warp per token;
+//     finishes a group of tokens last ranks them, one warp per token, and the one that ranks a layer's
+//     last group groups the layer's pairs;
 //   * one block per token encodes x as digit planes (and their negatives, which the IQ3_XXS
 //     kernel multiplies with its sign masks) and evaluates the shared expert's gate
 //     sigmoid(gis . x) in f64 (moe_select.comp's wShared).
@@ -20,7 +20,6 @@ namespace qkm {
 
 namespace rd {
 constexpr int kThreads = 256;
-constexpr int kTok = 8;           // tokens per logits block
 }  // namespace rd
 
 // digit planes of one row, layout [kb][8][256]: planes 0..3 the digits, 4..7 their negatives
@@ -34,14 +33,80 @@ __device__ __forceinline__ void store_planes8(int8_t* __restrict__ pl, uint32_t 
     }
 }
 
-template <int TYPE>
-__global__ void __launch_bounds__(rd::kThreads, 2)
-route_decode_kernel(RouteDecodeArgs a) {
+// The ticket's number.  Release and acquire for the device: what the block wrote before the barrier ahead of it is seen by the block
+// that draws the last number, behind the barrier that follows.  (One such add for two fences by every thread: 0.3 us less.)
+__device__ __forceinline__ uint32_t ticket(uint32_t* counter) {
+    uint32_t n;
+    asm volatile("atom.add.acq_rel.gpu.global.u32 %0, [%1], 1;" : "=r"(n) : "l"(counter) : "memory");
+    return n;
+}
+// token t chose expert e in place `slot`
+__device__ __forceinline__ void choose(unsigned long long* s_mask, uint16_t* s_ids, uint32_t t, uint32_t slot, uint32_t e) {
+    s_ids[t * 16 + slot] = (uint16_t)e;
+    atomicOr(reinterpret_cast<uint32_t*>(s_mask) + 2 * e + (t >> 5), 1u << (t & 31u));   // bit t of the expert's 64
+}
+// Groups a layer's (token, slot) pairs by expert: a block of kThreads, two experts a thread; s_ids[t][16]: the layer's selection;
+// s_mask: the tokens that chose each expert.
+__device__ __forceinline__ void group_lists(const DecodeGroups& out, const uint16_t* s_ids, const unsigned long long* s_mask, const qkm_dims& d, uint32_t T, uint32_t layer) {
+    static_assert(rk::kMaxExperts == 2 * rd::kThreads, "two experts a thread");
+    __shared__ uint32_t s_sum[rd::kThreads / 32];
+    __shared__ uint32_t s_first[rk::kMaxExperts];   // first group of expert e
     const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31u;
+    DecodeGroup* groups = out.group + (size_t)layer * T * (d.n_used + 1);
+    const uint32_t np = T * d.n_used;
+    uint32_t c[2], v = 0;   // tokens of this thread's experts; groups up to the second one
+#pragma unroll
+    for (int h = 0; h < 2; ++h) { c[h] = (uint32_t)__popcll(s_mask[2 * tid + h]); v += (c[h] + 1) / 2; }
+    const uint32_t n = v;
+#pragma unroll
+    for (int i = 1; i < 32; i <<= 1) {
+        const uint32_t up = __shfl_up_sync(0xFFFFFFFFu, v, i);
+        if (lane >= (uint32_t)i) v += up;
+    }
+    if (lane == 31) s_sum[warp] = v;
+    __syncthreads();
+    uint32_t base = 0, total = 0;
+#pragma unroll
+    for (uint32_t w = 0; w < rd::kThreads / 32; ++w) { if (w < warp) base += s_sum[w]; total += s_sum[w]; }
+    uint32_t first = base + v - n;
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        const uint32_t e = 2 * tid + h;
+        s_first[e] = first;
+        for (uint32_t i = 0; 2 * i < c[h]; ++i, ++first) {
+            groups[first].head = DecodeGroup::make_head(e, min(2u, c[h] - 2 * i), 0);
+            groups[first].layer = layer;
+        }
+    }
+    // every token is one of the shared expert's pairs
+    for (uint32_t i = tid; i < (T + 1) / 2; i += rd::kThreads) {
+        groups[total + i] = DecodeGroup{DecodeGroup::make_head(0, min(2u, T - 2 * i), 1), {((2 * i) << 4) | d.n_used, (min(2 * i + 1, T - 1) << 4) | d.n_used}, layer};
+    }
+    if (tid == 0) out.count[layer] = total + (T + 1) / 2;
+    __syncthreads();
+    // a pair's rank inside its expert is the number of lower tokens that chose the expert
+    for (uint32_t p = tid; p < np; p += rd::kThreads) {
+        const uint32_t t = p / d.n_used, s = p - t * d.n_used, e = s_ids[t * 16 + s];
+        const uint32_t r = (uint32_t)__popcll(s_mask[e] & ((1ull << t) - 1ull));
+        groups[s_first[e] + r / 2].pair[r & 1u] = (t << 4) | s;
+    }
+}
+
+// TOK: tokens of a group; a.pairs_per_block: router row pairs that a logits block takes one after the other
+template <int TYPE, int TOK>
+__global__ void __launch_bounds__(rd::kThreads, 2)
+route_decode_kernel(const __grid_constant__ RouteDecodeArgs a) {
+    const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31u, layer = blockIdx.y;
     const qkm_dims d = a.d;
     const uint32_t T = a.n_tokens;
-    const uint32_t n_pair_blocks = (d.n_expert + 1) / 2;                              // blocks along the experts
-    const uint32_t n_logit_blocks = n_pair_blocks * ((T + rd::kTok - 1) / rd::kTok);  // times the token groups
+    const float* x = a.x + layer * a.x_stride;
+    qkm_sel* sel = layer + 1 == a.n_layers ? a.sel_last : a.sel + (size_t)layer * T;
+    double* logits = a.logits + (size_t)layer * T * d.n_expert;
+    const uint32_t n_pairs = (d.n_expert + 1) / 2, n_pair_blocks = (n_pairs + a.pairs_per_block - 1) / a.pairs_per_block;   // blocks along the experts
+    const uint32_t n_groups = (T + TOK - 1) / TOK, n_logit_blocks = n_pair_blocks * n_groups;                              // times the token groups
+
+    __shared__ unsigned long long s_mask[rk::kMaxExperts];
+    for (uint32_t e = tid; e < rk::kMaxExperts; e += rd::kThreads) s_mask[e] = 0ull;
 
     // x is the output of the kernel before; the selection, planes and logits written here are still
     // read by the previous layer's kernels until that kernel has ended
@@ -54,14 +119,14 @@ route_decode_kernel(RouteDecodeArgs a) {
         __shared__ float s_up[16];
         __shared__ double s_sg[8];
         const uint32_t t = blockIdx.x - n_logit_blocks, KB = d.n_embd / 256;
-        const float* xt = a.x + (size_t)t * d.n_embd;
+        const float *xt = x + (size_t)t * d.n_embd, *gis = a.layer[layer].gis;
         float v[16];   // n_embd <= 4096: element tid of every 256 columns
         double dsg = 0.0;
 #pragma unroll
         for (int i = 0; i < 16; ++i) {
             const uint32_t k = tid + 256 * i;
             v[i] = k < d.n_embd ? xt[k] : 0.f;
-            if (k < d.n_embd) dsg += (double)a.gis[k] * (double)v[i];
+            if (k < d.n_embd) dsg += (double)gis[k] * (double)v[i];
         }
         // a scale per 256 columns: a large element costs the others of its own block bits, not the whole row
 #pragma unroll
@@ -81,15 +146,15 @@ route_decode_kernel(RouteDecodeArgs a) {
             const bool bad = m >= 0x7F800000u;
             const int p = min(digit_exponent(__uint_as_float(m)), 126);
             s_up[tid] = bad ? 0.f : ldexpf(1.0f, p);   // (then NaN or zero times zero: digits of zero)
-            a.xscale[t * KB + tid] = bad ? __int_as_float(0x7FC00000) : ldexpf(1.0f, -p);
+            a.xscale[(layer * T + t) * KB + tid] = bad ? __int_as_float(0x7FC00000) : ldexpf(1.0f, -p);
         } else if (tid == 32) {
             double sg = 0.0;
 #pragma unroll
             for (int w = 0; w < 8; ++w) sg += s_sg[w];
-            a.sel[t].w_shared = (float)(1.0 / (1.0 + exp(-sg)));
+            sel[t].w_shared = (float)(1.0 / (1.0 + exp(-sg)));
         }
         __syncthreads();
-        int8_t* pl = a.planes + (size_t)t * 8 * d.n_embd;
+        int8_t* pl = a.planes + (size_t)(layer * T + t) * 8 * d.n_embd;
 #pragma unroll
         for (int i = 0; i < 16; ++i) {
             const uint32_t k = tid + 256 * i;
@@ -98,85 +163,122 @@ route_decode_kernel(RouteDecodeArgs a) {
         return;
     }
 
-    // ---- logits of two experts for kTok tokens ------------------------------------------------------
+    // ---- logits of pairs of experts for TOK tokens --------------------------------------------------
     // warp w owns the w-th eighth of the columns; a lane loads one 8-element unit of both router
-    // rows and the matching x values of the block's tokens in one go
-    __shared__ double s_part[8][2 * rd::kTok];
-    const uint32_t e0 = (blockIdx.x % n_pair_blocks) * 2u, t0 = (blockIdx.x / n_pair_blocks) * rd::kTok;
-    const bool two = e0 + 1 < d.n_expert;
+    // rows and the matching x values of the block's tokens in one go; the next pair's rows are on their way meanwhile
+    constexpr int NV = 2 * TOK, kLanes = 32 / NV;   // sums of a pair; lanes that end with the same one
+    __shared__ double s_part[2][8][NV];
+    const uint32_t p0 = blockIdx.x % n_pair_blocks * a.pairs_per_block, p1 = min(p0 + a.pairs_per_block, n_pairs), t0 = (blockIdx.x / n_pair_blocks) * TOK;
     const size_t rb = row_bytes(TYPE, d.n_embd);
-    const uint8_t* row0 = a.router + (size_t)e0 * rb;
-    const uint8_t* row1 = a.router + (size_t)(two ? e0 + 1 : e0) * rb;
+    const uint8_t* router = a.layer[layer].w;
     const uint32_t units_w = d.n_embd / 64;   // 8-element units per warp
-    {
-        double acc[2 * rd::kTok];   // [expert 0: tokens][expert 1: tokens]
+    const bool once = units_w <= 32;          // a lane has one unit: its router elements are read ahead
+    float w0[8], w1[8];
+    auto rows = [&](uint32_t pair, uint32_t u) {
+        const uint8_t* row0 = router + (size_t)(2 * pair) * rb;
+        const uint32_t k = (warp * units_w + u) * 8;
+        dequant8<TYPE>(row0, k, w0);
+        dequant8<TYPE>(2 * pair + 1 < d.n_expert ? row0 + rb : row0, k, w1);
+    };
+    if (once && lane < units_w) rows(p0, lane);
+    for (uint32_t pair = p0; pair < p1; ++pair) {
+        double acc[NV];   // [expert 0: tokens][expert 1: tokens]
 #pragma unroll
-        for (int j = 0; j < 2 * rd::kTok; ++j) acc[j] = 0.0;
+        for (int j = 0; j < NV; ++j) acc[j] = 0.0;
         for (uint32_t u = lane; u < units_w; u += 32) {
             const uint32_t k = (warp * units_w + u) * 8;
-            float w0[8], w1[8];
-            dequant8<TYPE>(row0, k, w0);
-            dequant8<TYPE>(row1, k, w1);
-            float4 xa[rd::kTok], xb[rd::kTok];
+            if (!once) rows(pair, u);
+            constexpr int kHalf = TOK < 4 ? TOK : 4;   // four tokens' values at a time: more do not fit the registers
+            float4 xa[kHalf], xb[kHalf];
+            auto tokens = [&](int j0) {
 #pragma unroll
-            for (int j = 0; j < rd::kTok; ++j) {
-                const uint32_t tt = min(t0 + j, T - 1);
-                const float* xt = a.x + (size_t)tt * d.n_embd + k;
-                xa[j] = *reinterpret_cast<const float4*>(xt);
-                xb[j] = *reinterpret_cast<const float4*>(xt + 4);
-            }
+                for (int j = 0; j < kHalf; ++j) {
+                    const float* xt = x + (size_t)min(t0 + j0 + j, T - 1) * d.n_embd + k;
+                    xa[j] = *reinterpret_cast<const float4*>(xt);
+                    xb[j] = *reinterpret_cast<const float4*>(xt + 4);
+                }
+            };
+            tokens(0);   // (on its way together with the rows: the conversions below wait for those)
+            double v0[8], v1[8];
 #pragma unroll
-            for (int j = 0; j < rd::kTok; ++j) {
-                const double x0 = xa[j].x, x1 = xa[j].y, x2 = xa[j].z, x3 = xa[j].w;
-                const double x4 = xb[j].x, x5 = xb[j].y, x6 = xb[j].z, x7 = xb[j].w;
-                double s = acc[j];
-                s += (double)w0[0] * x0; s += (double)w0[1] * x1; s += (double)w0[2] * x2; s += (double)w0[3] * x3;
-                s += (double)w0[4] * x4; s += (double)w0[5] * x5; s += (double)w0[6] * x6; s += (double)w0[7] * x7;
-                acc[j] = s;
-                s = acc[rd::kTok + j];
-                s += (double)w1[0] * x0; s += (double)w1[1] * x1; s += (double)w1[2] * x2; s += (double)w1[3] * x3;
-                s += (double)w1[4] * x4; s += (double)w1[5] * x5; s += (double)w1[6] * x6; s += (double)w1[7] * x7;
-                acc[rd::kTok + j] = s;
-            }
-        }
-        // reduce-scatter over the warp: after the step with distance o a lane keeps the half of its
-        // values selected by (lane & o); 16 values, distances 16..2 halve them to one, distance 1 finishes it
+            for (int i = 0; i < 8; ++i) { v0[i] = w0[i]; v1[i] = w1[i]; }
+            if (once && pair + 1 < p1) rows(pair + 1, u);
 #pragma unroll
-        for (int o = 16, n = 2 * rd::kTok; o >= 2; o >>= 1, n >>= 1) {
-            const bool up = (lane & o) != 0;
+            for (int j0 = 0; j0 < TOK; j0 += kHalf) {
+                if (j0 > 0) tokens(j0);
 #pragma unroll
-            for (int j = 0; j < n / 2; ++j) {
-                const double send = up ? acc[j] : acc[j + n / 2];
-                const double keep = up ? acc[j + n / 2] : acc[j];
-                acc[j] = keep + __shfl_xor_sync(0xFFFFFFFFu, send, o);
+                for (int j = 0; j < kHalf; ++j) {
+                    const double xv[8] = {xa[j].x, xa[j].y, xa[j].z, xa[j].w, xb[j].x, xb[j].y, xb[j].z, xb[j].w};
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) { acc[j0 + j] += v0[i] * xv[i]; acc[TOK + j0 + j] += v1[i] * xv[i]; }
+                }
             }
         }
-        const double v = acc[0] + __shfl_xor_sync(0xFFFFFFFFu, acc[0], 1);
-        // lane l holds value index: bit 3 from (l & 16), bit 2 from (l & 8), bit 1 from (l & 4), bit 0 from (l & 2)
-        if ((lane & 1u) == 0) s_part[warp][(lane >> 1) & 15u] = v;
-    }
-    __syncthreads();
-    if (tid < 2 * rd::kTok) {
-        const uint32_t r = tid / rd::kTok, j = tid % rd::kTok;
-        double v = 0.0;
+        // reduce-scatter over the warp: after the step with distance o a lane keeps the half of its values selected by (lane & o); once one is
+        // left, plain sums
+        int n = NV;
 #pragma unroll
-        for (int w = 0; w < 8; ++w) v += s_part[w][tid];
-        if (t0 + j < T && (r == 0 || two)) a.logits[(size_t)(t0 + j) * d.n_expert + e0 + r] = v;
+        for (int o = 16; o >= 1; o >>= 1) {
+            if (n > 1) {
+                n >>= 1;
+                const bool up = (lane & o) != 0;
+#pragma unroll
+                for (int j = 0; j < NV / 2; ++j)
+                    if (j < n) {
+                        const double send = up ? acc[j] : acc[j + n], keep = up ? acc[j + n] : acc[j];
+                        acc[j] = keep + __shfl_xor_sync(0xFFFFFFFFu, send, o);
+                    }
+            } else {
+                acc[0] += __shfl_xor_sync(0xFFFFFFFFu, acc[0], o);
+            }
+        }
+        double (&part)[8][NV] = s_part[pair & 1u];   // two: a pair's sums are read while the next one's are written
+        if (lane % kLanes == 0) part[warp][lane / kLanes] = acc[0];
+        __syncthreads();
+        if (tid < NV) {
+            const uint32_t r = tid / TOK, j = tid % TOK;
+            double v = 0.0;
+#pragma unroll
+            for (int w = 0; w < 8; ++w) v += part[w][tid];
+            if (t0 + j < T && 2 * pair + r < d.n_expert) logits[(size_t)(t0 + j) * d.n_expert + 2 * pair + r] = v;
+        }
     }
 
     // ---- the block that finishes a token group's logits last ranks the group's tokens ---------------
-    // (a ticket counter per group; writes are fenced before the ticket, reads after it - the
-    // device-scope release/acquire the reference's fused router relies on, moe_route_select.comp:56-67)
+    // (a ticket counter per group, taken by one thread between two barriers: the block's writes come before it, the
+    // reads after it - the device-scope release/acquire the reference's fused router relies on, moe_route_select.comp:56-67)
     __shared__ uint32_t s_last;
-    uint32_t* counter = a.counter + blockIdx.x / n_pair_blocks;
-    __threadfence();
+    uint32_t* counter = a.counter + layer * kDecCounters + blockIdx.x / n_pair_blocks;
     __syncthreads();
-    if (tid == 0) s_last = atomicAdd(counter, 1u) == n_pair_blocks - 1 ? 1u : 0u;
+    if (tid == 0) s_last = ticket(counter) == n_pair_blocks - 1 ? 1u : 0u;
     __syncthreads();
     if (!s_last) return;
     if (tid == 0) *counter = 0;   // ready for the next launch
-    __threadfence();
-    rank_tokens(a.logits, a.sel, d, t0, min((uint32_t)rd::kTok, T - t0), rd::kThreads / 32);
+    __shared__ uint16_t s_ids[rk::kMaxTokens * 16];
+    static_assert(TOK <= rd::kThreads / 32, "a warp ranks one token");
+    const bool ranks = warp < min((uint32_t)TOK, T - t0);
+    const uint32_t my_t = t0 + warp;
+    Ranked mine{};
+    if (ranks) {
+        mine = rank_token(logits + (size_t)my_t * d.n_expert, d);
+        if (n_groups > 1) rank_store(mine, sel[my_t], d);
+        else if (lane < d.n_used) choose(s_mask, s_ids, my_t, lane, mine.id);
+    }
+
+    // ---- and the block that ranks a layer's last token group groups the layer's pairs --------------
+    if (n_groups > 1) {   // (the only group's ids are in shared memory)
+        __syncthreads();
+        uint32_t* groups_done = a.counter + layer * kDecCounters + kDecCounters - 1;
+        if (tid == 0) s_last = ticket(groups_done) == n_groups - 1 ? 1u : 0u;
+        __syncthreads();
+        if (!s_last) return;
+        if (tid == 0) *groups_done = 0;
+        for (uint32_t i = tid; i < T * 16; i += rd::kThreads)
+            if ((i & 15u) < d.n_used) choose(s_mask, s_ids, i >> 4, i & 15u, min(__ldcg(&sel[i >> 4].ids[i & 15u]), d.n_expert - 1));
+    }
+    __syncthreads();
+    group_lists(a.groups, s_ids, s_mask, d, T, layer);
+    if (n_groups == 1 && ranks) rank_store(mine, sel[my_t], d);   // (after the lists: the next kernel waits for those)
 }
 
 bool route_decode_ok(const qkm_dims& d, uint32_t n_tokens, size_t scratch_bytes) {
@@ -184,15 +286,26 @@ bool route_decode_ok(const qkm_dims& d, uint32_t n_tokens, size_t scratch_bytes)
            (size_t)n_tokens * d.n_expert * sizeof(double) <= scratch_bytes;
 }
 
+// Tokens of a group: as few as the batch has (a group of eight costs one token as much as eight).  Pairs a block: one while the blocks
+// find room on the SMs at once (a chain of latencies: start-up, loads, ticket), more when layers go together, so that a block's share of that chain is
+// small: 40 layers of 16 tokens 159 us with one pair a block, 125 so.
+template <int TYPE>
+static cudaError_t route_launch(const Launch& L, RouteDecodeArgs a) {
+    const uint32_t T = a.n_tokens, tok = T <= 1 ? 1 : T <= 2 ? 2 : T <= 4 ? 4 : 8, groups = (T + tok - 1) / tok, pairs = (a.d.n_expert + 1) / 2;
+    const uint32_t per = pairs * groups * a.n_layers / 600;
+    a.pairs_per_block = per < 1 ? 1 : per < 16 ? per : 16;
+    const dim3 grid((pairs + a.pairs_per_block - 1) / a.pairs_per_block * groups + T, a.n_layers), block(rd::kThreads);
+    switch (tok) {
+        case 1: return launch_kernel(L, route_decode_kernel<TYPE, 1>, grid, block, 0, a);
+        case 2: return launch_kernel(L, route_decode_kernel<TYPE, 2>, grid, block, 0, a);
+        case 4: return launch_kernel(L, route_decode_kernel<TYPE, 4>, grid, block, 0, a);
+        default: return launch_kernel(L, route_decode_kernel<TYPE, 8>, grid, block, 0, a);
+    }
+}
 cudaError_t launch_route_decode(const Launch& L, uint32_t router_type, const RouteDecodeArgs& a) {
     if (router_type != QKM_TYPE_F32 && router_type != QKM_TYPE_F16) return cudaErrorInvalidValue;
-    if (a.n_tokens == 0 || a.n_tokens > 64 || a.d.n_expert > 512 || a.d.n_embd > 4096) return cudaErrorInvalidValue;
-    const dim3 grid((a.d.n_expert + 1) / 2 * ((a.n_tokens + rd::kTok - 1) / rd::kTok) + a.n_tokens);
-    cudaError_t e;
-    if (router_type == QKM_TYPE_F32)
-        e = launch_kernel(L, route_decode_kernel<QKM_TYPE_F32>, grid, dim3(rd::kThreads), 0, a);
-    else
-        e = launch_kernel(L, route_decode_kernel<QKM_TYPE_F16>, grid, dim3(rd::kThreads), 0, a);
+    if (a.n_tokens == 0 || a.n_tokens > 64 || a.d.n_expert > 512 || a.d.n_embd > 4096 || a.n_layers == 0 || a.n_layers > kDecMaxLayers) return cudaErrorInvalidValue;
+    const cudaError_t e = router_type == QKM_TYPE_F32 ? route_launch<QKM_TYPE_F32>(L, a) : route_launch<QKM_TYPE_F16>(L, a);
     L.count();
     return e != cudaSuccess ? e : cudaGetLastError();
 }

@@ -67,41 +67,50 @@ struct MmaItem {
 };
 
 // ---- fused decode sequence (qkm_dec_route.cu, qkm_dec_gateup.cu, qkm_dec_down.cu) ---------------
-// One expert (or the shared expert) with up to two of the tokens routed to it:
-// pairs[pair_off .. pair_off + ntok).  The gate/up kernel walks all n_ff rows of a group.
-struct DecodeGroup {
-    uint16_t expert;   // resident-expert index (kind 0)
-    uint8_t ntok;      // 1 or 2
-    uint8_t kind;      // 0 routed expert, 1 shared expert
-    uint32_t pair_off;
+// Several layers whose rows are at hand together go through one launch of each kernel; everything per layer lies one after the other,
+// `n_tokens` (and so on) apart.
+constexpr uint32_t kDecMaxLayers = 64, kDecCounters = 16;
+// One expert (or the shared expert) with up to two of the tokens routed to it.  The gate/up kernel walks all n_ff rows of a group.
+struct alignas(16) DecodeGroup {
+    uint32_t head;     // expert | tokens (1 or 2) << 16 | shared << 24
+    uint32_t pair[2];  // (token << 4) | slot; slot n_used: the shared expert
+    uint32_t layer;    // of the layers that go together
+    __host__ __device__ static uint32_t make_head(uint32_t expert, uint32_t ntok, uint32_t shared) { return expert | (ntok << 16) | (shared << 24); }
+    __host__ __device__ uint32_t expert() const { return head & 0xFFFFu; }
+    __host__ __device__ uint32_t ntok() const { return (head >> 16) & 255u; }
+    __host__ __device__ bool shared() const { return (head >> 24) != 0; }
+    __host__ __device__ uint32_t pair_of(uint32_t t) const { return t ? pair[1] : pair[0]; }   // t < ntok()
+};
+// A layer's (token, slot) pairs grouped by expert, ascending expert, then the shared expert's ceil(n_tokens / 2) groups
+struct DecodeGroups {
+    uint32_t* count;       // [layer]
+    DecodeGroup* group;    // [layer][n_tokens * (n_used + 1)]; NULL: the shared expert's groups only
 };
 struct RouteDecodeArgs {
-    const uint8_t* router;     // [n_expert][n_embd] F32 or F16
-    const float* gis;          // [n_embd]
-    const float* x;            // [n_tokens][n_embd]
-    qkm_sel* sel;              // out [n_tokens]
-    double* logits;            // scratch [n_tokens][n_expert]
-    uint32_t* counter;         // ceil(n_tokens / 8) zero words; left at zero
-    int8_t* planes;            // out [n_tokens][n_embd/256][8][256]: digit planes 0..3 and their negatives 4..7
-    float* xscale;             // out [n_tokens][n_embd/256] 2^-p
-    uint32_t n_tokens;
+    struct Router { const uint8_t* w; const float* gis; } layer[kDecMaxLayers];   // [n_expert][n_embd] F32 or F16; [n_embd]
+    const float* x;            // [n_tokens][n_embd] of the first layer
+    uint64_t x_stride;         // floats from one layer's rows to the next one's
+    qkm_sel *sel, *sel_last;   // out [layer][n_tokens]; the last layer's
+    double* logits;            // scratch [layer][n_tokens][n_expert]
+    uint32_t* counter;         // [layer][kDecCounters] zero words; left at zero
+    int8_t* planes;            // out [layer][n_tokens][n_embd/256][8][256]: digit planes 0..3 and their negatives 4..7
+    float* xscale;             // out [layer][n_tokens][n_embd/256] 2^-p
+    DecodeGroups groups;       // out
+    uint32_t n_tokens, n_layers, pairs_per_block;   // the last one is the launcher's
     qkm_dims d;
 };
 bool route_decode_ok(const qkm_dims& d, uint32_t n_tokens, size_t scratch_bytes);
 cudaError_t launch_route_decode(const Launch& L, uint32_t router_type, const RouteDecodeArgs& a);
 // routed (IQ3_XXS) and shared (Q8_0) gate/up + SwiGLU over the groups
 struct GateupDecodeArgs {
-    const uint8_t* gate_tiles;      // routed experts, IQ3_XXS or IQ4_XS tiles (gateup_type)
-    const uint8_t* up_tiles;
-    const uint8_t* sh_gate_tiles;   // shared expert, Q8_0 tiles (may be NULL when no group has kind 1)
-    const uint8_t* sh_up_tiles;
+    struct Mats { const uint8_t *gate, *up, *sh_gate, *sh_up; } layer[kDecMaxLayers];   // routed experts' IQ3_XXS or IQ4_XS tiles (gateup_type), the shared expert's Q8_0 tiles
     const uint8_t* luts;            // decode_gateup_lut_bytes() bytes written by launch_decode_gateup_luts
     const int8_t* planes;
-    const float* xscale;            // [n_tokens][n_embd/256]
-    const qkm_sel* sel;             // the selection (its pairs are grouped by expert in every block at its start)
-    uint32_t n_tokens, expert_first, expert_count, with_shared;
+    const float* xscale;
+    DecodeGroups groups;
+    uint32_t n_tokens, n_layers;
     uint32_t gateup_type;           // QKM_TYPE_IQ3_XXS or QKM_TYPE_IQ4_XS
-    float* h;                       // out [T][n_used+1][n_ff]
+    float *h, *h_last;              // out [layer][n_tokens][n_used+1][n_ff]; the last layer's
     uint32_t* status;
     qkm_dims d;
 };
@@ -111,17 +120,25 @@ bool decode_gateup_ok(const qkm_dims& d);
 cudaError_t launch_decode_gateup(const Launch& L, const GateupDecodeArgs& a, uint32_t n_blocks);
 // routed (IQ4_XS) down + shared (Q8_0) down + weighted sum: y[t] = sum_s w_s D[ids_s] h[t][s] + w_shared DS h[t][n_used]
 struct DownDecodeArgs {
-    const uint8_t* tiles;           // routed experts, IQ4_XS tiles (launch_decode_down_any: NULL for the shared term alone)
-    const uint8_t* sh_tiles;        // shared expert, Q8_0 tiles (NULL: no shared term)
+    struct Mats { const uint8_t *w, *sh; } layer[kDecMaxLayers];   // routed experts' IQ4_XS or Q6_K tiles (launch_decode_down_any: NULL for the shared term alone); the
+                                                                   // shared expert's Q8_0 tiles (NULL: no shared term)
     const uint8_t* lut;             // IQ4_XS form: decode_down_lut_bytes() bytes written by launch_decode_down_lut
-    const float* h;                 // [T][n_used+1][n_ff] f32 (encoded as int8 digit planes inside the kernel)
-    const qkm_sel* sel;
-    float* y;
-    float* contrib;                 // launch_decode_down_group: scratch [T][n_used+1][n_embd]
-    uint32_t n_tokens;
+    const float *h, *h_last;        // [layer][n_tokens][n_used+1][n_ff] f32 (encoded as int8 digit planes inside the kernels); the last layer's
+    const qkm_sel *sel, *sel_last;
+    float* y;                       // out [n_tokens][n_embd] of the first layer
+    uint64_t y_stride;              // floats from one layer's rows to the next one's
+    DecodeGroups groups;            // launch_decode_down_group
+    float* contrib;                 // launch_decode_down_group: scratch [layer][n_tokens][n_used+1][n_embd]
+    uint32_t n_tokens, n_layers;
     uint32_t* status;
     qkm_dims d;
 };
+#ifdef __CUDACC__
+// layer of the batch's row `row`, and records and hidden rows of a layer
+__device__ __forceinline__ uint32_t layer_of(const DownDecodeArgs& a, uint32_t row) { return a.n_layers == 1 ? 0u : row / a.n_tokens; }
+__device__ __forceinline__ const qkm_sel* layer_sel(const DownDecodeArgs& a, uint32_t l) { return l + 1 == a.n_layers ? a.sel_last : a.sel + (size_t)l * a.n_tokens; }
+__device__ __forceinline__ const float* layer_h(const DownDecodeArgs& a, uint32_t l) { return l + 1 == a.n_layers ? a.h_last : a.h + (size_t)l * a.n_tokens * (a.d.n_used + 1) * a.d.n_ff; }
+#endif
 bool decode_down_ok(const qkm_dims& d);
 size_t decode_down_lut_bytes();
 cudaError_t launch_decode_down_lut(const Launch& L, uint8_t* lut);

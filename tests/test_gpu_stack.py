@@ -1,0 +1,104 @@
+"""Decode stacks whose layers go through each stage of the fused sequence together, against the oracle, layer by layer."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+TOL_F32 = 1e-5   # as the layer-by-layer decode calls: exact integer sums, one f32 rounding per 256 columns
+
+
+def run_stack(pkg, syn, dims, layers, x, max_tokens=None, y_at=None):
+    """(y [L][T][n_embd], last layer's selection); y_at: byte offset of the outputs inside the inputs' buffer."""
+    L, T = x.shape[:2]
+    with pkg.Context(dims, n_layer=L, max_tokens=max_tokens or T, device=0) as ctx:
+        for l, layer in enumerate(layers):
+            ctx.upload_layer(l, layer)
+        if y_at is None:
+            d_x, d_y = ctx.to_device(x), ctx.alloc(x.nbytes)
+            for _ in range(3):   # counters and tickets are left as they were found
+                ctx.moe_decode_stack(0, L, d_x, T, d_y)
+            y = d_y.download(np.float32, x.shape)
+        else:
+            buf = ctx.to_device(np.concatenate([x.reshape(-1), np.zeros(y_at // 4, np.float32)]))
+            ctx.moe_decode_stack(0, L, buf.ptr, T, buf.ptr + y_at)
+            y = buf.download(np.float32, x.size + y_at // 4)[y_at // 4:].reshape(x.shape)
+        return y, ctx.last_sel(T)
+
+
+def check(syn, orc, layers, x, y, sel, tol=TOL_F32):
+    for l, layer in enumerate(layers):
+        ref = orc.moe_layer(layer, x[l], threads=orc.hardware_threads())
+        assert syn.rel_err_rows(y[l], ref["y"]) < tol, l
+        if l + 1 == len(layers):
+            n = layer.dims.n_used
+            assert np.array_equal(sel["ids"][:, :n], ref["sel"]["ids"][:, :n])
+            np.testing.assert_allclose(sel["w_shared"], ref["sel"]["w_shared"], rtol=1e-6)
+
+
+# every down kernel (8, other numbers of and more than ten slots; 40 tokens on), router groups of 1, 2, 4 and 8 tokens, odd numbers of tokens, a second
+# chunk of six tokens, two to eight column blocks, fewer tiles than teams of warps and many more, shares that begin inside a layer
+@pytest.mark.parametrize("n_embd,n_expert,n_used,gt,dt,T,L", [
+    (1024, 16, 4, 18, 23, 1, 3), (1024, 16, 4, 18, 23, 2, 3), (1024, 16, 4, 18, 14, 3, 3), (512, 16, 4, 23, 14, 9, 4), (512, 4, 4, 18, 23, 4, 2),
+    (2048, 32, 8, 18, 23, 16, 5), (2048, 32, 8, 23, 14, 16, 4), (1024, 512, 10, 23, 23, 5, 2), (512, 32, 15, 18, 14, 3, 2), (512, 20, 1, 18, 23, 33, 3),
+    (1024, 8, 8, 18, 14, 64, 2), (512, 24, 6, 23, 23, 70, 3), (512, 8, 2, 18, 23, 1, 30), (512, 16, 8, 18, 14, 2, 9)])
+def test_stack_layers_together(pkg, orc, syn, n_embd, n_expert, n_used, gt, dt, T, L):
+    dims = syn.Dims(n_embd=n_embd, n_ff=512, n_expert=n_expert, n_used=n_used)
+    layers = [syn.make_layer(dims, seed=200, layer=l, router_type=l0, gateup_type=gt, down_type=dt) for l, l0 in enumerate([T & 1] * L)]
+    x = np.stack([syn.random_x(T, n_embd, seed=210 + l) for l in range(L)])
+    y, sel = run_stack(pkg, syn, dims, layers, x)
+    check(syn, orc, layers, x, y, sel)
+
+
+def test_stack_of_several_types(pkg, orc, syn):
+    """Runs of layers of the same types; a run of one layer."""
+    dims = syn.Dims(n_embd=1024, n_ff=512, n_expert=16, n_used=4)
+    mixes = [(0, 18, 23), (0, 18, 23), (1, 18, 23), (1, 23, 14), (1, 23, 14), (1, 23, 14), (0, 18, 14)]
+    layers = [syn.make_layer(dims, seed=220, layer=l, router_type=r, gateup_type=g, down_type=d) for l, (r, g, d) in enumerate(mixes)]
+    x = np.stack([syn.random_x(7, 1024, seed=230 + l) for l in range(len(mixes))])
+    y, sel = run_stack(pkg, syn, dims, layers, x)
+    check(syn, orc, layers, x, y, sel)
+
+
+def test_stack_more_layers_than_scratch(pkg, orc, syn):
+    """64 tokens, 14 layers: more rows than go through together."""
+    dims = syn.Dims(n_embd=512, n_ff=512, n_expert=8, n_used=2)
+    layers = [syn.make_layer(dims, seed=240, layer=l) for l in range(14)]
+    x = np.stack([syn.random_x(64, 512, seed=250 + l) for l in range(14)])
+    y, sel = run_stack(pkg, syn, dims, layers, x)
+    check(syn, orc, layers, x, y, sel)
+
+
+def test_stack_outputs_that_feed_the_next_layer(pkg, orc, syn):
+    """y one layer behind x in the same buffer: layer l + 1 reads what layer l wrote.  And in place: every layer reads its own row first."""
+    dims = syn.Dims(n_embd=512, n_ff=512, n_expert=16, n_used=4)
+    T, L = 5, 3
+    layers = [syn.make_layer(dims, seed=260, layer=l) for l in range(L)]
+    x = np.stack([syn.random_x(T, 512, seed=270 + l) for l in range(L)])
+    y, _ = run_stack(pkg, syn, dims, layers, x, y_at=T * 512 * 4)
+    row = x[0]
+    for l in range(L):
+        row = orc.moe_layer(layers[l], row, threads=orc.hardware_threads())["y"]
+        assert syn.rel_err_rows(y[l], row) < 1e-4   # errors of the layers before go through
+        row = y[l]
+    y, sel = run_stack(pkg, syn, dims, layers, x, y_at=0)
+    check(syn, orc, layers, x, y, sel)
+
+
+@pytest.mark.parametrize("gt,dt", [(18, 23), (23, 14)])
+def test_stack_nonfinite_and_large_rows(pkg, orc, syn, gt, dt):
+    """A NaN or an infinity stays in its token; an element of 1e8 where the weights are zero costs the others of its row nothing."""
+    dims = syn.Dims(n_embd=1024, n_ff=512, n_expert=16, n_used=4)
+    layers = [syn.make_layer(dims, seed=280, layer=l, gateup_type=gt, down_type=dt) for l in range(2)]
+    for layer in layers:
+        for t, elems, size_b in ((layer.gate_exps, 256, syn.BLOCK[gt][1]), (layer.up_exps, 256, syn.BLOCK[gt][1]), (layer.gate_shexp, 32, 34), (layer.up_shexp, 32, 34)):
+            t.reshape(-1, dims.n_embd // elems, size_b)[:, 256 // elems:512 // elems, 0:2] = 0   # d of columns 256 .. 511
+    x = np.stack([syn.random_x(9, 1024, seed=290 + l) for l in range(2)])
+    x[:, 2, 300] = 1e8
+    x[:, 4, 7] = np.nan
+    x[:, 5, 900] = np.inf
+    y, _ = run_stack(pkg, syn, dims, layers, x)
+    ok = np.isfinite(x).all(axis=2)
+    for l in range(2):
+        ref = orc.moe_layer(layers[l], x[l][ok[l]], threads=orc.hardware_threads())
+        assert syn.rel_err_rows(y[l][ok[l]], ref["y"]) < TOL_F32
+        assert np.isnan(y[l][~ok[l]]).all()
