@@ -92,8 +92,9 @@ __device__ __forceinline__ void group_lists(const DecodeGroups& out, const uint1
     }
 }
 
-// TOK: tokens of a group; a.pairs_per_block: router row pairs that a logits block takes one after the other
-template <int TYPE, int TOK>
+// TOK: tokens of a group; a.pairs_per_block: router row pairs that a logits block takes one after the other; KEEP: the tokens' x stays in
+// registers as doubles for all of them (n_embd <= 2048)
+template <int TYPE, int TOK, bool KEEP>
 __global__ void __launch_bounds__(rd::kThreads, 2)
 route_decode_kernel(const __grid_constant__ RouteDecodeArgs a) {
     const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31u, layer = blockIdx.y;
@@ -181,10 +182,41 @@ route_decode_kernel(const __grid_constant__ RouteDecodeArgs a) {
         dequant8<TYPE>(2 * pair + 1 < d.n_expert ? row0 + rb : row0, k, w1);
     };
     if (once && lane < units_w) rows(p0, lane);
+    constexpr int kKept = KEEP ? TOK : 1;
+    double xd[kKept][8];
+    if (KEEP && lane < units_w) {
+        const uint32_t k = (warp * units_w + lane) * 8;
+        float4 xa[kKept], xb[kKept];
+#pragma unroll
+        for (int j = 0; j < kKept; ++j) {
+            const float* xt = x + (size_t)min(t0 + j, T - 1) * d.n_embd + k;
+            xa[j] = *reinterpret_cast<const float4*>(xt);
+            xb[j] = *reinterpret_cast<const float4*>(xt + 4);
+        }
+#pragma unroll
+        for (int j = 0; j < kKept; ++j) {
+            xd[j][0] = xa[j].x; xd[j][1] = xa[j].y; xd[j][2] = xa[j].z; xd[j][3] = xa[j].w;
+            xd[j][4] = xb[j].x; xd[j][5] = xb[j].y; xd[j][6] = xb[j].z; xd[j][7] = xb[j].w;
+        }
+    }
     for (uint32_t pair = p0; pair < p1; ++pair) {
         double acc[NV];   // [expert 0: tokens][expert 1: tokens]
 #pragma unroll
         for (int j = 0; j < NV; ++j) acc[j] = 0.0;
+        if (KEEP) {
+            if (lane < units_w) {
+                float c0[8], c1[8];
+#pragma unroll
+                for (int i = 0; i < 8; ++i) { c0[i] = w0[i]; c1[i] = w1[i]; }
+                if (pair + 1 < p1) rows(pair + 1, lane);
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    const double v0 = c0[i], v1 = c1[i];
+#pragma unroll
+                    for (int j = 0; j < kKept; ++j) { acc[j] += v0 * xd[j][i]; acc[TOK + j] += v1 * xd[j][i]; }
+                }
+            }
+        } else
         for (uint32_t u = lane; u < units_w; u += 32) {
             const uint32_t k = (warp * units_w + u) * 8;
             if (!once) rows(pair, u);
@@ -289,17 +321,29 @@ bool route_decode_ok(const qkm_dims& d, uint32_t n_tokens, size_t scratch_bytes)
 // Tokens of a group: as few as the batch has (a group of eight costs one token as much as eight).  Pairs a block: one while the blocks
 // find room on the SMs at once (a chain of latencies: start-up, loads, ticket), more when layers go together, so that a block's share of that chain is
 // small: 40 layers of 16 tokens 159 us with one pair a block, 125 so.
+// Blocks of several pairs keep the x of up to four tokens as doubles (the converter takes 16 lanes a cycle and SM, the f64 units 64): 24 layers of
+// one token 124 -> 119 us for the whole call, 40 layers of 16 tokens 2,066 -> 2,031 as groups of four, 12 of 64 1,970 -> 1,934.  With one pair a block
+// there is nothing to keep it for (a step of 3 tokens 341 -> 348 us), and below kFour pairs two groups of four are more blocks than one of eight is worth
+// (24 layers of 5 tokens 541 -> 554).
+template <int TYPE, int TOK, bool KEEP>
+static cudaError_t route_launch(const Launch& L, const RouteDecodeArgs& a, uint32_t groups) {
+    const uint32_t pairs = (a.d.n_expert + 1) / 2;
+    const dim3 grid((pairs + a.pairs_per_block - 1) / a.pairs_per_block * groups + a.n_tokens, a.n_layers);
+    return launch_kernel(L, route_decode_kernel<TYPE, TOK, KEEP>, grid, dim3(rd::kThreads), 0, a);
+}
 template <int TYPE>
 static cudaError_t route_launch(const Launch& L, RouteDecodeArgs a) {
-    const uint32_t T = a.n_tokens, tok = T <= 1 ? 1 : T <= 2 ? 2 : T <= 4 ? 4 : 8, groups = (T + tok - 1) / tok, pairs = (a.d.n_expert + 1) / 2;
-    const uint32_t per = pairs * groups * a.n_layers / 600;
+    constexpr uint32_t kFour = 4800;
+    const uint32_t T = a.n_tokens, pairs = (a.d.n_expert + 1) / 2;
+    const bool fits = a.d.n_embd <= 2048, four = fits && T > 8 && pairs * ((T + 3) / 4) * a.n_layers >= kFour;
+    const uint32_t tok = T <= 1 ? 1 : T <= 2 ? 2 : T <= 4 || four ? 4 : 8, groups = (T + tok - 1) / tok, per = pairs * groups * a.n_layers / 600;
     a.pairs_per_block = per < 1 ? 1 : per < 16 ? per : 16;
-    const dim3 grid((pairs + a.pairs_per_block - 1) / a.pairs_per_block * groups + T, a.n_layers), block(rd::kThreads);
+    const bool keep = fits && a.pairs_per_block > 1;
     switch (tok) {
-        case 1: return launch_kernel(L, route_decode_kernel<TYPE, 1>, grid, block, 0, a);
-        case 2: return launch_kernel(L, route_decode_kernel<TYPE, 2>, grid, block, 0, a);
-        case 4: return launch_kernel(L, route_decode_kernel<TYPE, 4>, grid, block, 0, a);
-        default: return launch_kernel(L, route_decode_kernel<TYPE, 8>, grid, block, 0, a);
+        case 1: return keep ? route_launch<TYPE, 1, true>(L, a, groups) : route_launch<TYPE, 1, false>(L, a, groups);
+        case 2: return keep ? route_launch<TYPE, 2, true>(L, a, groups) : route_launch<TYPE, 2, false>(L, a, groups);
+        case 4: return keep ? route_launch<TYPE, 4, true>(L, a, groups) : route_launch<TYPE, 4, false>(L, a, groups);
+        default: return route_launch<TYPE, 8, false>(L, a, groups);
     }
 }
 cudaError_t launch_route_decode(const Launch& L, uint32_t router_type, const RouteDecodeArgs& a) {

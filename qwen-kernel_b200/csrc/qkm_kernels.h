@@ -69,7 +69,7 @@ struct MmaItem {
 // ---- fused decode sequence (qkm_dec_route.cu, qkm_dec_gateup.cu, qkm_dec_down.cu) ---------------
 // Several layers whose rows are at hand together go through one launch of each kernel; everything per layer lies one after the other,
 // `n_tokens` (and so on) apart.
-constexpr uint32_t kDecMaxLayers = 64, kDecCounters = 16;
+constexpr uint32_t kDecMaxLayers = 64, kDecCounters = 20;
 // One expert (or the shared expert) with up to two of the tokens routed to it.  The gate/up kernel walks all n_ff rows of a group.
 struct alignas(16) DecodeGroup {
     uint32_t head;     // expert | tokens (1 or 2) << 16 | shared << 24

@@ -49,6 +49,17 @@ def test_stack_layers_together(pkg, orc, syn, n_embd, n_expert, n_used, gt, dt, 
     check(syn, orc, layers, x, y, sel)
 
 
+# router blocks of several pairs of experts, which keep up to four tokens' x: one, two and four tokens a group, the last group and the last block's pairs
+# not full, an odd number of experts, part of the lanes idle (512 columns) and none (2048)
+@pytest.mark.parametrize("n_embd,n_expert,T,L", [(512, 511, 1, 5), (512, 512, 2, 5), (512, 511, 4, 6), (512, 510, 3, 6), (512, 511, 13, 5), (2048, 64, 64, 10)])
+def test_stack_router_blocks_of_several_pairs(pkg, orc, syn, n_embd, n_expert, T, L):
+    dims = syn.Dims(n_embd=n_embd, n_ff=256, n_expert=n_expert, n_used=8)
+    layers = [syn.make_layer(dims, seed=240, router_type=T & 1)] * L
+    x = np.stack([syn.random_x(T, n_embd, seed=250 + l) for l in range(L)])
+    y, sel = run_stack(pkg, syn, dims, layers, x)
+    check(syn, orc, layers, x, y, sel)
+
+
 def test_stack_of_several_types(pkg, orc, syn):
     """Runs of layers of the same types; a run of one layer."""
     dims = syn.Dims(n_embd=1024, n_ff=512, n_expert=16, n_used=4)
