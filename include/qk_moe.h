@@ -236,9 +236,9 @@ QKM_API int qkm_moe_forward_host(qkm_ctx *c, uint32_t layer, int mode, const flo
  * together, unless x and y overlap without being the same array. */
 QKM_API int qkm_moe_decode_stack(qkm_ctx *c, uint32_t layer_first, uint32_t layer_count,
                                  const float *x, uint32_t n_tokens, float *y);
-/* The same with HOST buffers [layer_count][T][n_embd], then a stream synchronise.  From eight
- * layers on (and on a stream of the caller's) the stack runs in four chunks of layers (two layers,
- * two halves of the rest, two layers): all input
+/* The same with HOST buffers [layer_count][T][n_embd], then a stream synchronise.  From six
+ * layers and 1.5 MB of rows on (and on a stream of the caller's) the stack runs in three chunks of layers (a sixteenth, the
+ * rest, a sixteenth): all input
  * copies are queued at once on a copy stream, a chunk starts when its rows have arrived and its
  * outputs leave on a third stream while the next chunk computes.  Pinned host memory makes the
  * copies asynchronous. */

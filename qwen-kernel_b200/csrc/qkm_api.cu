@@ -122,7 +122,8 @@ struct qkm_ctx {
     } stack_graphs[kStackGraphs];
     uint64_t stack_clock = 0;
     // the host-buffer form of the stack copies chunk k+1 in and chunk k-1 out while chunk k computes
-    static constexpr int kStackChunks = 4;
+    static constexpr int kStackChunks = 3;
+    static constexpr size_t kStackChunkBytes = 3u << 19;   // rows below which the stack with host buffers is not cut, see qkm_moe_decode_stack_host
     cudaStream_t copy_in = nullptr, copy_out = nullptr;
     cudaEvent_t ev_in[kStackChunks] = {}, ev_out[kStackChunks] = {}, ev_copies = nullptr;
     void drop_stack_graphs() {
@@ -914,7 +915,7 @@ extern "C" QKM_API int qkm_moe_decode_stack_host(qkm_ctx* c, uint32_t first, uin
     }
     const size_t layer_elems = (size_t)n * c->cfg.dims.n_embd;
     const size_t bytes = (size_t)count * layer_elems * sizeof(float);
-    if (c->stream == nullptr || c->profiling || count < 2u * qkm_ctx::kStackChunks) {
+    if (c->stream == nullptr || c->profiling || bytes < qkm_ctx::kStackChunkBytes || count < 2u * qkm_ctx::kStackChunks) {
         QKM_CUDA(c, cudaMemcpyAsync(c->stack_x, x_host, bytes, cudaMemcpyHostToDevice, c->stream));
         if (int rc = qkm_moe_decode_stack(c, first, count, c->stack_x, n, c->stack_y)) return rc;
         QKM_CUDA(c, cudaMemcpyAsync(y_host, c->stack_y, bytes, cudaMemcpyDeviceToHost, c->stream));
@@ -922,7 +923,9 @@ extern "C" QKM_API int qkm_moe_decode_stack_host(qkm_ctx* c, uint32_t first, uin
     }
     // Chunks of layers: all input copies are queued on their own stream at once, chunk k computes as soon
     // as its rows are there, and its outputs leave on a third stream while chunk k+1 computes.  Only the
-    // first chunk's copy in and the last chunk's copy out are not hidden, so these two chunks are short.
+    // first chunk's copy in and the last chunk's copy out are not hidden, so these two chunks are short (a sixteenth: their layers
+    // take longer than the copies of the rest).  A chunk more costs about 25 us, since its layers do not go with the others', and a
+    // copy that is not hidden 1 us per 55 KB: below 1.5 MB the whole stack is one chunk.
     if (!c->ev_copies) {   // made last; what an earlier try got is kept
         for (cudaStream_t* s : {&c->copy_in, &c->copy_out}) if (!*s) QKM_CUDA(c, cudaStreamCreateWithFlags(s, cudaStreamNonBlocking));
         for (cudaEvent_t& ev : c->ev_in) if (!ev) QKM_CUDA(c, cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
@@ -930,9 +933,8 @@ extern "C" QKM_API int qkm_moe_decode_stack_host(qkm_ctx* c, uint32_t first, uin
         QKM_CUDA(c, cudaEventCreateWithFlags(&c->ev_copies, cudaEventDisableTiming));
     }
     constexpr uint32_t K = qkm_ctx::kStackChunks;
-    // two layers first and two last (what is not hidden is their copy in and copy out), the rest in halves
-    static_assert(K == 4, "chunk boundaries below are written for four chunks");
-    const uint32_t lo[K + 1] = {0u, 2u, 2u + (count - 4u) / 2u, count - 2u, count};
+    static_assert(K == 3, "chunk boundaries below are written for three chunks");
+    const uint32_t ends = (count + 15u) / 16u, lo[K + 1] = {0u, ends, count - ends, count};
     // whatever the stream still holds (it reads or writes the staging buffers) comes first
     QKM_CUDA(c, cudaEventRecord(c->ev_copies, c->stream));
     QKM_CUDA(c, cudaStreamWaitEvent(c->copy_in, c->ev_copies, 0));

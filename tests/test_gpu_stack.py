@@ -113,3 +113,26 @@ def test_stack_nonfinite_and_large_rows(pkg, orc, syn, gt, dt):
         ref = orc.moe_layer(layers[l], x[l][ok[l]], threads=orc.hardware_threads())
         assert syn.rel_err_rows(y[l][ok[l]], ref["y"]) < TOL_F32
         assert np.isnan(y[l][~ok[l]]).all()
+
+
+def test_host_buffers_in_chunks(pkg, syn):
+    """From 1.5 MB of rows on the host-buffer form runs in three chunks of layers, the copies on streams of their own: the same results as the
+    device form, on a repeated call too, and one layer less than chunks need takes one copy each way."""
+    import torch
+    dims, T, L = syn.Dims(n_embd=512, n_ff=256, n_expert=16, n_used=4), 64, 14
+    x = np.stack([syn.random_x(T, dims.n_embd, seed=300 + l) for l in range(L)])
+    assert x.nbytes >= 3 << 19 and x[:5].nbytes < 3 << 19
+    with pkg.Context(dims, n_layer=L, max_tokens=T, device=0) as ctx:
+        for l in range(L):
+            ctx.upload_layer(l, syn.make_layer(dims, seed=301, layer=l))
+        stream = torch.cuda.Stream(torch.device("cuda", 0))
+        ctx.set_stream(stream.cuda_stream)
+        d_x, d_y = ctx.to_device(x), ctx.alloc(x.nbytes)
+        ctx.moe_decode_stack(0, L, d_x, T, d_y)
+        want = d_y.download(np.float32, x.shape)
+        for n in (L, L, 5):
+            y = np.zeros_like(x[:n])
+            ctx.moe_decode_stack_host(0, n, x.ctypes.data, T, y.ctypes.data)
+            for l in range(n):   # (64 tokens of a batch: the same kernels, other shares of the list and so another order of some sums at most)
+                assert syn.rel_err_rows(y[l], want[l]) < 1e-6
+        ctx.set_stream(0)
