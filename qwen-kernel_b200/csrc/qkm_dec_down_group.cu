@@ -88,7 +88,7 @@ decode_down_group_kernel(const __grid_constant__ DownDecodeArgs a) {
     if (warp == 0) layer_cuts(s_cuts, a.groups, a.n_tokens, a.n_layers, 1, 1);
     __syncthreads();
     uint32_t left;   // tiles still to do
-    ListPlace at = list_share(s_cuts, a.n_tokens, a.n_layers, by_tiles, 1, 1, team_global, by_teams, left);
+    ListPlace at = list_share(s_cuts, a.n_tokens, a.n_layers, by_tiles, 1, Divisor(1), team_global, by_teams, left);
     auto group = [&](const ListPlace& p) { return decode_group(a.groups, a.n_tokens, d.n_used, p.l, p.gi); };
     const size_t mat_tiles = (size_t)KB * RT;
 

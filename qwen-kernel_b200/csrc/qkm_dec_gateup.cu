@@ -61,7 +61,8 @@ constexpr uint32_t kRed4 = kRings4 + kWarps * kRingBytes4;
 constexpr uint32_t kEnd4 = kRed4 + kWarps * 2 * kRedFloats * 4 + 128;
 constexpr int kQ8Quarter = 2 * 544;                 // two 32-column blocks of a Q8_0 tile: d and quants of 16 rows each
 constexpr uint32_t kFewGroups = 64;                 // so many groups are read together with their number
-constexpr uint32_t kCostRouted = 8, kCostShared = 10;   // relative time of a routed / a shared tile (40 layers of 16 tokens with 9: 1,895 us, 10: 1,867, 11: 1,878)
+// relative time of a routed / a shared tile: of one layer, and of several together (40 layers of 16 tokens with 9: 1,895 us, 10: 1,867, 11: 1,878)
+constexpr uint32_t kCostRouted = 8, kCostShared1 = 11, kCostShared = 10;
 }  // namespace dg
 
 size_t decode_gateup_lut_bytes() { return dg::kTabBytes; }
@@ -227,7 +228,8 @@ decode_gateup_kernel(const __grid_constant__ GateupDecodeArgs a) {
     }
 
     const uint32_t teams_total = gridDim.x * n_teams, team_global = blockIdx.x * n_teams + team;
-    const Divisor by_teams(teams_total), by_tiles(RT);
+    const uint32_t cost_shared = a.n_layers == 1 ? dg::kCostShared1 : dg::kCostShared;
+    const Divisor by_teams(teams_total), by_tiles(RT), by_shared(cost_shared);
 
     // Up to here nothing depended on the router kernel, so a block scheduled early (programmatic
     // dependent launch) has its barriers and table copy under way while that kernel's tail runs.  The
@@ -238,13 +240,13 @@ decode_gateup_kernel(const __grid_constant__ GateupDecodeArgs a) {
     // This team's contiguous share of the flat list.  A shared-expert (Q8_0) tile takes longer
     // than a routed one (four ring stages, each a round trip), so the cut is made in cost units:
     // kCostRouted per routed tile, kCostShared per shared tile (a layer's shared groups come last).
-    if (warp == 0) layer_cuts(s_cuts, a.groups, a.n_tokens, a.n_layers, dg::kCostRouted, dg::kCostShared);
+    if (warp == 0) layer_cuts(s_cuts, a.groups, a.n_tokens, a.n_layers, dg::kCostRouted, cost_shared);
     // A few rows of one layer: the records come with the count, not one trip to L2 after it (unwritten ones are not looked at)
     const bool few = a.groups.group && a.n_layers == 1 && a.n_tokens * (d.n_used + 1) <= dg::kFewGroups;
     if (few && tid >= 64 && tid - 64 < a.n_tokens * (d.n_used + 1)) s_few[tid - 64] = __ldcg(reinterpret_cast<const uint4*>(a.groups.group) + (tid - 64));
     __syncthreads();
     uint32_t left;   // tiles still to do
-    ListPlace f_at = list_share(s_cuts, a.n_tokens, a.n_layers, by_tiles, dg::kCostRouted, dg::kCostShared, team_global, by_teams, left);   // next group to fetch
+    ListPlace f_at = list_share(s_cuts, a.n_tokens, a.n_layers, by_tiles, dg::kCostRouted, by_shared, team_global, by_teams, left);   // next group to fetch
     uint32_t rt = f_at.rt;   // the consumers' tile in its group
     // Lane 0 brings the records, two groups ahead of the consumers' (the producer is at most one group ahead of them: RT >= 4, two stages).
     // In shared memory, since a record in registers costs the IQ3_XXS form spills (50 us of 1950 at 40 layers of 16 tokens).

@@ -176,7 +176,7 @@ struct Divisor {
     }
 };
 // The warp's share of the list when it is cut into by_parts.d equal costs: its first place, and in `n` its tiles.  Even lanes look for the share's begin, odd ones for its end.  (A list's cost in tiles fits 32 bits: at most 768 rows.)
-__device__ __forceinline__ ListPlace list_share(const LayerCuts& c, uint32_t n_tokens, uint32_t n_layers, const Divisor& by_tiles, uint32_t routed, uint32_t shared, uint32_t part, const Divisor& by_parts,
+__device__ __forceinline__ ListPlace list_share(const LayerCuts& c, uint32_t n_tokens, uint32_t n_layers, const Divisor& by_tiles, uint32_t routed, const Divisor& by_shared, uint32_t part, const Divisor& by_parts,
                                                 uint32_t& n) {
     const uint32_t tiles = by_tiles.d, cut = part + (threadIdx.x & 1u), total = c.cost[n_layers] * tiles, q = by_parts(total);
     const uint32_t want = q * cut + by_parts((total - q * by_parts.d) * cut);   // total * cut / parts; in tiles times weight
@@ -187,7 +187,7 @@ __device__ __forceinline__ ListPlace list_share(const LayerCuts& c, uint32_t n_t
         else last = m - 1;
     }
     const uint32_t n_groups = c.groups[l + 1] - c.groups[l], n_routed = n_groups - (n_tokens + 1) / 2, left = want - c.cost[l] * tiles, r = n_routed * tiles * routed;
-    const uint32_t t = min(left <= r ? left / routed : n_routed * tiles + (left - r) / shared, n_groups * tiles);
+    const uint32_t t = min(left <= r ? left / routed : n_routed * tiles + by_shared(left - r), n_groups * tiles);
     const uint32_t at = c.groups[l] * tiles + t, gi = by_tiles(t);
     n = __shfl_sync(0xFFFFFFFFu, at, 1) - __shfl_sync(0xFFFFFFFFu, at, 0);
     return ListPlace{__shfl_sync(0xFFFFFFFFu, l, 0), __shfl_sync(0xFFFFFFFFu, gi, 0), __shfl_sync(0xFFFFFFFFu, t - gi * tiles, 0)};

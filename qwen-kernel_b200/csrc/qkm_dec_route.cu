@@ -318,7 +318,7 @@ bool route_decode_ok(const qkm_dims& d, uint32_t n_tokens, size_t scratch_bytes)
            (size_t)n_tokens * d.n_expert * sizeof(double) <= scratch_bytes;
 }
 
-// Tokens of a group: as few as the batch has (a group of eight costs one token as much as eight).  Pairs a block: one while the blocks
+// Tokens of a group: as few as the batch has (a group of eight costs one token as much as eight).  Pairs a block: one for a layer on its own and while the blocks
 // find room on the SMs at once (a chain of latencies: start-up, loads, ticket), more when layers go together, so that a block's share of that chain is
 // small: 40 layers of 16 tokens 159 us with one pair a block, 125 so.
 // Blocks of several pairs keep the x of up to four tokens as doubles (the converter takes 16 lanes a cycle and SM, the f64 units 64): 24 layers of
@@ -335,8 +335,8 @@ template <int TYPE>
 static cudaError_t route_launch(const Launch& L, RouteDecodeArgs a) {
     constexpr uint32_t kFour = 4800;
     const uint32_t T = a.n_tokens, pairs = (a.d.n_expert + 1) / 2;
-    const bool fits = a.d.n_embd <= 2048, four = fits && T > 8 && pairs * ((T + 3) / 4) * a.n_layers >= kFour;
-    const uint32_t tok = T <= 1 ? 1 : T <= 2 ? 2 : T <= 4 || four ? 4 : 8, groups = (T + tok - 1) / tok, per = pairs * groups * a.n_layers / 600;
+    const bool fits = a.d.n_embd <= 2048, four = fits && a.n_layers > 1 && T > 8 && pairs * ((T + 3) / 4) * a.n_layers >= kFour;
+    const uint32_t tok = T <= 1 ? 1 : T <= 2 ? 2 : T <= 4 || four ? 4 : 8, groups = (T + tok - 1) / tok, per = a.n_layers == 1 ? 1 : pairs * groups * a.n_layers / 600;
     a.pairs_per_block = per < 1 ? 1 : per < 16 ? per : 16;
     const bool keep = fits && a.pairs_per_block > 1;
     switch (tok) {
