@@ -219,7 +219,8 @@ cudaError_t alloc_decode(qkm_ctx* c) {
     const qkm_dims& d = c->cfg.dims;
     const uint32_t T = c->cfg.max_tokens < 64 ? c->cfg.max_tokens : 64;
     const uint64_t rows = c->ecount == d.n_expert ? (uint64_t)c->cfg.n_layer * T : 0;
-    c->dec_rows = rows < kDecRows ? (uint32_t)rows : kDecRows;
+    const uint32_t together = kDecRows < decode_gateup_rows((uint32_t)c->n_sms) ? kDecRows : decode_gateup_rows((uint32_t)c->n_sms), most = together < T ? T : together;
+    c->dec_rows = rows < most ? (uint32_t)rows : most;
     const size_t R = c->dec_rows, S = d.n_used + 1;
     const bool grouped = decode_down_group_ok(d) && (T >= 40 || !decode_down_any_ok(d));
     const Want want[] = {
@@ -646,7 +647,8 @@ static int decode_fused(qkm_ctx* c, uint32_t first, uint32_t count, const float*
     const qkm_layer_weights& w = c->layers[first].w;
     const qkm_dims& d = c->cfg.dims;
     const uint32_t nb = (uint32_t)c->n_sms;
-    const DecodeGroups groups{c->dec_counts, c->dec_groups};
+    // a layer on its own: the blocks of the kernels behind the router group its pairs themselves
+    const DecodeGroups groups = count == 1 ? DecodeGroups{} : DecodeGroups{c->dec_counts, c->dec_groups};
     RouteDecodeArgs ra{};
     GateupDecodeArgs ga{};
     DownDecodeArgs da{};
@@ -662,7 +664,7 @@ static int decode_fused(qkm_ctx* c, uint32_t first, uint32_t count, const float*
     ra.planes = c->dec_planes; ra.xscale = c->dec_xscale; ra.groups = groups; ra.n_tokens = n; ra.n_layers = count; ra.d = d;
     QKM_LAUNCH(c, launch_route_decode(c->Lchain(), w.router_type, ra));
     c->prof_mark("moe.route");
-    ga.luts = c->lut_gu; ga.planes = c->dec_planes; ga.xscale = c->dec_xscale; ga.groups = groups; ga.n_tokens = n; ga.n_layers = count;
+    ga.luts = c->lut_gu; ga.planes = c->dec_planes; ga.xscale = c->dec_xscale; ga.groups = groups; ga.sel = sel; ga.n_tokens = n; ga.n_layers = count;
     ga.gateup_type = w.gateup_type; ga.h = c->dec_h; ga.h_last = h; ga.status = c->status; ga.d = d;
     QKM_LAUNCH(c, launch_decode_gateup(c->Lchain(), ga, nb));
     c->prof_mark("moe.gu");

@@ -38,13 +38,17 @@ template <bool Q6> struct Cfg {
     static constexpr uint32_t kLow = 9;                                                   // IQ4_XS: rings below the table, up against it; the others above
     static constexpr uint32_t kScratch = Q6 ? kWarps * kRing : kHigh + (kWarps - kLow) * kRing;   // Q6_K: from the aligned start
     static constexpr uint32_t kRed = kScratch + kWarps * 1024;                            // digits of a warp's 256 columns, one token at a time
-    static constexpr uint32_t kEnd = kRed + kWarps * 2 * kGroupTiles * 16 * 2 * 4;        // [warp][buffer][tile][row][token]
+    static constexpr uint32_t kRedBytes = kWarps * 2 * kGroupTiles * 16 * 2 * 4;          // [warp][buffer][tile][row][token]
+    static constexpr uint32_t kList = kRed + kRedBytes;                                   // groups of a layer on its own
+    static constexpr uint32_t kEnd = kList + rk::kMaxGroups * sizeof(DecodeGroup);
+    static_assert(sizeof(OwnScratch) <= kRedBytes, "the grouping's working set lies where the partial sums come later");
     static constexpr uint32_t kDyn = Q6 ? kEnd + 128 : kEnd - 1024;                       // the first KB of the window is the system's
 };
 static_assert(Cfg<true>::kDyn <= 231000 && Cfg<false>::kDyn <= 231000 && kHalfQ8 <= kTileIq4, "with the static part at most 227 KB");
 }  // namespace dp
 
-template <bool Q6>
+// ONE: one layer, whose pairs the block groups itself; else the router kernel's lists
+template <bool Q6, bool ONE>
 __global__ void __launch_bounds__(dp::kWarps * 32, 1)
 decode_down_group_kernel(const __grid_constant__ DownDecodeArgs a) {
     using C = dp::Cfg<Q6>;
@@ -68,9 +72,13 @@ decode_down_group_kernel(const __grid_constant__ DownDecodeArgs a) {
     const uint32_t my_dig = base + C::kScratch + warp * 1024;
     uint8_t* dig = smem_raw + (my_dig - win0);
     float* red = reinterpret_cast<float*>(smem_raw + (base + C::kRed - win0));
+    DecodeGroup* own_list = reinterpret_cast<DecodeGroup*>(smem_raw + (base + C::kList - win0));
+    OwnScratch& own = *reinterpret_cast<OwnScratch*>(red);
+    const uint32_t n_layers = ONE ? 1 : a.n_layers;
     const uint32_t my_bar = smem_addr(&s_bar[warp * dp::kStages]), bar_tab = smem_addr(&s_bar[dp::kWarps * dp::kStages]);
     bool timed_out = false;
 
+    if (ONE) own.mask[tid] = 0ull;
     if (lane == 0) {
         for (uint32_t s = 0; s < dp::kStages; ++s) mbar_init(my_bar + 8 * s, 1);
         if (warp == 0) mbar_init(bar_tab, 1);
@@ -85,11 +93,18 @@ decode_down_group_kernel(const __grid_constant__ DownDecodeArgs a) {
     const Divisor by_teams(teams_total), by_tiles(RT);
 
     // the selection and its groups were final before the gate/up kernel released this one
-    if (warp == 0) layer_cuts(s_cuts, a.groups, a.n_tokens, a.n_layers, 1, 1);
-    __syncthreads();
+    if (ONE) {
+        own_groups<dp::kWarps * 32>(own, own_list, s_cuts, layer_sel(a, 0), d, a.n_tokens, 1, 1);
+    } else {
+        if (warp == 0) layer_cuts(s_cuts, a.groups, a.n_tokens, n_layers, 1, 1);
+        __syncthreads();
+    }
     uint32_t left;   // tiles still to do
-    ListPlace at = list_share(s_cuts, a.n_tokens, a.n_layers, by_tiles, 1, Divisor(1), team_global, by_teams, left);
-    auto group = [&](const ListPlace& p) { return decode_group(a.groups, a.n_tokens, d.n_used, p.l, p.gi); };
+    ListPlace at = list_share(s_cuts, a.n_tokens, n_layers, by_tiles, 1, Divisor(1), team_global, by_teams, left);
+    auto group = [&](const ListPlace& p) {
+        const uint4 v = ONE ? reinterpret_cast<const uint4*>(own_list)[p.gi] : __ldcg(reinterpret_cast<const uint4*>(decode_group_at(a.groups, a.n_tokens, d.n_used, p.l, p.gi)));
+        return DecodeGroup{v.x, {v.y, v.z}, v.w};
+    };
     const size_t mat_tiles = (size_t)KB * RT;
 
     // producer cursor; lane 0 only.  A routed tile is one stage, a shared tile two.
@@ -104,7 +119,7 @@ decode_down_group_kernel(const __grid_constant__ DownDecodeArgs a) {
             p_new = false;
             const DecodeGroup r = group(p_at);
             p_shared = r.shared();
-            p_src = p_shared ? a.layer[p_at.l].sh + ((size_t)kb * RT + p_at.rt) * kTileQ8 : a.layer[p_at.l].w + ((size_t)r.expert() * mat_tiles + (size_t)kb * RT + p_at.rt) * C::kTile;
+            p_src = p_shared ? a.layer[ONE ? 0 : p_at.l].sh + ((size_t)kb * RT + p_at.rt) * kTileQ8 : a.layer[ONE ? 0 : p_at.l].w + ((size_t)r.expert() * mat_tiles + (size_t)kb * RT + p_at.rt) * C::kTile;
         }
         const uint32_t n = p_shared ? dp::kHalfQ8 : C::kTile;
         mbar_expect_tx(my_bar + 8 * stage, n);
@@ -125,7 +140,7 @@ decode_down_group_kernel(const __grid_constant__ DownDecodeArgs a) {
     uint32_t stage = 0, phase = 0, e_n = 0, e_buf = 0;   // tiles waiting for the team's sum (the last e_n up to at.rt): count, buffer
     bool new_group = true, live = false;
     DecodeGroup rec{}, rec_next{};
-    if (left) rec_next = group(at);   // a group's record is read while the group before is worked on
+    if (!ONE && left) rec_next = group(at);   // a group's record is read while the group before is worked on
     size_t out = 0;                          // where this thread's sums of the current group go: (token, slot) of token slot lt & 1
     constexpr int NB = Q6 ? 2 : 1;
     uint32_t b0[NB][8], b1[NB][8];           // B operands (Q6_K: per token)
@@ -138,17 +153,21 @@ decode_down_group_kernel(const __grid_constant__ DownDecodeArgs a) {
     for (; left; --left) {
         if (new_group) {
             new_group = false;
-            rec = rec_next;
-            ListPlace after = at;
-            after.next_group(s_cuts);
-            if (after.l < a.n_layers) rec_next = group(after);
+            if (ONE) {
+                rec = group(at);
+            } else {
+                rec = rec_next;
+                ListPlace after = at;
+                after.next_group(s_cuts);
+                if (after.l < n_layers) rec_next = group(after);
+            }
             const bool shared = rec.shared();
-            const float* h = layer_h(a, at.l);
-            const qkm_sel* sel = layer_sel(a, at.l);
+            const float* h = layer_h(a, ONE ? 0 : at.l);
+            const qkm_sel* sel = layer_sel(a, ONE ? 0 : at.l);
             live = (lt & 1u) < rec.ntok();
             if (live) {
                 const uint32_t pr = rec.pair_of(lt & 1u);
-                out = ((size_t)(at.l * a.n_tokens + (pr >> 4)) * n_slots + (pr & 15u)) * d.n_embd;
+                out = ((size_t)((ONE ? 0 : at.l * a.n_tokens) + (pr >> 4)) * n_slots + (pr & 15u)) * d.n_embd;
             }
             float wt[2] = {0.f, 0.f};        // routing weight x plane scale
             float4 hv4[2][2];
@@ -340,22 +359,22 @@ bool decode_down_group_better(const qkm_dims& d, uint32_t type, uint32_t n) {
 }
 bool decode_down_group_ok(const qkm_dims& d) { return d.n_ff == 512 && d.n_used <= 15 && d.n_embd % 64 == 0 && d.n_expert <= rk::kMaxExperts; }
 
-template <bool Q6>
+template <bool Q6, bool ONE>
 static cudaError_t group_launch(const Launch& L, const DownDecodeArgs& a, uint32_t n_blocks) {
     const size_t smem = dp::Cfg<Q6>::kDyn;
-    if (const cudaError_t e = allow_dynamic_smem<decode_down_group_kernel<Q6>>((int)smem)) return e;
-    if (const cudaError_t e = launch_kernel(L, decode_down_group_kernel<Q6>, dim3(n_blocks), dim3(dp::kWarps * 32), smem, a)) return e;
+    if (const cudaError_t e = allow_dynamic_smem<decode_down_group_kernel<Q6, ONE>>((int)smem)) return e;
+    if (const cudaError_t e = launch_kernel(L, decode_down_group_kernel<Q6, ONE>, dim3(n_blocks), dim3(dp::kWarps * 32), smem, a)) return e;
     const uint32_t n = a.n_layers * a.n_tokens * (a.d.n_embd / 4);
     const cudaError_t e = launch_kernel(L, decode_fold_kernel, dim3((n + 255) / 256), dim3(256), 0, (const float*)a.contrib, a.y, a.y_stride, a.d.n_used + 1, a.d.n_embd, a.n_tokens, n);
     L.count(2);
     return e != cudaSuccess ? e : cudaGetLastError();
 }
 cudaError_t launch_decode_down_group(const Launch& L, const DownDecodeArgs& a, uint32_t type, uint32_t n_blocks) {
-    if (!decode_down_group_ok(a.d) || !a.contrib || !a.groups.group || a.n_tokens > rk::kMaxTokens) return cudaErrorInvalidValue;
+    if (!decode_down_group_ok(a.d) || !a.contrib || (a.n_layers != 1 && !a.groups.group) || a.n_tokens > rk::kMaxTokens) return cudaErrorInvalidValue;
     if (a.n_tokens == 0) return cudaSuccess;
-    if (type == QKM_TYPE_Q6_K) return group_launch<true>(L, a, n_blocks);
+    if (type == QKM_TYPE_Q6_K) return a.n_layers == 1 ? group_launch<true, true>(L, a, n_blocks) : group_launch<true, false>(L, a, n_blocks);
     if (type != QKM_TYPE_IQ4_XS || !a.lut) return cudaErrorInvalidValue;
-    return group_launch<false>(L, a, n_blocks);
+    return a.n_layers == 1 ? group_launch<false, true>(L, a, n_blocks) : group_launch<false, false>(L, a, n_blocks);
 }
 
 }  // namespace qkm

@@ -8,7 +8,7 @@
 //
 // Several layers whose rows are at hand together go through one launch: the list of work runs over all of them, so start-up, first
 // tiles and the uneven end are paid once (12 to 13 us of each kernel did not depend on the work: one layer of 16 tokens 41 us, 40 layers
-// together 27 us each).
+// together 27 us each).  A layer on its own takes a form without the other layers' bookkeeping.
 //
 // Work: the flat list of (layer, group, 16-row tile) - a group is an expert with up to two
 // tokens, n_ff / 16 tiles each - is cut evenly and contiguously over teams of KB = n_embd / 256
@@ -54,13 +54,14 @@ constexpr int kGroupTiles = 4;                      // tiles between two team-wi
 constexpr int kRedFloats = kGroupTiles * 16 * 2 * 2;   // per warp and buffer: tile, row, token, matrix
 constexpr uint32_t kHigh = kTab + kTabBytes;
 constexpr uint32_t kRed = kHigh + (kWarps - kLowRingWarps) * kRingBytes;
-constexpr uint32_t kEnd = kRed + kWarps * 2 * kRedFloats * 4;
+constexpr uint32_t kRedBytes = kWarps * 2 * kRedFloats * 4, kListBytes = rk::kMaxGroups * sizeof(DecodeGroup);   // the list: of a layer's groups, or of those in the teams' shares
+constexpr uint32_t kList = kRed + kRedBytes;
+static_assert(sizeof(OwnScratch) <= kRedBytes, "the grouping's working set lies where the partial sums come later");
 // IQ4_XS form, offsets from the (128-byte aligned) start of the dynamic area: barriers, rings, scratch
 constexpr uint32_t kRings4 = 1024;
 constexpr uint32_t kRed4 = kRings4 + kWarps * kRingBytes4;
-constexpr uint32_t kEnd4 = kRed4 + kWarps * 2 * kRedFloats * 4 + 128;
+constexpr uint32_t kList4 = kRed4 + kRedBytes;
 constexpr int kQ8Quarter = 2 * 544;                 // two 32-column blocks of a Q8_0 tile: d and quants of 16 rows each
-constexpr uint32_t kFewGroups = 64;                 // so many groups are read together with their number
 // relative time of a routed / a shared tile: of one layer, and of several together (40 layers of 16 tokens with 9: 1,895 us, 10: 1,867, 11: 1,878)
 constexpr uint32_t kCostRouted = 8, kCostShared1 = 11, kCostShared = 10;
 }  // namespace dg
@@ -184,15 +185,14 @@ __device__ __forceinline__ void q8_quarter(uint32_t q, uint32_t lane, uint32_t g
     }
 }
 
-template <bool IQ4>
+// ONE: one layer, whose pairs the block groups itself (from a.sel; NULL: the shared expert's groups only); else the router kernel's lists
+template <bool IQ4, bool ONE>
 __global__ void __launch_bounds__(dg::kWarps * 32, 1)
 decode_gateup_kernel(const __grid_constant__ GateupDecodeArgs a) {
     constexpr int kTileR = IQ4 ? kTileIq4 : kTileIq3;                       // routed tile bytes
     constexpr int kStageB = IQ4 ? dg::kStageBytes4 : dg::kStageBytes, kRingB = IQ4 ? dg::kRingBytes4 : dg::kRingBytes;
     extern __shared__ __align__(128) uint8_t smem_raw[];
     __shared__ LayerCuts s_cuts;
-    __shared__ uint4 s_few[dg::kFewGroups];
-    __shared__ uint4 s_rec[dg::kWarps][2];   // the records of the group a warp works on and of the next one
     const uint32_t base = smem_addr(smem_raw);
     const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31u, g = lane >> 2, t = lane & 3u;
     const qkm_dims d = a.d;
@@ -200,6 +200,7 @@ decode_gateup_kernel(const __grid_constant__ GateupDecodeArgs a) {
     const uint32_t n_teams = dg::kWarps / KB;
     const uint32_t team = warp / KB, kb = warp - team * KB;
     const uint32_t RT = d.n_ff / 16;              // tiles per group
+    const uint32_t team_threads = KB * 32, lt = tid - team * team_threads;
 
     const uint32_t base4 = (base + 127u) & ~127u;                        // IQ4_XS form: everything relative to here
     const uint32_t bar_base = IQ4 ? base4 : (base + 15u) & ~15u;         // kWarps * kStages ring barriers, then the table's
@@ -213,9 +214,12 @@ decode_gateup_kernel(const __grid_constant__ GateupDecodeArgs a) {
                         : warp < (uint32_t)dg::kLowRingWarps ? low_ring + warp * dg::kRingBytes
                                                              : dg::kHigh + (warp - dg::kLowRingWarps) * dg::kRingBytes;
     float* red = reinterpret_cast<float*>(smem_raw + ((IQ4 ? base4 + dg::kRed4 : dg::kRed) - base));
+    DecodeGroup* own_list = reinterpret_cast<DecodeGroup*>(smem_raw + ((IQ4 ? base4 + dg::kList4 : dg::kList) - base));
+    OwnScratch& own = *reinterpret_cast<OwnScratch*>(red);
     const uint32_t my_bar = bar_base + warp * dg::kStages * 8;
     bool timed_out = false;
 
+    if (ONE) own.mask[tid] = 0ull;
     if (lane == 0) {
         for (int s = 0; s < dg::kStages; ++s) mbar_init(my_bar + 8 * s, 1);
         if (warp == 0) mbar_init(tab_bar, 1);
@@ -228,7 +232,7 @@ decode_gateup_kernel(const __grid_constant__ GateupDecodeArgs a) {
     }
 
     const uint32_t teams_total = gridDim.x * n_teams, team_global = blockIdx.x * n_teams + team;
-    const uint32_t cost_shared = a.n_layers == 1 ? dg::kCostShared1 : dg::kCostShared;
+    const uint32_t n_layers = ONE ? 1 : a.n_layers, cost_shared = ONE ? dg::kCostShared1 : dg::kCostShared;
     const Divisor by_teams(teams_total), by_tiles(RT), by_shared(cost_shared);
 
     // Up to here nothing depended on the router kernel, so a block scheduled early (programmatic
@@ -240,32 +244,33 @@ decode_gateup_kernel(const __grid_constant__ GateupDecodeArgs a) {
     // This team's contiguous share of the flat list.  A shared-expert (Q8_0) tile takes longer
     // than a routed one (four ring stages, each a round trip), so the cut is made in cost units:
     // kCostRouted per routed tile, kCostShared per shared tile (a layer's shared groups come last).
-    if (warp == 0) layer_cuts(s_cuts, a.groups, a.n_tokens, a.n_layers, dg::kCostRouted, cost_shared);
-    // A few rows of one layer: the records come with the count, not one trip to L2 after it (unwritten ones are not looked at)
-    const bool few = a.groups.group && a.n_layers == 1 && a.n_tokens * (d.n_used + 1) <= dg::kFewGroups;
-    if (few && tid >= 64 && tid - 64 < a.n_tokens * (d.n_used + 1)) s_few[tid - 64] = __ldcg(reinterpret_cast<const uint4*>(a.groups.group) + (tid - 64));
-    __syncthreads();
+    if (ONE) {
+        own_groups<dg::kWarps * 32>(own, own_list, s_cuts, a.sel, d, a.n_tokens, dg::kCostRouted, cost_shared);
+    } else {
+        if (warp == 0) layer_cuts(s_cuts, a.groups, a.n_tokens, n_layers, dg::kCostRouted, cost_shared);
+        __syncthreads();
+    }
     uint32_t left;   // tiles still to do
-    ListPlace f_at = list_share(s_cuts, a.n_tokens, a.n_layers, by_tiles, dg::kCostRouted, by_shared, team_global, by_teams, left);   // next group to fetch
-    uint32_t rt = f_at.rt;   // the consumers' tile in its group
-    // Lane 0 brings the records, two groups ahead of the consumers' (the producer is at most one group ahead of them: RT >= 4, two stages).
-    // In shared memory, since a record in registers costs the IQ3_XXS form spills (50 us of 1950 at 40 layers of 16 tokens).
-    const uint32_t my_rec = smem_addr(&s_rec[warp][0]);
-    auto fetch = [&](uint32_t slot) {
-        if (f_at.l >= a.n_layers) return;
-        if (few) s_rec[warp][slot] = s_few[f_at.gi];
-        else if (a.groups.group) ldgsts16(my_rec + 16 * slot, a.groups.group + (size_t)f_at.l * a.n_tokens * (d.n_used + 1) + f_at.gi);
-        else {
-            const DecodeGroup r = decode_group(a.groups, a.n_tokens, d.n_used, f_at.l, f_at.gi);
-            s_rec[warp][slot] = make_uint4(r.head, r.pair[0], r.pair[1], r.layer);
+    const ListPlace at = list_share(s_cuts, a.n_tokens, n_layers, by_tiles, dg::kCostRouted, by_shared, team_global, by_teams, left);
+    uint32_t rt = at.rt;   // the consumers' tile in its group
+    DecodeGroup* my_list = own_list + (ONE ? 0 : team * (rk::kMaxGroups / n_teams));   // ONE: the layer's groups; else the share's
+    if (!ONE) {   // they fit: decode_gateup_rows
+        const uint32_t first = s_cuts.groups[at.l] + at.gi, n = left ? by_tiles(rt + left + RT - 1) : 0;
+        for (uint32_t i = lt; i < n; i += team_threads) {
+            uint32_t l = at.l;
+            while (s_cuts.groups[l + 1] <= first + i) ++l;
+            reinterpret_cast<uint4*>(my_list)[i] = __ldcg(reinterpret_cast<const uint4*>(decode_group_at(a.groups, a.n_tokens, d.n_used, l, first + i - s_cuts.groups[l])));
         }
-        f_at.next_group(s_cuts);
-    };
-    auto record = [&](uint32_t slot) {
-        const uint4 v = lds128(my_rec + 16 * slot);
+        asm volatile("bar.sync %0, %1;" ::"r"(team + 1), "r"(team_threads) : "memory");
+    }
+    // (read again where it is needed: a record in registers costs the IQ3_XXS form spills, 50 us of 1950 at 40 layers of 16 tokens)
+    const uint32_t recs = smem_addr(my_list);
+    auto record = [&](uint32_t i) {
+        const uint4 v = lds128(recs + 16 * i);
         return DecodeGroup{v.x, {v.y, v.z}, v.w};
     };
-    uint32_t k = 0, p_k = 0;   // groups begun by the consumers, by the producer: their records' places
+    // (a record's place is computed when a group begins: counters cost the IQ3_XXS form spills, 2.5 % of its time)
+    const uint32_t total = (ONE ? at.gi * RT : 0) + rt + left;
     const size_t mat_tiles = (size_t)KB * RT;
 
     // producer cursor over (tile, quarter); lane 0 only.  A routed tile is one stage, a shared
@@ -280,9 +285,8 @@ decode_gateup_kernel(const __grid_constant__ GateupDecodeArgs a) {
         if (p_left == 0) return;
         if (p_new) {   // first call, or the previous group is finished
             p_new = false;
-            ldgsts_wait();
-            const DecodeGroup r = record(p_k++ & 1u);
-            const GateupDecodeArgs::Mats& m = a.layer[r.layer];
+            const DecodeGroup r = record((total - p_left) / RT);
+            const GateupDecodeArgs::Mats& m = a.layer[ONE ? 0 : r.layer];
             p_shared = r.shared();
             if (!p_shared) {
                 const size_t tile = (size_t)r.expert() * mat_tiles + (size_t)kb * RT + p_rt;
@@ -310,14 +314,11 @@ decode_gateup_kernel(const __grid_constant__ GateupDecodeArgs a) {
             if (++p_q == 4) { p_q = 0; p_g += kTileQ8; p_u += kTileQ8; next_tile(); }
         }
     };
-    if (lane == 0) {
-        if (left) { fetch(0); fetch(1); }
+    if (lane == 0)
         for (int s = 0; s < dg::kStages; ++s) issue(s);
-    }
 
     const uint32_t grid_c = dg::kTab + lane * 4;
     const uint32_t i_off = 64 * g + piece_at(g, t), s_off = 32 * g + 16 * ((t >> 1) ^ ((g >> 2) & 1u)) + 8 * (t & 1u);   // this lane's pieces of row g (rows g+8 alike)
-    const uint32_t team_threads = KB * 32, lt = tid - team * team_threads;
     uint32_t cnt = 0;   // stages consumed by this warp
     uint32_t b0[8], b1[8], n0[8], n1[8];
     float wcol0 = 0.f, wcol1 = 0.f;   // digit weights of the two C columns of this lane (2t, 2t+1)
@@ -331,17 +332,15 @@ decode_gateup_kernel(const __grid_constant__ GateupDecodeArgs a) {
     for (; left; --left) {
         if (new_group) {
             new_group = false;
-            if (lane == 0) ldgsts_wait();
-            __syncwarp();
-            const DecodeGroup rec = record(k & 1u);
+            const DecodeGroup rec = record((total - left) / RT);
             shared = rec.shared();
-            const uint32_t row0 = rec.layer * a.n_tokens;   // the layer's first row of the planes
+            const uint32_t row0 = ONE ? 0 : rec.layer * a.n_tokens;   // the layer's first row of the planes
             {
                 const uint32_t ets = lt & 1u;   // the reduction below gives this thread token slot (j & 1) == (lt & 1)
                 h = nullptr;
                 if (ets < rec.ntok()) {
                     const uint32_t pr = rec.pair_of(ets), tok = pr >> 4, slot = pr & 15u;
-                    h = (rec.layer + 1 == a.n_layers ? a.h_last : a.h + (size_t)row0 * (d.n_used + 1) * d.n_ff) + ((size_t)tok * (d.n_used + 1) + slot) * d.n_ff;
+                    h = (ONE || rec.layer + 1 == n_layers ? a.h_last : a.h + (size_t)row0 * (d.n_used + 1) * d.n_ff) + ((size_t)tok * (d.n_used + 1) + slot) * d.n_ff;
                 }
             }
             // B operand: column g of the MMA = (token slot g >> 2, digit g & 3); this warp's 256 columns
@@ -375,9 +374,6 @@ decode_gateup_kernel(const __grid_constant__ GateupDecodeArgs a) {
                 wcol0 = sc * w0;
                 wcol1 = sc * w0 * 128.f;
             }
-            __syncwarp();   // every lane has used its record
-            if (lane == 0) fetch(k & 1u);
-            ++k;
         }
         float ga, gb, ua, ub;
         // The token's other two digits sit in lane t^1.  The exchange comes before the stage is filled again: it needs what was read last, so
@@ -460,7 +456,6 @@ decode_gateup_kernel(const __grid_constant__ GateupDecodeArgs a) {
         }
         if (++rt == RT) { rt = 0; new_group = true; }
     }
-    if (lane == 0) ldgsts_wait();   // a record that the share did not get to
     if (timed_out && lane == 0) atomicExch(a.status, (uint32_t)kStatusWaitTimeout);
 }
 
@@ -469,23 +464,25 @@ bool decode_gateup_ok(const qkm_dims& d) {
     return d.n_embd % 256 == 0 && KB >= 2 && KB <= 8 && (KB & (KB - 1)) == 0 && d.n_ff % 64 == 0 && d.n_used <= 15;
 }
 
-cudaError_t launch_decode_gateup(const Launch& L, const GateupDecodeArgs& a, uint32_t n_blocks) {
-    if (!decode_gateup_ok(a.d)) return cudaErrorInvalidValue;
-    if (a.gateup_type == QKM_TYPE_IQ4_XS) {
-        const size_t smem4 = dg::kEnd4;
-        cudaError_t e4 = cudaFuncSetAttribute(decode_gateup_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem4);
-        if (e4 != cudaSuccess) return e4;
-        e4 = launch_kernel(L, decode_gateup_kernel<true>, dim3(n_blocks), dim3(dg::kWarps * 32), smem4, a);
-        L.count();
-        return e4 != cudaSuccess ? e4 : cudaGetLastError();
-    }
-    if (a.gateup_type != QKM_TYPE_IQ3_XXS) return cudaErrorInvalidValue;
-    const size_t smem = dg::kEnd;   // the dynamic area must reach from wherever it starts to the end of the scratch
-    cudaError_t e = cudaFuncSetAttribute(decode_gateup_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-    e = launch_kernel(L, decode_gateup_kernel<false>, dim3(n_blocks), dim3(dg::kWarps * 32), smem, a);
+template <bool IQ4, bool ONE>
+static cudaError_t gateup_launch(const Launch& L, const GateupDecodeArgs& a, uint32_t n_blocks) {
+    const size_t smem = (IQ4 ? dg::kList4 + 128 : dg::kList) + dg::kListBytes;   // IQ3_XXS: the dynamic area must reach the list's end from wherever it starts
+    if (const cudaError_t e = cudaFuncSetAttribute(decode_gateup_kernel<IQ4, ONE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)) return e;
+    const cudaError_t e = launch_kernel(L, decode_gateup_kernel<IQ4, ONE>, dim3(n_blocks), dim3(dg::kWarps * 32), smem, a);
     L.count();
     return e != cudaSuccess ? e : cudaGetLastError();
+}
+// The records of a team's share of several layers find room in its part of the list: at most so many (layer, token) rows.  (A row has up to 16
+// groups, and a share of routed tiles, the cheaper ones, has the most: one of n_teams * n_blocks shares gets at most
+// 16 rows * kCostShared / (n_teams * n_blocks * kCostRouted) groups and two begun ones, with 8 rows a block 160 / n_teams + 2 of 800 / n_teams.)
+uint32_t decode_gateup_rows(uint32_t n_blocks) { return 8 * n_blocks; }
+
+cudaError_t launch_decode_gateup(const Launch& L, const GateupDecodeArgs& a, uint32_t n_blocks) {
+    if (!decode_gateup_ok(a.d) || a.n_tokens > rk::kMaxTokens || a.n_layers > kDecMaxLayers) return cudaErrorInvalidValue;
+    if (a.n_layers != 1 && (!a.groups.group || a.n_layers * a.n_tokens > decode_gateup_rows(n_blocks))) return cudaErrorInvalidValue;
+    if (a.gateup_type != QKM_TYPE_IQ3_XXS && a.gateup_type != QKM_TYPE_IQ4_XS) return cudaErrorInvalidValue;
+    if (a.gateup_type == QKM_TYPE_IQ4_XS) return a.n_layers == 1 ? gateup_launch<true, true>(L, a, n_blocks) : gateup_launch<true, false>(L, a, n_blocks);
+    return a.n_layers == 1 ? gateup_launch<false, true>(L, a, n_blocks) : gateup_launch<false, false>(L, a, n_blocks);
 }
 
 }  // namespace qkm

@@ -1,8 +1,11 @@
 // Ranking of f64 router logits (one warp per token) and the list of work that the kernels which go by expert walk, for decode-sized
 // batches of one or more layers.
 //
-// The router kernel ranks a group of tokens in the block that finishes the group's logits last; the block that ranks a layer's
-// last tokens groups the layer's pairs.
+// The router kernel ranks a group of tokens in the block that finishes the group's logits last.  Of layers that go together, the block
+// that ranks a layer's last tokens groups its pairs for the kernels behind.  A layer on its own is grouped by each block of those kernels
+// for itself: one block at the router's end, the lists' way through the L2 and their reads there are a chain that nothing hides, 3 to 6 us of
+// a layer (a decode step of 256 experts, top 8: 1 token 27.0 -> 24.6 us, 16: 80.7 -> 74.1, 64: 182.1 -> 170.3; of 512, top 10: 3 tokens 42.6 ->
+// 40.6, 64: 252.6 -> 247.0).
 //
 // Rules (the reference's): top n_used by raw logit, lowest id on ties
 // (shaders/moe_select_256.comp:60-61), non-finite logits at the floor -3.4e38
@@ -17,6 +20,7 @@ namespace qkm {
 
 namespace rk {
 constexpr uint32_t kMaxTokens = 64, kMaxExperts = 512;
+constexpr uint32_t kMaxGroups = (kMaxTokens * 16 + kMaxExperts) / 2 + kMaxTokens / 2;   // of a layer: 800
 constexpr float kFloor = -3.4e38f;
 }  // namespace rk
 
@@ -123,27 +127,18 @@ struct LayerCuts {
     uint32_t groups[kDecMaxLayers + 1];   // first group of each layer
     uint32_t cost[kDecMaxLayers + 1];     // and what the groups before it cost, in tiles of a routed group times its weight
 };
-// group `gi` of layer `l`; past the end of the layer's list: the shared expert's groups when there is no list
-__device__ __forceinline__ DecodeGroup decode_group(const DecodeGroups& g, uint32_t n_tokens, uint32_t n_used, uint32_t l, uint32_t gi) {
-    if (g.group) {
-        const uint4 v = __ldcg(reinterpret_cast<const uint4*>(g.group + (size_t)l * n_tokens * (n_used + 1) + gi));
-        return DecodeGroup{v.x, {v.y, v.z}, v.w};
-    }
-    return DecodeGroup{DecodeGroup::make_head(0, min(2u, n_tokens - 2 * gi), 1), {((2 * gi) << 4) | n_used, (min(2 * gi + 1, n_tokens - 1) << 4) | n_used}, l};
+// group `gi` of layer `l`
+__device__ __forceinline__ const DecodeGroup* decode_group_at(const DecodeGroups& g, uint32_t n_tokens, uint32_t n_used, uint32_t l, uint32_t gi) {
+    return g.group + (size_t)l * n_tokens * (n_used + 1) + gi;
 }
 // By one warp: a routed group costs `routed`, a shared one `shared` (relative, per tile).
 __device__ __forceinline__ void layer_cuts(LayerCuts& c, const DecodeGroups& g, uint32_t n_tokens, uint32_t n_layers, uint32_t routed, uint32_t shared) {
     const uint32_t lane = threadIdx.x & 31u, n_shared = (n_tokens + 1) / 2;
-    if (n_layers == 1) {   // (without the sums: they are in the way of the first tile)
-        const uint32_t n = g.group ? __ldcg(g.count) : n_shared;
-        if (lane == 0) { c.groups[0] = 0; c.cost[0] = 0; c.groups[1] = n; c.cost[1] = (n - n_shared) * routed + n_shared * shared; }
-        return;
-    }
     uint32_t groups = 0, cost = 0;   // of the layers before
     if (lane == 0) { c.groups[0] = 0; c.cost[0] = 0; }
     for (uint32_t l0 = 0; l0 < n_layers; l0 += 32) {
         uint32_t n = 0;
-        if (l0 + lane < n_layers) n = g.group ? __ldcg(g.count + l0 + lane) : n_shared;
+        if (l0 + lane < n_layers) n = __ldcg(g.count + l0 + lane);
         uint32_t k = l0 + lane < n_layers ? (n - n_shared) * routed + n_shared * shared : 0u;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
@@ -155,12 +150,87 @@ __device__ __forceinline__ void layer_cuts(LayerCuts& c, const DecodeGroups& g, 
         cost += __shfl_sync(0xFFFFFFFFu, k, 31);
     }
 }
+// ---- a layer's (token, slot) pairs grouped by expert ----
+// token t chose expert e in place `slot`
+__device__ __forceinline__ void choose(unsigned long long* s_mask, uint16_t* s_ids, uint32_t t, uint32_t slot, uint32_t e) {
+    s_ids[t * 16 + slot] = (uint16_t)e;
+    atomicOr(reinterpret_cast<uint32_t*>(s_mask) + 2 * e + (t >> 5), 1u << (t & 31u));   // bit t of the expert's 64
+}
+// By a block of THREADS: writes the layer's groups, returns how many.  s_ids[t][16]: the layer's selection; s_mask: the tokens that chose each
+// expert; np: pairs in them (T * n_used, or none: the shared expert's groups only); s_first, s_sum: scratch for an entry an
+// expert and a warp.  groups: in global or in the block's shared memory.
+template <uint32_t THREADS>
+__device__ __forceinline__ uint32_t group_pairs(DecodeGroup* groups, uint32_t* s_first, uint32_t* s_sum, const uint16_t* s_ids, const unsigned long long* s_mask,
+                                                uint32_t n_used, uint32_t np, uint32_t T, uint32_t layer) {
+    constexpr int PER = rk::kMaxExperts / THREADS;
+    static_assert(PER * THREADS == rk::kMaxExperts, "whole experts a thread");
+    const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31u, n_shared = (T + 1) / 2;
+    uint32_t c[PER], v = 0;   // tokens of this thread's experts; groups up to the last one
+#pragma unroll
+    for (int h = 0; h < PER; ++h) { c[h] = (uint32_t)__popcll(s_mask[PER * tid + h]); v += (c[h] + 1) / 2; }
+    const uint32_t n = v;
+#pragma unroll
+    for (int i = 1; i < 32; i <<= 1) {
+        const uint32_t up = __shfl_up_sync(0xFFFFFFFFu, v, i);
+        if (lane >= (uint32_t)i) v += up;
+    }
+    if (lane == 31) s_sum[warp] = v;
+    __syncthreads();
+    uint32_t base = 0, total = 0;
+#pragma unroll
+    for (uint32_t w = 0; w < THREADS / 32; ++w) { if (w < warp) base += s_sum[w]; total += s_sum[w]; }
+    uint32_t first = base + v - n;
+#pragma unroll
+    for (int h = 0; h < PER; ++h) {
+        const uint32_t e = PER * tid + h;
+        s_first[e] = first;
+        for (uint32_t i = 0; 2 * i < c[h]; ++i, ++first) {
+            groups[first].head = DecodeGroup::make_head(e, min(2u, c[h] - 2 * i), 0);
+            groups[first].layer = layer;
+        }
+    }
+    // every token is one of the shared expert's pairs
+    for (uint32_t i = tid; i < n_shared; i += THREADS)
+        groups[total + i] = DecodeGroup{DecodeGroup::make_head(0, min(2u, T - 2 * i), 1), {((2 * i) << 4) | n_used, (min(2 * i + 1, T - 1) << 4) | n_used}, layer};
+    __syncthreads();
+    // a pair's rank inside its expert is the number of lower tokens that chose the expert
+    for (uint32_t p = tid; p < np; p += THREADS) {
+        const uint32_t t = p / n_used, s = p - t * n_used, e = s_ids[t * 16 + s];
+        const uint32_t r = (uint32_t)__popcll(s_mask[e] & ((1ull << t) - 1ull));
+        groups[s_first[e] + r / 2].pair[r & 1u] = (t << 4) | s;
+    }
+    return total + n_shared;
+}
+// Working set of own_groups, dead behind it.
+struct OwnScratch {
+    unsigned long long mask[rk::kMaxExperts];
+    uint32_t first[rk::kMaxExperts], sum[rk::kMaxExperts / 32];
+    uint16_t ids[rk::kMaxTokens * 16];
+};
+// A layer on its own: the block's list of its groups, and the list's cuts, from the tokens' records (NULL: the shared expert's
+// groups only).  By a block of THREADS with S.mask zero; ends with a barrier.
+template <uint32_t THREADS>
+__device__ __forceinline__ void own_groups(OwnScratch& S, DecodeGroup* list, LayerCuts& cuts, const qkm_sel* sel, const qkm_dims& d, uint32_t T, uint32_t routed, uint32_t shared) {
+    constexpr uint32_t PER = rk::kMaxTokens * 16 / THREADS;
+    uint32_t id[PER];
+#pragma unroll
+    for (uint32_t k = 0; k < PER; ++k) {
+        const uint32_t i = threadIdx.x + k * THREADS;
+        if (sel && i < T * 16) id[k] = __ldcg(&sel[i >> 4].ids[i & 15u]);
+    }
+#pragma unroll
+    for (uint32_t k = 0; k < PER; ++k) {
+        const uint32_t i = threadIdx.x + k * THREADS;
+        if (sel && i < T * 16 && (i & 15u) < d.n_used) choose(S.mask, S.ids, i >> 4, i & 15u, min(id[k], d.n_expert - 1));
+    }
+    __syncthreads();
+    const uint32_t n = group_pairs<THREADS>(list, S.first, S.sum, S.ids, S.mask, d.n_used, sel ? T * d.n_used : 0, T, 0), n_shared = (T + 1) / 2;
+    if (threadIdx.x == 0) { cuts.groups[0] = 0; cuts.cost[0] = 0; cuts.groups[1] = n; cuts.cost[1] = (n - n_shared) * routed + n_shared * shared; }
+    __syncthreads();
+}
 // A place in the list: layer, group of the layer, tile of the group.  `tiles` tiles a group.
 struct ListPlace {
     uint32_t l, gi, rt;
-    __device__ __forceinline__ void next(const LayerCuts& c, uint32_t tiles) {
-        if (++rt == tiles) { rt = 0; next_group(c); }
-    }
     __device__ __forceinline__ void next_group(const LayerCuts& c) {
         if (++gi == c.groups[l + 1] - c.groups[l]) { gi = 0; ++l; }
     }
@@ -175,7 +245,8 @@ struct Divisor {
         return q + (x - q * d >= d ? 1u : 0u);
     }
 };
-// The warp's share of the list when it is cut into by_parts.d equal costs: its first place, and in `n` its tiles.  Even lanes look for the share's begin, odd ones for its end.  (A list's cost in tiles fits 32 bits: at most 768 rows.)
+// The warp's share of the list when it is cut into by_parts.d equal costs: its first place, and in `n` its tiles.  Even lanes
+// look for the share's begin, odd ones for its end.  (A list's cost in tiles fits 32 bits: at most 768 rows.)
 __device__ __forceinline__ ListPlace list_share(const LayerCuts& c, uint32_t n_tokens, uint32_t n_layers, const Divisor& by_tiles, uint32_t routed, const Divisor& by_shared, uint32_t part, const Divisor& by_parts,
                                                 uint32_t& n) {
     const uint32_t tiles = by_tiles.d, cut = part + (threadIdx.x & 1u), total = c.cost[n_layers] * tiles, q = by_parts(total);

@@ -40,58 +40,6 @@ __device__ __forceinline__ uint32_t ticket(uint32_t* counter) {
     asm volatile("atom.add.acq_rel.gpu.global.u32 %0, [%1], 1;" : "=r"(n) : "l"(counter) : "memory");
     return n;
 }
-// token t chose expert e in place `slot`
-__device__ __forceinline__ void choose(unsigned long long* s_mask, uint16_t* s_ids, uint32_t t, uint32_t slot, uint32_t e) {
-    s_ids[t * 16 + slot] = (uint16_t)e;
-    atomicOr(reinterpret_cast<uint32_t*>(s_mask) + 2 * e + (t >> 5), 1u << (t & 31u));   // bit t of the expert's 64
-}
-// Groups a layer's (token, slot) pairs by expert: a block of kThreads, two experts a thread; s_ids[t][16]: the layer's selection;
-// s_mask: the tokens that chose each expert.
-__device__ __forceinline__ void group_lists(const DecodeGroups& out, const uint16_t* s_ids, const unsigned long long* s_mask, const qkm_dims& d, uint32_t T, uint32_t layer) {
-    static_assert(rk::kMaxExperts == 2 * rd::kThreads, "two experts a thread");
-    __shared__ uint32_t s_sum[rd::kThreads / 32];
-    __shared__ uint32_t s_first[rk::kMaxExperts];   // first group of expert e
-    const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31u;
-    DecodeGroup* groups = out.group + (size_t)layer * T * (d.n_used + 1);
-    const uint32_t np = T * d.n_used;
-    uint32_t c[2], v = 0;   // tokens of this thread's experts; groups up to the second one
-#pragma unroll
-    for (int h = 0; h < 2; ++h) { c[h] = (uint32_t)__popcll(s_mask[2 * tid + h]); v += (c[h] + 1) / 2; }
-    const uint32_t n = v;
-#pragma unroll
-    for (int i = 1; i < 32; i <<= 1) {
-        const uint32_t up = __shfl_up_sync(0xFFFFFFFFu, v, i);
-        if (lane >= (uint32_t)i) v += up;
-    }
-    if (lane == 31) s_sum[warp] = v;
-    __syncthreads();
-    uint32_t base = 0, total = 0;
-#pragma unroll
-    for (uint32_t w = 0; w < rd::kThreads / 32; ++w) { if (w < warp) base += s_sum[w]; total += s_sum[w]; }
-    uint32_t first = base + v - n;
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-        const uint32_t e = 2 * tid + h;
-        s_first[e] = first;
-        for (uint32_t i = 0; 2 * i < c[h]; ++i, ++first) {
-            groups[first].head = DecodeGroup::make_head(e, min(2u, c[h] - 2 * i), 0);
-            groups[first].layer = layer;
-        }
-    }
-    // every token is one of the shared expert's pairs
-    for (uint32_t i = tid; i < (T + 1) / 2; i += rd::kThreads) {
-        groups[total + i] = DecodeGroup{DecodeGroup::make_head(0, min(2u, T - 2 * i), 1), {((2 * i) << 4) | d.n_used, (min(2 * i + 1, T - 1) << 4) | d.n_used}, layer};
-    }
-    if (tid == 0) out.count[layer] = total + (T + 1) / 2;
-    __syncthreads();
-    // a pair's rank inside its expert is the number of lower tokens that chose the expert
-    for (uint32_t p = tid; p < np; p += rd::kThreads) {
-        const uint32_t t = p / d.n_used, s = p - t * d.n_used, e = s_ids[t * 16 + s];
-        const uint32_t r = (uint32_t)__popcll(s_mask[e] & ((1ull << t) - 1ull));
-        groups[s_first[e] + r / 2].pair[r & 1u] = (t << 4) | s;
-    }
-}
-
 // TOK: tokens of a group; a.pairs_per_block: router row pairs that a logits block takes one after the other; KEEP: the tokens' x stays in
 // registers as doubles for all of them (n_embd <= 2048)
 template <int TYPE, int TOK, bool KEEP>
@@ -288,14 +236,15 @@ route_decode_kernel(const __grid_constant__ RouteDecodeArgs a) {
     if (tid == 0) *counter = 0;   // ready for the next launch
     __shared__ uint16_t s_ids[rk::kMaxTokens * 16];
     static_assert(TOK <= rd::kThreads / 32, "a warp ranks one token");
-    const bool ranks = warp < min((uint32_t)TOK, T - t0);
+    const bool ranks = warp < min((uint32_t)TOK, T - t0), lists = a.groups.group != nullptr;
     const uint32_t my_t = t0 + warp;
     Ranked mine{};
     if (ranks) {
         mine = rank_token(logits + (size_t)my_t * d.n_expert, d);
-        if (n_groups > 1) rank_store(mine, sel[my_t], d);
+        if (n_groups > 1 || !lists) rank_store(mine, sel[my_t], d);
         else if (lane < d.n_used) choose(s_mask, s_ids, my_t, lane, mine.id);
     }
+    if (!lists) return;
 
     // ---- and the block that ranks a layer's last token group groups the layer's pairs --------------
     if (n_groups > 1) {   // (the only group's ids are in shared memory)
@@ -309,7 +258,9 @@ route_decode_kernel(const __grid_constant__ RouteDecodeArgs a) {
             if ((i & 15u) < d.n_used) choose(s_mask, s_ids, i >> 4, i & 15u, min(__ldcg(&sel[i >> 4].ids[i & 15u]), d.n_expert - 1));
     }
     __syncthreads();
-    group_lists(a.groups, s_ids, s_mask, d, T, layer);
+    __shared__ uint32_t s_sum[rd::kThreads / 32], s_first[rk::kMaxExperts];
+    const uint32_t n = group_pairs<rd::kThreads>(a.groups.group + (size_t)layer * T * (d.n_used + 1), s_first, s_sum, s_ids, s_mask, d.n_used, T * d.n_used, T, layer);
+    if (tid == 0) a.groups.count[layer] = n;
     if (n_groups == 1 && ranks) rank_store(mine, sel[my_t], d);   // (after the lists: the next kernel waits for those)
 }
 

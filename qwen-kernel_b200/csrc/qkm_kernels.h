@@ -84,7 +84,7 @@ struct alignas(16) DecodeGroup {
 // A layer's (token, slot) pairs grouped by expert, ascending expert, then the shared expert's ceil(n_tokens / 2) groups
 struct DecodeGroups {
     uint32_t* count;       // [layer]
-    DecodeGroup* group;    // [layer][n_tokens * (n_used + 1)]; NULL: the shared expert's groups only
+    DecodeGroup* group;    // [layer][n_tokens * (n_used + 1)]
 };
 struct RouteDecodeArgs {
     struct Router { const uint8_t* w; const float* gis; } layer[kDecMaxLayers];   // [n_expert][n_embd] F32 or F16; [n_embd]
@@ -95,7 +95,7 @@ struct RouteDecodeArgs {
     uint32_t* counter;         // [layer][kDecCounters] zero words; left at zero
     int8_t* planes;            // out [layer][n_tokens][n_embd/256][8][256]: digit planes 0..3 and their negatives 4..7
     float* xscale;             // out [layer][n_tokens][n_embd/256] 2^-p
-    DecodeGroups groups;       // out
+    DecodeGroups groups;       // out; NULL: none are made (one layer)
     uint32_t n_tokens, n_layers, pairs_per_block;   // the last one is the launcher's
     qkm_dims d;
 };
@@ -108,6 +108,7 @@ struct GateupDecodeArgs {
     const int8_t* planes;
     const float* xscale;
     DecodeGroups groups;
+    const qkm_sel* sel;             // one layer: its records, from which each block groups the pairs itself; NULL: the shared expert alone
     uint32_t n_tokens, n_layers;
     uint32_t gateup_type;           // QKM_TYPE_IQ3_XXS or QKM_TYPE_IQ4_XS
     float *h, *h_last;              // out [layer][n_tokens][n_used+1][n_ff]; the last layer's
@@ -117,6 +118,7 @@ struct GateupDecodeArgs {
 size_t decode_gateup_lut_bytes();
 cudaError_t launch_decode_gateup_luts(const Launch& L, uint8_t* luts);
 bool decode_gateup_ok(const qkm_dims& d);
+uint32_t decode_gateup_rows(uint32_t n_blocks);   // (layer, token) rows of several layers that go together, at most
 cudaError_t launch_decode_gateup(const Launch& L, const GateupDecodeArgs& a, uint32_t n_blocks);
 // routed (IQ4_XS) down + shared (Q8_0) down + weighted sum: y[t] = sum_s w_s D[ids_s] h[t][s] + w_shared DS h[t][n_used]
 struct DownDecodeArgs {
@@ -127,7 +129,7 @@ struct DownDecodeArgs {
     const qkm_sel *sel, *sel_last;
     float* y;                       // out [n_tokens][n_embd] of the first layer
     uint64_t y_stride;              // floats from one layer's rows to the next one's
-    DecodeGroups groups;            // launch_decode_down_group
+    DecodeGroups groups;            // launch_decode_down_group; NULL: one layer, whose pairs each block groups itself
     float* contrib;                 // launch_decode_down_group: scratch [layer][n_tokens][n_used+1][n_embd]
     uint32_t n_tokens, n_layers;
     uint32_t* status;

@@ -136,3 +136,25 @@ def test_host_buffers_in_chunks(pkg, syn):
             for l in range(n):   # (64 tokens of a batch: the same kernels, other shares of the list and so another order of some sums at most)
                 assert syn.rel_err_rows(y[l], want[l]) < 1e-6
         ctx.set_stream(0)
+
+
+# one token and one pair, an odd and a full batch, every expert chosen by all or by few, the most groups that a layer can have (512 experts, 15 of them
+# used), the down kernel that goes by expert (40 tokens on) and those that do not
+@pytest.mark.parametrize("n_embd,n_expert,n_used,gt,dt,T", [
+    (512, 1, 1, 18, 23, 1), (512, 512, 15, 18, 23, 64), (1024, 512, 10, 23, 14, 63), (2048, 20, 8, 18, 23, 40), (512, 15, 15, 23, 23, 2), (512, 16, 4, 18, 14, 39)])
+def test_layer_on_its_own_and_in_a_stack(pkg, orc, syn, n_embd, n_expert, n_used, gt, dt, T):
+    """A layer's blocks group its pairs themselves, a stack's router groups them: the same bits, and the oracle's values."""
+    dims = syn.Dims(n_embd=n_embd, n_ff=512, n_expert=n_expert, n_used=n_used)
+    layers = [syn.make_layer(dims, seed=320, layer=l, gateup_type=gt, down_type=dt) for l in range(2)]
+    x = np.stack([syn.random_x(T, n_embd, seed=330 + l) for l in range(2)])
+    with pkg.Context(dims, n_layer=2, max_tokens=T, device=0) as ctx:
+        for l, layer in enumerate(layers):
+            ctx.upload_layer(l, layer)
+        d_x, d_y = ctx.to_device(x), ctx.alloc(x.nbytes)
+        ctx.moe_decode_stack(0, 2, d_x, T, d_y)
+        together = d_y.download(np.float32, x.shape)
+        for l in range(2):
+            ctx.moe_decode(l, d_x.ptr + l * x[0].nbytes, T, d_y.ptr + l * x[0].nbytes)
+        y, sel = d_y.download(np.float32, x.shape), ctx.last_sel(T)
+    assert np.array_equal(y, together)
+    check(syn, orc, layers, x, y, sel)
