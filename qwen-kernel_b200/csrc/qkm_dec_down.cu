@@ -289,8 +289,8 @@ decode_down_kernel(const __grid_constant__ DownDecodeArgs a) {
                 vb += w_sh * (sdb * ((float)c[2] * dw0 + (float)c[3] * dw1));
             }
             // digits 0, 1 sit in lane t = 0 and 2, 3 in t = 1
-            // (before the stage is filled again: no read of it is under way then, which the copy would not wait for)
             va += __shfl_xor_sync(0xFFFFFFFFu, va, 1); vb += __shfl_xor_sync(0xFFFFFFFFu, vb, 1);
+            stage_read();
             __syncwarp();
             if (lane == 0) issue(stage);
             if (t == 0) {

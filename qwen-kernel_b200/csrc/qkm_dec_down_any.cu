@@ -246,9 +246,9 @@ decode_down_any_kernel(const __grid_constant__ DownDecodeArgs a) {
                 va += w_sh * (f16_bits_to_f32((dw >> (16 * (g & 1u))) & 0xFFFFu) * ((float)c[0] * dw0 + (float)c[1] * dw1));
                 vb += w_sh * (f16_bits_to_f32((dw8 >> (16 * (g & 1u))) & 0xFFFFu) * ((float)c[2] * dw0 + (float)c[3] * dw1));
             }
-            // (before the stage is filled again: no read of it is under way then, which the copy would not wait for)
             va += __shfl_xor_sync(0xFFFFFFFFu, va, 1); vb += __shfl_xor_sync(0xFFFFFFFFu, vb, 1);
             if (Q6) { va += __shfl_xor_sync(0xFFFFFFFFu, va, 2); vb += __shfl_xor_sync(0xFFFFFFFFu, vb, 2); }
+            stage_read();
             __syncwarp();
             if (lane == 0) issue(stage);
             if (t == 0) {

@@ -146,6 +146,7 @@ decode_down_group_kernel(const __grid_constant__ DownDecodeArgs a) {
     uint32_t b0[NB][8], b1[NB][8];           // B operands (Q6_K: per token)
     float w0 = 0.f, w1 = 0.f;                // weights of this lane's two C columns (Q6_K: of the two tokens)
     auto next = [&]() {
+        stage_read();
         __syncwarp();
         if (lane == 0) issue(stage);
         if (++stage == dp::kStages) { stage = 0; phase ^= 1u; }
@@ -301,12 +302,10 @@ decode_down_group_kernel(const __grid_constant__ DownDecodeArgs a) {
                     va += f16_bits_to_f32((dw >> (16 * (g & 1u))) & 0xFFFFu) * ((float)c[0] * w0 + (float)c[1] * w1);
                     vb += f16_bits_to_f32((dw8 >> (16 * (g & 1u))) & 0xFFFFu) * ((float)c[2] * w0 + (float)c[3] * w1);
                 }
-                vb = __shfl_sync(0xFFFFFFFFu, vb, lane);   // (as below)
                 next();
             }
         }
         // the token's other two digits sit in lane t^1
-        // (before the stage is filled again: no read of it is under way then, which the copy would not wait for)
         va += __shfl_xor_sync(0xFFFFFFFFu, va, 1); vb += __shfl_xor_sync(0xFFFFFFFFu, vb, 1);
         if (!rec.shared()) next();
         if ((t & 1u) == 0) {

@@ -242,9 +242,9 @@ decode_down_q6k_kernel(const __grid_constant__ DownDecodeArgs a) {
                 va += w_sh * (sda * ((float)c[0] * dws0 + (float)c[1] * dws1));
                 vb += w_sh * (sdb * ((float)c[2] * dws0 + (float)c[3] * dws1));
             }
-            // (before the stage is filled again: no read of it is under way then, which the copy would not wait for)
             va += __shfl_xor_sync(0xFFFFFFFFu, va, 1); vb += __shfl_xor_sync(0xFFFFFFFFu, vb, 1);
             va += __shfl_xor_sync(0xFFFFFFFFu, va, 2); vb += __shfl_xor_sync(0xFFFFFFFFu, vb, 2);
+            stage_read();
             __syncwarp();
             if (lane == 0) issue(stage);
             if (t == 0) {

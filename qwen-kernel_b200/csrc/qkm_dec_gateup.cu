@@ -376,9 +376,7 @@ decode_gateup_kernel(const __grid_constant__ GateupDecodeArgs a) {
             }
         }
         float ga, gb, ua, ub;
-        // The token's other two digits sit in lane t^1.  The exchange comes before the stage is filled again: it needs what was read last, so
-        // no read is under way any more.  (A copy does not wait for reads that are: with the refill first, a tile's last rows got the scales of
-        // the tile after next, once in some ten thousand launches.)
+        // the token's other two digits sit in lane t^1
         auto both_halves = [&]() {
             ga += __shfl_xor_sync(0xFFFFFFFFu, ga, 1); gb += __shfl_xor_sync(0xFFFFFFFFu, gb, 1);
             ua += __shfl_xor_sync(0xFFFFFFFFu, ua, 1); ub += __shfl_xor_sync(0xFFFFFFFFu, ub, 1);
@@ -409,6 +407,7 @@ decode_gateup_kernel(const __grid_constant__ GateupDecodeArgs a) {
             ub = (f16_bits_to_f32((uwb >> sh) & 0xFFFFu) * 0.25f) * ((float)iu[2] * wcol0 + (float)iu[3] * wcol1);
             }
             both_halves();
+            stage_read();
             __syncwarp();
             if (lane == 0) issue(stage);
             ++cnt;
@@ -421,7 +420,7 @@ decode_gateup_kernel(const __grid_constant__ GateupDecodeArgs a) {
                 const uint32_t sbase = ring + stage * kStageB;
                 q8_quarter(sbase, lane, g, b0[2 * q], b1[2 * q], b0[2 * q + 1], b1[2 * q + 1], wcol0, wcol1, ga, gb);
                 q8_quarter(sbase + dg::kQ8Quarter, lane, g, b0[2 * q], b1[2 * q], b0[2 * q + 1], b1[2 * q + 1], wcol0, wcol1, ua, ub);
-                ub = __shfl_sync(0xFFFFFFFFu, ub, lane);   // (what was read last has come back)
+                stage_read();
                 __syncwarp();
                 if (lane == 0) issue(stage);
                 ++cnt;

@@ -240,6 +240,7 @@ gemv_stream_kernel(const uint8_t* __restrict__ W, const float* __restrict__ x, f
                 if (lane == 0) y[(size_t)t * M + (size_t)tile * rows_per_tile + r] = acc;
             }
         }
+        stage_read();
         __syncthreads();   // every warp is done with this stage
         if (tid == 0) issue(stage);
     }

@@ -160,7 +160,8 @@ gemv_mma_kernel(const __grid_constant__ CUtensorMap tmap, const float* __restric
             acc[q][0] = acc[q][1] = acc[q + 1][0] = acc[q + 1][1] = 0.f;
             const uint32_t i = i0 + q;
             if (i < my_tiles) {   // block-uniform
-                // refill the two stages this warp read one pair ago (its loads have returned), then wait for the pair
+                // refill the two stages this warp read one pair ago, then wait for the pair
+                stage_read();
                 __syncwarp();
                 if (lane == 0) {
                     if (i + n_stages - 2 < my_tiles) issue(i + n_stages - 2);
@@ -183,8 +184,7 @@ gemv_mma_kernel(const __grid_constant__ CUtensorMap tmap, const float* __restric
                     else { q8_block_mma<true>(ca, b0[sb], b1[sb], plane_w, fa0, fa1); q8_block_mma<true>(cb, b0[sb], b1[sb], plane_w, fb0, fb1); }
                     ca = na; cb = nb;
                 }
-                // The two digit-plane pairs of a row sit in lanes t = 0 and t = 1.  (Before the stages are filled again: no read of them is under way
-                // then, which the copies would not wait for.)
+                // the two digit-plane pairs of a row sit in lanes t = 0 and t = 1
                 fa0 += __shfl_xor_sync(0xFFFFFFFFu, fa0, 1); fa1 += __shfl_xor_sync(0xFFFFFFFFu, fa1, 1);
                 fb0 += __shfl_xor_sync(0xFFFFFFFFu, fb0, 1); fb1 += __shfl_xor_sync(0xFFFFFFFFu, fb1, 1);
                 acc[q][0] = fa0; acc[q][1] = fa1;
@@ -473,6 +473,7 @@ gemv_tile_kernel(const uint8_t* __restrict__ W, const float* __restrict__ x, flo
             } else {
                 q6k_tile<false>(blk0, blk1, t, b0, b1, v0, v1);
             }
+            stage_read();
             __syncwarp();
             if (lane == 0) mbar_arrive(bar_empty + 8 * c_stage);
             if (++c_stage == n_stages) { c_stage = 0; c_phase ^= 1u; }

@@ -33,6 +33,10 @@ __device__ __forceinline__ void bulk_g2s(uint32_t dst, const void* src, uint32_t
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
                  ::"r"(dst), "l"(src), "r"(bytes), "r"(bar) : "memory");
 }
+// Behind a thread's last read of a ring stage, ahead of the barrier (warp, block or mbarrier) that hands the stage to the thread that fills it
+// again: a bulk copy is a write by the async proxy, which neither waits for ordinary reads under way nor is ordered behind them by a barrier
+// alone.  (Without it the last reads of a tile returned the bytes of the tile after next, once in some ten thousand launches.)
+__device__ __forceinline__ void stage_read() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
     uint32_t ok;
     asm volatile(
