@@ -255,13 +255,13 @@ def test_decode_stack_and_errors(pkg, orc, syn):
 
 
 def test_decode_stack_host_buffers_in_chunks(pkg, orc, syn):
-    """The host-buffer form of the stack (copies inside): nine layers run as chunks of layers, each
-    its own graph, with the copies on their own streams; three layers take the plain form.  Both equal
-    the layer-by-layer calls bit for bit, on a repeated call (graphs replayed) and after a call with
-    another token count and with device buffers in between (more argument sets than one graph)."""
+    """The host-buffer form of the stack (copies inside) on layers outside the fused sequence (n_ff = 256): nine layers of 1.6 MB of rows
+    run as three chunks, the longest from a graph, with the copies on their own streams; fewer rows or layers take one copy each way.  All
+    equal the layer-by-layer calls bit for bit, on a repeated call (graph replayed) and after a call with another token count and with
+    device buffers in between (other argument sets)."""
     import torch
     dims = syn.Dims(n_embd=512, n_ff=256, n_expert=16, n_used=4)
-    T, L = 5, 9
+    T, L = 86, 9
     layers = [syn.make_layer(dims, seed=52, layer=l) for l in range(L)]
     x = np.stack([syn.random_x(T, dims.n_embd, seed=80 + l) for l in range(L)])
     with pkg.Context(dims, n_layer=L, max_tokens=T, device=0) as ctx:

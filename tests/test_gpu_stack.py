@@ -7,8 +7,9 @@ pytestmark = pytest.mark.gpu
 TOL_F32 = 1e-5   # as the layer-by-layer decode calls: exact integer sums, one f32 rounding per 256 columns
 
 
-def run_stack(pkg, syn, dims, layers, x, max_tokens=None, y_at=None):
-    """(y [L][T][n_embd], last layer's selection); y_at: byte offset of the outputs inside the inputs' buffer."""
+def run_stack(pkg, syn, dims, layers, x, max_tokens=None, y_at=None, runs=None):
+    """(y [L][T][n_embd], last layer's selection); y_at: byte offset of the outputs inside the inputs' buffer; runs: how many times layers go
+    through the stages together, three or four launches each."""
     L, T = x.shape[:2]
     with pkg.Context(dims, n_layer=L, max_tokens=max_tokens or T, device=0) as ctx:
         for l, layer in enumerate(layers):
@@ -16,7 +17,9 @@ def run_stack(pkg, syn, dims, layers, x, max_tokens=None, y_at=None):
         if y_at is None:
             d_x, d_y = ctx.to_device(x), ctx.alloc(x.nbytes)
             for _ in range(3):   # counters and tickets are left as they were found
+                before = ctx.launch_count()
                 ctx.moe_decode_stack(0, L, d_x, T, d_y)
+            assert runs is None or 3 * runs <= ctx.launch_count() - before <= 4 * runs
             y = d_y.download(np.float32, x.shape)
         else:
             buf = ctx.to_device(np.concatenate([x.reshape(-1), np.zeros(y_at // 4, np.float32)]))
@@ -45,18 +48,19 @@ def test_stack_layers_together(pkg, orc, syn, n_embd, n_expert, n_used, gt, dt, 
     dims = syn.Dims(n_embd=n_embd, n_ff=512, n_expert=n_expert, n_used=n_used)
     layers = [syn.make_layer(dims, seed=200, layer=l, router_type=l0, gateup_type=gt, down_type=dt) for l, l0 in enumerate([T & 1] * L)]
     x = np.stack([syn.random_x(T, n_embd, seed=210 + l) for l in range(L)])
-    y, sel = run_stack(pkg, syn, dims, layers, x)
+    y, sel = run_stack(pkg, syn, dims, layers, x, runs=2 if T > 64 else 1)
     check(syn, orc, layers, x, y, sel)
 
 
-# router blocks of several pairs of experts, which keep up to four tokens' x: one, two and four tokens a group, the last group and the last block's pairs
-# not full, an odd number of experts, part of the lanes idle (512 columns) and none (2048)
-@pytest.mark.parametrize("n_embd,n_expert,T,L", [(512, 511, 1, 5), (512, 512, 2, 5), (512, 511, 4, 6), (512, 510, 3, 6), (512, 511, 13, 5), (2048, 64, 64, 10)])
+# router blocks of several pairs of experts: those that keep up to four tokens' x (one, two and four tokens a group) and those that read eight tokens' for
+# each pair; the last group and the last block's pairs not full, an odd number of experts, part of the lanes idle (512 columns) and none (2048)
+@pytest.mark.parametrize("n_embd,n_expert,T,L", [
+    (512, 511, 1, 5), (512, 512, 2, 5), (512, 511, 4, 6), (512, 510, 3, 6), (512, 511, 13, 5), (2048, 64, 64, 10), (512, 511, 6, 6), (512, 256, 8, 10), (512, 255, 21, 5)])
 def test_stack_router_blocks_of_several_pairs(pkg, orc, syn, n_embd, n_expert, T, L):
-    dims = syn.Dims(n_embd=n_embd, n_ff=256, n_expert=n_expert, n_used=8)
+    dims = syn.Dims(n_embd=n_embd, n_ff=512, n_expert=n_expert, n_used=8)
     layers = [syn.make_layer(dims, seed=240, router_type=T & 1)] * L
     x = np.stack([syn.random_x(T, n_embd, seed=250 + l) for l in range(L)])
-    y, sel = run_stack(pkg, syn, dims, layers, x)
+    y, sel = run_stack(pkg, syn, dims, layers, x, runs=1)
     check(syn, orc, layers, x, y, sel)
 
 
@@ -66,7 +70,7 @@ def test_stack_of_several_types(pkg, orc, syn):
     mixes = [(0, 18, 23), (0, 18, 23), (1, 18, 23), (1, 23, 14), (1, 23, 14), (1, 23, 14), (0, 18, 14)]
     layers = [syn.make_layer(dims, seed=220, layer=l, router_type=r, gateup_type=g, down_type=d) for l, (r, g, d) in enumerate(mixes)]
     x = np.stack([syn.random_x(7, 1024, seed=230 + l) for l in range(len(mixes))])
-    y, sel = run_stack(pkg, syn, dims, layers, x)
+    y, sel = run_stack(pkg, syn, dims, layers, x, runs=4)
     check(syn, orc, layers, x, y, sel)
 
 
@@ -75,7 +79,7 @@ def test_stack_more_layers_than_scratch(pkg, orc, syn):
     dims = syn.Dims(n_embd=512, n_ff=512, n_expert=8, n_used=2)
     layers = [syn.make_layer(dims, seed=240, layer=l) for l in range(14)]
     x = np.stack([syn.random_x(64, 512, seed=250 + l) for l in range(14)])
-    y, sel = run_stack(pkg, syn, dims, layers, x)
+    y, sel = run_stack(pkg, syn, dims, layers, x, runs=2)
     check(syn, orc, layers, x, y, sel)
 
 
@@ -115,27 +119,31 @@ def test_stack_nonfinite_and_large_rows(pkg, orc, syn, gt, dt):
         assert np.isnan(y[l][~ok[l]]).all()
 
 
-def test_host_buffers_in_chunks(pkg, syn):
-    """From 1.5 MB of rows on the host-buffer form runs in three chunks of layers, the copies on streams of their own: the same results as the
-    device form, on a repeated call too, and one layer less than chunks need takes one copy each way."""
+# 64 tokens and fewer, both down kernels that go by expert and one that does not
+@pytest.mark.parametrize("gt,dt,T,L", [(18, 23, 64, 14), (23, 14, 64, 13), (18, 14, 24, 40)])
+def test_host_buffers_in_chunks(pkg, orc, syn, gt, dt, T, L):
+    """From 1.5 MB of rows on the host-buffer form runs in three chunks of layers that go together, the copies on streams of their own: the bits of the
+    layer-by-layer calls, on repeated calls too (scratch and tickets are the chunks' in turn), and fewer layers than chunks need in one."""
     import torch
-    dims, T, L = syn.Dims(n_embd=512, n_ff=256, n_expert=16, n_used=4), 64, 14
+    dims = syn.Dims(n_embd=512, n_ff=512, n_expert=16, n_used=4)
     x = np.stack([syn.random_x(T, dims.n_embd, seed=300 + l) for l in range(L)])
-    assert x.nbytes >= 3 << 19 and x[:5].nbytes < 3 << 19
+    assert x.nbytes >= 3 << 19
+    layer = syn.make_layer(dims, seed=301, gateup_type=gt, down_type=dt)
     with pkg.Context(dims, n_layer=L, max_tokens=T, device=0) as ctx:
         for l in range(L):
-            ctx.upload_layer(l, syn.make_layer(dims, seed=301, layer=l))
+            ctx.upload_layer(l, layer)
+        want = np.stack([ctx.moe_forward_host(l, x[l], mode=0) for l in range(L)])
         stream = torch.cuda.Stream(torch.device("cuda", 0))
         ctx.set_stream(stream.cuda_stream)
-        d_x, d_y = ctx.to_device(x), ctx.alloc(x.nbytes)
-        ctx.moe_decode_stack(0, L, d_x, T, d_y)
-        want = d_y.download(np.float32, x.shape)
-        for n in (L, L, 5):
+        for n, chunks in ((L, 3), (L, 3), (5, 1), (L, 3)):
             y = np.zeros_like(x[:n])
+            before = ctx.launch_count()
             ctx.moe_decode_stack_host(0, n, x.ctypes.data, T, y.ctypes.data)
-            for l in range(n):   # (64 tokens of a batch: the same kernels, other shares of the list and so another order of some sums at most)
-                assert syn.rel_err_rows(y[l], want[l]) < 1e-6
+            assert 3 * chunks <= ctx.launch_count() - before <= 4 * chunks
+            assert np.array_equal(y, want[:n])
         ctx.set_stream(0)
+    for l in (0, L // 2, L - 1):
+        assert syn.rel_err_rows(want[l], orc.moe_layer(layer, x[l], threads=orc.hardware_threads())["y"]) < TOL_F32
 
 
 # one token and one pair, an odd and a full batch, every expert chosen by all or by few, the most groups that a layer can have (512 experts, 15 of them
