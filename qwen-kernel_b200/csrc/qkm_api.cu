@@ -309,7 +309,7 @@ extern "C" QKM_API qkm_ctx* qkm_open(const qkm_config* cfg, char* err, size_t er
                 return nullptr;
             }
         }
-        c->dec_ok = decode_gateup_ok(d) && d.n_embd <= 4096;
+        c->dec_ok = decode_gateup_ok(d);
         if (c->dec_ok) {
             if ((e = alloc_decode(c)) != cudaSuccess) {
                 bail("qkm_open: cudaMalloc of decode scratch", cudaGetErrorString(e));
@@ -681,7 +681,7 @@ static int decode_fused(qkm_ctx* c, uint32_t first, uint32_t count, const float*
 // The fused sequence's limits; the tensors' are in qkm_layer_dev::fused_ok.
 static bool decode_fused_ok(const qkm_ctx* c, uint32_t n) {
     const qkm_dims& d = c->cfg.dims;
-    return n && c->dec_ok && c->dec_rows && route_decode_ok(d, n < 64 ? n : 64, c->route_scratch_bytes) && (decode_down_ok(d) || decode_down_any_ok(d) || c->dec_contrib);
+    return n && c->dec_ok && c->dec_rows && route_decode_ok(d) && (decode_down_ok(d) || decode_down_any_ok(d) || c->dec_contrib);
 }
 
 // Layers [first, first + count), all ready for the fused sequence, at most 64 tokens at a time: in runs of the same types, as many layers at once

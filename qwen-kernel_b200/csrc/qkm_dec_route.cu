@@ -41,7 +41,7 @@ __device__ __forceinline__ uint32_t ticket(uint32_t* counter) {
     return n;
 }
 // TOK: tokens of a group; a.pairs_per_block: router row pairs that a logits block takes one after the other; KEEP: the tokens' x stays in
-// registers as doubles for all of them (n_embd <= 2048)
+// registers as doubles for all of them
 template <int TYPE, int TOK, bool KEEP>
 __global__ void __launch_bounds__(rd::kThreads, 2)
 route_decode_kernel(const __grid_constant__ RouteDecodeArgs a) {
@@ -69,17 +69,17 @@ route_decode_kernel(const __grid_constant__ RouteDecodeArgs a) {
         __shared__ double s_sg[8];
         const uint32_t t = blockIdx.x - n_logit_blocks, KB = d.n_embd / 256;
         const float *xt = x + (size_t)t * d.n_embd, *gis = a.layer[layer].gis;
-        float v[16];   // n_embd <= 4096: element tid of every 256 columns
+        float v[8];   // n_embd <= 2048: element tid of every 256 columns
         double dsg = 0.0;
 #pragma unroll
-        for (int i = 0; i < 16; ++i) {
+        for (int i = 0; i < 8; ++i) {
             const uint32_t k = tid + 256 * i;
             v[i] = k < d.n_embd ? xt[k] : 0.f;
             if (k < d.n_embd) dsg += (double)gis[k] * (double)v[i];
         }
         // a scale per 256 columns: a large element costs the others of its own block bits, not the whole row
 #pragma unroll
-        for (int i = 0; i < 16; ++i)
+        for (int i = 0; i < 8; ++i)
             if (256u * i < d.n_embd) {
                 const float ax = fabsf(v[i]);
                 const uint32_t m = __reduce_max_sync(0xFFFFFFFFu, ax <= 3.0e38f ? __float_as_uint(ax) : 0x7F800000u);   // non-negative floats order like their bits
@@ -105,7 +105,7 @@ route_decode_kernel(const __grid_constant__ RouteDecodeArgs a) {
         __syncthreads();
         int8_t* pl = a.planes + (size_t)(layer * T + t) * 8 * d.n_embd;
 #pragma unroll
-        for (int i = 0; i < 16; ++i) {
+        for (int i = 0; i < 8; ++i) {
             const uint32_t k = tid + 256 * i;
             if (k < d.n_embd) store_planes8(pl, k, digits4(__float2int_rn(v[i] * s_up[i])));
         }
@@ -120,20 +120,17 @@ route_decode_kernel(const __grid_constant__ RouteDecodeArgs a) {
     const uint32_t p0 = blockIdx.x % n_pair_blocks * a.pairs_per_block, p1 = min(p0 + a.pairs_per_block, n_pairs), t0 = (blockIdx.x / n_pair_blocks) * TOK;
     const size_t rb = row_bytes(TYPE, d.n_embd);
     const uint8_t* router = a.layer[layer].w;
-    const uint32_t units_w = d.n_embd / 64;   // 8-element units per warp
-    const bool once = units_w <= 32;          // a lane has one unit: its router elements are read ahead
+    const uint32_t units_w = d.n_embd / 64, k = (warp * units_w + lane) * 8;   // 8-element units of a warp: at most one a lane; its first column
     float w0[8], w1[8];
-    auto rows = [&](uint32_t pair, uint32_t u) {
+    auto rows = [&](uint32_t pair) {
         const uint8_t* row0 = router + (size_t)(2 * pair) * rb;
-        const uint32_t k = (warp * units_w + u) * 8;
         dequant8<TYPE>(row0, k, w0);
         dequant8<TYPE>(2 * pair + 1 < d.n_expert ? row0 + rb : row0, k, w1);
     };
-    if (once && lane < units_w) rows(p0, lane);
+    if (lane < units_w) rows(p0);
     constexpr int kKept = KEEP ? TOK : 1;
     double xd[kKept][8];
     if (KEEP && lane < units_w) {
-        const uint32_t k = (warp * units_w + lane) * 8;
         float4 xa[kKept], xb[kKept];
 #pragma unroll
         for (int j = 0; j < kKept; ++j) {
@@ -156,7 +153,7 @@ route_decode_kernel(const __grid_constant__ RouteDecodeArgs a) {
                 float c0[8], c1[8];
 #pragma unroll
                 for (int i = 0; i < 8; ++i) { c0[i] = w0[i]; c1[i] = w1[i]; }
-                if (pair + 1 < p1) rows(pair + 1, lane);
+                if (pair + 1 < p1) rows(pair + 1);
 #pragma unroll
                 for (int i = 0; i < 8; ++i) {
                     const double v0 = c0[i], v1 = c1[i];
@@ -165,9 +162,7 @@ route_decode_kernel(const __grid_constant__ RouteDecodeArgs a) {
                 }
             }
         } else
-        for (uint32_t u = lane; u < units_w; u += 32) {
-            const uint32_t k = (warp * units_w + u) * 8;
-            if (!once) rows(pair, u);
+        if (lane < units_w) {
             constexpr int kHalf = TOK < 4 ? TOK : 4;   // four tokens' values at a time: more do not fit the registers
             float4 xa[kHalf], xb[kHalf];
             auto tokens = [&](int j0) {
@@ -182,7 +177,7 @@ route_decode_kernel(const __grid_constant__ RouteDecodeArgs a) {
             double v0[8], v1[8];
 #pragma unroll
             for (int i = 0; i < 8; ++i) { v0[i] = w0[i]; v1[i] = w1[i]; }
-            if (once && pair + 1 < p1) rows(pair + 1, u);
+            if (pair + 1 < p1) rows(pair + 1);
 #pragma unroll
             for (int j0 = 0; j0 < TOK; j0 += kHalf) {
                 if (j0 > 0) tokens(j0);
@@ -264,10 +259,7 @@ route_decode_kernel(const __grid_constant__ RouteDecodeArgs a) {
     if (n_groups == 1 && ranks) rank_store(mine, sel[my_t], d);   // (after the lists: the next kernel waits for those)
 }
 
-bool route_decode_ok(const qkm_dims& d, uint32_t n_tokens, size_t scratch_bytes) {
-    return n_tokens > 0 && n_tokens <= 64 && d.n_expert <= 512 && d.n_used <= 16 && d.n_embd <= 4096 && d.n_embd % 64 == 0 &&
-           (size_t)n_tokens * d.n_expert * sizeof(double) <= scratch_bytes;
-}
+bool route_decode_ok(const qkm_dims& d) { return d.n_expert <= rk::kMaxExperts && d.n_embd <= 2048; }
 
 // Tokens of a group: as few as the batch has (a group of eight costs one token as much as eight).  Pairs a block: one for a layer on its own and while the blocks
 // find room on the SMs at once (a chain of latencies: start-up, loads, ticket), more when layers go together, so that a block's share of that chain is
@@ -286,10 +278,10 @@ template <int TYPE>
 static cudaError_t route_launch(const Launch& L, RouteDecodeArgs a) {
     constexpr uint32_t kFour = 4800;
     const uint32_t T = a.n_tokens, pairs = (a.d.n_expert + 1) / 2;
-    const bool fits = a.d.n_embd <= 2048, four = fits && a.n_layers > 1 && T > 8 && pairs * ((T + 3) / 4) * a.n_layers >= kFour;
+    const bool four = a.n_layers > 1 && T > 8 && pairs * ((T + 3) / 4) * a.n_layers >= kFour;
     const uint32_t tok = T <= 1 ? 1 : T <= 2 ? 2 : T <= 4 || four ? 4 : 8, groups = (T + tok - 1) / tok, per = a.n_layers == 1 ? 1 : pairs * groups * a.n_layers / 600;
     a.pairs_per_block = per < 1 ? 1 : per < 16 ? per : 16;
-    const bool keep = fits && a.pairs_per_block > 1;
+    const bool keep = a.pairs_per_block > 1;
     switch (tok) {
         case 1: return keep ? route_launch<TYPE, 1, true>(L, a, groups) : route_launch<TYPE, 1, false>(L, a, groups);
         case 2: return keep ? route_launch<TYPE, 2, true>(L, a, groups) : route_launch<TYPE, 2, false>(L, a, groups);
@@ -299,7 +291,7 @@ static cudaError_t route_launch(const Launch& L, RouteDecodeArgs a) {
 }
 cudaError_t launch_route_decode(const Launch& L, uint32_t router_type, const RouteDecodeArgs& a) {
     if (router_type != QKM_TYPE_F32 && router_type != QKM_TYPE_F16) return cudaErrorInvalidValue;
-    if (a.n_tokens == 0 || a.n_tokens > 64 || a.d.n_expert > 512 || a.d.n_embd > 4096 || a.n_layers == 0 || a.n_layers > kDecMaxLayers) return cudaErrorInvalidValue;
+    if (a.n_tokens == 0 || a.n_tokens > rk::kMaxTokens || !route_decode_ok(a.d) || a.n_layers == 0 || a.n_layers > kDecMaxLayers) return cudaErrorInvalidValue;
     const cudaError_t e = router_type == QKM_TYPE_F32 ? route_launch<QKM_TYPE_F32>(L, a) : route_launch<QKM_TYPE_F16>(L, a);
     L.count();
     return e != cudaSuccess ? e : cudaGetLastError();

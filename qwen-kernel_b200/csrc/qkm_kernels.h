@@ -99,7 +99,7 @@ struct RouteDecodeArgs {
     uint32_t n_tokens, n_layers, pairs_per_block;   // the last one is the launcher's
     qkm_dims d;
 };
-bool route_decode_ok(const qkm_dims& d, uint32_t n_tokens, size_t scratch_bytes);
+bool route_decode_ok(const qkm_dims& d);
 cudaError_t launch_route_decode(const Launch& L, uint32_t router_type, const RouteDecodeArgs& a);
 // routed (IQ3_XXS) and shared (Q8_0) gate/up + SwiGLU over the groups
 struct GateupDecodeArgs {
