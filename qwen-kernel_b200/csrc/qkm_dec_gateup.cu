@@ -62,8 +62,9 @@ constexpr uint32_t kRings4 = 1024;
 constexpr uint32_t kRed4 = kRings4 + kWarps * kRingBytes4;
 constexpr uint32_t kList4 = kRed4 + kRedBytes;
 constexpr int kQ8Quarter = 2 * 544;                 // two 32-column blocks of a Q8_0 tile: d and quants of 16 rows each
-// relative time of a routed / a shared tile: of one layer, and of several together (40 layers of 16 tokens with 9: 1,895 us, 10: 1,867, 11: 1,878)
-constexpr uint32_t kCostRouted = 8, kCostShared1 = 11, kCostShared = 10;
+// Relative time of a routed / a shared tile.  11 instead of 10 changes layers that go together by -2.5 to +1.1 % (mostly less than two runs
+// differ) and a layer on its own by -1.3 to +0.4 %, but one token's from 23.5 to 25.2 us.
+constexpr uint32_t kCostRouted = 8, kCostShared = 10;
 }  // namespace dg
 
 size_t decode_gateup_lut_bytes() { return dg::kTabBytes; }
@@ -232,8 +233,8 @@ decode_gateup_kernel(const __grid_constant__ GateupDecodeArgs a) {
     }
 
     const uint32_t teams_total = gridDim.x * n_teams, team_global = blockIdx.x * n_teams + team;
-    const uint32_t n_layers = ONE ? 1 : a.n_layers, cost_shared = ONE ? dg::kCostShared1 : dg::kCostShared;
-    const Divisor by_teams(teams_total), by_tiles(RT), by_shared(cost_shared);
+    const uint32_t n_layers = ONE ? 1 : a.n_layers;
+    const Divisor by_teams(teams_total), by_tiles(RT), by_shared(dg::kCostShared);
 
     // Up to here nothing depended on the router kernel, so a block scheduled early (programmatic
     // dependent launch) has its barriers and table copy under way while that kernel's tail runs.  The
@@ -245,9 +246,9 @@ decode_gateup_kernel(const __grid_constant__ GateupDecodeArgs a) {
     // than a routed one (four ring stages, each a round trip), so the cut is made in cost units:
     // kCostRouted per routed tile, kCostShared per shared tile (a layer's shared groups come last).
     if (ONE) {
-        own_groups<dg::kWarps * 32>(own, own_list, s_cuts, a.sel, d, a.n_tokens, dg::kCostRouted, cost_shared);
+        own_groups<dg::kWarps * 32>(own, own_list, s_cuts, a.sel, d, a.n_tokens, dg::kCostRouted, dg::kCostShared);
     } else {
-        if (warp == 0) layer_cuts(s_cuts, a.groups, a.n_tokens, n_layers, dg::kCostRouted, cost_shared);
+        if (warp == 0) layer_cuts(s_cuts, a.groups, a.n_tokens, n_layers, dg::kCostRouted, dg::kCostShared);
         __syncthreads();
     }
     uint32_t left;   // tiles still to do
@@ -278,8 +279,11 @@ decode_gateup_kernel(const __grid_constant__ GateupDecodeArgs a) {
     uint32_t p_left = left, p_q = 0;
     uint32_t p_rt = rt;
     bool p_new = true;                            // the group record must be (re)loaded
-    const uint8_t* p_g = nullptr;                 // next tile of the gate (routed) / shared gate matrix
+    // Next tile of the gate and the up matrix, routed or shared: pointers, or ONE: its number, since the matrices are the parameters' first then
+    // (with pointers the IQ3_XXS form spills, 4 % of its time; of several layers the number and the layer cost 5 %).
+    const uint8_t* p_g = nullptr;
     const uint8_t* p_u = nullptr;
+    uint32_t p_tile = 0;
     bool p_shared = false;
     auto issue = [&](uint32_t stage) {
         if (p_left == 0) return;
@@ -288,7 +292,9 @@ decode_gateup_kernel(const __grid_constant__ GateupDecodeArgs a) {
             const DecodeGroup r = record((total - p_left) / RT);
             const GateupDecodeArgs::Mats& m = a.layer[ONE ? 0 : r.layer];
             p_shared = r.shared();
-            if (!p_shared) {
+            if (ONE) {
+                p_tile = (p_shared ? 0 : r.expert() * (uint32_t)mat_tiles) + kb * RT + p_rt;
+            } else if (!p_shared) {
                 const size_t tile = (size_t)r.expert() * mat_tiles + (size_t)kb * RT + p_rt;
                 p_g = m.gate + tile * kTileR; p_u = m.up + tile * kTileR;
             } else {
@@ -303,15 +309,19 @@ decode_gateup_kernel(const __grid_constant__ GateupDecodeArgs a) {
         const uint32_t bar = my_bar + 8 * stage, dst = ring + stage * kStageB;
         if (!p_shared) {
             mbar_expect_tx(bar, 2 * kTileR);
-            bulk_g2s(dst, p_g, kTileR, bar);
-            bulk_g2s(dst + kTileR, p_u, kTileR, bar);
-            p_g += kTileR; p_u += kTileR;
+            bulk_g2s(dst, ONE ? a.layer[0].gate + (size_t)p_tile * kTileR : p_g, kTileR, bar);
+            bulk_g2s(dst + kTileR, ONE ? a.layer[0].up + (size_t)p_tile * kTileR : p_u, kTileR, bar);
+            if (ONE) { ++p_tile; } else { p_g += kTileR; p_u += kTileR; }
             next_tile();
         } else {
             mbar_expect_tx(bar, 2 * dg::kQ8Quarter);   // a quarter = two 32-column blocks = one 1088-byte piece
-            bulk_g2s(dst, p_g + dg::kQ8Quarter * p_q, dg::kQ8Quarter, bar);
-            bulk_g2s(dst + dg::kQ8Quarter, p_u + dg::kQ8Quarter * p_q, dg::kQ8Quarter, bar);
-            if (++p_q == 4) { p_q = 0; p_g += kTileQ8; p_u += kTileQ8; next_tile(); }
+            bulk_g2s(dst, (ONE ? a.layer[0].sh_gate + (size_t)p_tile * kTileQ8 : p_g) + dg::kQ8Quarter * p_q, dg::kQ8Quarter, bar);
+            bulk_g2s(dst + dg::kQ8Quarter, (ONE ? a.layer[0].sh_up + (size_t)p_tile * kTileQ8 : p_u) + dg::kQ8Quarter * p_q, dg::kQ8Quarter, bar);
+            if (++p_q == 4) {
+                p_q = 0;
+                if (ONE) { ++p_tile; } else { p_g += kTileQ8; p_u += kTileQ8; }
+                next_tile();
+            }
         }
     };
     if (lane == 0)

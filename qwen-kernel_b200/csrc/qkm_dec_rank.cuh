@@ -4,8 +4,8 @@
 // The router kernel ranks a group of tokens in the block that finishes the group's logits last.  Of layers that go together, the block
 // that ranks a layer's last tokens groups its pairs for the kernels behind.  A layer on its own is grouped by each block of those kernels
 // for itself: one block at the router's end, the lists' way through the L2 and their reads there are a chain that nothing hides, 3 to 6 us of
-// a layer (a decode step of 256 experts, top 8: 1 token 27.0 -> 24.6 us, 16: 80.7 -> 74.1, 64: 182.1 -> 170.3; of 512, top 10: 3 tokens 42.6 ->
-// 40.6, 64: 252.6 -> 247.0).
+// a layer (a decode step of 256 experts, top 8: 1 token 27.0 -> 23.6 us, 16: 80.9 -> 71.9, 64: 182.4 -> 168.4; of 512, top 10: 3 tokens 42.6 ->
+// 39.7, 64: 252.5 -> 242.9; with the kernels' forms for one layer).
 //
 // Rules (the reference's): top n_used by raw logit, lowest id on ties
 // (shaders/moe_select_256.comp:60-61), non-finite logits at the floor -3.4e38

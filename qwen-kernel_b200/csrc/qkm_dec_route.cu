@@ -261,13 +261,15 @@ route_decode_kernel(const __grid_constant__ RouteDecodeArgs a) {
 
 bool route_decode_ok(const qkm_dims& d) { return d.n_expert <= rk::kMaxExperts && d.n_embd <= 2048; }
 
-// Tokens of a group: as few as the batch has (a group of eight costs one token as much as eight).  Pairs a block: one for a layer on its own and while the blocks
-// find room on the SMs at once (a chain of latencies: start-up, loads, ticket), more when layers go together, so that a block's share of that chain is
-// small: 40 layers of 16 tokens 159 us with one pair a block, 125 so.
+// Tokens of a group: as few as the batch has (a group of eight costs one token as much as eight).  Pairs a block: one for a layer on its own and while
+// the blocks find room on the SMs at once (a chain of latencies: start-up, loads, ticket), more when layers go together, so that a block's share of
+// that chain is small: 40 layers of 16 tokens 159 us with one pair a block, 125 so.  About kBlocks blocks: with half as many 24 layers of one token
+// 117 -> 119 us for the whole call, 12 of one 71 -> 74, 6 of 12 243 -> 250; with twice as many 24 of one 117 -> 120, 24 of 5 413 -> 422, 6 of 16
+// 301 -> 308 (but 4 of 3, 512 experts, 85 -> 82).  At most 8, 16 or 32 pairs a block: the same.
 // Blocks of several pairs keep the x of up to four tokens as doubles (the converter takes 16 lanes a cycle and SM, the f64 units 64): 24 layers of
-// one token 124 -> 119 us for the whole call, 40 layers of 16 tokens 2,066 -> 2,031 as groups of four, 12 of 64 1,970 -> 1,934.  With one pair a block
-// there is nothing to keep it for (a step of 3 tokens 341 -> 348 us), and below kFour pairs two groups of four are more blocks than one of eight is worth
-// (24 layers of 5 tokens 541 -> 554).
+// one token 124 -> 119 us, and so groups of four go ahead of groups of eight where they find several pairs a block: 12 layers of 64 tokens
+// 1,712 -> 1,669, 4 of 12 173 -> 170, 2 of 9 (512 experts) 114 -> 111.  With one pair a block there is nothing to keep it for, and groups of four are
+// more blocks than one of eight is worth (2 layers of 16 tokens 121 -> 124, a step of 3 tokens with it kept 341 -> 348).
 template <int TYPE, int TOK, bool KEEP>
 static cudaError_t route_launch(const Launch& L, const RouteDecodeArgs& a, uint32_t groups) {
     const uint32_t pairs = (a.d.n_expert + 1) / 2;
@@ -276,11 +278,11 @@ static cudaError_t route_launch(const Launch& L, const RouteDecodeArgs& a, uint3
 }
 template <int TYPE>
 static cudaError_t route_launch(const Launch& L, RouteDecodeArgs a) {
-    constexpr uint32_t kFour = 4800;
+    constexpr uint32_t kBlocks = 600, kMostPairs = 16;
     const uint32_t T = a.n_tokens, pairs = (a.d.n_expert + 1) / 2;
-    const bool four = a.n_layers > 1 && T > 8 && pairs * ((T + 3) / 4) * a.n_layers >= kFour;
-    const uint32_t tok = T <= 1 ? 1 : T <= 2 ? 2 : T <= 4 || four ? 4 : 8, groups = (T + tok - 1) / tok, per = a.n_layers == 1 ? 1 : pairs * groups * a.n_layers / 600;
-    a.pairs_per_block = per < 1 ? 1 : per < 16 ? per : 16;
+    const bool four = a.n_layers > 1 && T > 8 && pairs * ((T + 3) / 4) * a.n_layers >= 2 * kBlocks;
+    const uint32_t tok = T <= 1 ? 1 : T <= 2 ? 2 : T <= 4 || four ? 4 : 8, groups = (T + tok - 1) / tok, per = a.n_layers == 1 ? 1 : pairs * groups * a.n_layers / kBlocks;
+    a.pairs_per_block = per < 1 ? 1 : per < kMostPairs ? per : kMostPairs;
     const bool keep = a.pairs_per_block > 1;
     switch (tok) {
         case 1: return keep ? route_launch<TYPE, 1, true>(L, a, groups) : route_launch<TYPE, 1, false>(L, a, groups);
