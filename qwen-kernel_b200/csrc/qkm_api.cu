@@ -11,6 +11,7 @@
 #include <cstdio>
 #include <cstring>
 #include <new>
+#include <type_traits>
 #include <vector>
 
 #include "qkm_alloc.h"
@@ -65,15 +66,21 @@ struct qkm_ctx {
     int8_t* planes8 = nullptr;         // [min(max_tokens, 64)][n_embd/256][8][256]: of the expert-parallel calls' local tokens
     uint8_t* lut_gu = nullptr;         // table images the decode kernels copy to shared memory
     uint8_t* lut_dd = nullptr;         // table image of the decode IQ4_XS down kernel
-    // its scratch, for dec_rows (layer, token) rows at a time; the last layer's records and hidden rows go to sel and h
-    uint32_t dec_rows = 0;
-    double* dec_logits = nullptr;      // [row][n_expert]
-    qkm_sel* dec_sel = nullptr;
-    int8_t* dec_planes = nullptr;      // [row][8 n_embd]
-    float *dec_xscale = nullptr, *dec_h = nullptr;        // [row][n_embd/256], [row][n_used+1][n_ff]
-    float* dec_contrib = nullptr;      // [row][n_used+1][n_embd], for the down kernel that groups by expert
-    DecodeGroup* dec_groups = nullptr; // [row][n_used+1]
-    uint32_t* dec_counts = nullptr;    // [kDecMaxLayers]
+    // its scratch for a number of (layer, token) rows; the last layer's records and hidden rows go to sel and h
+    struct DecScratch {
+        void* mem = nullptr;           // the one allocation that all of it lies in
+        uint32_t rows = 0;
+        double* logits = nullptr;      // [row][n_expert]
+        int8_t* planes = nullptr;      // [row][8 n_embd]
+        float* xscale = nullptr;       // [row][n_embd/256]
+        float* contrib = nullptr;      // [row][n_used+1][n_embd], for the down kernel that groups by expert
+        // of several layers
+        qkm_sel* sel = nullptr;
+        float* h = nullptr;            // [row][n_used+1][n_ff]
+        DecodeGroup* groups = nullptr; // [row][n_used+1]
+        uint32_t* counts = nullptr;    // [kDecMaxLayers]
+    } dec_one, dec_many;               // for a layer on its own; for several (see stack_scratch)
+    bool dec_grouped = false;          // contrib is there
     uint8_t* lut_pf = nullptr;         // table image of the prefill GEMMs
     uint32_t* status_host = nullptr;  // pinned mirror
     bool shapes_stream_ok = false;
@@ -212,25 +219,75 @@ int layer_ready(qkm_ctx* c, uint32_t layer) {
     return QKM_OK;
 }
 
-// Scratch of the fused decode sequence: a stack's layers go through it together, as many as kDecRows (layer, token) rows allow (40 layers of 16
-// tokens, 12 of 64; 113 KB a row for 256 experts, top 8).
+// Scratch of the fused decode sequence: a stack's layers go through it together, as many as kDecRows (layer, token) rows allow: 40 layers of 16
+// tokens, 12 of 64; 39 KB a row for 256 experts, top 8, and 74 KB more where the down kernel groups by expert (batches from 40 tokens on).  With
+// 192 rows stacks of 64 tokens take 2 to 7 % longer, with 384 up to 1 %, with 1152 the same.
 constexpr uint32_t kDecRows = 768;
+// Up to this much for several layers is taken at qkm_open (a few slots); more only when a stack is first decoded (0.33 ms, once), since contexts
+// that prefill, or that decode layer by layer, have no use for it.
+constexpr size_t kDecAtOpen = 8u << 20;
+
+// Bytes of the scratch for `rows` rows; with s.mem set, where its parts lie.
+size_t dec_layout(const qkm_ctx* c, qkm_ctx::DecScratch& s, uint32_t rows, bool several) {
+    const qkm_dims& d = c->cfg.dims;
+    const size_t R = rows, S = d.n_used + 1;
+    size_t at = 0;
+    auto part = [&](auto& p, size_t bytes) {
+        if (s.mem) p = reinterpret_cast<std::remove_reference_t<decltype(p)>>((uint8_t*)s.mem + at);
+        at += (bytes + 255) / 256 * 256;
+    };
+    part(s.logits, R * d.n_expert * sizeof(double));
+    part(s.planes, R * 8 * d.n_embd);
+    part(s.xscale, R * (d.n_embd / 256) * sizeof(float));
+    if (c->dec_grouped) part(s.contrib, R * S * d.n_embd * sizeof(float));
+    if (several) {
+        part(s.sel, R * sizeof(qkm_sel));
+        part(s.h, R * S * d.n_ff * sizeof(float));
+        part(s.groups, R * S * sizeof(DecodeGroup));
+        part(s.counts, kDecMaxLayers * sizeof(uint32_t));
+    }
+    return at;
+}
+cudaError_t dec_alloc(const qkm_ctx* c, qkm_ctx::DecScratch& s, uint32_t rows, bool several) {
+    if (const cudaError_t e = cudaMalloc(&s.mem, dec_layout(c, s, rows, several))) {
+        s.mem = nullptr;
+        cudaGetLastError();   // reported by the caller; the next launch's check must not find it
+        return e;
+    }
+    dec_layout(c, s, s.rows = rows, several);
+    return cudaSuccess;
+}
+uint32_t dec_most_tokens(const qkm_ctx* c) { return c->cfg.max_tokens < 64 ? c->cfg.max_tokens : 64; }
+uint32_t dec_most_rows(const qkm_ctx* c) {
+    const uint32_t T = dec_most_tokens(c), fit = decode_gateup_rows((uint32_t)c->n_sms), most = kDecRows < fit ? kDecRows : fit;
+    const uint64_t rows = (uint64_t)c->cfg.n_layer * T;
+    return rows < most ? (uint32_t)rows : most;
+}
 cudaError_t alloc_decode(qkm_ctx* c) {
     const qkm_dims& d = c->cfg.dims;
-    const uint32_t T = c->cfg.max_tokens < 64 ? c->cfg.max_tokens : 64;
-    const uint64_t rows = c->ecount == d.n_expert ? (uint64_t)c->cfg.n_layer * T : 0;
-    const uint32_t together = kDecRows < decode_gateup_rows((uint32_t)c->n_sms) ? kDecRows : decode_gateup_rows((uint32_t)c->n_sms), most = together < T ? T : together;
-    c->dec_rows = rows < most ? (uint32_t)rows : most;
-    const size_t R = c->dec_rows, S = d.n_used + 1;
-    const bool grouped = decode_down_group_ok(d) && (T >= 40 || !decode_down_any_ok(d));
-    const Want want[] = {
-        {(void**)&c->planes8, (size_t)T * 8 * d.n_embd}, {(void**)&c->lut_gu, decode_gateup_lut_bytes()}, {(void**)&c->lut_dd, decode_down_lut_bytes()},
-        {(void**)&c->dec_logits, R * d.n_expert * sizeof(double)}, {(void**)&c->dec_sel, R * sizeof(qkm_sel)}, {(void**)&c->dec_planes, R * 8 * d.n_embd},
-        {(void**)&c->dec_xscale, R * (d.n_embd / 256) * sizeof(float)}, {(void**)&c->dec_h, R * S * d.n_ff * sizeof(float)},
-        {(void**)&c->dec_contrib, grouped ? R * S * d.n_embd * sizeof(float) : 0}, {(void**)&c->dec_groups, R * S * sizeof(DecodeGroup)},
-        {(void**)&c->dec_counts, kDecMaxLayers * sizeof(uint32_t)},
-    };
-    return dev_alloc_all(want);
+    const uint32_t T = dec_most_tokens(c);
+    const Want want[] = {{(void**)&c->planes8, (size_t)T * 8 * d.n_embd}, {(void**)&c->lut_gu, decode_gateup_lut_bytes()}, {(void**)&c->lut_dd, decode_down_lut_bytes()}};
+    if (const cudaError_t e = dev_alloc_all(want)) return e;
+    if (c->ecount != d.n_expert) return cudaSuccess;   // the fused sequence wants every expert
+    c->dec_grouped = decode_down_group_ok(d) && (T >= 40 || !decode_down_any_ok(d));
+    if (const cudaError_t e = dec_alloc(c, c->dec_one, T, false)) return e;
+    if (c->cfg.n_layer > 1 && dec_layout(c, c->dec_many, dec_most_rows(c), true) <= kDecAtOpen) return dec_alloc(c, c->dec_many, dec_most_rows(c), true);
+    return cudaSuccess;
+}
+// Whether the scratch for several layers is there, made when it is first wanted.  Where it cannot be had - the stream is being captured, or the
+// memory is short - the layers go one by one.
+bool stack_scratch(qkm_ctx* c) {
+    if (c->dec_many.mem) return true;
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(c->stream, &st) != cudaSuccess || st != cudaStreamCaptureStatusNone) {
+        cudaGetLastError();
+        return false;
+    }
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;   // (another thread's capture is not broken by it)
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    const cudaError_t e = dec_alloc(c, c->dec_many, dec_most_rows(c), true);
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    return e == cudaSuccess;
 }
 
 }  // namespace
@@ -363,8 +420,7 @@ extern "C" QKM_API void qkm_close(qkm_ctx* c) {
     for (auto& dm : c->dense) if (dm.tiles) cudaFree(dm.tiles);
     void* scratch[] = {c->argmax_scratch, c->dense_xb, c->dense_scale, c->sel, c->h, c->route_scratch, c->offsets, c->pairs, c->contrib, c->y2, c->x_stage, c->y_stage,
                        c->stack_x, c->stack_y, c->xscale, c->n_items, c->status, c->route_counter,
-                       c->planes8, c->lut_gu, c->lut_dd, c->lut_pf, c->dec_logits, c->dec_sel, c->dec_planes, c->dec_xscale, c->dec_h, c->dec_contrib,
-                       c->dec_groups, c->dec_counts,
+                       c->planes8, c->lut_gu, c->lut_dd, c->lut_pf, c->dec_one.mem, c->dec_many.mem,
                        c->xb, c->xnorm, c->hb, c->hscale, c->contrib_p, c->mma_items[0], c->mma_items[1],
                        c->pos_of, c->group_counts, c->ep_counts, c->ep_send_tok, c->ep_send_pos};
     for (void* p : scratch) if (p) cudaFree(p);
@@ -648,7 +704,8 @@ static int decode_fused(qkm_ctx* c, uint32_t first, uint32_t count, const float*
     const qkm_dims& d = c->cfg.dims;
     const uint32_t nb = (uint32_t)c->n_sms;
     // a layer on its own: the blocks of the kernels behind the router group its pairs themselves
-    const DecodeGroups groups = count == 1 ? DecodeGroups{} : DecodeGroups{c->dec_counts, c->dec_groups};
+    const qkm_ctx::DecScratch& m = count == 1 ? c->dec_one : c->dec_many;
+    const DecodeGroups groups{m.counts, m.groups};   // (none for one layer)
     RouteDecodeArgs ra{};
     GateupDecodeArgs ga{};
     DownDecodeArgs da{};
@@ -660,17 +717,17 @@ static int decode_fused(qkm_ctx* c, uint32_t first, uint32_t count, const float*
         ga.layer[l] = {t[2], t[3], t[5], t[6]};
         da.layer[l] = {t[4], t[7]};
     }
-    ra.x = x; ra.x_stride = x_stride; ra.sel = c->dec_sel; ra.sel_last = sel; ra.logits = c->dec_logits; ra.counter = c->route_counter;
-    ra.planes = c->dec_planes; ra.xscale = c->dec_xscale; ra.groups = groups; ra.n_tokens = n; ra.n_layers = count; ra.d = d;
+    ra.x = x; ra.x_stride = x_stride; ra.sel = m.sel; ra.sel_last = sel; ra.logits = m.logits; ra.counter = c->route_counter;
+    ra.planes = m.planes; ra.xscale = m.xscale; ra.groups = groups; ra.n_tokens = n; ra.n_layers = count; ra.d = d;
     QKM_LAUNCH(c, launch_route_decode(c->Lchain(), w.router_type, ra));
     c->prof_mark("moe.route");
-    ga.luts = c->lut_gu; ga.planes = c->dec_planes; ga.xscale = c->dec_xscale; ga.groups = groups; ga.sel = sel; ga.n_tokens = n; ga.n_layers = count;
-    ga.gateup_type = w.gateup_type; ga.h = c->dec_h; ga.h_last = h; ga.status = c->status; ga.d = d;
+    ga.luts = c->lut_gu; ga.planes = m.planes; ga.xscale = m.xscale; ga.groups = groups; ga.sel = sel; ga.n_tokens = n; ga.n_layers = count;
+    ga.gateup_type = w.gateup_type; ga.h = m.h; ga.h_last = h; ga.status = c->status; ga.d = d;
     QKM_LAUNCH(c, launch_decode_gateup(c->Lchain(), ga, nb));
     c->prof_mark("moe.gu");
-    da.lut = c->lut_dd; da.h = c->dec_h; da.h_last = h; da.sel = c->dec_sel; da.sel_last = sel; da.y = y; da.y_stride = y_stride;
-    da.groups = groups; da.contrib = c->dec_contrib; da.n_tokens = n; da.n_layers = count; da.status = c->status; da.d = d;
-    if (c->dec_contrib && decode_down_group_better(d, w.down_type, n)) QKM_LAUNCH(c, launch_decode_down_group(c->Lchain(), da, w.down_type, nb));
+    da.lut = c->lut_dd; da.h = m.h; da.h_last = h; da.sel = m.sel; da.sel_last = sel; da.y = y; da.y_stride = y_stride;
+    da.groups = groups; da.contrib = m.contrib; da.n_tokens = n; da.n_layers = count; da.status = c->status; da.d = d;
+    if (c->dec_grouped && decode_down_group_better(d, w.down_type, n)) QKM_LAUNCH(c, launch_decode_down_group(c->Lchain(), da, w.down_type, nb));
     else if (!decode_down_ok(d)) QKM_LAUNCH(c, launch_decode_down_any(c->Lchain(), da, w.down_type, nb));
     else if (w.down_type == QKM_TYPE_IQ4_XS) QKM_LAUNCH(c, launch_decode_down(c->Lchain(), da, nb));
     else QKM_LAUNCH(c, launch_decode_down_q6k(c->Lchain(), da, nb));
@@ -681,15 +738,16 @@ static int decode_fused(qkm_ctx* c, uint32_t first, uint32_t count, const float*
 // The fused sequence's limits; the tensors' are in qkm_layer_dev::fused_ok.
 static bool decode_fused_ok(const qkm_ctx* c, uint32_t n) {
     const qkm_dims& d = c->cfg.dims;
-    return n && c->dec_ok && c->dec_rows && route_decode_ok(d) && (decode_down_ok(d) || decode_down_any_ok(d) || c->dec_contrib);
+    return n && c->dec_ok && c->dec_one.mem && route_decode_ok(d) && (decode_down_ok(d) || decode_down_any_ok(d) || c->dec_grouped);
 }
 
 // Layers [first, first + count), all ready for the fused sequence, at most 64 tokens at a time: in runs of the same types, as many layers at once
 // as the scratch holds.
 static int decode_layers(qkm_ctx* c, uint32_t first, uint32_t count, const float* x, uint64_t x_stride, uint32_t n, float* y, uint64_t y_stride) {
     const qkm_dims& d = c->cfg.dims;
+    const uint32_t rows = count > 1 && stack_scratch(c) ? c->dec_many.rows : 0;
     for (uint32_t t = 0; t < n; t += 64) {
-        const uint32_t nt = n - t < 64 ? n - t : 64, most = c->dec_rows / nt < kDecMaxLayers ? c->dec_rows / nt : kDecMaxLayers;
+        const uint32_t nt = n - t < 64 ? n - t : 64, most = rows / nt < kDecMaxLayers ? rows / nt : kDecMaxLayers;
         for (uint32_t l = 0, k = 1; l < count; l += k, k = 1) {
             const qkm_layer_weights& w = c->layers[first + l].w;
             for (; l + k < count && k < most; ++k) {

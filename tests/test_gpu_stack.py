@@ -166,3 +166,69 @@ def test_layer_on_its_own_and_in_a_stack(pkg, orc, syn, n_embd, n_expert, n_used
         y, sel = d_y.download(np.float32, x.shape), ctx.last_sel(T)
     assert np.array_equal(y, together)
     check(syn, orc, layers, x, y, sel)
+
+
+def test_stack_scratch_comes_with_the_first_stack(pkg, syn):
+    """A context for many layers and slots holds no more at its opening than one for a single layer, but for a few MB; a stack's first call takes the
+    rest once, and only once."""
+    import torch
+    dims = syn.Dims()
+    free = lambda: (torch.cuda.synchronize(), torch.cuda.mem_get_info(0)[0])[1]
+
+    def opened(n_layer):
+        before = free()
+        ctx = pkg.Context(dims, n_layer=n_layer, max_tokens=64, device=0)
+        return ctx, before - free()
+
+    torch.zeros(1, device="cuda")
+    opened(1)[0].close()   # (what a first context sets up for the process)
+    one, few = opened(1)
+    one.close()
+    ctx, many = opened(40)
+    with ctx:
+        assert many - few <= 12 << 20, (few, many)
+        small = syn.make_layer(dims, seed=340)
+        for l in range(2):
+            ctx.upload_layer(l, small)
+        d = ctx.alloc(2 * 2 * 3 * dims.n_embd * 4)
+        at = []
+        for _ in range(3):
+            ctx.moe_decode_stack(0, 2, d, 3, d.ptr + 2 * 3 * dims.n_embd * 4)
+            at.append(free())
+        assert at[0] == at[1] == at[2]
+
+
+@pytest.mark.parametrize("T", [5, 64])
+def test_stack_first_called_under_capture(pkg, syn, T):
+    """No scratch for several layers yet and none can be had: the layers go one by one, and a replay gives the bits of the call outside."""
+    import torch
+    dims, L = syn.Dims(n_embd=1024, n_ff=512, n_expert=16, n_used=8), 14
+    layer = syn.make_layer(dims, seed=350)
+    x = torch.from_numpy(np.stack([syn.random_x(T, dims.n_embd, seed=351 + l) for l in range(L)])).cuda()
+    y, z = torch.zeros_like(x), torch.zeros_like(x)
+    stream = torch.cuda.Stream()
+    with pkg.Context(dims, n_layer=L, max_tokens=64, device=0) as ctx:
+        for l in range(L):
+            ctx.upload_layer(l, layer)
+        torch.cuda.synchronize()
+        ctx.set_stream(stream.cuda_stream)
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=stream):
+            before = ctx.launch_count()
+            ctx.moe_decode_stack(0, L, x.data_ptr(), T, y.data_ptr())
+            assert ctx.launch_count() - before >= 3 * L
+        for _ in range(2):
+            graph.replay()
+        torch.cuda.synchronize()
+        before = ctx.launch_count()
+        ctx.moe_decode_stack(0, L, x.data_ptr(), T, z.data_ptr())
+        stream.synchronize()
+        assert ctx.launch_count() - before <= 8
+        assert torch.isfinite(z).all() and torch.equal(y, z)
+        y.zero_()
+        torch.cuda.synchronize()
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(y, z)
+        ctx.set_stream(0)
+        del graph
