@@ -368,12 +368,12 @@ def run_ours(args, pkg, syn):
     # per-kernel timing of the dominant kernels over the same inputs (CUDA events, this stream)
     if rank == 0:
         kern = time_kernels(ctx, pkg, syn, torch, dev, stream, L, S, x_dev, distinct, dims)
-        dom = max(kern.values(), key=lambda k: k["ms_per_layer"])
+        dom = max(kern.values(), key=lambda k: k["ms_per_pass"])
         line["roofline"] = {
             "bound": "hbm", "kernel": dom["name"], "achieved": dom["gbs"], "peak": peaks["hbm_gbs"], "unit": "GB/s",
             "frac": dom["gbs"] / peaks["hbm_gbs"], "peak_source": peaks["source"] + " copy bandwidth",
             "frac_of_nominal_8TBs": dom["gbs"] / 8000.0, "traffic": ncu_traffic(dom["name"]),
-            "bytes_per_launch": dom["bytes_per_launch"], "ms_per_launch": dom["ms_per_layer"]}
+            "bytes_per_pass": dom["bytes_per_pass"], "ms_per_pass": dom["ms_per_pass"]}
         line["kernels"] = kern
         threads = orc.hardware_threads() or 1
         if world == 1:
@@ -384,6 +384,10 @@ def run_ours(args, pkg, syn):
             one = cpu_moe_sample(syn, orc_mod, dims, 4, 1, 1, syn.F16, syn.IQ3_XXS, syn.IQ4_XS)
             line["cpu_baseline"]["single_thread"] = {"value": 4 / (one * L), "unit": "tok/s", "cores": 1,
                                                      "sample": f"1 of {L} layers x 4 rows on one thread, scaled by layers"}
+            # the same layers one call each, as a program with an attention block between them makes them
+            with torch.cuda.stream(stream):
+                one_ms = timed(torch, R, stream, lambda: [ctx.moe_decode(l, x_dev[l], S, y_dev[l]) for l in range(L)], args.steps, 3)
+            line["decode_layer_by_layer"] = {"us_per_layer": one_ms * 1e3 / L, "tok_s": S / (one_ms * 1e-3)}
             line["decode_batch1"] = run_batch1(ctx, syn, torch, R, stream, L, dims, x_all, peaks, orc, layers_keep)
     R.barrier()
     ctx.close()
@@ -392,7 +396,7 @@ def run_ours(args, pkg, syn):
 
     # ---- the other type mixes the reference loads (src/main.cpp:1283-1291): a Q6_K down tensor, IQ4_XS
     # gate/up tensors.  Same three-kernel decode sequence on their own tile layouts.  Four rotating
-    # layers, same 16 slots.
+    # layers, called one by one, same 16 slots.
     if not args.no_sub and world == 1:
         QL = 4
         for key, gt, dt, what in (("decode_q6k_down", syn.IQ3_XXS, syn.Q6_K, "Q6_K down tensors (decode_down_q6k_kernel)"),
@@ -406,16 +410,17 @@ def run_ours(args, pkg, syn):
             with torch.cuda.stream(sq):
                 xq = torch.from_numpy(x_all[:QL].copy()).to(dev)
                 yq = torch.empty_like(xq)
-            cq.moe_decode_stack(0, QL, xq, S, yq); R.barrier()
+            q_pass = lambda: [cq.moe_decode(l, xq[l], S, yq[l]) for l in range(QL)]
+            q_pass(); R.barrier()
             refq = orc.moe_layer(q_layers[0], x_all[0], threads=orc.hardware_threads())
             errq = syn.rel_err_rows(yq[0].cpu().numpy(), refq["y"])
             assert errq < 1e-5, f"{key}: layer output error {errq}"
-            msq = timed(torch, R, sq, lambda: cq.moe_decode_stack(0, QL, xq, S, yq), args.steps, 3) / QL
-            line[key] = {"us_per_layer": msq * 1e3, "tok_s_through_40_layers": S / (msq * 40e-3),
+            msq = timed(torch, R, sq, q_pass, args.steps, 3) / QL
+            line[key] = {"us_per_layer": msq * 1e3, "tok_s_through_40_layers_one_by_one": S / (msq * 40e-3),
                          "rel_err_vs_oracle": errq, "layers_rotated": QL,
                          "note": f"working set {QL} layers x 0.4-0.5 GB > L2; {what}"}
             cq.close()
-            del xq, yq, cq
+            del xq, yq, q_pass, cq
             torch.cuda.empty_cache()
 
     # ---- the other configurations, as sub-objects of the same line
@@ -432,12 +437,12 @@ def run_ours(args, pkg, syn):
 
 
 def ncu_traffic(stage: str):
-    """DRAM bytes per launch (dram__bytes_read.sum + dram__bytes_write.sum) of a decode stage's
-    kernel, from profiles/ncu_traffic.json - written when the ncu capture summarised under
-    profiles/ was taken, with the commit it was taken at.  None when the file has no entry."""
+    """DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) and algorithmic bytes of a decode stage's launch, from
+    profiles/ncu_traffic.json - written when the ncu capture summarised under profiles/ was taken, of the layers and
+    tokens that the file names.  None when the file has no entry."""
     p = os.path.join(ROOT, "profiles", "ncu_traffic.json")
     try:
-        return json.load(open(p)).get(stage, {}).get("dram_bytes_per_launch")
+        return json.load(open(p)).get(stage)
     except Exception:
         return None
 
@@ -697,28 +702,30 @@ def run_gemv_sweep(args, pkg, syn, torch, R: Ranks, orc, peaks):
 def run_batch1(ctx, syn, torch, R, stream, L, dims, x_all, peaks, orc, layers_keep):
     """one MoE layer, decode batch 1 (the reference's `qk moe <layer>`
     harness, src/main.cpp:1221-1243: us per layer and GB/s over the weight bytes one token
-    touches).  The call rotates over all L layers of the stack (one token through each, replayed
-    as a graph), so every layer's weights come from HBM, not from L2: a cold figure, as stated."""
+    touches).  One call a layer, rotating over all L layers, so every layer's weights come from HBM, not from L2: a cold
+    figure, as stated.  (The stack call's layers go together, which no layer on its own does: its time is given beside it.)"""
     dev = R.dev
     with torch.cuda.stream(stream):
         x1 = torch.from_numpy(np.ascontiguousarray(x_all[:, :1])).to(dev)
         y1 = torch.empty_like(x1)
-    ctx.moe_decode_stack(0, L, x1, 1, y1); R.barrier()
+    one_by_one = lambda: [ctx.moe_decode(l, x1[l], 1, y1[l]) for l in range(L)]
+    one_by_one(); R.barrier()
     ref = orc.moe_layer(layers_keep[0], x_all[0, :1])
     err = syn.rel_err_rows(y1[0].cpu().numpy(), ref["y"])
     assert err < 1e-5, f"batch-1 layer output error {err}"
-    ms = timed(torch, R, stream, lambda: ctx.moe_decode_stack(0, L, x1, 1, y1), 20, 3) / L
+    ms = timed(torch, R, stream, one_by_one, 20, 3) / L
+    together = timed(torch, R, stream, lambda: ctx.moe_decode_stack(0, L, x1, 1, y1), 20, 3)
     nbytes = syn.layer_touched_bytes(dims, syn.F16, syn.IQ3_XXS, syn.IQ4_XS, dims.n_used)
     return {"workload": f"one layer, one token; rotating over {L} layers so weights stream from HBM (cold)",
             "us_per_layer": ms * 1e3, "active_bytes_per_layer": nbytes, "gbs": nbytes / (ms * 1e-3) / 1e9,
             "frac_of_measured_copy": nbytes / (ms * 1e-3) / 1e9 / peaks["hbm_gbs"], "frac_of_nominal_8TBs": nbytes / (ms * 1e-3) / 8e12,
-            "rel_err_vs_oracle": err}
+            "rel_err_vs_oracle": err, "stack_call_us": together * 1e3, "stack_call_layers": L}
 
 
 def time_kernels(ctx, pkg, syn, torch, dev, stream, L, S, x_dev, distinct, dims, reps=5):
-    """Average duration of every stage of the fused decode sequence (one launch per layer
-    per pass), from CUDA events recorded on the launching stream between the stages
-    (qkm_profile_*), with the algorithmic weight bytes each stage touches."""
+    """Average duration of every stage of a pass of the stack call that the headline times (all layers go through a stage
+    together), from CUDA events recorded on the launching stream between the stages (qkm_profile_*), with the algorithmic
+    weight bytes each stage touches."""
     rb = syn.row_bytes
     mean_u = float(np.mean(distinct))
     # the shared expert's matrices ride inside the routed kernels of the fused sequence
@@ -727,20 +734,19 @@ def time_kernels(ctx, pkg, syn, torch, dev, stream, L, S, x_dev, distinct, dims,
         "moe.gu": mean_u * 2 * dims.n_ff * rb(syn.IQ3_XXS, dims.n_embd) + 2 * dims.n_ff * rb(syn.Q8_0, dims.n_embd),
         "moe.dn": mean_u * dims.n_embd * rb(syn.IQ4_XS, dims.n_ff) + dims.n_embd * rb(syn.Q8_0, dims.n_ff),
     }
-    y = torch.empty(S, dims.n_embd, device=dev)
+    y = torch.empty_like(x_dev)
     ctx.profile_enable(True)
     acc = {}
     for _ in range(reps):
-        for l in range(L):
-            ctx.moe_decode(l, x_dev[l], S, y)
-            for k, v in ctx.profile_read().items():
-                acc[k] = acc.get(k, 0.0) + v
+        ctx.moe_decode_stack(0, L, x_dev, S, y)
+        for k, v in ctx.profile_read().items():
+            acc[k] = acc.get(k, 0.0) + v
     ctx.profile_enable(False)
     out = {}
     for k, v in acc.items():
-        ms = v / (reps * L)
-        nbytes = stage_bytes.get(k, 0)
-        out[k] = {"name": k, "ms_per_layer": ms, "bytes_per_launch": nbytes, "gbs": nbytes / (ms * 1e-3) / 1e9 if ms > 0 else 0.0}
+        ms = v / reps
+        nbytes = stage_bytes.get(k, 0) * L
+        out[k] = {"name": k, "ms_per_pass": ms, "bytes_per_pass": nbytes, "gbs": nbytes / (ms * 1e-3) / 1e9 if ms > 0 else 0.0}
     return out
 
 

@@ -249,7 +249,9 @@ QKM_API int qkm_moe_decode_stack_host(qkm_ctx *c, uint32_t layer_first, uint32_t
  * sequence, reported per label).  While enabled, qkm_moe_decode / qkm_moe_prefill
  * record a CUDA event on the context's stream after each stage; qkm_profile_read
  * synchronises and returns, for the LAST fused call, the number of stages, their
- * labels (16 bytes each, NUL-terminated) and their durations in milliseconds. */
+ * labels (16 bytes each, NUL-terminated) and their durations in milliseconds.
+ * A stack whose layers go together is one fused call; a label comes once for each
+ * run of layers or chunk of 64 tokens (16 stages at most are kept). */
 QKM_API int qkm_profile_enable(qkm_ctx *c, int on);
 QKM_API int qkm_profile_read(qkm_ctx *c, char *labels, float *ms, uint32_t max_stages);
 /* Selection records of the last fused call (device -> host copy, syncs). */

@@ -420,11 +420,15 @@ class Context:
         self.check(self.lib.qkm_profile_enable(self.h, int(on)))
 
     def profile_read(self) -> dict:
-        """Stage label -> milliseconds of the last fused call (synchronises)."""
+        """Stage label -> milliseconds of the last fused call (synchronises); runs of several layers or chunks of tokens are added up."""
         labels = C.create_string_buffer(16 * 16)
         ms = (C.c_float * 16)()
         n = self.check(self.lib.qkm_profile_read(self.h, labels, ms, 16))
-        return {labels.raw[16 * i:16 * i + 16].split(b"\0")[0].decode(): float(ms[i]) for i in range(n)}
+        out = {}
+        for i in range(n):
+            label = labels.raw[16 * i:16 * i + 16].split(b"\0")[0].decode()
+            out[label] = out.get(label, 0.0) + float(ms[i])
+        return out
 
     def last_sel(self, n) -> np.ndarray:
         sel = np.zeros(n, SEL_DTYPE)

@@ -918,9 +918,12 @@ extern "C" QKM_API int qkm_moe_decode_stack(qkm_ctx* c, uint32_t first, uint32_t
     // every layer's rows are at hand: the layers go through each stage together, unless an output overlaps a later layer's input
     const qkm_dims& d = c->cfg.dims;
     const uint64_t stride = (uint64_t)n * d.n_embd, xa = (uint64_t)(uintptr_t)x, ya = (uint64_t)(uintptr_t)y, bytes = count * stride * sizeof(float);
-    bool together = !c->profiling && decode_fused_ok(c, n) && (xa == ya || xa + bytes <= ya || ya + bytes <= xa);
+    bool together = decode_fused_ok(c, n) && (xa == ya || xa + bytes <= ya || ya + bytes <= xa);
     for (uint32_t l = 0; l < count && together; ++l) together = c->layers[first + l].fused_ok;
-    if (together) return decode_layers(c, first, count, x, stride, n, y, stride);
+    if (together) {
+        c->prof_begin();
+        return decode_layers(c, first, count, x, stride, n, y, stride);
+    }
     if (c->stream == nullptr || c->profiling || count < 2) return decode_stack_eager(c, first, count, x, n, y);
     qkm_ctx::StackGraph* g = nullptr;
     for (auto& e : c->stack_graphs)

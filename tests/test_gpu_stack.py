@@ -232,3 +232,24 @@ def test_stack_first_called_under_capture(pkg, syn, T):
         assert torch.equal(y, z)
         ctx.set_stream(0)
         del graph
+
+
+def test_stack_stage_times(pkg, syn):
+    """While stages are timed a stack takes the launches it takes otherwise, and a stage's time is all its runs' together."""
+    dims, T, L = syn.Dims(n_embd=512, n_ff=512, n_expert=16, n_used=4), 6, 4
+    layers = [syn.make_layer(dims, seed=360, layer=l, down_type=23 if l < 2 else 14) for l in range(L)]   # two runs
+    x = np.stack([syn.random_x(T, dims.n_embd, seed=361 + l) for l in range(L)])
+    with pkg.Context(dims, n_layer=L, max_tokens=T, device=0) as ctx:
+        for l, layer in enumerate(layers):
+            ctx.upload_layer(l, layer)
+        d_x, d_y = ctx.to_device(x), ctx.alloc(x.nbytes)
+        ctx.moe_decode_stack(0, L, d_x, T, d_y)
+        want = d_y.download(np.float32, x.shape)
+        ctx.profile_enable(True)
+        before = ctx.launch_count()
+        ctx.moe_decode_stack(0, L, d_x, T, d_y)
+        assert ctx.launch_count() - before == 6
+        ms = ctx.profile_read()
+        assert set(ms) == {"moe.route", "moe.gu", "moe.dn"} and all(0 < v < 100 for v in ms.values())
+        ctx.profile_enable(False)
+        assert np.array_equal(d_y.download(np.float32, x.shape), want)
