@@ -223,9 +223,9 @@ int layer_ready(qkm_ctx* c, uint32_t layer) {
 // tokens, 12 of 64; 39 KB a row for 256 experts, top 8, and 74 KB more where the down kernel groups by expert (batches from 40 tokens on).  With
 // 192 rows stacks of 64 tokens take 2 to 7 % longer, with 384 up to 1 %, with 1152 the same.
 constexpr uint32_t kDecRows = 768;
-// Up to this much for several layers is taken at qkm_open (a few slots); more only when a stack is first decoded (0.33 ms, once), since contexts
-// that prefill, or that decode layer by layer, have no use for it.
-constexpr size_t kDecAtOpen = 8u << 20;
+// Up to this much for several layers is taken at qkm_open: what a context for fewer than 40 tokens, one that decodes, can need.  More only when a
+// stack is first decoded (0.33 ms as a rule, once), since contexts that prefill, or step through their layers one by one, have no use for 85 to 105 MB.
+constexpr size_t kDecAtOpen = 40u << 20;
 
 // Bytes of the scratch for `rows` rows; with s.mem set, where its parts lie.
 size_t dec_layout(const qkm_ctx* c, qkm_ctx::DecScratch& s, uint32_t rows, bool several) {
