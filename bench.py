@@ -373,7 +373,7 @@ def run_ours(args, pkg, syn):
         line["roofline"] = {
             "bound": "hbm", "kernel": dom["name"], "achieved": dom["gbs"], "peak": peaks["hbm_gbs"], "unit": "GB/s",
             "frac": dom["gbs"] / peaks["hbm_gbs"], "peak_source": peaks["source"] + " copy bandwidth",
-            "frac_of_nominal_8TBs": dom["gbs"] / 8000.0, "traffic": ncu_traffic(dom["name"]),
+            "frac_of_nominal_8TBs": dom["gbs"] / 8000.0, "traffic": (ncu_traffic(dom["name"]) or {}).get("dram_bytes_per_launch"), "traffic_launch": ncu_traffic(dom["name"]),
             "bytes_per_launch": dom["bytes_per_pass"] / runs, "ms_per_launch": dom["ms_per_pass"] / runs}
         line["kernels"] = kern
         threads = orc.hardware_threads() or 1

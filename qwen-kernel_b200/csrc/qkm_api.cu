@@ -904,7 +904,7 @@ static int decode_stack_eager(qkm_ctx* c, uint32_t first, uint32_t count, const 
 }
 
 // Layers of the fused sequence go through each of its stages together: three or four launches for the stack, not for a layer (40 layers of
-// 16 tokens 2,740 us as a graph of their launches, 1,920 together; 24 layers of one token 560 and 124).  What is left - an output that
+// 16 tokens 2,740 us as a graph of their launches, 1,870 to 1,990 together; 24 layers of one token 560 and 114).  What is left - an output that
 // overlaps a later layer's input, a layer outside the fused sequence - goes layer by layer: the launches are captured into a CUDA graph the
 // first time an argument set is seen and replayed afterwards.  Capture needs a real stream: on the legacy default stream, while
 // profiling, or after an upload, the launches are issued one by one.

@@ -5,7 +5,7 @@
 // Replaces moe_down_iq4.comp / moe_down_q6k.comp + moe_down_q8b.comp and the slot-order sum of add_rms3_grouped.comp:22-27.
 //
 // The token-major kernels unpack an expert's weights once for every token that chose it.  Here the pairs are grouped by expert as in
-// the gate/up kernel (the router kernel's lists, over all layers of the call), a group is an expert with up to two of its tokens, and a
+// the gate/up kernel (of several layers the router kernel's lists, of one by every block itself), a group is an expert with up to two of its tokens, and a
 // team of two warps (one per 256 columns) walks 16-row tiles of a contiguous share of the (group, tile) list: at 64 tokens of 256 experts,
 // top 8, 317 groups instead of 512 pairs.  The price is the grouping, the contribution rows' way through the L2 and a second
 // launch, about 7 us together.
@@ -119,7 +119,8 @@ decode_down_group_kernel(const __grid_constant__ DownDecodeArgs a) {
             p_new = false;
             const DecodeGroup r = group(p_at);
             p_shared = r.shared();
-            p_src = p_shared ? a.layer[ONE ? 0 : p_at.l].sh + ((size_t)kb * RT + p_at.rt) * kTileQ8 : a.layer[ONE ? 0 : p_at.l].w + ((size_t)r.expert() * mat_tiles + (size_t)kb * RT + p_at.rt) * C::kTile;
+            const DownDecodeArgs::Mats& m = a.layer[ONE ? 0 : p_at.l];
+            p_src = p_shared ? m.sh + ((size_t)kb * RT + p_at.rt) * kTileQ8 : m.w + ((size_t)r.expert() * mat_tiles + (size_t)kb * RT + p_at.rt) * C::kTile;
         }
         const uint32_t n = p_shared ? dp::kHalfQ8 : C::kTile;
         mbar_expect_tx(my_bar + 8 * stage, n);

@@ -7,8 +7,8 @@
 // decode), and the shared expert rides in the same work list as groups of its own.
 //
 // Several layers whose rows are at hand together go through one launch: the list of work runs over all of them, so start-up, first
-// tiles and the uneven end are paid once (12 to 13 us of each kernel did not depend on the work: one layer of 16 tokens 41 us, 40 layers
-// together 27 us each).  A layer on its own takes a form without the other layers' bookkeeping.
+// tiles and the uneven end are paid once (12 to 13 us of each kernel did not depend on the work: one layer of 16 tokens 38 us, 40 layers
+// together 26 us each).  A layer on its own takes a form without the other layers' bookkeeping.
 //
 // Work: the flat list of (layer, group, 16-row tile) - a group is an expert with up to two
 // tokens, n_ff / 16 tiles each - is cut evenly and contiguously over teams of KB = n_embd / 256

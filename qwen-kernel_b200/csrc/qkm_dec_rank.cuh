@@ -247,8 +247,8 @@ struct Divisor {
 };
 // The warp's share of the list when it is cut into by_parts.d equal costs: its first place, and in `n` its tiles.  Even lanes
 // look for the share's begin, odd ones for its end.  (A list's cost in tiles fits 32 bits: at most 768 rows.)
-__device__ __forceinline__ ListPlace list_share(const LayerCuts& c, uint32_t n_tokens, uint32_t n_layers, const Divisor& by_tiles, uint32_t routed, const Divisor& by_shared, uint32_t part, const Divisor& by_parts,
-                                                uint32_t& n) {
+__device__ __forceinline__ ListPlace list_share(const LayerCuts& c, uint32_t n_tokens, uint32_t n_layers, const Divisor& by_tiles, uint32_t routed,
+                                                const Divisor& by_shared, uint32_t part, const Divisor& by_parts, uint32_t& n) {
     const uint32_t tiles = by_tiles.d, cut = part + (threadIdx.x & 1u), total = c.cost[n_layers] * tiles, q = by_parts(total);
     const uint32_t want = q * cut + by_parts((total - q * by_parts.d) * cut);   // total * cut / parts; in tiles times weight
     uint32_t l = 0, last = n_layers - 1;   // the last layer that does not begin after `want`

@@ -6,8 +6,8 @@
 //   * logits blocks: pairs of router rows and up to eight tokens each, f64 accumulation - the logits are
 //     those of the CPU reference's f64 router (src/main.cpp:1320-1324) up to the order of the
 //     f64 additions, so they are ranked as they are, without an error bound; the block that
-//     finishes a group of tokens last ranks them, one warp per token, and the one that ranks a layer's
-//     last group groups the layer's pairs;
+//     finishes a group of tokens last ranks them, one warp per token, and, of several layers, the one that ranks
+//     a layer's last group groups the layer's pairs;
 //   * one block per token encodes x as digit planes (and their negatives, which the IQ3_XXS
 //     kernel multiplies with its sign masks) and evaluates the shared expert's gate
 //     sigmoid(gis . x) in f64 (moe_select.comp's wShared).
@@ -263,7 +263,7 @@ bool route_decode_ok(const qkm_dims& d) { return d.n_expert <= rk::kMaxExperts &
 
 // Tokens of a group: as few as the batch has (a group of eight costs one token as much as eight).  Pairs a block: one for a layer on its own and while
 // the blocks find room on the SMs at once (a chain of latencies: start-up, loads, ticket), more when layers go together, so that a block's share of
-// that chain is small: 40 layers of 16 tokens 159 us with one pair a block, 125 so.  About kBlocks blocks: with half as many 24 layers of one token
+// that chain is small: 40 layers of 16 tokens 159 us with one pair a block, 119 so.  About kBlocks blocks: with half as many 24 layers of one token
 // 117 -> 119 us for the whole call, 12 of one 71 -> 74, 6 of 12 243 -> 250; with twice as many 24 of one 117 -> 120, 24 of 5 413 -> 422, 6 of 16
 // 301 -> 308 (but 4 of 3, 512 experts, 85 -> 82).  At most 8, 16 or 32 pairs a block: the same.
 // Blocks of several pairs keep the x of up to four tokens as doubles (the converter takes 16 lanes a cycle and SM, the f64 units 64): 24 layers of
