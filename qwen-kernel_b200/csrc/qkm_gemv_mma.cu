@@ -473,14 +473,14 @@ gemv_tile_kernel(const uint8_t* __restrict__ W, const float* __restrict__ x, flo
             } else {
                 q6k_tile<false>(blk0, blk1, t, b0, b1, v0, v1);
             }
-            stage_read();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(bar_empty + 8 * c_stage);
-            if (++c_stage == n_stages) { c_stage = 0; c_phase ^= 1u; }
+            // (ahead of the stage's way back: with what was read last in hand no read of it is under way)
             v0 += __shfl_xor_sync(0xFFFFFFFFu, v0, 1); v1 += __shfl_xor_sync(0xFFFFFFFFu, v1, 1);
             if (TYPE == QKM_TYPE_Q6_K) {   // all four lanes of a row hold a share
                 v0 += __shfl_xor_sync(0xFFFFFFFFu, v0, 2); v1 += __shfl_xor_sync(0xFFFFFFFFu, v1, 2);
             }
+            __syncwarp();
+            if (lane == 0) mbar_arrive(bar_empty + 8 * c_stage);
+            if (++c_stage == n_stages) { c_stage = 0; c_phase ^= 1u; }
             if (t == 0) { rw[q * gq::kRows + g] = v0; rw[q * gq::kRows + g + 8] = v1; }
         }
         __syncthreads();
