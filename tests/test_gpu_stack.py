@@ -225,13 +225,19 @@ def test_stack_first_called_under_capture(pkg, syn, T):
         stream.synchronize()
         assert ctx.launch_count() - before <= 8
         assert torch.isfinite(z).all() and torch.equal(y, z)
-        y.zero_()
-        torch.cuda.synchronize()
-        graph.replay()
-        torch.cuda.synchronize()
-        assert torch.equal(y, z)
+        together = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(together, stream=stream):   # with the scratch there: the layers together
+            before = ctx.launch_count()
+            ctx.moe_decode_stack(0, L, x.data_ptr(), T, y.data_ptr())
+            assert ctx.launch_count() - before <= 8
+        for g in (graph, together, graph, together):
+            y.zero_()
+            torch.cuda.synchronize()
+            g.replay()
+            torch.cuda.synchronize()
+            assert torch.equal(y, z)
         ctx.set_stream(0)
-        del graph
+        del graph, together, g
 
 
 def test_stack_stage_times(pkg, syn):
